@@ -4,6 +4,7 @@ import pathlib
 
 _HERE = pathlib.Path(__file__).resolve().parent
 _LIB = None
+_FRONT = None
 
 
 class RkError(RuntimeError):
@@ -110,6 +111,27 @@ def lib():
         L.rk_debug_set_prefill_perturb.argtypes = [C.c_int]
         _LIB = L
     return _LIB
+
+
+def front():
+    """The native front end (csrc/rk_front.cpp): checks, allocation and the call, in one step from torch tensors.  Raises
+    if it was never built: there is no other path."""
+    global _FRONT
+    if _FRONT is None:
+        lib()                                   # the front end is linked against the library beside it
+        so = _HERE / "_rk_front.so"
+        if not so.exists():
+            raise RuntimeError(f"{so} is missing: run `python radiance-kernels_b200/build.py`")
+        import importlib.machinery
+        import importlib.util
+
+        import torch                            # noqa: F401  (its libraries have to be in the process first)
+        loader = importlib.machinery.ExtensionFileLoader("_rk_front", str(so))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_rk_front", loader))
+        loader.exec_module(mod)
+        mod.set_error(check)
+        _FRONT = mod
+    return _FRONT
 
 
 def check(code, where):
