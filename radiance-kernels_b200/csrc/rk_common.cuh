@@ -74,12 +74,10 @@ template <int FMT> RK_DEVINL uint32_t encode_rne(float xf) {
 // e = ceil(log2(amax / FMT_MAX)); returns e, the clamped E8M0 code and 2^-e.
 template <int FMT> RK_DEVINL void block_scale(float amax, uint32_t& code, float& pow2_neg_e) {
   using F = FmtT<FMT>;
-  const uint32_t ab = __float_as_uint(amax);
-  const int e = ((int)((ab >> 23) & 0xFFu) - 127 - F::emax) + ((ab & 0x7FFFFFu) > F::thresh ? 1 : 0);
-  int sc = e + 127;
-  sc = sc < 0 ? 0 : (sc > 254 ? 254 : sc);
-  code = (uint32_t)sc;
-  pow2_neg_e = __uint_as_float((uint32_t)(127 - e) << 23);
+  // the carry of the addition is the "+1 above the largest mantissa"; t = biased exponent of amax with it
+  const uint32_t t = (__float_as_uint(amax) + (0x7FFFFFu - F::thresh)) >> 23;
+  code = (uint32_t)max((int)t - F::emax, 0);                            // at most 255 - emax
+  pow2_neg_e = __uint_as_float((uint32_t)(254 + F::emax - (int)t) << 23);
 }
 
 // Exact decode of an element code to fp32.

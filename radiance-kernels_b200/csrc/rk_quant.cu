@@ -21,6 +21,7 @@
 // to it on every finite fp32 input (all 2^32 bit patterns are swept in the GPU
 // tests); blocks that hold a NaN or an infinity take the integer encoder.
 #include <algorithm>
+#include <type_traits>
 
 #include "rk_common.cuh"
 #include "rk_internal.h"
@@ -150,6 +151,70 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const float4* __rest
   }
 }
 
+// 8 consecutive elements as loaded: 8 bf16 or 8 fp32.  PIECE = bytes per load instruction (16, or 4 for an unaligned base)
+template <bool BF16IN> struct Raw8 { uint32_t w[BF16IN ? 4 : 8]; };
+template <bool BF16IN, int PIECE> RK_DEVINL Raw8<BF16IN> load_raw8(const uint8_t* src) {
+  constexpr int kWords = BF16IN ? 4 : 8;
+  Raw8<BF16IN> r;
+  if (PIECE == 16) {
+#pragma unroll
+    for (int i = 0; i < kWords / 4; ++i) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(src) + i);
+      r.w[4 * i] = q.x; r.w[4 * i + 1] = q.y; r.w[4 * i + 2] = q.z; r.w[4 * i + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) r.w[i] = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
+  }
+  return r;
+}
+// the same elements as fp32 (exact)
+template <bool BF16IN> RK_DEVINL void widen8(const Raw8<BF16IN>& r, float (&v)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (BF16IN) v[j] = __uint_as_float((j & 1) ? (r.w[j / 2] & 0xFFFF0000u) : (r.w[j / 2] << 16));
+    else v[j] = __uint_as_float(r.w[j]);
+  }
+}
+
+// (Scalar products on purpose: mul.f32x2 takes two cycles of the heavy FMA pipe, and packing its operands adds moves.)
+// max(|a|, |b|, |c|), NaN if any of them is
+RK_DEVINL float max3_abs_nan(float a, float b, float c) { float d; asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+RK_DEVINL float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+
+// One lane's 8 N elements of a 32-element block that 4 / N consecutive lanes share (they call together): the codes and the
+// block's scale code.  Returns false where the block holds a NaN or an infinity (the maximum lets NaN through, so one
+// comparison tells): its codes are then those of the COLD form, which takes the maximum without the NaNs, as the
+// reference's compare loop does, and the integer encoder.  A caller runs the hot form over all it has and the cold one
+// again only if some block asked for it, so that the hot loop carries no code that never runs.
+// UNIT: no block scale (codes under 2^0, scale code 127).
+template <int FMT, bool UNIT, int N, bool COLD> RK_DEVINL bool quantize_lanes(const float (&v)[N][8], int lane, uint2 (&w)[N], uint32_t& scode) {
+  constexpr int kLanes = 4 / N;
+  const uint32_t mask = (0xFu >> (4 - kLanes)) << (lane & (32 - kLanes));
+  float m = 0.0f;
+#pragma unroll
+  for (int h = 0; h < N; ++h)
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) m = COLD ? fmaxf(m, fmaxf(fabsf(v[h][j]), fabsf(v[h][j + 1]))) : max3_abs_nan(m, v[h][j], v[h][j + 1]);
+#pragma unroll
+  for (int s = 1; s < kLanes; s *= 2) {
+    const float o = __shfl_xor_sync(mask, m, s);
+    m = COLD ? fmaxf(m, o) : max_nan(m, o);
+  }
+  float p2 = 1.0f;
+  scode = UNIT ? 127u : 0u;
+  if (!UNIT && m > 0.0f) block_scale<FMT>(m, scode, p2);
+#pragma unroll
+  for (int h = 0; h < N; ++h) {
+    float s[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = __fmul_rn(v[h][j], p2);
+    w[h] = COLD ? make_uint2(ref_encode4<FMT>(s[0], s[1], s[2], s[3]), ref_encode4<FMT>(s[4], s[5], s[6], s[7]))
+                : make_uint2(hw_encode4<FMT>(s[0], s[1], s[2], s[3]), hw_encode4<FMT>(s[4], s[5], s[6], s[7]));
+  }
+  return m < __int_as_float(0x7f800000);
+}
+
 // RoPE fused with the block quantizer, so that rotated Q / K never exist in HBM as fp32: rotate-half form with
 // half-width caches (lib/golden/golden.py:229-236): out[:half] = c0 cos - c1 sin, out[half:] = c1 cos + c0 sin,
 // every product and sum rounded on its own (no fused multiply-add, as numpy float32 does), then the lib/golden block
@@ -225,71 +290,206 @@ __global__ void __launch_bounds__(256) rope_quantize_rows_kernel(const float* __
 // normalized activation never exists in HBM as fp32.  Bit-exact with the reference's fp32 path
 // (lib/golden/golden.py:203-216): the sum of squares runs in index order with every product and sum rounded on its
 // own, mean = ss / K, rms = 1 / sqrt(mean + eps) (correctly rounded square root and division), y = (x * rms) * gamma.
-// A warp owns 32 rows.  Per 32-column chunk it loads a 32 x 32 tile with coalesced row reads into shared memory;
-// lane L then walks row L of the tile: in the first pass it extends its row's sequential sum, in the second pass
-// the chunk is exactly one MX block of its row (amax, scale, codes: 32 bytes stored at once).
 // UNIT: no block scale (code = E4M3(y) under 2^0, every scale byte 0x7F), the reference kernel's own choice
 // (kernels/rmsnorm_qkv_fused/gen_data.py:33-41: the prologue owns the row scaling).
-template <int FMT, bool BF16IN, bool UNIT>
-__global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const void* __restrict__ xin, int64_t rows, int K,
-                                                               const float* __restrict__ gamma, float eps,
-                                                               uint8_t* __restrict__ codes, uint8_t* __restrict__ scales) {
-  __shared__ float tile_all[8][32][33];
-  __shared__ float gam_all[8][32];
+//
+// The index-order sum is a chain of K dependent additions per row, 4.3 cycles each: 9 us for K = 4096, about what the
+// input takes to arrive from HBM.  So all chains of the machine run at once -- a CTA owns up to 16 rows, one lane of one
+// warp each -- and that warp does nothing but 16-byte shared-memory reads and additions (5.1 cycles a step alone on its
+// scheduler, 6.7 beside the other CTAs; with the squares in its own instruction stream 6.4 and 9).  Four other warps load
+// the rows two chunks of 256 elements ahead in registers and leave the squares in one of two buffers whose row pitch (1040
+// bytes) gives eight lanes reading 16 bytes of their own rows eight different bank groups.  When the chains are done all
+// warps normalize and quantize; the input then comes from L2 (DRAM reads it once), and that phase is bound by its
+// instructions.
+// 8192 x 4096 bf16: 1362 us with one warp per 32 rows doing both passes from 4-byte shared-memory reads, now 38.5 us.
+namespace rms {
+constexpr int kThreads = 256, kWarps = kThreads / 32, kHelpers = 4, kCtasPerSm = 4;
+constexpr int kChunk = 256, kPitch = kChunk * 4 + 16, kBufs = 2;        // elements per chunk, bytes of a row of squares
+constexpr int kHalf = kChunk / 8;                                       // float4s of a row: first halves of the lanes' eight, then second
+constexpr int kMaxRows = 16;
+constexpr int kRowsPerHelper = (kMaxRows + kHelpers - 1) / kHelpers;
+constexpr int kFull = 1, kEmpty = kFull + kBufs;                        // named barriers
+}  // namespace rms
+// barrier ID or ID + 1 (constants: a register would make the kernel claim all sixteen)
+template <int ID> RK_DEVINL void named_sync(int which) {
+  if (which) asm volatile("bar.sync %0, %1;" ::"n"(ID + 1), "n"((1 + rms::kHelpers) * 32) : "memory");
+  else asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"((1 + rms::kHelpers) * 32) : "memory");
+}
+template <int ID> RK_DEVINL void named_arrive(int which) {
+  if (which) asm volatile("bar.arrive %0, %1;" ::"n"(ID + 1), "n"((1 + rms::kHelpers) * 32) : "memory");
+  else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"((1 + rms::kHelpers) * 32) : "memory");
+}
+
+// PIECE: bytes of one global load: 16, or 4 where x or gamma is not 16-byte aligned.
+template <int FMT, bool BF16IN, bool UNIT, int PIECE>
+__global__ void __launch_bounds__(rms::kThreads, rms::kCtasPerSm)
+rmsnorm_quantize_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int rows_per_cta, const float* __restrict__ gamma,
+                        float eps, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales) {
+  using namespace rms;
+  extern __shared__ __align__(16) uint8_t rms_smem[];                   // [kBufs][n_rows][kPitch] squares
+  __shared__ float rms_row[kMaxRows];
+  constexpr int kElem = BF16IN ? 2 : 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float (*tile)[33] = tile_all[warp];
-  float* gam = gam_all[warp];
-  const int64_t n_groups = (rows + 31) / 32;
-  for (int64_t grp = (int64_t)blockIdx.x * 8 + warp; grp < n_groups; grp += (int64_t)gridDim.x * 8) {
-    const int64_t row0 = grp * 32;
-    auto load_tile = [&](int c0) {
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) {
-        const int64_t r = row0 + i;
-        float v = 0.0f;
-        if (r < rows) {
-          if (BF16IN) v = __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(xin)[r * K + c0 + lane] << 16);
-          else v = reinterpret_cast<const float*>(xin)[r * K + c0 + lane];
-        }
-        tile[i][lane] = v;
-      }
-    };
+  // Schedulers: the chains run on the first two, the squares on the other two (a burst of squares beside a chain takes
+  // its issue slots).  Blocks go to the SMs in rounds of gridDim / kCtasPerSm: alternate rounds take warp 0 and warp 1.
+  const int chain_warp = (int)(blockIdx.x / ((gridDim.x + kCtasPerSm - 1) / kCtasPerSm)) & 1;
+  const int helper = (warp & 2) ? (warp & 1) + (warp >> 2) * 2 : -1;       // warps 2, 3, 6, 7
+  const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
+  const int n_rows = (int)min((int64_t)rows_per_cta, rows - row0);
+  const int64_t row_bytes = (int64_t)K * kElem;
+  const uint8_t* xr = x + row0 * row_bytes;
+  const int n_chunks = (K + kChunk - 1) / kChunk;
+  const int buf_bytes = n_rows * kPitch;
+
+  if (warp == chain_warp) {
+    // ---- the chains ---------------------------------------------------------------------------------------------
     float ss = 0.0f;
-    for (int c0 = 0; c0 < K; c0 += 32) {
-      load_tile(c0);
-      __syncwarp();
+    for (int c = 0; c < n_chunks; ++c) {
+      named_sync<kFull>(c & 1);
+      if (lane < n_rows) {
+        const float4* src = reinterpret_cast<const float4*>(rms_smem + (c & 1) * buf_bytes + lane * kPitch);
+        const int n4 = min(kChunk, K - c * kChunk) / 4;                 // a multiple of 8
+        float4 s[2][4];
+        auto fetch = [&](int i, float4 (&d)[4]) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) { const float v = tile[lane][j]; ss = __fadd_rn(ss, __fmul_rn(v, v)); }
+          for (int q = 0; q < 4; ++q) d[q] = src[(q & 1) * kHalf + i / 2 + q / 2];
+        };
+        auto chain = [&](const float4 (&d)[4]) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            ss = __fadd_rn(ss, d[q].x); ss = __fadd_rn(ss, d[q].y);
+            ss = __fadd_rn(ss, d[q].z); ss = __fadd_rn(ss, d[q].w);
+          }
+        };
+        fetch(0, s[0]);
+        for (int i = 0; i < n4; i += 8) {
+          fetch(i + 4, s[1]);
+          chain(s[0]);
+          fetch(i + 8 < n4 ? i + 8 : 0, s[0]);
+          chain(s[1]);
+        }
+      }
       __syncwarp();
+      if (c + kBufs < n_chunks) named_arrive<kEmpty>(c & 1);
     }
-    const float rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
-    const int64_t r = row0 + lane;
-    for (int c0 = 0; c0 < K; c0 += 32) {
-      load_tile(c0);
-      gam[lane] = gamma[c0 + lane];
-      __syncwarp();
-      float y[32];
-      float amax = 0.0f, nonfinite = 0.0f;
+    if (lane < n_rows) rms_row[lane] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+  } else if (helper >= 0) {
+    // ---- squares: rows helper, helper + 4, ... of every chunk, two chunks ahead in registers (one for fp32 input) -------
+    constexpr int kAhead = BF16IN ? 2 : 1;
+    Raw8<BF16IN> raw[kAhead][kRowsPerHelper];
+    const int n_mine = (n_rows - helper + kHelpers - 1) / kHelpers;     // rows of this warp
+    const int64_t row_step = kHelpers * row_bytes;
+    const uint8_t* src = xr + helper * row_bytes + lane * 8 * kElem;    // advances by a chunk with every fetch
+    float4* const dst0 = reinterpret_cast<float4*>(rms_smem + helper * kPitch) + lane;
+    auto fetch = [&](int c, Raw8<BF16IN> (&d)[kRowsPerHelper]) {
+      if (c * kChunk + lane * 8 < K) {
+        const uint8_t* q = src;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        y[j] = __fmul_rn(__fmul_rn(tile[lane][j], rms), gam[j]);
-        amax = fmaxf(amax, fabsf(y[j]));
-        nonfinite = fmaf(y[j], 0.0f, nonfinite);
+        for (int k = 0; k < kRowsPerHelper; ++k) {
+          if (k < n_mine) d[k] = load_raw8<BF16IN, PIECE>(q);
+          q += row_step;
+        }
       }
-      __syncwarp();
-      uint32_t scode = UNIT ? 127u : 0u; float p2 = 1.0f;
-      if (!UNIT && amax > 0.0f) block_scale<FMT>(amax, scode, p2);
-      uint32_t w[8];
+      src += kChunk * kElem;
+    };
+    auto square = [&](int c, const Raw8<BF16IN> (&d)[kRowsPerHelper]) {
+      if (c >= kBufs) named_sync<kEmpty>(c & 1);
+      float4* dst = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(dst0) + (c & 1) * buf_bytes);
+      if (c * kChunk + lane * 8 < K) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        w[q] = (nonfinite == 0.0f) ? hw_encode4<FMT>(y[4 * q] * p2, y[4 * q + 1] * p2, y[4 * q + 2] * p2, y[4 * q + 3] * p2)
-                                   : ref_encode4<FMT>(y[4 * q] * p2, y[4 * q + 1] * p2, y[4 * q + 2] * p2, y[4 * q + 3] * p2);
-      if (r < rows) {
-        uint4* dst = reinterpret_cast<uint4*>(codes + r * K + c0);
-        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        scales[r * (K / 32) + c0 / 32] = (uint8_t)scode;
+        for (int k = 0; k < kRowsPerHelper; ++k) {
+          if (k < n_mine) {
+            float v[8];
+            widen8<BF16IN>(d[k], v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(v[j], v[j]);
+            dst[k * (kHelpers * kPitch / 16)] = make_float4(v[0], v[1], v[2], v[3]);
+            dst[k * (kHelpers * kPitch / 16) + kHalf] = make_float4(v[4], v[5], v[6], v[7]);
+          }
+        }
       }
+      named_arrive<kFull>(c & 1);
+    };
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) fetch(a, raw[a]);
+    for (int c = 0; c < n_chunks; c += kAhead) {
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        if (c + a < n_chunks) {
+          square(c + a, raw[a]);
+          fetch(c + a + kAhead, raw[a]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- normalize and quantize: a warp keeps 512 columns (16 per lane, 2 lanes per block; gamma in registers) and walks
+  // the rows, the loads of two more rows in flight; with fewer column units than warps several warps share one ------------
+  // (Scale bytes meet in shared memory first: a byte store per 32 elements cost a fifth of this phase.)
+  const bool stage_scales = K / 32 <= kBufs * kPitch;                   // they fit where the squares were
+  const int per_row = (K + 511) / 512, parts = max(1, kWarps / per_row);
+  const int part = warp / per_row;
+  auto quantize_rows = [&](auto cold_tag) -> bool {
+    constexpr bool COLD = decltype(cold_tag)::value;
+    bool finite = true;
+    if (part >= parts) return finite;
+    for (int u = warp - part * per_row; u < per_row; u += kWarps) {
+      const int col = u * 512 + lane * 16;
+      if (col >= K) continue;                                           // whole 2-lane groups: K % 32 == 0
+      const int64_t src_step = parts * row_bytes, dst_step = (int64_t)parts * K;
+      const int sc_step = parts * (K / 32);
+      const uint8_t* src = xr + part * row_bytes + (int64_t)col * kElem;
+      uint8_t* dst = codes + (row0 + part) * K + col;
+      uint8_t* sdst = (stage_scales ? rms_smem : scales + row0 * (K / 32)) + part * (K / 32) + col / 32;
+      float g[2][8];
+      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col)), g[0]);
+      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col + 8)), g[1]);
+      constexpr int kAhead = COLD || !BF16IN ? 1 : 2;
+      Raw8<BF16IN> raw[kAhead][2];
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        if (part + a * parts < n_rows) { raw[a][0] = load_raw8<BF16IN, PIECE>(src); raw[a][1] = load_raw8<BF16IN, PIECE>(src + 8 * kElem); }
+        src += src_step;
+      }
+#pragma unroll 1
+      for (int r0 = part; r0 < n_rows; r0 += kAhead * parts) {
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) {
+          const int r = r0 + a * parts;
+          if (r < n_rows) {
+            const float rms = rms_row[r];
+            float v[2][8];
+            widen8<BF16IN>(raw[a][0], v[0]);
+            widen8<BF16IN>(raw[a][1], v[1]);
+            if (r + kAhead * parts < n_rows) { raw[a][0] = load_raw8<BF16IN, PIECE>(src); raw[a][1] = load_raw8<BF16IN, PIECE>(src + 8 * kElem); }
+            src += src_step;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[h][j] = __fmul_rn(__fmul_rn(v[h][j], rms), g[h][j]);
+            uint32_t scode;
+            uint2 w[2];
+            finite &= quantize_lanes<FMT, UNIT, 2, COLD>(v, lane, w, scode);
+            __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0].x, w[0].y, w[1].x, w[1].y));
+            if ((lane & 1) == 0) *sdst = (uint8_t)scode;
+            dst += dst_step;
+            sdst += sc_step;
+          }
+        }
+      }
+    }
+    return finite;
+  };
+  if (__syncthreads_or(!quantize_rows(std::false_type{}))) quantize_rows(std::true_type{});
+  if (stage_scales) {
+    __syncthreads();
+    const int n = n_rows * (K / 32);                                    // contiguous in memory, as the CTA's rows are
+    uint8_t* out = scales + row0 * (K / 32);
+    if ((reinterpret_cast<uintptr_t>(out) & 3) == 0 && (n & 3) == 0) {
+      for (int i = threadIdx.x; i < n / 4; i += kThreads) reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(rms_smem)[i];
+    } else {
+      for (int i = threadIdx.x; i < n; i += kThreads) out[i] = rms_smem[i];
     }
   }
 }
@@ -909,11 +1109,28 @@ int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads
 int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const float* gamma, float eps, int fmt,
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   if (rows == 0 || K == 0) return RK_OK;
-  const int64_t groups = (rows + 31) / 32;
-  const int grid = (int)std::min<int64_t>((groups + 7) / 8, (int64_t)num_sms() * 8);
-#define RK_RN(BF, UN) RK_DISPATCH_FMT(fmt, (rmsnorm_quantize_kernel<F, BF, UN><<<grid, 256, 0, st>>>(x, rows, K, gamma, eps, codes, scales)))
-  if (bf16) { if (unit_scale) { RK_RN(true, true); } else { RK_RN(true, false); } }
-  else      { if (unit_scale) { RK_RN(false, true); } else { RK_RN(false, false); } }
+  // Rows per CTA: as few whole waves of resident CTAs as kMaxRows each allow, with the rows spread evenly over them (one
+  // wave and 14 rows for 8192); one row per CTA below one CTA per slot, so that few rows still reach every SM.
+  const int64_t slots = (int64_t)num_sms() * rms::kCtasPerSm;
+  const int64_t waves = (rows + slots * rms::kMaxRows - 1) / (slots * rms::kMaxRows);
+  const int per_cta = (int)((rows + slots * waves - 1) / (slots * waves));
+  const int64_t grid = (rows + per_cta - 1) / per_cta;
+  if (grid > 0x7FFFFFFF) return RK_ERR_BAD_SHAPE;
+  const int smem = rms::kBufs * per_cta * rms::kPitch;
+  const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
+  const uint8_t* xb = reinterpret_cast<const uint8_t*>(x);
+#define RK_RN(BF, UN, PC) RK_DISPATCH_FMT(fmt, {                                                                            \
+    auto kern = rmsnorm_quantize_kernel<F, BF, UN, PC>;                                                                    \
+    if (smem > 48 * 1024) {                                                                                                \
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rms::kBufs * rms::kMaxRows * rms::kPitch); \
+      if (e != cudaSuccess) return (int)e;                                                                                 \
+    }                                                                                                                      \
+    kern<<<(unsigned)grid, rms::kThreads, smem, st>>>(xb, rows, K, per_cta, gamma, eps, codes, scales);                      \
+  })
+#define RK_RNB(BF, UN) if (wide) { RK_RN(BF, UN, 16); } else { RK_RN(BF, UN, 4); }
+  if (bf16) { if (unit_scale) { RK_RNB(true, true); } else { RK_RNB(true, false); } }
+  else      { if (unit_scale) { RK_RNB(false, true); } else { RK_RNB(false, false); } }
+#undef RK_RNB
 #undef RK_RN
   return (int)cudaGetLastError();
 }

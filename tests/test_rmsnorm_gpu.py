@@ -64,3 +64,22 @@ def test_zero_rows_and_huge_rows():
     want_c, want_s = oracle.quantize(oracle.rmsnorm(x, gamma, 1e-6))
     c, s = rk.rmsnorm_mx_quantize(torch.from_numpy(x).cuda(), torch.from_numpy(gamma).cuda(), 1e-6)
     assert np.array_equal(np_(c), want_c) and np.array_equal(np_(s), want_s)
+
+
+@pytest.mark.parametrize("rows,K,bf16,shift,inf_gamma", [(1, 96, True, 0, False), (593, 288, False, 0, True), (593, 544, True, 2, False),
+                                                         (9473, 64, True, 0, True), (2400, 800, False, 1, False), (3, 66592, True, 0, False)])
+def test_row_groups_chunks_and_alignment(rows, K, bf16, shift, inf_gamma):
+    """Ragged row groups (one CTA slot per row and one row more, two waves), ragged column chunks, a base that is only 4-byte
+    aligned, scale rows too long to meet in shared memory, and an infinite gamma (blocks that need the integer encoder)."""
+    rng = np.random.default_rng(rows + K)
+    x = rng.standard_normal((rows, K)).astype(np.float32)
+    gamma = (0.75 + 0.5 * rng.random(K)).astype(np.float32)
+    if inf_gamma:
+        gamma[K // 2] = np.inf
+    flat = torch.empty(rows * K + shift, dtype=torch.bfloat16 if bf16 else torch.float32, device="cuda")
+    xt = flat[shift:].view(rows, K)
+    xt.copy_(torch.from_numpy(x))
+    want_c, want_s = _expect(np_(xt.float()), gamma, 1e-5, 0, False)
+    c, s = rk.rmsnorm_mx_quantize(xt, torch.from_numpy(gamma).cuda(), 1e-5)
+    assert np.array_equal(np_(s), want_s)
+    assert np.array_equal(np_(c), want_c)
