@@ -500,14 +500,13 @@ int rk_attn_decode_num_splits(const rk_decode_args* a) {
   if (check_decode_shape(a) != RK_OK) return 0;
   const int tiles = (a->L + 127) / 128;
   if (a->num_splits > 0) return a->num_splits < tiles ? a->num_splits : tiles;
-  // Pick the split count with the lowest modelled time (microseconds; fitted to B = 1 .. 64 at L = 4096 .. 32768 with
-  // 32 and 64 heads on 8): streaming time = bytes / bandwidth, where the bandwidth grows with the number of CTAs in
-  // flight as (CTAs / slots)^0.8 up to the 6.5 TB/s of a full machine (two CTAs fit on an SM; 128 CTAs reach 3.3
-  // TB/s, 256 reach 5) and a last, partly filled wave costs half of what strict waves would; plus 10 us for the
-  // first wave and 3 for each further one.  Fewer splits win unless more are 3 % faster.  (The wave-efficiency rule
-  // used before took 23 splits at B = 8, L = 32768: 142 us against 118 with 4; and 4 at B = 64, L = 4096: 146 us
-  // against 126 with 1.)
-  const long slots = (long)decode_ctas_per_sm(*a) * num_sms(), units = (long)a->B * a->H_kv;
+  const long slots = 2L * num_sms(), units = (long)a->B * a->H_kv;
+  if (decode_uses_tc(*a)) return (int)std::max(1L, std::min(64L, (num_sms() + units - 1) / units));   // equal ranges: about as many per unit
+  // mma.sync kernel (6-bit and 4-bit caches), two CTAs per SM: the split count with the lowest modelled time (microseconds;
+  // fitted to B = 1 .. 64 at L = 4096 .. 32768 with 32 and 64 heads on 8): streaming time = bytes / bandwidth, where the
+  // bandwidth grows with the number of CTAs in flight as (CTAs / slots)^0.8 up to that of a full machine and a last,
+  // partly filled wave costs half of what strict waves would; plus 10 us for the first wave and 3 for each further one.
+  // Fewer splits win unless more are 3 % faster.
   const double stream_us = (double)units * tiles * (2.0 * 128 * 132 / 6.5e6);      // K + V tile with scales at 6.5 TB/s
   int best = 1; double best_t = 1e30;
   for (int s = 1; s <= 64 && (s == 1 || tiles / s >= 4); ++s) {
@@ -524,7 +523,7 @@ int rk_attn_decode_num_splits(const rk_decode_args* a) {
 size_t rk_attn_decode_workspace_bytes(const rk_decode_args* a) {
   const int ns = rk_attn_decode_num_splits(a);
   if (ns <= 0) return 0;
-  return (size_t)a->B * a->H * ns * (128 + 2) * sizeof(float);
+  return decode_workspace_bytes(*a, ns);
 }
 
 int rk_attn_decode(const rk_decode_args* a, void* stream) {

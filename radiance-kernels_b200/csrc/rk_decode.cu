@@ -27,6 +27,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "rk_common.cuh"
@@ -440,8 +441,73 @@ int make_tmap_u8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t S, int
 #include "rk_decode_tc.cuh"
 namespace rk {
 
-// Which kernel serves a call: the tcgen05 kernel handles d = 128 with up to 4 query heads per KV head; everything
-// else (and a forced choice through the test hook: 1 = mma.sync kernel, 2 = tcgen05 kernel) takes the mma.sync kernel.
+// log-sum-exp combine of the tcgen05 kernel's partials: one CTA per (batch, head), thread = column of d.  A unit that one
+// CTA of the main kernel held whole has its result already; a sequence without keys gets zeros here.
+constexpr int kMaxCombine = 512;                  // partials of one unit: CTAs of the main kernel, or the caller's splits
+__global__ void __launch_bounds__(128) decode_tc_combine_kernel(const DecodeTcParams p, int main_grid) {
+  __shared__ float weight[kMaxCombine];
+  __shared__ float wred[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float NEG_INF = __int_as_float(0xff800000);
+  const int bh = blockIdx.x, b = bh / p.H, hkv = (bh - b * p.H) / p.grp, hg = bh - b * p.H - hkv * p.grp;
+  grid_dependency_wait();
+  grid_dependents_launch();
+  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;     // the partials are not all there
+  const int n_unit = dtc_tiles(dtc_len(p, b));
+  if (n_unit == 0) {
+    p.o[(size_t)bh * 128 + tid] = __float2bfloat16_rn(0.0f);
+    if (p.lse && tid == 0) p.lse[bh] = NEG_INF;
+    return;
+  }
+  int n, c0 = 0, total = 0;
+  if (p.nsplit > 0) {
+    const int per = (n_unit + p.nsplit - 1) / p.nsplit;
+    n = (n_unit + per - 1) / per;
+  } else {
+    total = p.starts[0];
+    const int64_t first = p.starts[1 + b * p.H_kv + hkv];
+    c0 = (int)(((first + 1) * main_grid - 1) / total);             // the CTA whose range holds a tile
+    n = (int)(((first + n_unit) * main_grid - 1) / total) - c0 + 1;
+  }
+  if (n == 1) return;
+  auto at = [&](int i) -> size_t { return p.nsplit > 0 ? (size_t)bh * p.nsplit + i : ((size_t)(c0 + i) * 2 + (i == 0 ? 1 : 0)) * p.grp + hg; };
+  float m = NEG_INF;
+  for (int i = tid; i < n; i += 128) {
+    // with fewer tiles than CTAs some ranges are empty and left nothing
+    const bool none = p.nsplit == 0 && dtc_first(total, c0 + i, main_grid) == dtc_first(total, c0 + i + 1, main_grid);
+    const float mi = none ? NEG_INF : p.part_ml[at(i) * 2];
+    weight[i] = mi;
+    m = fmaxf(m, mi);
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+  if (lane == 0) wred[warp] = m;
+  __syncthreads();
+  m = fmaxf(fmaxf(wred[0], wred[1]), fmaxf(wred[2], wred[3]));
+  float l = 0.0f;
+  for (int i = tid; i < n; i += 128) {
+    const float mi = weight[i];
+    const float f = mi == NEG_INF ? 0.0f : exp2f(mi - m);
+    weight[i] = f;
+    if (mi != NEG_INF) l += f * p.part_ml[at(i) * 2 + 1];
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) l += __shfl_xor_sync(0xffffffffu, l, s);
+  if (lane == 0) wred[4 + warp] = l;
+  __syncthreads();
+  l = (wred[4] + wred[5]) + (wred[6] + wred[7]);
+  float acc = 0.0f;
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) {
+    const float f = weight[i];
+    if (f > 0.0f) acc += f * p.part_o[at(i) * 128 + tid];
+  }
+  p.o[(size_t)bh * 128 + tid] = __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 1.0f));
+  if (p.lse && tid == 0) p.lse[bh] = l > 0.0f ? m * 0.6931471805599453f + logf(l) : NEG_INF;
+}
+
+// Which kernel serves a call: the tcgen05 kernel handles d = 128 with up to 8 query heads per KV head; everything
+// else (and a forced choice through the test hook: 1 = mma.sync kernel) takes the mma.sync kernel.
 int g_decode_path = 0;
 bool decode_uses_tc(const rk_decode_args& a) {
   // 6-bit and 4-bit caches hold one code per byte, which the tensor core does not read: the mma.sync kernel converts them
@@ -449,50 +515,75 @@ bool decode_uses_tc(const rk_decode_args& a) {
   if (g_decode_path == 1) return false;
   return can;
 }
-int decode_ctas_per_sm(const rk_decode_args& a) { return decode_uses_tc(a) ? dtc::kCtasPerSm : 2; }
+
+// CTAs of the tcgen05 kernel without a split count from the caller: one per SM (never more than there can be tiles).
+static int decode_tc_grid(const rk_decode_args& a) {
+  const int64_t units = (int64_t)a.B * a.H_kv, tiles = units * ((a.L + dtc::kTile - 1) / dtc::kTile);
+  return (int)std::min<int64_t>(std::min<int64_t>(num_sms(), kMaxCombine), tiles);
+}
+
+size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits) {
+  if (!decode_uses_tc(a) || a.num_splits > 0) return (size_t)a.B * a.H * num_splits * (128 + 2) * sizeof(float);
+  return (size_t)decode_tc_grid(a) * 2 * (a.H / a.H_kv) * (128 + 2) * sizeof(float) + (1 + (size_t)a.B * a.H_kv) * sizeof(int32_t);
+}
+
+template <int HH>
+static int launch_decode_tc(const rk_decode_args& a, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeTcParams& t, int grid,
+                            cudaStream_t st) {
+  const int smem_bytes = dtc::Lay<HH>::total + 1024;
+  cudaError_t e = cudaFuncSetAttribute(decode_tc_kernel<HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  if (e != cudaSuccess) return (int)e;
+  // A = the cache tile in its own 8-bit format (E4M3 or E5M2: no thread decodes a cache byte, so the format is
+  // one field of the instruction descriptor), B = the MXFP8 terms of Q / P, always E4M3
+  const uint32_t idesc_qk = make_idesc(a.kv_fmt, RK_FMT_E4M3, false, false, 128, dtc::kNq);
+  const uint32_t idesc_pv = make_idesc(a.kv_fmt, RK_FMT_E4M3, true, true, 128, dtc::Lay<HH>::kNp);
+  if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
+  e = launch_pdl(decode_tc_kernel<HH>, dim3(grid), dim3(dtc::kThreads), smem_bytes, st, tk, tv, t, idesc_qk, idesc_pv);
+  if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
+  if (e != cudaSuccess) return (int)e;
+  return (int)launch_pdl(decode_tc_combine_kernel, dim3(a.B * a.H), dim3(128), 0, st, t, grid);
+}
 
 int launch_decode(const rk_decode_args& a, int nsplit, cudaStream_t st) {
   CUtensorMap tk, tv;
   int rc;
   if ((rc = make_tmap_u8_3d(&tk, a.k, (int64_t)a.B * a.H_kv, a.L, a.d)) != RK_OK) return rc;
   if ((rc = make_tmap_u8_3d(&tv, a.v, (int64_t)a.B * a.H_kv, a.L, a.d)) != RK_OK) return rc;
+  const size_t BH = (size_t)a.B * a.H;
+  const int grp = a.H / a.H_kv;
+  const float scale = a.softmax_scale > 0.0f ? a.softmax_scale : 1.0f / sqrtf((float)a.d);
+  int* status = device_status_word();
+  if (!status) return RK_ERR_NO_DEVICE;
+  if (decode_uses_tc(a)) {
+    const int grid = a.num_splits > 0 ? (int)((int64_t)a.B * a.H_kv * nsplit) : decode_tc_grid(a);
+    const size_t parts = a.num_splits > 0 ? BH * nsplit : (size_t)grid * 2 * grp;
+    DecodeTcParams t;
+    t.q = reinterpret_cast<const __nv_bfloat16*>(a.q);
+    t.k_scale = a.k_scale; t.v_scale = a.v_scale; t.kv_len = a.kv_len;
+    t.o = reinterpret_cast<__nv_bfloat16*>(a.o); t.lse = a.lse;
+    t.part_o = reinterpret_cast<float*>(a.workspace);
+    t.part_ml = t.part_o + parts * 128;
+    t.starts = reinterpret_cast<int32_t*>(t.part_ml + parts * 2);
+    t.status = status;
+    t.B = a.B; t.H = a.H; t.H_kv = a.H_kv; t.L = a.L; t.grp = grp; t.nsplit = a.num_splits > 0 ? nsplit : 0;
+    t.scale_log2 = scale * 1.4426950408889634f;
+    return grp <= 4 ? launch_decode_tc<4>(a, tk, tv, t, grid, st) : launch_decode_tc<8>(a, tk, tv, t, grid, st);
+  }
   DecodeParams p;
   p.q = reinterpret_cast<const __nv_bfloat16*>(a.q);
   p.k_scale = a.k_scale; p.v_scale = a.v_scale; p.kv_len = a.kv_len;
-  const size_t BH = (size_t)a.B * a.H;
   p.part_o = reinterpret_cast<float*>(a.workspace);
   p.part_ml = p.part_o + BH * nsplit * 128;
-  p.status = device_status_word();
-  if (!p.status) return RK_ERR_NO_DEVICE;
-  p.B = a.B; p.H = a.H; p.H_kv = a.H_kv; p.L = a.L; p.grp = a.H / a.H_kv; p.nsplit = nsplit;
-  const float scale = a.softmax_scale > 0.0f ? a.softmax_scale : 1.0f / sqrtf((float)a.d);
+  p.status = status;
+  p.B = a.B; p.H = a.H; p.H_kv = a.H_kv; p.L = a.L; p.grp = grp; p.nsplit = nsplit;
   p.scale_log2 = scale * 1.4426950408889634f;
   cudaError_t e;
-  dim3 grid(nsplit, a.H_kv, a.B);
-  if (decode_uses_tc(a)) {
-    DecodeTcParams t;
-    t.q = p.q; t.k_scale = p.k_scale; t.v_scale = p.v_scale; t.kv_len = p.kv_len;
-    t.part_o = p.part_o; t.part_ml = p.part_ml; t.status = p.status;
-    t.B = p.B; t.H = p.H; t.H_kv = p.H_kv; t.L = p.L; t.grp = p.grp; t.nsplit = p.nsplit; t.scale_log2 = p.scale_log2;
-    const bool eight = p.grp > 4;                        // head capacity 4 (two P buffers) or 8 (one)
-    const int smem_bytes = (eight ? dtc::Lay<8>::total : dtc::Lay<4>::total) + 1024;
-    auto kern = eight ? decode_tc_kernel<8> : decode_tc_kernel<4>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes)) != cudaSuccess) return (int)e;
-    // A = the cache tile in its own 8-bit format (E4M3 or E5M2: no thread decodes a cache byte, so the format is
-    // one field of the instruction descriptor), B = the MXFP8 terms of Q / P, always E4M3
-    const uint32_t idesc_qk = make_idesc(a.kv_fmt, RK_FMT_E4M3, false, false, 128, dtc::kNq);
-    const uint32_t idesc_pv = make_idesc(a.kv_fmt, RK_FMT_E4M3, true, false, 128, eight ? dtc::Lay<8>::kNp : dtc::Lay<4>::kNp);
-    if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
-    kern<<<grid, dtc::kThreads, smem_bytes, st>>>(tk, tv, t, idesc_qk, idesc_pv);
-    if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
-  } else {
-    auto kern = a.kv_fmt == RK_FMT_E5M2 ? decode_kernel<1> : a.kv_fmt == RK_FMT_E2M3 ? decode_kernel<2> :
-                a.kv_fmt == RK_FMT_E3M2 ? decode_kernel<3> : a.kv_fmt == RK_FMT_E2M1 ? decode_kernel<4> : decode_kernel<0>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmemBytes)) != cudaSuccess) return (int)e;
-    if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
-    kern<<<grid, kDecThreads, kDecSmemBytes, st>>>(tk, tv, p);
-    if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
-  }
+  auto kern = a.kv_fmt == RK_FMT_E5M2 ? decode_kernel<1> : a.kv_fmt == RK_FMT_E2M3 ? decode_kernel<2> :
+              a.kv_fmt == RK_FMT_E3M2 ? decode_kernel<3> : a.kv_fmt == RK_FMT_E2M1 ? decode_kernel<4> : decode_kernel<0>;
+  if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmemBytes)) != cudaSuccess) return (int)e;
+  if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
+  kern<<<dim3(nsplit, a.H_kv, a.B), kDecThreads, kDecSmemBytes, st>>>(tk, tv, p);
+  if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   const int warps_per_cta = 4;
   decode_combine_kernel<<<(int)((BH + warps_per_cta - 1) / warps_per_cta), warps_per_cta * 32, 0, st>>>(

@@ -1,6 +1,6 @@
 // Split-KV decode attention over an MXFP8 KV cache on the 5th-generation tensor cores.
 //
-// Same semantics and same partial format as rk_decode.cu (prefill at S_q = 1, GQA head map
+// Same semantics as rk_decode.cu (prefill at S_q = 1, GQA head map
 // kernels/flash_attention_mx_gqa/kernel.cpp:109-115; K and V decoded exactly, fp32 softmax state, no P
 // requant in the reference sense), but the raw E4M3 bytes of K and V go from shared memory straight into
 // tcgen05 block-scaled MMAs, so no thread ever converts a cache byte:
@@ -10,22 +10,33 @@
 //                                                                B = the query heads as 2 MXFP8 terms each
 //                                                                (q = hi + lo exactly: bf16 has 8 significant
 //                                                                bits, an E4M3 term 4), N = 16
-//   O^T[d][n]    += V_tile^T[128 d x 128 keys] . Pterms^T        A = V tile as TMA wrote it (MN-major), unit
-//                                                                scales; B = P, per (head, 32-column group g of
-//                                                                d, term): p * 2^(sv[key][g]) as 2 MXFP8 terms
-//                                                                with one E8M0 scale per 32 keys, N = 32
+//   O^T[d][n]    += V_tile^T[128 d x 128 keys] . Pterms          A = V tile as TMA wrote it (MN-major), unit
+//                                                                scales; B = P (MN-major: a key's codes side by
+//                                                                side), per (32-column group q of d, term, head):
+//                                                                p * 2^(sv[key][q]) as 2 MXFP8 terms with one E8M0
+//                                                                scale per 32 keys, N = 8 HH
 //
-// V's scale belongs to (key, 32-column group of d); a block-scaled MMA has one scale per (row, 32 keys), so the
-// scale is folded into P: column (h, g) of B carries p[h][key] * 2^(sv[key][g] - svmax[g]) and its block scale
-// carries svmax[g] (the largest V scale among the block's 32 keys) and the exponent of the block's largest p.
-// Row d of O^T only uses the columns of its own group g = d / 32.
+// V's scale belongs to (key, 32-column group of d); a block-scaled MMA has one scale per (row, 32 keys), so the scale is
+// folded into P: column (q, term, h) of B carries p[h][key] * 2^(sv[key][q] - svmax[q]), and its block scale carries
+// svmax[q] (the largest V scale among the block's 32 keys) and the exponent of the block's largest p.  A power of two
+// moves an E4M3 code by 8 per step, so a key's p is converted once per head and the four groups' codes are byte
+// subtractions on packed words.  Row d of O^T only uses the columns of its own group q = d / 32.
 //
-// One CTA = (batch, KV head, split): 4 worker warps (thread = key for S and P, thread = column d for O), one
-// TMA warp, one MMA warp; a stage holds 128 keys.  The running maximum is CTA-wide per head; O is rescaled in
-// TMEM only when a maximum grew by more than 2^8 since the last rescale (p stays below 2^8 in between, which the
-// block scales absorb), so the common tile touches O not at all.
+// One CTA per SM, and the CTAs share the key tiles of the whole call evenly: the tiles of all sequences in a row (each
+// sequence as long as it is) are cut into as many equal ranges as there are CTAs.  A range is a list of segments, each a
+// run of tiles of one (batch, KV head) unit; a unit that lies in one range is finished here, one that crosses ranges leaves
+// partials for the combine kernel.  (One split count for all sequences lets the longest ones set the time.)
 //
-// Included by rk_decode.cu (one translation unit: both kernels share the combine kernel and the launcher).
+// A tile is a serial chain -- S from TMEM, maximum, exponentials, P in shared memory, P V -- several times as long as its
+// bytes take to arrive, so four groups of four worker warps each take every fourth tile, with accumulators and references
+// of their own that meet at the end of a segment.  One warp loads, one issues S = K Q^T, one O += V^T P.
+//   worker warp w: group w / 4, thread = key (w % 4) * 32 + lane of the tile for S and P, and column d of O^T.
+// p of a warp's 32 keys is relative to their own maximum rounded up to an integer m_w (log2 domain), which the block scale
+// undoes exactly: nothing in a tile waits for the other warps' maxima but the scale bytes.  O and the row sums are relative
+// to a reference m_ref of the group, the first tile's largest m_w; fp32 carries them while later maxima stay below m_ref +
+// 32 (and V scales below theirs), so O is rescaled about never.
+//
+// Included by rk_decode.cu (one translation unit: both kernels share the launcher).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -37,53 +48,54 @@
 namespace rk {
 
 namespace dtc {
-constexpr int kWorkers = 4;                       // worker warps
-constexpr int kThreads = (kWorkers + 2) * 32;     // + TMA warp + MMA warp
+constexpr int kGroups = 4;                        // worker groups of four warps
+constexpr int kWorkers = 4 * kGroups;             // worker warps
+constexpr int kWarpTma = kWorkers, kWarpQk = kWorkers + 1, kWarpPv = kWorkers + 2;
+constexpr int kThreads = (kWorkers + 3) * 32;
 constexpr int kTile = 128;                        // keys per stage
 constexpr int kD = 128;
-#ifndef RK_X_DTC_STAGES
-#define RK_X_DTC_STAGES 3
-#endif
-constexpr int kStages = RK_X_DTC_STAGES;
-constexpr int kCtasPerSm = kStages <= 3 ? 2 : 1;
-constexpr int kMaxGrp = 8;                        // query heads per KV head handled by this kernel (HH = 4 or 8 rows of capacity)
+constexpr int kMaxGrp = 8;                        // query heads per KV head this kernel handles
 constexpr int kNq = 16;                           // B rows of the QK^T MMA: term * HH + h (rows past 2 HH stay zero)
 constexpr int kTileBytes = kTile * kD;            // 16384
 constexpr int kStageBytes = 2 * kTileBytes + 2 * 512;   // K, V, K scales [128][4], V scales [128][4]
-constexpr float kLazyLog2 = 8.0f;                 // rescale O when a running maximum grew by more than this
+constexpr float kBump = 32.0f;                    // rescale O when a maximum passes its reference by more than 2^this
 
-// Per head capacity HH: B rows of the PV MMA = term * 4 HH + h * 4 + g; with 8 heads one P buffer instead of two keeps
-// the CTA inside the shared memory that lets two CTAs share an SM.
+// Per head capacity HH (4 or 8): column n of the PV MMA = q * 2 HH + term * HH + h.
 template <int HH> struct Lay {
   static constexpr int kNp = 8 * HH;
-  static constexpr int kPBufs = HH == 4 ? 2 : 1;
-  static constexpr int kPBytes = kNp * 128;       // one P tile: [kNp rows][128 B], K-major SW128
+  static constexpr int kStages = HH == 8 ? 5 : 6;
+  // P tiles: rows of 128 bytes (128-byte swizzle), one row per key; a group's tile takes kNp bytes of each row
+  static constexpr int kPerAtom = 128 / kNp;
+  static constexpr int kPBytes = kGroups / kPerAtom * kTileBytes;
   // shared-memory map (offsets from a 1024-byte aligned base)
   static constexpr int stage_off = 0;
   static constexpr int p_off = kStages * kStageBytes;
-  static constexpr int q_off = p_off + kPBufs * kPBytes;       // [16 rows][128 B], K-major SW128
-  static constexpr int sfp_off = q_off + 2048;                 // 2 x 512-byte scale atoms for P
-  static constexpr int sfq_off = sfp_off + 2 * 512;            // scale atom of the query terms
-  static constexpr int one_off = sfq_off + 512;                // scale atom of ones (code 127) for V
-  static constexpr int xchg_off = one_off + 512;               // [2][4 warps][8 heads] floats (tile maxima)
-  static constexpr int bar_off = xchg_off + 2 * 32 * 4;
-  static constexpr int misc_off = bar_off + 32 * 8;            // tmem base, abort flag
+  static constexpr int q_off = p_off + kPBytes;                // [2 segments][16 rows][128 B], K-major SW128
+  static constexpr int sfp_off = q_off + 2 * 2048;             // a 512-byte scale atom of P per group
+  static constexpr int sfq_off = sfp_off + kGroups * 512;      // scale atoms of the query terms, [2 segments]
+  static constexpr int one_off = sfq_off + 2 * 512;            // scale atom of ones (code 127) for V
+  static constexpr int xchg_off = one_off + 512;               // [groups][2][4 warps][16] floats: m_w of the heads, then svmax
+  static constexpr int ref_off = xchg_off + kGroups * 2 * 4 * 16 * 4;   // [16 warps][16] floats: references, same order
+  static constexpr int seg_off = ref_off + kWorkers * 16 * 4;  // end of a segment: [groups][8] references, [groups][4 warps][8] sums
+  static constexpr int bar_off = seg_off + kGroups * (8 + 32) * 4;
+  static constexpr int bFull = 0, bEmpty = bFull + kStages, bSF = bEmpty + kStages, bSE = bSF + kGroups, bPF = bSE + kGroups,
+                       bMX = bPF + kGroups, bPV = bMX + kGroups, bQF = bPV + kGroups, bQE = bQF + 2, bSeg = bQE + 2, bDrain = bSeg + 1,
+                       nBars = bDrain + 2;
+  static constexpr int misc_off = bar_off + nBars * 8;         // tmem base, abort flag
   static constexpr int total = misc_off + 16;
   static_assert(kStageBytes % 1024 == 0 && p_off % 1024 == 0 && q_off % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+  static_assert(kPBytes >= kGroups * HH * 512, "the segment's merge uses the P tiles");
+  static_assert(total + 1024 <= 232448, "shared memory of a CTA");
 };
-enum { bFull = 0, bEmpty = bFull + kStages, bSF = bEmpty + kStages, bSE = bSF + 2, bPF = bSE + 2, bPV = bPF + 2,
-       bMX = bPV + 2, bDrain = bMX + 2, nBars = bDrain + 1 };
-static_assert(nBars <= 32, "barrier slots");
 
 // TMEM columns
-constexpr uint32_t cS = 0;          // 2 x 16
-constexpr uint32_t cO = 32;         // up to 64
-constexpr uint32_t cSfK = 96;       // 4 per stage
-constexpr uint32_t cSfQ = cSfK + 4 * kStages;
-constexpr uint32_t cSfP = cSfQ + 4; // 2 x 4
-constexpr uint32_t cSfOne = cSfP + 8;
-constexpr uint32_t kTmemCols = 128;
-static_assert(cSfOne + 4 <= kTmemCols, "TMEM map");
+constexpr uint32_t cS = 0;                        // 16 per group
+constexpr uint32_t cO = 64;                       // up to 64 per group
+constexpr uint32_t cSfK = 320;                    // 4 per stage
+constexpr uint32_t cSfQ = 344;                    // 4 per segment parity
+constexpr uint32_t cSfP = 352;                    // 4 per group
+constexpr uint32_t cSfOne = 368;
+constexpr uint32_t kTmemCols = 512;
 }  // namespace dtc
 
 struct DecodeTcParams {
@@ -91,11 +103,93 @@ struct DecodeTcParams {
   const uint8_t* k_scale;
   const uint8_t* v_scale;
   const int32_t* kv_len;
-  float* part_o;    // [B*H][nsplit][128]
-  float* part_ml;   // [B*H][nsplit][2]   (reference maximum in the log2 domain, l)
+  __nv_bfloat16* o;
+  float* lse;
+  float* part_o;    // nsplit > 0: [B*H][nsplit][128]; 0: [CTA][2][grp][128] -- a CTA leaves at most two partials, of the unit its
+                    // range begins inside of (slot 0) and of the one its range ends inside of (slot 1)
+  float* part_ml;   // the same indices, [2]: reference maximum in the log2 domain, l
+  int32_t* starts;  // nsplit == 0: [1 + B * H_kv] tiles of the whole call, then each non-empty unit's first tile
   int* status;
-  int B, H, H_kv, L, grp, nsplit;
+  int B, H, H_kv, L, grp, nsplit;                 // nsplit: the caller's split count per unit, or 0 for equal ranges
   float scale_log2;
+};
+
+RK_DEVINL int dtc_len(const DecodeTcParams& p, int b) { return p.kv_len ? min(max(p.kv_len[b], 0), p.L) : p.L; }
+RK_DEVINL int dtc_tiles(int len) { return (len + dtc::kTile - 1) / dtc::kTile; }
+// first tile of CTA c of g when t tiles are shared evenly
+RK_DEVINL int dtc_first(int t, int c, int g) { return (int)((int64_t)t * c / g); }
+
+// The segments of a CTA's range of tiles, in order.  Every warp walks its own copy.
+struct DtcSegments {
+  int b, hkv, t0, n;        // current segment: tiles t0 .. t0 + n - 1 of unit (b, hkv)
+  int len, n_unit;          // keys and tiles of the unit
+  int left;                 // tiles of the range from this segment on; 0 = done
+  int first;                // index of the segment's first tile in the whole call (nsplit == 0)
+
+  RK_DEVINL void clip() { n = min(n_unit - t0, left); }
+  RK_DEVINL void seek(const DecodeTcParams& p) { len = dtc_len(p, b); n_unit = dtc_tiles(len); }
+  RK_DEVINL void next(const DecodeTcParams& p) {
+    left -= n;
+    first += n;
+    t0 = 0;
+    if (left <= 0) return;
+    if (++hkv == p.H_kv) {
+      hkv = 0;
+      do { ++b; seek(p); } while (n_unit == 0);
+    }
+    clip();
+  }
+  // whole warp; total = tiles of the whole call
+  RK_DEVINL void start(const DecodeTcParams& p, int lane, int& total) {
+    total = 0;
+    if (p.nsplit > 0) {
+      const int split = blockIdx.x % p.nsplit, u = blockIdx.x / p.nsplit;
+      b = u / p.H_kv; hkv = u % p.H_kv;
+      seek(p);
+      const int per = (n_unit + p.nsplit - 1) / p.nsplit;
+      t0 = split * per;
+      left = max(0, min(n_unit, t0 + per) - t0);
+      first = 0;
+      clip();
+      return;
+    }
+    if (!p.kv_len) {
+      n_unit = dtc_tiles(p.L); len = p.L;
+      total = p.B * p.H_kv * n_unit;
+      first = dtc_first(total, blockIdx.x, gridDim.x);
+      left = dtc_first(total, blockIdx.x + 1, gridDim.x) - first;
+      const int u = first / n_unit;
+      b = u / p.H_kv; hkv = u % p.H_kv; t0 = first - u * n_unit;
+      clip();
+      return;
+    }
+    for (int i = lane; i < p.B; i += 32) total += dtc_tiles(dtc_len(p, i));
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
+    total *= p.H_kv;
+    first = dtc_first(total, blockIdx.x, gridDim.x);
+    left = dtc_first(total, blockIdx.x + 1, gridDim.x) - first;
+    b = hkv = t0 = n = n_unit = len = 0;
+    if (left <= 0) return;
+    int base = 0;                                              // tiles of the sequences before this block of 32
+    for (int i0 = 0;; i0 += 32) {
+      const int mine = i0 + lane < p.B ? dtc_tiles(dtc_len(p, i0 + lane)) * p.H_kv : 0;
+      int incl = mine;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) { const int o = __shfl_up_sync(0xffffffffu, incl, s); if (lane >= s) incl += o; }
+      const uint32_t past = __ballot_sync(0xffffffffu, base + incl > first);
+      if (past) {
+        const int w = __ffs(past) - 1;
+        b = i0 + w;
+        const int off = first - base - __shfl_sync(0xffffffffu, incl - mine, w);
+        seek(p);
+        hkv = off / n_unit; t0 = off - hkv * n_unit;
+        clip();
+        return;
+      }
+      base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  }
 };
 
 // two fp32 -> two E4M3 codes, RNE, saturating: bits 15:8 = code(hi), bits 7:0 = code(lo)
@@ -120,93 +214,367 @@ RK_DEVINL uint32_t redux_max_u32(uint32_t v) {
 // byte offset of (row n, byte x) in a K-major tile with 128-byte rows and the 128-byte swizzle
 RK_DEVINL int sw128(int n, int x) { return n * 128 + ((((x >> 4) ^ (n & 7))) << 4) + (x & 15); }
 
-// order-preserving map fp32 -> u32 (for integer max reductions) and back
-RK_DEVINL uint32_t f32_to_ordered(float f) {
-  const uint32_t b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-RK_DEVINL float ordered_to_f32(uint32_t u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u); }
 // 2^e as fp32 for an integer e; below the normal range the result is 0, above it the largest power of two
 RK_DEVINL float pow2i(int e) {
   const int f = e + 127;
   return __uint_as_float(f <= 0 ? 0u : ((uint32_t)(f > 254 ? 254 : f) << 23));
 }
 
+// maximum over the warp (NaNs lose)
+RK_DEVINL float redux_max_f32(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+// Four packed E4M3 codes divided by 2^(d / 8): d8 = d in every byte, d a multiple of 8 up to 120.  Codes that leave the
+// normal range become 0 (or lose their hidden bit), an absolute error of 2^-15 of the block's largest element.  SIGN: codes
+// may be negative.
+template <bool SIGN> RK_DEVINL uint32_t e4m3x4_down(uint32_t w, uint32_t d8) {
+  const uint32_t r = (w | 0x80808080u) - d8, m = r & 0x80808080u;       // bit 7 is left where the magnitude was at least d
+  const uint32_t mag = r & (m - (m >> 7));
+  return SIGN ? mag | (w & 0x80808080u) : mag;
+}
+
+// A worker warp: thread = key kt of a tile (S, P) and column d = kt (O).
 template <int HH>
-__global__ void __launch_bounds__(dtc::kThreads, dtc::kCtasPerSm)
+RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t* bars, uint32_t tmem_base, volatile int* abort_flag,
+                                DtcSegments& seg, int warp, int lane) {
+  using namespace dtc;
+  using L = Lay<HH>;
+  constexpr int kStages = L::kStages;
+  const float NEG_INF = __int_as_float(0xff800000);
+  const int g = warp >> 2, wq = warp & 3, kt = wq * 32 + lane;
+  const uint32_t lane_addr = ((uint32_t)(wq * 32)) << 16;
+  const uint32_t s_addr = tmem_base + lane_addr + cS + g * 16;
+  const uint32_t o_addr = tmem_base + lane_addr + cO + g * 64 + wq * 2 * HH;    // row d = kt: only the columns of its q = wq count
+  // this key's row of the group's P tile; 16-byte chunk i of it sits at (chunk0 + i) ^ (kt & 7)
+  uint8_t* prow = smem + L::p_off + (g / L::kPerAtom) * kTileBytes + kt * 128;
+  const int chunk0 = (g % L::kPerAtom) * (L::kNp / 16);
+  float* xchg = reinterpret_cast<float*>(smem + L::xchg_off) + g * 128;          // [2][4 warps][16]
+  float* ref = reinterpret_cast<float*>(smem + L::ref_off) + warp * 16;          // this warp's copy of the group's references
+  float* seg_m = reinterpret_cast<float*>(smem + L::seg_off);                    // [groups][8]
+  float* seg_l = seg_m + kGroups * 8;                                            // [groups][4 warps][8]
+  uint32_t seg_par = 0;
+  auto meet = [&]() -> bool {                                                    // all worker warps
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars[L::bSeg]);
+    const bool r = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSeg], seg_par, abort_flag, p.status, 506));
+    seg_par ^= 1;
+    return r;
+  };
+  bool ok = true;
+  int j0 = 0;                                                                    // tiles of this CTA before the segment
+
+  for (; seg.left > 0 && ok; j0 += seg.n, seg.next(p)) {
+    float l_part[HH];
+#pragma unroll
+    for (int h = 0; h < HH; ++h) l_part[h] = 0.0f;
+    float ref_item = 0.0f;                                                       // lane & 15: m_ref of a head, then V scale references
+    const int i_first = (g - j0) & (kGroups - 1);
+    int use = 0;                                                                 // parity of the last tile's barriers + 1
+
+    for (int i = i_first; i < seg.n; i += kGroups) {
+      const int j = j0 + i, st = j % kStages, par = (j / kGroups) & 1;
+      uint8_t* sb = smem + L::stage_off + st * kStageBytes;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSF + g], par, abort_flag, p.status, 501));
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t c[2 * HH];
+      if (HH == 8) tmem_ld16(s_addr, c); else tmem_ld8(s_addr, c);
+      uint32_t svw = *reinterpret_cast<const uint32_t*>(sb + 2 * kTileBytes + 512 + kt * 4);
+      tc_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[L::bSE + g]);
+
+      // ---- scores, the warp's maxima ----------------------------------------------------------------------------
+      float s[HH], mw[HH];
+#pragma unroll
+      for (int h = 0; h < HH; ++h) s[h] = __uint_as_float(c[h]) + __uint_as_float(c[HH + h]);
+      const bool tail = (seg.t0 + i + 1) * kTile > seg.len;
+      const bool valid = (seg.t0 + i) * kTile + kt < seg.len;
+      if (tail && !valid) {
+#pragma unroll
+        for (int h = 0; h < HH; ++h) s[h] = NEG_INF;
+        svw = 0u;
+      }
+#pragma unroll
+      for (int h = 0; h < HH; ++h) mw[h] = fmaxf(ceilf(redux_max_f32(s[h]) * p.scale_log2), -1.0e30f);   // log2 domain
+      uint32_t svmax[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) svmax[q] = redux_max_u32((svw >> (8 * q)) & 0xFFu);
+      float* xw = xchg + par * 64 + wq * 16;
+      if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < HH; h += 4) *reinterpret_cast<float4*>(xw + h) = make_float4(mw[h], mw[h + 1], mw[h + 2], mw[h + 3]);
+        *reinterpret_cast<float4*>(xw + 8) = make_float4((float)svmax[0], (float)svmax[1], (float)svmax[2], (float)svmax[3]);
+        mbar_arrive(&bars[L::bMX + g]);
+      }
+
+      // ---- p = 2^(s - m_w + 8) in two terms; a word holds the codes of four heads --------------------------------------
+      uint32_t hi[HH / 4], lo[HH / 4];
+#pragma unroll
+      for (int h = 0; h < HH; h += 4) {
+        uint32_t ch[2], cl[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float& p0 = s[h + 2 * e];
+          float& p1 = s[h + 2 * e + 1];
+          p0 = ex2_approx(fmaf(p0, p.scale_log2, 8.0f - mw[h + 2 * e]));       // at most 2^8; masked keys give 0
+          p1 = ex2_approx(fmaf(p1, p.scale_log2, 8.0f - mw[h + 2 * e + 1]));
+          ch[e] = cvt_e4m3x2(p1, p0);
+          float a1, a0;
+          e4m3x2_to_f32(ch[e], a1, a0);
+          cl[e] = cvt_e4m3x2((p1 - a1) * 16.0f, (p0 - a0) * 16.0f);
+        }
+        hi[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
+        lo[h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
+      }
+      // the P tile is free once the P V that read it (the group's previous tile in this segment) has completed
+      if (i != i_first) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
+        if (!ok) break;
+      }
+      uint32_t d8[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) d8[q] = min(svmax[q] - ((svw >> (8 * q)) & 0xFFu), 15u) * 0x08080808u;
+      if (HH == 8) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) =
+              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<false>(hi[HH / 4 - 1], d8[q]),
+                         e4m3x4_down<true>(lo[0], d8[q]), e4m3x4_down<true>(lo[HH / 4 - 1], d8[q]));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; q += 2)
+          *reinterpret_cast<uint4*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4)) =
+              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
+                         e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
+      }
+      if (tail && !valid) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
+        uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) vrow[q] = make_uint4(0u, 0u, 0u, 0u);
+      }
+
+      // ---- references, scale bytes, row sums --------------------------------------------------------------------
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504));
+      if (!ok) break;
+      const int item = lane & 15;
+      {
+        const float* xr = xchg + par * 64 + (lane >> 4) * 32 + item;
+        float top = fmaxf(xr[0], xr[16]);
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+        // every warp of the group sees the same maxima and references, so this is uniform over the group
+        if (__any_sync(0xffffffffu, top > ref_item + kBump) || i == i_first) {
+          if (i == i_first) ref_item = top;
+          const float fresh = fmaxf(ref_item, top);
+          if (i != i_first) {
+            // rescale this thread's row of O (the previous P V has landed, see above) and the row sums
+            tc_fence_after();
+            uint32_t o[2 * HH];
+            if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
+            tc_wait_ld();
+            const float down = ref_item - fresh, down_v = __shfl_sync(0xffffffffu, down, 8 + wq);
+#pragma unroll
+            for (int h = 0; h < HH; ++h) {
+              const float dh = __shfl_sync(0xffffffffu, down, h);
+              const float f = ex2_approx(fmaxf(dh + down_v, -126.0f));
+              o[h] = __float_as_uint(__uint_as_float(o[h]) * f);
+              o[HH + h] = __float_as_uint(__uint_as_float(o[HH + h]) * f);
+              l_part[h] *= ex2_approx(dh);
+            }
+            if (HH == 8) tmem_st16(o_addr, o); else tmem_st8(o_addr, o);
+            tc_wait_st();
+          }
+          ref_item = fresh;
+          __syncwarp();
+          if (lane < 16) ref[lane] = ref_item;
+          __syncwarp();
+        }
+      }
+      // steps from the reference to this warp's own maxima: at most 32 each; far below it the product vanishes anyway
+      const int step = __float2int_rn(fmaxf(xw[item] - ref_item, -200.0f));
+      const int step_h = __shfl_sync(0xffffffffu, step, lane & (HH - 1));
+#pragma unroll
+      for (int part = 0; part < L::kNp / 32; ++part) {          // block scale of column n for this warp's 32 keys (k-block = wq)
+        const int n = part * 32 + lane, q = n / (2 * HH), term = (n / HH) & 1;
+        const int code = min(max(127 + step_h + __shfl_sync(0xffffffffu, step, 8 + q), 5), 254) - 4 * term;
+        smem[L::sfp_off + g * 512 + lane * 16 + part * 4 + wq] = (uint8_t)code;
+      }
+#pragma unroll
+      for (int h = 0; h < HH; h += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(ref + h);
+        l_part[h] = fmaf(s[h], ex2_approx(mw[h] - m.x - 8.0f), l_part[h]);
+        l_part[h + 1] = fmaf(s[h + 1], ex2_approx(mw[h + 1] - m.y - 8.0f), l_part[h + 1]);
+        l_part[h + 2] = fmaf(s[h + 2], ex2_approx(mw[h + 2] - m.z - 8.0f), l_part[h + 2]);
+        l_part[h + 3] = fmaf(s[h + 3], ex2_approx(mw[h + 3] - m.w - 8.0f), l_part[h + 3]);
+      }
+      fence_proxy_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[L::bPF + g]);
+      use = par + 1;
+    }
+    if (!ok) break;
+
+    // ---- end of the segment: row d = kt of every group's O^T, merged ------------------------------------------------
+    float oh[HH];
+#pragma unroll
+    for (int h = 0; h < HH; ++h) oh[h] = 0.0f;
+    if (use > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], use - 1, abort_flag, p.status, 505));
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t o[2 * HH];
+      if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
+      tc_wait_ld();
+      tc_fence_before();
+      const int e = (int)ref[8 + wq] - 127 - 8, e0 = e / 2;                       // in two factors: e can be -135
+#pragma unroll
+      for (int h = 0; h < HH; ++h) oh[h] = (__uint_as_float(o[h]) + __uint_as_float(o[HH + h])) * pow2i(e0) * pow2i(e - e0);
+    }
+#pragma unroll
+    for (int h = 0; h < HH; ++h) {
+      float l = l_part[h];
+#pragma unroll
+      for (int x = 16; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+      if (lane == 0) seg_l[(g * 4 + wq) * 8 + h] = l;
+    }
+    if (wq == 0 && lane < 8) seg_m[g * 8 + lane] = use > 0 ? ref_item : NEG_INF;
+    if (!(ok = meet())) break;
+    float* red = reinterpret_cast<float*>(smem + L::p_off) + g * HH * 128;       // [HH][128], where the P tiles were
+#pragma unroll
+    for (int h = 0; h < HH; ++h) {
+      const float m = fmaxf(fmaxf(seg_m[h], seg_m[8 + h]), fmaxf(seg_m[16 + h], seg_m[24 + h]));
+      red[h * 128 + kt] = use > 0 ? oh[h] * ex2_approx(seg_m[g * 8 + h] - m) : 0.0f;
+    }
+    if (!(ok = meet())) break;
+    const bool whole = seg.n == seg.n_unit;
+    const size_t bh0 = (size_t)seg.b * p.H + seg.hkv * p.grp;
+    for (int idx = threadIdx.x; idx < p.grp * 128; idx += kWorkers * 32) {       // heads g, g + 4
+      const int h = idx >> 7, d = idx & 127;
+      const float m = fmaxf(fmaxf(seg_m[h], seg_m[8 + h]), fmaxf(seg_m[16 + h], seg_m[24 + h]));
+      float acc = 0.0f, l = 0.0f;
+#pragma unroll
+      for (int x = 0; x < kGroups; ++x) {
+        acc += reinterpret_cast<const float*>(smem + L::p_off)[(x * HH + h) * 128 + d];
+        const float lx = (seg_l[x * 32 + h] + seg_l[x * 32 + 8 + h]) + (seg_l[x * 32 + 16 + h] + seg_l[x * 32 + 24 + h]);
+        l += seg_m[x * 8 + h] == NEG_INF ? 0.0f : lx * ex2_approx(seg_m[x * 8 + h] - m);
+      }
+      if (whole) {
+        p.o[(bh0 + h) * 128 + d] = __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 1.0f));
+        if (p.lse && d == 0) p.lse[bh0 + h] = l > 0.0f ? m * 0.6931471805599453f + logf(l) : NEG_INF;
+      } else {
+        const size_t at = p.nsplit > 0 ? (bh0 + h) * p.nsplit + blockIdx.x % p.nsplit
+                                       : ((size_t)blockIdx.x * 2 + (seg.t0 > 0 ? 0 : 1)) * p.grp + h;
+        p.part_o[at * 128 + d] = acc;
+        if (d == 0) { p.part_ml[at * 2] = m; p.part_ml[at * 2 + 1] = l; }
+      }
+    }
+    if (p.nsplit == 0 && seg.t0 == 0 && threadIdx.x == 0) p.starts[1 + seg.b * p.H_kv + seg.hkv] = seg.first;
+    if (seg.left > seg.n && !(ok = meet())) break;               // red has been read: the P tiles may be written again
+  }
+}
+
+// One query head as two MXFP8 terms, q = hi + lo (the lib/golden block rule on q, then on the residual): a warp, four
+// elements per lane.  Heads past grp give zeros.
+template <int HH> RK_DEVINL void dtc_query_head(const DecodeTcParams& p, uint8_t* smem, int b, int hkv, int h, int buf, int lane) {
+  using L = dtc::Lay<HH>;
+  float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (h < p.grp) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p.q + ((size_t)b * p.H + hkv * p.grp + h) * dtc::kD + lane * 4);
+    x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xFFFF0000u);
+    x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xFFFF0000u);
+  }
+#pragma unroll
+  for (int term = 0; term < 2; ++term) {
+    float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));       // the 8 lanes of one 32-wide block of d
+    uint32_t code = 127u;
+    float p2 = 1.0f;
+    if (amax > 0.0f && amax < 3.0e38f) block_scale<0>(amax, code, p2);
+    const float back = e8m0_to_f32(code);
+    const uint32_t c01 = cvt_e4m3x2(x[1] * p2, x[0] * p2), c23 = cvt_e4m3x2(x[3] * p2, x[2] * p2);
+    float d0, d1, d2, d3;
+    e4m3x2_to_f32(c01, d1, d0);
+    e4m3x2_to_f32(c23, d3, d2);
+    x[0] -= d0 * back; x[1] -= d1 * back; x[2] -= d2 * back; x[3] -= d3 * back;      // residual, exact
+    const int n = term * HH + h;
+    *reinterpret_cast<uint32_t*>(smem + L::q_off + buf * 2048 + sw128(n, lane * 4)) = c01 | (c23 << 16);
+    if ((lane & 7) == 0) smem[L::sfq_off + buf * 512 + n * 16 + (lane >> 3)] = (uint8_t)code;
+  }
+}
+
+template <int HH>
+__global__ void __launch_bounds__(dtc::kThreads, 1)
 decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                  const DecodeTcParams p, const uint32_t idesc_qk, const uint32_t idesc_pv) {
   using namespace dtc;
   using L = Lay<HH>;
+  constexpr int kStages = L::kStages;
   extern __shared__ __align__(1024) uint8_t dtc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dtc_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bar_off);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc_off + 4);
-  float* xchg = reinterpret_cast<float*>(smem + L::xchg_off);
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;   // an earlier launch gave up on a wait
-  const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
-  const int bhkv = b * p.H_kv + hkv;
-  const int len = p.kv_len ? min(max(p.kv_len[b], 0), p.L) : p.L;
-  const int n_tiles_all = (len + kTile - 1) / kTile;
-  const int tiles_per_split = (n_tiles_all + p.nsplit - 1) / p.nsplit;
-  const int tile0 = split * tiles_per_split;
-  const int n_tiles = max(0, min(n_tiles_all, tile0 + tiles_per_split) - tile0);
-  const float NEG_INF = __int_as_float(0xff800000);
 
-  // ---- set-up: barriers, TMEM, constant shared-memory regions, the query terms ------------------------------
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[bSF + i], 1); mbar_init(&bars[bSE + i], kWorkers); mbar_init(&bars[bPF + i], kWorkers);
-      mbar_init(&bars[bPV + i], 1); mbar_init(&bars[bMX + i], kWorkers);
-    }
-    mbar_init(&bars[bDrain], 1);
+  // ---- set-up that touches nothing an earlier kernel of the stream may still be writing ------------------------------
+  if (warp == kWarpQk) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
+  if (warp == kWarpTma && lane == 0) {
+    prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
     *abort_flag = 0;
+    for (int i = 0; i < kStages; ++i) mbar_init(&bars[L::bFull + i], 1);
     fence_barrier_init();
   }
-  if (warp == kWorkers + 1) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
-  if (warp < kWorkers) {
-    const int t = threadIdx.x;                                    // 0..127
-    // P tiles: rows of heads that do not exist stay zero for ever; scale atoms start as ones (code 127)
-    for (int i = t; i < L::kPBufs * L::kPBytes / 16; i += 128) reinterpret_cast<uint4*>(smem + L::p_off)[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = t; i < 2048 / 16; i += 128) reinterpret_cast<uint4*>(smem + L::sfp_off)[i] = make_uint4(0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
-    // rows of the query tile that no head writes below stay zero
-    reinterpret_cast<uint4*>(smem + L::q_off)[t] = make_uint4(0u, 0u, 0u, 0u);
-    asm volatile("bar.sync 1, 128;" ::: "memory");                  // fills done before the query terms land in them
-    // query heads h = warp, warp + 4 as two MXFP8 terms each: q = hi + lo (lib/golden block rule on q, then on the residual)
-#pragma unroll
-    for (int h = warp; h < HH; h += kWorkers) {
-      float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (h < p.grp) {
-        const uint2 raw = *reinterpret_cast<const uint2*>(p.q + ((size_t)b * p.H + hkv * p.grp + h) * kD + lane * 4);
-        x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xFFFF0000u);
-        x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xFFFF0000u);
-      }
-#pragma unroll
-      for (int term = 0; term < 2; ++term) {
-        float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));   // the 8 lanes of one 32-wide block of d
-        uint32_t code = 127u;
-        float p2 = 1.0f;
-        if (amax > 0.0f && amax < 3.0e38f) block_scale<0>(amax, code, p2);
-        const float back = e8m0_to_f32(code);
-        uint32_t word = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t c = encode_rne<0>(x[e] * p2);
-          word |= c << (8 * e);
-          x[e] -= decode_elem<0>(c) * back;                          // residual, exact
-        }
-        const int n = term * HH + h;
-        *reinterpret_cast<uint32_t*>(smem + L::q_off + sw128(n, lane * 4)) = word;
-        if ((lane & 7) == 0) smem[L::sfq_off + n * 16 + (lane >> 3)] = (uint8_t)code;
-      }
+  if (warp == kWarpPv) {
+    for (int i = L::bEmpty + lane; i < L::nBars; i += 32) {
+      const bool per_warp = i >= L::bSE && i < L::bPV;                // SE, PF, MX: the four warps of a group
+      mbar_init(&bars[i], i == L::bSeg ? kWorkers : per_warp ? 4 : 1);
     }
+    fence_barrier_init();
+  }
+  if (warp < kWorkers) {
+    for (int i = threadIdx.x; i < 2 * 2048 / 16; i += kWorkers * 32) reinterpret_cast<uint4*>(smem + L::q_off)[i] = make_uint4(0u, 0u, 0u, 0u);
+    // scale atoms of P, of the query terms and of V start as ones
+    for (int i = threadIdx.x; i < (kGroups + 3) * 512 / 16; i += kWorkers * 32)
+      reinterpret_cast<uint4*>(smem + L::sfp_off)[i] = make_uint4(0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+    // items of the exchange that no head has stay zero
+    for (int i = threadIdx.x; i < kGroups * 2 * 4 * 16 / 4; i += kWorkers * 32) reinterpret_cast<uint4*>(smem + L::xchg_off)[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  grid_dependency_wait();
+  grid_dependents_launch();
+  const int stopped = threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0;
+  DtcSegments seg;
+  int total;
+  seg.start(p, lane, total);
+  if (__syncthreads_or(stopped)) {                                    // an earlier launch gave up on a wait
+    if (warp == kWarpQk) tmem_dealloc(*tmem_slot, kTmemCols);
+    return;
+  }
+  if (p.nsplit == 0 && blockIdx.x == 0 && threadIdx.x == 0) p.starts[0] = total;
+
+  auto issue_tile = [&](int j, int tile) {                            // loads of the j-th tile of this CTA
+    const int st = j % kStages;
+    uint8_t* sb = smem + L::stage_off + st * kStageBytes;
+    const int key0 = tile * kTile, bhkv = seg.b * p.H_kv + seg.hkv;
+    // scale rows past L are not read: the copy is clipped to the cache extent (L % 4 == 0 keeps it a 16-byte multiple)
+    const uint32_t sbytes = (uint32_t)min(kTile, p.L - key0) * 4u;
+    mbar_arrive_expect_tx(&bars[L::bFull + st], 2u * kTileBytes + 2u * sbytes);
+    tma_load_3d(sb, &tmap_k, &bars[L::bFull + st], 0, key0, bhkv);
+    bulk_load_1d(sb + 2 * kTileBytes, p.k_scale + ((size_t)bhkv * p.L + key0) * 4, sbytes, &bars[L::bFull + st]);
+    tma_load_3d(sb + kTileBytes, &tmap_v, &bars[L::bFull + st], 0, key0, bhkv);
+    bulk_load_1d(sb + 2 * kTileBytes + 512, p.v_scale + ((size_t)bhkv * p.L + key0) * 4, sbytes, &bars[L::bFull + st]);
+  };
+  const int n_early = min(kStages, seg.left > 0 ? seg.n : 0);         // tiles whose loads run under the rest of the set-up
+  if (warp == kWarpTma) {
+    if (lane == 0)
+      for (int j = 0; j < n_early; ++j) issue_tile(j, seg.t0 + j);
+  } else if (warp < kWorkers) {
+    if (warp < HH && seg.left > 0) dtc_query_head<HH>(p, smem, seg.b, seg.hkv, warp, 0, lane);
     fence_proxy_async_smem();
   }
   tc_fence_before();
@@ -215,286 +583,105 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
 
-  if (warp == kWorkers) {
-    // ================= TMA producer =================
-    if (lane == 0) {
-      prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % kStages;
-        if (j >= kStages && !mbar_wait<20000>(&bars[bEmpty + st], ((j / kStages) - 1) & 1, abort_flag, p.status, 511)) break;
-        uint8_t* sb = smem + L::stage_off + st * kStageBytes;
-        const int key0 = (tile0 + j) * kTile;
-        // scale rows past L are not read: the copy is clipped to the cache extent (L % 4 == 0 keeps it a 16-byte multiple)
-        const uint32_t sbytes = (uint32_t)min(kTile, p.L - key0) * 4u;
-        mbar_arrive_expect_tx(&bars[bFull + st], 2u * kTileBytes + 2u * sbytes);
-        tma_load_3d(sb, &tmap_k, &bars[bFull + st], 0, key0, bhkv);
-        tma_load_3d(sb + kTileBytes, &tmap_v, &bars[bFull + st], 0, key0, bhkv);
-        bulk_load_1d(sb + 2 * kTileBytes, p.k_scale + ((size_t)bhkv * p.L + key0) * 4, sbytes, &bars[bFull + st]);
-        bulk_load_1d(sb + 2 * kTileBytes + 512, p.v_scale + ((size_t)bhkv * p.L + key0) * 4, sbytes, &bars[bFull + st]);
+  if (warp == kWarpTma) {
+    // ================= loads; query terms of every segment after the first =================
+    int j = 0;
+    for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
+      if (s > 0) {
+        if (s >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQE + (s & 1)], ((s >> 1) - 1) & 1, abort_flag, p.status, 512));
+        if (!ok) break;
+#pragma unroll 1
+        for (int h = 0; h < p.grp; ++h) dtc_query_head<HH>(p, smem, seg.b, seg.hkv, h, s & 1, lane);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[L::bQF + (s & 1)]);
+      }
+      for (int i = 0; i < seg.n && ok; ++i, ++j) {
+        if (j < n_early) continue;
+        if (j >= kStages) ok = __all_sync(0xffffffffu, mbar_wait<20000>(&bars[L::bEmpty + j % kStages], (j / kStages - 1) & 1, abort_flag, p.status, 511));
+        if (ok && lane == 0) issue_tile(j, seg.t0 + i);
       }
     }
-  } else if (warp == kWorkers + 1) {
-    // ================= MMA issuer (all lanes re-tile the key scales, lane 0 issues) =================
-    const uint32_t q_addr = smem_u32(smem + L::q_off), p_addr = smem_u32(smem + L::p_off);
-    auto issue_pv = [&](int i) -> bool {                            // lane 0 only
-      const int buf = i & 1, sti = i % kStages;
-      if (!mbar_wait(&bars[bPF + buf], (i >> 1) & 1, abort_flag, p.status, 523)) return false;
-      tc_fence_after();
-      tc_cp_32x128b_warpx4(tmem_base + cSfP + buf * 4, make_smem_desc(smem_u32(smem + L::sfp_off + buf * 512), 0, 128, kLayoutNone));
-      const uint32_t v_addr = smem_u32(smem + L::stage_off + sti * kStageBytes + kTileBytes);
-      const int pbuf = L::kPBufs == 2 ? buf : 0;
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        // A = V tile [keys][d]: d is the contiguous (M) dimension, 32 keys per instruction
-        const uint64_t adesc = make_smem_desc(v_addr + kk * 4096, kTileBytes, 1024, kLayoutSw128);
-        const uint64_t bdesc = make_smem_desc(p_addr + pbuf * L::kPBytes + kk * 32, 16, 1024, kLayoutSw128);
-        mma_mxf8f6f4_ss(tmem_base + cO, adesc, bdesc, idesc_with_sf(idesc_pv, kk, kk), tmem_base + cSfOne,
-                        tmem_base + cSfP + buf * 4, (i > 0 || kk > 0) ? 1u : 0u);
-      }
-      tc_commit(&bars[bPV + buf]);
-      tc_commit(&bars[bEmpty + sti]);
-      return true;
-    };
-    if (lane == 0 && n_tiles > 0) {
-      tc_cp_32x128b_warpx4(tmem_base + cSfQ, make_smem_desc(smem_u32(smem + L::sfq_off), 0, 128, kLayoutNone));
-      tc_cp_32x128b_warpx4(tmem_base + cSfOne, make_smem_desc(smem_u32(smem + L::one_off), 0, 128, kLayoutNone));
-    }
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int st = j % kStages;
-      uint8_t* sb = smem + L::stage_off + st * kStageBytes;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[bFull + st], (j / kStages) & 1, abort_flag, p.status, 521));
+  } else if (warp == kWarpQk) {
+    // ================= S^T = K Q^T (all lanes re-tile the key scales, lane 0 issues) =================
+    const uint64_t dk = make_smem_desc(smem_u32(smem + L::stage_off), 16, 1024, kLayoutSw128);
+    const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
+    const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::stage_off + 2 * kTileBytes), 0, 128, kLayoutNone);
+    if (lane == 0) tc_cp_32x128b_warpx4(tmem_base + cSfOne, make_smem_desc(smem_u32(smem + L::one_off), 0, 128, kLayoutNone));
+    int j = 0;
+    for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
+      if (s > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQF + (s & 1)], (s & 1) ? (s >> 1) & 1 : ((s >> 1) - 1) & 1, abort_flag, p.status, 525));
       if (!ok) break;
-      // key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32
-      uint32_t* ks = reinterpret_cast<uint32_t*>(sb + 2 * kTileBytes);
-      uint32_t w[4];
+      if (lane == 0)
+        tc_cp_32x128b_warpx4(tmem_base + cSfQ + (s & 1) * 4, make_smem_desc(smem_u32(smem + L::sfq_off + (s & 1) * 512), 0, 128, kLayoutNone));
+      for (int i = 0; i < seg.n && ok; ++i, ++j) {
+        const int st = j % kStages, g = j & (kGroups - 1);
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 521));
+        if (!ok) break;
+        // key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32
+        uint32_t* ks = reinterpret_cast<uint32_t*>(smem + L::stage_off + st * kStageBytes + 2 * kTileBytes);
+        uint32_t w[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = ks[q * 32 + lane];
-      __syncwarp();
-      *reinterpret_cast<uint4*>(ks + lane * 4) = make_uint4(w[0], w[1], w[2], w[3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      int good = 1;
-      if (lane == 0) {
-        tc_cp_32x128b_warpx4(tmem_base + cSfK + st * 4, make_smem_desc(smem_u32(ks), 0, 128, kLayoutNone));
-        if (j >= 2 && !mbar_wait(&bars[bSE + (j & 1)], ((j - 2) >> 1) & 1, abort_flag, p.status, 522)) good = 0;
-        if (good) {
+        for (int q = 0; q < 4; ++q) w[q] = ks[q * 32 + lane];
+        __syncwarp();
+        *reinterpret_cast<uint4*>(ks + lane * 4) = make_uint4(w[0], w[1], w[2], w[3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (j >= kGroups) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSE + g], (j / kGroups - 1) & 1, abort_flag, p.status, 522));
+        if (ok && lane == 0) {
           tc_fence_after();
-          const uint32_t k_addr = smem_u32(sb);
+          const uint32_t so = (uint32_t)(st * (kStageBytes >> 4));
+          tc_cp_32x128b_warpx4(tmem_base + cSfK + st * 4, dsfk + so);
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const uint64_t adesc = make_smem_desc(k_addr + kk * 32, 16, 1024, kLayoutSw128);
-            const uint64_t bdesc = make_smem_desc(q_addr + kk * 32, 16, 1024, kLayoutSw128);
-            mma_mxf8f6f4_ss(tmem_base + cS + (j & 1) * 16, adesc, bdesc, idesc_with_sf(idesc_qk, kk, kk),
-                            tmem_base + cSfK + st * 4, tmem_base + cSfQ, kk > 0 ? 1u : 0u);
-          }
-          tc_commit(&bars[bSF + (j & 1)]);
-          if (j >= 1 && !issue_pv(j - 1)) good = 0;
+          for (int kk = 0; kk < 4; ++kk)
+            mma_mxf8f6f4_ss(tmem_base + cS + g * 16, dk + so + kk * 2, dq + (uint32_t)((s & 1) * (2048 >> 4)) + kk * 2,
+                            idesc_with_sf(idesc_qk, kk, kk), tmem_base + cSfK + st * 4, tmem_base + cSfQ + (s & 1) * 4, kk > 0 ? 1u : 0u);
+          tc_commit(&bars[L::bSF + g]);
+          if (i == seg.n - 1) tc_commit(&bars[L::bQE + (s & 1)]);
         }
       }
-      ok = __shfl_sync(0xffffffffu, good, 0) != 0;
     }
-    if (lane == 0 && n_tiles > 0) {
-      if (ok) ok = issue_pv(n_tiles - 1);
-      tc_commit(&bars[bDrain]);
-      mbar_wait(&bars[bDrain], 0, abort_flag, p.status, 524);
+    if (lane == 0) {
+      tc_commit(&bars[L::bDrain]);
+      mbar_wait(&bars[L::bDrain], 0, abort_flag, p.status, 524);
     }
     __syncwarp();
-  }
-  else {
-    // ================= workers: thread = key kt of the tile (S, P), thread = column d = kt (O) =================
-    const int kt = warp * 32 + lane;
-    const uint32_t lane_addr = ((uint32_t)(warp * 32)) << 16;
-    float m_ref[HH], m_run[HH], l_part[HH];
-#pragma unroll
-    for (int h = 0; h < HH; ++h) { m_ref[h] = NEG_INF; m_run[h] = NEG_INF; l_part[h] = 0.0f; }
-
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int buf = j & 1, st = j % kStages;
-      uint8_t* sb = smem + L::stage_off + st * kStageBytes;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[bSF + buf], (j >> 1) & 1, abort_flag, p.status, 501));
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t c[16];
-      tmem_ld16(tmem_base + lane_addr + cS + buf * 16, c);
-      tc_wait_ld();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[bSE + buf]);
-
-      const int key = (tile0 + j) * kTile + kt;
-      const bool valid = key < len;
-      const bool tail = (tile0 + j + 1) * kTile > len;
-      float s[HH];
-      float* xw = xchg + (buf * kWorkers + warp) * HH;
-#pragma unroll
-      for (int h = 0; h < HH; ++h) {
-        s[h] = valid ? (__uint_as_float(c[h]) + __uint_as_float(c[HH + h])) * p.scale_log2 : NEG_INF;   // log2 domain
-        const uint32_t wmax = redux_max_u32(f32_to_ordered(s[h]));
-        if (lane == 0) xw[h] = ordered_to_f32(wmax);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[bMX + buf]);
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[bMX + buf], (j >> 1) & 1, abort_flag, p.status, 504));
-      if (!ok) break;
-      float m_new[HH];
-      // every thread of the CTA holds the same m_run / m_ref / m_new, so the decision below is CTA-uniform
-      bool bump = (j == 0);
-#pragma unroll
-      for (int h = 0; h < HH; ++h) {
-        const float* xr = xchg + buf * kWorkers * HH + h;
-        m_new[h] = fmaxf(m_run[h], fmaxf(fmaxf(xr[0], xr[HH]), fmaxf(xr[2 * HH], xr[3 * HH])));
-        bump = bump || (m_new[h] > m_ref[h] + kLazyLog2);
-        m_run[h] = m_new[h];
-      }
-      if (bump) {
-        if (j > 0) {
-          // rescale O (this thread's row d = kt, all columns) once the previous PV has landed
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars[bPV + ((j - 1) & 1)], ((j - 1) >> 1) & 1, abort_flag, p.status, 502));
+  } else if (warp == kWarpPv) {
+    // ================= O^T += V^T P (one lane) =================
+    if (lane == 0) {
+      // A = V tile [keys][d] and B = P tile [keys][n]: both have the keys as rows (32 rows of 128 bytes per instruction)
+      const uint64_t dv = make_smem_desc(smem_u32(smem + L::stage_off + kTileBytes), kTileBytes, 1024, kLayoutSw128);
+      const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), kTileBytes, 1024, kLayoutSw128);
+      const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
+      int j = 0;
+      for (; seg.left > 0 && ok; seg.next(p)) {
+        for (int i = 0; i < seg.n && ok; ++i, ++j) {
+          const int st = j % kStages, g = j & (kGroups - 1);
+          ok = mbar_wait(&bars[L::bPF + g], (j / kGroups) & 1, abort_flag, p.status, 523);
           if (!ok) break;
           tc_fence_after();
-          float corr[HH];
+          tc_cp_32x128b_warpx4(tmem_base + cSfP + g * 4, dsfp + (uint32_t)(g * (512 >> 4)));
+          const uint64_t dvt = dv + (uint32_t)(st * (kStageBytes >> 4));
+          const uint64_t dpt = dp + (uint32_t)((g / L::kPerAtom) * (kTileBytes >> 4) + (g % L::kPerAtom) * (L::kNp >> 4));
 #pragma unroll
-          for (int h = 0; h < HH; ++h) { corr[h] = ex2_approx(m_ref[h] - m_new[h]); l_part[h] *= corr[h]; }
-#pragma unroll
-          for (int part = 0; part < L::kNp / 32; ++part) {
-            uint32_t o[32];
-            tmem_ld32(tmem_base + lane_addr + cO + part * 32, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int n = 0; n < 32; ++n) o[n] = __float_as_uint(__uint_as_float(o[n]) * corr[((part * 32 + n) % (4 * HH)) >> 2]);
-            tmem_st32(tmem_base + lane_addr + cO + part * 32, o);
-          }
-          tc_wait_st();
-        }
-#pragma unroll
-        for (int h = 0; h < HH; ++h) m_ref[h] = m_new[h];
-      }
-
-      // ---- p, row sums, block exponents -------------------------------------------------------------------
-      float ph[HH];
-      uint32_t eh[HH];     // biased exponent of the largest p of this warp's 32 keys, per head
-      uint32_t emin = 255u, emax = 0u;
-#pragma unroll
-      for (int h = 0; h < HH; ++h) {
-        const float pr = ex2_approx(s[h] - m_ref[h]);            // <= 2^8; masked keys give 0
-        l_part[h] += pr;
-        eh[h] = redux_max_u32(__float_as_uint(pr)) >> 23;
-        ph[h] = pr * pow2i(134 - (int)eh[h]);
-        emin = min(emin, eh[h]); emax = max(emax, eh[h]);
-      }
-      const uint32_t svw = valid ? *reinterpret_cast<const uint32_t*>(sb + 2 * kTileBytes + 512 + kt * 4) : 0u;
-      uint32_t svmax[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) svmax[g] = redux_max_u32((svw >> (8 * g)) & 0xFFu);
-      // element (h, g) = p * 2^(sv[g] - svmax[g]) * 2^(7 - (eh - 127)) <= 2^8 under the block scale code
-      // svmax[g] + eh[h] - 134 (kept >= 4 so that the low term's code, 4 less, exists)
-      float fg[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) fg[g] = pow2i((int)((svw >> (8 * g)) & 0xFFu) - (int)svmax[g]);
-      const uint32_t smin = min(min(svmax[0], svmax[1]), min(svmax[2], svmax[3]));
-      const uint32_t smax = max(max(svmax[0], svmax[1]), max(svmax[2], svmax[3]));
-      const bool plain = (smin + emin >= 138u) && (smax + emax <= 388u);      // every code in [4, 254]
-
-      // the P buffer is free once the PV that read it has completed: two tiles ago with two buffers, the last one with one
-      if (j >= L::kPBufs) {
-        const int i = j - L::kPBufs;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[bPV + (i & 1)], (i >> 1) & 1, abort_flag, p.status, 503));
-        if (!ok) break;
-      }
-      uint8_t* pt = smem + L::p_off + (L::kPBufs == 2 ? buf : 0) * L::kPBytes;
-#pragma unroll
-      for (int h = 0; h < HH; ++h) {
-#pragma unroll
-        for (int g = 0; g < 4; g += 2) {
-          float v0 = ph[h] * fg[g], v1 = ph[h] * fg[g + 1];
-          if (!plain) {     // block scale code clamped: move the difference into the elements
-            const int r0 = (int)svmax[g] + (int)eh[h] - 134, r1 = (int)svmax[g + 1] + (int)eh[h] - 134;
-            v0 *= pow2i(r0 - min(max(r0, 4), 254));
-            v1 *= pow2i(r1 - min(max(r1, 4), 254));
-          }
-          const uint32_t hi = cvt_e4m3x2(v1, v0);
-          float a1, a0;
-          e4m3x2_to_f32(hi, a1, a0);
-          const uint32_t lo = cvt_e4m3x2((v1 - a1) * 16.0f, (v0 - a0) * 16.0f);
-          const int n = h * 4 + g;
-          pt[sw128(n, kt)] = (uint8_t)hi;
-          pt[sw128(n + 1, kt)] = (uint8_t)(hi >> 8);
-          pt[sw128(4 * HH + n, kt)] = (uint8_t)lo;
-          pt[sw128(4 * HH + n + 1, kt)] = (uint8_t)(lo >> 8);
+          for (int kk = 0; kk < 4; ++kk)
+            mma_mxf8f6f4_ss(tmem_base + cO + g * 64, dvt + kk * (4096 >> 4), dpt + kk * (4096 >> 4), idesc_with_sf(idesc_pv, kk, kk),
+                            tmem_base + cSfOne, tmem_base + cSfP + g * 4, (i >= kGroups || kk > 0) ? 1u : 0u);
+          tc_commit(&bars[L::bPV + g]);
+          tc_commit(&bars[L::bEmpty + st]);
         }
       }
-#pragma unroll
-      for (int part = 0; part < L::kNp / 32; ++part) {   // block scale of column n for this warp's 32 keys (k-block = warp)
-        const int n = part * 32 + lane;
-        const int term = n / (4 * HH), hh = (n >> 2) % HH, gg = n & 3;
-        const uint32_t sv_s = gg == 0 ? svmax[0] : gg == 1 ? svmax[1] : gg == 2 ? svmax[2] : svmax[3];
-        uint32_t eh_s = eh[0];
-#pragma unroll
-        for (int h = 1; h < HH; ++h) eh_s = (hh == h) ? eh[h] : eh_s;
-        const int code = min(max((int)sv_s + (int)eh_s - 134, 4), 254) - 4 * term;
-        smem[L::sfp_off + buf * 512 + (n & 31) * 16 + (n >> 5) * 4 + warp] = (uint8_t)code;
-      }
-      if (tail && !valid) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
-        uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vrow[i] = make_uint4(0u, 0u, 0u, 0u);
-      }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[bPF + buf]);
+      tc_commit(&bars[L::bDrain + 1]);
+      mbar_wait(&bars[L::bDrain + 1], 0, abort_flag, p.status, 526);
     }
-
-    // ---- epilogue: O^T row d = kt, the columns of group g = warp -------------------------------------------
-    float oh[HH];
-#pragma unroll
-    for (int h = 0; h < HH; ++h) oh[h] = 0.0f;
-    if (ok && n_tiles > 0) {
-      const int last = n_tiles - 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[bPV + (last & 1)], (last >> 1) & 1, abort_flag, p.status, 505));
-      if (ok) {
-        tc_fence_after();
-#pragma unroll
-        for (int part = 0; part < L::kNp / 32; ++part) {
-          uint32_t o[32];
-          tmem_ld32(tmem_base + lane_addr + cO + part * 32, o);
-          tc_wait_ld();
-#pragma unroll
-          for (int n = 0; n < 32; ++n) {
-            const int col = part * 32 + n;                       // = term * 4 HH + h * 4 + g: both terms add up
-            if ((col & 3) == warp) oh[(col % (4 * HH)) >> 2] += __uint_as_float(o[n]);
-          }
-        }
-      }
-    }
-    float* lsum = reinterpret_cast<float*>(smem + L::p_off);        // [HH heads][128 threads]: the P tiles are free now
-#pragma unroll
-    for (int h = 0; h < HH; ++h) lsum[h * 128 + kt] = l_part[h];
-    asm volatile("bar.sync 1, 128;" ::: "memory");                  // workers only; every worker reaches this point
-    if (ok) {
-#pragma unroll
-      for (int h = 0; h < HH; ++h) {
-        if (h < p.grp) {
-          const size_t bh = (size_t)b * p.H + hkv * p.grp + h;
-          p.part_o[(bh * p.nsplit + split) * 128 + kt] = oh[h];
-        }
-      }
-      if (kt < p.grp) {
-        float l = 0.0f;
-        for (int i = 0; i < 128; ++i) l += lsum[kt * 128 + i];
-        float mr = m_ref[0];
-#pragma unroll
-        for (int h = 1; h < HH; ++h) mr = (kt == h) ? m_ref[h] : mr;
-        const size_t bh = (size_t)b * p.H + hkv * p.grp + kt;
-        p.part_ml[(bh * p.nsplit + split) * 2] = mr;
-        p.part_ml[(bh * p.nsplit + split) * 2 + 1] = l;
-      }
-    }
+    __syncwarp();
+  } else {
+    decode_tc_worker<HH>(p, smem, bars, tmem_base, abort_flag, seg, warp, lane);
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == dtc::kWorkers + 1) { tc_fence_after(); tmem_dealloc(tmem_base, dtc::kTmemCols); }
+  if (warp == kWarpQk) { tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols); }
 }
 
 }  // namespace rk

@@ -52,6 +52,19 @@ int launch_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile, int iter
 int launch_wait_runs_out(int limit_us, bool noalloc, cudaStream_t st);   // test hook: a bounded wait that must give up
 extern int g_decode_path;                                   // test hook: 0 = by shape, 1 = mma.sync kernel only
 bool decode_uses_tc(const rk_decode_args& a);                // true when the tcgen05 decode kernel serves this call
-int decode_ctas_per_sm(const rk_decode_args& a);             // resident CTAs per SM of the kernel that serves it
+size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits);   // of the kernel that serves the call
+
+// Launch with the programmatic attribute: the kernel's set-up runs while the kernel before it in the stream finishes.  Only
+// for kernels in which every CTA calls grid_dependency_wait() before it touches memory another kernel may use.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 }  // namespace rk
