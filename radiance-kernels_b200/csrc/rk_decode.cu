@@ -441,69 +441,99 @@ int make_tmap_u8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t S, int
 #include "rk_decode_tc.cuh"
 namespace rk {
 
-// log-sum-exp combine of the tcgen05 kernel's partials: one CTA per (batch, head), thread = column of d.  A unit that one
-// CTA of the main kernel held whole has its result already; a sequence without keys gets zeros here.
+// log-sum-exp combine of the tcgen05 kernel's partials: one CTA per (batch, head); a warp takes every eighth partial, four
+// columns per lane.  A unit that one CTA of the main kernel held whole has its result already; a sequence without keys gets
+// zeros here.
+// The kernel is a chain of memory latencies on top of the main kernel's end (7.4 us of a 23 us step when it read the status,
+// the length, the unit's first tile, the maxima and the rows one after the other, 40 us for 148 partials).  Which partials it
+// needs depends on kv_len alone, which nothing still running writes (the main kernel lets this one start only after its own
+// wait), so that is worked out before the wait; after it the maxima and the rows of a warp's first partials load together.
 constexpr int kMaxCombine = 512;                  // partials of one unit: CTAs of the main kernel, or the caller's splits
-__global__ void __launch_bounds__(128) decode_tc_combine_kernel(const DecodeTcParams p, int main_grid) {
-  __shared__ float weight[kMaxCombine];
-  __shared__ float wred[8];
+constexpr int kCombineWarps = 8;
+__global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(const DecodeTcParams p, int main_grid) {
+  constexpr int kBatch = 4;                                        // partials of a warp in flight
+  __shared__ float4 acc_sm[kCombineWarps][32];
+  __shared__ float2 ml_sm[kCombineWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float NEG_INF = __int_as_float(0xff800000);
   const int bh = blockIdx.x, b = bh / p.H, hkv = (bh - b * p.H) / p.grp, hg = bh - b * p.H - hkv * p.grp;
-  grid_dependency_wait();
-  grid_dependents_launch();
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;     // the partials are not all there
   const int n_unit = dtc_tiles(dtc_len(p, b));
-  if (n_unit == 0) {
-    p.o[(size_t)bh * 128 + tid] = __float2bfloat16_rn(0.0f);
-    if (p.lse && tid == 0) p.lse[bh] = NEG_INF;
-    return;
-  }
-  int n, c0 = 0, total = 0;
+  int n = 0, c0 = 0, total = 0;
   if (p.nsplit > 0) {
-    const int per = (n_unit + p.nsplit - 1) / p.nsplit;
+    const int per = max(1, (n_unit + p.nsplit - 1) / p.nsplit);
     n = (n_unit + per - 1) / per;
-  } else {
-    total = p.starts[0];
-    const int64_t first = p.starts[1 + b * p.H_kv + hkv];
+  } else if (n_unit > 0) {
+    int before = 0;                                                // tiles of the sequences before b; of all
+    for (int i = lane; i < p.B; i += 32) {
+      const int ti = dtc_tiles(dtc_len(p, i));
+      total += ti;
+      before += i < b ? ti : 0;
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) { total += __shfl_xor_sync(0xffffffffu, total, s); before += __shfl_xor_sync(0xffffffffu, before, s); }
+    total *= p.H_kv;
+    const int64_t first = (int64_t)before * p.H_kv + (int64_t)hkv * n_unit;
     c0 = (int)(((first + 1) * main_grid - 1) / total);             // the CTA whose range holds a tile
     n = (int)(((first + n_unit) * main_grid - 1) / total) - c0 + 1;
   }
-  if (n == 1) return;
   auto at = [&](int i) -> size_t { return p.nsplit > 0 ? (size_t)bh * p.nsplit + i : ((size_t)(c0 + i) * 2 + (i == 0 ? 1 : 0)) * p.grp + hg; };
-  float m = NEG_INF;
-  for (int i = tid; i < n; i += 128) {
-    // with fewer tiles than CTAs some ranges are empty and left nothing
-    const bool none = p.nsplit == 0 && dtc_first(total, c0 + i, main_grid) == dtc_first(total, c0 + i + 1, main_grid);
-    const float mi = none ? NEG_INF : p.part_ml[at(i) * 2];
-    weight[i] = mi;
-    m = fmaxf(m, mi);
-  }
+  // with fewer tiles than CTAs some ranges are empty and left nothing
+  auto none = [&](int i) { return p.nsplit == 0 && total < main_grid && dtc_first(total, c0 + i, main_grid) == dtc_first(total, c0 + i + 1, main_grid); };
+  grid_dependency_wait();
+  grid_dependents_launch();
+  if (n == 1) return;
+  float m = NEG_INF, l = 0.0f;                                     // of this warp's partials
+  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int i0 = warp; i0 < n; i0 += kBatch * kCombineWarps) {
+    float2 ml[kBatch];
+    float4 row[kBatch];
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-  if (lane == 0) wred[warp] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(wred[0], wred[1]), fmaxf(wred[2], wred[3]));
-  float l = 0.0f;
-  for (int i = tid; i < n; i += 128) {
-    const float mi = weight[i];
-    const float f = mi == NEG_INF ? 0.0f : exp2f(mi - m);
-    weight[i] = f;
-    if (mi != NEG_INF) l += f * p.part_ml[at(i) * 2 + 1];
-  }
+    for (int k = 0; k < kBatch; ++k) {
+      const int i = i0 + k * kCombineWarps;
+      ml[k] = make_float2(NEG_INF, 0.0f);
+      row[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (i < n && !none(i)) {
+        ml[k] = __ldcg(reinterpret_cast<const float2*>(p.part_ml) + at(i));
+        row[k] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at(i) * 128) + lane);
+      }
+    }
+    float top = m;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) l += __shfl_xor_sync(0xffffffffu, l, s);
-  if (lane == 0) wred[4 + warp] = l;
-  __syncthreads();
-  l = (wred[4] + wred[5]) + (wred[6] + wred[7]);
-  float acc = 0.0f;
-#pragma unroll 4
-  for (int i = 0; i < n; ++i) {
-    const float f = weight[i];
-    if (f > 0.0f) acc += f * p.part_o[at(i) * 128 + tid];
+    for (int k = 0; k < kBatch; ++k) top = fmaxf(top, ml[k].x);
+    if (top == NEG_INF) continue;
+    const float keep = exp2f(m - top);                             // m = -inf: 0
+    l *= keep; acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+    m = top;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const float f = exp2f(ml[k].x - top);
+      l += f * ml[k].y;
+      acc.x += f * row[k].x; acc.y += f * row[k].y; acc.z += f * row[k].z; acc.w += f * row[k].w;
+    }
   }
-  p.o[(size_t)bh * 128 + tid] = __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 1.0f));
-  if (p.lse && tid == 0) p.lse[bh] = l > 0.0f ? m * 0.6931471805599453f + logf(l) : NEG_INF;
+  acc_sm[warp][lane] = acc;
+  if (lane == 0) ml_sm[warp] = make_float2(m, l);
+  const int stopped = tid == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0;     // the partials are not all there
+  if (__syncthreads_or(stopped) || warp != 0) return;
+  float top = NEG_INF;
+#pragma unroll
+  for (int w = 0; w < kCombineWarps; ++w) top = fmaxf(top, ml_sm[w].x);
+  l = 0.0f;
+  acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int w = 0; w < kCombineWarps; ++w) {
+    const float f = ml_sm[w].x == NEG_INF ? 0.0f : exp2f(ml_sm[w].x - top);
+    const float4 a = acc_sm[w][lane];
+    l += f * ml_sm[w].y;
+    acc.x += f * a.x; acc.y += f * a.y; acc.z += f * a.z; acc.w += f * a.w;
+  }
+  const float inv = l > 0.0f ? 1.0f / l : 1.0f;
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+  uint2 out;
+  out.x = *reinterpret_cast<const uint32_t*>(&lo);
+  out.y = *reinterpret_cast<const uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(p.o + (size_t)bh * 128 + lane * 4) = out;
+  if (p.lse && lane == 0) p.lse[bh] = l > 0.0f ? top * 0.6931471805599453f + logf(l) : NEG_INF;
 }
 
 // Which kernel serves a call: the tcgen05 kernel handles d = 128 with up to 8 query heads per KV head; everything
@@ -524,7 +554,7 @@ static int decode_tc_grid(const rk_decode_args& a) {
 
 size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits) {
   if (!decode_uses_tc(a) || a.num_splits > 0) return (size_t)a.B * a.H * num_splits * (128 + 2) * sizeof(float);
-  return (size_t)decode_tc_grid(a) * 2 * (a.H / a.H_kv) * (128 + 2) * sizeof(float) + (1 + (size_t)a.B * a.H_kv) * sizeof(int32_t);
+  return (size_t)decode_tc_grid(a) * 2 * (a.H / a.H_kv) * (128 + 2) * sizeof(float);
 }
 
 template <int HH>
@@ -541,7 +571,7 @@ static int launch_decode_tc(const rk_decode_args& a, const CUtensorMap& tk, cons
   e = launch_pdl(decode_tc_kernel<HH>, dim3(grid), dim3(dtc::kThreads), smem_bytes, st, tk, tv, t, idesc_qk, idesc_pv);
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_pdl(decode_tc_combine_kernel, dim3(a.B * a.H), dim3(128), 0, st, t, grid);
+  return (int)launch_pdl(decode_tc_combine_kernel, dim3(a.B * a.H), dim3(kCombineWarps * 32), 0, st, t, grid);
 }
 
 int launch_decode(const rk_decode_args& a, int nsplit, cudaStream_t st) {
@@ -563,7 +593,6 @@ int launch_decode(const rk_decode_args& a, int nsplit, cudaStream_t st) {
     t.o = reinterpret_cast<__nv_bfloat16*>(a.o); t.lse = a.lse;
     t.part_o = reinterpret_cast<float*>(a.workspace);
     t.part_ml = t.part_o + parts * 128;
-    t.starts = reinterpret_cast<int32_t*>(t.part_ml + parts * 2);
     t.status = status;
     t.B = a.B; t.H = a.H; t.H_kv = a.H_kv; t.L = a.L; t.grp = grp; t.nsplit = a.num_splits > 0 ? nsplit : 0;
     t.scale_log2 = scale * 1.4426950408889634f;

@@ -29,7 +29,8 @@
 //
 // A tile is a serial chain -- S from TMEM, maximum, exponentials, P in shared memory, P V -- several times as long as its
 // bytes take to arrive, so four groups of four worker warps each take every fourth tile, with accumulators and references
-// of their own that meet at the end of a segment.  One warp loads, one issues S = K Q^T, one O += V^T P.
+// of their own that meet at the end of a segment.  One warp loads, one puts the tiles' key scales into the order of a scale
+// atom, one issues S = K Q^T, one O += V^T P (with the scales in the issuer a tile took it 1100 cycles, as long as HBM).
 //   worker warp w: group w / 4, thread = key (w % 4) * 32 + lane of the tile for S and P, and column d of O^T.
 // p of a warp's 32 keys is relative to their own maximum rounded up to an integer m_w (log2 domain), which the block scale
 // undoes exactly: nothing in a tile waits for the other warps' maxima but the scale bytes.  O and the row sums are relative
@@ -50,8 +51,8 @@ namespace rk {
 namespace dtc {
 constexpr int kGroups = 4;                        // worker groups of four warps
 constexpr int kWorkers = 4 * kGroups;             // worker warps
-constexpr int kWarpTma = kWorkers, kWarpQk = kWorkers + 1, kWarpPv = kWorkers + 2;
-constexpr int kThreads = (kWorkers + 3) * 32;
+constexpr int kWarpTma = kWorkers, kWarpSf = kWorkers + 1, kWarpQk = kWorkers + 2, kWarpPv = kWorkers + 3;
+constexpr int kThreads = (kWorkers + 4) * 32;
 constexpr int kTile = 128;                        // keys per stage
 constexpr int kD = 128;
 constexpr int kMaxGrp = 8;                        // query heads per KV head this kernel handles
@@ -79,7 +80,8 @@ template <int HH> struct Lay {
   static constexpr int seg_off = ref_off + kWorkers * 16 * 4;  // end of a segment: [groups][8] references, [groups][4 warps][8] sums
   static constexpr int bar_off = seg_off + kGroups * (8 + 32) * 4;
   static constexpr int bFull = 0, bEmpty = bFull + kStages, bSF = bEmpty + kStages, bSE = bSF + kGroups, bPF = bSE + kGroups,
-                       bMX = bPF + kGroups, bPV = bMX + kGroups, bQF = bPV + kGroups, bQE = bQF + 2, bSeg = bQE + 2, bDrain = bSeg + 1,
+                       bMX = bPF + kGroups, bPV = bMX + kGroups, bKS = bPV + kGroups, bQF = bKS + kStages, bQE = bQF + 2, bSeg = bQE + 2,
+                       bDrain = bSeg + 1,
                        nBars = bDrain + 2;
   static constexpr int misc_off = bar_off + nBars * 8;         // tmem base, abort flag
   static constexpr int total = misc_off + 16;
@@ -108,7 +110,6 @@ struct DecodeTcParams {
   float* part_o;    // nsplit > 0: [B*H][nsplit][128]; 0: [CTA][2][grp][128] -- a CTA leaves at most two partials, of the unit its
                     // range begins inside of (slot 0) and of the one its range ends inside of (slot 1)
   float* part_ml;   // the same indices, [2]: reference maximum in the log2 domain, l
-  int32_t* starts;  // nsplit == 0: [1 + B * H_kv] tiles of the whole call, then each non-empty unit's first tile
   int* status;
   int B, H, H_kv, L, grp, nsplit;                 // nsplit: the caller's split count per unit, or 0 for equal ranges
   float scale_log2;
@@ -117,20 +118,21 @@ struct DecodeTcParams {
 RK_DEVINL int dtc_len(const DecodeTcParams& p, int b) { return p.kv_len ? min(max(p.kv_len[b], 0), p.L) : p.L; }
 RK_DEVINL int dtc_tiles(int len) { return (len + dtc::kTile - 1) / dtc::kTile; }
 // first tile of CTA c of g when t tiles are shared evenly
-RK_DEVINL int dtc_first(int t, int c, int g) { return (int)((int64_t)t * c / g); }
+RK_DEVINL int dtc_first(int t, int c, int g) {
+  const uint32_t q = (uint32_t)t / (uint32_t)g, r = (uint32_t)t - q * (uint32_t)g;      // t c / g without a 64-bit division (g < 2^16)
+  return (int)(q * (uint32_t)c + r * (uint32_t)c / (uint32_t)g);
+}
 
 // The segments of a CTA's range of tiles, in order.  Every warp walks its own copy.
 struct DtcSegments {
   int b, hkv, t0, n;        // current segment: tiles t0 .. t0 + n - 1 of unit (b, hkv)
   int len, n_unit;          // keys and tiles of the unit
   int left;                 // tiles of the range from this segment on; 0 = done
-  int first;                // index of the segment's first tile in the whole call (nsplit == 0)
 
   RK_DEVINL void clip() { n = min(n_unit - t0, left); }
   RK_DEVINL void seek(const DecodeTcParams& p) { len = dtc_len(p, b); n_unit = dtc_tiles(len); }
   RK_DEVINL void next(const DecodeTcParams& p) {
     left -= n;
-    first += n;
     t0 = 0;
     if (left <= 0) return;
     if (++hkv == p.H_kv) {
@@ -139,9 +141,8 @@ struct DtcSegments {
     }
     clip();
   }
-  // whole warp; total = tiles of the whole call
-  RK_DEVINL void start(const DecodeTcParams& p, int lane, int& total) {
-    total = 0;
+  RK_DEVINL void start(const DecodeTcParams& p, int lane) {      // whole warp
+    int total = 0, first;                                        // tiles of the whole call; the CTA's first of them
     if (p.nsplit > 0) {
       const int split = blockIdx.x % p.nsplit, u = blockIdx.x / p.nsplit;
       b = u / p.H_kv; hkv = u % p.H_kv;
@@ -149,7 +150,6 @@ struct DtcSegments {
       const int per = (n_unit + p.nsplit - 1) / p.nsplit;
       t0 = split * per;
       left = max(0, min(n_unit, t0 + per) - t0);
-      first = 0;
       clip();
       return;
     }
@@ -163,7 +163,9 @@ struct DtcSegments {
       clip();
       return;
     }
-    for (int i = lane; i < p.B; i += 32) total += dtc_tiles(dtc_len(p, i));
+    const int len0 = lane < p.B ? dtc_len(p, lane) : 0;           // the first 32 lengths are read once (a load is 0.4 us here)
+    total = dtc_tiles(len0);
+    for (int i = lane + 32; i < p.B; i += 32) total += dtc_tiles(dtc_len(p, i));
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
     total *= p.H_kv;
@@ -173,7 +175,8 @@ struct DtcSegments {
     if (left <= 0) return;
     int base = 0;                                              // tiles of the sequences before this block of 32
     for (int i0 = 0;; i0 += 32) {
-      const int mine = i0 + lane < p.B ? dtc_tiles(dtc_len(p, i0 + lane)) * p.H_kv : 0;
+      const int my_len = i0 == 0 ? len0 : i0 + lane < p.B ? dtc_len(p, i0 + lane) : 0;
+      const int mine = dtc_tiles(my_len) * p.H_kv;
       int incl = mine;
 #pragma unroll
       for (int s = 1; s < 32; s <<= 1) { const int o = __shfl_up_sync(0xffffffffu, incl, s); if (lane >= s) incl += o; }
@@ -182,7 +185,8 @@ struct DtcSegments {
         const int w = __ffs(past) - 1;
         b = i0 + w;
         const int off = first - base - __shfl_sync(0xffffffffu, incl - mine, w);
-        seek(p);
+        len = __shfl_sync(0xffffffffu, my_len, w);
+        n_unit = dtc_tiles(len);
         hkv = off / n_unit; t0 = off - hkv * n_unit;
         clip();
         return;
@@ -472,21 +476,19 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         if (d == 0) { p.part_ml[at * 2] = m; p.part_ml[at * 2 + 1] = l; }
       }
     }
-    if (p.nsplit == 0 && seg.t0 == 0 && threadIdx.x == 0) p.starts[1 + seg.b * p.H_kv + seg.hkv] = seg.first;
     if (seg.left > seg.n && !(ok = meet())) break;               // red has been read: the P tiles may be written again
   }
 }
 
-// One query head as two MXFP8 terms, q = hi + lo (the lib/golden block rule on q, then on the residual): a warp, four
-// elements per lane.  Heads past grp give zeros.
-template <int HH> RK_DEVINL void dtc_query_head(const DecodeTcParams& p, uint8_t* smem, int b, int hkv, int h, int buf, int lane) {
+// One lane's four elements of query head h of a unit; heads past grp give zeros.
+RK_DEVINL uint2 dtc_query_load(const DecodeTcParams& p, int b, int hkv, int h, int lane) {
+  if (h >= p.grp) return make_uint2(0u, 0u);
+  return __ldg(reinterpret_cast<const uint2*>(p.q + ((size_t)b * p.H + hkv * p.grp + h) * dtc::kD + lane * 4));
+}
+// The head as two MXFP8 terms, q = hi + lo (the lib/golden block rule on q, then on the residual): a warp together.
+template <int HH> RK_DEVINL void dtc_query_store(uint8_t* smem, uint2 raw, int h, int buf, int lane) {
   using L = dtc::Lay<HH>;
-  float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (h < p.grp) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p.q + ((size_t)b * p.H + hkv * p.grp + h) * dtc::kD + lane * 4);
-    x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xFFFF0000u);
-    x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xFFFF0000u);
-  }
+  float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000u)};
 #pragma unroll
   for (int term = 0; term < 2; ++term) {
     float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
@@ -549,13 +551,13 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
   grid_dependents_launch();
   const int stopped = threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0;
   DtcSegments seg;
-  int total;
-  seg.start(p, lane, total);
+  seg.start(p, lane);
+  if (warp < kWorkers) fence_proxy_async_smem();                      // the fills above
+  tc_fence_before();
   if (__syncthreads_or(stopped)) {                                    // an earlier launch gave up on a wait
     if (warp == kWarpQk) tmem_dealloc(*tmem_slot, kTmemCols);
     return;
   }
-  if (p.nsplit == 0 && blockIdx.x == 0 && threadIdx.x == 0) p.starts[0] = total;
 
   auto issue_tile = [&](int j, int tile) {                            // loads of the j-th tile of this CTA
     const int st = j % kStages;
@@ -570,55 +572,39 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
     bulk_load_1d(sb + 2 * kTileBytes + 512, p.v_scale + ((size_t)bhkv * p.L + key0) * 4, sbytes, &bars[L::bFull + st]);
   };
   const int n_early = min(kStages, seg.left > 0 ? seg.n : 0);         // tiles whose loads run under the rest of the set-up
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
   if (warp == kWarpTma) {
     if (lane == 0)
       for (int j = 0; j < n_early; ++j) issue_tile(j, seg.t0 + j);
-  } else if (warp < kWorkers) {
-    if (warp < HH && seg.left > 0) dtc_query_head<HH>(p, smem, seg.b, seg.hkv, warp, 0, lane);
+  } else if (warp < HH) {                                             // first query terms: the only thing S waits for beside its tile
+    if (seg.left > 0) dtc_query_store<HH>(smem, dtc_query_load(p, seg.b, seg.hkv, warp, lane), warp, 0, lane);
     fence_proxy_async_smem();
+    asm volatile("bar.arrive 1, %0;" ::"n"((HH + 1) * 32) : "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
 
   if (warp == kWarpTma) {
-    // ================= loads; query terms of every segment after the first =================
+    // ================= loads =================
     int j = 0;
-    for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
-      if (s > 0) {
-        if (s >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQE + (s & 1)], ((s >> 1) - 1) & 1, abort_flag, p.status, 512));
-        if (!ok) break;
-#pragma unroll 1
-        for (int h = 0; h < p.grp; ++h) dtc_query_head<HH>(p, smem, seg.b, seg.hkv, h, s & 1, lane);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[L::bQF + (s & 1)]);
-      }
+    for (; seg.left > 0 && ok; seg.next(p)) {
       for (int i = 0; i < seg.n && ok; ++i, ++j) {
         if (j < n_early) continue;
         if (j >= kStages) ok = __all_sync(0xffffffffu, mbar_wait<20000>(&bars[L::bEmpty + j % kStages], (j / kStages - 1) & 1, abort_flag, p.status, 511));
         if (ok && lane == 0) issue_tile(j, seg.t0 + i);
       }
     }
-  } else if (warp == kWarpQk) {
-    // ================= S^T = K Q^T (all lanes re-tile the key scales, lane 0 issues) =================
-    const uint64_t dk = make_smem_desc(smem_u32(smem + L::stage_off), 16, 1024, kLayoutSw128);
-    const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
-    const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::stage_off + 2 * kTileBytes), 0, 128, kLayoutNone);
-    if (lane == 0) tc_cp_32x128b_warpx4(tmem_base + cSfOne, make_smem_desc(smem_u32(smem + L::one_off), 0, 128, kLayoutNone));
+  } else if (warp == kWarpSf) {
+    // ================= key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32, in place; and the query terms of
+    // the next segment, loaded at the beginning of a segment and put down at its end =================
     int j = 0;
-    for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
-      if (s > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQF + (s & 1)], (s & 1) ? (s >> 1) & 1 : ((s >> 1) - 1) & 1, abort_flag, p.status, 525));
-      if (!ok) break;
-      if (lane == 0)
-        tc_cp_32x128b_warpx4(tmem_base + cSfQ + (s & 1) * 4, make_smem_desc(smem_u32(smem + L::sfq_off + (s & 1) * 512), 0, 128, kLayoutNone));
+    for (int s = 0; seg.left > 0 && ok; ++s) {
+      DtcSegments next = seg;
+      uint2 nq[HH];
       for (int i = 0; i < seg.n && ok; ++i, ++j) {
-        const int st = j % kStages, g = j & (kGroups - 1);
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 521));
+        const int st = j % kStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 527));
         if (!ok) break;
-        // key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32
         uint32_t* ks = reinterpret_cast<uint32_t*>(smem + L::stage_off + st * kStageBytes + 2 * kTileBytes);
         uint32_t w[4];
 #pragma unroll
@@ -627,15 +613,54 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
         *reinterpret_cast<uint4*>(ks + lane * 4) = make_uint4(w[0], w[1], w[2], w[3]);
         fence_proxy_async_smem();
         __syncwarp();
-        if (j >= kGroups) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSE + g], (j / kGroups - 1) & 1, abort_flag, p.status, 522));
-        if (ok && lane == 0) {
+        if (lane == 0) mbar_arrive(&bars[L::bKS + st]);
+        if (i == 0) {
+          next.next(p);
+          if (next.left > 0) {
+#pragma unroll
+            for (int h = 0; h < HH; ++h) nq[h] = dtc_query_load(p, next.b, next.hkv, h, lane);
+          }
+        }
+      }
+      if (ok && next.left > 0) {
+        if (s >= 1) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQE + ((s + 1) & 1)], (((s + 1) >> 1) - 1) & 1, abort_flag, p.status, 512));
+        if (!ok) break;
+#pragma unroll
+        for (int h = 0; h < HH; ++h) dtc_query_store<HH>(smem, nq[h], h, (s + 1) & 1, lane);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[L::bQF + ((s + 1) & 1)]);
+      }
+      seg = next;
+    }
+  } else if (warp == kWarpQk) {
+    // ================= S^T = K Q^T (one lane) =================
+    asm volatile("bar.sync 1, %0;" ::"n"((HH + 1) * 32) : "memory");
+    if (lane == 0) {
+      const uint64_t dk = make_smem_desc(smem_u32(smem + L::stage_off), 16, 1024, kLayoutSw128);
+      const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
+      const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::stage_off + 2 * kTileBytes), 0, 128, kLayoutNone);
+      tc_cp_32x128b_warpx4(tmem_base + cSfOne, make_smem_desc(smem_u32(smem + L::one_off), 0, 128, kLayoutNone));
+      int j = 0;
+      for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
+        if (s > 0) ok = mbar_wait(&bars[L::bQF + (s & 1)], (s & 1) ? (s >> 1) & 1 : ((s >> 1) - 1) & 1, abort_flag, p.status, 525);
+        if (!ok) break;
+        tc_cp_32x128b_warpx4(tmem_base + cSfQ + (s & 1) * 4, make_smem_desc(smem_u32(smem + L::sfq_off + (s & 1) * 512), 0, 128, kLayoutNone));
+        const uint64_t dqs = dq + (uint32_t)((s & 1) * (2048 >> 4));
+        for (int i = 0; i < seg.n && ok; ++i, ++j) {
+          const int st = j % kStages, g = j & (kGroups - 1);
+          // (the tile itself has landed: the scale warp waited for it; the second wait orders it for this thread)
+          ok = mbar_wait(&bars[L::bKS + st], (j / kStages) & 1, abort_flag, p.status, 528) &&
+               mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 521);
+          if (ok && j >= kGroups) ok = mbar_wait(&bars[L::bSE + g], (j / kGroups - 1) & 1, abort_flag, p.status, 522);
+          if (!ok) break;
           tc_fence_after();
           const uint32_t so = (uint32_t)(st * (kStageBytes >> 4));
           tc_cp_32x128b_warpx4(tmem_base + cSfK + st * 4, dsfk + so);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tmem_base + cS + g * 16, dk + so + kk * 2, dq + (uint32_t)((s & 1) * (2048 >> 4)) + kk * 2,
-                            idesc_with_sf(idesc_qk, kk, kk), tmem_base + cSfK + st * 4, tmem_base + cSfQ + (s & 1) * 4, kk > 0 ? 1u : 0u);
+            mma_mxf8f6f4_ss(tmem_base + cS + g * 16, dk + so + kk * 2, dqs + kk * 2, idesc_with_sf(idesc_qk, kk, kk),
+                            tmem_base + cSfK + st * 4, tmem_base + cSfQ + (s & 1) * 4, kk > 0 ? 1u : 0u);
           tc_commit(&bars[L::bSF + g]);
           if (i == seg.n - 1) tc_commit(&bars[L::bQE + (s & 1)]);
         }

@@ -505,6 +505,8 @@ __global__ void __launch_bounds__(128) kv_append_kernel(const float* __restrict_
   const int cpr = d / 8;                                     // chunks per row (a multiple of 4)
   const int64_t rows = (int64_t)B * H_kv, nchunks = 2 * rows * cpr;
   const int lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_dependents_launch();
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c - lane < nchunks; c += (int64_t)gridDim.x * blockDim.x) {
     const bool live = c < nchunks;
     const int64_t cc = live ? c : 0;
@@ -1168,7 +1170,7 @@ int launch_kv_append(const float* k_new, const float* v_new, int B, int H_kv, in
   const int64_t total = 2LL * B * H_kv * (d / 8);
   if (total == 0) return RK_OK;
   const int grid = grid_for(total, 128, 8);
-  RK_DISPATCH_FMT(fmt, (kv_append_kernel<F><<<grid, 128, 0, st>>>(k_new, v_new, B, H_kv, L, d, pos, k_codes, k_scales, v_codes, v_scales)));
+  RK_DISPATCH_FMT(fmt, return (int)launch_pdl(kv_append_kernel<F>, dim3(grid), dim3(128), 0, st, k_new, v_new, B, H_kv, L, d, pos, k_codes, k_scales, v_codes, v_scales));
   return (int)cudaGetLastError();
 }
 
