@@ -28,14 +28,17 @@
 // partials for the combine kernel.  (One split count for all sequences lets the longest ones set the time.)
 //
 // A tile is a serial chain -- S from TMEM, maximum, exponentials, P in shared memory, P V -- several times as long as its
-// bytes take to arrive, so four groups of four worker warps each take every fourth tile, with accumulators and references
-// of their own that meet at the end of a segment.  One warp loads, one puts the tiles' key scales into the order of a scale
-// atom, one issues S = K Q^T, one O += V^T P (with the scales in the issuer a tile took it 1100 cycles, as long as HBM).
+// bytes take to arrive, so four groups of four worker warps each take every fourth tile.  One warp loads, one puts the
+// tiles' key scales into the order of a scale atom, one issues S = K Q^T, one O += V^T P (with the scales in the issuer a
+// tile took it 1100 cycles, as long as HBM).
 //   worker warp w: group w / 4, thread = key (w % 4) * 32 + lane of the tile for S and P, and column d of O^T.
 // p of a warp's 32 keys is relative to their own maximum rounded up to an integer m_w (log2 domain), which the block scale
 // undoes exactly: nothing in a tile waits for the other warps' maxima but the scale bytes.  O and the row sums are relative
-// to a reference m_ref of the group, the first tile's largest m_w; fp32 carries them while later maxima stay below m_ref +
-// 32 (and V scales below theirs), so O is rescaled about never.
+// to a reference m_ref, the first tile's largest m_w, that is handed from tile to tile; fp32 carries them while later maxima
+// stay below m_ref + 32 (and V scales below theirs), so O is rescaled about never.
+// A segment ends in the group of its last tile alone: it reads O (one of four accumulators, used in turn) and the row sums
+// the other warps left, while those are in the next segment's tiles.  (With a meeting of all workers at its end a segment
+// cost 5000 cycles, four tiles' time.)
 //
 // Included by rk_decode.cu (one translation unit: both kernels share the launcher).
 #pragma once
@@ -59,12 +62,13 @@ constexpr int kMaxGrp = 8;                        // query heads per KV head thi
 constexpr int kNq = 16;                           // B rows of the QK^T MMA: term * HH + h (rows past 2 HH stay zero)
 constexpr int kTileBytes = kTile * kD;            // 16384
 constexpr int kStageBytes = 2 * kTileBytes + 2 * 512;   // K, V, K scales [128][4], V scales [128][4]
+constexpr int kOBufs = 4, kRing = 8;              // accumulators in turn; tiles whose references are kept
 constexpr float kBump = 32.0f;                    // rescale O when a maximum passes its reference by more than 2^this
 
 // Per head capacity HH (4 or 8): column n of the PV MMA = q * 2 HH + term * HH + h.
 template <int HH> struct Lay {
   static constexpr int kNp = 8 * HH;
-  static constexpr int kStages = HH == 8 ? 5 : 6;
+  static constexpr int kStages = 5;
   // P tiles: rows of 128 bytes (128-byte swizzle), one row per key; a group's tile takes kNp bytes of each row
   static constexpr int kPerAtom = 128 / kNp;
   static constexpr int kPBytes = kGroups / kPerAtom * kTileBytes;
@@ -76,23 +80,23 @@ template <int HH> struct Lay {
   static constexpr int sfq_off = sfp_off + kGroups * 512;      // scale atoms of the query terms, [2 segments]
   static constexpr int one_off = sfq_off + 2 * 512;            // scale atom of ones (code 127) for V
   static constexpr int xchg_off = one_off + 512;               // [groups][2][4 warps][16] floats: m_w of the heads, then svmax
-  static constexpr int ref_off = xchg_off + kGroups * 2 * 4 * 16 * 4;   // [16 warps][16] floats: references, same order
-  static constexpr int seg_off = ref_off + kWorkers * 16 * 4;  // end of a segment: [groups][8] references, [groups][4 warps][8] sums
-  static constexpr int bar_off = seg_off + kGroups * (8 + 32) * 4;
+  static constexpr int ring_off = xchg_off + kGroups * 2 * 4 * 16 * 4;  // [8 tiles][16] floats: references after a tile, same order
+  static constexpr int ref_off = ring_off + kRing * 16 * 4;    // [16 warps][16] floats: the references a warp's sums are relative to
+  static constexpr int seg_off = ref_off + kWorkers * 16 * 4;  // end of a segment: [kOBufs][16 warps][8] float2: sum, its reference
+  static constexpr int bar_off = seg_off + kOBufs * kWorkers * 8 * 8;
   static constexpr int bFull = 0, bEmpty = bFull + kStages, bSF = bEmpty + kStages, bSE = bSF + kGroups, bPF = bSE + kGroups,
-                       bMX = bPF + kGroups, bPV = bMX + kGroups, bKS = bPV + kGroups, bQF = bKS + kStages, bQE = bQF + 2, bSeg = bQE + 2,
-                       bDrain = bSeg + 1,
+                       bMX = bPF + kGroups, bPV = bMX + kGroups, bKS = bPV + kGroups, bQF = bKS + kStages, bQE = bQF + 2, bRef = bQE + 2,
+                       bSL = bRef + kRing, bOE = bSL + kOBufs, bDrain = bOE + kOBufs,
                        nBars = bDrain + 2;
   static constexpr int misc_off = bar_off + nBars * 8;         // tmem base, abort flag
   static constexpr int total = misc_off + 16;
   static_assert(kStageBytes % 1024 == 0 && p_off % 1024 == 0 && q_off % 1024 == 0, "swizzled tiles need 1024-byte alignment");
-  static_assert(kPBytes >= kGroups * HH * 512, "the segment's merge uses the P tiles");
   static_assert(total + 1024 <= 232448, "shared memory of a CTA");
 };
 
 // TMEM columns
 constexpr uint32_t cS = 0;                        // 16 per group
-constexpr uint32_t cO = 64;                       // up to 64 per group
+constexpr uint32_t cO = 64;                       // up to 64 per accumulator
 constexpr uint32_t cSfK = 320;                    // 4 per stage
 constexpr uint32_t cSfQ = 344;                    // 4 per segment parity
 constexpr uint32_t cSfP = 352;                    // 4 per group
@@ -250,32 +254,25 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
   const int g = warp >> 2, wq = warp & 3, kt = wq * 32 + lane;
   const uint32_t lane_addr = ((uint32_t)(wq * 32)) << 16;
   const uint32_t s_addr = tmem_base + lane_addr + cS + g * 16;
-  const uint32_t o_addr = tmem_base + lane_addr + cO + g * 64 + wq * 2 * HH;    // row d = kt: only the columns of its q = wq count
+  const uint32_t o_row = tmem_base + lane_addr + cO + wq * 2 * HH;               // row d = kt: only the columns of its q = wq count
   // this key's row of the group's P tile; 16-byte chunk i of it sits at (chunk0 + i) ^ (kt & 7)
   uint8_t* prow = smem + L::p_off + (g / L::kPerAtom) * kTileBytes + kt * 128;
   const int chunk0 = (g % L::kPerAtom) * (L::kNp / 16);
   float* xchg = reinterpret_cast<float*>(smem + L::xchg_off) + g * 128;          // [2][4 warps][16]
-  float* ref = reinterpret_cast<float*>(smem + L::ref_off) + warp * 16;          // this warp's copy of the group's references
-  float* seg_m = reinterpret_cast<float*>(smem + L::seg_off);                    // [groups][8]
-  float* seg_l = seg_m + kGroups * 8;                                            // [groups][4 warps][8]
-  uint32_t seg_par = 0;
-  auto meet = [&]() -> bool {                                                    // all worker warps
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars[L::bSeg]);
-    const bool r = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSeg], seg_par, abort_flag, p.status, 506));
-    seg_par ^= 1;
-    return r;
-  };
+  float* ring = reinterpret_cast<float*>(smem + L::ring_off);                    // [kRing][16]
+  float* ref = reinterpret_cast<float*>(smem + L::ref_off) + warp * 16;          // what this warp's sums are relative to
+  float2* sums = reinterpret_cast<float2*>(smem + L::seg_off);                   // [kOBufs][16 warps][8]
+  const int item = lane & 15;                                                    // 0..7: a head, 8..11: a group of 32 columns of d
   bool ok = true;
   int j0 = 0;                                                                    // tiles of this CTA before the segment
 
-  for (; seg.left > 0 && ok; j0 += seg.n, seg.next(p)) {
+  for (int sg = 0; seg.left > 0 && ok; ++sg, j0 += seg.n, seg.next(p)) {
+    const uint32_t o_addr = o_row + (sg % kOBufs) * 64;
     float l_part[HH];
 #pragma unroll
     for (int h = 0; h < HH; ++h) l_part[h] = 0.0f;
-    float ref_item = 0.0f;                                                       // lane & 15: m_ref of a head, then V scale references
+    float ref_item = 0.0f;                                                       // of this lane's item, as in ref[]
     const int i_first = (g - j0) & (kGroups - 1);
-    int use = 0;                                                                 // parity of the last tile's barriers + 1
 
     for (int i = i_first; i < seg.n; i += kGroups) {
       const int j = j0 + i, st = j % kStages, par = (j / kGroups) & 1;
@@ -334,8 +331,8 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         hi[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
         lo[h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
       }
-      // the P tile is free once the P V that read it (the group's previous tile in this segment) has completed
-      if (i != i_first) {
+      // the P tile is free once the P V that read it (the group's previous tile) has completed
+      if (j >= kGroups) {
         ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
         if (!ok) break;
       }
@@ -362,38 +359,50 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
       }
 
       // ---- references, scale bytes, row sums --------------------------------------------------------------------
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504));
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504) &&
+                                       (i == 0 || mbar_wait(&bars[L::bRef + (j - 1) % kRing], ((j - 1) / kRing) & 1, abort_flag, p.status, 507)));
       if (!ok) break;
-      const int item = lane & 15;
       {
         const float* xr = xchg + par * 64 + (lane >> 4) * 32 + item;
         float top = fmaxf(xr[0], xr[16]);
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+        const float before = i == 0 ? top : ring[((j - 1) % kRing) * 16 + item];
         // every warp of the group sees the same maxima and references, so this is uniform over the group
-        if (__any_sync(0xffffffffu, top > ref_item + kBump) || i == i_first) {
-          if (i == i_first) ref_item = top;
-          const float fresh = fmaxf(ref_item, top);
-          if (i != i_first) {
-            // rescale this thread's row of O (the previous P V has landed, see above) and the row sums
-            tc_fence_after();
-            uint32_t o[2 * HH];
-            if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
-            tc_wait_ld();
-            const float down = ref_item - fresh, down_v = __shfl_sync(0xffffffffu, down, 8 + wq);
-#pragma unroll
-            for (int h = 0; h < HH; ++h) {
-              const float dh = __shfl_sync(0xffffffffu, down, h);
-              const float f = ex2_approx(fmaxf(dh + down_v, -126.0f));
-              o[h] = __float_as_uint(__uint_as_float(o[h]) * f);
-              o[HH + h] = __float_as_uint(__uint_as_float(o[HH + h]) * f);
-              l_part[h] *= ex2_approx(dh);
-            }
-            if (HH == 8) tmem_st16(o_addr, o); else tmem_st8(o_addr, o);
-            tc_wait_st();
-          }
-          ref_item = fresh;
+        const bool bump = __any_sync(0xffffffffu, top > before + kBump);
+        const float now = bump ? fmaxf(before, top) : before;
+        if (wq == 0) {
+          if (lane < 16) ring[(j % kRing) * 16 + lane] = now;
           __syncwarp();
-          if (lane < 16) ref[lane] = ref_item;
+          if (lane == 0) mbar_arrive(&bars[L::bRef + j % kRing]);
+        }
+        if (bump) {
+          // rescale this thread's row of O once the tile before has been added; its own P V comes after this
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + ((j - 1) & (kGroups - 1))], ((j - 1) / kGroups) & 1, abort_flag, p.status, 502));
+          if (!ok) break;
+          tc_fence_after();
+          uint32_t o[2 * HH];
+          if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
+          tc_wait_ld();
+          const float down = before - now, down_v = __shfl_sync(0xffffffffu, down, 8 + wq);
+#pragma unroll
+          for (int h = 0; h < HH; ++h) {
+            const float f = ex2_approx(fmaxf(__shfl_sync(0xffffffffu, down, h) + down_v, -126.0f));
+            o[h] = __float_as_uint(__uint_as_float(o[h]) * f);
+            o[HH + h] = __float_as_uint(__uint_as_float(o[HH + h]) * f);
+          }
+          if (HH == 8) tmem_st16(o_addr, o); else tmem_st8(o_addr, o);
+          tc_wait_st();
+        }
+        if (i == i_first || __any_sync(0xffffffffu, now != ref_item)) {
+          // first tile of the segment here, or a reference moved here or in another group: this warp's sums follow
+          if (i != i_first) {
+            const float down = ref_item - now;
+#pragma unroll
+            for (int h = 0; h < HH; ++h) l_part[h] *= ex2_approx(__shfl_sync(0xffffffffu, down, h));
+          }
+          ref_item = now;
+          __syncwarp();
+          if (lane < 16) ref[lane] = now;
           __syncwarp();
         }
       }
@@ -418,65 +427,84 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[L::bPF + g]);
-      use = par + 1;
     }
     if (!ok) break;
 
-    // ---- end of the segment: row d = kt of every group's O^T, merged ------------------------------------------------
-    float oh[HH];
+    // ---- end of the segment: every warp leaves its row sums; the group of the last tile puts the result together --------
+    const int ob = sg % kOBufs;
+    if (sg >= kOBufs) {                                            // the slot has been read
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bOE + ob], (sg / kOBufs - 1) & 1, abort_flag, p.status, 508));
+      if (!ok) break;
+    }
+    {
+      // 32 lanes x HH sums -> lane h holds head h: halve the heads while folding the lanes
+      float v[HH];
 #pragma unroll
-    for (int h = 0; h < HH; ++h) oh[h] = 0.0f;
-    if (use > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], use - 1, abort_flag, p.status, 505));
+      for (int h = 0; h < HH; ++h) v[h] = l_part[h];
+#pragma unroll
+      for (int w = HH / 2; w >= 1; w >>= 1) {
+        const bool up = (lane & w) != 0;
+#pragma unroll
+        for (int h = 0; h < w; ++h) {
+          const float give = up ? v[h] : v[h + w], keep = up ? v[h + w] : v[h];
+          v[h] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+        }
+      }
+      float l = v[0];
+#pragma unroll
+      for (int x = HH; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+      if (lane < HH) sums[(ob * kWorkers + warp) * 8 + lane] = make_float2(l, ref_item);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[L::bSL + ob]);
+    }
+    const int j_last = j0 + seg.n - 1;
+    if ((j_last & (kGroups - 1)) == g) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], (j_last / kGroups) & 1, abort_flag, p.status, 505) &&
+                                       mbar_wait(&bars[L::bSL + ob], (sg / kOBufs) & 1, abort_flag, p.status, 506));
       if (!ok) break;
       tc_fence_after();
       uint32_t o[2 * HH];
       if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
+      // row sums: lane = (warp of 16, half of the heads); this warp's references are the segment's last
+      float l[HH / 2];
+      {
+        const int w = lane & 15, h0 = (lane >> 4) * (HH / 2);
+#pragma unroll
+        for (int k = 0; k < HH / 2; ++k) {
+          const float2 s = sums[(ob * kWorkers + w) * 8 + h0 + k];
+          l[k] = s.x == 0.0f ? 0.0f : s.x * ex2_approx(s.y - ref[h0 + k]);
+        }
+#pragma unroll
+        for (int x = 8; x >= 1; x >>= 1)
+#pragma unroll
+          for (int k = 0; k < HH / 2; ++k) l[k] += __shfl_xor_sync(0xffffffffu, l[k], x);
+      }
       tc_wait_ld();
       tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[L::bOE + ob]);
       const int e = (int)ref[8 + wq] - 127 - 8, e0 = e / 2;                       // in two factors: e can be -135
+      const float back = pow2i(e0), back2 = pow2i(e - e0);
+      const bool whole = seg.n == seg.n_unit;
+      const size_t bh0 = (size_t)seg.b * p.H + seg.hkv * p.grp;
 #pragma unroll
-      for (int h = 0; h < HH; ++h) oh[h] = (__uint_as_float(o[h]) + __uint_as_float(o[HH + h])) * pow2i(e0) * pow2i(e - e0);
-    }
-#pragma unroll
-    for (int h = 0; h < HH; ++h) {
-      float l = l_part[h];
-#pragma unroll
-      for (int x = 16; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
-      if (lane == 0) seg_l[(g * 4 + wq) * 8 + h] = l;
-    }
-    if (wq == 0 && lane < 8) seg_m[g * 8 + lane] = use > 0 ? ref_item : NEG_INF;
-    if (!(ok = meet())) break;
-    float* red = reinterpret_cast<float*>(smem + L::p_off) + g * HH * 128;       // [HH][128], where the P tiles were
-#pragma unroll
-    for (int h = 0; h < HH; ++h) {
-      const float m = fmaxf(fmaxf(seg_m[h], seg_m[8 + h]), fmaxf(seg_m[16 + h], seg_m[24 + h]));
-      red[h * 128 + kt] = use > 0 ? oh[h] * ex2_approx(seg_m[g * 8 + h] - m) : 0.0f;
-    }
-    if (!(ok = meet())) break;
-    const bool whole = seg.n == seg.n_unit;
-    const size_t bh0 = (size_t)seg.b * p.H + seg.hkv * p.grp;
-    for (int idx = threadIdx.x; idx < p.grp * 128; idx += kWorkers * 32) {       // heads g, g + 4
-      const int h = idx >> 7, d = idx & 127;
-      const float m = fmaxf(fmaxf(seg_m[h], seg_m[8 + h]), fmaxf(seg_m[16 + h], seg_m[24 + h]));
-      float acc = 0.0f, l = 0.0f;
-#pragma unroll
-      for (int x = 0; x < kGroups; ++x) {
-        acc += reinterpret_cast<const float*>(smem + L::p_off)[(x * HH + h) * 128 + d];
-        const float lx = (seg_l[x * 32 + h] + seg_l[x * 32 + 8 + h]) + (seg_l[x * 32 + 16 + h] + seg_l[x * 32 + 24 + h]);
-        l += seg_m[x * 8 + h] == NEG_INF ? 0.0f : lx * ex2_approx(seg_m[x * 8 + h] - m);
+      for (int h = 0; h < HH; ++h) {
+        const float lh = __shfl_sync(0xffffffffu, l[h % (HH / 2)], h / (HH / 2) * 16);
+        if (h < p.grp) {
+          const float acc = (__uint_as_float(o[h]) + __uint_as_float(o[HH + h])) * back * back2, m = ref[h];
+          if (whole) {
+            p.o[(bh0 + h) * 128 + kt] = __float2bfloat16_rn(acc * (lh > 0.0f ? 1.0f / lh : 1.0f));
+            if (p.lse && kt == 0) p.lse[bh0 + h] = lh > 0.0f ? m * 0.6931471805599453f + logf(lh) : NEG_INF;
+          } else {
+            const size_t at = p.nsplit > 0 ? (bh0 + h) * p.nsplit + blockIdx.x % p.nsplit
+                                           : ((size_t)blockIdx.x * 2 + (seg.t0 > 0 ? 0 : 1)) * p.grp + h;
+            p.part_o[at * 128 + kt] = acc;
+            if (kt == 0) { p.part_ml[at * 2] = m; p.part_ml[at * 2 + 1] = lh; }
+          }
+        }
       }
-      if (whole) {
-        p.o[(bh0 + h) * 128 + d] = __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 1.0f));
-        if (p.lse && d == 0) p.lse[bh0 + h] = l > 0.0f ? m * 0.6931471805599453f + logf(l) : NEG_INF;
-      } else {
-        const size_t at = p.nsplit > 0 ? (bh0 + h) * p.nsplit + blockIdx.x % p.nsplit
-                                       : ((size_t)blockIdx.x * 2 + (seg.t0 > 0 ? 0 : 1)) * p.grp + h;
-        p.part_o[at * 128 + d] = acc;
-        if (d == 0) { p.part_ml[at * 2] = m; p.part_ml[at * 2 + 1] = l; }
-      }
+      __syncwarp();                                              // ref[] has been read
     }
-    if (seg.left > seg.n && !(ok = meet())) break;               // red has been read: the P tiles may be written again
   }
 }
 
@@ -535,7 +563,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
   if (warp == kWarpPv) {
     for (int i = L::bEmpty + lane; i < L::nBars; i += 32) {
       const bool per_warp = i >= L::bSE && i < L::bPV;                // SE, PF, MX: the four warps of a group
-      mbar_init(&bars[i], i == L::bSeg ? kWorkers : per_warp ? 4 : 1);
+      const bool four = per_warp || (i >= L::bOE && i < L::bDrain), all = i >= L::bSL && i < L::bOE;
+      mbar_init(&bars[i], all ? kWorkers : four ? 4 : 1);
     }
     fence_barrier_init();
   }
@@ -679,7 +708,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
       const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), kTileBytes, 1024, kLayoutSw128);
       const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
       int j = 0;
-      for (; seg.left > 0 && ok; seg.next(p)) {
+      for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
+        if (s >= kOBufs) ok = mbar_wait(&bars[L::bOE + s % kOBufs], (s / kOBufs - 1) & 1, abort_flag, p.status, 529);
         for (int i = 0; i < seg.n && ok; ++i, ++j) {
           const int st = j % kStages, g = j & (kGroups - 1);
           ok = mbar_wait(&bars[L::bPF + g], (j / kGroups) & 1, abort_flag, p.status, 523);
@@ -690,8 +720,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
           const uint64_t dpt = dp + (uint32_t)((g / L::kPerAtom) * (kTileBytes >> 4) + (g % L::kPerAtom) * (L::kNp >> 4));
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tmem_base + cO + g * 64, dvt + kk * (4096 >> 4), dpt + kk * (4096 >> 4), idesc_with_sf(idesc_pv, kk, kk),
-                            tmem_base + cSfOne, tmem_base + cSfP + g * 4, (i >= kGroups || kk > 0) ? 1u : 0u);
+            mma_mxf8f6f4_ss(tmem_base + cO + (s % kOBufs) * 64, dvt + kk * (4096 >> 4), dpt + kk * (4096 >> 4), idesc_with_sf(idesc_pv, kk, kk),
+                            tmem_base + cSfOne, tmem_base + cSfP + g * 4, (i > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&bars[L::bPV + g]);
           tc_commit(&bars[L::bEmpty + st]);
         }

@@ -254,3 +254,37 @@ def test_kv_cache_append_then_decode_in_a_loop(fmt):
     assert torch.equal(kc[1, :, :100], kc_all[1, :, :100]) and bool((kc[1, :, 100:] == 0x7F).all())
     oc, os_ = oracle.quantize(np_(V[0, 0, :T]), axis=1, fmt=fmt)
     assert np.array_equal(np_(vc[0, 0, :T]), oc) and np.array_equal(np_(vs[0, 0, :T]), os_)
+
+
+@pytest.mark.parametrize("grp,case", [(4, "short"), (8, "short"), (4, "rising"), (8, "rising"), (4, "v jump"), (8, "v jump"), (1, "few tiles")])
+def test_ranges_and_references(grp, case):
+    """The tcgen05 kernel's equal ranges of tiles and its running references: many short sequences per CTA (empty ones, single
+    keys and tile edges among them), fewer tiles than CTAs, scores that rise by far more than 2^32 over the keys and V block
+    scales that do (O is then rescaled, again and again, while other tiles are in flight)."""
+    Hkv, d = 2, 128
+    B, L = {"short": (71, 520), "rising": (2, 3000), "v jump": (2, 3000), "few tiles": (3, 132)}[case]
+    rng = np.random.default_rng(grp)
+    lens = rng.choice([0, 1, 127, 128, 129, 256, 384, 520], B).astype(np.int32) if case == "short" else np.array([L, 0, 5] if B == 3 else [L, L - 77], np.int32)
+    g = torch.Generator(device="cuda").manual_seed(grp)
+    q = torch.randn(B, grp * Hkv, d, generator=g, device="cuda").bfloat16()
+    K = torch.randn(B, Hkv, L, d, generator=g, device="cuda")
+    V = torch.randn(B, Hkv, L, d, generator=g, device="cuda")
+    step = torch.arange(L, device="cuda", dtype=torch.float32).view(1, 1, L, 1) / L
+    if case == "rising":
+        K = K * 0.25 + step * 40.0 * q.float().view(B, Hkv, grp, d)[:, :, :1].sign()      # the first head of a group climbs by some 500
+    if case == "v jump":
+        V = V * torch.exp2(torch.floor(step * 100.0 - 60.0))
+    kc, ks = rk.mx_quantize(K)
+    vc, vs = rk.mx_quantize(V)
+    lse = torch.empty(B, grp * Hkv, dtype=torch.float32, device="cuda")
+    o = rk.attn_decode(q, kc, vc, ks, vs, kv_len=torch.from_numpy(lens).cuda(), lse=lse)
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+    ref = oracle.attn_decode(np_(q.view(torch.uint16)), np_(kc), np_(vc), np_(ks), np_(vs), softmax_scale=d ** -0.5, kv_len=lens, want_lse=True)
+    got, want = np_(o.float()), ref["o_f32"]
+    assert np.isfinite(got).all()
+    big = max(1.0, float(np.abs(want).max()))
+    assert np.abs(got - want).max() <= MAX_ABS * big and errors(got, want)[1] <= REL_L2
+    full = lens > 0
+    assert np.abs(np_(lse)[full] - ref["lse"][full]).max() < 2e-3
+    assert (got[~full] == 0).all()
