@@ -348,8 +348,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // an earlier launch on this device gave up on a wait: do nothing until the host has read the status
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
   // heavy (late) query tiles first within a head; heads adjacent so a KV head's tiles share L2
   // work order: see PrefillParams::head_group (heaviest query tiles of a whole group of heads first)
   const int n_bh = p.B * p.H;
@@ -389,10 +387,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     fence_barrier_init();
   }
   if (warp == kNumSoftmaxWarps + 1) { tmem_alloc(tmem_ptr, kTmemCols); tmem_relinquish(); }
+  grid_dependency_wait();
+  grid_dependents_launch();
   tc_fence_before();
-  __syncthreads();
+  // an earlier launch on this device gave up on a wait: do nothing until the host has read the status
+  const int stopped = __syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
+  if (stopped) {
+    if (warp == kNumSoftmaxWarps + 1) tmem_dealloc(tmem_base, kTmemCols);
+    return;
+  }
 
   if (n_tiles == 0) {
     // no visible key: O = 0 (the l <= 0 guard of finalize_O, kernels/flash_attention_mx_gemma/flash_mx_impl.hpp:554-560)
@@ -595,9 +600,9 @@ static int launch_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return (int)e;
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
-  kern<<<grid, kNumThreads, smem_bytes, st>>>(tq, tk, tv, p, idesc_qk, idesc_pv);
+  e = launch_pdl(kern, grid, dim3(kNumThreads), smem_bytes, st, tq, tk, tv, p, idesc_qk, idesc_pv);
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
-  return (int)cudaGetLastError();
+  return (int)e;
 }
 
 float* g_prefill_dbg = nullptr;   // set by rk_debug_set_prefill_dump (tests only)
@@ -649,7 +654,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
   const uint32_t idesc_pv = make_idesc(RK_FMT_E4M3, a.kv_fmt, false, /*B MN-major*/ !kv6, 128, 128);
   dim3 grid(p.n_q_tiles * a.H * a.B, 1, 1);
   const bool cap = a.softcap > 0.0f;
-  if (a.d <= 128) return launch_prefill2c(tq, tk, tv, p, idesc_qk, idesc_pv, cap, a.B, st);   // two query tiles per CTA
+  if (a.d <= 128) return launch_prefill2c(tq, tk, tv, p, idesc_qk, idesc_pv, cap, st);   // two query tiles per CTA
   if (p.dbg)      // the stage dump lives in instantiations of its own: the kernels that ship carry none of its code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)
                : launch_cfg<2, 2, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st);

@@ -157,7 +157,7 @@ extern float* g_prefill_dbg;
 
 // Two query tiles per CTA, one thread per row, correction warps (d <= 128); defined in rk_prefill2c.cu.
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
-                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, int B, cudaStream_t st);
+                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st);
 extern int g_prefill_perturb;   // test hook: PrefillParams::perturb of the next launches
 
 }  // namespace rk
