@@ -59,7 +59,7 @@ static PrefillWs prefill_ws(const rk_prefill_args& a) {
   w.k_sf = off; off = align_up(off + (size_t)a.B * a.H_kv * nkt * dch * 512, 1024);
   w.v_sf = off; off = align_up(off + (size_t)a.B * a.H_kv * nkt * dch * 512, 1024);
   w.v_codes = off;
-  if (a.v_scale_axis == RK_V_SCALES_ALONG_D) off = align_up(off + (size_t)a.B * a.H_kv * a.S_kv * a.d, 1024);
+  if (a.v_scale_axis == RK_V_SCALES_ALONG_D && a.kv_fmt < RK_FMT_E2M3) off = align_up(off + (size_t)a.B * a.H_kv * a.S_kv * a.d, 1024);
   // 6-bit and 4-bit operands: densely packed copies (Q, K along d; V transposed, along the keys), rows padded to
   // 128 codes; sized for 6 bits, which also holds 4
   const size_t dp = dch * 128, skp = nkt * 128;
@@ -192,7 +192,7 @@ int rk_mx_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, i
   if (batch < 0 || S < 0 || d <= 0 || d % 32 != 0) return RK_ERR_BAD_SHAPE;
   if (fmt < 0 || fmt > RK_FMT_E2M1) return RK_ERR_BAD_FORMAT;
   if (!aligned(codes, 4) || !aligned(out_codes, 4) || !aligned(out_scales, 4)) return RK_ERR_MISALIGNED;
-  return launch_rebase_v(codes, scales, batch, S, d, fmt, out_codes, out_scales, false, (cudaStream_t)stream);
+  return launch_rebase_v(codes, scales, batch, S, d, fmt, out_codes, out_scales, false, (cudaStream_t)stream, RetileJobs{});
 }
 
 static size_t packed_len(int64_t n, int fmt) { return (size_t)((n + 127) / 128 * 128) * fmt_bits(fmt) / 8; }
@@ -207,7 +207,10 @@ int rk_mx_pack_rows(const uint8_t* codes, int64_t rows, int64_t d, int fmt, uint
   if (rows < 0 || d <= 0 || d % 16 != 0) return RK_ERR_BAD_SHAPE;
   if (fmt < RK_FMT_E2M3 || fmt > RK_FMT_E2M1) return RK_ERR_BAD_FORMAT;
   if (!aligned(codes, 16) || !aligned(out, 16)) return RK_ERR_MISALIGNED;
-  return launch_pack_rows(codes, rows, d, fmt_bits(fmt), out, (cudaStream_t)stream);
+  PackJobs one = {};
+  one.n = 1;
+  one.job[0] = PackJob{codes, out, rows, fmt_bits(fmt)};
+  return launch_pack_rows(one, d, (cudaStream_t)stream, RetileJobs{});
 }
 
 size_t rk_mx_packed_vt_bytes(int64_t batch, int64_t S, int64_t d, int fmt) {
@@ -220,7 +223,7 @@ int rk_mx_pack_vt(const uint8_t* v_codes, int64_t batch, int64_t S, int64_t d, i
   if (batch < 0 || S <= 0 || d <= 0 || d % 16 != 0) return RK_ERR_BAD_SHAPE;
   if (fmt < RK_FMT_E2M3 || fmt > RK_FMT_E2M1) return RK_ERR_BAD_FORMAT;
   if (!aligned(v_codes, 16) || !aligned(out, 16)) return RK_ERR_MISALIGNED;
-  return launch_pack_transpose(v_codes, batch, S, d, fmt_bits(fmt), out, (cudaStream_t)stream);
+  return launch_pack_v(v_codes, nullptr, batch, S, d, fmt, out, nullptr, (cudaStream_t)stream);
 }
 
 int rk_attn_prefill_block_n(const rk_prefill_args* a) { (void)a; return 128; }
@@ -241,60 +244,46 @@ int rk_attn_prefill(const rk_prefill_args* a, void* stream) {
   uint8_t* ws = reinterpret_cast<uint8_t*>(a->workspace);
   const int64_t bhq = (int64_t)a->B * a->H, bhkv = (int64_t)a->B * a->H_kv;
 
-  // Q / K scales -> scale-factor atoms (or the caller's atoms as they lie)
-  const uint8_t* q_sf = ws + w.q_sf;
-  const uint8_t* k_sf = ws + w.k_sf;
-  const uint8_t* v_sf = ws + w.v_sf;
-  // the usual call (row-major Q and K scales, V scaled along d): the V re-blocking launch re-tiles the Q and K scales
-  // on the side, two launches in all instead of four
-  const bool fused_retile = a->q_scale_layout == RK_SCALES_ROWMAJOR && a->k_scale_layout == RK_SCALES_ROWMAJOR &&
-                            a->v_scale_axis == RK_V_SCALES_ALONG_D;
-  if (!fused_retile) {
-    if (a->q_scale_layout == RK_SCALES_SF_ATOMS) {
-      if (!aligned(a->q_scale, 16)) return RK_ERR_MISALIGNED;
-      q_sf = a->q_scale;
-    } else if ((rc = (a->q_scale_layout == RK_SCALES_GROUPMAJOR ? launch_retile_groupscales : launch_retile_rowscales)(
-                    a->q_scale, bhq, a->S_q, a->d, ws + w.q_sf, st)) != RK_OK) {
-      return rc;
-    }
-    if (a->k_scale_layout == RK_SCALES_SF_ATOMS) {
-      if (!aligned(a->k_scale, 16)) return RK_ERR_MISALIGNED;
-      k_sf = a->k_scale;
-    } else if ((rc = (a->k_scale_layout == RK_SCALES_GROUPMAJOR ? launch_retile_groupscales : launch_retile_rowscales)(
-                    a->k_scale, bhkv, a->S_kv, a->d, ws + w.k_sf, st)) != RK_OK) {
-      return rc;
-    }
-  }
-  const uint8_t* v_codes = a->v;
-  if (a->v_scale_axis == RK_V_SCALES_ALONG_D) {
-    if (a->S_kv % 128 != 0 || a->d % 128 != 0) {
-      // atoms of ragged tiles keep bytes the re-blocking pass never writes: make them 2^0
-      cudaError_t e = cudaMemsetAsync(ws + w.v_sf, 0x7F, w.v_codes - w.v_sf, st);
-      if (e != cudaSuccess) return (int)e;
-    }
-    if ((rc = launch_rebase_v(a->v, a->v_scale, bhkv, a->S_kv, a->d, a->kv_fmt, ws + w.v_codes, ws + w.v_sf, true, st,
-                              fused_retile ? a->q_scale : nullptr, bhq, a->S_q, ws + w.q_sf, fused_retile ? a->k_scale : nullptr,
-                              ws + w.k_sf)) != RK_OK)
-      return rc;
-    v_codes = ws + w.v_codes;
-  } else if (a->v_scale_layout == RK_SCALES_SF_ATOMS) {
-    if (!aligned(a->v_scale, 16)) return RK_ERR_MISALIGNED;
-    v_sf = a->v_scale;
-  } else {
-    if ((rc = launch_retile_keyscales(a->v_scale, bhkv, a->S_kv, a->d, ws + w.v_sf, st)) != RK_OK) return rc;
-  }
-  const uint8_t* q_codes = a->q;
-  const uint8_t* k_codes = a->k;
+  // Block scales -> scale-factor atoms, or the caller's atoms as they lie.  The re-tiling rides along with the first
+  // preparation kernel the call needs; it is a launch of its own only where there is no other.
+  RetileJobs jobs = {};
+  auto atoms_of = [&](const uint8_t* scale, int layout, int kind, int64_t batch, int64_t S, size_t ws_off, const uint8_t*& sf) {
+    if (layout == RK_SCALES_SF_ATOMS) { sf = scale; return aligned(scale, 16); }
+    jobs.job[jobs.n++] = RetileJob{scale, ws + ws_off, batch, S, a->d, kind};
+    sf = ws + ws_off;
+    return true;
+  };
+  const uint8_t *q_sf, *k_sf, *v_sf = ws + w.v_sf;
+  const bool along_d = a->v_scale_axis == RK_V_SCALES_ALONG_D;
+  if (!atoms_of(a->q_scale, a->q_scale_layout, a->q_scale_layout == RK_SCALES_GROUPMAJOR ? 1 : 0, bhq, a->S_q, w.q_sf, q_sf) ||
+      !atoms_of(a->k_scale, a->k_scale_layout, a->k_scale_layout == RK_SCALES_GROUPMAJOR ? 1 : 0, bhkv, a->S_kv, w.k_sf, k_sf) ||
+      (!along_d && !atoms_of(a->v_scale, a->v_scale_layout, 2, bhkv, a->S_kv, w.v_sf, v_sf)))
+    return RK_ERR_MISALIGNED;
+  const uint8_t *q_codes = a->q, *k_codes = a->k, *v_codes = a->v;
+  // 6-bit and 4-bit codes, one per byte: densely packed copies for the tensor core's operand loads
+  PackJobs packs = {};
   if (a->q_fmt >= RK_FMT_E2M3 && !a->q_packed) {
-    if ((rc = launch_pack_rows(a->q, bhq * a->S_q, a->d, fmt_bits(a->q_fmt), ws + w.q6, st)) != RK_OK) return rc;
+    packs.job[packs.n++] = PackJob{a->q, ws + w.q6, bhq * a->S_q, fmt_bits(a->q_fmt)};
     q_codes = ws + w.q6;
   }
-  if (a->kv_fmt >= RK_FMT_E2M3 && !a->kv_packed) {
-    if ((rc = launch_pack_rows(a->k, bhkv * a->S_kv, a->d, fmt_bits(a->kv_fmt), ws + w.k6, st)) != RK_OK) return rc;
+  const bool pack_v = a->kv_fmt >= RK_FMT_E2M3 && !a->kv_packed;
+  if (pack_v) {
+    packs.job[packs.n++] = PackJob{a->k, ws + w.k6, bhkv * a->S_kv, fmt_bits(a->kv_fmt)};
     k_codes = ws + w.k6;
-    if ((rc = launch_pack_transpose(v_codes, bhkv, a->S_kv, a->d, fmt_bits(a->kv_fmt), ws + w.v6t, st)) != RK_OK) return rc;
-    v_codes = ws + w.v6t;
   }
+  if (packs.n > 0) {
+    if ((rc = launch_pack_rows(packs, a->d, st, jobs)) != RK_OK) return rc;
+    jobs.n = 0;
+  }
+  if (pack_v) {
+    if ((rc = launch_pack_v(a->v, along_d ? a->v_scale : nullptr, bhkv, a->S_kv, a->d, a->kv_fmt, ws + w.v6t, ws + w.v_sf, st)) != RK_OK) return rc;
+    v_codes = ws + w.v6t;
+  } else if (along_d) {
+    if ((rc = launch_rebase_v(a->v, a->v_scale, bhkv, a->S_kv, a->d, a->kv_fmt, ws + w.v_codes, ws + w.v_sf, true, st, jobs)) != RK_OK) return rc;
+    jobs.n = 0;
+    v_codes = ws + w.v_codes;
+  }
+  if (jobs.n > 0 && (rc = launch_retile_scales(jobs, st)) != RK_OK) return rc;
   return launch_prefill(*a, q_codes, k_codes, v_codes, q_sf, k_sf, v_sf, st);
 }
 

@@ -15,13 +15,20 @@ int* device_status_word();     // per-device int inside the library image, zero 
 int launch_quantize_rows_bf16(const void* x, int64_t rows, int64_t cols, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st);
 int launch_quantize_rows(const float* x, int64_t rows, int64_t cols, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st);
 int launch_quantize_keys(const float* x, int64_t batch, int64_t rows, int64_t cols, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st);
+// Block scales to re-tile into scale-factor atoms beside other preparation work: up to Q's, K's and V's (kind: where they lie,
+// see retile_scales_body).
+struct RetileJob { const uint8_t* in; uint8_t* out; int64_t batch, S, d; int kind; };
+struct RetileJobs { int n; RetileJob job[3]; };
 int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt,
-                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const uint8_t* q_scales = nullptr,
-                    int64_t bhq = 0, int64_t S_q = 0, uint8_t* q_atoms = nullptr, const uint8_t* k_scales = nullptr,
-                    uint8_t* k_atoms = nullptr);
-int launch_retile_rowscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st);
-int launch_pack_rows(const uint8_t* in, int64_t rows, int64_t d, int bits, uint8_t* out, cudaStream_t st);
-int launch_pack_transpose(const uint8_t* in, int64_t batch, int64_t S, int64_t d, int bits, uint8_t* out, cudaStream_t st);
+                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const RetileJobs& jobs);
+int launch_retile_scales(const RetileJobs& jobs, cudaStream_t st);
+struct PackJob { const uint8_t* in; uint8_t* out; int64_t rows; int bits; };     // byte codes [rows][d] -> dense rows
+struct PackJobs { int n; PackJob job[2]; };
+int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, const RetileJobs& jobs);
+// V [batch][S][d], one code per byte -> dense transposed [batch][d][Sp * bits / 8].  scales != nullptr: V is scaled along d and is
+// re-blocked along the keys on the way, the new scales going to `atoms`.
+int launch_pack_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt, uint8_t* out,
+                  uint8_t* atoms, cudaStream_t st);
 int launch_verify_encoder(int fmt, unsigned long long* mismatches, uint32_t* first_bad, cudaStream_t st);
 int launch_quantize_rows_ex(const void* x, bool bf16, int64_t batch, int64_t S, int64_t d, int fmt, uint8_t* codes,
                             uint8_t* scales, int layout, cudaStream_t st);
@@ -31,13 +38,11 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st);
 int launch_mx_gemm_hw(const uint8_t* A, const uint8_t* B, const uint8_t* SA, const uint8_t* SB, int M, int N, int K,
                       uint16_t* C, cudaStream_t st);
-int launch_retile_groupscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st);
 int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads, int nblk, int Bk, int d, uint8_t* k,
                             uint8_t* ks, cudaStream_t st);
-int launch_retile_keyscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st);
 
-// q/k/v_codes: byte codes as the caller gave them, or -- for 6-bit formats -- the packed copies made by
-// launch_pack_rows (Q, K) and launch_pack_transpose (V, stored [d][keys]).
+// q/k/v_codes: byte codes as the caller gave them, or -- for 6- and 4-bit formats -- the packed copies made by
+// launch_pack_rows (Q, K) and launch_pack_v (V, stored [d][keys]).
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st);
 

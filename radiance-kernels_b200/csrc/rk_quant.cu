@@ -697,12 +697,17 @@ template <int FMT> __device__ __noinline__ uint32_t rb_rare_recode(uint32_t cw, 
   return out;
 }
 
-// scales along d, row-major [batch][S][d/32]  ->  atoms [batch][ntile][dch][512]
-// (rows beyond S and blocks beyond d/32 get code 0x7F = 2^0); one thread per (atom, row) writes 4 bytes.
-RK_DEVINL void retile_rowscales_body(const uint8_t* __restrict__ in, int64_t batch, int64_t S, int64_t d,
-                                     uint8_t* __restrict__ out, int64_t tid, int64_t nthreads) {
-  const int64_t nbd = d / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
-  const int64_t total = batch * ntile * dch * 128;
+// Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one thread per (atom, row or column)
+// writes 4 bytes; rows, columns and blocks past the edge get code 0x7F = 2^0.
+//   kRows   along d, row-major [batch][S][d/32]
+//   kGroups along d, group-major [batch][d/32][S] (the reference's QK_A_scales_row[FA_GK][FA_SQ] per head,
+//           kernels/flash_attention_mx/gen_data.py:82-83)
+//   kKeys   along keys, row-major [batch][ceil(S/32)][d]
+enum RetileKind { kRows = 0, kGroups = 1, kKeys = 2 };
+RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t tid, int64_t nthreads) {
+  const int64_t S = job.S, d = job.d;
+  const int64_t nbd = d / 32, nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
+  const int64_t total = job.batch * ntile * dch * 128;
   for (int64_t t = tid; t < total; t += nthreads) {
     const int r = (int)(t % 128);
     const int64_t atom = t / 128;
@@ -716,20 +721,56 @@ RK_DEVINL void retile_rowscales_body(const uint8_t* __restrict__ in, int64_t bat
     } else {
       ch = atom % dch; tile = (atom / dch) % ntile; bt = atom / (dch * ntile);
     }
-    const int64_t row = tile * 128 + r;
-    uint32_t w = 0;
+    uint32_t w = 0x7F7F7F7Fu;
+    if (job.kind == kKeys) {
+      const int64_t col = ch * 128 + r;
+      if (col < d) {
+        w = 0;
 #pragma unroll
-    for (int kb = 0; kb < 4; kb++) {
-      const int64_t blk = ch * 4 + kb;
-      const uint32_t sc = (row < S && blk < nbd) ? in[(bt * S + row) * nbd + blk] : 0x7Fu;
-      w |= sc << (8 * kb);
+        for (int k = 0; k < 4; k++) w |= (tile * 4 + k < nkb ? (uint32_t)job.in[(bt * nkb + tile * 4 + k) * d + col] : 0x7Fu) << (8 * k);
+      }
+    } else {
+      const int64_t row = tile * 128 + r;
+      if (row < S) {
+        if (job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0) {
+          w = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
+        } else {
+          w = 0;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const int64_t blk = ch * 4 + k;
+            w |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
+          }
+        }
+      }
     }
-    *reinterpret_cast<uint32_t*>(out + atom * 512 + sf_atom_offset(r, 0)) = w;
+    *reinterpret_cast<uint32_t*>(job.out + atom * 512 + sf_atom_offset(r, 0)) = w;
   }
 }
-// Two row-major scale tensors (Q's and K's) that the re-blocking launch re-tiles on the side, so that the usual
-// prefill call is two launches (this one and the attention kernel) instead of four; in == nullptr: nothing to do.
-struct RetileJobs { const uint8_t* in[2]; uint8_t* out[2]; int64_t batch[2], S[2], d[2]; };
+// The jobs of a prefill call ride along with whichever preparation kernel it needs anyway (a launch costs more than they do).
+RK_DEVINL void retile_jobs(const RetileJobs& jobs) {
+#pragma unroll 1
+  for (int i = 0; i < jobs.n; ++i)
+    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+__global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs jobs) {
+  grid_dependency_wait();
+  grid_dependents_launch();
+  retile_jobs(jobs);
+}
+
+// Bytes of key-scale atoms that belong to no block (columns past d, key blocks past S): 2^0.  The re-blocking kernel writes the
+// others, bytes of its own.
+RK_DEVINL void fill_ragged_atoms(uint8_t* __restrict__ atoms, int64_t batch, int64_t S, int64_t d) {
+  const int64_t nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128, total = batch * ntile * dch * 128;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int n = (int)(t & 127);
+    const int64_t atom = t >> 7, col = (atom % dch) * 128 + n, kb0 = (atom / dch) % ntile * 4;
+    uint8_t* w = atoms + atom * 512 + sf_atom_offset(n, 0);
+    for (int k = 0; k < 4; ++k)
+      if (col >= d || kb0 + k >= nkb) w[k] = 0x7Fu;
+  }
+}
 
 // Four lanes share one unit = 16 adjacent columns x one 32-key block: lane "rg" holds rows 8 rg .. 8 rg + 7 as
 // eight 16-byte words in registers between the two passes (all loads of a thread in flight together), the
@@ -741,11 +782,10 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
                                                           int64_t batch, int64_t S, int64_t d,
                                                           uint8_t* __restrict__ out_codes, uint8_t* __restrict__ out_scales,
                                                           const RetileJobs jobs) {
-#pragma unroll
-  for (int jb = 0; jb < 2; ++jb)
-    if (jobs.in[jb])
-      retile_rowscales_body(jobs.in[jb], jobs.batch[jb], jobs.S[jb], jobs.d[jb], jobs.out[jb],
-                            (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+  grid_dependency_wait();
+  grid_dependents_launch();
+  retile_jobs(jobs);
+  if (TILED && (S % 128 != 0 || d % 128 != 0)) fill_ragged_atoms(out_scales, batch, S, d);
   const int64_t c16n = d / 16, nkb = (S + 31) / 32, nbd = d / 32;
   const int64_t units = batch * nkb * c16n;
   const int64_t ntile = (S + 127) / 128, dch = (d + 127) / 128;   // atom grid of the TILED layout
@@ -777,21 +817,22 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
     using R = RebaseT<FMT>;
     uint32_t bad = 0u;
     {
-      // rows past a ragged end read as zero codes under a mid-range scale: they change nothing
+      // rows past a ragged end read as the smallest normal codes under the smallest scale the integer path takes: no real row
+      // is below them, so they change nothing (as zero codes they would take the slow path for rare rows)
       uint4 cw[8];
       uint32_t s8[8];
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const int j = rg * 8 + i;
         const bool in = j < n;
-        cw[i] = in ? __ldg(reinterpret_cast<const uint4*>(cb + (int64_t)j * d)) : make_uint4(0u, 0u, 0u, 0u);
-        s8[i] = in ? (uint32_t)__ldg(sb + (int64_t)j * nbd) : 127u;
+        cw[i] = in ? __ldg(reinterpret_cast<const uint4*>(cb + (int64_t)j * d)) : make_uint4(R::LOW4, R::LOW4, R::LOW4, R::LOW4);
+        s8[i] = in ? (uint32_t)__ldg(sb + (int64_t)j * nbd) : 0u;
       }
       // pass 1: largest L per column; word x of a row holds columns 4x .. 4x+3, lanes (0, 2) in lo[x], (1, 3) in hi[x]
       uint32_t lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
       for (int i = 0; i < 8; i++) {
-        bad |= (s8[i] - R::S_LO > 240u - R::S_LO) ? 1u : 0u;
+        bad |= (s8[i] - R::S_LO > 240u - R::S_LO && rg * 8 + i < n) ? 1u : 0u;
         s8[i] *= (uint32_t)R::ONE * 0x00010001u;
         const uint32_t wv[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
         // one test per row: does any of its 16 codes have a zero exponent field (zero or subnormal)?
@@ -822,7 +863,7 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
       bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, 16);
       if (bad == 0u) {
         // s' = L_max / 8 - 15 (+1 when the mantissa bits are 7) in both 16-bit lanes at once; all-zero columns
-        // (L_max = 0) get scale code 0
+        // (L_max = 0, or that of a row past the end) get scale code 0
         uint32_t sub_lo[4], sub_hi[4];
 #pragma unroll
         for (int x = 0; x < 4; x++) {
@@ -832,8 +873,8 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
             constexpr uint32_t M2 = (uint32_t)(R::ONE - 1) * 0x00010001u, Q2 = (0xFFFFu >> R::MB) * 0x00010001u;
             uint32_t sn = (v[h] >> R::MB) & Q2;
             if (R::PLUS1) sn += (((v[h] & M2) + 0x00010001u) >> R::MB) & 0x00010001u;
-            if ((v[h] & 0xFFFFu) == 0u) sn = (sn & 0xFFFF0000u) | (uint32_t)R::OFF;          // an all-zero column: scale code 0
-            if ((v[h] >> 16) == 0u) sn = (sn & 0x0000FFFFu) | ((uint32_t)R::OFF << 16);
+            if ((v[h] & 0xFFFFu) <= (uint32_t)R::ONE) sn = (sn & 0xFFFF0000u) | (uint32_t)R::OFF;   // nothing but zeros: scale code 0
+            if ((v[h] >> 16) <= (uint32_t)R::ONE) sn = (sn & 0x0000FFFFu) | ((uint32_t)R::OFF << 16);
             v[h] = sn - (uint32_t)R::OFF * 0x00010001u;
           }
           sub_lo[x] = v[0] << R::MB;
@@ -845,6 +886,7 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
         // pass 2: lanes carry tt + 0x4000 (tt = L - 8 s') so that they stay non-negative
 #pragma unroll
         for (int i = 0; i < 8; i++) {
+          if (rg * 8 + i >= n) break;
           const uint32_t wv[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
           uint32_t ov[4];
           // lanes that leave the normal range (tt < 8) set bit 15 of their half; zero / subnormal inputs set bit 7
@@ -861,8 +903,7 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
             for (int x = 0; x < 4; x++)
               if (rare[x] != 0u) ov[x] = rb_rare_recode<FMT>(wv[x], (int)((s8[i] & 0xFFFFu) >> R::MB), sub_lo[x], sub_hi[x]);
           }
-          const int j = rg * 8 + i;
-          if (j < n) *reinterpret_cast<uint4*>(ob + (int64_t)j * d) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
+          *reinterpret_cast<uint4*>(ob + (int64_t)(rg * 8 + i) * d) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
         }
       }
     }
@@ -881,52 +922,6 @@ __global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restr
     } else {
       *reinterpret_cast<uint32_t*>(out_scales + (bt * nkb + kb) * d + col0) = sc[0] | (sc[1] << 8) | (sc[2] << 16) | (sc[3] << 24);
     }
-  }
-}
-
-// scales along keys, row-major [batch][ceil(S/32)][d]  ->  atoms [batch][ntile][dch][512]
-__global__ void retile_keyscales_kernel(const uint8_t* __restrict__ in, int64_t batch, int64_t S, int64_t d,
-                                        uint8_t* __restrict__ out) {
-  const int64_t nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
-  const int64_t total = batch * ntile * dch * 128;   // one thread per (atom, column n): writes 4 bytes
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int n = (int)(t % 128);
-    const int64_t atom = t / 128, nc = atom % dch, kt = (atom / dch) % ntile, bt = atom / (dch * ntile);
-    const int64_t col = nc * 128 + n;
-    uint32_t w = 0;
-#pragma unroll
-    for (int kbi = 0; kbi < 4; kbi++) {
-      const int64_t kb = kt * 4 + kbi;
-      const uint32_t s = (kb < nkb && col < d) ? in[(bt * nkb + kb) * d + col] : 0x7Fu;
-      w |= s << (8 * kbi);
-    }
-    *reinterpret_cast<uint32_t*>(out + atom * 512 + sf_atom_offset(n, 0)) = w;
-  }
-}
-
-__global__ void retile_rowscales_kernel(const uint8_t* __restrict__ in, int64_t batch, int64_t S, int64_t d,
-                                        uint8_t* __restrict__ out) {
-  retile_rowscales_body(in, batch, S, d, out, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
-}
-
-// scales along d, group-major [batch][d/32][S] (the reference's QK_A_scales_row[FA_GK][FA_SQ] per head,
-// kernels/flash_attention_mx/gen_data.py:82-83)  ->  atoms [batch][ntile][dch][512]
-__global__ void retile_groupscales_kernel(const uint8_t* __restrict__ in, int64_t batch, int64_t S, int64_t d,
-                                          uint8_t* __restrict__ out) {
-  const int64_t nbd = d / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
-  const int64_t total = batch * ntile * dch * 128;   // one thread per (atom, row): writes 4 bytes; a warp reads 32 adjacent rows
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(t % 128);
-    const int64_t atom = t / 128, ch = atom % dch, tile = (atom / dch) % ntile, bt = atom / (dch * ntile);
-    const int64_t row = tile * 128 + r;
-    uint32_t w = 0;
-#pragma unroll
-    for (int kb = 0; kb < 4; kb++) {
-      const int64_t blk = ch * 4 + kb;
-      const uint32_t sc = (row < S && blk < nbd) ? in[(bt * nbd + blk) * S + row] : 0x7Fu;
-      w |= sc << (8 * kb);
-    }
-    *reinterpret_cast<uint32_t*>(out + atom * 512 + sf_atom_offset(r, 0)) = w;
   }
 }
 
@@ -961,82 +956,224 @@ __global__ void __launch_bounds__(256) import_kt_blocks_kernel(const uint8_t* __
   }
 }
 
-// 16 codes of BITS bits each -> BITS/2 32-bit words, code i in bits [BITS*i, BITS*i + BITS) (the order TMA's
-// 16U6_ALIGN16B / 16U4_ALIGN16B types expand from)
-template <int BITS> RK_DEVINL void pack16(const uint32_t* c, uint32_t* w) {
+// ---- dense 6- and 4-bit operands -------------------------------------------------------------------------------------
+// four byte codes -> BITS * 4 bits, code i at bits [BITS * i, BITS * i + BITS)
+template <int BITS> RK_DEVINL uint32_t pack4(uint32_t w) {
   if (BITS == 4) {
-    uint32_t a = 0, b = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { a |= (c[i] & 0xFu) << (4 * i); b |= (c[8 + i] & 0xFu) << (4 * i); }
-    w[0] = a; w[1] = b;
-    return;
+    w = (w & 0x000F000Fu) | ((w >> 4) & 0x00F000F0u);
+    return (w & 0xFFu) | ((w >> 8) & 0xFF00u);
   }
-  uint64_t lo = 0, hi = 0;     // 96 bits
+  w = (w & 0x003F003Fu) | ((w >> 2) & 0x0FC00FC0u);
+  return (w & 0xFFFu) | ((w >> 4) & 0xFFF000u);
+}
+// groups of four packed codes -> 32-bit words in order (the order TMA's 16U6_ALIGN16B / 16U4_ALIGN16B types expand from):
+// N groups of 24 bits -> 3 N / 4 words, or of 16 bits -> N / 2 words
+template <int BITS, int N> RK_DEVINL void join_groups(const uint32_t (&c)[N], uint32_t (&w)[N * BITS / 8]) {
+  if (BITS == 4) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const uint64_t v = c[i] & 0x3Fu;
-    const int bit = 6 * i;
-    if (bit < 64) { lo |= v << bit; if (bit + 6 > 64) hi |= v >> (64 - bit); }
-    else hi |= v << (bit - 64);
+    for (int i = 0; i < N / 2; ++i) w[i] = c[2 * i] | (c[2 * i + 1] << 16);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+      w[3 * i] = c[4 * i] | (c[4 * i + 1] << 24);
+      w[3 * i + 1] = (c[4 * i + 1] >> 8) | (c[4 * i + 2] << 16);
+      w[3 * i + 2] = (c[4 * i + 2] >> 16) | (c[4 * i + 3] << 8);
+    }
   }
-  w[0] = (uint32_t)lo; w[1] = (uint32_t)(lo >> 32); w[2] = (uint32_t)hi;
 }
 
 // byte codes [rows][d] -> packed [rows][dp * BITS/8 bytes], dp = d rounded up to 128, padding codes 0
-template <int BITS>
-__global__ void pack_rows_kernel(const uint8_t* __restrict__ in, int64_t rows, int64_t d, int64_t dp, uint8_t* __restrict__ out) {
-  const int64_t groups = dp / 16, total = rows * groups;
+template <int BITS> RK_DEVINL void pack_rows_body(const PackJob& job, int64_t d, int64_t dp) {
+  const int64_t groups = dp / 16, total = job.rows * groups;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = t / groups, gidx = t % groups;
-    uint32_t c[16], w[3];
-    if (gidx * 16 < d) {
-      const uint4 v = *reinterpret_cast<const uint4*>(in + r * d + gidx * 16);
-      const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int i = 0; i < 16; ++i) c[i] = (ww[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+    int64_t r, g;
+    if (total < (int64_t)1 << 31) { const uint32_t q = (uint32_t)t / (uint32_t)groups; r = q; g = (uint32_t)t - q * (uint32_t)groups; }
+    else { r = t / groups; g = t % groups; }
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (g * 16 < d) v = __ldcs(reinterpret_cast<const uint4*>(job.in + r * d + g * 16));
+    const uint32_t c[4] = {pack4<BITS>(v.x), pack4<BITS>(v.y), pack4<BITS>(v.z), pack4<BITS>(v.w)};
+    uint32_t w[BITS / 2];
+    join_groups<BITS, 4>(c, w);
+    uint8_t* o = job.out + r * (dp * BITS / 8) + g * (2 * BITS);
+    if (BITS == 4) {
+      *reinterpret_cast<uint2*>(o) = make_uint2(w[0], w[1]);
     } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) c[i] = 0;
+      for (int i = 0; i < BITS / 2; ++i) reinterpret_cast<uint32_t*>(o)[i] = w[i];
     }
-    pack16<BITS>(c, w);
-    uint32_t* o = reinterpret_cast<uint32_t*>(out + r * (dp * BITS / 8) + gidx * (2 * BITS));
-    o[0] = w[0]; o[1] = w[1];
-    if (BITS == 6) o[2] = w[2];
+  }
+}
+__global__ void __launch_bounds__(256) pack_rows_kernel(const PackJobs packs, int64_t d, int64_t dp, const RetileJobs jobs) {
+  grid_dependency_wait();
+  grid_dependents_launch();
+  retile_jobs(jobs);
+#pragma unroll 1
+  for (int i = 0; i < packs.n; ++i) {
+    if (packs.job[i].bits == 4) pack_rows_body<4>(packs.job[i], d, dp);
+    else pack_rows_body<6>(packs.job[i], d, dp);
   }
 }
 
-// byte codes [batch][S][d] -> packed transposed [batch][d][Sp * BITS/8 bytes], Sp = S rounded up to 128.
-// One CTA = one tile of 128 keys x 128 columns through shared memory: coalesced 16-byte reads along d, then each
-// thread packs 16 keys of one column and the 8 threads of a column write 96 (64) contiguous bytes.
-template <int BITS>
-__global__ void __launch_bounds__(256) pack_transpose_kernel(const uint8_t* __restrict__ in, int64_t batch, int64_t S, int64_t d,
-                                                              int64_t Sp, uint8_t* __restrict__ out) {
-  __shared__ uint8_t tile[128][128 + 4];                       // [key][col], rows padded by one word against bank conflicts
-  const int64_t ktiles = Sp / 128, ctiles = (d + 127) / 128;
-  const int64_t ntiles = batch * ktiles * ctiles;
-  for (int64_t tix = blockIdx.x; tix < ntiles; tix += gridDim.x) {
-    const int64_t ct = tix % ctiles, kt = (tix / ctiles) % ktiles, bt = tix / (ctiles * ktiles);
-    const int64_t key0 = kt * 128, col0 = ct * 128;
-    __syncthreads();                                           // the previous tile has been read out
-    for (int i = threadIdx.x; i < 128 * 8; i += 256) {         // 128 rows x 8 chunks of 16 columns
-      const int r = i >> 3, ch = i & 7;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (key0 + r < S && col0 + ch * 16 < d) v = *reinterpret_cast<const uint4*>(in + (bt * S + key0 + r) * d + col0 + ch * 16);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&tile[r][ch * 16]);
-      dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 128 * 8; i += 256) {         // 128 columns x 8 groups of 16 keys
-      const int col = i >> 3, gi = i & 7;
-      if (col0 + col >= d) continue;
-      uint32_t c[16], w[3];
+// V for the tensor core in a 6- or 4-bit format: byte codes [batch][S][d] -> packed transposed [batch][d][Sp * BITS/8], Sp = S
+// rounded up to 128 (sub-byte operands may not be MN-major).  REBASE: V comes scaled along d and is re-blocked along the keys
+// on the way (decode exactly, block rule down each column, encode: the same result as rebase_v_kernel), the new block scales
+// going to the scale-factor atoms.
+// One CTA = 128 keys x 128 columns, a warp = one 32-key block, a thread = 4 columns x 32 keys in registers, all its loads in
+// flight.  In these formats zero and subnormal codes are common, which the integer form of the re-blocking kernel pays for
+// row by row; here a pair of codes goes through the hardware converter to f16, times the row's scale relative to the block's
+// largest (exact: every value is a multiple of 2^-4 or coarser, f16 reaches down to 2^-24, and blocks whose scales span more
+// than 2^14 take the slow form), the column maxima are packed f16 operations, and pairs of keys of one column go back through
+// the converter in the order in which they are packed.  The packed words meet in shared memory and leave in 16-byte stores.
+// 33.5 M codes E3M2: re-blocking 138 us and transposition 27 us as kernels of their own, PACKV_NOW us here.
+template <int FMT> RK_DEVINL uint32_t decode_f16x2(uint32_t codes) {            // two codes in the low bytes -> packed f16
+  uint32_t r;
+  if (FMT == 3) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e3m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  else asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e2m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  return r;
+}
+RK_DEVINL uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+RK_DEVINL float f16_lo(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, l;\n\t}" : "=f"(r) : "r"(v)); return r; }
+RK_DEVINL float f16_hi(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "r"(v)); return r; }
+// codes of four consecutive keys, packed
+template <int FMT> RK_DEVINL uint32_t encode_pack4(float a, float b, float c, float d) {
+  uint32_t r;
+  if (FMT == 4) {
+    asm("{\n\t.reg .b8 l, h;\n\tcvt.rn.satfinite.e2m1x2.f32 l, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 h, %4, %3;\n\tmov.b32 %0, {l, h, l, h};\n\t}"
+        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
+    return r & 0xFFFFu;
+  }
+  return pack4<6>(hw_encode4<FMT>(a, b, c, d));
+}
+template <int FMT, bool REBASE>
+__global__ void __launch_bounds__(128) pack_v_kernel(const uint8_t* __restrict__ in, const uint8_t* __restrict__ scales, int64_t S, int64_t d,
+                                                     int64_t Sp, uint8_t* __restrict__ out, uint8_t* __restrict__ atoms) {
+  constexpr int BITS = FMT == 4 ? 4 : 6, kWords = BITS, kRow = 4 * kWords, kPitch = kRow + 1;   // words per key block, per column; pitch
+  __shared__ uint32_t buf[128 * kPitch];
+  __shared__ __align__(16) uint32_t fac[4][128];             // [32-column block][key]: packed f16 2^(s - smax)
+  __shared__ int smax_sm[4][4];                                  // [32-column block][key block], -1: the slow form
+  const int lane = threadIdx.x & 31, kb = threadIdx.x >> 5;
+  const int64_t ktiles = Sp / 128, dch = (d + 127) / 128, nbd = d / 32;
+  const int64_t ch = blockIdx.x % dch, kt = blockIdx.x / dch % ktiles, bt = blockIdx.x / (dch * ktiles);
+  const int64_t key0 = kt * 128 + kb * 32, col0 = ch * 128 + lane * 4;
+  grid_dependency_wait();
+  grid_dependents_launch();
+  const int n = (int)max((int64_t)0, min((int64_t)32, S - key0));    // keys of this block that exist
+  const uint8_t* src = in + (bt * S + key0) * d + col0;
+  uint32_t w[32];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) c[k] = tile[gi * 16 + k][col];
-      pack16<BITS>(c, w);
-      uint32_t* o = reinterpret_cast<uint32_t*>(out + (bt * d + col0 + col) * (Sp * BITS / 8) + (kt * 8 + gi) * (2 * BITS));
-      o[0] = w[0]; o[1] = w[1];
-      if (BITS == 6) o[2] = w[2];
+  for (int k = 0; k < 32; ++k) w[k] = (k < n && col0 < d) ? __ldg(reinterpret_cast<const uint32_t*>(src + k * d)) : 0u;
+  uint32_t packed[4][8];                                         // [column][groups of four keys]
+  uint32_t code[4] = {0x7Fu, 0x7Fu, 0x7Fu, 0x7Fu};               // new scale codes; of columns and blocks that do not exist, 2^0
+  if (REBASE) {
+    const uint8_t* sk = scales + (bt * S + key0 + lane) * nbd + ch * 4;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const bool live = lane < n && ch * 4 + b < nbd;
+      const int s = live ? (int)__ldg(sk + b) : -1;
+      const int top = __reduce_max_sync(0xffffffffu, s), low = __reduce_min_sync(0xffffffffu, live ? s : 255);
+      fac[b][kb * 32 + lane] = live ? (uint32_t)max(15 + s - top, 1) * 0x04000400u : 0u;
+      if (lane == 0) smax_sm[b][kb] = (top < 0 || (low >= 20 && top <= 235 && top - low <= 14)) ? max(top, 0) : -1;
     }
+    __syncwarp();
+    const int blk = lane >> 3, smax = smax_sm[blk][kb];
+    if (smax >= 0) {
+      uint32_t x[32], y[32], mx = 0u, my = 0u;                    // columns 0, 1 and 2, 3 of the thread
+#pragma unroll
+      for (int k = 0; k < 32; k += 4) {
+        const uint4 f4 = *reinterpret_cast<const uint4*>(&fac[blk][kb * 32 + k]);
+        const uint32_t f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t c = FMT == 4 ? (w[k + e] & 0x0F0F0F0Fu) << 2 : w[k + e] & 0x3F3F3F3Fu;     // an E2M1 code, shifted, is the E2M3 code of its value
+          x[k + e] = hmul2(decode_f16x2<FMT>(c), f[e]);
+          y[k + e] = hmul2(decode_f16x2<FMT>(c >> 16), f[e]);
+          mx = max_u16x2(mx, x[k + e] & 0x7FFF7FFFu);
+          my = max_u16x2(my, y[k + e] & 0x7FFF7FFFu);
+        }
+      }
+      const float unit = __uint_as_float((uint32_t)smax << 23);                                     // 2^(smax - 127)
+      const float am[4] = {f16_lo(mx) * unit, f16_hi(mx) * unit, f16_lo(my) * unit, f16_hi(my) * unit};
+      float f[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t sc = 0; float p2 = 1.0f;
+        if (am[q] > 0.0f) block_scale<FMT>(am[q], sc, p2);
+        if (n > 0 && col0 < d) code[q] = sc;
+        f[q] = unit * p2;
+      }
+#pragma unroll
+      for (int k = 0; k < 32; k += 4) {
+        packed[0][k / 4] = encode_pack4<FMT>(f16_lo(x[k]) * f[0], f16_lo(x[k + 1]) * f[0], f16_lo(x[k + 2]) * f[0], f16_lo(x[k + 3]) * f[0]);
+        packed[1][k / 4] = encode_pack4<FMT>(f16_hi(x[k]) * f[1], f16_hi(x[k + 1]) * f[1], f16_hi(x[k + 2]) * f[1], f16_hi(x[k + 3]) * f[1]);
+        packed[2][k / 4] = encode_pack4<FMT>(f16_lo(y[k]) * f[2], f16_lo(y[k + 1]) * f[2], f16_lo(y[k + 2]) * f[2], f16_lo(y[k + 3]) * f[2]);
+        packed[3][k / 4] = encode_pack4<FMT>(f16_hi(y[k]) * f[3], f16_hi(y[k + 1]) * f[3], f16_hi(y[k + 2]) * f[3], f16_hi(y[k + 3]) * f[3]);
+      }
+    } else {
+      // block scales far apart or near the ends of the range: through fp32, element by element
+      const uint8_t* sb = scales + (bt * S + key0) * nbd + col0 / 32;
+      float am[4] = {0.f, 0.f, 0.f, 0.f}, p2[4];
+      for (int k = 0; k < n; ++k) {
+        const uint32_t c = *reinterpret_cast<const uint32_t*>(src + k * d), s = sb[k * nbd];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) am[q] = fmaxf(am[q], fabsf(decode_scaled<FMT>((c >> (8 * q)) & 0xFFu, s)));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { code[q] = 0; p2[q] = 1.0f; if (am[q] > 0.0f) block_scale<FMT>(am[q], code[q], p2[q]); }
+#pragma unroll
+      for (int g = 0; g < 8; ++g)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) packed[q][g] = 0u;
+#pragma unroll 1
+      for (int k = 0; k < n; ++k) {
+        const uint32_t c = *reinterpret_cast<const uint32_t*>(src + k * d), s = sb[k * nbd];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t e = encode_rne<FMT>(decode_scaled<FMT>((c >> (8 * q)) & 0xFFu, s) * p2[q]) << (BITS * (k & 3));
+#pragma unroll
+          for (int g = 0; g < 8; ++g) packed[q][g] |= (k >> 2) == g ? e : 0u;
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = lane * 4 + q;
+      atoms[((bt * ktiles + kt) * dch + ch) * 512 + sf_atom_offset(c, kb)] = (uint8_t)code[q];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 32; k += 4) {                               // 4 keys x 4 columns of bytes, transposed
+      const uint32_t a = __byte_perm(w[k], w[k + 1], 0x5140), b = __byte_perm(w[k + 2], w[k + 3], 0x5140);
+      const uint32_t c = __byte_perm(w[k], w[k + 1], 0x7362), e = __byte_perm(w[k + 2], w[k + 3], 0x7362);
+      packed[0][k / 4] = pack4<BITS>(__byte_perm(a, b, 0x5410));
+      packed[1][k / 4] = pack4<BITS>(__byte_perm(a, b, 0x7632));
+      packed[2][k / 4] = pack4<BITS>(__byte_perm(c, e, 0x5410));
+      packed[3][k / 4] = pack4<BITS>(__byte_perm(c, e, 0x7632));
+    }
+  }
+  // word i of column c sits at (i + c / 32) % kRow: with the odd pitch a store of 32 lanes then touches all banks
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t o[kWords];
+    join_groups<BITS, 8>(packed[q], o);
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      int at = kb * kWords + i + (lane >> 3);
+      at -= at >= kRow ? kRow : 0;
+      buf[(lane * 4 + q) * kPitch + at] = o[i];
+    }
+  }
+  __syncthreads();
+  const int cols = (int)min((int64_t)128, d - ch * 128);
+  for (int i = threadIdx.x; i < cols * (kRow / 4); i += 128) {
+    const int c = i / (kRow / 4), chunk = i - c * (kRow / 4);
+    uint32_t v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      int at = chunk * 4 + e + (c >> 5);
+      at -= at >= kRow ? kRow : 0;
+      v[e] = buf[c * kPitch + at];
+    }
+    *reinterpret_cast<uint4*>(out + (bt * d + ch * 128 + c) * (Sp * BITS / 8) + kt * (kRow * 4) + chunk * 16) = make_uint4(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -1093,11 +1230,11 @@ int launch_quantize_keys_atoms(const float* x, int64_t batch, int64_t rows, int6
   return (int)cudaGetLastError();
 }
 
-int launch_retile_groupscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st) {
-  const int64_t total = batch * ((S + 127) / 128) * ((d + 127) / 128) * 128;
-  if (total == 0) return RK_OK;
-  retile_groupscales_kernel<<<grid_for(total, 256, 8), 256, 0, st>>>(in, batch, S, d, out);
-  return (int)cudaGetLastError();
+int launch_retile_scales(const RetileJobs& jobs, cudaStream_t st) {
+  int64_t most = 0;
+  for (int i = 0; i < jobs.n; ++i) most = std::max(most, jobs.job[i].batch * ((jobs.job[i].S + 127) / 128) * ((jobs.job[i].d + 127) / 128) * 128);
+  if (most == 0) return RK_OK;
+  return (int)launch_pdl(retile_scales_kernel, dim3(grid_for(most, 128, 16)), dim3(128), 0, st, jobs);
 }
 
 int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads, int nblk, int Bk, int d, uint8_t* k,
@@ -1174,54 +1311,32 @@ int launch_kv_append(const float* k_new, const float* v_new, int B, int H_kv, in
   return (int)cudaGetLastError();
 }
 
-// q_scales / k_scales (optional, both or neither): row-major E8M0 scales of Q [bhq][S_q][d/32] and K [batch][S][d/32]
-// re-tiled into atoms by the same launch.
 int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt,
-                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const uint8_t* q_scales,
-                    int64_t bhq, int64_t S_q, uint8_t* q_atoms, const uint8_t* k_scales, uint8_t* k_atoms) {
+                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const RetileJobs& jobs) {
   const int64_t total = ((batch * ((S + 31) / 32) * (d / 16) + 7) / 8) * 32;     // 4 lanes per 16-column unit, whole warps
   if (total == 0) return RK_OK;
   const int grid = grid_for(total, 128, 16);      // four CTAs are resident per SM; four waves of them end more evenly than two (-6 %)
-  RetileJobs jobs = {};
-  if (q_scales && k_scales) {
-    jobs.in[0] = q_scales; jobs.out[0] = q_atoms; jobs.batch[0] = bhq; jobs.S[0] = S_q; jobs.d[0] = d;
-    jobs.in[1] = k_scales; jobs.out[1] = k_atoms; jobs.batch[1] = batch; jobs.S[1] = S; jobs.d[1] = d;
-  }
-  if (tiled) { RK_DISPATCH_FMT(fmt, (rebase_v_kernel<F, true><<<grid, 128, 0, st>>>(codes, scales, batch, S, d, out_codes, out_scales, jobs))); }
-  else       { RK_DISPATCH_FMT(fmt, (rebase_v_kernel<F, false><<<grid, 128, 0, st>>>(codes, scales, batch, S, d, out_codes, out_scales, jobs))); }
-  return (int)cudaGetLastError();
+  if (tiled) { RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, true>, dim3(grid), dim3(128), 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs)); }
+  else       { RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, false>, dim3(grid), dim3(128), 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs)); }
+  return RK_OK;
 }
 
-int launch_retile_rowscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st) {
-  const int64_t total = batch * ((S + 127) / 128) * ((d + 127) / 128) * 128;
-  if (total == 0) return RK_OK;
-  retile_rowscales_kernel<<<grid_for(total, 256, 8), 256, 0, st>>>(in, batch, S, d, out);
-  return (int)cudaGetLastError();
+int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, const RetileJobs& jobs) {
+  const int64_t dp = (d + 127) / 128 * 128;
+  int64_t most = 0;
+  for (int i = 0; i < packs.n; ++i) most = std::max(most, packs.job[i].rows * (dp / 16));
+  if (most == 0) return RK_OK;
+  return (int)launch_pdl(pack_rows_kernel, dim3(grid_for(most, 256, 16)), dim3(256), 0, st, packs, d, dp, jobs);
 }
 
-int launch_retile_keyscales(const uint8_t* in, int64_t batch, int64_t S, int64_t d, uint8_t* out, cudaStream_t st) {
-  const int64_t total = batch * ((S + 127) / 128) * ((d + 127) / 128) * 128;
-  if (total == 0) return RK_OK;
-  retile_keyscales_kernel<<<grid_for(total, 256, 8), 256, 0, st>>>(in, batch, S, d, out);
-  return (int)cudaGetLastError();
-}
-
-// bits = 6 (E2M3, E3M2) or 4 (E2M1)
-int launch_pack_rows(const uint8_t* in, int64_t rows, int64_t d, int bits, uint8_t* out, cudaStream_t st) {
-  const int64_t dp = (d + 127) / 128 * 128, total = rows * (dp / 16);
-  if (total == 0) return RK_OK;
-  if (bits == 4) pack_rows_kernel<4><<<grid_for(total, 256, 8), 256, 0, st>>>(in, rows, d, dp, out);
-  else pack_rows_kernel<6><<<grid_for(total, 256, 8), 256, 0, st>>>(in, rows, d, dp, out);
-  return (int)cudaGetLastError();
-}
-
-int launch_pack_transpose(const uint8_t* in, int64_t batch, int64_t S, int64_t d, int bits, uint8_t* out, cudaStream_t st) {
-  const int64_t Sp = (S + 127) / 128 * 128, tiles = batch * (Sp / 128) * ((d + 127) / 128);
-  if (tiles == 0) return RK_OK;
-  const int grid = (int)min(tiles, (int64_t)num_sms() * 8);
-  if (bits == 4) pack_transpose_kernel<4><<<grid, 256, 0, st>>>(in, batch, S, d, Sp, out);
-  else pack_transpose_kernel<6><<<grid, 256, 0, st>>>(in, batch, S, d, Sp, out);
-  return (int)cudaGetLastError();
+int launch_pack_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt, uint8_t* out,
+                  uint8_t* atoms, cudaStream_t st) {
+  const int64_t Sp = (S + 127) / 128 * 128, grid = batch * (Sp / 128) * ((d + 127) / 128);
+  if (grid == 0) return RK_OK;
+  if (grid > 0x7FFFFFFF) return RK_ERR_BAD_SHAPE;
+  auto kern = scales ? (fmt == RK_FMT_E2M3 ? pack_v_kernel<2, true> : fmt == RK_FMT_E3M2 ? pack_v_kernel<3, true> : pack_v_kernel<4, true>)
+                     : (fmt == RK_FMT_E2M1 ? pack_v_kernel<4, false> : pack_v_kernel<2, false>);
+  return (int)launch_pdl(kern, dim3((unsigned)grid), dim3(128), 0, st, codes, scales, S, d, Sp, out, atoms);
 }
 
 // Runs the exhaustive encoder check for one format over all 2^32 fp32 bit patterns.
