@@ -18,13 +18,13 @@ int launch_quantize_keys(const float* x, int64_t batch, int64_t rows, int64_t co
 // Block scales to re-tile into scale-factor atoms beside other preparation work: up to Q's, K's and V's (kind: where they lie,
 // see retile_scales_body).
 struct RetileJob { const uint8_t* in; uint8_t* out; int64_t batch, S, d; int kind; };
-struct RetileJobs { int n; RetileJob job[3]; };
+struct RetileJobs { int n, ctas; RetileJob job[3]; };      // ctas: set by the launch functions
 int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt,
-                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const RetileJobs& jobs);
-int launch_retile_scales(const RetileJobs& jobs, cudaStream_t st);
+                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, RetileJobs jobs);
+int launch_retile_scales(RetileJobs jobs, cudaStream_t st);
 struct PackJob { const uint8_t* in; uint8_t* out; int64_t rows; int bits; };     // byte codes [rows][d] -> dense rows
 struct PackJobs { int n; PackJob job[2]; };
-int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, const RetileJobs& jobs);
+int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, RetileJobs jobs);
 // V [batch][S][d], one code per byte -> dense transposed [batch][d][Sp * bits / 8].  scales != nullptr: V is scaled along d and is
 // re-blocked along the keys on the way, the new scales going to `atoms`.
 int launch_pack_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt, uint8_t* out,

@@ -596,105 +596,18 @@ template <int FMT> RK_DEVINL float decode_scaled(uint32_t c, uint32_t s) {
   return decode_elem<FMT>(c) * e8m0_to_f32(s);
 }
 
-// Generic re-blocking of one (4 columns x up to 32 keys) block through fp32: decode every element exactly,
-// block rule down each column, encode.  Used for formats other than E4M3 and for E4M3 blocks that hold
-// subnormal codes or extreme scale codes.
-template <int FMT>
-__device__ __noinline__ void rebase_block_generic(const uint8_t* cb, const uint8_t* sb, int n, int64_t d, int64_t nbd,
-                                                  uint8_t* ob, uint32_t (&sc)[4]) {
-  float amax[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int j = 0; j < n; j++) {
-    const uint32_t cw = *reinterpret_cast<const uint32_t*>(cb + (int64_t)j * d);
-    const uint32_t sj = sb[(int64_t)j * nbd];
-#pragma unroll
-    for (int q = 0; q < 4; q++) amax[q] = fmaxf(amax[q], fabsf(decode_scaled<FMT>((cw >> (8 * q)) & 0xFFu, sj)));
+// The slow form: a thread's NC columns of a block, element by element through fp32; keys k0 .. k0 + 7 are written.
+template <int FMT, int NC>
+__device__ __noinline__ void rebase_slow(const uint8_t* cb, const uint8_t* sb, int n, int k0, int64_t d, int64_t nbd, uint8_t* ob, uint32_t (&sc)[NC]) {
+#pragma unroll 1
+  for (int c = 0; c < NC; ++c) {
+    float amax = 0.0f, p2 = 1.0f;
+    uint32_t code = 0;
+    for (int j = 0; j < n; ++j) amax = fmaxf(amax, fabsf(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd])));
+    if (amax > 0.0f) block_scale<FMT>(amax, code, p2);
+    sc[c] = code;
+    for (int j = k0; j < min(n, k0 + 8); ++j) ob[j * d + c] = (uint8_t)encode_rne<FMT>(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd]) * p2);
   }
-  float p2[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) { sc[q] = 0; p2[q] = 1.0f; if (amax[q] > 0.0f) block_scale<FMT>(amax[q], sc[q], p2[q]); }
-  for (int j = 0; j < n; j++) {
-    const uint32_t cw = *reinterpret_cast<const uint32_t*>(cb + (int64_t)j * d);
-    const uint32_t sj = sb[(int64_t)j * nbd];
-    *reinterpret_cast<uint32_t*>(ob + (int64_t)j * d) =
-        ref_encode4<FMT>(decode_scaled<FMT>(cw & 0xFFu, sj) * p2[0], decode_scaled<FMT>((cw >> 8) & 0xFFu, sj) * p2[1],
-                         decode_scaled<FMT>((cw >> 16) & 0xFFu, sj) * p2[2], decode_scaled<FMT>(cw >> 24, sj) * p2[3]);
-  }
-}
-
-// ---- re-blocking in integer arithmetic ------------------------------------------------------------------------
-// Written out for E4M3 (the other formats differ in the constants of RebaseT): a normal code c (magnitude bits
-// mag = c & 0x7F >= 8) under scale code s has the value (1 + m/8) * 2^(L/8 - 134) with L = mag + 8 s (m = L & 7),
-// so the largest |value| of a block is the largest L, the block rule gives the new scale code
-// s' = L_max/8 - 15 (+1 when the mantissa of the maximum is 7, i.e. above 1.75 = 448/256; only E4M3 has a top
-// mantissa that its largest normal lacks), and an element's new code is sign | (L - 8 s') whenever that is a
-// normal code; smaller ones are rounded to nearest-even into the subnormal grid.  A subnormal input is first
-// normalised to the same (1 + m/8) * 2^x form, which gives it a (possibly negative) pseudo-magnitude.
-// Identical to decoding to fp32 and re-quantizing (which the generic path does).
-// Two elements ride in one register as 16-bit lanes (L < 4096), maxima by max.u16x2.
-template <int FMT> struct RebaseT {
-  static constexpr int MB = FmtT<FMT>::mbits;                                        // mantissa bits
-  static constexpr uint32_t MAG = (1u << (FmtT<FMT>::ebits + FmtT<FMT>::mbits)) - 1u;   // magnitude bits of a code
-  static constexpr uint32_t SIGN = MAG + 1u;
-  static constexpr int ONE = 1 << MB;                                                // smallest normal magnitude
-  static constexpr int OFF = FmtT<FMT>::bias + FmtT<FMT>::emax;                      // s' = L_max / ONE - OFF
-  static constexpr bool PLUS1 = (FmtT<FMT>::max_mant != ONE - 1);                    // the block rule's "+1" can fire
-  static constexpr uint32_t S_LO = OFF + MB + 1;                                     // scale codes the integer path takes
-  static constexpr uint32_t MAG2 = MAG | (MAG << 16), SIGN4 = SIGN * 0x01010101u;
-  static constexpr uint32_t EXP4 = (MAG & ~(uint32_t)(ONE - 1)) * 0x01010101u, LOW4 = (uint32_t)ONE * 0x01010101u;
-};
-RK_DEVINL uint32_t max_u16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-// pseudo-magnitude of a subnormal code, mag in 1 .. ONE-1: value = mag * 2^x = (1 + m'/ONE) * 2^(x')
-template <int FMT> RK_DEVINL int rb_subnormal_mag(int mag) {
-  using R = RebaseT<FMT>;
-  const int p = 31 - __clz(mag);                       // 0 .. MB-1
-  return ((mag << (R::MB - p)) & (R::ONE - 1)) + R::ONE * (p - R::MB + 1);
-}
-// new code (without sign) of an element with L - ONE s' = tt
-template <int FMT> RK_DEVINL uint32_t rb_code_from_tt(int tt) {
-  using R = RebaseT<FMT>;
-  if (tt >= R::ONE) return (uint32_t)tt;
-  const int sh = 1 - (tt >> R::MB);                    // >= 1: below the smallest normal
-  return sh > R::MB + 2 ? 0u : round_shift((uint32_t)R::ONE | (uint32_t)(tt & (R::ONE - 1)), sh);
-}
-// non-zero when some byte of w has a zero exponent field (zero or subnormal code)
-template <int FMT> RK_DEVINL uint32_t rb_exp0_bits(uint32_t w) {
-  using R = RebaseT<FMT>;
-  const uint32_t e = w & R::EXP4;
-  return (e - R::LOW4) & ~e & 0x80808080u;
-}
-RK_DEVINL uint32_t addmax_u16x2(uint32_t a, uint32_t b, uint32_t c) {   // max(a + b, c) in both 16-bit lanes
-  uint32_t r;
-  asm("{ .reg .b32 t; add.u16x2 t, %1, %2; max.u16x2 %0, t, %3; }" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-  return r;
-}
-
-// Rare rows (a zero or subnormal code among the four): per-byte L, packed as lanes (0, 2) and (1, 3).
-template <int FMT> __device__ __noinline__ uint2 rb_rare_l(uint32_t cw, int sj) {
-  using R = RebaseT<FMT>;
-  uint32_t l[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int mag = (int)((cw >> (8 * q)) & R::MAG);
-    l[q] = mag == 0 ? 0u : (uint32_t)((mag >= R::ONE ? mag : rb_subnormal_mag<FMT>(mag)) + R::ONE * sj) & 0xFFFFu;
-  }
-  return make_uint2(l[0] | (l[2] << 16), l[1] | (l[3] << 16));
-}
-// Rare rows of the second pass: some lane leaves the normal range, or an input was zero / subnormal.
-// sub02 / sub13 carry ONE * s' of columns (0, 2) and (1, 3) as 16-bit lanes.
-template <int FMT> __device__ __noinline__ uint32_t rb_rare_recode(uint32_t cw, int sj, uint32_t sub02, uint32_t sub13) {
-  using R = RebaseT<FMT>;
-  uint32_t out = cw & R::SIGN4;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int mag = (int)((cw >> (8 * q)) & R::MAG);
-    const int sub = (int)((((q & 1) ? sub13 : sub02) >> (16 * (q >> 1))) & 0xFFFFu);
-    if (mag != 0) out |= rb_code_from_tt<FMT>((mag >= R::ONE ? mag : rb_subnormal_mag<FMT>(mag)) + R::ONE * sj - sub) << (8 * q);
-  }
-  return out;
 }
 
 // Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one thread per (atom, row or column)
@@ -747,11 +660,14 @@ RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t tid, int64_t nth
     *reinterpret_cast<uint32_t*>(job.out + atom * 512 + sf_atom_offset(r, 0)) = w;
   }
 }
-// The jobs of a prefill call ride along with whichever preparation kernel it needs anyway (a launch costs more than they do).
-RK_DEVINL void retile_jobs(const RetileJobs& jobs) {
+// The jobs of a prefill call ride along with whichever preparation kernel it needs anyway (a launch costs more than they do):
+// its first jobs.ctas CTAs do them, true for those.
+RK_DEVINL bool retile_jobs(const RetileJobs& jobs) {
+  if ((int)blockIdx.x >= jobs.ctas) return false;
 #pragma unroll 1
   for (int i = 0; i < jobs.n; ++i)
-    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)jobs.ctas * blockDim.x);
+  return true;
 }
 __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs jobs) {
   grid_dependency_wait();
@@ -759,168 +675,176 @@ __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs job
   retile_jobs(jobs);
 }
 
-// Bytes of key-scale atoms that belong to no block (columns past d, key blocks past S): 2^0.  The re-blocking kernel writes the
-// others, bytes of its own.
-RK_DEVINL void fill_ragged_atoms(uint8_t* __restrict__ atoms, int64_t batch, int64_t S, int64_t d) {
-  const int64_t nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128, total = batch * ntile * dch * 128;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int n = (int)(t & 127);
-    const int64_t atom = t >> 7, col = (atom % dch) * 128 + n, kb0 = (atom / dch) % ntile * 4;
-    uint8_t* w = atoms + atom * 512 + sf_atom_offset(n, 0);
-    for (int k = 0; k < 4; ++k)
-      if (col >= d || kb0 + k >= nkb) w[k] = 0x7Fu;
-  }
+// ---- V re-blocking: scales along d -> MX blocks along the keys --------------------------------------------------------
+// Decode exactly, then the block rule down each column: the same as decoding to fp32 and quantizing again.  The hot form does
+// it in f16: a pair of codes goes through the hardware converter, times the row's scale relative to the block's largest, the
+// column maxima are packed maxima, the column's factor (a power of two, at least 1) is one more packed product, and the
+// pair goes back through the converter.  All of it is exact: values of a format are multiples of 2^-9 (E4M3), 2^-16 (E5M2) or
+// 2^-4 (the others) and f16 reaches down to 2^-24, so it holds while the block's scales span no more than kSpan and a column's
+// factor stays an f16; other blocks and columns take the slow form through fp32, element by element.
+template <int FMT> struct RebaseT { static constexpr int kSpan = FMT == 1 ? 8 : 14; };
+// two codes in the low bytes -> packed f16 (exact); an E2M1 code, shifted, is the E2M3 code of its value
+template <int FMT> RK_DEVINL uint32_t decode_f16x2(uint32_t codes) {
+  uint32_t r;
+  if (FMT == 0) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  else if (FMT == 1) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e5m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  else if (FMT == 3) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e3m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  else asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e2m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
+  return r;
+}
+// a word of four codes as the converter takes them
+template <int FMT> RK_DEVINL uint32_t clean_codes(uint32_t w) {
+  return FMT == 4 ? (w & 0x0F0F0F0Fu) << 2 : FMT >= 2 ? w & 0x3F3F3F3Fu : w;
+}
+RK_DEVINL uint32_t max_u16x2(uint32_t a, uint32_t b) { uint32_t r; asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+RK_DEVINL uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+RK_DEVINL float f16_lo(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, l;\n\t}" : "=f"(r) : "r"(v)); return r; }
+RK_DEVINL float f16_hi(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "r"(v)); return r; }
+// packed f16 pairs -> four codes (finite, exact values: as encode_rne)
+template <int FMT> RK_DEVINL uint32_t encode_f16x4(uint32_t lo, uint32_t hi) {
+  uint32_t r;
+  if (FMT == 0) asm("{\n\t.reg .b16 a, b;\n\tcvt.rn.satfinite.e4m3x2.f16x2 a, %1;\n\tcvt.rn.satfinite.e4m3x2.f16x2 b, %2;\n\tmov.b32 %0, {a, b};\n\t}" : "=r"(r) : "r"(lo), "r"(hi));
+  else if (FMT == 1) asm("{\n\t.reg .b16 a, b;\n\tcvt.rn.satfinite.e5m2x2.f16x2 a, %1;\n\tcvt.rn.satfinite.e5m2x2.f16x2 b, %2;\n\tmov.b32 %0, {a, b};\n\t}" : "=r"(r) : "r"(lo), "r"(hi));
+  else r = hw_encode4<FMT>(f16_lo(lo), f16_hi(lo), f16_lo(hi), f16_hi(hi));
+  return r;
 }
 
-// Four lanes share one unit = 16 adjacent columns x one 32-key block: lane "rg" holds rows 8 rg .. 8 rg + 7 as
-// eight 16-byte words in registers between the two passes (all loads of a thread in flight together), the
-// column maxima meet by two shuffles.  A warp covers 8 adjacent units, so each 16-byte access of a warp touches
-// four full 128-byte lines.  Blocks with scale codes outside [S_LO, 240] go through the generic fp32 path, each
-// lane taking 4 of the unit's 16 columns over all 32 keys.
-template <int FMT, bool TILED>
-__global__ void __launch_bounds__(128, 4) rebase_v_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
-                                                          int64_t batch, int64_t S, int64_t d,
-                                                          uint8_t* __restrict__ out_codes, uint8_t* __restrict__ out_scales,
-                                                          const RetileJobs jobs) {
+// A CTA = 128 keys x 8 NC columns at a time, a warp = 32 of the keys, a lane = 8 of them x NC adjacent columns, all its loads
+// in flight; the column maxima meet by two shuffles.  NC = 8, or 4 where the codes are not 8-byte aligned.
+// 67 M codes E4M3: 53 us in integer arithmetic on the codes (12 instructions per code, 16 warps per SM, rows with a zero or
+// subnormal code on a path of their own), 32 us here (36 beside the scales' re-tiling).
+constexpr int kRebaseThreads = 128;
+template <int FMT, bool TILED, int NC>
+__global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
+                                                                 int64_t batch, int64_t S, int64_t d, uint8_t* __restrict__ out_codes,
+                                                                 uint8_t* __restrict__ out_scales, const RetileJobs jobs) {
+  constexpr int NW = NC / 4, NB = NC / 4;                          // words per key of a thread; 32-column blocks of a warp
+  __shared__ __align__(4) uint8_t sc_sm[8 * NC * 4];
+  __shared__ __align__(16) uint32_t fac_sm[kRebaseThreads / 32][NB][32];
   grid_dependency_wait();
   grid_dependents_launch();
-  retile_jobs(jobs);
-  if (TILED && (S % 128 != 0 || d % 128 != 0)) fill_ragged_atoms(out_scales, batch, S, d);
-  const int64_t c16n = d / 16, nkb = (S + 31) / 32, nbd = d / 32;
-  const int64_t units = batch * nkb * c16n;
-  const int64_t ntile = (S + 127) / 128, dch = (d + 127) / 128;   // atom grid of the TILED layout
-  const int64_t warps_total = (units + 7) / 8;
-  const int lane = threadIdx.x & 31, rg = lane >> 3;
-  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < warps_total;
-       w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t u = w * 8 + (lane & 7);
-    const bool valid = u < units;
-    const int64_t uu = valid ? u : 0;
-    // unit index -> (batch, key block, column group): in 32 bits whenever it fits (a 64-bit division by a run-time
-    // value is about a hundred instructions, and there are three of them per unit)
-    int64_t c16, kb, bt;
-    if (units < (int64_t)1 << 31) {
-      const uint32_t u32 = (uint32_t)uu, q = u32 / (uint32_t)c16n;
-      c16 = u32 - q * (uint32_t)c16n;
-      const uint32_t b32 = q / (uint32_t)nkb;
-      kb = q - b32 * (uint32_t)nkb;
+  if (retile_jobs(jobs)) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k0 = (lane >> 3) * 8, b = (lane & 7) * NC / 32;
+  const int64_t nkb = (S + 31) / 32, nbd = d / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
+  const int64_t cun = TILED ? dch * (16 / NC) : (d + 8 * NC - 1) / (8 * NC), units = batch * ntile * cun, stride = gridDim.x - jobs.ctas;
+  for (int64_t u = (int64_t)blockIdx.x - jobs.ctas; u < units; u += stride) {
+    int64_t cu, kt, bt;
+    if (units < (int64_t)1 << 31) {                                // 32-bit divisions whenever the index fits
+      const uint32_t q = (uint32_t)u / (uint32_t)cun;
+      cu = (uint32_t)u - q * (uint32_t)cun;
+      const uint32_t b32 = q / (uint32_t)ntile;
+      kt = q - b32 * (uint32_t)ntile;
       bt = b32;
     } else {
-      c16 = uu % c16n; kb = (uu / c16n) % nkb; bt = uu / (c16n * nkb);
+      cu = u % cun; kt = u / cun % ntile; bt = u / (cun * ntile);
     }
-    const int64_t r0 = kb * 32;
-    const int n = valid ? (int)min((int64_t)32, S - r0) : 0;      // keys of this block that exist
-    const uint8_t* cb = codes + (bt * S + r0) * d + c16 * 16;
-    const uint8_t* sb = scales + (bt * S + r0) * nbd + c16 / 2;
-    uint8_t* ob = out_codes + (bt * S + r0) * d + c16 * 16;
-    uint32_t sc[4];                                               // new scale codes of columns 4 rg .. 4 rg + 3
-    using R = RebaseT<FMT>;
-    uint32_t bad = 0u;
-    {
-      // rows past a ragged end read as the smallest normal codes under the smallest scale the integer path takes: no real row
-      // is below them, so they change nothing (as zero codes they would take the slow path for rare rows)
-      uint4 cw[8];
-      uint32_t s8[8];
+    const int64_t kb = kt * 4 + warp;
+    const int64_t row0 = bt * S + kb * 32, col = cu * 8 * NC + (lane & 7) * NC;
+    const int n = (int)max((int64_t)0, min((int64_t)32, S - kb * 32));   // keys of this block that exist
+    const bool in = col < d && n > 0;
+    const uint8_t* src = codes + row0 * d + col;
+    uint32_t w[8][NW];
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int j = rg * 8 + i;
-        const bool in = j < n;
-        cw[i] = in ? __ldg(reinterpret_cast<const uint4*>(cb + (int64_t)j * d)) : make_uint4(R::LOW4, R::LOW4, R::LOW4, R::LOW4);
-        s8[i] = in ? (uint32_t)__ldg(sb + (int64_t)j * nbd) : 0u;
-      }
-      // pass 1: largest L per column; word x of a row holds columns 4x .. 4x+3, lanes (0, 2) in lo[x], (1, 3) in hi[x]
-      uint32_t lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        bad |= (s8[i] - R::S_LO > 240u - R::S_LO && rg * 8 + i < n) ? 1u : 0u;
-        s8[i] *= (uint32_t)R::ONE * 0x00010001u;
-        const uint32_t wv[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
-        // one test per row: does any of its 16 codes have a zero exponent field (zero or subnormal)?
-        if ((rb_exp0_bits<FMT>(wv[0]) | rb_exp0_bits<FMT>(wv[1]) | rb_exp0_bits<FMT>(wv[2]) | rb_exp0_bits<FMT>(wv[3])) == 0u) {
-#pragma unroll
-          for (int x = 0; x < 4; x++) {
-            lo[x] = addmax_u16x2(wv[x] & R::MAG2, s8[i], lo[x]);
-            hi[x] = addmax_u16x2((wv[x] >> 8) & R::MAG2, s8[i], hi[x]);
-          }
-        } else {
-#pragma unroll
-          for (int x = 0; x < 4; x++) {
-            uint2 l = make_uint2((wv[x] & R::MAG2) + s8[i], ((wv[x] >> 8) & R::MAG2) + s8[i]);
-            if (rb_exp0_bits<FMT>(wv[x]) != 0u) l = rb_rare_l<FMT>(wv[x], (int)((s8[i] & 0xFFFFu) >> R::MB));
-            lo[x] = max_u16x2(lo[x], l.x);
-            hi[x] = max_u16x2(hi[x], l.y);
-          }
-        }
-      }
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        lo[x] = max_u16x2(lo[x], __shfl_xor_sync(0xFFFFFFFFu, lo[x], 8));
-        hi[x] = max_u16x2(hi[x], __shfl_xor_sync(0xFFFFFFFFu, hi[x], 8));
-        lo[x] = max_u16x2(lo[x], __shfl_xor_sync(0xFFFFFFFFu, lo[x], 16));
-        hi[x] = max_u16x2(hi[x], __shfl_xor_sync(0xFFFFFFFFu, hi[x], 16));
-      }
-      bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, 8);
-      bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, 16);
-      if (bad == 0u) {
-        // s' = L_max / 8 - 15 (+1 when the mantissa bits are 7) in both 16-bit lanes at once; all-zero columns
-        // (L_max = 0, or that of a row past the end) get scale code 0
-        uint32_t sub_lo[4], sub_hi[4];
-#pragma unroll
-        for (int x = 0; x < 4; x++) {
-          uint32_t v[2] = {lo[x], hi[x]};
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            constexpr uint32_t M2 = (uint32_t)(R::ONE - 1) * 0x00010001u, Q2 = (0xFFFFu >> R::MB) * 0x00010001u;
-            uint32_t sn = (v[h] >> R::MB) & Q2;
-            if (R::PLUS1) sn += (((v[h] & M2) + 0x00010001u) >> R::MB) & 0x00010001u;
-            if ((v[h] & 0xFFFFu) <= (uint32_t)R::ONE) sn = (sn & 0xFFFF0000u) | (uint32_t)R::OFF;   // nothing but zeros: scale code 0
-            if ((v[h] >> 16) <= (uint32_t)R::ONE) sn = (sn & 0x0000FFFFu) | ((uint32_t)R::OFF << 16);
-            v[h] = sn - (uint32_t)R::OFF * 0x00010001u;
-          }
-          sub_lo[x] = v[0] << R::MB;
-          sub_hi[x] = v[1] << R::MB;
-          if (x == rg) {
-            sc[0] = v[0] & 0xFFFFu; sc[1] = v[1] & 0xFFFFu; sc[2] = v[0] >> 16; sc[3] = v[1] >> 16;
-          }
-        }
-        // pass 2: lanes carry tt + 0x4000 (tt = L - 8 s') so that they stay non-negative
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          if (rg * 8 + i >= n) break;
-          const uint32_t wv[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
-          uint32_t ov[4];
-          // lanes that leave the normal range (tt < 8) set bit 15 of their half; zero / subnormal inputs set bit 7
-          uint32_t rare[4];
-#pragma unroll
-          for (int x = 0; x < 4; x++) {
-            const uint32_t t_lo = (wv[x] & R::MAG2) + s8[i] + (0x40004000u - sub_lo[x]);
-            const uint32_t t_hi = ((wv[x] >> 8) & R::MAG2) + s8[i] + (0x40004000u - sub_hi[x]);
-            ov[x] = (wv[x] & R::SIGN4) | (t_lo & R::MAG2) | ((t_hi & R::MAG2) << 8);
-            rare[x] = (((t_lo - (0x40004000u + (uint32_t)R::ONE * 0x00010001u)) | (t_hi - (0x40004000u + (uint32_t)R::ONE * 0x00010001u))) & 0x80008000u) | rb_exp0_bits<FMT>(wv[x]);
-          }
-          if ((rare[0] | rare[1] | rare[2] | rare[3]) != 0u) {      // one branch per row in the common case
-#pragma unroll
-            for (int x = 0; x < 4; x++)
-              if (rare[x] != 0u) ov[x] = rb_rare_recode<FMT>(wv[x], (int)((s8[i] & 0xFFFFu) >> R::MB), sub_lo[x], sub_hi[x]);
-          }
-          *reinterpret_cast<uint4*>(ob + (int64_t)(rg * 8 + i) * d) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
-        }
+    for (int i = 0; i < 8; ++i) {
+      const bool live = in && k0 + i < n;
+      const uint8_t* q = src + (k0 + i) * d;
+      if (NC == 8) {
+        const uint2 v = live ? __ldg(reinterpret_cast<const uint2*>(q)) : make_uint2(0u, 0u);
+        w[i][0] = v.x; w[i][NW - 1] = v.y;
+      } else {
+        w[i][0] = live ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
       }
     }
-    if (!valid) continue;
-    if (bad != 0u) rebase_block_generic<FMT>(cb + rg * 4, sb, n, d, nbd, ob + rg * 4, sc);
-    const int64_t col0 = c16 * 16 + rg * 4;
-    if (TILED) {
-      const int64_t kt = kb / 4;
-      const int kbi = (int)(kb % 4);
+    // the rows' scales relative to the block's largest, as packed f16; lane = key
+    int smax = 0;
+    bool hot = true;
+    const uint8_t* sk = scales + (row0 + lane) * nbd + cu * NB;
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int64_t col = col0 + q;
-        const int64_t atom = (bt * ntile + kt) * dch + col / 128;
-        out_scales[atom * 512 + sf_atom_offset((int)(col % 128), kbi)] = (uint8_t)sc[q];
+    for (int c = 0; c < NB; ++c) {
+      const bool live = lane < n && cu * NB + c < nbd;
+      const int s = live ? (int)__ldg(sk + c) : -1;
+      const int top = __reduce_max_sync(0xffffffffu, s), low = __reduce_min_sync(0xffffffffu, live ? s : 255);
+      fac_sm[warp][c][lane] = live ? (uint32_t)max(15 + s - top, 1) * 0x04000400u : 0u;
+      if (c == b) { smax = max(top, 0); hot = low >= 20 && top <= 235 && top - low <= RebaseT<FMT>::kSpan; }
+    }
+    __syncwarp();
+    uint32_t m[2 * NW];                                            // maxima of column pairs
+#pragma unroll
+    for (int i = 0; i < 2 * NW; ++i) m[i] = 0u;
+    uint32_t x[8][2 * NW];
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      const uint4 f4 = *reinterpret_cast<const uint4*>(&fac_sm[warp][b][k0 + i]);
+      const uint32_t f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+          const uint32_t c = clean_codes<FMT>(w[i + e][q]);
+          x[i + e][2 * q] = hmul2(decode_f16x2<FMT>(c), f[e]);
+          x[i + e][2 * q + 1] = hmul2(decode_f16x2<FMT>(c >> 16), f[e]);
+          m[2 * q] = max_u16x2(m[2 * q], x[i + e][2 * q] & 0x7FFF7FFFu);
+          m[2 * q + 1] = max_u16x2(m[2 * q + 1], x[i + e][2 * q + 1] & 0x7FFF7FFFu);
+        }
+    }
+    __syncwarp();                                                  // fac_sm has been read
+#pragma unroll
+    for (int i = 0; i < 2 * NW; ++i) {
+      m[i] = max_u16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+      m[i] = max_u16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], 16));
+    }
+    uint32_t sc[NC], f[2 * NW];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) sc[q] = 0x7Fu;                    // of columns and key blocks that do not exist: 2^0
+    if (in) {
+    const float unit = __uint_as_float((uint32_t)smax << 23);      // 2^(smax - 127)
+#pragma unroll
+    for (int i = 0; i < 2 * NW; ++i) {
+      f[i] = 0u;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float am = (h ? f16_hi(m[i]) : f16_lo(m[i])) * unit;
+        uint32_t code = 0; float p2;
+        int up = 0;                                                // log2 of the column's factor
+        if (am > 0.0f) { block_scale<FMT>(am, code, p2); up = (int)(__float_as_uint(p2) >> 23) - 254 + smax; }
+        hot = hot && up <= 15 && (FMT > 1 || am < __int_as_float(0x7f800000));      // (NaN and infinity encodings are numbers here)
+        sc[2 * i + h] = code;
+        f[i] |= (uint32_t)((15 + up) & 31) << (10 + 16 * h);
+      }
+    }
+    uint8_t* dst = out_codes + row0 * d + col;
+    if (hot) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (k0 + i >= n) break;
+        uint32_t o[NW];
+#pragma unroll
+        for (int q = 0; q < NW; ++q) o[q] = encode_f16x4<FMT>(hmul2(x[i][2 * q], f[2 * q]), hmul2(x[i][2 * q + 1], f[2 * q + 1]));
+        if (NC == 8) *reinterpret_cast<uint2*>(dst + (k0 + i) * d) = make_uint2(o[0], o[NW - 1]);
+        else *reinterpret_cast<uint32_t*>(dst + (k0 + i) * d) = o[0];
       }
     } else {
-      *reinterpret_cast<uint32_t*>(out_scales + (bt * nkb + kb) * d + col0) = sc[0] | (sc[1] << 8) | (sc[2] << 16) | (sc[3] << 24);
+      rebase_slow<FMT, NC>(src, scales + row0 * nbd + col / 32, n, k0, d, nbd, dst, sc);
+    }
+    }
+    if (TILED) {
+      // the four warps' scale bytes of a column are one word of its atom
+      if ((lane >> 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < NC; ++q) sc_sm[((lane & 7) * NC + q) * 4 + warp] = (uint8_t)sc[q];
+      }
+      __syncthreads();
+      for (int c = threadIdx.x; c < 8 * NC; c += kRebaseThreads) {
+        const int64_t n128 = cu * 8 * NC + c;
+        *reinterpret_cast<uint32_t*>(out_scales + ((bt * ntile + kt) * dch + n128 / 128) * 512 + sf_atom_offset((int)(n128 % 128), 0)) =
+            *reinterpret_cast<const uint32_t*>(sc_sm + c * 4);
+      }
+      __syncthreads();
+    } else if (in) {
+      // each of the four lanes of a column group writes a quarter of its scale codes
+#pragma unroll
+      for (int q = 0; q < NC; ++q)
+        if (q / (NC / 4) == (lane >> 3)) out_scales[(bt * nkb + kb) * d + col + q] = (uint8_t)sc[q];
     }
   }
 }
@@ -982,35 +906,58 @@ template <int BITS, int N> RK_DEVINL void join_groups(const uint32_t (&c)[N], ui
   }
 }
 
-// byte codes [rows][d] -> packed [rows][dp * BITS/8 bytes], dp = d rounded up to 128, padding codes 0
-template <int BITS> RK_DEVINL void pack_rows_body(const PackJob& job, int64_t d, int64_t dp) {
-  const int64_t groups = dp / 16, total = job.rows * groups;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r, g;
-    if (total < (int64_t)1 << 31) { const uint32_t q = (uint32_t)t / (uint32_t)groups; r = q; g = (uint32_t)t - q * (uint32_t)groups; }
-    else { r = t / groups; g = t % groups; }
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (g * 16 < d) v = __ldcs(reinterpret_cast<const uint4*>(job.in + r * d + g * 16));
-    const uint32_t c[4] = {pack4<BITS>(v.x), pack4<BITS>(v.y), pack4<BITS>(v.z), pack4<BITS>(v.w)};
-    uint32_t w[BITS / 2];
-    join_groups<BITS, 4>(c, w);
-    uint8_t* o = job.out + r * (dp * BITS / 8) + g * (2 * BITS);
-    if (BITS == 4) {
-      *reinterpret_cast<uint2*>(o) = make_uint2(w[0], w[1]);
-    } else {
+// byte codes [rows][d] -> packed [rows][dp * BITS/8 bytes], dp = d rounded up to 128, padding codes 0.  A warp packs 512 codes at
+// a time, 16 per lane, four times' loads in flight; the 6-bit words (12 bytes per lane) pass through shared memory to leave in
+// 16-byte stores (one 16-byte load in flight and three 4-byte stores at a stride of 12 left HBM at a third of its rate).
+template <int BITS> RK_DEVINL void pack_rows_body(const PackJob& job, int64_t d, int64_t dp, uint32_t* stage, int64_t warp0, int64_t warps) {
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  const int64_t groups = dp / 16, total = job.rows * groups;          // a multiple of 8
+  for (int64_t c0 = warp0 * 32; c0 < total; c0 += U * 32 * warps) {
+    uint4 v[U];
 #pragma unroll
-      for (int i = 0; i < BITS / 2; ++i) reinterpret_cast<uint32_t*>(o)[i] = w[i];
+    for (int u = 0; u < U; ++u) {
+      const int64_t t = c0 + u * 32 * warps + lane;
+      v[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (t < total) {
+        if (dp == d) {
+          v[u] = __ldcs(reinterpret_cast<const uint4*>(job.in) + t);
+        } else {
+          const int64_t r = t / groups, g = t - r * groups;
+          if (g * 16 < d) v[u] = __ldcs(reinterpret_cast<const uint4*>(job.in + r * d + g * 16));
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t first = c0 + u * 32 * warps;
+      if (first >= total) break;
+      const int n = (int)min((int64_t)32, total - first);             // lanes with codes
+      const uint32_t c[4] = {pack4<BITS>(v[u].x), pack4<BITS>(v[u].y), pack4<BITS>(v[u].z), pack4<BITS>(v[u].w)};
+      uint32_t w[BITS / 2];
+      join_groups<BITS, 4>(c, w);
+      if (BITS == 4) {
+        if (lane < n) __stcs(reinterpret_cast<uint2*>(job.out) + first + lane, make_uint2(w[0], w[1]));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) stage[lane * 3 + i] = w[i % (BITS / 2)];
+        __syncwarp();
+        if (lane < n * 3 / 4) __stcs(reinterpret_cast<uint4*>(job.out + first * 12) + lane, reinterpret_cast<const uint4*>(stage)[lane]);
+        __syncwarp();
+      }
     }
   }
 }
 __global__ void __launch_bounds__(256) pack_rows_kernel(const PackJobs packs, int64_t d, int64_t dp, const RetileJobs jobs) {
+  __shared__ __align__(16) uint32_t stage[8][96];
   grid_dependency_wait();
   grid_dependents_launch();
-  retile_jobs(jobs);
+  if (retile_jobs(jobs)) return;
+  const int64_t warp0 = ((int64_t)blockIdx.x - jobs.ctas) * 8 + (threadIdx.x >> 5), warps = ((int64_t)gridDim.x - jobs.ctas) * 8;
 #pragma unroll 1
   for (int i = 0; i < packs.n; ++i) {
-    if (packs.job[i].bits == 4) pack_rows_body<4>(packs.job[i], d, dp);
-    else pack_rows_body<6>(packs.job[i], d, dp);
+    if (packs.job[i].bits == 4) pack_rows_body<4>(packs.job[i], d, dp, stage[threadIdx.x >> 5], warp0, warps);
+    else pack_rows_body<6>(packs.job[i], d, dp, stage[threadIdx.x >> 5], warp0, warps);
   }
 }
 
@@ -1020,20 +967,9 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const PackJobs packs, in
 // going to the scale-factor atoms.
 // One CTA = 128 keys x 128 columns, a warp = one 32-key block, a thread = 4 columns x 32 keys in registers, all its loads in
 // flight.  In these formats zero and subnormal codes are common, which the integer form of the re-blocking kernel pays for
-// row by row; here a pair of codes goes through the hardware converter to f16, times the row's scale relative to the block's
-// largest (exact: every value is a multiple of 2^-4 or coarser, f16 reaches down to 2^-24, and blocks whose scales span more
-// than 2^14 take the slow form), the column maxima are packed f16 operations, and pairs of keys of one column go back through
+// row by row.  Here as there the codes go through f16, and pairs of keys of one column go back through
 // the converter in the order in which they are packed.  The packed words meet in shared memory and leave in 16-byte stores.
-// 33.5 M codes E3M2: re-blocking 138 us and transposition 27 us as kernels of their own, PACKV_NOW us here.
-template <int FMT> RK_DEVINL uint32_t decode_f16x2(uint32_t codes) {            // two codes in the low bytes -> packed f16
-  uint32_t r;
-  if (FMT == 3) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e3m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  else asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e2m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  return r;
-}
-RK_DEVINL uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-RK_DEVINL float f16_lo(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, l;\n\t}" : "=f"(r) : "r"(v)); return r; }
-RK_DEVINL float f16_hi(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "r"(v)); return r; }
+// 33.5 M codes E3M2: re-blocking 138 us and transposition 27 us as kernels of their own, 31 us here.
 // codes of four consecutive keys, packed
 template <int FMT> RK_DEVINL uint32_t encode_pack4(float a, float b, float c, float d) {
   uint32_t r;
@@ -1045,7 +981,7 @@ template <int FMT> RK_DEVINL uint32_t encode_pack4(float a, float b, float c, fl
   return pack4<6>(hw_encode4<FMT>(a, b, c, d));
 }
 template <int FMT, bool REBASE>
-__global__ void __launch_bounds__(128) pack_v_kernel(const uint8_t* __restrict__ in, const uint8_t* __restrict__ scales, int64_t S, int64_t d,
+__global__ void __launch_bounds__(128, 8) pack_v_kernel(const uint8_t* __restrict__ in, const uint8_t* __restrict__ scales, int64_t S, int64_t d,
                                                      int64_t Sp, uint8_t* __restrict__ out, uint8_t* __restrict__ atoms) {
   constexpr int BITS = FMT == 4 ? 4 : 6, kWords = BITS, kRow = 4 * kWords, kPitch = kRow + 1;   // words per key block, per column; pitch
   __shared__ uint32_t buf[128 * kPitch];
@@ -1072,7 +1008,7 @@ __global__ void __launch_bounds__(128) pack_v_kernel(const uint8_t* __restrict__
       const int s = live ? (int)__ldg(sk + b) : -1;
       const int top = __reduce_max_sync(0xffffffffu, s), low = __reduce_min_sync(0xffffffffu, live ? s : 255);
       fac[b][kb * 32 + lane] = live ? (uint32_t)max(15 + s - top, 1) * 0x04000400u : 0u;
-      if (lane == 0) smax_sm[b][kb] = (top < 0 || (low >= 20 && top <= 235 && top - low <= 14)) ? max(top, 0) : -1;
+      if (lane == 0) smax_sm[b][kb] = (top < 0 || (low >= 20 && top <= 235 && top - low <= RebaseT<FMT>::kSpan)) ? max(top, 0) : -1;
     }
     __syncwarp();
     const int blk = lane >> 3, smax = smax_sm[blk][kb];
@@ -1084,7 +1020,7 @@ __global__ void __launch_bounds__(128) pack_v_kernel(const uint8_t* __restrict__
         const uint32_t f[4] = {f4.x, f4.y, f4.z, f4.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const uint32_t c = FMT == 4 ? (w[k + e] & 0x0F0F0F0Fu) << 2 : w[k + e] & 0x3F3F3F3Fu;     // an E2M1 code, shifted, is the E2M3 code of its value
+          const uint32_t c = clean_codes<FMT>(w[k + e]);
           x[k + e] = hmul2(decode_f16x2<FMT>(c), f[e]);
           y[k + e] = hmul2(decode_f16x2<FMT>(c >> 16), f[e]);
           mx = max_u16x2(mx, x[k + e] & 0x7FFF7FFFu);
@@ -1230,11 +1166,16 @@ int launch_quantize_keys_atoms(const float* x, int64_t batch, int64_t rows, int6
   return (int)cudaGetLastError();
 }
 
-int launch_retile_scales(const RetileJobs& jobs, cudaStream_t st) {
+// CTAs of `threads` threads for the re-tiling jobs beside other work
+static int retile_ctas(const RetileJobs& jobs, int threads) {
   int64_t most = 0;
   for (int i = 0; i < jobs.n; ++i) most = std::max(most, jobs.job[i].batch * ((jobs.job[i].S + 127) / 128) * ((jobs.job[i].d + 127) / 128) * 128);
-  if (most == 0) return RK_OK;
-  return (int)launch_pdl(retile_scales_kernel, dim3(grid_for(most, 128, 16)), dim3(128), 0, st, jobs);
+  return most == 0 ? 0 : grid_for(most, threads, 4);
+}
+
+int launch_retile_scales(RetileJobs jobs, cudaStream_t st) {
+  if ((jobs.ctas = retile_ctas(jobs, 128)) == 0) return RK_OK;
+  return (int)launch_pdl(retile_scales_kernel, dim3(jobs.ctas), dim3(128), 0, st, jobs);
 }
 
 int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads, int nblk, int Bk, int d, uint8_t* k,
@@ -1312,21 +1253,26 @@ int launch_kv_append(const float* k_new, const float* v_new, int B, int H_kv, in
 }
 
 int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt,
-                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, const RetileJobs& jobs) {
-  const int64_t total = ((batch * ((S + 31) / 32) * (d / 16) + 7) / 8) * 32;     // 4 lanes per 16-column unit, whole warps
-  if (total == 0) return RK_OK;
-  const int grid = grid_for(total, 128, 16);      // four CTAs are resident per SM; four waves of them end more evenly than two (-6 %)
-  if (tiled) { RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, true>, dim3(grid), dim3(128), 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs)); }
-  else       { RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, false>, dim3(grid), dim3(128), 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs)); }
+                    uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, RetileJobs jobs) {
+  const bool wide = ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out_codes)) & 7) == 0;
+  const int64_t units = batch * ((S + 127) / 128) * (wide ? (d + 63) / 64 : d / 32);
+  if (units == 0) return RK_OK;
+  jobs.ctas = retile_ctas(jobs, kRebaseThreads);
+  const dim3 grid(jobs.ctas + grid_for(units * kRebaseThreads, kRebaseThreads, 28)), block(kRebaseThreads);      // four waves of the resident CTAs
+#define RK_RB(TI, N) RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, TI, N>, grid, block, 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs))
+  if (wide) { if (tiled) { RK_RB(true, 8); } else { RK_RB(false, 8); } }
+  else      { if (tiled) { RK_RB(true, 4); } else { RK_RB(false, 4); } }
+#undef RK_RB
   return RK_OK;
 }
 
-int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, const RetileJobs& jobs) {
+int launch_pack_rows(const PackJobs& packs, int64_t d, cudaStream_t st, RetileJobs jobs) {
   const int64_t dp = (d + 127) / 128 * 128;
   int64_t most = 0;
   for (int i = 0; i < packs.n; ++i) most = std::max(most, packs.job[i].rows * (dp / 16));
   if (most == 0) return RK_OK;
-  return (int)launch_pdl(pack_rows_kernel, dim3(grid_for(most, 256, 16)), dim3(256), 0, st, packs, d, dp, jobs);
+  jobs.ctas = retile_ctas(jobs, 256);
+  return (int)launch_pdl(pack_rows_kernel, dim3(jobs.ctas + grid_for((most + 3) / 4, 256, 16)), dim3(256), 0, st, packs, d, dp, jobs);
 }
 
 int launch_pack_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt, uint8_t* out,
