@@ -30,7 +30,8 @@
 // A tile is a serial chain -- S from TMEM, maximum, exponentials, P in shared memory, P V -- several times as long as its
 // bytes take to arrive, so four groups of four worker warps each take every fourth tile.  One warp loads, one puts the
 // tiles' key scales into the order of a scale atom, one issues S = K Q^T, one O += V^T P (with the scales in the issuer a
-// tile took it 1100 cycles, as long as HBM).
+// tile took it 1100 cycles, as long as HBM), one prepares the query terms of the next segment (loading and quantizing eight
+// heads takes longer than a tile, so in another warp's stream it held back every short sequence).
 //   worker warp w: group w / 4, thread = key (w % 4) * 32 + lane of the tile for S and P, and column d of O^T.
 // p of a warp's 32 keys is relative to their own maximum rounded up to an integer m_w (log2 domain), which the block scale
 // undoes exactly: nothing in a tile waits for the other warps' maxima but the scale bytes.  O and the row sums are relative
@@ -54,8 +55,9 @@ namespace rk {
 namespace dtc {
 constexpr int kGroups = 4;                        // worker groups of four warps
 constexpr int kWorkers = 4 * kGroups;             // worker warps
-constexpr int kWarpTma = kWorkers, kWarpSf = kWorkers + 1, kWarpQk = kWorkers + 2, kWarpPv = kWorkers + 3;
-constexpr int kThreads = (kWorkers + 4) * 32;
+constexpr int kWarpTma = kWorkers, kWarpSf = kWorkers + 1, kWarpQk = kWorkers + 2, kWarpPv = kWorkers + 3,
+              kWarpQ = kWorkers + 4;
+constexpr int kThreads = (kWorkers + 5) * 32;
 constexpr int kTile = 128;                        // keys per stage
 constexpr int kD = 128;
 constexpr int kMaxGrp = 8;                        // query heads per KV head this kernel handles
@@ -234,6 +236,13 @@ RK_DEVINL float redux_max_f32(float v) {
   asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
+// The bounded wait of the kernel's loops, in its short form (the code of a tile runs cold at the start of every launch, and a
+// short sequence is over before it is warm).  False, with the code recorded, when it gave up.
+RK_DEVINL bool dtc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__builtin_expect(mbar_wait_lean(bar, parity, abort_flag), 1)) return true;
+  report_wait_failure(abort_flag, status, code);
+  return false;
+}
 // Four packed E4M3 codes divided by 2^(d / 8): d8 = d in every byte, d a multiple of 8 up to 120.  Codes that leave the
 // normal range become 0 (or lose their hidden bit), an absolute error of 2^-15 of the block's largest element.  SIGN: codes
 // may be negative.
@@ -277,7 +286,7 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
     for (int i = i_first; i < seg.n; i += kGroups) {
       const int j = j0 + i, st = j % kStages, par = (j / kGroups) & 1;
       uint8_t* sb = smem + L::stage_off + st * kStageBytes;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bSF + g], par, abort_flag, p.status, 501));
+      ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bSF + g], par, abort_flag, p.status, 501));
       if (!ok) break;
       tc_fence_after();
       uint32_t c[2 * HH];
@@ -333,7 +342,7 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
       }
       // the P tile is free once the P V that read it (the group's previous tile) has completed
       if (j >= kGroups) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
+        ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
         if (!ok) break;
       }
       uint32_t d8[4];
@@ -352,15 +361,15 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
               make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
                          e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
       }
-      if (tail && !valid) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
+      if (__builtin_expect(tail && !valid, 0)) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
         uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);
 #pragma unroll
         for (int q = 0; q < 8; ++q) vrow[q] = make_uint4(0u, 0u, 0u, 0u);
       }
 
       // ---- references, scale bytes, row sums --------------------------------------------------------------------
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504) &&
-                                       (i == 0 || mbar_wait(&bars[L::bRef + (j - 1) % kRing], ((j - 1) / kRing) & 1, abort_flag, p.status, 507)));
+      ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504) &&
+                                       (i == 0 || dtc_wait(&bars[L::bRef + (j - 1) % kRing], ((j - 1) / kRing) & 1, abort_flag, p.status, 507)));
       if (!ok) break;
       {
         const float* xr = xchg + par * 64 + (lane >> 4) * 32 + item;
@@ -375,9 +384,9 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bRef + j % kRing]);
         }
-        if (bump) {
+        if (__builtin_expect(bump, 0)) {
           // rescale this thread's row of O once the tile before has been added; its own P V comes after this
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + ((j - 1) & (kGroups - 1))], ((j - 1) / kGroups) & 1, abort_flag, p.status, 502));
+          ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + ((j - 1) & (kGroups - 1))], ((j - 1) / kGroups) & 1, abort_flag, p.status, 502));
           if (!ok) break;
           tc_fence_after();
           uint32_t o[2 * HH];
@@ -433,7 +442,7 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
     // ---- end of the segment: every warp leaves its row sums; the group of the last tile puts the result together --------
     const int ob = sg % kOBufs;
     if (sg >= kOBufs) {                                            // the slot has been read
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bOE + ob], (sg / kOBufs - 1) & 1, abort_flag, p.status, 508));
+      ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bOE + ob], (sg / kOBufs - 1) & 1, abort_flag, p.status, 508));
       if (!ok) break;
     }
     {
@@ -459,8 +468,8 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
     }
     const int j_last = j0 + seg.n - 1;
     if ((j_last & (kGroups - 1)) == g) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bPV + g], (j_last / kGroups) & 1, abort_flag, p.status, 505) &&
-                                       mbar_wait(&bars[L::bSL + ob], (sg / kOBufs) & 1, abort_flag, p.status, 506));
+      ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + g], (j_last / kGroups) & 1, abort_flag, p.status, 505) &&
+                                       dtc_wait(&bars[L::bSL + ob], (sg / kOBufs) & 1, abort_flag, p.status, 506));
       if (!ok) break;
       tc_fence_after();
       uint32_t o[2 * HH];
@@ -513,28 +522,40 @@ RK_DEVINL uint2 dtc_query_load(const DecodeTcParams& p, int b, int hkv, int h, i
   if (h >= p.grp) return make_uint2(0u, 0u);
   return __ldg(reinterpret_cast<const uint2*>(p.q + ((size_t)b * p.H + hkv * p.grp + h) * dtc::kD + lane * 4));
 }
-// The head as two MXFP8 terms, q = hi + lo (the lib/golden block rule on q, then on the residual): a warp together.
-template <int HH> RK_DEVINL void dtc_query_store(uint8_t* smem, uint2 raw, int h, int buf, int lane) {
+// N heads from h0 on as two MXFP8 terms each, q = hi + lo (the lib/golden block rule on q, then on the residual): a warp
+// together, the heads side by side so that their shuffles overlap.
+template <int HH, int N> RK_DEVINL void dtc_query_store(uint8_t* smem, const uint2 (&raw)[N], int h0, int buf, int lane) {
   using L = dtc::Lay<HH>;
-  float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000u)};
+  float x[N][4];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    x[i][0] = __uint_as_float(raw[i].x << 16); x[i][1] = __uint_as_float(raw[i].x & 0xFFFF0000u);
+    x[i][2] = __uint_as_float(raw[i].y << 16); x[i][3] = __uint_as_float(raw[i].y & 0xFFFF0000u);
+  }
 #pragma unroll
   for (int term = 0; term < 2; ++term) {
-    float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));       // the 8 lanes of one 32-wide block of d
-    uint32_t code = 127u;
-    float p2 = 1.0f;
-    if (amax > 0.0f && amax < 3.0e38f) block_scale<0>(amax, code, p2);
-    const float back = e8m0_to_f32(code);
-    const uint32_t c01 = cvt_e4m3x2(x[1] * p2, x[0] * p2), c23 = cvt_e4m3x2(x[3] * p2, x[2] * p2);
-    float d0, d1, d2, d3;
-    e4m3x2_to_f32(c01, d1, d0);
-    e4m3x2_to_f32(c23, d3, d2);
-    x[0] -= d0 * back; x[1] -= d1 * back; x[2] -= d2 * back; x[3] -= d3 * back;      // residual, exact
-    const int n = term * HH + h;
-    *reinterpret_cast<uint32_t*>(smem + L::q_off + buf * 2048 + sw128(n, lane * 4)) = c01 | (c23 << 16);
-    if ((lane & 7) == 0) smem[L::sfq_off + buf * 512 + n * 16 + (lane >> 3)] = (uint8_t)code;
+    float amax[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) amax[i] = fmaxf(fmaxf(fabsf(x[i][0]), fabsf(x[i][1])), fmaxf(fabsf(x[i][2]), fabsf(x[i][3])));
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1)                                   // the 8 lanes of one 32-wide block of d
+#pragma unroll
+      for (int i = 0; i < N; ++i) amax[i] = fmaxf(amax[i], __shfl_xor_sync(0xffffffffu, amax[i], s));
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      uint32_t code = 127u;
+      float p2 = 1.0f;
+      if (amax[i] > 0.0f && amax[i] < 3.0e38f) block_scale<0>(amax[i], code, p2);
+      const float back = e8m0_to_f32(code);
+      const uint32_t c01 = cvt_e4m3x2(x[i][1] * p2, x[i][0] * p2), c23 = cvt_e4m3x2(x[i][3] * p2, x[i][2] * p2);
+      float d0, d1, d2, d3;
+      e4m3x2_to_f32(c01, d1, d0);
+      e4m3x2_to_f32(c23, d3, d2);
+      x[i][0] -= d0 * back; x[i][1] -= d1 * back; x[i][2] -= d2 * back; x[i][3] -= d3 * back;      // residual, exact
+      const int n = term * HH + h0 + i;
+      *reinterpret_cast<uint32_t*>(smem + L::q_off + buf * 2048 + sw128(n, lane * 4)) = c01 | (c23 << 16);
+      if ((lane & 7) == 0) smem[L::sfq_off + buf * 512 + n * 16 + (lane >> 3)] = (uint8_t)code;
+    }
   }
 }
 
@@ -607,7 +628,10 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
     if (lane == 0)
       for (int j = 0; j < n_early; ++j) issue_tile(j, seg.t0 + j);
   } else if (warp < HH) {                                             // first query terms: the only thing S waits for beside its tile
-    if (seg.left > 0) dtc_query_store<HH>(smem, dtc_query_load(p, seg.b, seg.hkv, warp, lane), warp, 0, lane);
+    if (seg.left > 0) {
+      const uint2 raw[1] = {dtc_query_load(p, seg.b, seg.hkv, warp, lane)};
+      dtc_query_store<HH, 1>(smem, raw, warp, 0, lane);
+    }
     fence_proxy_async_smem();
     asm volatile("bar.arrive 1, %0;" ::"n"((HH + 1) * 32) : "memory");
   }
@@ -619,20 +643,17 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
     for (; seg.left > 0 && ok; seg.next(p)) {
       for (int i = 0; i < seg.n && ok; ++i, ++j) {
         if (j < n_early) continue;
-        if (j >= kStages) ok = __all_sync(0xffffffffu, mbar_wait<20000>(&bars[L::bEmpty + j % kStages], (j / kStages - 1) & 1, abort_flag, p.status, 511));
+        if (j >= kStages) ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bEmpty + j % kStages], (j / kStages - 1) & 1, abort_flag, p.status, 511));
         if (ok && lane == 0) issue_tile(j, seg.t0 + i);
       }
     }
   } else if (warp == kWarpSf) {
-    // ================= key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32, in place; and the query terms of
-    // the next segment, loaded at the beginning of a segment and put down at its end =================
+    // ================= key scales [key][4] -> scale atom: word (key % 32) * 4 + key / 32, in place =================
     int j = 0;
-    for (int s = 0; seg.left > 0 && ok; ++s) {
-      DtcSegments next = seg;
-      uint2 nq[HH];
+    for (; seg.left > 0 && ok; seg.next(p)) {
       for (int i = 0; i < seg.n && ok; ++i, ++j) {
         const int st = j % kStages;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 527));
+        ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 527));
         if (!ok) break;
         uint32_t* ks = reinterpret_cast<uint32_t*>(smem + L::stage_off + st * kStageBytes + 2 * kTileBytes);
         uint32_t w[4];
@@ -643,24 +664,21 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[L::bKS + st]);
-        if (i == 0) {
-          next.next(p);
-          if (next.left > 0) {
-#pragma unroll
-            for (int h = 0; h < HH; ++h) nq[h] = dtc_query_load(p, next.b, next.hkv, h, lane);
-          }
-        }
       }
-      if (ok && next.left > 0) {
-        if (s >= 1) ok = __all_sync(0xffffffffu, mbar_wait(&bars[L::bQE + ((s + 1) & 1)], (((s + 1) >> 1) - 1) & 1, abort_flag, p.status, 512));
-        if (!ok) break;
+    }
+  } else if (warp == kWarpQ) {
+    // ================= query terms of every segment after the first, up to two segments ahead =================
+    if (seg.left > 0) seg.next(p);
+    for (int s = 1; seg.left > 0 && ok; ++s, seg.next(p)) {
+      uint2 raw[HH];
 #pragma unroll
-        for (int h = 0; h < HH; ++h) dtc_query_store<HH>(smem, nq[h], h, (s + 1) & 1, lane);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[L::bQF + ((s + 1) & 1)]);
-      }
-      seg = next;
+      for (int h = 0; h < HH; ++h) raw[h] = dtc_query_load(p, seg.b, seg.hkv, h, lane);
+      if (s >= 2) ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bQE + (s & 1)], ((s >> 1) - 1) & 1, abort_flag, p.status, 512));
+      if (!ok) break;
+      dtc_query_store<HH, HH>(smem, raw, 0, s & 1, lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[L::bQF + (s & 1)]);
     }
   } else if (warp == kWarpQk) {
     // ================= S^T = K Q^T (one lane) =================
@@ -672,16 +690,16 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
       tc_cp_32x128b_warpx4(tmem_base + cSfOne, make_smem_desc(smem_u32(smem + L::one_off), 0, 128, kLayoutNone));
       int j = 0;
       for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
-        if (s > 0) ok = mbar_wait(&bars[L::bQF + (s & 1)], (s & 1) ? (s >> 1) & 1 : ((s >> 1) - 1) & 1, abort_flag, p.status, 525);
+        if (s > 0) ok = dtc_wait(&bars[L::bQF + (s & 1)], (s & 1) ? (s >> 1) & 1 : ((s >> 1) - 1) & 1, abort_flag, p.status, 525);
         if (!ok) break;
         tc_cp_32x128b_warpx4(tmem_base + cSfQ + (s & 1) * 4, make_smem_desc(smem_u32(smem + L::sfq_off + (s & 1) * 512), 0, 128, kLayoutNone));
         const uint64_t dqs = dq + (uint32_t)((s & 1) * (2048 >> 4));
         for (int i = 0; i < seg.n && ok; ++i, ++j) {
           const int st = j % kStages, g = j & (kGroups - 1);
           // (the tile itself has landed: the scale warp waited for it; the second wait orders it for this thread)
-          ok = mbar_wait(&bars[L::bKS + st], (j / kStages) & 1, abort_flag, p.status, 528) &&
-               mbar_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 521);
-          if (ok && j >= kGroups) ok = mbar_wait(&bars[L::bSE + g], (j / kGroups - 1) & 1, abort_flag, p.status, 522);
+          ok = dtc_wait(&bars[L::bKS + st], (j / kStages) & 1, abort_flag, p.status, 528) &&
+               dtc_wait(&bars[L::bFull + st], (j / kStages) & 1, abort_flag, p.status, 521);
+          if (ok && j >= kGroups) ok = dtc_wait(&bars[L::bSE + g], (j / kGroups - 1) & 1, abort_flag, p.status, 522);
           if (!ok) break;
           tc_fence_after();
           const uint32_t so = (uint32_t)(st * (kStageBytes >> 4));
@@ -697,7 +715,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
     }
     if (lane == 0) {
       tc_commit(&bars[L::bDrain]);
-      mbar_wait(&bars[L::bDrain], 0, abort_flag, p.status, 524);
+      dtc_wait(&bars[L::bDrain], 0, abort_flag, p.status, 524);
     }
     __syncwarp();
   } else if (warp == kWarpPv) {
@@ -709,10 +727,10 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
       const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
       int j = 0;
       for (int s = 0; seg.left > 0 && ok; ++s, seg.next(p)) {
-        if (s >= kOBufs) ok = mbar_wait(&bars[L::bOE + s % kOBufs], (s / kOBufs - 1) & 1, abort_flag, p.status, 529);
+        if (s >= kOBufs) ok = dtc_wait(&bars[L::bOE + s % kOBufs], (s / kOBufs - 1) & 1, abort_flag, p.status, 529);
         for (int i = 0; i < seg.n && ok; ++i, ++j) {
           const int st = j % kStages, g = j & (kGroups - 1);
-          ok = mbar_wait(&bars[L::bPF + g], (j / kGroups) & 1, abort_flag, p.status, 523);
+          ok = dtc_wait(&bars[L::bPF + g], (j / kGroups) & 1, abort_flag, p.status, 523);
           if (!ok) break;
           tc_fence_after();
           tc_cp_32x128b_warpx4(tmem_base + cSfP + g * 4, dsfp + (uint32_t)(g * (512 >> 4)));
@@ -727,7 +745,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
         }
       }
       tc_commit(&bars[L::bDrain + 1]);
-      mbar_wait(&bars[L::bDrain + 1], 0, abort_flag, p.status, 526);
+      dtc_wait(&bars[L::bDrain + 1], 0, abort_flag, p.status, 526);
     }
     __syncwarp();
   } else {
