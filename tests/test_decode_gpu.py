@@ -256,15 +256,15 @@ def test_kv_cache_append_then_decode_in_a_loop(fmt):
     assert np.array_equal(np_(vc[0, 0, :T]), oc) and np.array_equal(np_(vs[0, 0, :T]), os_)
 
 
-@pytest.mark.parametrize("grp,case", [(4, "short"), (8, "short"), (4, "rising"), (8, "rising"), (4, "v jump"), (8, "v jump"), (1, "few tiles")])
+@pytest.mark.parametrize("grp,case", [(4, "short"), (8, "short"), (4, "many"), (8, "many"), (4, "rising"), (8, "rising"), (4, "v jump"), (8, "v jump"), (1, "few tiles")])
 def test_ranges_and_references(grp, case):
-    """The tcgen05 kernel's equal ranges of tiles and its running references: many short sequences per CTA (empty ones, single
-    keys and tile edges among them), fewer tiles than CTAs, scores that rise by far more than 2^32 over the keys and V block
+    """The tcgen05 kernel's equal ranges of tiles and its running references: a few and many short sequences per CTA (empty ones,
+    single keys and tile edges among them), fewer tiles than CTAs, scores that rise by far more than 2^32 over the keys and V block
     scales that do (O is then rescaled, again and again, while other tiles are in flight)."""
     Hkv, d = 2, 128
-    B, L = {"short": (71, 520), "rising": (2, 3000), "v jump": (2, 3000), "few tiles": (3, 132)}[case]
+    B, L = {"short": (71, 520), "many": (900, 260), "rising": (2, 3000), "v jump": (2, 3000), "few tiles": (3, 132)}[case]
     rng = np.random.default_rng(grp)
-    lens = rng.choice([0, 1, 127, 128, 129, 256, 384, 520], B).astype(np.int32) if case == "short" else np.array([L, 0, 5] if B == 3 else [L, L - 77], np.int32)
+    lens = rng.choice([n for n in (0, 1, 127, 128, 129, 256, 384, 520) if n <= L], B).astype(np.int32) if B > 3 else np.array([L, 0, 5] if B == 3 else [L, L - 77], np.int32)
     g = torch.Generator(device="cuda").manual_seed(grp)
     q = torch.randn(B, grp * Hkv, d, generator=g, device="cuda").bfloat16()
     K = torch.randn(B, Hkv, L, d, generator=g, device="cuda")
