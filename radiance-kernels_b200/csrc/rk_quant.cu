@@ -1293,7 +1293,8 @@ int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, 
   const dim3 grid(jobs.ctas + grid_for(units * kRebaseThreads, kRebaseThreads, 28)), block(kRebaseThreads);      // four waves of the resident CTAs
 #define RK_RB(TI, N) RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, TI, N>, grid, block, 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs))
   if (wide) { if (tiled) { RK_RB(true, 8); } else { RK_RB(false, 8); } }
-  else      { if (tiled) { RK_RB(true, 4); } else { RK_RB(false, 4); } }
+  else if (tiled) return RK_ERR_MISALIGNED;              // (prefill's codes and workspace lie on 16-byte boundaries)
+  else { RK_RB(false, 4); }
 #undef RK_RB
   return RK_OK;
 }

@@ -281,3 +281,39 @@ def test_stage_parity_s_and_requantized_p(d, qmul):
     m_gpu, l_gpu = ml[:, 0] * np.log(2.0), ml[:, 1]
     assert np.abs(m_gpu - r["m"][rows]).max() <= 4e-6 * np.abs(r["m"][rows]).max() + 1e-6
     assert np.abs(l_gpu / r["l"][rows] - 1.0).max() <= 1e-4
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Skv,d,kw", [
+    (1, 148, 4, 33, 160, 128, dict(causal=False)),                # 148 query tiles: one for every SM, a CTA each
+    (1, 149, 149, 33, 160, 128, dict(causal=False)),              # one more: a CTA takes two, here one that exists
+    (1, 50, 10, 300, 300, 64, dict(causal=True)),                 # three tiles of a head: the last pair has one
+    (3, 17, 17, 257, 257, 128, dict(causal=True, window=140)),
+    (2, 40, 8, 256, 400, 128, dict(causal=True, q_pos0=144, softcap=5.0)),
+    (1, 4, 4, 509, 700, 128, dict(causal=True, q_pos0=191, window=130, softcap=5.0)),
+    (1, 2, 1, 1, 129, 128, dict(causal=True, q_pos0=128)),        # one query, one key in the last key tile
+    (1, 2, 2, 130, 65, 64, dict(causal=True))])                   # keys of one half of a key tile, and one of the other
+def test_grids_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, Sq, Skv, d, kw):
+    """Grids of at most one query tile per SM put both softmax groups on one tile (64 keys each of every key tile), larger
+    ones give a CTA two tiles; odd numbers of tiles, masks that cut a key tile in either half."""
+    _check(prefill_vs_oracle(B, H, Hkv, Sq, Skv, d, seed=61, **kw))
+
+
+@pytest.mark.parametrize("fmt", [rk.E4M3, rk.E5M2, rk.E2M3, rk.E3M2, rk.E2M1])
+@pytest.mark.parametrize("S,d", [(31, 64), (129, 64), (333, 128), (160, 256)])
+def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
+    """V with scales along d, re-blocked (and for 6- and 4-bit codes packed and transposed) by the call, against the same V
+    re-blocked by the oracle and handed over with scales along the keys: bit for bit the same output, because the attention
+    kernel then reads the same operands.  Row scales that span 2^50 inside a block take the slow form."""
+    rng = np.random.default_rng(71 + fmt)
+    Q, K, V = randn_qkv(1, 3, 3, 140, S, d, seed=73)
+    qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V, fmt=fmt)
+    vs[0, 0] = torch.from_numpy(rng.integers(80, 131, size=(S, d // 32), dtype=np.uint8)).cuda()
+    vs[0, 1] = torch.from_numpy(rng.integers(122, 131, size=(S, d // 32), dtype=np.uint8)).cuda()
+    pairs = [oracle.rebase_v(np_(vc[0, h]), np_(vs[0, h]), fmt) for h in range(3)]
+    rc, rs = (torch.from_numpy(np.stack([x[i] for x in pairs])[None]).cuda() for i in range(2))
+    kw = dict(causal=False, q_fmt=fmt, kv_fmt=fmt)
+    got = rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+    want = rk.attn_prefill(qc, kc, rc, qs, ks, rs, v_scale_axis=rk.V_SCALES_ALONG_KEYS, **kw)
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+    assert torch.isfinite(want.float()).all() and torch.equal(got, want)

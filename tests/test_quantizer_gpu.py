@@ -225,3 +225,33 @@ def test_bf16_input_quantizer_equals_fp32_path(fmt):
     assert torch.equal(cb, cf) and torch.equal(sb, sf)
     oc, os_ = oracle.quantize(np_(x.float()), fmt=fmt)
     assert np.array_equal(np_(cb), oc) and np.array_equal(np_(sb), os_)
+
+
+@pytest.mark.parametrize("fmt", [rk.E4M3, rk.E3M2])
+@pytest.mark.parametrize("S,d", [(37, 32), (130, 64), (64, 96)])
+def test_rebase_of_codes_on_a_four_byte_boundary(S, d, fmt):
+    """Codes that start on a 4-byte boundary only take four columns a thread instead of eight."""
+    g = torch.Generator(device="cuda").manual_seed(81)
+    c0, s = rk.mx_quantize(torch.randn(2, S, d, generator=g, device="cuda"), fmt)
+    c = torch.empty(c0.numel() + 4, dtype=torch.uint8, device="cuda")[4:].view(c0.shape)
+    c.copy_(c0)
+    assert c.data_ptr() % 8 == 4
+    rc, rs = rk.mx_rebase_v(c, s, fmt)
+    for b in range(2):
+        oc, os_ = oracle.rebase_v(np_(c0[b]), np_(s[b]), fmt)
+        assert np.array_equal(np_(rc[b]), oc) and np.array_equal(np_(rs[b]), os_)
+
+
+@pytest.mark.parametrize("copies,S,d", [(37, 2051, 128), (2, 18945, 256)])
+def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
+    """Large inputs: two rows of one position share a thread's reads of the caches (an odd number of rows leaves one alone);
+    a NaN and an infinity in either of the two."""
+    rng = np.random.default_rng(83)
+    x = rng.standard_normal((copies, S, d), dtype=np.float32)
+    x[0, 3, 5], x[1, 7, d - 1], x[copies - 1, S - 1, d // 2] = np.nan, np.inf, -np.inf
+    ang = (np.arange(S)[:, None] * (10000.0 ** (-(np.arange(d // 2) * 2.0 / d)))[None, :]).astype(np.float32)
+    c, s = np.cos(ang), np.sin(ang)
+    codes, scales = rk.rope_mx_quantize(*(torch.from_numpy(a).cuda() for a in (x[None], c, s)))
+    y = oracle.rope(x.reshape(-1, d), np.tile(np.arange(S, dtype=np.int32), copies), c, s)
+    oc, os_ = oracle.quantize(y)
+    assert np.array_equal(np_(codes).reshape(-1, d), oc) and np.array_equal(np_(scales).reshape(-1, d // 32), os_)
