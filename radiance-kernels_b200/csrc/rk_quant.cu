@@ -624,16 +624,19 @@ template <int FMT> RK_DEVINL float decode_scaled(uint32_t c, uint32_t s) {
   return decode_elem<FMT>(c) * e8m0_to_f32(s);
 }
 
-// The slow form: a thread's NC columns of a block, element by element through fp32; keys k0 .. k0 + 7 are written.
+// The slow form: a thread's NC columns of a block, element by element through fp32; keys k0 .. k0 + 7 are written, and the
+// scale codes of NC / 4 columns from c0 on are returned.
 template <int FMT, int NC>
-__device__ __noinline__ void rebase_slow(const uint8_t* cb, const uint8_t* sb, int n, int k0, int64_t d, int64_t nbd, uint8_t* ob, uint32_t (&sc)[NC]) {
+__device__ __noinline__ void rebase_slow(const uint8_t* cb, const uint8_t* sb, int n, int k0, int64_t d, int64_t nbd, uint8_t* ob, int c0, uint32_t (&sc)[NC / 4]) {
 #pragma unroll 1
   for (int c = 0; c < NC; ++c) {
     float amax = 0.0f, p2 = 1.0f;
     uint32_t code = 0;
     for (int j = 0; j < n; ++j) amax = fmaxf(amax, fabsf(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd])));
     if (amax > 0.0f) block_scale<FMT>(amax, code, p2);
-    sc[c] = code;
+#pragma unroll
+    for (int h = 0; h < NC / 4; ++h)
+      if (c == c0 + h) sc[h] = code;
     for (int j = k0; j < min(n, k0 + 8); ++j) ob[j * d + c] = (uint8_t)encode_rne<FMT>(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd]) * p2);
   }
 }
@@ -816,51 +819,58 @@ __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8
         }
     }
     __syncwarp();                                                  // fac_sm has been read
-#pragma unroll
-    for (int i = 0; i < 2 * NW; ++i) {
-      m[i] = max_u16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
-      m[i] = max_u16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], 16));
-    }
-    uint32_t sc[NC], f[2 * NW];
-#pragma unroll
-    for (int q = 0; q < NC; ++q) sc[q] = 0x7Fu;                    // of columns and key blocks that do not exist: 2^0
-    if (in) {
-    const float unit = __uint_as_float((uint32_t)smax << 23);      // 2^(smax - 127)
-#pragma unroll
-    for (int i = 0; i < 2 * NW; ++i) {
-      f[i] = 0u;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float am = (h ? f16_hi(m[i]) : f16_lo(m[i])) * unit;
-        uint32_t code = 0; float p2;
-        int up = 0;                                                // log2 of the column's factor
-        if (am > 0.0f) { block_scale<FMT>(am, code, p2); up = (int)(__float_as_uint(p2) >> 23) - 254 + smax; }
-        hot = hot && up <= 15 && (FMT > 1 || am < __int_as_float(0x7f800000));      // (NaN and infinity encodings are numbers here)
-        sc[2 * i + h] = code;
-        f[i] |= (uint32_t)((15 + up) & 31) << (10 + 16 * h);
-      }
-    }
-    uint8_t* dst = out_codes + row0 * d + col;
-    if (hot) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (k0 + i >= n) break;
-        uint32_t o[NW];
-#pragma unroll
-        for (int q = 0; q < NW; ++q) o[q] = encode_f16x4<FMT>(hmul2(x[i][2 * q], f[2 * q]), hmul2(x[i][2 * q + 1], f[2 * q + 1]));
-        if (NC == 8) *reinterpret_cast<uint2*>(dst + (k0 + i) * d) = make_uint2(o[0], o[NW - 1]);
-        else *reinterpret_cast<uint32_t*>(dst + (k0 + i) * d) = o[0];
-      }
+    // The four lanes of a column group end up with the maxima of a quarter of its columns each, work out those scales and
+    // hand the factors back.
+    constexpr int CP = NC / 4;                                     // columns of a lane's quarter
+    const bool h16 = lane & 16, h8 = lane & 8;
+    uint32_t mine;
+    if (NC == 8) {
+      const uint32_t a = max_u16x2(h16 ? m[NW] : m[0], __shfl_xor_sync(0xffffffffu, h16 ? m[0] : m[NW], 16));
+      const uint32_t c = max_u16x2(h16 ? m[2 * NW - 1] : m[1], __shfl_xor_sync(0xffffffffu, h16 ? m[1] : m[2 * NW - 1], 16));
+      mine = max_u16x2(h8 ? c : a, __shfl_xor_sync(0xffffffffu, h8 ? a : c, 8));
     } else {
-      rebase_slow<FMT, NC>(src, scales + row0 * nbd + col / 32, n, k0, d, nbd, dst, sc);
+      mine = max_u16x2(h16 ? m[1] : m[0], __shfl_xor_sync(0xffffffffu, h16 ? m[0] : m[1], 16));
+      mine = max_u16x2(mine, __shfl_xor_sync(0xffffffffu, mine, 8));
+      if (h8) mine >>= 16;
     }
+    const float unit = __uint_as_float((uint32_t)smax << 23);      // 2^(smax - 127)
+    uint32_t sc[CP], fac = 0u, f[2 * NW];
+#pragma unroll
+    for (int h = 0; h < CP; ++h) {
+      const float am = (h ? f16_hi(mine) : f16_lo(mine)) * unit;
+      uint32_t code = 0; float p2;
+      int up = 0;                                                  // log2 of the column's factor
+      if (am > 0.0f) { block_scale<FMT>(am, code, p2); up = (int)(__float_as_uint(p2) >> 23) - 254 + smax; }
+      hot = hot && up <= 15 && (FMT > 1 || am < __int_as_float(0x7f800000));        // (NaN and infinity encodings are numbers here)
+      sc[h] = in ? code : 0x7Fu;                                   // of columns and key blocks that do not exist: 2^0
+      fac |= (uint32_t)((15 + up) & 31) << (10 + 16 * h);
+    }
+    hot = (__ballot_sync(0xffffffffu, !hot) & (0x01010101u << (lane & 7))) == 0u;
+#pragma unroll
+    for (int i = 0; i < 2 * NW; ++i) {
+      f[i] = __shfl_sync(0xffffffffu, fac, (lane & 7) + (NC == 8 ? 8 * i : 16 * i));
+      if (NC == 4) f[i] |= __shfl_sync(0xffffffffu, fac, (lane & 7) + 16 * i + 8) << 16;
+    }
+    if (in) {
+      uint8_t* dst = out_codes + row0 * d + col;
+      if (hot) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (k0 + i >= n) break;
+          uint32_t o[NW];
+#pragma unroll
+          for (int q = 0; q < NW; ++q) o[q] = encode_f16x4<FMT>(hmul2(x[i][2 * q], f[2 * q]), hmul2(x[i][2 * q + 1], f[2 * q + 1]));
+          if (NC == 8) *reinterpret_cast<uint2*>(dst + (k0 + i) * d) = make_uint2(o[0], o[NW - 1]);
+          else *reinterpret_cast<uint32_t*>(dst + (k0 + i) * d) = o[0];
+        }
+      } else {
+        rebase_slow<FMT, NC>(src, scales + row0 * nbd + col / 32, n, k0, d, nbd, dst, (lane >> 3) * CP, sc);
+      }
     }
     if (TILED) {
       // the four warps' scale bytes of a column are one word of its atom
-      if ((lane >> 3) == 0) {
 #pragma unroll
-        for (int q = 0; q < NC; ++q) sc_sm[((lane & 7) * NC + q) * 4 + warp] = (uint8_t)sc[q];
-      }
+      for (int h = 0; h < CP; ++h) sc_sm[((lane & 7) * NC + (lane >> 3) * CP + h) * 4 + warp] = (uint8_t)sc[h];
       __syncthreads();
       for (int c = threadIdx.x; c < 8 * NC; c += kRebaseThreads) {
         const int64_t n128 = cu * 8 * NC + c;
@@ -869,10 +879,8 @@ __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8
       }
       __syncthreads();
     } else if (in) {
-      // each of the four lanes of a column group writes a quarter of its scale codes
 #pragma unroll
-      for (int q = 0; q < NC; ++q)
-        if (q / (NC / 4) == (lane >> 3)) out_scales[(bt * nkb + kb) * d + col + q] = (uint8_t)sc[q];
+      for (int h = 0; h < CP; ++h) out_scales[(bt * nkb + kb) * d + col + (lane >> 3) * CP + h] = (uint8_t)sc[h];
     }
   }
 }
