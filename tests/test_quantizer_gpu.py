@@ -255,3 +255,8 @@ def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
     y = oracle.rope(x.reshape(-1, d), np.tile(np.arange(S, dtype=np.int32), copies), c, s)
     oc, os_ = oracle.quantize(y)
     assert np.array_equal(np_(codes).reshape(-1, d), oc) and np.array_equal(np_(scales).reshape(-1, d // 32), os_)
+
+
+def test_hardware_converter_of_the_four_bit_format_on_every_fp32():
+    """The same sweep for E2M1, whose converter packs two codes into a byte."""
+    test_hardware_converter_equals_reference_encoder_on_every_fp32(rk.E2M1)
