@@ -260,3 +260,23 @@ def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
 def test_hardware_converter_of_the_four_bit_format_on_every_fp32():
     """The same sweep for E2M1, whose converter packs two codes into a byte."""
     test_hardware_converter_equals_reference_encoder_on_every_fp32(rk.E2M1)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 4), (33, 36), (47, 100), (129, 64), (40, 160)])
+def test_quantize_keys_ragged_blocks(rows, cols):
+    """Blocks along the keys at ragged rows and columns, a zero column, NaN and infinity; row-major scales and atoms."""
+    rng = np.random.default_rng(91)
+    x = (rng.standard_normal((2, rows, cols)) * 2.0 ** rng.integers(-30, 30, size=(2, 1, cols))).astype(np.float32)
+    x[0, :, 1] = 0.0
+    x[1, rows - 1, cols - 1], x[1, 0, cols - 2], x[1, rows // 2, 0] = np.nan, -np.inf, np.inf
+    codes, scales = rk.mx_quantize_keys(torch.from_numpy(x).cuda())
+    codes2, atoms = rk.mx_quantize_keys_ex(torch.from_numpy(x).cuda(), rk.E4M3, rk.SCALES_SF_ATOMS)
+    assert torch.equal(codes, codes2)
+    a = np_(atoms).reshape(2, (rows + 127) // 128, (cols + 127) // 128, 512)
+    for b in range(2):
+        oc, os_ = oracle.quantize(x[b], axis=0)
+        assert np.array_equal(np_(codes[b]), oc) and np.array_equal(np_(scales[b]), os_)
+        for kb in range(os_.shape[0]):
+            for n in range(cols):
+                r = n % 128
+                assert a[b, kb // 4, n // 128, (r % 32) * 16 + r // 32 * 4 + kb % 4] == os_[kb, n]
