@@ -762,9 +762,9 @@ template <int FMT> RK_DEVINL uint32_t encode_f16x4(uint32_t lo, uint32_t hi) {
 }
 
 // A CTA = 128 keys x 8 NC columns at a time, a warp = 32 of the keys, a lane = 8 of them x NC adjacent columns, all its loads
-// in flight; the column maxima meet by two shuffles.  NC = 8, or 4 where the codes are not 8-byte aligned.
+// in flight; the column maxima meet by the shuffles of a reduce-scatter.  NC = 8, or 4 where the codes are not 8-byte aligned.
 // 67 M codes E4M3: 53 us in integer arithmetic on the codes (12 instructions per code, 16 warps per SM, rows with a zero or
-// subnormal code on a path of their own), 32 us here (36 beside the scales' re-tiling).
+// subnormal code on a path of their own), 30 us here (33 beside the scales' re-tiling).
 constexpr int kRebaseThreads = 128;
 template <int FMT, bool TILED, int NC>
 __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
