@@ -1026,7 +1026,8 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const PackJobs packs, in
 // flight.  In these formats zero and subnormal codes are common, which the integer form of the re-blocking kernel pays for
 // row by row.  Here as there the codes go through f16, and pairs of keys of one column go back through
 // the converter in the order in which they are packed.  The packed words meet in shared memory and leave in 16-byte stores.
-// 33.5 M codes E3M2: re-blocking 138 us and transposition 27 us as kernels of their own, 31 us here.
+// 33.5 M codes E3M2: re-blocking 138 us and transposition 27 us as kernels of their own, 31 us here.  (Seven CTAs per SM: eight spill
+// more registers, five and six leave too few loads in flight: 1 and 2 us slower.)
 // codes of four consecutive keys, packed
 template <int FMT> RK_DEVINL uint32_t encode_pack4(float a, float b, float c, float d) {
   uint32_t r;
@@ -1038,7 +1039,7 @@ template <int FMT> RK_DEVINL uint32_t encode_pack4(float a, float b, float c, fl
   return pack4<6>(hw_encode4<FMT>(a, b, c, d));
 }
 template <int FMT, bool REBASE>
-__global__ void __launch_bounds__(128, 8) pack_v_kernel(const uint8_t* __restrict__ in, const uint8_t* __restrict__ scales, int64_t S, int64_t d,
+__global__ void __launch_bounds__(128, 7) pack_v_kernel(const uint8_t* __restrict__ in, const uint8_t* __restrict__ scales, int64_t S, int64_t d,
                                                      int64_t Sp, uint8_t* __restrict__ out, uint8_t* __restrict__ atoms) {
   constexpr int BITS = FMT == 4 ? 4 : 6, kWords = BITS, kRow = 4 * kWords, kPitch = kRow + 1;   // words per key block, per column; pitch
   __shared__ uint32_t buf[128 * kPitch];
