@@ -33,10 +33,13 @@
 // tile took it 1100 cycles, as long as HBM), one prepares the query terms of the next segment (loading and quantizing eight
 // heads takes longer than a tile, so in another warp's stream it held back every short sequence).
 //   worker warp w: group w / 4, thread = key (w % 4) * 32 + lane of the tile for S and P, and column d of O^T.
-// p of a warp's 32 keys is relative to their own maximum rounded up to an integer m_w (log2 domain), which the block scale
-// undoes exactly: nothing in a tile waits for the other warps' maxima but the scale bytes.  O and the row sums are relative
-// to a reference m_ref, the first tile's largest m_w, that is handed from tile to tile; fp32 carries them while later maxima
-// stay below m_ref + 32 (and V scales below theirs), so O is rescaled about never.
+// p, O and the row sums are relative to a reference m_ref per head (and to one V scale per group of 32 columns): the first
+// tile's maximum, handed from tile to tile, and replaced by a tile's own maximum where that is more than 2^8 above it (V scales:
+// 2^32), so O is rescaled about never.  The p of the key that set the reference is 1, which two terms hold exactly: with the
+// weight on few keys it is the error of the largest p that counts.  (References that are integers, so that the codes need not
+// wait for the other warps' maxima, leave that p with the rounding of any other: errors of 6.0e-4 of the result instead of
+// 5.2e-4 with queries of four times unit variance, 5.8e-4 instead of 4.1e-4 with twelve times.)  A warp's block scale carries
+// the power of two of the largest p of its 32 keys.
 // A segment ends in the group of its last tile alone: it reads O (one of four accumulators, used in turn) and the row sums
 // the other warps left, while those are in the next segment's tiles.  (With a meeting of all workers at its end a segment
 // cost 5000 cycles, four tiles' time.)
@@ -65,7 +68,7 @@ constexpr int kNq = 16;                           // B rows of the QK^T MMA: ter
 constexpr int kTileBytes = kTile * kD;            // 16384
 constexpr int kStageBytes = 2 * kTileBytes + 2 * 512;   // K, V, K scales [128][4], V scales [128][4]
 constexpr int kOBufs = 4, kRing = 8;              // accumulators in turn; tiles whose references are kept
-constexpr float kBump = 32.0f;                    // rescale O when a maximum passes its reference by more than 2^this
+constexpr float kBump = 8.0f, kBumpV = 32.0f;     // rescale O when a maximum (a V scale) passes its reference by more than 2^this
 
 // Per head capacity HH (4 or 8): column n of the PV MMA = q * 2 HH + term * HH + h.
 template <int HH> struct Lay {
@@ -81,7 +84,7 @@ template <int HH> struct Lay {
   static constexpr int sfp_off = q_off + 2 * 2048;             // a 512-byte scale atom of P per group
   static constexpr int sfq_off = sfp_off + kGroups * 512;      // scale atoms of the query terms, [2 segments]
   static constexpr int one_off = sfq_off + 2 * 512;            // scale atom of ones (code 127) for V
-  static constexpr int xchg_off = one_off + 512;               // [groups][2][4 warps][16] floats: m_w of the heads, then svmax
+  static constexpr int xchg_off = one_off + 512;               // [groups][2][4 warps][16] floats: maxima of the heads, then svmax
   static constexpr int ring_off = xchg_off + kGroups * 2 * 4 * 16 * 4;  // [8 tiles][16] floats: references after a tile, same order
   static constexpr int ref_off = ring_off + kRing * 16 * 4;    // [16 warps][16] floats: the references a warp's sums are relative to
   static constexpr int seg_off = ref_off + kWorkers * 16 * 4;  // end of a segment: [kOBufs][16 warps][8] float2: sum, its reference
@@ -298,9 +301,9 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
       if (lane == 0) mbar_arrive(&bars[L::bSE + g]);
 
       // ---- scores, the warp's maxima ----------------------------------------------------------------------------
-      float s[HH], mw[HH];
+      float s[HH];
 #pragma unroll
-      for (int h = 0; h < HH; ++h) s[h] = __uint_as_float(c[h]) + __uint_as_float(c[HH + h]);
+      for (int h = 0; h < HH; ++h) s[h] = (__uint_as_float(c[h]) + __uint_as_float(c[HH + h])) * p.scale_log2;   // log2 domain
       const bool tail = (seg.t0 + i + 1) * kTile > seg.len;
       const bool valid = (seg.t0 + i) * kTile + kt < seg.len;
       if (tail && !valid) {
@@ -308,66 +311,21 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         for (int h = 0; h < HH; ++h) s[h] = NEG_INF;
         svw = 0u;
       }
-#pragma unroll
-      for (int h = 0; h < HH; ++h) mw[h] = fmaxf(ceilf(redux_max_f32(s[h]) * p.scale_log2), -1.0e30f);   // log2 domain
       uint32_t svmax[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) svmax[q] = redux_max_u32((svw >> (8 * q)) & 0xFFu);
       float* xw = xchg + par * 64 + wq * 16;
-      if (lane == 0) {
 #pragma unroll
-        for (int h = 0; h < HH; h += 4) *reinterpret_cast<float4*>(xw + h) = make_float4(mw[h], mw[h + 1], mw[h + 2], mw[h + 3]);
+      for (int h = 0; h < HH; h += 4) {
+        const float4 m = make_float4(redux_max_f32(s[h]), redux_max_f32(s[h + 1]), redux_max_f32(s[h + 2]), redux_max_f32(s[h + 3]));
+        if (lane == 0) *reinterpret_cast<float4*>(xw + h) = m;
+      }
+      if (lane == 0) {
         *reinterpret_cast<float4*>(xw + 8) = make_float4((float)svmax[0], (float)svmax[1], (float)svmax[2], (float)svmax[3]);
         mbar_arrive(&bars[L::bMX + g]);
       }
 
-      // ---- p = 2^(s - m_w + 8) in two terms; a word holds the codes of four heads --------------------------------------
-      uint32_t hi[HH / 4], lo[HH / 4];
-#pragma unroll
-      for (int h = 0; h < HH; h += 4) {
-        uint32_t ch[2], cl[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float& p0 = s[h + 2 * e];
-          float& p1 = s[h + 2 * e + 1];
-          p0 = ex2_approx(fmaf(p0, p.scale_log2, 8.0f - mw[h + 2 * e]));       // at most 2^8; masked keys give 0
-          p1 = ex2_approx(fmaf(p1, p.scale_log2, 8.0f - mw[h + 2 * e + 1]));
-          ch[e] = cvt_e4m3x2(p1, p0);
-          float a1, a0;
-          e4m3x2_to_f32(ch[e], a1, a0);
-          cl[e] = cvt_e4m3x2((p1 - a1) * 16.0f, (p0 - a0) * 16.0f);
-        }
-        hi[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
-        lo[h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
-      }
-      // the P tile is free once the P V that read it (the group's previous tile) has completed
-      if (j >= kGroups) {
-        ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
-        if (!ok) break;
-      }
-      uint32_t d8[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) d8[q] = min(svmax[q] - ((svw >> (8 * q)) & 0xFFu), 15u) * 0x08080808u;
-      if (HH == 8) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) =
-              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<false>(hi[HH / 4 - 1], d8[q]),
-                         e4m3x4_down<true>(lo[0], d8[q]), e4m3x4_down<true>(lo[HH / 4 - 1], d8[q]));
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; q += 2)
-          *reinterpret_cast<uint4*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4)) =
-              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
-                         e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
-      }
-      if (__builtin_expect(tail && !valid, 0)) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
-        uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) vrow[q] = make_uint4(0u, 0u, 0u, 0u);
-      }
-
-      // ---- references, scale bytes, row sums --------------------------------------------------------------------
+      // ---- references ---------------------------------------------------------------------------------------------
       ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504) &&
                                        (i == 0 || dtc_wait(&bars[L::bRef + (j - 1) % kRing], ((j - 1) / kRing) & 1, abort_flag, p.status, 507)));
       if (!ok) break;
@@ -375,9 +333,10 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         const float* xr = xchg + par * 64 + (lane >> 4) * 32 + item;
         float top = fmaxf(xr[0], xr[16]);
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+        top = fmaxf(top, -1.0e30f);
         const float before = i == 0 ? top : ring[((j - 1) % kRing) * 16 + item];
         // every warp of the group sees the same maxima and references, so this is uniform over the group
-        const bool bump = __any_sync(0xffffffffu, top > before + kBump);
+        const bool bump = __any_sync(0xffffffffu, top > before + (item < 8 ? kBump : kBumpV));
         const float now = bump ? fmaxf(before, top) : before;
         if (wq == 0) {
           if (lane < 16) ring[(j % kRing) * 16 + lane] = now;
@@ -415,22 +374,68 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
           __syncwarp();
         }
       }
-      // steps from the reference to this warp's own maxima: at most 32 each; far below it the product vanishes anyway
-      const int step = __float2int_rn(fmaxf(xw[item] - ref_item, -200.0f));
+      // ---- p = 2^(s - m_ref), scaled into [2^7, 2^8) by the warp's largest, in two terms; a word holds the codes of four heads ----
+      // (s is rounded before m_ref is taken off: with one rounding for both, as fmaf has, the largest p of scores beyond 2^24
+      // would not be 1.)
+      // Steps from the references to this warp's own maxima: heads at most 9, V scales at most 32; far below, the product vanishes.
+      const int eh = max((int)(__float_as_uint(ex2_approx(xw[item] - ref_item)) >> 23), 7);
+      const int step = item < 8 ? eh - 126 : __float2int_rn(fmaxf(xw[item] - ref_item, -200.0f));
       const int step_h = __shfl_sync(0xffffffffu, step, lane & (HH - 1));
+      const float scale_up = __uint_as_float((uint32_t)(261 - eh) << 23);              // 2^(8 - step)
+      uint32_t hi[HH / 4], lo[HH / 4];
+#pragma unroll
+      for (int h = 0; h < HH; h += 4) {
+        const float4 m4 = *reinterpret_cast<const float4*>(ref + h);
+        const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+        uint32_t ch[2], cl[2];
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          float p0 = ex2_approx(s[h + e] - m[e]);                  // masked keys give 0
+          float p1 = ex2_approx(s[h + e + 1] - m[e + 1]);
+          l_part[h + e] += p0;
+          l_part[h + e + 1] += p1;
+          p0 *= __shfl_sync(0xffffffffu, scale_up, h + e);
+          p1 *= __shfl_sync(0xffffffffu, scale_up, h + e + 1);
+          ch[e / 2] = cvt_e4m3x2(p1, p0);
+          float a1, a0;
+          e4m3x2_to_f32(ch[e / 2], a1, a0);
+          cl[e / 2] = cvt_e4m3x2((p1 - a1) * 16.0f, (p0 - a0) * 16.0f);
+        }
+        hi[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
+        lo[h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
+      }
+      // the P tile is free once the P V that read it (the group's previous tile) has completed
+      if (j >= kGroups) {
+        ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
+        if (!ok) break;
+      }
+      uint32_t d8[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) d8[q] = min(svmax[q] - ((svw >> (8 * q)) & 0xFFu), 15u) * 0x08080808u;
+      if (HH == 8) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) =
+              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<false>(hi[HH / 4 - 1], d8[q]),
+                         e4m3x4_down<true>(lo[0], d8[q]), e4m3x4_down<true>(lo[HH / 4 - 1], d8[q]));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; q += 2)
+          *reinterpret_cast<uint4*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4)) =
+              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
+                         e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
+      }
+      if (__builtin_expect(tail && !valid, 0)) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
+        uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) vrow[q] = make_uint4(0u, 0u, 0u, 0u);
+      }
+
 #pragma unroll
       for (int part = 0; part < L::kNp / 32; ++part) {          // block scale of column n for this warp's 32 keys (k-block = wq)
         const int n = part * 32 + lane, q = n / (2 * HH), term = (n / HH) & 1;
         const int code = min(max(127 + step_h + __shfl_sync(0xffffffffu, step, 8 + q), 5), 254) - 4 * term;
         smem[L::sfp_off + g * 512 + lane * 16 + part * 4 + wq] = (uint8_t)code;
-      }
-#pragma unroll
-      for (int h = 0; h < HH; h += 4) {
-        const float4 m = *reinterpret_cast<const float4*>(ref + h);
-        l_part[h] = fmaf(s[h], ex2_approx(mw[h] - m.x - 8.0f), l_part[h]);
-        l_part[h + 1] = fmaf(s[h + 1], ex2_approx(mw[h + 1] - m.y - 8.0f), l_part[h + 1]);
-        l_part[h + 2] = fmaf(s[h + 2], ex2_approx(mw[h + 2] - m.z - 8.0f), l_part[h + 2]);
-        l_part[h + 3] = fmaf(s[h + 3], ex2_approx(mw[h + 3] - m.w - 8.0f), l_part[h + 3]);
       }
       fence_proxy_async_smem();
       tc_fence_before();

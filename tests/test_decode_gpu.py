@@ -288,3 +288,56 @@ def test_ranges_and_references(grp, case):
     full = lens > 0
     assert np.abs(np_(lse)[full] - ref["lse"][full]).max() < 2e-3
     assert (got[~full] == 0).all()
+
+
+@pytest.mark.parametrize("grp,kmul,lens", [(4, 1.0, [1, 1, 1, 1]), (8, 300.0, [3000, 1000, 129, 2]), (4, 3.0e7, [3000, 1000, 129, 1]), (1, 1.0e9, [3000, 700, 300, 5])])
+def test_a_key_with_all_the_weight_gives_its_v_row_exactly(grp, kmul, lens):
+    """One key is all a row sees, or its score lies 30 above every other one (scores up to 1e10): the p of the largest score is 1,
+    which the two MXFP8 terms of P hold exactly, so O is the key's decoded V, bit for bit (an E4M3 code times a power of two is
+    a bf16; the other keys add less than e^-30)."""
+    B, Hkv, L, d = len(lens), 2, max(lens) // 4 * 4 + 4, 128
+    g = torch.Generator(device="cuda").manual_seed(grp)
+    q = torch.randn(B, grp * Hkv, d, generator=g, device="cuda").bfloat16()
+    kc, ks, vc, vs = _quantized_cache(B, Hkv, L, seed=50 + grp, kmul=kmul)
+    o = rk.attn_decode(q, kc, vc, ks, vs, kv_len=torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+    k, v = _decoded(kc, ks), _decoded(vc, vs)
+    seen = 0
+    for b in range(B):
+        s = torch.einsum("hgd,hkd->hgk", q[b].double().view(Hkv, grp, d), k[b, :, :lens[b]]) * d ** -0.5
+        top, at = s.topk(min(2, lens[b]), -1)
+        for h in range(Hkv):
+            for x in range(grp):
+                if lens[b] == 1 or top[h, x, 0] - top[h, x, 1] > 30:
+                    seen += 1
+                    assert torch.equal(o[b, h * grp + x].double(), v[b, h, at[h, x, 0]]), (b, h, x)
+    assert seen >= B * Hkv * grp // 2
+
+
+def _decoded(codes, scales):
+    return codes.view(torch.float8_e4m3fn).double() * torch.exp2(scales.double() - 127).repeat_interleave(32, -1)
+
+
+def _error_beyond_rounding(o, q, kc, ks, vc, vs):
+    """Relative 2-norm of O's error against 64 bits, and what of it exceeds that of rounding the exact O to bf16."""
+    (B, H, d), Hkv = q.shape, kc.shape[1]
+    want = torch.empty(B, H, d, dtype=torch.float64, device="cuda")
+    for b in range(B):
+        s = torch.einsum("hgd,hkd->hgk", q[b].double().view(Hkv, H // Hkv, d), _decoded(kc[b], ks[b])) * d ** -0.5
+        want[b] = torch.einsum("hgk,hkd->hgd", torch.softmax(s, -1), _decoded(vc[b], vs[b])).reshape(H, d)
+    rel = float((o.double() - want).norm() / want.norm())
+    rounding = float((want.float().bfloat16().double() - want).norm() / want.norm())
+    return rel, max(rel ** 2 - rounding ** 2, 0.0) ** 0.5
+
+
+@pytest.mark.parametrize("grp", [4, 8])
+def test_error_of_peaked_rows(grp):
+    """Queries of twelve times unit variance: most of the weight lies on a key or two, and its error is that of their p.  Beyond
+    the rounding of O to bf16 there are 4.1e-4 with the p of the largest score exact (5.8e-4 with one rounded like all others)."""
+    g = torch.Generator(device="cuda").manual_seed(51)
+    q = (torch.randn(32, 8 * grp, 128, generator=g, device="cuda") * 12.0).bfloat16()
+    kc, ks, vc, vs = _quantized_cache(32, 8, 4096, seed=52)
+    rel, beyond = _error_beyond_rounding(rk.attn_decode(q, kc, vc, ks, vs), q, kc, ks, vc, vs)
+    assert rk.last_device_status() == 0
+    assert beyond <= 5.0e-4, (rel, beyond)
