@@ -20,7 +20,7 @@
 // folded into P: column (q, term, h) of B carries p[h][key] * 2^(sv[key][q] - svmax[q]), and its block scale carries
 // svmax[q] (the largest V scale among the block's 32 keys) and the exponent of the block's largest p.  A power of two
 // moves an E4M3 code by 8 per step, so a key's p is converted once per head and the four groups' codes are byte
-// subtractions on packed words.  Row d of O^T only uses the columns of its own group q = d / 32.
+// subtractions on packed words (where the V scales of a block lie more than kFarOctaves apart: once per head and group).  Row d of O^T only uses the columns of its own group q = d / 32.
 //
 // One CTA per SM, and the CTAs share the key tiles of the whole call evenly: the tiles of all sequences in a row (each
 // sequence as long as it is) are cut into as many equal ranges as there are CTAs.  A range is a list of segments, each a
@@ -68,6 +68,7 @@ constexpr int kNq = 16;                           // B rows of the QK^T MMA: ter
 constexpr int kTileBytes = kTile * kD;            // 16384
 constexpr int kStageBytes = 2 * kTileBytes + 2 * 512;   // K, V, K scales [128][4], V scales [128][4]
 constexpr int kOBufs = 4, kRing = 8;              // accumulators in turn; tiles whose references are kept
+constexpr uint32_t kFarOctaves = 4;               // V scales further below their block's largest are not taken by moving codes
 constexpr float kBump = 8.0f, kBumpV = 32.0f;     // rescale O when a maximum (a V scale) passes its reference by more than 2^this
 
 // Per head capacity HH (4 or 8): column n of the PV MMA = q * 2 HH + term * HH + h.
@@ -246,6 +247,15 @@ RK_DEVINL bool dtc_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag
   report_wait_failure(abort_flag, status, code);
   return false;
 }
+// bit 7 of every byte that is at least N (1 .. 128)
+template <uint32_t N> RK_DEVINL uint32_t bytes_at_least(uint32_t w) { return (((w & 0x7F7F7F7Fu) + (128u - N) * 0x01010101u) | w) & 0x80808080u; }
+// p = hi + lo / 16 in E4M3, two heads at a time: bits 15:8 of the codes = p1, bits 7:0 = p0
+RK_DEVINL void p_terms(float p1, float p0, uint32_t& hi, uint32_t& lo) {
+  hi = cvt_e4m3x2(p1, p0);
+  float a1, a0;
+  e4m3x2_to_f32(hi, a1, a0);
+  lo = cvt_e4m3x2((p1 - a1) * 16.0f, (p0 - a0) * 16.0f);
+}
 // Four packed E4M3 codes divided by 2^(d / 8): d8 = d in every byte, d a multiple of 8 up to 120.  Codes that leave the
 // normal range become 0 (or lose their hidden bit), an absolute error of 2^-15 of the block's largest element.  SIGN: codes
 // may be negative.
@@ -325,6 +335,10 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         mbar_arrive(&bars[L::bMX + g]);
       }
 
+      // octaves from each V scale to its block's largest; is one far (scale code 0 is a block of zeros)?
+      const uint32_t dw = (svmax[0] | (svmax[1] << 8) | (svmax[2] << 16) | (svmax[3] << 24)) - svw;
+      const bool far = __any_sync(0xffffffffu, (bytes_at_least<kFarOctaves + 1>(dw) & bytes_at_least<1>(svw)) != 0u);
+
       // ---- references ---------------------------------------------------------------------------------------------
       ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bMX + g], par, abort_flag, p.status, 504) &&
                                        (i == 0 || dtc_wait(&bars[L::bRef + (j - 1) % kRing], ((j - 1) / kRing) & 1, abort_flag, p.status, 507)));
@@ -335,33 +349,32 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
         top = fmaxf(top, -1.0e30f);
         const float before = i == 0 ? top : ring[((j - 1) % kRing) * 16 + item];
-        // every warp of the group sees the same maxima and references, so this is uniform over the group
-        const bool bump = __any_sync(0xffffffffu, top > before + (item < 8 ? kBump : kBumpV));
-        const float now = bump ? fmaxf(before, top) : before;
+        // every warp of the group sees the same maxima and references, so what follows is uniform over the group
+        const float now = top > before + (item < 8 ? kBump : kBumpV) ? top : before;
         if (wq == 0) {
           if (lane < 16) ring[(j % kRing) * 16 + lane] = now;
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bRef + j % kRing]);
         }
-        if (__builtin_expect(bump, 0)) {
-          // rescale this thread's row of O once the tile before has been added; its own P V comes after this
-          ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + ((j - 1) & (kGroups - 1))], ((j - 1) / kGroups) & 1, abort_flag, p.status, 502));
-          if (!ok) break;
-          tc_fence_after();
-          uint32_t o[2 * HH];
-          if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
-          tc_wait_ld();
-          const float down = before - now, down_v = __shfl_sync(0xffffffffu, down, 8 + wq);
-#pragma unroll
-          for (int h = 0; h < HH; ++h) {
-            const float f = ex2_approx(fmaxf(__shfl_sync(0xffffffffu, down, h) + down_v, -126.0f));
-            o[h] = __float_as_uint(__uint_as_float(o[h]) * f);
-            o[HH + h] = __float_as_uint(__uint_as_float(o[HH + h]) * f);
-          }
-          if (HH == 8) tmem_st16(o_addr, o); else tmem_st8(o_addr, o);
-          tc_wait_st();
-        }
         if (i == i_first || __any_sync(0xffffffffu, now != ref_item)) {
+          if (__any_sync(0xffffffffu, now != before)) {
+            // rescale this thread's row of O once the tile before has been added; its own P V comes after this
+            ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + ((j - 1) & (kGroups - 1))], ((j - 1) / kGroups) & 1, abort_flag, p.status, 502));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t o[2 * HH];
+            if (HH == 8) tmem_ld16(o_addr, o); else tmem_ld8(o_addr, o);
+            tc_wait_ld();
+            const float down = before - now, down_v = __shfl_sync(0xffffffffu, down, 8 + wq);
+#pragma unroll
+            for (int h = 0; h < HH; ++h) {
+              const float f = ex2_approx(fmaxf(__shfl_sync(0xffffffffu, down, h) + down_v, -126.0f));
+              o[h] = __float_as_uint(__uint_as_float(o[h]) * f);
+              o[HH + h] = __float_as_uint(__uint_as_float(o[HH + h]) * f);
+            }
+            if (HH == 8) tmem_st16(o_addr, o); else tmem_st8(o_addr, o);
+            tc_wait_st();
+          }
           // first tile of the segment here, or a reference moved here or in another group: this warp's sums follow
           if (i != i_first) {
             const float down = ref_item - now;
@@ -390,16 +403,14 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         uint32_t ch[2], cl[2];
 #pragma unroll
         for (int e = 0; e < 4; e += 2) {
-          float p0 = ex2_approx(s[h + e] - m[e]);                  // masked keys give 0
-          float p1 = ex2_approx(s[h + e + 1] - m[e + 1]);
+          float &p0 = s[h + e], &p1 = s[h + e + 1];
+          p0 = ex2_approx(p0 - m[e]);                              // masked keys give 0
+          p1 = ex2_approx(p1 - m[e + 1]);
           l_part[h + e] += p0;
           l_part[h + e + 1] += p1;
           p0 *= __shfl_sync(0xffffffffu, scale_up, h + e);
           p1 *= __shfl_sync(0xffffffffu, scale_up, h + e + 1);
-          ch[e / 2] = cvt_e4m3x2(p1, p0);
-          float a1, a0;
-          e4m3x2_to_f32(ch[e / 2], a1, a0);
-          cl[e / 2] = cvt_e4m3x2((p1 - a1) * 16.0f, (p0 - a0) * 16.0f);
+          p_terms(p1, p0, ch[e / 2], cl[e / 2]);
         }
         hi[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
         lo[h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
@@ -409,21 +420,42 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         ok = __all_sync(0xffffffffu, dtc_wait(&bars[L::bPV + g], par ^ 1, abort_flag, p.status, 503));
         if (!ok) break;
       }
-      uint32_t d8[4];
+      // A code moved down loses what falls below the normal range, 2^-15 of the block's largest element: nothing while the V scales
+      // of its keys lie close together, but all of a heavy key whose scale lies far below that of a light one.  Blocks with
+      // such keys are converted again for every group of columns, which rounds into the subnormals.
+      if (__builtin_expect(!far, 1)) {
+        uint32_t d8[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) d8[q] = min(svmax[q] - ((svw >> (8 * q)) & 0xFFu), 15u) * 0x08080808u;
-      if (HH == 8) {
+        for (int q = 0; q < 4; ++q) d8[q] = min((dw >> (8 * q)) & 0xFFu, 15u) * 0x08080808u;
+        if (HH == 8) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) =
-              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<false>(hi[HH / 4 - 1], d8[q]),
-                         e4m3x4_down<true>(lo[0], d8[q]), e4m3x4_down<true>(lo[HH / 4 - 1], d8[q]));
+          for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) =
+                make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<false>(hi[HH / 4 - 1], d8[q]),
+                           e4m3x4_down<true>(lo[0], d8[q]), e4m3x4_down<true>(lo[HH / 4 - 1], d8[q]));
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; q += 2)
+            *reinterpret_cast<uint4*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4)) =
+                make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
+                           e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
+        }
       } else {
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const float f = __uint_as_float((127u - min((dw >> (8 * q)) & 0xFFu, 127u)) << 23);
+          uint32_t w[2 * HH / 4];                                   // hi words, then lo words
 #pragma unroll
-        for (int q = 0; q < 4; q += 2)
-          *reinterpret_cast<uint4*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4)) =
-              make_uint4(e4m3x4_down<false>(hi[0], d8[q]), e4m3x4_down<true>(lo[0], d8[q]),
-                         e4m3x4_down<false>(hi[0], d8[q + 1]), e4m3x4_down<true>(lo[0], d8[q + 1]));
+          for (int h = 0; h < HH; h += 4) {
+            uint32_t ch[2], cl[2];
+            p_terms(s[h + 1] * f, s[h] * f, ch[0], cl[0]);
+            p_terms(s[h + 3] * f, s[h + 2] * f, ch[1], cl[1]);
+            w[h / 4] = __byte_perm(ch[0], ch[1], 0x5410);
+            w[HH / 4 + h / 4] = __byte_perm(cl[0], cl[1], 0x5410);
+          }
+          if (HH == 8) *reinterpret_cast<uint4*>(prow + (((chunk0 + q) ^ (kt & 7)) << 4)) = make_uint4(w[0], w[1], w[HH / 4], w[2 * HH / 4 - 1]);
+          else *reinterpret_cast<uint2*>(prow + (((chunk0 + q / 2) ^ (kt & 7)) << 4) + (q & 1) * 8) = make_uint2(w[0], w[HH / 4]);
+        }
       }
       if (__builtin_expect(tail && !valid, 0)) {   // a key past kv_len: its V row may hold anything; 0 * NaN must not reach the accumulator
         uint4* vrow = reinterpret_cast<uint4*>(sb + kTileBytes + kt * 128);

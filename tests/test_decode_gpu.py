@@ -341,3 +341,25 @@ def test_error_of_peaked_rows(grp):
     rel, beyond = _error_beyond_rounding(rk.attn_decode(q, kc, vc, ks, vs), q, kc, ks, vc, vs)
     assert rk.last_device_status() == 0
     assert beyond <= 5.0e-4, (rel, beyond)
+
+
+@pytest.mark.parametrize("grp", [4, 8])
+@pytest.mark.parametrize("octaves,bound", [(4, 7e-4), (5, 7e-4), (8, 7e-4), (12, 4.5e-3)])
+def test_error_where_light_keys_have_the_large_v_scales(octaves, bound, grp):
+    """One key in 32 has V scales some octaves above the others' and next to no weight: the weights of the others, moved down by
+    those octaves, must keep their bits.  Two E4M3 terms reach down to 2^-22 of a block's largest element; the errors beyond
+    rounding that this leaves are 6.1e-4, 6.1e-4, 6.2e-4 and 3.6e-3 (codes moved without rounding into the subnormals, 2^-15: 6.1e-4,
+    8e-4, 1.4e-2, 0.31)."""
+    g = torch.Generator(device="cuda").manual_seed(53)
+    B, Hkv, L, d = 32, 8, 1024, 128
+    q = torch.randn(B, Hkv * grp, d, generator=g, device="cuda").bfloat16()
+    K, V = (torch.randn(B, Hkv, L, d, generator=g, device="cuda") for _ in range(2))
+    first = q.view(B, Hkv, grp, d)[:, :, :1]                       # of every group of heads: the one the light keys are made for
+    K[:, :, ::32] -= 3.0 * first.float()
+    V[:, :, ::32] *= 2.0 ** octaves
+    kc, ks = rk.mx_quantize(K)
+    vc, vs = rk.mx_quantize(V)
+    o = rk.attn_decode(q, kc, vc, ks, vs).view(B, Hkv, grp, d)[:, :, 0]
+    assert rk.last_device_status() == 0
+    rel, beyond = _error_beyond_rounding(o, first[:, :, 0], kc, ks, vc, vs)
+    assert beyond <= bound, (rel, beyond)
