@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(128) rope_quantize_rows_kernel(const float* __
   grid_dependency_wait();
   grid_dependents_launch();
   const bool finite = rope_rows<FMT, U, false>(x, rows, d, pos, seq_len, pos0, cos_h, sin_h, codes, scales);
-  if (__syncthreads_or(!finite)) rope_rows<FMT, 1, true>(x, rows, d, pos, seq_len, pos0, cos_h, sin_h, codes, scales);
+  if (__syncthreads_or(!finite)) rope_rows<FMT, U, true>(x, rows, d, pos, seq_len, pos0, cos_h, sin_h, codes, scales);      // the same rows
 }
 
 // RMSNorm fused with the block quantizer: the prologue of the QKV projection (kernels/rmsnorm_qkv_fused), so that the

@@ -245,7 +245,7 @@ def test_rebase_of_codes_on_a_four_byte_boundary(S, d, fmt):
 @pytest.mark.parametrize("copies,S,d", [(37, 2051, 128), (2, 18945, 256)])
 def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
     """Large inputs: two rows of one position share a thread's reads of the caches (an odd number of rows leaves one alone);
-    a NaN and an infinity in either of the two."""
+    a NaN in the first row of a pair, infinities in others."""
     rng = np.random.default_rng(83)
     x = rng.standard_normal((copies, S, d), dtype=np.float32)
     x[0, 3, 5], x[1, 7, d - 1], x[copies - 1, S - 1, d // 2] = np.nan, np.inf, -np.inf
@@ -255,6 +255,24 @@ def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
     y = oracle.rope(x.reshape(-1, d), np.tile(np.arange(S, dtype=np.int32), copies), c, s)
     oc, os_ = oracle.quantize(y)
     assert np.array_equal(np_(codes).reshape(-1, d), oc) and np.array_equal(np_(scales).reshape(-1, d // 32), os_)
+
+
+@pytest.mark.parametrize("fmt", [rk.E4M3, rk.E5M2, rk.E2M3, rk.E3M2, rk.E2M1])
+def test_rope_quantize_nan_in_each_row_of_a_pair(fmt):
+    """A NaN in the first and in the second row of a pair, in later pairs, in the odd row left alone, at the ends of a row and of
+    the input: the block it lies in (and its partner in the other half) takes the form that leaves NaNs out of the maximum, the
+    other elements of the block keep their codes, and no other row changes."""
+    copies, S, d = 37, 2051, 128
+    rng = np.random.default_rng(84)
+    x = rng.standard_normal((copies, S, d), dtype=np.float32)
+    for at in ((0, 0, 0), (1, 7, d - 1), (1, S - 1, 40), (2, 1000, 64), (17, 1025, 9), (18, S // 2, 63), (35, 3, 100), (copies - 1, 0, 31), (copies - 1, S - 1, 0)):
+        x[at] = np.nan
+    ang = (np.arange(S)[:, None] * (10000.0 ** (-(np.arange(d // 2) * 2.0 / d)))[None, :]).astype(np.float32)
+    c, s = np.cos(ang), np.sin(ang)
+    codes, scales = rk.rope_mx_quantize(*(torch.from_numpy(a).cuda() for a in (x, c, s)), fmt=fmt)
+    y = oracle.rope(x.reshape(-1, d), np.tile(np.arange(S, dtype=np.int32), copies), c, s)
+    oc, os_ = oracle.quantize(y, fmt=fmt)
+    assert np.array_equal(np_(scales).reshape(-1, d // 32), os_) and np.array_equal(np_(codes).reshape(-1, d), oc)
 
 
 def test_hardware_converter_of_the_four_bit_format_on_every_fp32():
