@@ -527,13 +527,13 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
     l += f * ml_sm[w].y;
     acc.x += f * a.x; acc.y += f * a.y; acc.z += f * a.z; acc.w += f * a.w;
   }
-  const float inv = l > 0.0f ? 1.0f / l : 1.0f;
+  const float inv = dtc_inverse(l);
   const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
   uint2 out;
   out.x = *reinterpret_cast<const uint32_t*>(&lo);
   out.y = *reinterpret_cast<const uint32_t*>(&hi);
   *reinterpret_cast<uint2*>(p.o + (size_t)bh * 128 + lane * 4) = out;
-  if (p.lse && lane == 0) p.lse[bh] = l > 0.0f ? top * 0.6931471805599453f + logf(l) : NEG_INF;
+  if (p.lse && lane == 0) p.lse[bh] = dtc_lse(top, l);
 }
 
 // Which kernel serves a call: the tcgen05 kernel handles d = 128 with up to 8 query heads per KV head; everything

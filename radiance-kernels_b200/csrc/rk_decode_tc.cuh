@@ -126,6 +126,10 @@ struct DecodeTcParams {
 };
 
 RK_DEVINL int dtc_len(const DecodeTcParams& p, int b) { return p.kv_len ? min(max(p.kv_len[b], 0), p.L) : p.L; }
+// 1 / l and the log-sum-exp.  l is 0 without keys; a NaN score makes it NaN and must reach every column of O: the codes of a NaN p
+// that were moved down are numbers.
+RK_DEVINL float dtc_inverse(float l) { return l == 0.0f ? 1.0f : 1.0f / l; }
+RK_DEVINL float dtc_lse(float m, float l) { return l == 0.0f ? __int_as_float(0xff800000) : m * 0.6931471805599453f + logf(l); }
 RK_DEVINL int dtc_tiles(int len) { return (len + dtc::kTile - 1) / dtc::kTile; }
 // first tile of CTA c of g when t tiles are shared evenly
 RK_DEVINL int dtc_first(int t, int c, int g) {
@@ -539,8 +543,8 @@ RK_DEVINL void decode_tc_worker(const DecodeTcParams& p, uint8_t* smem, uint64_t
         if (h < p.grp) {
           const float acc = (__uint_as_float(o[h]) + __uint_as_float(o[HH + h])) * back * back2, m = ref[h];
           if (whole) {
-            p.o[(bh0 + h) * 128 + kt] = __float2bfloat16_rn(acc * (lh > 0.0f ? 1.0f / lh : 1.0f));
-            if (p.lse && kt == 0) p.lse[bh0 + h] = lh > 0.0f ? m * 0.6931471805599453f + logf(lh) : NEG_INF;
+            p.o[(bh0 + h) * 128 + kt] = __float2bfloat16_rn(acc * dtc_inverse(lh));
+            if (p.lse && kt == 0) p.lse[bh0 + h] = dtc_lse(m, lh);
           } else {
             const size_t at = p.nsplit > 0 ? (bh0 + h) * p.nsplit + blockIdx.x % p.nsplit
                                            : ((size_t)blockIdx.x * 2 + (seg.t0 > 0 ? 0 : 1)) * p.grp + h;

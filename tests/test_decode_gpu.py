@@ -363,3 +363,35 @@ def test_error_where_light_keys_have_the_large_v_scales(octaves, bound, grp):
     assert rk.last_device_status() == 0
     rel, beyond = _error_beyond_rounding(o, first[:, :, 0], kc, ks, vc, vs)
     assert beyond <= bound, (rel, beyond)
+
+
+@pytest.mark.parametrize("fmt,code", [(rk.E4M3, 0x7F), (rk.E4M3, 0xFF), (rk.E5M2, 0x7C), (rk.E5M2, 0x7F)])
+@pytest.mark.parametrize("grp,num_splits", [(4, 0), (8, 0), (4, 3)])
+def test_a_nan_score_reaches_every_column(grp, num_splits, fmt, code):
+    """One key inside kv_len with a NaN (or, in E5M2, an infinity) among its codes and V scales below its neighbours': the score is
+    no number, so no column of O is one, nor the log-sum-exp, wherever the unit's tiles were cut; other units are untouched."""
+    B, Hkv, L, d = 3, 2, 3000, 128
+    g = torch.Generator(device="cuda").manual_seed(57)
+    q = torch.randn(B, Hkv * grp, d, generator=g, device="cuda").bfloat16()
+    q[:, :, 17] = 1.0                                              # (a negative query element would make an infinity a score of -inf)
+    K, V = (torch.randn(B, Hkv, L, d, generator=g, device="cuda") for _ in range(2))
+    hit = [(0, 0, 5), (0, 1, 2999), (2, 0, 1290)]
+    for octaves, (b, h, k) in zip((-2, -4, -11), hit):
+        V[b, h, k] *= 2.0 ** octaves
+        V[b, h, k, 32:64] *= 2.0 ** octaves
+    kc, ks = rk.mx_quantize(K, fmt)
+    vc, vs = rk.mx_quantize(V, fmt)
+    kw = dict(kv_fmt=fmt, num_splits=num_splits)
+    lse = torch.empty(2, B, Hkv * grp, dtype=torch.float32, device="cuda")
+    clean = rk.attn_decode(q, kc, vc, ks, vs, lse=lse[0], **kw).view(B, Hkv, grp, d)
+    for b, h, k in hit:
+        kc[b, h, k, 17] = code
+    o = rk.attn_decode(q, kc, vc, ks, vs, lse=lse[1], **kw).view(B, Hkv, grp, d)
+    assert rk.last_device_status() == 0
+    lse = lse.view(2, B, Hkv, grp)
+    for b in range(B):
+        for h in range(Hkv):
+            if any((b, h) == at[:2] for at in hit):
+                assert o[b, h].isnan().all() and lse[1, b, h].isnan().all(), (b, h)
+            else:
+                assert torch.equal(o[b, h], clean[b, h]) and torch.equal(lse[1, b, h], lse[0, b, h]), (b, h)
