@@ -230,6 +230,10 @@ typedef struct rk_decode_args {
   size_t workspace_bytes;
 } rk_decode_args;
 
+/* Splits per (batch, head) the call is cut into on average, and the workspace it wants; both depend on kv_fmt.  With
+ * num_splits = 0 an 8-bit cache is cut into equal ranges of tiles, one per SM, whatever the sequences' lengths: a range
+ * leaves up to two partials per head of a group, and a workspace of B * H * rk_attn_decode_num_splits() * 130 floats, smaller
+ * than rk_attn_decode_workspace_bytes() where there are few units, is taken too, at fewer ranges. */
 RK_API int rk_attn_decode_num_splits(const rk_decode_args* a);
 RK_API size_t rk_attn_decode_workspace_bytes(const rk_decode_args* a);
 RK_API int rk_attn_decode(const rk_decode_args* a, void* stream);

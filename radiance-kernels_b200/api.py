@@ -225,16 +225,20 @@ def kv_cache_append(k_new, v_new, pos, k_codes, k_scales, v_codes, v_scales, fmt
     front().kv_cache_append(k_new, v_new, pos, k_codes, k_scales, v_codes, v_scales, fmt)
 
 
-def attn_decode_num_splits(B, H, H_kv, L, d=128, num_splits=0):
+def attn_decode_num_splits(B, H, H_kv, L, d=128, num_splits=0, kv_fmt=E4M3):
     a = DecodeArgs()
-    a.B, a.H, a.H_kv, a.L, a.d, a.num_splits = B, H, H_kv, L, d, num_splits
+    a.B, a.H, a.H_kv, a.L, a.d, a.num_splits, a.kv_fmt = B, H, H_kv, L, d, num_splits, kv_fmt
     return lib().rk_attn_decode_num_splits(C.byref(a))
 
 
-def attn_decode_workspace_bytes(B, H, H_kv, L, d=128, num_splits=0):
+def attn_decode_workspace_bytes(B, H, H_kv, L, d=128, num_splits=0, kv_fmt=None):
+    """Bytes of attn_decode's workspace for a cache format; without one, enough for each of them."""
     a = DecodeArgs()
     a.B, a.H, a.H_kv, a.L, a.d, a.num_splits = B, H, H_kv, L, d, num_splits
-    return lib().rk_attn_decode_workspace_bytes(C.byref(a))
+    sizes = []
+    for a.kv_fmt in (E4M3, E2M1) if kv_fmt is None else (kv_fmt,):       # one format of each kernel
+        sizes.append(lib().rk_attn_decode_workspace_bytes(C.byref(a)))
+    return max(sizes)
 
 
 def _check_decode_tensors(q, k, v, k_scale, v_scale, kv_len, out, lse):

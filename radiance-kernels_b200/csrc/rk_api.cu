@@ -523,7 +523,7 @@ int rk_attn_decode(const rk_decode_args* a, void* stream) {
       !aligned(a->v_scale, 16) || !aligned(a->o, 16))
     return RK_ERR_MISALIGNED;
   const int ns = rk_attn_decode_num_splits(a);
-  if (!a->workspace || a->workspace_bytes < rk_attn_decode_workspace_bytes(a) || !aligned(a->workspace, 16))
+  if (!a->workspace || a->workspace_bytes < std::min(decode_workspace_bytes(*a, ns), decode_workspace_least(*a, ns)) || !aligned(a->workspace, 16))
     return RK_ERR_WORKSPACE;
   return launch_decode(*a, ns, (cudaStream_t)stream);
 }

@@ -546,15 +546,24 @@ bool decode_uses_tc(const rk_decode_args& a) {
   return can;
 }
 
-// CTAs of the tcgen05 kernel without a split count from the caller: one per SM (never more than there can be tiles).
-static int decode_tc_grid(const rk_decode_args& a) {
+// CTAs of the tcgen05 kernel without a split count from the caller: one per SM (never more than there can be tiles), or fewer where
+// the partials of that many, two per CTA and head of a group, do not fit the workspace.
+static size_t decode_tc_cta_bytes(const rk_decode_args& a) { return (size_t)2 * (a.H / a.H_kv) * (128 + 2) * sizeof(float); }
+static int decode_tc_grid(const rk_decode_args& a, size_t workspace_bytes) {
   const int64_t units = (int64_t)a.B * a.H_kv, tiles = units * ((a.L + dtc::kTile - 1) / dtc::kTile);
-  return (int)std::min<int64_t>(std::min<int64_t>(num_sms(), kMaxCombine), tiles);
+  const size_t fit = workspace_bytes / decode_tc_cta_bytes(a);
+  return (int)std::min<size_t>(fit, std::min<int64_t>(std::min<int64_t>(num_sms(), kMaxCombine), tiles));
 }
 
 size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits) {
-  if (!decode_uses_tc(a) || a.num_splits > 0) return (size_t)a.B * a.H * num_splits * (128 + 2) * sizeof(float);
-  return (size_t)decode_tc_grid(a) * 2 * (a.H / a.H_kv) * (128 + 2) * sizeof(float);
+  if (!decode_uses_tc(a) || a.num_splits > 0) return decode_workspace_least(a, num_splits);
+  return decode_tc_grid(a, SIZE_MAX) * decode_tc_cta_bytes(a);
+}
+
+// num_splits partials per head: what a call needs at least
+size_t decode_workspace_least(const rk_decode_args& a, int num_splits) {
+  const size_t rows = (size_t)a.B * a.H * num_splits * (128 + 2) * sizeof(float);
+  return decode_uses_tc(a) && a.num_splits == 0 ? std::max(rows, decode_tc_cta_bytes(a)) : rows;
 }
 
 template <int HH>
@@ -585,7 +594,7 @@ int launch_decode(const rk_decode_args& a, int nsplit, cudaStream_t st) {
   int* status = device_status_word();
   if (!status) return RK_ERR_NO_DEVICE;
   if (decode_uses_tc(a)) {
-    const int grid = a.num_splits > 0 ? (int)((int64_t)a.B * a.H_kv * nsplit) : decode_tc_grid(a);
+    const int grid = a.num_splits > 0 ? (int)((int64_t)a.B * a.H_kv * nsplit) : decode_tc_grid(a, a.workspace_bytes);
     const size_t parts = a.num_splits > 0 ? BH * nsplit : (size_t)grid * 2 * grp;
     DecodeTcParams t;
     t.q = reinterpret_cast<const __nv_bfloat16*>(a.q);

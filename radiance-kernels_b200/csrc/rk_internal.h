@@ -57,7 +57,8 @@ int launch_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile, int iter
 int launch_wait_runs_out(int limit_us, bool noalloc, cudaStream_t st);   // test hook: a bounded wait that must give up
 extern int g_decode_path;                                   // test hook: 0 = by shape, 1 = mma.sync kernel only
 bool decode_uses_tc(const rk_decode_args& a);                // true when the tcgen05 decode kernel serves this call
-size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits);   // of the kernel that serves the call
+size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits);   // of the kernel that serves the call, at its full grid
+size_t decode_workspace_least(const rk_decode_args& a, int num_splits);   // the smallest it runs with
 
 // Launch with the programmatic attribute: the kernel's set-up runs while the kernel before it in the stream finishes.  Only
 // for kernels in which every CTA calls grid_dependency_wait() before it touches memory another kernel may use.

@@ -95,6 +95,20 @@ def test_decode_argument_errors():
     assert L.rk_attn_decode(C.byref(a), None) == -2
 
 
+def test_decode_workspace_of_every_format():
+    """The helper without a format gives a workspace that every cache format is content with, as before the formats' kernels
+    differed in what they need; with one, what the library asks for."""
+    for B, H, H_kv, L, ns in ((64, 32, 8, 32768, 0), (1, 32, 8, 32768, 0), (1, 8, 8, 132, 0), (2, 8, 2, 4096, 5), (3, 16, 2, 1000, 0)):
+        a = DecodeArgs()
+        a.B, a.H, a.H_kv, a.L, a.d, a.num_splits = B, H, H_kv, L, 128, ns
+        for a.kv_fmt in range(5):
+            need = rk.lib().rk_attn_decode_workspace_bytes(C.byref(a))
+            assert need > 0 and rk.attn_decode_workspace_bytes(B, H, H_kv, L, num_splits=ns, kv_fmt=a.kv_fmt) == need
+            assert rk.attn_decode_workspace_bytes(B, H, H_kv, L, num_splits=ns) >= need
+            assert rk.attn_decode_num_splits(B, H, H_kv, L, num_splits=ns, kv_fmt=a.kv_fmt) == rk.lib().rk_attn_decode_num_splits(C.byref(a))
+    assert rk.attn_decode_workspace_bytes(1, 6, 2, 1024) == 0              # a shape that decode does not take
+
+
 def test_quantizer_argument_errors():
     L = rk.lib()
     assert L.rk_mx_quantize(None, 4, 32, 0, None, None, None) == -1

@@ -395,3 +395,26 @@ def test_a_nan_score_reaches_every_column(grp, num_splits, fmt, code):
                 assert o[b, h].isnan().all() and lse[1, b, h].isnan().all(), (b, h)
             else:
                 assert torch.equal(o[b, h], clean[b, h]) and torch.equal(lse[1, b, h], lse[0, b, h]), (b, h)
+
+
+@pytest.mark.parametrize("fmt", [rk.E4M3, rk.E5M2, rk.E2M3, rk.E3M2, rk.E2M1])
+@pytest.mark.parametrize("B,H,Hkv,L,num_splits", [(1, 8, 2, 8192, 0), (1, 4, 4, 2048, 0), (40, 8, 2, 640, 0), (2, 8, 2, 1000, 3)])
+def test_workspaces_sized_by_the_helpers(B, H, Hkv, L, num_splits, fmt):
+    """A workspace of the helper's size without a format, of its size for the format, and of one partial per split and head
+    (fewer ranges then): each is taken, nothing is written past it, and the outputs agree."""
+    g = torch.Generator(device="cuda").manual_seed(58)
+    q = torch.randn(B, H, 128, generator=g, device="cuda").bfloat16()
+    kc, ks = rk.mx_quantize(torch.randn(B, Hkv, L, 128, generator=g, device="cuda"), fmt)
+    vc, vs = rk.mx_quantize(torch.randn(B, Hkv, L, 128, generator=g, device="cuda"), fmt)
+    kw = dict(kv_fmt=fmt, num_splits=num_splits)
+    want = rk.attn_decode(q, kc, vc, ks, vs, **kw).float()
+    shape = dict(B=B, H=H, H_kv=Hkv, L=L, num_splits=num_splits)
+    for size in (rk.attn_decode_workspace_bytes(**shape), rk.attn_decode_workspace_bytes(**shape, kv_fmt=fmt),
+                 B * H * rk.attn_decode_num_splits(**shape, kv_fmt=fmt) * 130 * 4):
+        buf = torch.full((size + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+        got = rk.attn_decode(q, kc, vc, ks, vs, workspace=buf[:size], **kw).float()
+        assert bool((buf[size:] == 0xA5).all())
+        assert float((got - want).norm() / want.norm()) < 4e-3           # another cut: each side within a bf16 rounding of the exact O
+    with pytest.raises(rk.RkError):
+        rk.attn_decode(q, kc, vc, ks, vs, workspace=buf[:256], **kw)
+    assert rk.last_device_status() == 0
