@@ -144,13 +144,14 @@ PyObject* pair(Tensor a, Tensor b) {
   return r;
 }
 
-// The library call without the interpreter lock: a launch can block while the stream's queue is full.
+// The library call without the interpreter lock: a launch can block while the stream's queue is full.  (f also asks the tensors
+// for their pointers, which throws for those without storage: the lock is taken again on that way out, too.)
 template <class F> int unlocked(F&& f) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = f();
-  Py_END_ALLOW_THREADS
-  return rc;
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  return f();
 }
 
 bool float_or_bf16(const Tensor& t) { return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16; }

@@ -298,3 +298,21 @@ def test_quantize_keys_ragged_blocks(rows, cols):
             for n in range(cols):
                 r = n % 128
                 assert a[b, kb // 4, n // 128, (r % 32) * 16 + r // 32 * 4 + kb % 4] == os_[kb, n]
+
+
+def test_tensors_without_storage_raise():
+    """Tensors that have no memory to point at (a fake one, one inside vmap) give a Python error from every kind of entry point,
+    and the next call works."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        x, g = torch.empty(2, 4, 64, device="cuda"), torch.empty(64, device="cuda")
+        q, c, s = (torch.empty(*n, dtype=t, device="cuda") for n, t in (((1, 4, 128), torch.bfloat16), ((1, 4, 128, 128), torch.uint8), ((1, 4, 128, 4), torch.uint8)))
+        new, pos = torch.empty(1, 4, 128, device="cuda"), torch.empty(1, dtype=torch.int32, device="cuda")
+    for call in (lambda: rk.mx_quantize(x), lambda: rk.mx_quantize_ex(x), lambda: rk.mx_quantize_keys(x), lambda: rk.rmsnorm_mx_quantize(x, g, 1e-5),
+                 lambda: rk.attn_decode(q, c, c, s, s), lambda: rk.kv_cache_append(new, new, pos, c, s, c, s),
+                 lambda: rk.attn_prefill(c, c, c, s, s, s, causal=True),
+                 lambda: torch.vmap(lambda t: rk.mx_quantize(t)[0])(torch.zeros(3, 4, 64, device="cuda"))):
+        with pytest.raises(RuntimeError):
+            call()
+    codes, scales = rk.mx_quantize(torch.ones(4, 64, device="cuda"))
+    assert bool((scales == 127 - 8).all()) and bool((codes == 0x78).all())
