@@ -70,7 +70,9 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, c
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();      // reported here, not by the next call that asks for the last error as well
+  return e;
 }
 
 }  // namespace rk

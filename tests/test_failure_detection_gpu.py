@@ -77,6 +77,33 @@ def test_noalloc_decode_status_word_is_observable():
     assert (got.float() - want.float()).abs().max() < 2e-2
 
 
+def test_a_failed_launch_is_reported_once():
+    """A launch that the runtime refuses on the host (the default stream, while a stream that synchronizes with it is captured) returns
+    its error, and the calls after it, which succeed, do not report it again."""
+    rt = C.CDLL("libcudart.so.12")                                      # the one torch has loaded
+    L = rk.lib()
+    x = torch.randn(4, 64, device="cuda")
+    codes, scales = torch.empty(4, 64, dtype=torch.uint8, device="cuda"), torch.empty(4, 2, dtype=torch.uint8, device="cuda")
+    kt, kts = torch.zeros(64, 32, dtype=torch.uint8, device="cuda"), torch.zeros(2, 32, dtype=torch.uint8, device="cuda")
+    k, ks = torch.empty(32, 64, dtype=torch.uint8, device="cuda"), torch.empty(32, 2, dtype=torch.uint8, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    stream, graph = C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamCreate(C.byref(stream)) == 0
+    assert rt.cudaStreamBeginCapture(stream, 0) == 0
+    try:
+        refused = L.rk_mx_quantize(p(x), 4, 64, 0, p(codes), p(scales), None)
+    finally:
+        rt.cudaStreamEndCapture(stream, C.byref(graph))                 # the capture is invalid: an error, and no graph
+        rt.cudaGetLastError()
+        rt.cudaStreamDestroy(stream)
+    assert refused > 0
+    assert L.rk_import_kt_blocks(p(kt), p(kts), 1, 1, 32, 64, p(k), p(ks), None) == 0
+    assert L.rk_mx_quantize(p(x), 4, 64, 0, p(codes), p(scales), None) == 0
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+
+
 @pytest.mark.parametrize("shape", [(2, 4, 2, 1024, 128, False), (1, 2, 1, 640, 64, False), (1, 4, 4, 512, 128, True)])
 def test_schedule_perturbation_leaves_every_bit_of_o(shape):
     """A few hundred nanoseconds of sleep at every key tile in one warp role at a time (softmax of query tile A,
