@@ -197,11 +197,10 @@ PyObject* mx_quantize_keys(const Args& a) {            // x, fmt, scale_layout
   const int fmt = a.i32(1), layout = a.i32(2);
   need_cuda({&x});
   if (x.scalar_type() != at::kFloat || x.dim() < 2) value_error("mx_quantize_keys takes float32 [..., rows, cols]");
-  if (layout != RK_SCALES_ROWMAJOR && layout != RK_SCALES_SF_ATOMS) value_error("key scales are row-major or scale-factor atoms");
   const int64_t rows = x.size(-2), cols = x.size(-1), batch = x.numel() / std::max<int64_t>(rows * cols, 1);
   Tensor codes = empty_like_device(x, x.sizes(), at::kByte);
   Tensor scales = empty_like_device(x, layout == RK_SCALES_ROWMAJOR ? shape_of(lead_of(x, 2), {up(rows, 32), cols})
-                                                                     : scale_shape(lead_of(x, 2), rows, cols, layout), at::kByte);
+                                                                     : scale_shape(lead_of(x, 2), rows, cols, RK_SCALES_SF_ATOMS), at::kByte);   // (no other: the library says so)
   void* st = stream();
   check_code(unlocked([&] { return rk_mx_quantize_keys_ex(ptr<float>(x), batch, rows, cols, fmt, ptr(codes), ptr(scales), layout, st); }),
              "rk_mx_quantize_keys");
@@ -216,7 +215,7 @@ PyObject* mx_rebase_v(const Args& a) {                 // codes, scales, fmt
   if (codes.dim() < 2) value_error("mx_rebase_v takes codes [..., S, d]");
   const int64_t S = codes.size(-2), d = codes.size(-1), batch = codes.numel() / std::max<int64_t>(S * d, 1);
   if (scales.numel() < codes.numel() / 32) value_error("mx_rebase_v: fewer scales than blocks of codes");
-  Tensor oc = empty_like_device(codes, codes.sizes(), at::kByte);
+  Tensor oc = empty_like_device(codes, codes.sizes(), codes.scalar_type());
   Tensor os = empty_like_device(codes, shape_of(lead_of(codes, 2), {up(S, 32), d}), at::kByte);
   void* st = stream();
   check_code(unlocked([&] { return rk_mx_rebase_v(ptr(codes), ptr(scales), batch, S, d, fmt, ptr(oc), ptr(os), st); }), "rk_mx_rebase_v");

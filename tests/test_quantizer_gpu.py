@@ -316,3 +316,14 @@ def test_tensors_without_storage_raise():
             call()
     codes, scales = rk.mx_quantize(torch.ones(4, 64, device="cuda"))
     assert bool((scales == 127 - 8).all()) and bool((codes == 0x78).all())
+
+
+def test_errors_and_types_of_the_re_blocking_entry_points():
+    """A layout that key scales do not have is the library's error; re-blocked codes have the type of the codes given."""
+    x = torch.randn(64, 64, device="cuda")
+    with pytest.raises(rk.RkError):
+        rk.mx_quantize_keys_ex(x, rk.E4M3, rk.SCALES_GROUPMAJOR)
+    codes, scales = rk.mx_quantize(x)
+    want, ws = rk.mx_rebase_v(codes, scales)
+    got, gs = rk.mx_rebase_v(codes.view(torch.int8), scales)
+    assert got.dtype == torch.int8 and torch.equal(got.view(torch.uint8), want) and torch.equal(gs, ws)
