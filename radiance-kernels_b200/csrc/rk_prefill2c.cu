@@ -114,7 +114,9 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
   const bool dump = DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0;
   const float sc_mul = SOFTCAP ? 1.0f : p.scale_log2;
 
-  float m_run = NEG_INF, l_run = 0.0f;
+  // The row's sum is kept apart for the two halves of the key tiles, whether one thread has both or, with SPLIT, one each: a row comes
+  // out the same, bit for bit, in either form (a call cut into smaller ones crosses from one form to the other).
+  float m_run = NEG_INF, l_run = 0.0f, l_upper = 0.0f;
   bool ok = true;
   bool s_ready = false;       // results of early, non-blocking tests of the next tile's S barrier and P buffer
   int fail = 0;               // which wait gave up (reported after the loops: the tile body carries no reporting code)
@@ -218,7 +220,14 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
     // 2^(7-sc) puts the E4M3 code into bits [20,27) whatever the block scale code sc is (sc < 7 needs no other
     // path: all its non-zero elements lie within 2^6 of the block maximum).
     uint8_t* p_tile = smem + p_off + (grp * 2 + pb) * kTileBytes + row * 128;
-    uint64_t lsA = 0ull, lsB = 0ull;                                  // two packed pairs of partial row sums
+    uint64_t lsA = 0ull, lsB = 0ull;                                  // two packed pairs of partial row sums of a half
+    auto add_half = [&](float& l) {
+      float ls0, ls1, ls2, ls3;
+      unpack2(lsA, ls0, ls1);
+      unpack2(lsB, ls2, ls3);
+      l = fmaf(l, corr, (ls0 + ls1) + (ls2 + ls3));
+      lsA = lsB = 0ull;
+    };
     uint32_t scale_word = 0;
     uint64_t fmul2[kG];
 #pragma unroll
@@ -267,11 +276,9 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
       const int c0 = (4 * half + 2 * g) ^ (row & 7), c1 = (4 * half + 2 * g + 1) ^ (row & 7);     // 128-byte swizzle
       *reinterpret_cast<uint4*>(p_tile + c0 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4*>(p_tile + c1 * 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      if (g == 1) add_half(l_run);
     }
-    float ls0, ls1, ls2, ls3;
-    unpack2(lsA, ls0, ls1);
-    unpack2(lsB, ls2, ls3);
-    l_run = l_run * corr + ((ls0 + ls1) + (ls2 + ls3));
+    if (!SPLIT) add_half(l_upper);
     // the row's four block scales: bytes (row%32)*16 + (row/32)*4 + 0..3 of the 512-byte scale atom
     uint8_t* sf = smem + sfp_off + (grp * 2 + pb) * kSfAtomBytes + (row & 31) * 16 + (row >> 5) * 4;
     if (SPLIT) *reinterpret_cast<uint16_t*>(sf + half * 2) = (uint16_t)scale_word;
@@ -321,8 +328,9 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
     __syncwarp();
     if (lane == 0) mbar_arrive(&xchg_bar[(n_tiles & 3) * 4 + quad]);
     ok = __all_sync(0xffffffffu, mbar_wait(&xchg_bar[(n_tiles & 3) * 4 + quad], (n_tiles >> 2) & 1, abort_flag, p.status, 107));
-    if (ok) l_run += xr[(half ^ 1) * 128];
+    if (ok) l_upper = xr[(half ^ 1) * 128];
   }
+  l_run += l_upper;
 
   // ---- epilogue: O / l -> bf16 (finalize_O, flash_mx_impl.hpp:535-553) ----------------------------------------
   if (ok) {

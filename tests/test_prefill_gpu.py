@@ -317,3 +317,27 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
     torch.cuda.synchronize()
     assert rk.last_device_status() == 0
     assert torch.isfinite(want.float()).all() and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("B,H,Hkv,S,d,kw", [
+    (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles, chunks of at most 128
+    (2, 12, 4, 1090, 64, dict(causal=True, window=300)),          # 216, odd numbers of tiles per head
+    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0))])      # 160
+def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, S, d, kw):
+    """A call whose query tiles outnumber the SMs, against the same call cut by the host entry point and unit by unit, where each
+    piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in both forms)."""
+    Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=62)
+    qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
+    lse = torch.empty(B, H, S, dtype=torch.float32, device="cuda")
+    o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw)
+    sms, grp = torch.cuda.get_device_properties(0).multi_processor_count, H // Hkv
+    assert B * H * ((S + 127) // 128) > sms >= grp * ((S + 127) // 128)
+    for b in range(B):
+        for h in range(Hkv):
+            part = [t[b:b + 1, h * grp:(h + 1) * grp].contiguous() for t in (qc, qs)] + [t[b:b + 1, h:h + 1].contiguous() for t in (kc, ks, vc, vs)]
+            l1 = torch.empty(1, grp, S, dtype=torch.float32, device="cuda")
+            o1 = rk.attn_prefill(part[0], part[2], part[4], part[1], part[3], part[5], lse=l1, **kw)
+            assert torch.equal(o1[0], o[b, h * grp:(h + 1) * grp]) and torch.equal(l1[0], lse[b, h * grp:(h + 1) * grp]), (b, h)
+    runner = rk.PrefillHostRunner(*[t.cpu().pin_memory() for t in (qc, kc, vc, qs, ks, vs)], want_lse=True, **kw)
+    assert torch.equal(runner.run(), o.cpu()) and torch.equal(runner.lse, lse.cpu())
+    assert rk.last_device_status() == 0
