@@ -62,7 +62,7 @@ constexpr int misc_off = bar_off + nBars * 8;
 constexpr int corr_off = misc_off + 16;                    // [2 groups][4 slots][128] floats: the O rescale factors of a tile
 constexpr int total = corr_off + 2 * 4 * 128 * 4;
 // test hook: which role sleeps a little at every key tile (schedule perturbation)
-constexpr int kPerturbSoftmaxA = 1 /* 2 = softmax of tile B */, kPerturbCorr = 3, kPerturbTma = 4, kPerturbQk = 5, kPerturbPv = 6;
+constexpr int kPerturbSoftmaxA = 1 /* 2 = softmax of tile B (SPLIT: of keys 64-127) */, kPerturbCorr = 3, kPerturbTma = 4, kPerturbQk = 5, kPerturbPv = 6;
 }  // namespace c2
 
 template <uint32_t N> RK_DEVINL void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -124,7 +124,7 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
     const int pb = j & 1;
-    perturb(p, kPerturbSoftmaxA + grp, j);
+    perturb(p, kPerturbSoftmaxA + (SPLIT ? half : grp), j);
     const bool stamp = (quad == 0 && lane == 0);
     if (stamp) RK_STAMP(grp, j, 0);
     if (__builtin_expect(!__all_sync(0xffffffffu, s_ready), 0)) {   // a test issued during the previous tile said "not yet"
@@ -145,7 +145,7 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
 
     if (DUMP && dump && j == 0) {
 #pragma unroll
-      for (int c = 0; c < kN; ++c) p.dbg[row * 128 + c] = s[c];
+      for (int c = 0; c < kN; ++c) p.dbg[row * 128 + half * 64 + c] = s[c];
     }
 
     // ---- (soft-cap,) mask, block maxima ----------------------------------------------------------------
@@ -287,12 +287,13 @@ __device__ __forceinline__ void softmax_row_group(const PrefillParams& p, uint8_
     if (DUMP && dump && j == 0) {
       uint32_t* d32 = reinterpret_cast<uint32_t*>(p.dbg + 128 * 128);
 #pragma unroll
-      for (int lc = 0; lc < 8; ++lc) {
+      for (int lc = half * 4; lc < half * 4 + 2 * kG; ++lc) {
         const uint4 v4 = *reinterpret_cast<const uint4*>(p_tile + ((lc ^ (row & 7)) * 16));
         d32[row * 32 + lc * 4 + 0] = v4.x; d32[row * 32 + lc * 4 + 1] = v4.y;
         d32[row * 32 + lc * 4 + 2] = v4.z; d32[row * 32 + lc * 4 + 3] = v4.w;
       }
-      d32[128 * 32 + row] = scale_word;
+      if (SPLIT) reinterpret_cast<uint16_t*>(d32 + 128 * 32 + row)[half] = (uint16_t)scale_word;
+      else d32[128 * 32 + row] = scale_word;
     }
     // a look ahead at the next tile's S barrier and at its P buffer (free once the P.V that read it two tiles
     // before has finished): asked here, used at the top of the next tile
@@ -703,16 +704,18 @@ static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
                      uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st) {
-  if (p.dbg)      // the stage dump lives in an instantiation of its own, so that the kernel that ships carries none of its code
-    return softcap ? launch2c_cfg<true, true, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
-                   : launch2c_cfg<false, true, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st);
   // One query tile per CTA while every tile can have an SM: above that, two tiles per CTA share K, V and the SM (256 tiles:
   // 91 us in one wave of pairs against 110 in two of single tiles).
-  if ((int64_t)p.n_q_tiles * p.H * p.B <= num_sms())
-    return softcap ? launch2c_cfg<true, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
-                   : launch2c_cfg<false, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st);
-  return softcap ? launch2c_cfg<true, false, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
-                 : launch2c_cfg<false, false, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st);
+  const bool split = (int64_t)p.n_q_tiles * p.H * p.B <= num_sms();
+  if (p.dbg)      // the stage dump lives in instantiations of its own, so that the kernels that ship carry none of its code
+    return split ? (softcap ? launch2c_cfg<true, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
+                            : launch2c_cfg<false, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st))
+                 : (softcap ? launch2c_cfg<true, true, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
+                            : launch2c_cfg<false, true, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st));
+  return split ? (softcap ? launch2c_cfg<true, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
+                          : launch2c_cfg<false, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, st))
+               : (softcap ? launch2c_cfg<true, false, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st)
+                          : launch2c_cfg<false, false, false>(tq, tk, tv, p, idesc_qk, idesc_pv, st));
 }
 
 }  // namespace rk

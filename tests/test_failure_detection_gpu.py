@@ -104,10 +104,11 @@ def test_a_failed_launch_is_reported_once():
     assert rk.last_device_status() == 0
 
 
-@pytest.mark.parametrize("shape", [(2, 4, 2, 1024, 128, False), (1, 2, 1, 640, 64, False), (1, 4, 4, 512, 128, True)])
+@pytest.mark.parametrize("shape", [(2, 4, 2, 1024, 128, False), (1, 2, 1, 640, 64, False), (1, 4, 4, 512, 128, True),      # one query tile per CTA
+                                   (2, 16, 4, 900, 128, False), (1, 40, 8, 520, 64, False), (1, 52, 4, 384, 128, True)])  # two
 def test_schedule_perturbation_leaves_every_bit_of_o(shape):
     """A few hundred nanoseconds of sleep at every key tile in one warp role at a time (softmax of query tile A,
-    of tile B, correction, TMA producer, Q K^T issuer, P V issuer): if a hand-off between roles lacked a barrier the delayed
+    of tile B -- of the lower and of the upper keys where a CTA has one query tile --, correction, TMA producer, Q K^T issuer, P V issuer): if a hand-off between roles lacked a barrier the delayed
     role would read or overwrite something too early and O would change."""
     B, H, Hkv, S, d, cap = shape
     L = rk.lib()

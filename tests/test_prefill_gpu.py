@@ -66,9 +66,10 @@ def test_sliding_window_d128():
                                                       (256, 1280, 200, 0, 50.0), (128, 900, 1, 0, 0.0)])
 def test_sliding_window_skips_key_tiles_below_the_window(d, S, window, q_pos0, softcap):
     """Long sequences with a short window: most key tiles lie wholly below the window and are never loaded; the
-    result must equal the oracle's, which masks them (both kernels: d = 128 pairs of query tiles, d = 256)."""
-    _check(prefill_vs_oracle(1, 2, 1, S, S + q_pos0, d, causal=True, window=window, q_pos0=q_pos0, softcap=softcap,
-                             mul=0.5 if d == 256 else 1.0, seed=60 + window))
+    result must equal the oracle's, which masks them (d = 128 with one query tile per CTA and, at 20 heads, with two; d = 256)."""
+    for H in (2, 20) if d == 128 else (2,):
+        _check(prefill_vs_oracle(1, H, 1, S, S + q_pos0, d, causal=True, window=window, q_pos0=q_pos0, softcap=softcap,
+                                 mul=0.5 if d == 256 else 1.0, seed=60 + window))
 
 
 def test_ragged_lengths_and_offset():
@@ -90,13 +91,15 @@ def test_v_scales_along_keys_reference_layout():
 
 
 def test_e5m2_operands():
-    _check(prefill_vs_oracle(1, 2, 1, 256, 256, 128, causal=True, fmt=rk.E5M2, seed=11))
+    for H in (2, 76):                                              # a CTA per query tile, and one for two of them
+        _check(prefill_vs_oracle(1, H, 1, 256, 256, 128, causal=True, fmt=rk.E5M2, seed=11))
 
 
 def test_mxfp6_operands_e2m3_q_e3m2_kv():
     """MXFP6 variant: E2M3 queries, E3M2 keys and values (P stays E4M3), 6-bit codes packed for the tensor core."""
     import oracle
     for (B, H, Hkv, Sq, Skv, d, axis) in ((1, 2, 1, 256, 256, 128, rk.V_SCALES_ALONG_D), (1, 4, 2, 200, 333, 64, rk.V_SCALES_ALONG_KEYS),
+                                          (1, 76, 2, 256, 256, 128, rk.V_SCALES_ALONG_D), (2, 40, 2, 200, 333, 64, rk.V_SCALES_ALONG_KEYS),   # two query tiles per CTA
                                           (1, 2, 1, 384, 384, 256, rk.V_SCALES_ALONG_D)):
         Q, K, V = randn_qkv(B, H, Hkv, Sq, Skv, d, seed=31, mul=0.5)
         qc, qs = rk.mx_quantize(Q, rk.E2M3)
@@ -244,15 +247,16 @@ def test_full_size_head_slices_match_oracle():
         assert ma <= MAX_ABS and rl <= REL_L2, (sl, ma, rl)
 
 
-@pytest.mark.parametrize("d,qmul", [(128, 1.0), (128, 6.0), (64, 1.0)])
-def test_stage_parity_s_and_requantized_p(d, qmul):
-    """Stage-level parity on the first key tile of the last query tile (the kernels' debug dump): S = Q K^T within
+@pytest.mark.parametrize("d,qmul,H", [(128, 1.0, 1), (128, 6.0, 1), (64, 1.0, 1), (128, 1.0, 75), (128, 6.0, 75), (64, 1.0, 75)])
+def test_stage_parity_s_and_requantized_p(d, qmul, H):
+    """Stage-level parity on the first key tile of the last query tile of head 0 (the kernels' debug dump; one query tile per CTA with
+    one head, two with 75): S = Q K^T within
     fp32 reassociation error, and the requantized P -- E4M3 codes and E8M0 block scales -- equal to the oracle's.
     A code may differ by one step where the fp32 p sits on a truncation boundary; such elements are counted and
     must stay below 0.05 %."""
     import ctypes as C
     Sq = Skv = 256
-    Q, K, V = randn_qkv(1, 1, 1, Sq, Skv, d, seed=50, qmul=qmul)
+    Q, K, V = randn_qkv(1, H, H, Sq, Skv, d, seed=50, qmul=qmul)
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
     dbg = torch.zeros(32768, dtype=torch.float32, device="cuda")
     rk.lib().rk_debug_set_prefill_dump(C.c_void_p(dbg.data_ptr()))
@@ -263,7 +267,7 @@ def test_stage_parity_s_and_requantized_p(d, qmul):
         rk.lib().rk_debug_set_prefill_dump(None)
     assert rk.last_device_status() == 0
     scale = d ** -0.5
-    r = oracle.attn_prefill(np_(qc), np_(kc), np_(vc), np_(qs), np_(ks), np_(vs), causal=True, softmax_scale=scale,
+    r = oracle.attn_prefill(*(np_(t[:, :1]) for t in (qc, kc, vc, qs, ks, vs)), causal=True, softmax_scale=scale,
                             block_n=128, dump_slice=0)
     dd = np_(dbg)
     rows = slice(128, 256)                                    # the dump is the last query tile, key tile 0
