@@ -448,7 +448,6 @@ namespace rk {
 // the length, the unit's first tile, the maxima and the rows one after the other, 40 us for 148 partials).  Which partials it
 // needs depends on kv_len alone, which nothing still running writes (the main kernel lets this one start only after its own
 // wait), so that is worked out before the wait; after it the maxima and the rows of a warp's first partials load together.
-constexpr int kMaxCombine = 512;                  // partials of one unit: CTAs of the main kernel, or the caller's splits
 constexpr int kCombineWarps = 8;
 __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(const DecodeTcParams p, int main_grid) {
   constexpr int kBatch = 4;                                        // partials of a warp in flight
@@ -552,7 +551,7 @@ static size_t decode_tc_cta_bytes(const rk_decode_args& a) { return (size_t)2 * 
 static int decode_tc_grid(const rk_decode_args& a, size_t workspace_bytes) {
   const int64_t units = (int64_t)a.B * a.H_kv, tiles = units * ((a.L + dtc::kTile - 1) / dtc::kTile);
   const size_t fit = workspace_bytes / decode_tc_cta_bytes(a);
-  return (int)std::min<size_t>(fit, std::min<int64_t>(std::min<int64_t>(num_sms(), kMaxCombine), tiles));
+  return (int)std::min<size_t>(fit, std::min<int64_t>(num_sms(), tiles));
 }
 
 size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits) {

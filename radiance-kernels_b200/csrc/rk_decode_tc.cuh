@@ -37,7 +37,7 @@
 // tile's maximum, handed from tile to tile, and replaced by a tile's own maximum where that is more than 2^8 above it (V scales:
 // 2^32), so O is rescaled about never.  The p of the key that set the reference is 1, which two terms hold exactly: with the
 // weight on few keys it is the error of the largest p that counts.  (References that are integers, so that the codes need not
-// wait for the other warps' maxima, leave that p with the rounding of any other: errors of 6.0e-4 of the result instead of
+// wait for the other warps' maxima, leave that p with the rounding of any other: errors of 5.9e-4 of the result instead of
 // 5.2e-4 with queries of four times unit variance, 5.8e-4 instead of 4.1e-4 with twelve times.)  A warp's block scale carries
 // the power of two of the largest p of its 32 keys.
 // A segment ends in the group of its last tile alone: it reads O (one of four accumulators, used in turn) and the row sums
