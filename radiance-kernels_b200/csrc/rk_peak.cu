@@ -25,7 +25,7 @@ mxfp8_mma_loop_kernel(const uint8_t* __restrict__ a_tile, const uint8_t* __restr
                       uint32_t idesc) {
   using namespace peak;
   extern __shared__ __align__(1024) uint8_t peak_smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(peak_smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_smem(peak_smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + bar_off);       // [0] loads, [1] drain, [2], [3] pacing
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + misc_off + 4);

@@ -329,7 +329,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
                const uint32_t idesc_pv) {
   using L = SmemLayout<DCH, KV_STAGES>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_smem(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bar_off);
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + L::misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc_off + 4);

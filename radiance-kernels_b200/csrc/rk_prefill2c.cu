@@ -437,7 +437,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                  const uint32_t idesc_pv) {
   using namespace c2;
   extern __shared__ __align__(1024) uint8_t smem_raw2c[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw2c) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_smem(smem_raw2c);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + bar_off);
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + misc_off + 4);
