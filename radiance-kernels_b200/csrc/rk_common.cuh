@@ -182,6 +182,19 @@ RK_DEVINL bool mbar_wait_lean(uint64_t* bar, uint32_t parity, volatile int* abor
   } while (!*abort_flag && clock64() - t0 < kWaitLimitCycles);
   return false;
 }
+// The same in a dozen instructions, with sleeps between polls (SLEEP_NS > 0): for kernels whose code competes for the instruction cache.
+// The caller keeps the code of the wait that gave up and reports it once, outside its loops.  abort_flag nullptr: waits on when the
+// CTA has given up (drains).
+template <uint32_t SLEEP_NS = 0>
+RK_DEVINL bool mbar_wait_short(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const uint32_t t0 = (uint32_t)clock();
+#pragma unroll 1
+  while (!mbar_try_wait<0>(bar, parity)) {
+    if ((abort_flag && *abort_flag) || (uint32_t)clock() - t0 > (uint32_t)kWaitLimitCycles) return false;
+    if (SLEEP_NS) __nanosleep(SLEEP_NS);
+  }
+  return true;
+}
 RK_DEVINL void report_wait_failure(volatile int* abort_flag, int* status, int code) {
   *abort_flag = 1;
   atomicCAS(status, 0, code);
@@ -229,9 +242,46 @@ RK_DEVINL void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, ui
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
       ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+// TMA: 3-D tiled store shared -> global (what lies outside the tensor is left out); completion by bulk groups.
+RK_DEVINL void tma_store_3d(const void* tmap, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(tmap), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+RK_DEVINL void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N> RK_DEVINL void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }   // at most N groups still read their source
+RK_DEVINL void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 RK_DEVINL void prefetch_tmap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
+
+// Cluster launch control: a running CTA takes over the block index of one that has not started yet.  The answer (16 bytes) arrives
+// in shared memory and completes 16 bytes on the mbarrier.  After an answer "none left" no further request may be made.
+RK_DEVINL void clc_request(void* smem_answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(smem_answer)), "r"(smem_u32(bar)) : "memory");
+}
+RK_DEVINL bool clc_answer(const void* smem_answer, uint32_t& block_x) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .b64 lo, hi;\n\t.reg .pred p;\n\t"
+      "ld.shared.v2.b64 {lo, hi}, [%2];\n\t"
+      "mov.b128 r, {lo, hi};\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+      : "=r"(ok), "=r"(block_x) : "r"(smem_u32(smem_answer)) : "memory");
+  return ok != 0;
+}
+
+// One lane of a converged warp, the same one every time.
+RK_DEVINL bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0;
+}
+// A value that is the same in all lanes, in a form the compiler knows to be.
+RK_DEVINL int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
 // ---- TMEM / tcgen05 ----
 RK_DEVINL void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {   // whole warp

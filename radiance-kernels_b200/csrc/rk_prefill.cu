@@ -591,6 +591,20 @@ int make_tmap_sub8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t rows
   return r == CUDA_SUCCESS ? RK_OK : RK_ERR_BAD_SHAPE;
 }
 
+// O, bf16 [BH][S_q][d]; a box is 32 columns x 32 rows and leaves shared memory as 64 bytes per row (64-byte swizzle).
+static int make_tmap_o(CUtensorMap* m, const void* base, int64_t BH, int64_t S, int64_t d) {
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return RK_ERR_NO_DEVICE;
+  cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)S, (cuuint64_t)BH};
+  cuuint64_t strides[2] = {(cuuint64_t)(d * 2), (cuuint64_t)(S * d * 2)};
+  cuuint32_t box[3] = {32, 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? RK_OK : RK_ERR_BAD_SHAPE;
+}
+
 template <int DCH, int KV_STAGES, bool SOFTCAP, bool DUMP>
 static int launch_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
                       uint32_t idesc_qk, uint32_t idesc_pv, dim3 grid, cudaStream_t st) {
@@ -630,6 +644,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
   if (!p.status) return RK_ERR_NO_DEVICE;
   p.dbg = g_prefill_dbg;
   p.B = a.B; p.H = a.H; p.H_kv = a.H_kv; p.S_q = a.S_q; p.S_kv = a.S_kv; p.d = a.d;
+  p.group = a.H / a.H_kv;
   {
     // heads whose K and V (shared by the query heads of a KV head) fit in about 100 MB of L2, in equal groups
     const double per_head = 2.0 * a.S_kv * a.d * ((double)a.H_kv / a.H);
@@ -654,7 +669,12 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
   const uint32_t idesc_pv = make_idesc(RK_FMT_E4M3, a.kv_fmt, false, /*B MN-major*/ !kv6, 128, 128);
   dim3 grid(p.n_q_tiles * a.H * a.B, 1, 1);
   const bool cap = a.softcap > 0.0f;
-  if (a.d <= 128) return launch_prefill2c(tq, tk, tv, p, idesc_qk, idesc_pv, cap, st);   // two query tiles per CTA
+  if (a.d <= 128) {                                                                      // two query tiles per CTA
+    CUtensorMap to;
+    rc = make_tmap_o(&to, a.o, (int64_t)a.B * a.H, a.S_q, a.d);
+    if (rc != RK_OK) return rc;
+    return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
+  }
   if (p.dbg)      // the stage dump lives in instantiations of its own: the kernels that ship carry none of its code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)
                : launch_cfg<2, 2, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st);

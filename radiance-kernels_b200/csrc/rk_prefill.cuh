@@ -34,6 +34,7 @@ struct PrefillParams {
   int* status;
   float* dbg;          // optional stage dump of CTA (0,0,0), first key tile
   int B, H, H_kv, S_q, S_kv, d;
+  int group;           // query heads per KV head
   int n_q_tiles, n_kv_tiles;
   int head_group;      // (batch, head) pairs per work-order group: the heaviest query tiles of a whole group run first
   int q_pos0, causal, window;
@@ -156,7 +157,7 @@ int make_tmap_sub8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t rows
 extern float* g_prefill_dbg;
 
 // Two query tiles per CTA, one thread per row, correction warps (d <= 128); defined in rk_prefill2c.cu.
-int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
+int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                      uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st);
 extern int g_prefill_perturb;   // test hook: PrefillParams::perturb of the next launches
 
