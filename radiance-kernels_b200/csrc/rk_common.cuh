@@ -182,17 +182,17 @@ RK_DEVINL bool mbar_wait_lean(uint64_t* bar, uint32_t parity, volatile int* abor
   } while (!*abort_flag && clock64() - t0 < kWaitLimitCycles);
   return false;
 }
-// The same in a dozen instructions, with sleeps between polls (SLEEP_NS > 0): for kernels whose code competes for the instruction cache.
+// The same in a dozen instructions: for kernels whose code competes for the instruction cache.  LONG: a wait off the critical path; the
+// hardware may hold the warp for 2 us before it polls again, which leaves the issue slots to the others (a short prefill on 128 SMs
+// 45.8 -> 44.5 us; on the softmax warps' own waits it costs 2 %).
 // The caller keeps the code of the wait that gave up and reports it once, outside its loops.  abort_flag nullptr: waits on when the
 // CTA has given up (drains).
-template <uint32_t SLEEP_NS = 0>
+template <bool LONG = false>
 RK_DEVINL bool mbar_wait_short(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   const uint32_t t0 = (uint32_t)clock();
 #pragma unroll 1
-  while (!mbar_try_wait<0>(bar, parity)) {
+  while (!mbar_try_wait<LONG ? 2000 : 0>(bar, parity))
     if ((abort_flag && *abort_flag) || (uint32_t)clock() - t0 > (uint32_t)kWaitLimitCycles) return false;
-    if (SLEEP_NS) __nanosleep(SLEEP_NS);
-  }
   return true;
 }
 RK_DEVINL void report_wait_failure(volatile int* abort_flag, int* status, int code) {

@@ -41,14 +41,10 @@ namespace rk {
 namespace c2 {
 constexpr int kStages = 3;
 constexpr int kThreads = 512;
-#ifndef RK_SLEEP_NS
-#define RK_SLEEP_NS 100
-#endif
-constexpr uint32_t kSleepNs = RK_SLEEP_NS;     // back-off of the warps that wait off the critical path
 constexpr int kWarpCorr = 8, kWarpTma = 12, kWarpQk = 13, kWarpPv = 14;
 // Registers of a softmax, correction and issuer thread: 128 * (2 * softmax + correction + issuer) = 65536.  Measured (8 x 16 heads of
 // 4096): softmax 176 545 us, 184 527, 192 527, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
-constexpr uint32_t kRegSoftmax = 184, kRegCorr = 80, kRegIssue = 64;
+constexpr uint32_t kRegSoftmax = 176, kRegCorr = 88, kRegIssue = 72;
 constexpr uint32_t kRegSoftmaxSplit = 160, kRegCorrSplit = 96, kRegIssueSplit = 96;
 // TMEM columns
 constexpr uint32_t cS = 0, cO = 128 /* + g*128 */, cSfQ = 384 /* + g*4 */, cSfK = 392 /* + st*4 */,
@@ -93,8 +89,9 @@ constexpr int kReaders = 8 + 4 + 2;      // warps that read an item: softmax, co
 template <uint32_t N> RK_DEVINL void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> RK_DEVINL void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
+template <bool DUMP>
 RK_DEVINL void perturb(const PrefillParams& p, int role, int j) {
-  if (__builtin_expect(p.perturb == role, 0)) __nanosleep(400 + 97 * (j & 7));
+  if (DUMP && __builtin_expect(p.perturb == role, 0)) __nanosleep(400 + 97 * (j & 7));
 }
 
 // ---- softmax warps: thread = query row -----------------------------------------------------------------------
@@ -185,7 +182,7 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
     const int t = t0 + j, pb = t & 1;                         // barriers, P buffers and rescale slots count on from item to item
-    perturb(p, kPerturbSoftmaxA + (SPLIT ? half : grp), j);
+    perturb<DUMP>(p, kPerturbSoftmaxA + (SPLIT ? half : grp), j);
     const bool stamp = (quad == 0 && lane == 0);
     if (stamp) RK_STAMP(grp, j, 0);
     if (__builtin_expect(!__all_sync(0xffffffffu, s_ready), 0)) {   // a test issued during the previous tile said "not yet"
@@ -197,8 +194,6 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
 
     // first key of this tile (j counts from the first tile inside the window), and of this thread's scores
     const int key0 = (j + j0) * kBlockN, k0 = key0 + half * 64;
-    if (kMaskInTmem && __builtin_expect(j < n_low || j >= n_high, 0))
-      mask_scores<kG>(tmem_base + lane_addr + cS + half * 64, p, q_pos, k0);
 
     float s[kN];
 #pragma unroll
@@ -374,7 +369,20 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
       for (; j < n_high && ok; ++j) ok = tile(j, std::true_type{});
     for (; j < n_tiles && ok; ++j) ok = tile(j, std::false_type{});
   } else {
-    for (; j < n_tiles && ok; ++j) ok = tile(j, std::true_type{});
+    while (j < n_tiles && ok) {
+      int end = min(n_high, n_tiles);                // a run of tiles without a mask
+      if (j < n_low || j >= n_high) {                // one tile with
+        const int t = t0 + j;
+        const int w = wait_tile_inputs(s_full, t & 1, &pv_done[t & 1], ((t - 2) >> 1) & 1, t >= 2, abort_flag);
+        if (__any_sync(0xffffffffu, w != 0)) { fail = w ? w : 101; ok = false; break; }
+        tc_fence_after();
+        mask_scores<kG>(tmem_base + lane_addr + cS, p, q_pos, (j + j0) * kBlockN);
+        s_ready = true;
+        end = j + 1;
+      }
+#pragma unroll 1
+      for (; j < end && ok; ++j) ok = tile(j, std::true_type{});
+    }
   }
   if (SPLIT && ok) {                                                    // the row's sum: both halves
     float* xr = xchg + (n_tiles & 1) * 256 + row;
@@ -488,7 +496,7 @@ __device__ __forceinline__ void write_out_quadrant(const PrefillParams& p, const
 }
 
 // The tiles of one item; returns the code of the wait that gave up, or 0.  t0, t1: the two groups' tiles of earlier items.
-template <bool SPLIT>
+template <bool DUMP, bool SPLIT>
 __device__ __forceinline__ int correction_quadrant(const PrefillParams& p, const CUtensorMap* tmap_o, uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
                                                    volatile int* abort_flag, int nt0, int nt1, int t0, int t1, const Pending& out0, const Pending& out1) {
   using namespace c2;
@@ -499,19 +507,19 @@ __device__ __forceinline__ int correction_quadrant(const PrefillParams& p, const
   const float* corr_sm = reinterpret_cast<const float*>(smem + corr_off);
   const int o_chunks = p.d / 32, n_all = max(nt0, nt1);
   for (int j = 0; j < n_all; ++j) {
-    perturb(p, kPerturbCorr, j);
+    perturb<DUMP>(p, kPerturbCorr, j);
 #pragma unroll 1
     for (int g = 0; g < 2; ++g) {
       if (j >= (g == 0 ? nt0 : nt1)) continue;
       const int t = (g == 0 ? t0 : t1) + j;                   // this group's tile, counted over all items of the CTA
       if (quad == 0 && lane == 0) RK_STAMP(3, j, g * 4 + 0);
-      if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bCF + (g * 4 + (t & 3)) * 4 + quad], (t >> 2) & 1, abort_flag))) return 401;
+      if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bCF + (g * 4 + (t & 3)) * 4 + quad], (t >> 2) & 1, abort_flag))) return 401;
       const float corr = corr_sm[(g * 4 + (t & 3)) * 128 + row];
       if (quad == 0 && lane == 0) RK_STAMP(3, j, g * 4 + 1);
       if (t > 0) {
         // Always wait for the previous P.V of this tile, rescale or not: an arrival on the O-ready barrier then
         // implies that its previous phase has been consumed, which is what keeps the two-deep barrier from wrapping.
-        if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bPV + g * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort_flag))) return 402;
+        if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPV + g * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort_flag))) return 402;
       }
       if (j == 0) {
         if (!SPLIT && t > 0) write_out_quadrant(p, tmap_o, smem, tmem_base, g, t, g == 0 ? out0 : out1);   // the group's item before this one
@@ -658,7 +666,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     reg_dec<SPLIT ? kRegIssueSplit : kRegIssue>();
     int fail = 0;                                    // which wait gave up
     // before TMEM and shared memory go back: this thread's asynchronous work has finished, also where the CTA gives up
-    auto drain = [&](uint64_t* bar, uint32_t parity, int code) { if (!mbar_wait_short<kSleepNs>(bar, parity, nullptr) && !fail) fail = code; };
+    auto drain = [&](uint64_t* bar, uint32_t parity, int code) { if (!mbar_wait_short<true>(bar, parity, nullptr) && !fail) fail = code; };
     if (threadIdx.x == kWarpQk * 32) RK_STAMP_RAW(6);
     if (warp == kWarpTma) {
       // ================= TMA producer; hands out the items =================
@@ -671,10 +679,10 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           const int n_all = max(w.nt0, w.nt1);
           bool asked = false;
           for (int j = 0; j < n_all || j == 0; ++j) {
-            perturb(p, kPerturbTma, j);
+            perturb<DUMP>(p, kPerturbTma, j);
             if (j == 0) {
               // everybody has read the last item: this one takes its place, and the one after it is asked for
-              if (k > 0 && !mbar_wait_short<kSleepNs>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
+              if (k > 0 && !mbar_wait_short<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
               *reinterpret_cast<Work*>(smem + work_off) = w;
               mbar_arrive(&bars[bWF]);
               if (k == 0) {
@@ -690,7 +698,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               for (int g = 0; g < 2; ++g) {
                 if ((g == 0 ? w.nt0 : w.nt1) == 0) continue;
                 if ((q_used >> g) & 1) {             // Q K^T of the last item that had a tile in this place has finished
-                  if (!mbar_wait_short<kSleepNs>(&bars[bQE + g], (q_par >> g) & 1, abort_flag)) { fail = 203; break; }
+                  if (!mbar_wait_short<true>(&bars[bQE + g], (q_par >> g) & 1, abort_flag)) { fail = 203; break; }
                   q_par ^= 1 << g;
                 }
                 q_used |= 1 << g;
@@ -699,10 +707,10 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               if (fail) break;
             }
             if (n_all > 0) {
-              if (use > 0 && !mbar_wait_short<kSleepNs>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
+              if (use > 0 && !mbar_wait_short<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
               issue_kv(j, st);
               if (stopped) break;                    // O is written only where V has come
-              if (use > 0 && !mbar_wait_short<kSleepNs>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
+              if (use > 0 && !mbar_wait_short<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
               issue_v(j, st);
               if (++st == kStages) { st = 0; ++use; }
             }
@@ -716,7 +724,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           if (asked) drain(&bars[bClc], k & 1, 503);
           if (fail || stopped || !asked) break;
           if (!clc_answer(smem + clc_off, block)) {
-            if (!mbar_wait_short<kSleepNs>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
+            if (!mbar_wait_short<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
             w.qp = -1;
             *reinterpret_cast<Work*>(smem + work_off) = w;
             mbar_arrive(&bars[bWF]);
@@ -745,9 +753,9 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (more < 0) { fail = kFailWork; break; }
         const int nt0 = warp_uniform(w.nt0), nt1 = warp_uniform(w.nt1), n_all = max(nt0, nt1);
         for (int j = 0; j < n_all && !fail; ++j) {
-          perturb(p, kPerturbQk, j);
+          perturb<DUMP>(p, kPerturbQk, j);
           if (lane == 0) RK_STAMP(2, j, 0);
-          if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfK + st * 4, dsfk + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dkt = dk + (uint32_t)(st * (kTileBytes >> 4));
           if (lane == 0) RK_STAMP(2, j, 1);
@@ -800,8 +808,8 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (more < 0) { fail = kFailWork; break; }
         const int nt0 = warp_uniform(w.nt0), nt1 = warp_uniform(w.nt1), n_all = max(nt0, nt1);
         for (int i = 0; i < n_all && !fail; ++i) {
-          perturb(p, kPerturbPv, i);
-          if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
+          perturb<DUMP>(p, kPerturbPv, i);
+          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfV + st * 4, dsfv + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dvt = dv + (uint32_t)(st * (kTileBytes >> 4));
 #pragma unroll 1
@@ -809,8 +817,8 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (i >= (g == 0 ? nt0 : nt1)) continue;
             const int t = (g == 0 ? t0 : t1) + i, gb = g * 2 + (t & 1);
             const uint32_t par2 = (t >> 1) & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bPF + gb], par2, abort_flag))) { fail = 304; break; }      // P written
-            if (!__all_sync(0xffffffffu, mbar_wait_short<kSleepNs>(&bars[bOR + gb], par2, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's written out
+            if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPF + gb], par2, abort_flag))) { fail = 304; break; }      // P written
+            if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bOR + gb], par2, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's written out
             tc_fence_after();
             const uint64_t dpt = dp + (uint32_t)(gb * (kTileBytes >> 4));
             if (elect_one()) {
@@ -843,7 +851,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (more < 0) { fail = kFailWork; break; }
       if (more == 0 && SPLIT) break;
       if (more == 0) { w.nt0 = t0 > 0; w.nt1 = t1 > 0; }      // no item is left: once more, for the O of the last ones
-      fail = correction_quadrant<SPLIT>(p, &tmap_o, smem, bars, tmem_base, abort_flag, w.nt0, w.nt1, t0, t1, out0, out1);
+      fail = correction_quadrant<DUMP, SPLIT>(p, &tmap_o, smem, bars, tmem_base, abort_flag, w.nt0, w.nt1, t0, t1, out0, out1);
       if (fail || more == 0) break;
       t0 += w.nt0; t1 += w.nt1;
       if (w.nt0 > 0) out0 = Pending{2 * w.qp, w.bh};
@@ -904,7 +912,7 @@ int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   // One query tile per CTA while every tile can have an SM: above that, two tiles per CTA share K, V and the SM (256 tiles:
   // 91 us in one wave of pairs against 110 in two of single tiles).
   const bool split = (int64_t)p.n_q_tiles * p.H * p.B <= num_sms();
-  if (p.dbg)      // the stage dump lives in instantiations of its own, so that the kernels that ship carry none of its code
+  if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return split ? (softcap ? launch2c_cfg<true, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
                             : launch2c_cfg<false, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st))
                  : (softcap ? launch2c_cfg<true, true, false>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
