@@ -348,6 +348,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  int fail = 0;                                      // which wait of an issuer gave up
   // heavy (late) query tiles first within a head; heads adjacent so a KV head's tiles share L2
   // work order: see PrefillParams::head_group (heaviest query tiles of a whole group of heads first)
   const int n_bh = p.B * p.H;
@@ -447,94 +448,89 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
   } else if (warp == kNumSoftmaxWarps + 1) {
     // ================= issuer of S = Q K^T =================
-    // One thread issues; what it runs per key tile is kept short (a lone thread executes one instruction every few
-    // cycles): descriptors are built once, a tile's descriptor is the base plus an offset in its low word.
-    if (lane == 0) {
-      const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
-      const uint64_t dk = make_smem_desc(smem_u32(smem + L::k_off), 16, 1024, kLayoutSw128);
-      const uint64_t dsfq = make_smem_desc(smem_u32(smem + L::sfq_off), 0, 128, kLayoutNone);
-      const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::sfk_off), 0, 128, kLayoutNone);
-      uint32_t idesc_kk[4];
+    // The whole warp runs the loop and one elected lane issues: what an MMA takes (descriptors, addresses) then is in uniform registers.
+    // Inside one lane's branch each operand was moved there for every MMA (d <= 128: 660 cycles to issue four).
+    const uint32_t tm = warp_uniform(tmem_base);
+    const int nt = warp_uniform(n_tiles);
+    const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
+    const uint64_t dk = make_smem_desc(smem_u32(smem + L::k_off), 16, 1024, kLayoutSw128);
+    const uint64_t dsfq = make_smem_desc(smem_u32(smem + L::sfq_off), 0, 128, kLayoutNone);
+    const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::sfk_off), 0, 128, kLayoutNone);
+    if (!__all_sync(0xffffffffu, mbar_wait_short(q_full, 0, abort_flag))) fail = 301;
+    if (!fail && elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) idesc_kk[kk] = idesc_with_sf(idesc_qk, kk, kk);
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 301);
-      if (ok) {
-#pragma unroll
-        for (int ch = 0; ch < DCH; ++ch) tc_cp_32x128b_warpx4(tmem_base + kColSfQ + ch * 4, dsfq + (uint32_t)(ch * (kSfAtomBytes >> 4)));
-      }
-      int st = 0, use_par = 0;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        RK_STAMP(2, j, 0);
-        ok = mbar_wait(&k_full[st], use_par, abort_flag, p.status, 302);
-        RK_STAMP(2, j, 1);
-        if (ok && j > 0) ok = mbar_wait(s_empty, (j - 1) & 1, abort_flag, p.status, 305);
-        if (!ok) break;
-        tc_fence_after();
-        RK_STAMP(2, j, 2);
+      for (int ch = 0; ch < DCH; ++ch) tc_cp_32x128b_warpx4(tm + kColSfQ + ch * 4, dsfq + (uint32_t)(ch * (kSfAtomBytes >> 4)));
+    }
+    int st = 0;
+    uint32_t use_par = 0;
+    for (int j = 0; j < nt && !fail; ++j) {
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&k_full[st], use_par, abort_flag))) { fail = 302; break; }
+      if (j > 0 && !__all_sync(0xffffffffu, mbar_wait_short(s_empty, (j - 1) & 1, abort_flag))) { fail = 305; break; }
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int ch = 0; ch < DCH; ++ch)
-          tc_cp_32x128b_warpx4(tmem_base + kColSfK + st * 8 + ch * 4, dsfk + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
+          tc_cp_32x128b_warpx4(tm + kColSfK + st * 8 + ch * 4, dsfk + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
 #pragma unroll
         for (int ch = 0; ch < DCH; ++ch) {
           const uint64_t dqt = dq + (uint32_t)(ch * (kTileBytes >> 4));
           const uint64_t dkt = dk + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tmem_base + kColS, dqt + kk * 2, dkt + kk * 2, idesc_kk[kk], tmem_base + kColSfQ + ch * 4,
-                            tmem_base + kColSfK + st * 8 + ch * 4, (ch > 0 || kk > 0) ? 1u : 0u);
+            mma_mxf8f6f4_ss(tm + kColS, dqt + kk * 2, dkt + kk * 2, idesc_with_sf(idesc_qk, kk, kk), tm + kColSfQ + ch * 4, tm + kColSfK + st * 8 + ch * 4,
+                            (ch > 0 || kk > 0) ? 1u : 0u);
         }
-        tc_commit(&k_empty[st]);
         tc_commit(s_full);
-        RK_STAMP(2, j, 3);
-        if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
+        tc_commit(&k_empty[st]);
       }
-      // make sure nothing issued from this thread is still running before TMEM is released
-      tc_commit(drain);
-      mbar_wait(drain, 0, abort_flag, p.status, 306);
+      if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
     }
+    // make sure nothing issued from this warp is still running before TMEM is released
+    if (elect_one()) tc_commit(drain);
+    if (!mbar_wait_short<true>(drain, 0, nullptr) && !fail) fail = 306;
+    if (fail) report_wait_failure(abort_flag, p.status, fail);
     __syncwarp();
   } else {
     // ================= issuer of O += P V =================
-    if (lane == 0) {
-      const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), 16, 1024, kLayoutSw128);
-      // B = V tile, MN-major (d contiguous): 32 keys = 32 rows of 128 bytes; a 6-bit V is stored transposed,
-      // [d][keys], and is K-major like the K tile of QK^T
-      const uint64_t dv = p.v_transposed ? make_smem_desc(smem_u32(smem + L::v_off), 16, 1024, kLayoutSw128)
-                                         : make_smem_desc(smem_u32(smem + L::v_off), kTileBytes, 1024, kLayoutSw128);
-      const uint32_t v_kk = p.v_transposed ? 2u : (uint32_t)(4096 >> 4);
-      const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
-      const uint64_t dsfv = make_smem_desc(smem_u32(smem + L::sfv_off), 0, 128, kLayoutNone);
-      uint32_t idesc_kk[4];
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) idesc_kk[kk] = idesc_with_sf(idesc_pv, kk, kk);
-      bool ok = true;
-      int st = 0, use_par = 0;
-      for (int i = 0; i < n_tiles && ok; ++i) {
-        const int pb = i & 1;
-        ok = mbar_wait(&v_full[st], use_par, abort_flag, p.status, 303) &&
-             mbar_wait(&p_full[pb], (i >> 1) & 1, abort_flag, p.status, 304);
-        if (!ok) break;
-        tc_fence_after();
-        tc_cp_32x128b_warpx4(tmem_base + kColSfP + pb * 4, dsfp + (uint32_t)(pb * (kSfAtomBytes >> 4)));
+    const uint32_t tm = warp_uniform(tmem_base);
+    const int nt = warp_uniform(n_tiles);
+    const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), 16, 1024, kLayoutSw128);
+    // B = V tile, MN-major (d contiguous): 32 keys = 32 rows of 128 bytes, the second 128 columns of d a tile further on; a 6-bit V
+    // is stored transposed, [d][keys], and is K-major like the K tile of QK^T.
+    const uint64_t dv = p.v_transposed ? make_smem_desc(smem_u32(smem + L::v_off), 16, 1024, kLayoutSw128)
+                                       : make_smem_desc(smem_u32(smem + L::v_off), kTileBytes, 1024, kLayoutSw128);
+    const uint32_t v_kk = p.v_transposed ? 2u : (uint32_t)(4096 >> 4);
+    const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
+    const uint64_t dsfv = make_smem_desc(smem_u32(smem + L::sfv_off), 0, 128, kLayoutNone);
+    int st = 0;
+    uint32_t use_par = 0;
+    for (int i = 0; i < nt; ++i) {
+      const int pb = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&v_full[st], use_par, abort_flag))) { fail = 303; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&p_full[pb], (i >> 1) & 1, abort_flag))) { fail = 304; break; }
+      tc_fence_after();
+      const uint64_t dpt = dp + (uint32_t)(pb * (kTileBytes >> 4));
+      if (elect_one()) {
+        tc_cp_32x128b_warpx4(tm + kColSfP + pb * 4, dsfp + (uint32_t)(pb * (kSfAtomBytes >> 4)));
 #pragma unroll
         for (int ch = 0; ch < DCH; ++ch)
-          tc_cp_32x128b_warpx4(tmem_base + kColSfV + st * 8 + ch * 4, dsfv + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
-        const uint64_t dpt = dp + (uint32_t)(pb * (kTileBytes >> 4));
+          tc_cp_32x128b_warpx4(tm + kColSfV + st * 8 + ch * 4, dsfv + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
 #pragma unroll
         for (int ch = 0; ch < DCH; ++ch) {
           const uint64_t dvt = dv + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tmem_base + kColO + ch * 128, dpt + kk * 2, dvt + kk * v_kk, idesc_kk[kk],
-                            tmem_base + kColSfP + pb * 4, tmem_base + kColSfV + st * 8 + ch * 4, (i > 0 || kk > 0) ? 1u : 0u);
+            mma_mxf8f6f4_ss(tm + kColO + ch * 128, dpt + kk * 2, dvt + kk * v_kk, idesc_with_sf(idesc_pv, kk, kk), tm + kColSfP + pb * 4,
+                            tm + kColSfV + st * 8 + ch * 4, (i > 0 || kk > 0) ? 1u : 0u);
         }
-        tc_commit(&v_empty[st]);
         tc_commit(&pv_done[pb]);
-        if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
+        tc_commit(&v_empty[st]);
       }
-      tc_commit(drain2);
-      mbar_wait(drain2, 0, abort_flag, p.status, 308);
+      if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
     }
+    if (elect_one()) tc_commit(drain2);
+    if (!mbar_wait_short<true>(drain2, 0, nullptr) && !fail) fail = 308;
+    if (fail) report_wait_failure(abort_flag, p.status, fail);
     __syncwarp();
   }
 
