@@ -45,12 +45,61 @@ struct SmemLayout {
   static constexpr int sfv_off = sfk_off + KV_STAGES * DCH * kSfAtomBytes;
   static constexpr int sfp_off = sfv_off + KV_STAGES * DCH * kSfAtomBytes;
   static constexpr int bar_off = sfp_off + 2 * kSfAtomBytes;
-  // barriers: q_full, k_full[S], k_empty[S], v_full[S], v_empty[S], s_full, s_empty, p_full[2], pv_done[2], drain, pair[4], drain2
-  static constexpr int n_bars = 1 + 4 * KV_STAGES + 2 + 4 + 1 + 4 + 1;
+  // barriers: q_full, k_full[S], k_empty[S], v_full[S], v_empty[S], s_full, s_empty, p_full[2], pv_done[2], drain, pair[4], drain2, q_empty,
+  // answer about the next item, item published, item read by all; one to fill 16 bytes
+  static constexpr int n_bars = 1 + 4 * KV_STAGES + 2 + 4 + 1 + 4 + 1 + 4 + 1;
+  static_assert(n_bars % 2 == 0, "what follows is 16-byte aligned");
   static constexpr int misc_off = bar_off + n_bars * 8;
-  static constexpr int xchg_off = misc_off + 16;          // row-max / row-sum exchange: 3 x kParts x 128 floats
+  static constexpr int clc_off = misc_off + 16;
+  static constexpr int work_off = clc_off + 16;
+  static constexpr int xchg_off = work_off + 32;          // row-max / row-sum exchange: 3 x kParts x 128 floats
   static constexpr int total = xchg_off + 3 * kParts * 128 * 4;
 };
+
+// One work item: a query tile of a (batch, head).
+struct __align__(16) Item {
+  int qt;                  // query tile; -1: no item is left
+  int bh, bhkv;            // b * H + h, b * H_kv + h / group
+  int n_tiles, j0;         // key tiles, first key tile inside the window
+  int pad[3];
+};
+static_assert(sizeof(Item) == 32, "its place in shared memory");
+
+// What a softmax thread keeps from item to item.
+struct SoftmaxState {
+  int t;                   // key tiles of earlier items
+  uint32_t quad_par;       // parity of the next meeting of a lane quadrant's warps
+  int out_qt, out_bh;      // the item whose O is still in TMEM
+  float out_inv_l, out_lse;   // 1 / row sum of this thread's row, its log-sum-exp
+};
+
+// O / l -> bf16, each thread d / kParts of the columns of its row (finalize_O, kernels/flash_attention_mx_gqa/flash_mx_impl.hpp:535-553).
+__device__ __forceinline__ void write_out_rows(const PrefillParams& p, uint32_t tmem_base, const SoftmaxState& st) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = warp >> 2;
+  const int q_row = st.out_qt * kBlockM + quad * 32 + lane;
+  const bool live = q_row < p.S_q;
+  __nv_bfloat16* orow = p.o + ((size_t)st.out_bh * p.S_q + q_row) * p.d;
+  if (p.lse && live && part == 0) p.lse[(size_t)st.out_bh * p.S_q + q_row] = st.out_lse;
+  const int ncols = p.d / kParts;                 // 16, 32 or 64 output columns per thread
+#pragma unroll 1
+  for (int c16 = 0; c16 < ncols / 16; ++c16) {
+    uint32_t r[16];
+    const int col0 = part * ncols + c16 * 16;
+    tmem_ld16(tmem_base + (((uint32_t)(quad * 32)) << 16) + kColO + col0, r);
+    tc_wait_ld();
+    if (live) {
+      uint32_t packed[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * st.out_inv_l, __uint_as_float(r[2 * i + 1]) * st.out_inv_l);
+        packed[i] = *reinterpret_cast<const uint32_t*>(&b2);
+      }
+      uint4* dst = reinterpret_cast<uint4*>(orow + col0);
+      dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+    }
+  }
+}
 
 // ---- softmax warps -----------------------------------------------------------------------------
 // 4 * kParts warps: warp w serves TMEM lane quadrant q = w & 3 (rows 32q..32q+31) and the 32-key block
@@ -58,8 +107,8 @@ struct SmemLayout {
 // exchange their block maxima through shared memory (one bounded mbarrier per quadrant, one arrival per
 // warp); everything else is private.
 template <int DCH, int KV_STAGES, bool SOFTCAP, bool DUMP>
-__device__ __forceinline__ void softmax_rows(const PrefillParams& p, uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
-                                             volatile int* abort_flag, int qt, int bh, int n_tiles, int j0) {
+__device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
+                                             volatile int* abort_flag, int qt, int bh, int n_tiles, int j0, SoftmaxState& state) {
   using L = SmemLayout<DCH, KV_STAGES>;
   uint64_t* s_full = bars + 1 + 4 * KV_STAGES;
   uint64_t* s_empty = s_full + 1;
@@ -81,16 +130,17 @@ __device__ __forceinline__ void softmax_rows(const PrefillParams& p, uint8_t* sm
   float m_run = NEG_INF;   // running max, log2 domain (score * log2 e)
   float l_run = 0.0f;      // this thread's share of the row sum
   bool ok = true;
+  int fail = 0;            // which wait gave up
 
   // The body of a key tile exists twice: PLAIN for tiles no row of which needs a mask, and the general one with the
   // mask code.  The loop over plain tiles runs nearly all the time and is kept small and contiguous (the softmax
   // warps stall on instruction fetch; code inside the loop costs time even when it is jumped over).
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
-    const int pb = j & 1;
+    const int t = state.t + j, pb = t & 1;                    // barriers and buffers count on from item to item
     const int sslot = (warp == 0) ? 0 : (warp == 15 ? 1 : 7);
     if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 0);
-    if (!__all_sync(0xffffffffu, mbar_wait(s_full, j & 1, abort_flag, p.status, 101))) return false;
+    if (!__all_sync(0xffffffffu, mbar_wait_short(s_full, t & 1, abort_flag))) { fail = 101; return false; }
     tc_fence_after();
     if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 1);
 
@@ -154,7 +204,8 @@ __device__ __forceinline__ void softmax_rows(const PrefillParams& p, uint8_t* sm
       xchg[(pb * kParts + part) * 128 + row] = bmax;
       __syncwarp();
       if (lane == 0) mbar_arrive(&quadbar[quad]);
-      if (!__all_sync(0xffffffffu, mbar_wait(&quadbar[quad], j & 1, abort_flag, p.status, 104))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&quadbar[quad], state.quad_par, abort_flag))) { fail = 104; return false; }
+      state.quad_par ^= 1;
 #pragma unroll
       for (int o = 1; o < kParts; ++o) mx = fmaxf(mx, xchg[(pb * kParts + ((part + o) & (kParts - 1))) * 128 + row]);
     }
@@ -229,10 +280,12 @@ __device__ __forceinline__ void softmax_rows(const PrefillParams& p, uint8_t* sm
     if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 4);
     // ---- rescale this thread's share of O in TMEM once the previous PV has landed (it had the whole
     //      exp/requant phase above to finish, so this wait is normally free) ----------------------------
-    if (j > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, p.status, 102))) return false;
+    if (t > 0) {
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag))) { fail = 102; return false; }
       tc_fence_after();
-      if (__any_sync(0xffffffffu, corr != 1.0f)) {
+      if (j == 0) {
+        write_out_rows(p, tmem_base, state);                  // O of the item before this one: its last P V ran under this tile's softmax
+      } else if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll 1
         for (int ch = 0; ch < kOCols / 32; ++ch) {
           uint32_t r[32];
@@ -271,54 +324,28 @@ __device__ __forceinline__ void softmax_rows(const PrefillParams& p, uint8_t* sm
   for (; j < n_plain && ok; ++j) ok = tile(j, std::true_type{});
   for (; j < n_tiles && ok; ++j) ok = tile(j, std::false_type{});
 
-  // ---- epilogue: O / l -> bf16, each thread d / kParts of the columns -------------------------------
+  // ---- end of the item: the row's sum and log-sum-exp; O is written out under the next item's first tile ---------------
   float l_tot = l_run;
   if (ok) {
     xchg[(2 * kParts + part) * 128 + row] = l_run;
     __syncwarp();
     if (lane == 0) mbar_arrive(&quadbar[quad]);
-    ok = __all_sync(0xffffffffu, mbar_wait(&quadbar[quad], SOFTCAP ? (n_tiles & 1) : 0, abort_flag, p.status, 105));
-    if (ok) {
+    ok = __all_sync(0xffffffffu, mbar_wait_short(&quadbar[quad], state.quad_par, abort_flag));
+    state.quad_par ^= 1;
+    if (!ok) fail = 105;
 #pragma unroll
-      for (int o = 1; o < kParts; ++o) l_tot += xchg[(2 * kParts + ((part + o) & (kParts - 1))) * 128 + row];
-    }
+    for (int o = 1; o < kParts; ++o) l_tot += xchg[(2 * kParts + ((part + o) & (kParts - 1))) * 128 + row];
   }
-  if (ok) {
-    const int last = n_tiles - 1;
-    ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[last & 1], (last >> 1) & 1, abort_flag, p.status, 103));
+  if (!ok) { give_up(abort_flag, p.status, fail); return false; }
+  state.t += n_tiles;
+  state.out_qt = qt; state.out_bh = bh;
+  state.out_inv_l = (l_tot > 0.0f) ? 1.0f / l_tot : 1.0f;
+  if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && part == 0) {
+    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 0] = m_run;
+    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 1] = l_tot;
   }
-  if (ok) {
-    tc_fence_after();
-    const float inv_l = (l_tot > 0.0f) ? 1.0f / l_tot : 1.0f;
-    const bool live = q_row < p.S_q;
-    __nv_bfloat16* orow = p.o + ((size_t)bh * p.S_q + q_row) * p.d;
-    const int ncols = p.d / kParts;                 // 16, 32 or 64 output columns per thread
-    if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && part == 0) {
-      p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 0] = m_run;
-      p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 1] = l_tot;
-    }
-#pragma unroll 1
-    for (int c16 = 0; c16 < ncols / 16; ++c16) {
-      uint32_t r[16];
-      const int col0 = part * ncols + c16 * 16;
-      tmem_ld16(tmem_base + lane_addr + kColO + col0, r);
-      tc_wait_ld();
-      if (live) {
-        uint32_t packed[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * inv_l, __uint_as_float(r[2 * i + 1]) * inv_l);
-          packed[i] = *reinterpret_cast<const uint32_t*>(&b2);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(orow + col0);
-        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      }
-    }
-    if (p.lse && live && part == 0)
-      p.lse[(size_t)bh * p.S_q + q_row] = (l_tot > 0.0f) ? m_run * 0.6931471805599453f + logf(l_tot) : NEG_INF;
-  }
-  tc_fence_before();
+  state.out_lse = (l_tot > 0.0f) ? m_run * 0.6931471805599453f + logf(l_tot) : NEG_INF;
+  return true;
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
@@ -345,155 +372,233 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint64_t* pv_done = p_full + 2;
   uint64_t* drain = pv_done + 2;
   uint64_t* drain2 = drain + 5;       // after the four pair barriers
+  uint64_t* q_empty = drain2 + 1;
+  uint64_t* clc_bar = q_empty + 1;
+  uint64_t* work_full = clc_bar + 1;
+  uint64_t* work_empty = work_full + 1;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int fail = 0;                                      // which wait of an issuer gave up
-  // heavy (late) query tiles first within a head; heads adjacent so a KV head's tiles share L2
-  // work order: see PrefillParams::head_group (heaviest query tiles of a whole group of heads first)
-  const int n_bh = p.B * p.H;
-  const int per_group = p.n_q_tiles * p.head_group;
-  const int grp_i = (int)blockIdx.x / per_group, r = (int)blockIdx.x % per_group;
-  const int heads_here = min(p.head_group, n_bh - grp_i * p.head_group);
-  const int qt = p.n_q_tiles - 1 - r / heads_here;
-  const int bh_lin = grp_i * p.head_group + r % heads_here;
-  const int h = bh_lin % p.H, b = bh_lin / p.H;
-  const int bh = b * p.H + h;
-  const int bhkv = b * p.H_kv + h / (p.H / p.H_kv);
+  // work order over the block indices: see PrefillParams::head_group (heaviest query tiles of a whole group of heads first)
+  auto decode = [&](uint32_t block) -> Item {
+    Item w;
+    const uint32_t n_bh = p.B * p.H, per_group = p.n_q_tiles * p.head_group;
+    const uint32_t grp_i = block / per_group, r = block - grp_i * per_group;
+    const uint32_t heads_here = min((uint32_t)p.head_group, n_bh - grp_i * p.head_group);
+    const uint32_t down = r / heads_here;
+    w.qt = p.n_q_tiles - 1 - (int)down;
+    w.bh = grp_i * p.head_group + (r - down * heads_here);
+    w.bhkv = (uint32_t)w.bh / (uint32_t)p.group;
+    // key tiles this query tile needs: causal tiles wholly above the diagonal are never touched
+    // (blocks_used, kernels/flash_attention_mx_gqa/flash_attention_model.py:182-186)
+    w.n_tiles = p.n_kv_tiles;
+    if (p.causal) {
+      const int max_qpos = p.q_pos0 + min(w.qt * kBlockM + kBlockM, p.S_q) - 1;
+      w.n_tiles = max_qpos < 0 ? 0 : min(w.n_tiles, max_qpos / kBlockN + 1);
+    }
+    // sliding window: key tiles wholly below the window of the tile's first row are masked for every row of it
+    w.j0 = 0;
+    if (p.window > 0) {
+      const int first_key = p.q_pos0 + w.qt * kBlockM - p.window + 1;      // lowest key the first row may see
+      w.j0 = min(max(first_key, 0) / kBlockN, max(w.n_tiles - 1, 0));
+      w.n_tiles -= w.j0;                                                    // tiles j0 .. j0 + n_tiles - 1 are visited
+    }
+    w.pad[0] = w.pad[1] = w.pad[2] = 0;
+    return w;
+  };
+  Item w = {};
 
-  // key tiles this query tile needs: causal tiles wholly above the diagonal are never touched
-  // (blocks_used, kernels/flash_attention_mx_gqa/flash_attention_model.py:182-186)
-  int n_tiles = p.n_kv_tiles;
-  if (p.causal) {
-    const int max_qpos = p.q_pos0 + min(qt * kBlockM + kBlockM, p.S_q) - 1;
-    n_tiles = max_qpos < 0 ? 0 : min(n_tiles, max_qpos / kBlockN + 1);
-  }
-  // sliding window: key tiles wholly below the window of the tile's first row are masked for every row of it
-  int j0 = 0;
-  if (p.window > 0) {
-    const int first_key = p.q_pos0 + qt * kBlockM - p.window + 1;      // lowest key the first row may see
-    j0 = min(max(first_key, 0) / kBlockN, max(n_tiles - 1, 0));
-    n_tiles -= j0;                                                      // tiles j0 .. j0 + n_tiles - 1 are visited
-  }
-
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int i = 0; i < KV_STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    mbar_init(s_full, 1); mbar_init(s_empty, kNumSoftmaxWarps);
-    mbar_init(&p_full[0], kNumSoftmaxWarps); mbar_init(&p_full[1], kNumSoftmaxWarps);
-    mbar_init(&pv_done[0], 1); mbar_init(&pv_done[1], 1);
-    mbar_init(drain, 1); mbar_init(drain2, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&drain[1 + i], kParts);
-    *abort_flag = 0;
+  // The TMA warp sets up the barriers and goes on to its loads without waiting for the others, so that their latency runs under the
+  // rest of the set-up.
+  if (warp == kNumSoftmaxWarps) {
+    if (lane == 0) {
+      *abort_flag = 0;
+    }
+    for (int i = lane; i < L::n_bars; i += 32) {
+      uint64_t* bar = bars + i;
+      const int count = bar == s_empty || bar == p_full || bar == p_full + 1 ? kNumSoftmaxWarps
+                        : bar > drain && bar < drain2                        ? kParts
+                        : bar == work_empty                                  ? kNumSoftmaxWarps + 2
+                                                                             : 1;
+      mbar_init(bar, count);
+    }
     fence_barrier_init();
+    __syncwarp();
   }
   if (warp == kNumSoftmaxWarps + 1) { tmem_alloc(tmem_ptr, kTmemCols); tmem_relinquish(); }
-  grid_dependency_wait();
-  grid_dependents_launch();
   tc_fence_before();
-  // an earlier launch on this device gave up on a wait: do nothing until the host has read the status
-  const int stopped = __syncthreads_or(threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0);
+  if (warp == kNumSoftmaxWarps) asm volatile("bar.arrive 1, %0;" ::"n"(kNumThreads) : "memory");
+  else asm volatile("bar.sync 1, %0;" ::"n"(kNumThreads) : "memory");
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
-  if (stopped) {
-    if (warp == kNumSoftmaxWarps + 1) tmem_dealloc(tmem_base, kTmemCols);
-    return;
+  if (warp != kNumSoftmaxWarps) {                    // (the TMA producer waits where it starts its loads)
+    grid_dependency_wait();
+    grid_dependents_launch();
   }
+  const uint32_t tmem_base = warp == kNumSoftmaxWarps ? 0u : *tmem_ptr;
 
-  if (n_tiles == 0) {
-    // no visible key: O = 0 (the l <= 0 guard of finalize_O, kernels/flash_attention_mx_gemma/flash_mx_impl.hpp:554-560)
-    if (warp < 4) {
-      const int q_row = qt * kBlockM + threadIdx.x;
-      if (q_row < p.S_q) {
-        __nv_bfloat16* orow = p.o + ((size_t)bh * p.S_q + q_row) * p.d;
-        for (int c = 0; c < p.d; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0, 0, 0, 0);
-        if (p.lse) p.lse[(size_t)bh * p.S_q + q_row] = __int_as_float(0xff800000);
+  // The next item, for every warp but the TMA producer's: 1 taken, 0 none left, -1 a wait gave up.
+  uint32_t work_par = 0;
+  auto next_work = [&]() -> int {
+    if (!__all_sync(0xffffffffu, mbar_wait_short(work_full, work_par, abort_flag))) return -1;
+    work_par ^= 1;
+    w = *reinterpret_cast<const Item*>(smem + L::work_off);
+    if (w.qt < 0) return 0;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(work_empty);
+    return 1;
+  };
+  constexpr int kFailWork = 501;
+
+  if (warp < kNumSoftmaxWarps) {
+    SoftmaxState state = {0, 0, 0, 0, 0.0f, 0.0f};
+    int more;
+    while ((more = next_work()) != 0) {
+      if (more < 0) { give_up(abort_flag, p.status, kFailWork); break; }
+      if (w.n_tiles > 0) {
+        if (!softmax_rows<DCH, KV_STAGES, SOFTCAP, DUMP>(p, smem, bars, tmem_base, abort_flag, w.qt, w.bh, w.n_tiles, w.j0, state)) { more = -1; break; }
+      } else if (warp < 4) {
+        // no visible key: O = 0 (the l <= 0 guard of finalize_O, kernels/flash_attention_mx_gemma/flash_mx_impl.hpp:554-560)
+        const int q_row = w.qt * kBlockM + threadIdx.x;
+        if (q_row < p.S_q && *reinterpret_cast<volatile int*>(p.status) == 0) {
+          __nv_bfloat16* orow = p.o + ((size_t)w.bh * p.S_q + q_row) * p.d;
+          for (int c = 0; c < p.d; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0, 0, 0, 0);
+          if (p.lse) p.lse[(size_t)w.bh * p.S_q + q_row] = __int_as_float(0xff800000);
+        }
       }
     }
-  } else if (warp < kNumSoftmaxWarps) {
-    softmax_rows<DCH, KV_STAGES, SOFTCAP, DUMP>(p, smem, bars, tmem_base, abort_flag, qt, bh, n_tiles, j0);
+    if (more == 0 && state.t > 0) {                  // O of the last item
+      const int last = state.t - 1;
+      if (__all_sync(0xffffffffu, mbar_wait_short(&pv_done[last & 1], (last >> 1) & 1, abort_flag))) {
+        tc_fence_after();
+        write_out_rows(p, tmem_base, state);
+      } else {
+        give_up(abort_flag, p.status, 103);
+      }
+    }
   } else if (warp == kNumSoftmaxWarps) {
-    // ================= TMA producer =================
+    // ================= TMA producer; hands out the items =================
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      mbar_arrive_expect_tx(q_full, DCH * (p.q_tile_tx + kSfAtomBytes));
-      for (int ch = 0; ch < DCH; ++ch) {
-        tma_load_3d(smem + L::q_off + ch * kTileBytes, &tmap_q, q_full, ch * 128, qt * kBlockM, bh);
-        bulk_load_1d(smem + L::sfq_off + ch * kSfAtomBytes,
-                     p.q_sf + (((size_t)bh * p.n_q_tiles + qt) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, q_full);
-      }
-      bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j % KV_STAGES, use = j / KV_STAGES;
-        if (use > 0) ok = mbar_wait(&k_empty[st], (use - 1) & 1, abort_flag, p.status, 201);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&k_full[st], DCH * (p.kv_tile_tx + kSfAtomBytes));
-        for (int ch = 0; ch < DCH; ++ch) {
-          tma_load_3d(smem + L::k_off + (st * DCH + ch) * kTileBytes, &tmap_k, &k_full[st], ch * 128, (j + j0) * kBlockN, bhkv);
-          bulk_load_1d(smem + L::sfk_off + (st * DCH + ch) * kSfAtomBytes,
-                       p.k_sf + (((size_t)bhkv * p.n_kv_tiles + j + j0) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, &k_full[st]);
+      int stopped = 0, st = 0, q_used = 0;
+      uint32_t use = 0, q_par = 0, block = blockIdx.x;
+      for (uint32_t k = 0;; ++k) {
+        w = decode(block);
+        // everybody has read the last item: this one takes its place, and the one after it is asked for
+        if (k > 0 && !mbar_wait_short<true>(work_empty, (k - 1) & 1, abort_flag)) { fail = 502; break; }
+        *reinterpret_cast<Item*>(smem + L::work_off) = w;
+        mbar_arrive(work_full);
+        if (k == 0) {
+          grid_dependency_wait();
+          stopped = *reinterpret_cast<volatile int*>(p.status);       // an earlier launch gave up on a wait
         }
-        if (use > 0) ok = mbar_wait(&v_empty[st], (use - 1) & 1, abort_flag, p.status, 202);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&v_full[st], DCH * (p.kv_tile_tx + kSfAtomBytes));
-        for (int ch = 0; ch < DCH; ++ch) {
-          if (p.v_transposed)
-            tma_load_3d(smem + L::v_off + (st * DCH + ch) * kTileBytes, &tmap_v, &v_full[st], (j + j0) * kBlockN, ch * 128, bhkv);
-          else
-            tma_load_3d(smem + L::v_off + (st * DCH + ch) * kTileBytes, &tmap_v, &v_full[st], ch * 128, (j + j0) * kBlockN, bhkv);
-          bulk_load_1d(smem + L::sfv_off + (st * DCH + ch) * kSfAtomBytes,
-                       p.v_sf + (((size_t)bhkv * p.n_kv_tiles + j + j0) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, &v_full[st]);
+        mbar_arrive_expect_tx(clc_bar, 16);
+        clc_request(smem + L::clc_off, clc_bar);
+        for (int j = 0; j < w.n_tiles; ++j) {
+          if (j == 0) {
+            if (q_used) {                            // Q K^T of the last item has finished
+              if (!mbar_wait_short<true>(q_empty, q_par, abort_flag)) { fail = 203; break; }
+              q_par ^= 1;
+            }
+            q_used = 1;
+            mbar_arrive_expect_tx(q_full, DCH * (p.q_tile_tx + kSfAtomBytes));
+            for (int ch = 0; ch < DCH; ++ch) {
+              tma_load_3d(smem + L::q_off + ch * kTileBytes, &tmap_q, q_full, ch * 128, w.qt * kBlockM, w.bh);
+              bulk_load_1d(smem + L::sfq_off + ch * kSfAtomBytes,
+                           p.q_sf + (((size_t)w.bh * p.n_q_tiles + w.qt) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, q_full);
+            }
+          }
+          if (use > 0 && !mbar_wait_short<true>(&k_empty[st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
+          mbar_arrive_expect_tx(&k_full[st], DCH * (p.kv_tile_tx + kSfAtomBytes));
+          const int key = (j + w.j0) * kBlockN;
+          for (int ch = 0; ch < DCH; ++ch) {
+            tma_load_3d(smem + L::k_off + (st * DCH + ch) * kTileBytes, &tmap_k, &k_full[st], ch * 128, key, w.bhkv);
+            bulk_load_1d(smem + L::sfk_off + (st * DCH + ch) * kSfAtomBytes,
+                         p.k_sf + (((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, &k_full[st]);
+          }
+          if (stopped) break;                        // O is written only where V has come
+          if (use > 0 && !mbar_wait_short<true>(&v_empty[st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
+          mbar_arrive_expect_tx(&v_full[st], DCH * (p.kv_tile_tx + kSfAtomBytes));
+          for (int ch = 0; ch < DCH; ++ch) {         // transposed V: [d][keys]
+            tma_load_3d(smem + L::v_off + (st * DCH + ch) * kTileBytes, &tmap_v, &v_full[st], p.v_transposed ? key : ch * 128,
+                        p.v_transposed ? ch * 128 : key, w.bhkv);
+            bulk_load_1d(smem + L::sfv_off + (st * DCH + ch) * kSfAtomBytes,
+                         p.v_sf + (((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, &v_full[st]);
+          }
+          if (++st == KV_STAGES) { st = 0; ++use; }
         }
+        if (stopped) {
+          *abort_flag = kStopped;
+          if (w.n_tiles > 0) { mbar_wait_short<true>(q_full, 0, nullptr); mbar_wait_short<true>(&k_full[0], 0, nullptr); }
+        }
+        if (!mbar_wait_short<true>(clc_bar, k & 1, nullptr) && !fail) fail = 503;      // (also where the CTA gives up)
+        if (fail || stopped) break;
+        if (!clc_answer(smem + L::clc_off, block)) {
+          if (!mbar_wait_short<true>(work_empty, k & 1, abort_flag)) { fail = 502; break; }
+          w.qt = -1;
+          *reinterpret_cast<Item*>(smem + L::work_off) = w;
+          mbar_arrive(work_full);
+          break;
+        }
+        fence_proxy_async_smem();                    // the answer has been read before the next one may overwrite it
       }
+      if (fail) give_up(abort_flag, p.status, fail);
     }
+    __syncwarp();
   } else if (warp == kNumSoftmaxWarps + 1) {
     // ================= issuer of S = Q K^T =================
     // The whole warp runs the loop and one elected lane issues: what an MMA takes (descriptors, addresses) then is in uniform registers.
     // Inside one lane's branch each operand was moved there for every MMA (d <= 128: 660 cycles to issue four).
     const uint32_t tm = warp_uniform(tmem_base);
-    const int nt = warp_uniform(n_tiles);
     const uint64_t dq = make_smem_desc(smem_u32(smem + L::q_off), 16, 1024, kLayoutSw128);
     const uint64_t dk = make_smem_desc(smem_u32(smem + L::k_off), 16, 1024, kLayoutSw128);
     const uint64_t dsfq = make_smem_desc(smem_u32(smem + L::sfq_off), 0, 128, kLayoutNone);
     const uint64_t dsfk = make_smem_desc(smem_u32(smem + L::sfk_off), 0, 128, kLayoutNone);
-    if (!__all_sync(0xffffffffu, mbar_wait_short(q_full, 0, abort_flag))) fail = 301;
-    if (!fail && elect_one()) {
-#pragma unroll
-      for (int ch = 0; ch < DCH; ++ch) tc_cp_32x128b_warpx4(tm + kColSfQ + ch * 4, dsfq + (uint32_t)(ch * (kSfAtomBytes >> 4)));
-    }
-    int st = 0;
-    uint32_t use_par = 0;
-    for (int j = 0; j < nt && !fail; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&k_full[st], use_par, abort_flag))) { fail = 302; break; }
-      if (j > 0 && !__all_sync(0xffffffffu, mbar_wait_short(s_empty, (j - 1) & 1, abort_flag))) { fail = 305; break; }
-      tc_fence_after();
-      if (elect_one()) {
-#pragma unroll
-        for (int ch = 0; ch < DCH; ++ch)
-          tc_cp_32x128b_warpx4(tm + kColSfK + st * 8 + ch * 4, dsfk + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
-#pragma unroll
-        for (int ch = 0; ch < DCH; ++ch) {
-          const uint64_t dqt = dq + (uint32_t)(ch * (kTileBytes >> 4));
-          const uint64_t dkt = dk + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tm + kColS, dqt + kk * 2, dkt + kk * 2, idesc_with_sf(idesc_qk, kk, kk), tm + kColSfQ + ch * 4, tm + kColSfK + st * 8 + ch * 4,
-                            (ch > 0 || kk > 0) ? 1u : 0u);
+    int st = 0, t = 0;                               // t: key tiles so far
+    uint32_t use_par = 0, q_par = 0;
+    for (int more; !fail && (more = warp_uniform(next_work())) != 0;) {
+      if (more < 0) { fail = kFailWork; break; }
+      const int nt = warp_uniform(w.n_tiles);
+      for (int j = 0; j < nt; ++j, ++t) {
+        if (j == 0) {
+          if (!__all_sync(0xffffffffu, mbar_wait_short(q_full, q_par, abort_flag))) { fail = 301; break; }
+          q_par ^= 1;
+          if (elect_one()) {
+  #pragma unroll
+            for (int ch = 0; ch < DCH; ++ch) tc_cp_32x128b_warpx4(tm + kColSfQ + ch * 4, dsfq + (uint32_t)(ch * (kSfAtomBytes >> 4)));
+          }
         }
-        tc_commit(s_full);
-        tc_commit(&k_empty[st]);
+        if (!__all_sync(0xffffffffu, mbar_wait_short(&k_full[st], use_par, abort_flag))) { fail = 302; break; }
+        if (t > 0 && !__all_sync(0xffffffffu, mbar_wait_short(s_empty, (t - 1) & 1, abort_flag))) { fail = 305; break; }
+        tc_fence_after();
+        if (elect_one()) {
+  #pragma unroll
+          for (int ch = 0; ch < DCH; ++ch)
+            tc_cp_32x128b_warpx4(tm + kColSfK + st * 8 + ch * 4, dsfk + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
+  #pragma unroll
+          for (int ch = 0; ch < DCH; ++ch) {
+            const uint64_t dqt = dq + (uint32_t)(ch * (kTileBytes >> 4));
+            const uint64_t dkt = dk + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
+  #pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              mma_mxf8f6f4_ss(tm + kColS, dqt + kk * 2, dkt + kk * 2, idesc_with_sf(idesc_qk, kk, kk), tm + kColSfQ + ch * 4, tm + kColSfK + st * 8 + ch * 4,
+                              (ch > 0 || kk > 0) ? 1u : 0u);
+          }
+          tc_commit(s_full);
+          tc_commit(&k_empty[st]);
+          if (j == nt - 1) tc_commit(q_empty);
+        }
+        if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
       }
-      if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
     }
     // make sure nothing issued from this warp is still running before TMEM is released
     if (elect_one()) tc_commit(drain);
     if (!mbar_wait_short<true>(drain, 0, nullptr) && !fail) fail = 306;
-    if (fail) report_wait_failure(abort_flag, p.status, fail);
+    if (fail) give_up(abort_flag, p.status, fail);
     __syncwarp();
   } else {
     // ================= issuer of O += P V =================
     const uint32_t tm = warp_uniform(tmem_base);
-    const int nt = warp_uniform(n_tiles);
     const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), 16, 1024, kLayoutSw128);
     // B = V tile, MN-major (d contiguous): 32 keys = 32 rows of 128 bytes, the second 128 columns of d a tile further on; a 6-bit V
     // is stored transposed, [d][keys], and is K-major like the K tile of QK^T.
@@ -502,35 +607,39 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const uint32_t v_kk = p.v_transposed ? 2u : (uint32_t)(4096 >> 4);
     const uint64_t dsfp = make_smem_desc(smem_u32(smem + L::sfp_off), 0, 128, kLayoutNone);
     const uint64_t dsfv = make_smem_desc(smem_u32(smem + L::sfv_off), 0, 128, kLayoutNone);
-    int st = 0;
+    int st = 0, t = 0;
     uint32_t use_par = 0;
-    for (int i = 0; i < nt; ++i) {
-      const int pb = i & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&v_full[st], use_par, abort_flag))) { fail = 303; break; }
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&p_full[pb], (i >> 1) & 1, abort_flag))) { fail = 304; break; }
-      tc_fence_after();
-      const uint64_t dpt = dp + (uint32_t)(pb * (kTileBytes >> 4));
-      if (elect_one()) {
-        tc_cp_32x128b_warpx4(tm + kColSfP + pb * 4, dsfp + (uint32_t)(pb * (kSfAtomBytes >> 4)));
-#pragma unroll
-        for (int ch = 0; ch < DCH; ++ch)
-          tc_cp_32x128b_warpx4(tm + kColSfV + st * 8 + ch * 4, dsfv + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
-#pragma unroll
-        for (int ch = 0; ch < DCH; ++ch) {
-          const uint64_t dvt = dv + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_mxf8f6f4_ss(tm + kColO + ch * 128, dpt + kk * 2, dvt + kk * v_kk, idesc_with_sf(idesc_pv, kk, kk), tm + kColSfP + pb * 4,
-                            tm + kColSfV + st * 8 + ch * 4, (i > 0 || kk > 0) ? 1u : 0u);
+    for (int more; !fail && (more = warp_uniform(next_work())) != 0;) {
+      if (more < 0) { fail = kFailWork; break; }
+      const int nt = warp_uniform(w.n_tiles);
+      for (int i = 0; i < nt; ++i, ++t) {
+        const int pb = t & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait_short(&v_full[st], use_par, abort_flag))) { fail = 303; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait_short(&p_full[pb], (t >> 1) & 1, abort_flag))) { fail = 304; break; }      // (and O of the last item has been read)
+        tc_fence_after();
+        const uint64_t dpt = dp + (uint32_t)(pb * (kTileBytes >> 4));
+        if (elect_one()) {
+          tc_cp_32x128b_warpx4(tm + kColSfP + pb * 4, dsfp + (uint32_t)(pb * (kSfAtomBytes >> 4)));
+  #pragma unroll
+          for (int ch = 0; ch < DCH; ++ch)
+            tc_cp_32x128b_warpx4(tm + kColSfV + st * 8 + ch * 4, dsfv + (uint32_t)((st * DCH + ch) * (kSfAtomBytes >> 4)));
+  #pragma unroll
+          for (int ch = 0; ch < DCH; ++ch) {
+            const uint64_t dvt = dv + (uint32_t)((st * DCH + ch) * (kTileBytes >> 4));
+  #pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              mma_mxf8f6f4_ss(tm + kColO + ch * 128, dpt + kk * 2, dvt + kk * v_kk, idesc_with_sf(idesc_pv, kk, kk), tm + kColSfP + pb * 4,
+                              tm + kColSfV + st * 8 + ch * 4, (i > 0 || kk > 0) ? 1u : 0u);
+          }
+          tc_commit(&pv_done[pb]);
+          tc_commit(&v_empty[st]);
         }
-        tc_commit(&pv_done[pb]);
-        tc_commit(&v_empty[st]);
+        if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
       }
-      if (++st == KV_STAGES) { st = 0; use_par ^= 1; }
     }
     if (elect_one()) tc_commit(drain2);
     if (!mbar_wait_short<true>(drain2, 0, nullptr) && !fail) fail = 308;
-    if (fail) report_wait_failure(abort_flag, p.status, fail);
+    if (fail) give_up(abort_flag, p.status, fail);
     __syncwarp();
   }
 

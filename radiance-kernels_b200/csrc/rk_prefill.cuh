@@ -47,6 +47,12 @@ struct PrefillParams {
   float inv_cap_scale; // softmax_scale / softcap
 };
 
+// Value of a CTA's abort flag where an earlier launch gave up on a wait and this one does nothing (its waits end, and nothing is reported).
+constexpr int kStopped = 2;
+RK_DEVINL void give_up(volatile int* abort_flag, int* status, int code) {
+  if (*abort_flag != kStopped) report_wait_failure(abort_flag, status, code);
+}
+
 RK_DEVINL float fmax3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 // packed fp32 pairs (two lanes per instruction on the FMA pipe)
 RK_DEVINL void fma2(float a0, float a1, float b, float c, float& d0, float& d1) {      // d = a * b + c

@@ -82,7 +82,6 @@ struct __align__(16) Work {
   int pad[2];
 };
 static_assert(sizeof(Work) == 32, "its place in shared memory");
-constexpr int kStopped = 2;              // value of the abort flag where an earlier launch gave up and this one does nothing
 constexpr int kReaders = 8 + 4 + 2;      // warps that read an item: softmax, correction, Q K^T, P V
 }  // namespace c2
 
@@ -126,10 +125,6 @@ __device__ __forceinline__ int wait_tile_inputs(uint64_t* s_full, uint32_t s_par
   if (!mbar_wait_short(s_full, s_parity, abort_flag)) return 101;
   if (need_pv && !mbar_wait_short(pv_done, pv_parity, abort_flag)) return 102;
   return 0;
-}
-
-__device__ __forceinline__ void give_up(volatile int* abort_flag, int* status, int code) {
-  if (*abort_flag != c2::kStopped) report_wait_failure(abort_flag, status, code);
 }
 
 template <bool SOFTCAP, bool DUMP, bool SPLIT>
