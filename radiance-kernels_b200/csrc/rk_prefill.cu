@@ -13,12 +13,17 @@
 //   pack_scales_to_sfmem (flash_mx_impl.hpp:625-639)   -> one st.shared per row + tcgen05.cp
 //   rescale_accumulate / finalize_O (:508-553)         -> O kept in TMEM, rescaled in place
 //
-// One CTA = one 128-row query tile of one (batch, head).  608 threads:
-//   warps 0-15  softmax: four threads per query row (TMEM lane = row), one 32-key block of the tile each
-//   warp  16    TMA producer (one elected lane)
-//   warp  17    issuer of the S = Q K^T MMAs (one elected lane), TMEM allocation
-//   warp  18    issuer of the O += P V MMAs (one elected lane): a P V that waits for its P tile never holds back
-//               the next Q K^T, and each issuing thread runs a short instruction stream per key tile
+// A CTA works on one 128-row query tile of one (batch, head) at a time.  640 threads:
+//   warps 0-7   softmax of the even key tiles (counted over all query tiles of the CTA): two threads per query row (TMEM lane
+//               = row), two 32-key blocks each
+//   warps 8-15  softmax of the odd key tiles
+//   warp  16    TMA producer (one elected lane); hands out the query tiles
+//   warp  17    issuer of the S = Q K^T MMAs, TMEM allocation
+//   warp  18    issuer of the O += P V MMAs: a P V that waits for its P tile never holds back the next Q K^T
+//   warp  19    fills the warpgroup (registers are moved between warpgroups with setmaxnreg)
+// The two groups are half a tile apart: while one forms exponentials (special-function unit) the other caps scores, takes maxima and
+// rescales O (FMA and integer pipes).  All sixteen warps in the same phase of the same tile took 3600 cycles a tile with the
+// cap and 2900 without; 2 x 16/8 heads of 8192: capped 974 -> 894 us, without the cap 796 -> 726, two heads of 300 keys 14.5 -> 11.9.
 // Keys are walked in tiles of 128 (the online-softmax step, "block_n").
 //
 // Roofline: tensor-core bound by FLOP count (4*S_q*S_kv*d per head, half of it
@@ -45,15 +50,16 @@ struct SmemLayout {
   static constexpr int sfv_off = sfk_off + KV_STAGES * DCH * kSfAtomBytes;
   static constexpr int sfp_off = sfv_off + KV_STAGES * DCH * kSfAtomBytes;
   static constexpr int bar_off = sfp_off + 2 * kSfAtomBytes;
-  // barriers: q_full, k_full[S], k_empty[S], v_full[S], v_empty[S], s_full, s_empty, p_full[2], pv_done[2], drain, pair[4], drain2, q_empty,
-  // answer about the next item, item published, item read by all; one to fill 16 bytes
-  static constexpr int n_bars = 1 + 4 * KV_STAGES + 2 + 4 + 1 + 4 + 1 + 4 + 1;
+  // barriers: q_full, k_full[S], k_empty[S], v_full[S], v_empty[S], s_full[2], s_empty, p_full[2], pv_done[2], drain, drain2, q_empty,
+  // answer about the next item, item published, item read by all, row_bar[4 tiles][4 quadrants], end_bar[4]
+  static constexpr int n_bars = 1 + 4 * KV_STAGES + 2 + 1 + 2 + 2 + 2 + 4 + 16 + 4;
   static_assert(n_bars % 2 == 0, "what follows is 16-byte aligned");
   static constexpr int misc_off = bar_off + n_bars * 8;
   static constexpr int clc_off = misc_off + 16;
   static constexpr int work_off = clc_off + 16;
-  static constexpr int xchg_off = work_off + 32;          // row-max / row-sum exchange: 3 x kParts x 128 floats
-  static constexpr int total = xchg_off + 3 * kParts * 128 * 4;
+  static constexpr int xchg_off = work_off + 32;              // [4 key tiles][2 parts][128 rows] floats: row maxima of a tile
+  static constexpr int end_off = xchg_off + 4 * 2 * 128 * 4;  // [2 items][2 groups][2 parts][128 rows] float2: row sum and its maximum
+  static constexpr int total = end_off + 2 * 2 * 2 * 128 * 8;
 };
 
 // One work item: a query tile of a (batch, head).
@@ -65,231 +71,252 @@ struct __align__(16) Item {
 };
 static_assert(sizeof(Item) == 32, "its place in shared memory");
 
+constexpr int kNumSoftmaxWarps = 16;
+constexpr int kThreads256 = (kNumSoftmaxWarps + 4) * 32;
+// 512 * 104 + 128 * 64 = 640 * 96, the registers the block is launched with
+constexpr uint32_t kRegSoftmax256 = 104, kRegIssue256 = 64;
+template <uint32_t N> RK_DEVINL void reg_inc256() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <uint32_t N> RK_DEVINL void reg_dec256() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // What a softmax thread keeps from item to item.
 struct SoftmaxState {
   int t;                   // key tiles of earlier items
-  uint32_t quad_par;       // parity of the next meeting of a lane quadrant's warps
-  int out_qt, out_bh;      // the item whose O is still in TMEM
-  float out_inv_l, out_lse;   // 1 / row sum of this thread's row, its log-sum-exp
+  int items;               // earlier items that had key tiles
+  int out_qt, out_bh;      // the last of them, whose O is still in TMEM
 };
+struct SoftmaxBars { uint64_t *s_full, *s_empty, *p_full, *pv_done, *row_bar, *end_bar; };
 
-// O / l -> bf16, each thread d / kParts of the columns of its row (finalize_O, kernels/flash_attention_mx_gqa/flash_mx_impl.hpp:535-553).
-__device__ __forceinline__ void write_out_rows(const PrefillParams& p, uint32_t tmem_base, const SoftmaxState& st) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = warp >> 2;
-  const int q_row = st.out_qt * kBlockM + quad * 32 + lane;
+// O / l -> bf16 (finalize_O, kernels/flash_attention_mx_gqa/flash_mx_impl.hpp:535-553) by one of the two groups: a thread has half of the
+// columns of its row.  The row's sum is in four shares, one per group and part, each relative to the running maximum its threads saw last.
+template <int DCH, int KV_STAGES, bool DUMP>
+__device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* smem, const SoftmaxBars& bars, uint32_t tmem_base,
+                                               volatile int* abort_flag, const SoftmaxState& st) {
+  using L = SmemLayout<DCH, KV_STAGES>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = (warp >> 2) & 1, row = quad * 32 + lane;
+  const int item = st.items - 1;
+  if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.end_bar[quad], item & 1, abort_flag))) return false;
+  const float2* share = reinterpret_cast<const float2*>(smem + L::end_off) + (item & 1) * 4 * 128 + row;
+  const float NEG_INF = __int_as_float(0xff800000);
+  const float m = fmaxf(fmaxf(share[0].y, share[128].y), fmaxf(share[256].y, share[384].y));
+  float l = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) l += share[i * 128].y == NEG_INF ? 0.0f : share[i * 128].x * ex2_approx(share[i * 128].y - m);
+  const float inv_l = (l > 0.0f) ? 1.0f / l : 1.0f;
+  const int q_row = st.out_qt * kBlockM + row;
   const bool live = q_row < p.S_q;
-  __nv_bfloat16* orow = p.o + ((size_t)st.out_bh * p.S_q + q_row) * p.d;
-  if (p.lse && live && part == 0) p.lse[(size_t)st.out_bh * p.S_q + q_row] = st.out_lse;
-  const int ncols = p.d / kParts;                 // 16, 32 or 64 output columns per thread
+  if (DUMP && p.dbg && st.out_qt == p.n_q_tiles - 1 && st.out_bh == 0 && part == 0) {
+    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 0] = m;
+    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 1] = l;
+  }
+  if (p.lse && live && part == 0) p.lse[(size_t)st.out_bh * p.S_q + q_row] = (l > 0.0f) ? m * 0.6931471805599453f + logf(l) : NEG_INF;
+  const int ncols = p.d / 2;
+  __nv_bfloat16* orow = p.o + ((size_t)st.out_bh * p.S_q + q_row) * p.d + part * ncols;
 #pragma unroll 1
-  for (int c16 = 0; c16 < ncols / 16; ++c16) {
-    uint32_t r[16];
-    const int col0 = part * ncols + c16 * 16;
-    tmem_ld16(tmem_base + (((uint32_t)(quad * 32)) << 16) + kColO + col0, r);
+  for (int c = 0; c < ncols; c += 32) {
+    uint32_t r[32];
+    tmem_ld32(tmem_base + (((uint32_t)(quad * 32)) << 16) + kColO + part * ncols + c, r);
     tc_wait_ld();
     if (live) {
-      uint32_t packed[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * st.out_inv_l, __uint_as_float(r[2 * i + 1]) * st.out_inv_l);
-        packed[i] = *reinterpret_cast<const uint32_t*>(&b2);
+      for (int i = 0; i < 4; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i + 2 * e]) * inv_l, __uint_as_float(r[8 * i + 2 * e + 1]) * inv_l);
+          w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+        }
+        *reinterpret_cast<uint4*>(orow + c + 8 * i) = make_uint4(w[0], w[1], w[2], w[3]);
       }
-      uint4* dst = reinterpret_cast<uint4*>(orow + col0);
-      dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-      dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
     }
   }
+  return true;
 }
 
 // ---- softmax warps -----------------------------------------------------------------------------
-// 4 * kParts warps: warp w serves TMEM lane quadrant q = w & 3 (rows 32q..32q+31) and the 32-key block
-// w >> 2 of the tile, so a thread's keys are exactly one MX block of P.  The kParts threads of a row
-// exchange their block maxima through shared memory (one bounded mbarrier per quadrant, one arrival per
-// warp); everything else is private.
+// Group warp >> 3 takes the key tiles of its parity.  Warp w serves TMEM lane quadrant w & 3 (rows 32q..32q+31) and keys 64 * part .. + 63 of
+// the tile.  A tile's row maxima go through shared memory to the row's other thread and to the other group's two, which carry the
+// running maximum on to the next tile (one bounded mbarrier per tile and quadrant); each thread has its share of the row sum.
 template <int DCH, int KV_STAGES, bool SOFTCAP, bool DUMP>
-__device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
+__device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* smem, const SoftmaxBars& bars, uint32_t tmem_base,
                                              volatile int* abort_flag, int qt, int bh, int n_tiles, int j0, SoftmaxState& state) {
   using L = SmemLayout<DCH, KV_STAGES>;
-  uint64_t* s_full = bars + 1 + 4 * KV_STAGES;
-  uint64_t* s_empty = s_full + 1;
-  uint64_t* p_full = s_empty + 1;     // [2]
-  uint64_t* pv_done = p_full + 2;     // [2]
-  uint64_t* quadbar = pv_done + 3;    // [4]: the kParts warps of a lane quadrant meet here (bounded, unlike bar.sync)
-  float* xchg = reinterpret_cast<float*>(smem + L::xchg_off);   // [3][kParts][128 rows]
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int quad = warp & 3, part = warp >> 2;             // TMEM lane quadrant, 32-key block of the tile
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = warp >> 3, part = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
   const uint32_t lane_addr = ((uint32_t)(quad * 32)) << 16;
-  const int q_row = qt * kBlockM + row;
-  const int q_pos = p.q_pos0 + q_row;
   const float NEG_INF = __int_as_float(0xff800000);
-  constexpr int kOCols = DCH * 128 / kParts;               // O columns this thread rescales (32 or 64)
+  const float sc_mul = SOFTCAP ? 1.0f : p.scale_log2;
+  float* xchg = reinterpret_cast<float*>(smem + L::xchg_off) + row;     // + ((t & 3) * 2 + part) * 128
 
-  float m_run = NEG_INF;   // running max, log2 domain (score * log2 e)
-  float l_run = 0.0f;      // this thread's share of the row sum
+  float m_run = NEG_INF;   // running maximum at this thread's last tile, log2 domain (score * log2 e)
+  float l_run = 0.0f;      // this thread's share of the row sum, relative to it
   bool ok = true;
   int fail = 0;            // which wait gave up
 
-  // The body of a key tile exists twice: PLAIN for tiles no row of which needs a mask, and the general one with the
-  // mask code.  The loop over plain tiles runs nearly all the time and is kept small and contiguous (the softmax
-  // warps stall on instruction fetch; code inside the loop costs time even when it is jumped over).
+  // Tiles n_low .. n_high-1 need no mask for any row of this query tile: all 128 keys inside S_kv, the tile's last key not beyond the first
+  // row's position, its first key inside the last row's window.  The body exists twice: PLAIN for those, and with the mask code.
+  int n_low = 0, n_high = min(n_tiles, p.S_kv / kBlockN - j0);
+  {
+    const int q_first = p.q_pos0 + qt * kBlockM, q_last = q_first + kBlockM - 1;
+    if (p.causal) {
+      const int t = q_first - (kBlockN - 1);                            // (j + j0) * kBlockN <= t
+      n_high = min(n_high, t < 0 ? 0 : t / kBlockN + 1 - j0);
+    }
+    if (p.window > 0 && q_last >= p.window) n_low = (q_last - p.window) / kBlockN + 1 - j0;   // (j + j0) * kBlockN <= q_last - window
+  }
+
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
-    const int t = state.t + j, pb = t & 1;                    // barriers and buffers count on from item to item
-    const int sslot = (warp == 0) ? 0 : (warp == 15 ? 1 : 7);
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 0);
-    if (!__all_sync(0xffffffffu, mbar_wait_short(s_full, t & 1, abort_flag))) { fail = 101; return false; }
+    const int t = state.t + j;                                // barriers and buffers count on from item to item; t & 1 == grp
+    if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.s_full[grp], (t >> 1) & 1, abort_flag))) { fail = 101; return false; }
     tc_fence_after();
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 1);
-
-    // mask bounds relative to the tile's first key: key column c is masked iff c > hi || c <= lo
-    const int key0 = (j + j0) * kBlockN;                      // first key of this tile (j counts from the first tile inside the window)
-    const bool tail = (key0 + kBlockN > p.S_kv);
-    const bool diag = p.causal && (key0 + kBlockN - 1 > p.q_pos0 + qt * kBlockM);
-    const bool need_mask = !PLAIN && (tail || diag || (p.window > 0));
-    int hi = p.S_kv - 1 - key0;
-    if (p.causal) hi = min(hi, q_pos - key0);
-    const int lo = (p.window > 0) ? (q_pos - p.window - key0) : -1;
-
-    float s[32];
-    tmem_ld32(tmem_base + lane_addr + kColS + part * 32, reinterpret_cast<uint32_t*>(s));
+    float s[64];
+    tmem_ld32(tmem_base + lane_addr + kColS + part * 64, reinterpret_cast<uint32_t*>(s));
+    tmem_ld32(tmem_base + lane_addr + kColS + part * 64 + 32, reinterpret_cast<uint32_t*>(s) + 32);
     tc_wait_ld();
-    float mx_others = NEG_INF;
-    if (!SOFTCAP) {
-      // Row max without talking to the other warps: read the row's other three 32-key blocks as well
-      // (TMEM reads are cheap) and reduce them here.  The warps of a row then never wait for each other.
-#pragma unroll 1
-      for (int o = 1; o < kParts; ++o) {
-        const int blk = (part + o) & (kParts - 1);
-        float t[32];
-        tmem_ld32(tmem_base + lane_addr + kColS + blk * 32, reinterpret_cast<uint32_t*>(t));
-        tc_wait_ld();
-        if (need_mask) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) t[c] = (blk * 32 + c > hi || blk * 32 + c <= lo) ? NEG_INF : t[c];
-        }
-        float b0 = fmax3(t[0], t[1], t[2]), b1 = fmax3(t[3], t[4], t[5]);
-#pragma unroll
-        for (int c = 6; c < 30; c += 4) { b0 = fmax3(b0, t[c], t[c + 1]); b1 = fmax3(b1, t[c + 2], t[c + 3]); }
-        mx_others = fmax3(mx_others, fmax3(b0, b1, t[30]), t[31]);
-      }
-    }
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(s_empty);        // one arrival per warp: S may be overwritten once all 16 have read
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 2);
-
+    if (lane == 0) mbar_arrive(bars.s_empty);                 // one arrival per warp: the next Q K^T may have S once all 8 have read
     if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && j == 0) {
 #pragma unroll
-      for (int c = 0; c < 32; ++c) p.dbg[row * 128 + part * 32 + c] = s[c];
+      for (int c = 0; c < 64; ++c) p.dbg[row * 128 + part * 64 + c] = s[c];
     }
 
-    // ---- (soft-cap,) mask, block max ---------------------------------------------------------------
+    // ---- (soft-cap,) mask, block maxima ------------------------------------------------------------
     // Without a cap the max is taken on the raw scores (the scale is positive) and the scale is folded
     // into the exponent's FMA; with a cap s[] is replaced by the capped score in the log2 domain.
     if (SOFTCAP) softcap_scores(s, p.scale_log2, p.cap_log2, p.inv_cap_scale);   // cap * tanh(s * scale / cap), pre-multiplied by log2 e
-    if (need_mask) {
+    if (!PLAIN) {
+      const int k0 = (j + j0) * kBlockN + part * 64, q_pos = p.q_pos0 + qt * kBlockM + row;
+      int hi = p.S_kv - 1 - k0;                               // masked iff c > hi || c <= lo
+      if (p.causal) hi = min(hi, q_pos - k0);
+      const int lo = (p.window > 0) ? (q_pos - p.window - k0) : -1;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) s[c] = (part * 32 + c > hi || part * 32 + c <= lo) ? NEG_INF : s[c];
+      for (int c = 0; c < 64; ++c) s[c] = (c > hi || c <= lo) ? NEG_INF : s[c];
     }
-    float a0 = fmax3(s[0], s[1], s[2]), a1 = fmax3(s[3], s[4], s[5]);
+    float bmax[2];
+    {
+      float a0[2], a1[2];
 #pragma unroll
-    for (int c = 6; c < 30; c += 4) { a0 = fmax3(a0, s[c], s[c + 1]); a1 = fmax3(a1, s[c + 2], s[c + 3]); }
-    const float bmax = fmax3(a0, a1, fmaxf(s[30], s[31]));     // this block's max (raw / capped domain)
-    float mx = fmaxf(bmax, mx_others);
-    if (SOFTCAP) {
-      // the capped scores cost two MUFU ops each, so here the four threads of a row exchange block maxima
-      xchg[(pb * kParts + part) * 128 + row] = bmax;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&quadbar[quad]);
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&quadbar[quad], state.quad_par, abort_flag))) { fail = 104; return false; }
-      state.quad_par ^= 1;
+      for (int g = 0; g < 2; ++g) {
+        a0[g] = fmax3(s[g * 32 + 0], s[g * 32 + 1], s[g * 32 + 2]);
+        a1[g] = fmax3(s[g * 32 + 3], s[g * 32 + 4], s[g * 32 + 5]);
+      }
 #pragma unroll
-      for (int o = 1; o < kParts; ++o) mx = fmaxf(mx, xchg[(pb * kParts + ((part + o) & (kParts - 1))) * 128 + row]);
+      for (int c = 6; c < 30; c += 4) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          a0[g] = fmax3(a0[g], s[g * 32 + c], s[g * 32 + c + 1]);
+          a1[g] = fmax3(a1[g], s[g * 32 + c + 2], s[g * 32 + c + 3]);
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) bmax[g] = fmax3(a0[g], a1[g], fmaxf(s[g * 32 + 30], s[g * 32 + 31]));
     }
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 3);
-    const float sc_mul = SOFTCAP ? 1.0f : p.scale_log2;
-    const float m_new = fmaxf(m_run, mx * sc_mul);            // -inf * positive stays -inf
+    float tmax = fmaxf(bmax[0], bmax[1]) * sc_mul;            // -inf * positive stays -inf
+    xchg[((t & 3) * 2 + part) * 128] = tmax;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.row_bar[(t & 3) * 4 + quad]);
+    float m_prev = m_run;                                     // running maximum before this tile: the other group's last tile counts too
+    if (j > 0) {
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag))) { fail = 104; return false; }
+      m_prev = fmax3(m_prev, xchg[((t - 1) & 3) * 256], xchg[((t - 1) & 3) * 256 + 128]);
+    }
+    if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.row_bar[(t & 3) * 4 + quad], (t >> 2) & 1, abort_flag))) { fail = 106; return false; }
+    tmax = fmaxf(tmax, xchg[((t & 3) * 2 + (part ^ 1)) * 128]);
+    const float m_new = fmaxf(m_prev, tmax);
     // The exponent is formed as fma(s, scale, -m): for the row-max element that leaves the rounding
     // residue of s*scale (up to half an ulp of m) instead of exactly 0, and a p a hair below 1 would
     // drop the block scale by a binade.  Lowering the subtracted max by 2^-21 |m| keeps that p in
     // [1, 1 + 1e-5); the common factor cancels in O = sum(p v) / sum(p).
     const float m_use = (m_new == NEG_INF) ? 0.0f : (SOFTCAP ? m_new : fmaf(-fabsf(m_new), 4.76837158203125e-7f, m_new));
-    const float corr = (m_run == NEG_INF) ? 1.0f : ex2_approx(m_run - m_new);
+    const float corr = (m_prev == NEG_INF) ? 1.0f : ex2_approx(m_prev - m_new);       // of O
+    const float l_corr = (m_run == NEG_INF) ? 1.0f : ex2_approx(m_run - m_new);       // of this thread's share of the sum
     m_run = m_new;
+    if (t >= 2 && !__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp], ((t - 2) >> 1) & 1, abort_flag))) { fail = 107; return false; }   // P buffer free
 
-    // ---- p = 2^(x - m), row sum from the unquantised p, requant of this 32-key block ---------------
-    uint8_t* p_tile = smem + L::p_off + pb * kTileBytes + row * 128;
-    float ls0 = 0.0f, ls1 = 0.0f, ls2 = 0.0f, ls3 = 0.0f;
+    // ---- p = 2^(x - m), row sum from the unquantised p, requant per 32-key block ---------------------
+    // y = p * 2^(7-sc) has exponent field E - se + 7 = the E4M3 exponent field and keeps the mantissa, so the truncated code is y's
+    // bits [20,27); .ftz zeroes everything below 2^-6 of the block scale.  ex2.approx.ftz never returns a subnormal, so this holds whatever sc
+    // is (a block whose maximum lies below 2^-120 needs no other path: its non-zero elements all lie within 2^6 of that maximum).
+    uint8_t* p_tile = smem + L::p_off + grp * kTileBytes + row * 128;
+    uint64_t lsA = 0ull, lsB = 0ull;
+    uint32_t scale_pair = 0;
+    uint64_t fmul2[2];
 #pragma unroll
-    for (int c = 0; c < 32; c += 4) {
-      // two packed FMAs form the four exponents; the exponentials themselves go to the MUFU one by one
-      float x0, x1, x2, x3;
-      fma2(s[c + 0], s[c + 1], sc_mul, -m_use, x0, x1);
-      fma2(s[c + 2], s[c + 3], sc_mul, -m_use, x2, x3);
-      const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
-      s[c + 0] = p0; s[c + 1] = p1; s[c + 2] = p2; s[c + 3] = p3;
-      add2(ls0, ls1, p0, p1);
-      add2(ls2, ls3, p2, p3);
+    for (int g = 0; g < 2; ++g) {
+      // block max of p = 2^(block max of x - m): exp2 is monotone, so it is the p of the arg-max element; E8M0 code = its exponent field
+      // (se = floor(log2 pmax) <= 0; an all-zero block gives 0)
+      const float pmax = ex2_approx(fmaf(bmax[g], sc_mul, -m_use));
+      const int sc = min((int)(__float_as_uint(pmax) >> 23), 127);
+      scale_pair |= (uint32_t)sc << (8 * g);
+      const float f = __uint_as_float((uint32_t)(134 - sc) << 23);   // 2^(7-sc)
+      fmul2[g] = pack2(f, f);
     }
-    // block max of p = 2^(block max of x - m): exp2 is monotone, so it is the p of the arg-max element
-    const float pmax = ex2_approx(fmaf(bmax, sc_mul, -m_use));
-    // E8M0 code = exponent field of the block max (se = floor(log2 pmax) <= 0; an all-zero block gives 0)
-    int sc = (int)(__float_as_uint(pmax) >> 23);
-    sc = min(sc, 127);
-    uint32_t w[8];
-    {
-      // y = p * 2^(7-sc) has exponent field E - se + 7 = the E4M3 exponent field and keeps the mantissa,
-      // so the truncated code is y's bits [20,27); .ftz zeroes everything below 2^-6 of the block scale.
-      // ex2.approx.ftz never returns a subnormal, so this holds whatever sc is (a block whose maximum lies
-      // below 2^-120 needs no other path: its non-zero elements all lie within 2^6 of that maximum).
-      const float f = __uint_as_float((uint32_t)(134 - sc) << 23);
+    const uint64_t sc2 = pack2(sc_mul, sc_mul), nm2 = pack2(-m_use, -m_use);
+    auto exp4 = [&](int g, int c) {
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        float x0, x1;
+        unpack2(fma2p(pack2(s[g * 32 + c + e], s[g * 32 + c + e + 1]), sc2, nm2), x0, x1);
+        s[g * 32 + c + e] = ex2_approx(x0);
+        s[g * 32 + c + e + 1] = ex2_approx(x1);
+      }
+    };
+    auto requant4 = [&](int g, int c) -> uint32_t {
+      const uint64_t p01 = pack2(s[g * 32 + c + 0], s[g * 32 + c + 1]);
+      const uint64_t p23 = pack2(s[g * 32 + c + 2], s[g * 32 + c + 3]);
+      lsA = add2p(lsA, p01);
+      lsB = add2p(lsB, p23);
+      uint32_t y0, y1, y2, y3;
+      unpack2u(mul2p_ftz(p01, fmul2[g]), y0, y1);
+      unpack2u(mul2p_ftz(p23, fmul2[g]), y2, y3);
+      return pack_u8x2(y1 >> 20, y0 >> 20, pack_u8x2(y3 >> 20, y2 >> 20, 0u));
+    };
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) exp4(0, c);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      uint32_t w[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        float y0, y1, y2, y3;
-        mul2_ftz(s[q * 4 + 0], s[q * 4 + 1], f, y0, y1);
-        mul2_ftz(s[q * 4 + 2], s[q * 4 + 3], f, y2, y3);
-        w[q] = pack_u8x2(__float_as_uint(y1) >> 20, __float_as_uint(y0) >> 20,
-                         pack_u8x2(__float_as_uint(y3) >> 20, __float_as_uint(y2) >> 20, 0u));
+        if (g == 0) exp4(1, q * 4);
+        w[q] = requant4(g, q * 4);
       }
-    }
-    {
-      // two 16-byte chunks of this row, 128-byte swizzle: chunk index XOR (row % 8)
-      const int c0 = (2 * part) ^ (row & 7), c1 = (2 * part + 1) ^ (row & 7);
+      const int c0 = (4 * part + 2 * g) ^ (row & 7), c1 = (4 * part + 2 * g + 1) ^ (row & 7);     // 128-byte swizzle
       *reinterpret_cast<uint4*>(p_tile + c0 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4*>(p_tile + c1 * 16) = make_uint4(w[4], w[5], w[6], w[7]);
     }
-    l_run = l_run * corr + ((ls0 + ls1) + (ls2 + ls3));
-    smem[L::sfp_off + pb * kSfAtomBytes + (row & 31) * 16 + (row >> 5) * 4 + part] = (uint8_t)sc;
-
+    {
+      float ls0, ls1, ls2, ls3;
+      unpack2(lsA, ls0, ls1);
+      unpack2(lsB, ls2, ls3);
+      l_run = l_run * l_corr + ((ls0 + ls1) + (ls2 + ls3));
+    }
+    *reinterpret_cast<uint16_t*>(smem + L::sfp_off + grp * kSfAtomBytes + (row & 31) * 16 + (row >> 5) * 4 + part * 2) = (uint16_t)scale_pair;
     if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && j == 0) {
       // P codes as written (un-swizzled view) and the scale bytes, after the 128x128 S dump
       uint32_t* d32 = reinterpret_cast<uint32_t*>(p.dbg + 128 * 128);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int lc = part * 2 + c;
+      for (int lc = part * 4; lc < part * 4 + 4; ++lc) {
         const uint4 v4 = *reinterpret_cast<const uint4*>(p_tile + ((lc ^ (row & 7)) * 16));
         d32[row * 32 + lc * 4 + 0] = v4.x; d32[row * 32 + lc * 4 + 1] = v4.y;
         d32[row * 32 + lc * 4 + 2] = v4.z; d32[row * 32 + lc * 4 + 3] = v4.w;
       }
-      reinterpret_cast<uint8_t*>(d32 + 128 * 32)[row * 4 + part] = (uint8_t)sc;
+      reinterpret_cast<uint16_t*>(d32 + 128 * 32 + row)[part] = (uint16_t)scale_pair;
     }
 
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 4);
-    // ---- rescale this thread's share of O in TMEM once the previous PV has landed (it had the whole
-    //      exp/requant phase above to finish, so this wait is normally free) ----------------------------
+    // ---- rescale this thread's half of the row's O in TMEM once the other group's P V has landed ----------------------
     if (t > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag))) { fail = 102; return false; }
+      if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp ^ 1], ((t - 1) >> 1) & 1, abort_flag))) { fail = 102; return false; }
       tc_fence_after();
-      if (j == 0) {
-        write_out_rows(p, tmem_base, state);                  // O of the item before this one: its last P V ran under this tile's softmax
+      if (j == 0) {                                           // O of the item before this one: its last P V ran under this tile's softmax
+        if (!write_out_rows<DCH, KV_STAGES, DUMP>(p, smem, bars, tmem_base, abort_flag, state)) { fail = 105; return false; }
       } else if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll 1
-        for (int ch = 0; ch < kOCols / 32; ++ch) {
+        for (int ch = 0; ch < DCH * 2; ++ch) {
           uint32_t r[32];
-          const uint32_t addr = tmem_base + lane_addr + kColO + part * kOCols + ch * 32;
+          const uint32_t addr = tmem_base + lane_addr + kColO + part * (DCH * 64) + ch * 32;
           tmem_ld32(addr, r);
           tc_wait_ld();
 #pragma unroll
@@ -299,58 +326,30 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
         tc_wait_st();
       }
     }
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 5);
     fence_proxy_async_smem();   // make the st.shared P tile + scales visible to the tensor-core (async) proxy
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&p_full[pb]);
-    if (lane == 0 && sslot < 2) RK_STAMP(sslot, j, 6);
+    if (lane == 0) mbar_arrive(&bars.p_full[grp]);
     return true;
   };
 
-  // Tiles 0 .. n_plain-1 need no mask for any row of this query tile: no sliding window, all 128 keys inside S_kv,
-  // and the tile's last key not beyond the first row's position.  Both bounds grow with j, so the plain tiles come
-  // first; the general body decides again for every tile it gets.
-  int n_plain = 0;
-  if (p.window == 0) {
-    n_plain = min(n_tiles, p.S_kv / kBlockN - j0);
-    if (p.causal) {
-      const int t = p.q_pos0 + qt * kBlockM - (kBlockN - 1);            // plain iff (j + j0) * kBlockN <= t
-      n_plain = min(n_plain, t < 0 ? 0 : t / kBlockN + 1 - j0);
-    }
-    n_plain = max(n_plain, 0);
-  }
-  int j = 0;
-  for (; j < n_plain && ok; ++j) ok = tile(j, std::true_type{});
-  for (; j < n_tiles && ok; ++j) ok = tile(j, std::false_type{});
-
-  // ---- end of the item: the row's sum and log-sum-exp; O is written out under the next item's first tile ---------------
-  float l_tot = l_run;
-  if (ok) {
-    xchg[(2 * kParts + part) * 128 + row] = l_run;
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&quadbar[quad]);
-    ok = __all_sync(0xffffffffu, mbar_wait_short(&quadbar[quad], state.quad_par, abort_flag));
-    state.quad_par ^= 1;
-    if (!ok) fail = 105;
-#pragma unroll
-    for (int o = 1; o < kParts; ++o) l_tot += xchg[(2 * kParts + ((part + o) & (kParts - 1))) * 128 + row];
+  for (int j = grp ^ (state.t & 1); j < n_tiles && ok; j += 2) {
+    if (j >= n_low && j < n_high) ok = tile(j, std::true_type{});
+    else ok = tile(j, std::false_type{});
   }
   if (!ok) { give_up(abort_flag, p.status, fail); return false; }
+  reinterpret_cast<float2*>(smem + L::end_off)[((state.items & 1) * 4 + grp * 2 + part) * 128 + row] = make_float2(l_run, m_run);
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&bars.end_bar[quad]);
   state.t += n_tiles;
+  ++state.items;
   state.out_qt = qt; state.out_bh = bh;
-  state.out_inv_l = (l_tot > 0.0f) ? 1.0f / l_tot : 1.0f;
-  if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && part == 0) {
-    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 0] = m_run;
-    p.dbg[128 * 128 + 128 * 32 + 128 + row * 2 + 1] = l_tot;
-  }
-  state.out_lse = (l_tot > 0.0f) ? m_run * 0.6931471805599453f + logf(l_tot) : NEG_INF;
   return true;
 }
 
 // ---- the kernel ---------------------------------------------------------------------------------
 template <int DCH, int KV_STAGES, bool SOFTCAP, bool DUMP>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kThreads256, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p, const uint32_t idesc_qk,
                const uint32_t idesc_pv) {
@@ -366,16 +365,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   uint64_t* k_empty = k_full + KV_STAGES;
   uint64_t* v_full = k_empty + KV_STAGES;
   uint64_t* v_empty = v_full + KV_STAGES;
-  uint64_t* s_full = v_empty + KV_STAGES;
-  uint64_t* s_empty = s_full + 1;
-  uint64_t* p_full = s_empty + 1;
-  uint64_t* pv_done = p_full + 2;
+  uint64_t* s_full = v_empty + KV_STAGES;      // [2]: even and odd key tiles
+  uint64_t* s_empty = s_full + 2;
+  uint64_t* p_full = s_empty + 1;              // [2]
+  uint64_t* pv_done = p_full + 2;              // [2]
   uint64_t* drain = pv_done + 2;
-  uint64_t* drain2 = drain + 5;       // after the four pair barriers
+  uint64_t* drain2 = drain + 1;
   uint64_t* q_empty = drain2 + 1;
   uint64_t* clc_bar = q_empty + 1;
   uint64_t* work_full = clc_bar + 1;
   uint64_t* work_empty = work_full + 1;
+  uint64_t* row_bar = work_empty + 1;          // [4 tiles][4 quadrants]: row maxima written
+  uint64_t* end_bar = row_bar + 16;            // [4 quadrants]: row sums of an item written
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -417,8 +418,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
     for (int i = lane; i < L::n_bars; i += 32) {
       uint64_t* bar = bars + i;
-      const int count = bar == s_empty || bar == p_full || bar == p_full + 1 ? kNumSoftmaxWarps
-                        : bar > drain && bar < drain2                        ? kParts
+      const int count = bar == s_empty || bar == p_full || bar == p_full + 1 ? kNumSoftmaxWarps / 2
+                        : bar >= row_bar && bar < end_bar                    ? 2
+                        : bar >= end_bar && bar < end_bar + 4                ? 4
                         : bar == work_empty                                  ? kNumSoftmaxWarps + 2
                                                                              : 1;
       mbar_init(bar, count);
@@ -428,8 +430,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   }
   if (warp == kNumSoftmaxWarps + 1) { tmem_alloc(tmem_ptr, kTmemCols); tmem_relinquish(); }
   tc_fence_before();
-  if (warp == kNumSoftmaxWarps) asm volatile("bar.arrive 1, %0;" ::"n"(kNumThreads) : "memory");
-  else asm volatile("bar.sync 1, %0;" ::"n"(kNumThreads) : "memory");
+  if (warp == kNumSoftmaxWarps) asm volatile("bar.arrive 1, %0;" ::"n"(kThreads256) : "memory");
+  else asm volatile("bar.sync 1, %0;" ::"n"(kThreads256) : "memory");
   tc_fence_after();
   if (warp != kNumSoftmaxWarps) {                    // (the TMA producer waits where it starts its loads)
     grid_dependency_wait();
@@ -451,33 +453,37 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   constexpr int kFailWork = 501;
 
   if (warp < kNumSoftmaxWarps) {
-    SoftmaxState state = {0, 0, 0, 0, 0.0f, 0.0f};
+    reg_inc256<kRegSoftmax256>();
+    SoftmaxState state = {0, 0, 0, 0};
+    const SoftmaxBars sb = {s_full, s_empty, p_full, pv_done, row_bar, end_bar};
     int more;
     while ((more = next_work()) != 0) {
       if (more < 0) { give_up(abort_flag, p.status, kFailWork); break; }
       if (w.n_tiles > 0) {
-        if (!softmax_rows<DCH, KV_STAGES, SOFTCAP, DUMP>(p, smem, bars, tmem_base, abort_flag, w.qt, w.bh, w.n_tiles, w.j0, state)) { more = -1; break; }
+        if (!softmax_rows<DCH, KV_STAGES, SOFTCAP, DUMP>(p, smem, sb, tmem_base, abort_flag, w.qt, w.bh, w.n_tiles, w.j0, state)) { more = -1; break; }
       } else if (warp < 4) {
         // no visible key: O = 0 (the l <= 0 guard of finalize_O, kernels/flash_attention_mx_gemma/flash_mx_impl.hpp:554-560)
         const int q_row = w.qt * kBlockM + threadIdx.x;
         if (q_row < p.S_q && *reinterpret_cast<volatile int*>(p.status) == 0) {
           __nv_bfloat16* orow = p.o + ((size_t)w.bh * p.S_q + q_row) * p.d;
+#pragma unroll 1
           for (int c = 0; c < p.d; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0, 0, 0, 0);
           if (p.lse) p.lse[(size_t)w.bh * p.S_q + q_row] = __int_as_float(0xff800000);
         }
       }
     }
-    if (more == 0 && state.t > 0) {                  // O of the last item
+    if (more == 0 && state.t > 0 && (state.t & 1) == (warp >> 3)) {      // O of the last item
       const int last = state.t - 1;
-      if (__all_sync(0xffffffffu, mbar_wait_short(&pv_done[last & 1], (last >> 1) & 1, abort_flag))) {
+      bool ok = __all_sync(0xffffffffu, mbar_wait_short(&pv_done[last & 1], (last >> 1) & 1, abort_flag));
+      if (ok) {
         tc_fence_after();
-        write_out_rows(p, tmem_base, state);
-      } else {
-        give_up(abort_flag, p.status, 103);
+        ok = write_out_rows<DCH, KV_STAGES, DUMP>(p, smem, sb, tmem_base, abort_flag, state);
       }
+      if (!ok) give_up(abort_flag, p.status, 103);
     }
   } else if (warp == kNumSoftmaxWarps) {
     // ================= TMA producer; hands out the items =================
+    reg_dec256<kRegIssue256>();
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
       int stopped = 0, st = 0, q_used = 0;
@@ -545,7 +551,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       if (fail) give_up(abort_flag, p.status, fail);
     }
     __syncwarp();
+  } else if (warp == kNumSoftmaxWarps + 3) {
+    reg_dec256<kRegIssue256>();
   } else if (warp == kNumSoftmaxWarps + 1) {
+    reg_dec256<kRegIssue256>();
     // ================= issuer of S = Q K^T =================
     // The whole warp runs the loop and one elected lane issues: what an MMA takes (descriptors, addresses) then is in uniform registers.
     // Inside one lane's branch each operand was moved there for every MMA (d <= 128: 660 cycles to issue four).
@@ -584,7 +593,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
               mma_mxf8f6f4_ss(tm + kColS, dqt + kk * 2, dkt + kk * 2, idesc_with_sf(idesc_qk, kk, kk), tm + kColSfQ + ch * 4, tm + kColSfK + st * 8 + ch * 4,
                               (ch > 0 || kk > 0) ? 1u : 0u);
           }
-          tc_commit(s_full);
+          tc_commit(&s_full[t & 1]);
           tc_commit(&k_empty[st]);
           if (j == nt - 1) tc_commit(q_empty);
         }
@@ -597,6 +606,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     if (fail) give_up(abort_flag, p.status, fail);
     __syncwarp();
   } else {
+    reg_dec256<kRegIssue256>();
     // ================= issuer of O += P V =================
     const uint32_t tm = warp_uniform(tmem_base);
     const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), 16, 1024, kLayoutSw128);
@@ -719,7 +729,7 @@ static int launch_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return (int)e;
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
-  e = launch_pdl(kern, grid, dim3(kNumThreads), smem_bytes, st, tq, tk, tv, p, idesc_qk, idesc_pv);
+  e = launch_pdl(kern, grid, dim3(kThreads256), smem_bytes, st, tq, tk, tv, p, idesc_qk, idesc_pv);
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_after, st);
   return (int)e;
 }
