@@ -110,6 +110,7 @@ __device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* 
   }
   if (p.lse && live && part == 0) p.lse[(size_t)st.out_bh * p.S_q + q_row] = (l > 0.0f) ? m * 0.6931471805599453f + logf(l) : NEG_INF;
   const int ncols = p.d / 2;
+  const bool aligned32 = (reinterpret_cast<uintptr_t>(p.o) & 31) == 0;
   __nv_bfloat16* orow = p.o + ((size_t)st.out_bh * p.S_q + q_row) * p.d + part * ncols;
 #pragma unroll 1
   for (int c = 0; c < ncols; c += 32) {
@@ -118,14 +119,14 @@ __device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* 
     tc_wait_ld();
     if (live) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t w[4];
+      for (int i = 0; i < 2; ++i) {
+        uint32_t w[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[8 * i + 2 * e]) * inv_l, __uint_as_float(r[8 * i + 2 * e + 1]) * inv_l);
+        for (int e = 0; e < 8; ++e) {
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[16 * i + 2 * e]) * inv_l, __uint_as_float(r[16 * i + 2 * e + 1]) * inv_l);
           w[e] = *reinterpret_cast<const uint32_t*>(&b2);
         }
-        *reinterpret_cast<uint4*>(orow + c + 8 * i) = make_uint4(w[0], w[1], w[2], w[3]);
+        store_row32(orow + c + 16 * i, w, aligned32);
       }
     }
   }

@@ -417,6 +417,7 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
     tc_fence_after();
     if (quad == 0 && lane == 0) RK_STAMP(grp, 0, 6);
     __nv_bfloat16* orow = p.o + ((size_t)bh * p.S_q + q_row) * p.d;
+    const bool aligned32 = (reinterpret_cast<uintptr_t>(p.o) & 31) == 0;
     // the row's registers are free now: this group's half of the columns is fetched with one wait
     const int c32_0 = half * (p.d / 64), n_c32 = c32_0 + p.d / 64;
 #pragma unroll 1
@@ -429,15 +430,17 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           if (h + c < n_c32) {
-            uint32_t packed[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(r[c * 32 + 2 * i]) * inv_l, __uint_as_float(r[c * 32 + 2 * i + 1]) * inv_l);
-              packed[i] = *reinterpret_cast<const uint32_t*>(&b2);
+            for (int i = 0; i < 2; ++i) {
+              uint32_t w[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const float* f = reinterpret_cast<const float*>(r) + c * 32 + i * 16 + 2 * e;
+                const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[0] * inv_l, f[1] * inv_l);
+                w[e] = *reinterpret_cast<const uint32_t*>(&b2);
+              }
+              store_row32(orow + (h + c) * 32 + i * 16, w, aligned32);
             }
-            uint4* dst = reinterpret_cast<uint4*>(orow + (h + c) * 32);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
           }
         }
       }
