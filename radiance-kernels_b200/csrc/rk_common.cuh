@@ -102,7 +102,8 @@ RK_DEVINL float e8m0_to_f32(uint32_t c) { return __uint_as_float(c == 0 ? 0x0040
 RK_DEVINL uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // The first 1024-byte boundary of a dynamic shared array.  By an offset: after a cast through an integer the compiler no longer knows
 // that the pointer is into shared memory, stores become generic ones and every address it keeps takes two registers (d = 256
-// prefill, capped, 16 heads of 8192: 1065 us with the cast, 1017 without; 509 queries behind 3581 keys 47.2 -> 46.4).
+// prefill, capped, 16 heads of 8192: 1065 us with the cast, 1017 without; 509 queries behind 3581 keys 47.2 -> 46.4).  The decode
+// kernels keep the cast: the mma.sync kernel is 6-10 % faster with it (other registers, other order), the tcgen05 kernel within 2 % either way.
 RK_DEVINL uint8_t* align_smem(uint8_t* p) { return p + ((0u - smem_u32(p)) & 1023u); }
 
 RK_DEVINL void mbar_init(uint64_t* bar, uint32_t count) {

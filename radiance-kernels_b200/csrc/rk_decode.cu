@@ -127,7 +127,7 @@ template <int FMT>
 __global__ void __launch_bounds__(kDecThreads, 2)
 decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const DecodeParams p) {
   extern __shared__ __align__(1024) uint8_t dsmem_raw[];
-  uint8_t* smem = align_smem(dsmem_raw);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kDecStages * kDecStageBytes);
   uint64_t* empty = full + kDecStages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kDecStages);

@@ -608,7 +608,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_consta
   using L = Lay<HH>;
   constexpr int kStages = L::kStages;
   extern __shared__ __align__(1024) uint8_t dtc_smem_raw[];
-  uint8_t* smem = align_smem(dtc_smem_raw);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dtc_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::bar_off);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::misc_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::misc_off + 4);

@@ -491,7 +491,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       uint32_t use = 0, q_par = 0, block = blockIdx.x;
       for (uint32_t k = 0;; ++k) {
         w = decode(block);
-        // everybody has read the last item: this one takes its place, and the one after it is asked for
+        // everybody has read the last item: this one takes its place
         if (k > 0 && !mbar_wait_short<true>(work_empty, (k - 1) & 1, abort_flag)) { fail = 502; break; }
         *reinterpret_cast<Item*>(smem + L::work_off) = w;
         mbar_arrive(work_full);
@@ -499,8 +499,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           grid_dependency_wait();
           stopped = *reinterpret_cast<volatile int*>(p.status);       // an earlier launch gave up on a wait
         }
-        mbar_arrive_expect_tx(clc_bar, 16);
-        clc_request(smem + L::clc_off, clc_bar);
         for (int j = 0; j < w.n_tiles; ++j) {
           if (j == 0) {
             if (q_used) {                            // Q K^T of the last item has finished
@@ -538,8 +536,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           *abort_flag = kStopped;
           if (w.n_tiles > 0) { mbar_wait_short<true>(q_full, 0, nullptr); mbar_wait_short<true>(&k_full[0], 0, nullptr); }
         }
-        if (!mbar_wait_short<true>(clc_bar, k & 1, nullptr) && !fail) fail = 503;      // (also where the CTA gives up)
         if (fail || stopped) break;
+        // The next item is asked for now that this one's last loads are under way, and not earlier: the items that are left go to
+        // the SMs that are free first.
+        mbar_arrive_expect_tx(clc_bar, 16);
+        clc_request(smem + L::clc_off, clc_bar);
+        if (!mbar_wait_short<true>(clc_bar, k & 1, nullptr)) { fail = 503; break; }      // (also where the CTA gives up)
         if (!clc_answer(smem + L::clc_off, block)) {
           if (!mbar_wait_short<true>(work_empty, k & 1, abort_flag)) { fail = 502; break; }
           w.qt = -1;

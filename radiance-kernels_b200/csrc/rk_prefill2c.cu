@@ -675,22 +675,16 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         for (uint32_t k = 0;; ++k) {
           w = decode(block);
           const int n_all = max(w.nt0, w.nt1);
-          bool asked = false;
           for (int j = 0; j < n_all || j == 0; ++j) {
             perturb<DUMP>(p, kPerturbTma, j);
             if (j == 0) {
-              // everybody has read the last item: this one takes its place, and the one after it is asked for
+              // everybody has read the last item: this one takes its place
               if (k > 0 && !mbar_wait_short<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
               *reinterpret_cast<Work*>(smem + work_off) = w;
               mbar_arrive(&bars[bWF]);
               if (k == 0) {
                 grid_dependency_wait();
                 stopped = *reinterpret_cast<volatile int*>(p.status);       // an earlier launch gave up on a wait
-              }
-              if (!SPLIT) {
-                mbar_arrive_expect_tx(&bars[bClc], 16);
-                clc_request(smem + clc_off, &bars[bClc]);
-                asked = true;
               }
 #pragma unroll 1
               for (int g = 0; g < 2; ++g) {
@@ -719,8 +713,13 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (w.nt1 > 0) drain(&bars[bQB], 0, 301);
             if (n_all > 0) drain(&bars[bKF], 0, 302);
           }
-          if (asked) drain(&bars[bClc], k & 1, 503);
-          if (fail || stopped || !asked) break;
+          if (fail || stopped || SPLIT) break;
+          // The next item is asked for now that this one's last loads are under way, three tiles before its end, and not earlier: the items
+          // that are left go to the SMs that are free first.
+          mbar_arrive_expect_tx(&bars[bClc], 16);
+          clc_request(smem + clc_off, &bars[bClc]);
+          drain(&bars[bClc], k & 1, 503);
+          if (fail) break;
           if (!clc_answer(smem + clc_off, block)) {
             if (!mbar_wait_short<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
             w.qp = -1;
