@@ -345,3 +345,41 @@ def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm
     runner = rk.PrefillHostRunner(*[t.cpu().pin_memory() for t in (qc, kc, vc, qs, ks, vs)], want_lse=True, **kw)
     assert torch.equal(runner.run(), o.cpu()) and torch.equal(runner.lse, lse.cpu())
     assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Skv,d,kw", [
+    (5, 64, 32, 300, 300, 128, dict(causal=True)),                   # 640 pairs, every second without its second tile; two tiles at most
+    (3, 64, 32, 129, 389, 128, dict(causal=False)),                  # one key in the last tile, equal numbers of key tiles
+    (4, 48, 48, 520, 520, 64, dict(causal=True, window=129)),        # items that start inside the sequence
+    (2, 96, 96, 200, 200, 128, dict(causal=True, q_pos0=-130)),      # a tile without a visible key before one that has some
+    (2, 100, 50, 260, 390, 128, dict(causal=True, q_pos0=130, softcap=5.0)),
+    (3, 60, 20, 260, 260, 256, dict(causal=True)),                   # 540 items of one, two and three key tiles
+    (2, 80, 80, 140, 400, 256, dict(causal=False, softcap=50.0)),
+    (2, 90, 45, 200, 200, 256, dict(causal=True, q_pos0=-130, softcap=50.0)),
+    (1, 80, 80, 390, 390, 256, dict(causal=True, window=128)),
+])
+def test_many_items_per_sm(B, H, Hkv, Sq, Skv, d, kw):
+    """A CTA takes one item after the other: odd and even numbers of key tiles, items without one, the last O written out at the end."""
+    r = prefill_vs_oracle(B, H, Hkv, Sq, Skv, d, seed=31, want_lse=True, **kw)
+    # Millions of rows, some of few keys: beyond the general bound the bf16 rounding of |O| up to 5 (2^-8 |O|), and, where exp2 of the two sides
+    # falls on either side of a code boundary, one E4M3 step of a P, 2^-3 of its weight: 2^-3 * 0.1 * 4.5 for the largest |v|.
+    assert r["err"][1] <= REL_L2 and (np.abs(r["got"] - r["ref"]["o_f32"]) <= 0.056 + 2.0 ** -8 * np.abs(r["ref"]["o_f32"])).all(), r["err"]
+    seen = np.isfinite(r["ref"]["lse"])
+    assert (np.isfinite(r["lse"]) == seen).all() and np.abs(r["lse"][seen] - r["ref"]["lse"][seen]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("d,window", [(128, 1), (128, 127), (128, 128), (128, 129), (64, 256), (64, 257), (256, 127), (256, 129)])
+def test_window_edges_against_tile_edges(d, window):
+    _check(prefill_vs_oracle(2, 4, 2, 515, 600, d, causal=True, q_pos0=85, window=window, seed=32))
+
+
+@pytest.mark.parametrize("H,Sq,d", [(2, 150, 64), (2, 150, 128), (160, 150, 128), (2, 150, 256)])
+def test_o_at_a_16_byte_boundary(H, Sq, d):
+    """O need not be 32-byte aligned: rows then leave in 16-byte stores.  The same bits, nothing beside them."""
+    q, qs, k, ks, v, vs = quantize_inputs(*randn_qkv(1, H, H, Sq, Sq, d, 33))
+    want = rk.attn_prefill(q, k, v, qs, ks, vs, causal=True)
+    flat = torch.full((want.numel() + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = flat[8:8 + want.numel()].view(want.shape)
+    assert out.data_ptr() % 32 == 16
+    rk.attn_prefill(q, k, v, qs, ks, vs, causal=True, out=out)
+    assert torch.equal(out, want) and (flat[:8] == 7.0).all() and (flat[-8:] == 7.0).all()
