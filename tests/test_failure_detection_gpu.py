@@ -49,6 +49,28 @@ def test_bounded_wait_runs_out_and_is_reported_and_clears():
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("H,S,d,q_pos0", [(2, 300, 256, 0), (160, 200, 256, -130), (160, 100, 128, 0), (160, 200, 64, -130)])
+def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0):
+    """Every form of the prefill kernels, items of one key tile and query tiles without a visible key among them: neither O nor the
+    log-sum-exps are touched."""
+    L = rk.lib()
+    qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, S, S, d, seed=92))
+    o = torch.full((1, H, S, d), 7.0, dtype=torch.bfloat16, device="cuda")
+    lse = torch.full((1, H, S), 7.0, device="cuda")
+    assert rk.last_device_status() == 0
+    assert L.rk_debug_wait_runs_out(1000, 0, _stream()) == 0
+    torch.cuda.synchronize()
+    try:
+        rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
+        torch.cuda.synchronize()
+    finally:
+        status = rk.last_device_status()
+    assert status == WAIT_GAVE_UP and (o == 7.0).all() and (lse == 7.0).all()
+    rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0 and not (o == 7.0).all() and not (lse == 7.0).any()
+
+
 def test_noalloc_decode_status_word_is_observable():
     L = rk.lib()
     g = torch.Generator(device="cuda").manual_seed(91)
