@@ -25,13 +25,13 @@
 // item, so nothing drains in between: the next item's loads start while the last tiles of this one are worked on, group A goes
 // on while group B, one tile longer under a causal mask, finishes, and the correction warps write an item's O out while the softmax
 // warps are in their next tile.  With a CTA per pair an item of 16 tiles cost 17 000 cycles on top of them (start 4400, first loads,
-// a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 527 us, 4 x 32 / 8 heads of
-// 8192 2030 -> 1800 us.
+// a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
+// 8192 2030 -> 1764 us.
 //
 // SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle (chunks of a prompt, short prompts).  A key tile's time is
 // then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
 // on the same tile, group A on keys 0-63 of each key tile and group B on keys 64-127, and exchange their row maxima through
-// shared memory.  32 heads x 509 queries behind 3581 keys: the call 76 us with tile pairs on 64 SMs, 47 us now.
+// shared memory.  32 heads x 509 queries behind 3581 keys: the call 76 us with tile pairs on 64 SMs, 43.5 us now.
 #include <type_traits>
 
 #include "rk_prefill.cuh"
@@ -43,7 +43,7 @@ constexpr int kStages = 3;
 constexpr int kThreads = 512;
 constexpr int kWarpCorr = 8, kWarpTma = 12, kWarpQk = 13, kWarpPv = 14;
 // Registers of a softmax, correction and issuer thread: 128 * (2 * softmax + correction + issuer) = 65536.  Measured (8 x 16 heads of
-// 4096): softmax 176 545 us, 184 527, 192 527, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
+// 4096): softmax 168 515 us, 176 518, 184 521, 192 523, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
 constexpr uint32_t kRegSoftmax = 176, kRegCorr = 88, kRegIssue = 72;
 constexpr uint32_t kRegSoftmaxSplit = 160, kRegCorrSplit = 96, kRegIssueSplit = 96;
 // TMEM columns
