@@ -201,27 +201,6 @@ RK_DEVINL void report_wait_failure(volatile int* abort_flag, int* status, int co
   atomicCAS(status, 0, code);
 }
 
-// Bounded wait for warps that are not on the critical path (producers, issuers, correction): between polls the
-// warp sleeps `SLEEP_NS`, so that it leaves the issue slots of its scheduler to the warps that compute.  Same
-// give-up rule as mbar_wait.
-template <uint32_t SLEEP_NS>
-RK_DEVINL bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
-                                 uint64_t limit_ns = 2000000000ull) {
-  if (mbar_try_wait<0>(bar, parity)) return true;
-  const uint64_t t0 = global_timer_ns();
-  for (uint32_t it = 1;; ++it) {
-    __nanosleep(SLEEP_NS);
-    if (mbar_try_wait<0>(bar, parity)) return true;
-    if ((it & 63u) == 0u) {
-      if (*abort_flag || *reinterpret_cast<volatile int*>(status) != 0) { *abort_flag = 1; return false; }
-      if (global_timer_ns() - t0 > limit_ns) break;
-    }
-  }
-  *abort_flag = 1;
-  atomicCAS(status, 0, code);
-  return false;
-}
-
 // Programmatic dependent launch: a kernel launched with the attribute starts while the one before it in the stream still
 // runs; it waits here before it touches anything that one may write (or read, where it writes), and lets the one after
 // it start.  Both do nothing in an ordinary launch.
