@@ -45,7 +45,7 @@ constexpr int kWarpCorr = 8, kWarpTma = 12, kWarpQk = 13, kWarpPv = 14;
 // Registers of a softmax, correction and issuer thread: 128 * (2 * softmax + correction + issuer) = 65536.  Measured (8 x 16 heads of
 // 4096): softmax 168 515 us, 176 518, 184 521, 192 523, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
 constexpr uint32_t kRegSoftmax = 176, kRegCorr = 88, kRegIssue = 72;
-constexpr uint32_t kRegSoftmaxSplit = 160, kRegCorrSplit = 96, kRegIssueSplit = 96;
+constexpr uint32_t kRegSoftmaxSplit = 176, kRegCorrSplit = 80, kRegIssueSplit = 80;      // 509 queries behind 3581 keys: softmax 144 43.9 us, 160 44.4, 176 43.5, 192 43.6
 // TMEM columns
 constexpr uint32_t cS = 0, cO = 128 /* + g*128 */, cSfQ = 384 /* + g*4 */, cSfK = 392 /* + st*4 */,
                    cSfP = 404 /* + (g*2+pb)*4 */, cSfV = 420 /* + st*4 */;
