@@ -58,7 +58,7 @@ struct SmemLayout {
   static constexpr int clc_off = misc_off + 16;
   static constexpr int work_off = clc_off + 16;
   static constexpr int xchg_off = work_off + 32;              // [4 key tiles][2 parts][128 rows] floats: row maxima of a tile
-  static constexpr int end_off = xchg_off + 4 * 2 * 128 * 4;  // [2 items][2 groups][2 parts][128 rows] float2: row sum and its maximum
+  static constexpr int end_off = xchg_off + 4 * 2 * 128 * 4;  // [2 items][even, odd key tiles of the item][2 parts][128 rows] float2: row sum and its maximum
   static constexpr int total = end_off + 2 * 2 * 2 * 128 * 8;
 };
 
@@ -87,7 +87,9 @@ struct SoftmaxState {
 struct SoftmaxBars { uint64_t *s_full, *s_empty, *p_full, *pv_done, *row_bar, *end_bar; };
 
 // O / l -> bf16 (finalize_O, kernels/flash_attention_mx_gqa/flash_mx_impl.hpp:535-553) by one of the two groups: a thread has half of the
-// columns of its row.  The row's sum is in four shares, one per group and part, each relative to the running maximum its threads saw last.
+// columns of its row.  The row's sum is in four shares, one per part of the item's even and of its odd key tiles, each relative to the running
+// maximum its threads saw last.  They are added in that order, not in that of the groups: which group has the even tiles depends on the items
+// the CTA had before, and a row must not.
 template <int DCH, int KV_STAGES, bool DUMP>
 __device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* smem, const SoftmaxBars& bars, uint32_t tmem_base,
                                                volatile int* abort_flag, const SoftmaxState& st) {
@@ -339,7 +341,8 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     else ok = tile(j, std::false_type{});
   }
   if (!ok) { give_up(abort_flag, p.status, fail); return false; }
-  reinterpret_cast<float2*>(smem + L::end_off)[((state.items & 1) * 4 + grp * 2 + part) * 128 + row] = make_float2(l_run, m_run);
+  const int odd = grp ^ (state.t & 1);                         // this group had the item's tiles 0, 2, .. or 1, 3, ..
+  reinterpret_cast<float2*>(smem + L::end_off)[((state.items & 1) * 4 + odd * 2 + part) * 128 + row] = make_float2(l_run, m_run);
   __syncwarp();
   if (lane == 0) mbar_arrive(&bars.end_bar[quad]);
   state.t += n_tiles;

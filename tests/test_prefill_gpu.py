@@ -186,14 +186,15 @@ def test_lse_output():
     assert np.abs(r["lse"] - r["ref"]["lse"]).max() < 1e-3
 
 
-def test_bit_identical_across_runs():
+@pytest.mark.parametrize("B,H,Hkv,S,d,causal", [(2, 4, 2, 1024, 128, True), (2, 20, 10, 640, 256, False)])      # (40 x 5 query tiles of five key tiles)
+def test_bit_identical_across_runs(B, H, Hkv, S, d, causal):
     """Race check borrowed from the reference ("bit-identical O across 13 runs",
     kernels/flash_attention_mx/kernel.cpp:158-160)."""
-    Q, K, V = randn_qkv(2, 4, 2, 1024, 1024, 128, seed=13)
+    Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=13)
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
-    first = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True)
+    first = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
     for _ in range(5):
-        again = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True)
+        again = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
         assert torch.equal(first, again)
     assert rk.last_device_status() == 0
 
@@ -326,10 +327,12 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
 @pytest.mark.parametrize("B,H,Hkv,S,d,kw", [
     (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles, chunks of at most 128
     (2, 12, 4, 1090, 64, dict(causal=True, window=300)),          # 216, odd numbers of tiles per head
-    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0))])      # 160
+    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0)),       # 160
+    (2, 20, 10, 640, 256, dict(causal=False))])                   # 200 of five key tiles: a CTA's second item starts on an odd one
 def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, S, d, kw):
     """A call whose query tiles outnumber the SMs, against the same call cut by the host entry point and unit by unit, where each
-    piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in both forms)."""
+    piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in both forms, and at d = 256
+    whatever the CTA worked on before)."""
     Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=62)
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
     lse = torch.empty(B, H, S, dtype=torch.float32, device="cuda")
