@@ -341,10 +341,20 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     else ok = tile(j, std::false_type{});
   }
   if (!ok) { give_up(abort_flag, p.status, fail); return false; }
+  // The shares go over by threads that had a tile of the item, and by them alone: such a thread's last tile has waited for all that the shares' readers of
+  // the item before did (a P V of this item needs their O written out), so neither the shares of two items nor two phases of a barrier
+  // can meet.  One that had none, for an item of one key tile, would run ahead of its own partner; the group with the tile hands over empty shares for it.
   const int odd = grp ^ (state.t & 1);                         // this group had the item's tiles 0, 2, .. or 1, 3, ..
-  reinterpret_cast<float2*>(smem + L::end_off)[((state.items & 1) * 4 + odd * 2 + part) * 128 + row] = make_float2(l_run, m_run);
-  __syncwarp();
-  if (lane == 0) mbar_arrive(&bars.end_bar[quad]);
+  if (odd < n_tiles) {
+    float2* share = reinterpret_cast<float2*>(smem + L::end_off) + ((state.items & 1) * 4 + part) * 128 + row;
+    share[odd * 256] = make_float2(l_run, m_run);
+    if (n_tiles == 1) share[256] = make_float2(0.0f, NEG_INF);
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(&bars.end_bar[quad]);
+      if (n_tiles == 1) mbar_arrive(&bars.end_bar[quad]);
+    }
+  }
   state.t += n_tiles;
   ++state.items;
   state.out_qt = qt; state.out_bh = bh;

@@ -328,7 +328,10 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
     (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles, chunks of at most 128
     (2, 12, 4, 1090, 64, dict(causal=True, window=300)),          # 216, odd numbers of tiles per head
     (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0)),       # 160
-    (2, 20, 10, 640, 256, dict(causal=False))])                   # 200 of five key tiles: a CTA's second item starts on an odd one
+    (2, 20, 10, 640, 256, dict(causal=False)),                    # 200 of five key tiles: a CTA's second item starts on an odd one
+    (2, 20, 10, 640, 256, dict(causal=True, softcap=50.0)),       # items of one key tile at the end of the work order, one after the other
+    (6, 100, 50, 100, 256, dict(causal=True)),                    # 600 items of one key tile
+    (2, 100, 100, 128, 256, dict(causal=False, softcap=50.0))])
 def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, S, d, kw):
     """A call whose query tiles outnumber the SMs, against the same call cut by the host entry point and unit by unit, where each
     piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in both forms, and at d = 256
