@@ -466,6 +466,7 @@ __device__ __forceinline__ void write_out_quadrant(const PrefillParams& p, const
   const float inv_l = reinterpret_cast<const float*>(smem + corr_off)[at];
   const int row0 = it.qt * kBlockM + quad * 32;
   if (p.lse && row0 + lane < p.S_q) p.lse[(size_t)it.bh * p.S_q + row0 + lane] = reinterpret_cast<const float*>(smem + lse_off)[at];
+  if (row0 >= p.S_q) return;      // no row of this quadrant exists: every chunk below commits a copy, which is what the wait for a half of the stage counts on
   uint8_t* stage = smem + stage_off + quad * 4096;
   tc_fence_after();
 #pragma unroll 1
@@ -488,7 +489,7 @@ __device__ __forceinline__ void write_out_quadrant(const PrefillParams& p, const
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && row0 < p.S_q) { tma_store_3d(tmap_o, dst, ch * 32, row0, it.bh); bulk_commit(); }
+    if (lane == 0) { tma_store_3d(tmap_o, dst, ch * 32, row0, it.bh); bulk_commit(); }
   }
   tc_fence_before();
 }

@@ -186,7 +186,10 @@ def test_lse_output():
     assert np.abs(r["lse"] - r["ref"]["lse"]).max() < 1e-3
 
 
-@pytest.mark.parametrize("B,H,Hkv,S,d,causal", [(2, 4, 2, 1024, 128, True), (2, 20, 10, 640, 256, False)])      # (40 x 5 query tiles of five key tiles)
+@pytest.mark.parametrize("B,H,Hkv,S,d,causal", [
+    (2, 4, 2, 1024, 128, True),
+    (8, 64, 64, 200, 64, False), (8, 64, 64, 160, 128, False),      # the second query tile of every pair ends inside its TMEM lane quadrants
+    (2, 20, 10, 640, 256, False)])                                  # 200 query tiles of five key tiles
 def test_bit_identical_across_runs(B, H, Hkv, S, d, causal):
     """Race check borrowed from the reference ("bit-identical O across 13 runs",
     kernels/flash_attention_mx/kernel.cpp:158-160)."""
@@ -328,6 +331,9 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
     (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles, chunks of at most 128
     (2, 12, 4, 1090, 64, dict(causal=True, window=300)),          # 216, odd numbers of tiles per head
     (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0)),       # 160
+    (2, 100, 50, 200, 64, dict(causal=False)),                    # lane quadrants of the second query tile that have no row, after ones of the first that have
+    (2, 90, 90, 140, 128, dict(causal=False)),
+    (1, 20, 10, 1200, 128, dict(causal=True)),
     (2, 20, 10, 640, 256, dict(causal=False)),                    # 200 of five key tiles: a CTA's second item starts on an odd one
     (2, 20, 10, 640, 256, dict(causal=True, softcap=50.0)),       # items of one key tile at the end of the work order, one after the other
     (6, 100, 50, 100, 256, dict(causal=True)),                    # 600 items of one key tile
