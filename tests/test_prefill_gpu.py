@@ -359,6 +359,24 @@ def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("key,factor", [(5, 20.0), (5, 30.0), (70, 20.0), (70, 30.0)])
+def test_smaller_calls_give_the_same_bits_around_the_soft_caps_series_limit(key, factor):
+    """One key of every key tile has logits on both sides of cap / 8, the others far below: the exponential form of the cap for that key's
+    half of the tile and the series for the other, in pairs of query tiles (160) and with a CTA per tile."""
+    Q, K, V = randn_qkv(1, 40, 10, 500, 500, 128, seed=63, mul=0.3)
+    K[:, :, key::128] *= factor                                   # logits of standard deviation 1.8 and 2.7, 128 rows x 4 tiles of them a head
+    qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
+    kw = dict(causal=False, softcap=50.0)
+    lse = torch.empty(1, 40, 500, dtype=torch.float32, device="cuda")
+    o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw)
+    for h in range(10):
+        part = [t[:, h * 4:(h + 1) * 4].contiguous() for t in (qc, qs)] + [t[:, h:h + 1].contiguous() for t in (kc, ks, vc, vs)]
+        l1 = torch.empty(1, 4, 500, dtype=torch.float32, device="cuda")
+        o1 = rk.attn_prefill(part[0], part[2], part[4], part[1], part[3], part[5], lse=l1, **kw)
+        assert torch.equal(o1[0], o[0, h * 4:(h + 1) * 4]) and torch.equal(l1[0], lse[0, h * 4:(h + 1) * 4]), h
+    assert rk.last_device_status() == 0
+
+
 @pytest.mark.parametrize("B,H,Hkv,Sq,Skv,d,kw", [
     (5, 64, 32, 300, 300, 128, dict(causal=True)),                   # 640 pairs, every second without its second tile; two tiles at most
     (3, 64, 32, 129, 389, 128, dict(causal=False)),                  # one key in the last tile, equal numbers of key tiles
