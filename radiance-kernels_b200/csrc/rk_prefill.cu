@@ -102,7 +102,7 @@ __device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* 
   const float m = fmaxf(fmaxf(share[0].y, share[128].y), fmaxf(share[256].y, share[384].y));
   float l = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) l += share[i * 128].y == NEG_INF ? 0.0f : share[i * 128].x * ex2_approx(share[i * 128].y - m);
+  for (int i = 0; i < 4; ++i) l += share[i * 128].y == NEG_INF ? share[i * 128].x : share[i * 128].x * ex2_approx(share[i * 128].y - m);      // (0, or NaN where every score was)
   const float inv_l = (l > 0.0f) ? 1.0f / l : 1.0f;
   const int q_row = st.out_qt * kBlockM + row;
   const bool live = q_row < p.S_q;
