@@ -80,9 +80,10 @@ RK_DEVINL uint64_t mul2p_ftz(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f
 // The exponential is the one special-function instruction; the reciprocal is three Newton steps on the FMA pipe from
 // an integer first guess (error 0.12 -> 1.4e-2 -> 2e-4 -> 4e-8), because the special-function unit is what bounds
 // the capped kernels (it also has the softmax exponential to do).  k2 = 2 log2(e) scale / cap; the exponent is
-// clamped so that 1 + e stays finite.
+// clamped so that 1 + e stays finite (by a minimum that lets NaN through, as the series does).
+RK_DEVINL float fmin_nan(float a, float b) { float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
 RK_DEVINL void softcap_pair(float& s0, float& s1, float k2, uint64_t one2, uint64_t m2cap2, uint64_t cap2) {
-  const float e0 = ex2_approx(fminf(s0 * k2, 126.0f)), e1 = ex2_approx(fminf(s1 * k2, 126.0f));
+  const float e0 = ex2_approx(fmin_nan(s0 * k2, 126.0f)), e1 = ex2_approx(fmin_nan(s1 * k2, 126.0f));
   const uint64_t z = add2p(pack2(e0, e1), one2);                       // 1 + e in [1, 2^126]
   uint32_t z0, z1;
   unpack2u(z, z0, z1);

@@ -183,13 +183,14 @@ def test_dense_sub_byte_operands_give_the_same_output():
 @pytest.mark.parametrize("H", [1, 80])
 @pytest.mark.parametrize("d", [64, 128, 256])
 @pytest.mark.parametrize("tile", [0, 1])
-def test_a_key_tile_of_nan_scores_leaves_no_finite_row(H, d, tile):
+@pytest.mark.parametrize("softcap", [0.0, 50.0])
+def test_a_key_tile_of_nan_scores_leaves_no_finite_row(H, d, tile, softcap):
     """E5M2 infinities in all columns of a key tile's K: every score of that tile is NaN, O is NaN and the log-sum-exp -inf (what a row sum
     that is not positive gives), whichever thread or group of threads had the tile."""
     qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, 256, 256, d, seed=64), fmt=rk.E5M2)
     kc[:, :, tile * 128:(tile + 1) * 128] = 0x7C
     lse = torch.zeros(1, H, 256, device="cuda")
-    o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False, lse=lse, q_fmt=rk.E5M2, kv_fmt=rk.E5M2)
+    o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False, softcap=softcap, lse=lse, q_fmt=rk.E5M2, kv_fmt=rk.E5M2)
     assert torch.isnan(o).all() and torch.isneginf(lse).all()
     assert rk.last_device_status() == 0
 
