@@ -71,6 +71,9 @@ struct __align__(16) Item {
 };
 static_assert(sizeof(Item) == 32, "its place in shared memory");
 
+// test hook: roles
+constexpr int kPerturbGroup0 = 1 /* 2 = the other group */, kPerturbTma256 = 4, kPerturbQk256 = 5, kPerturbPv256 = 6;
+
 constexpr int kNumSoftmaxWarps = 16;
 constexpr int kThreads256 = (kNumSoftmaxWarps + 4) * 32;
 // 512 * 104 + 128 * 64 = 640 * 96, the registers the block is launched with
@@ -171,6 +174,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
     const int t = state.t + j;                                // barriers and buffers count on from item to item; t & 1 == grp
+    if (stops<DUMP>(p, kPerturbGroup0 + grp, j)) { fail = 101; return false; }
     if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.s_full[grp], (t >> 1) & 1, abort_flag))) { fail = 101; return false; }
     tc_fence_after();
     float s[64];
@@ -501,7 +505,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
       int stopped = 0, st = 0, q_used = 0;
-      uint32_t use = 0, q_par = 0, block = blockIdx.x;
+      uint32_t use = 0, k_loads = 0, q_par = 0, block = blockIdx.x;
       for (uint32_t k = 0;; ++k) {
         w = decode(block);
         // everybody has read the last item: this one takes its place
@@ -513,6 +517,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           stopped = *reinterpret_cast<volatile int*>(p.status);       // an earlier launch gave up on a wait
         }
         for (int j = 0; j < w.n_tiles; ++j) {
+          if (stops<DUMP>(p, kPerturbTma256, j)) { fail = 201; break; }
           if (j == 0) {
             if (q_used) {                            // Q K^T of the last item has finished
               if (!mbar_wait_short<true>(q_empty, q_par, abort_flag)) { fail = 203; break; }
@@ -534,6 +539,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             bulk_load_1d(smem + L::sfk_off + (st * DCH + ch) * kSfAtomBytes,
                          p.k_sf + (((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * DCH + ch) * kSfAtomBytes, kSfAtomBytes, &k_full[st]);
           }
+          ++k_loads;
           if (stopped) break;                        // O is written only where V has come
           if (use > 0 && !mbar_wait_short<true>(&v_empty[st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
           mbar_arrive_expect_tx(&v_full[st], DCH * (p.kv_tile_tx + kSfAtomBytes));
@@ -545,10 +551,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           }
           if (++st == KV_STAGES) { st = 0; ++use; }
         }
-        if (stopped) {
-          *abort_flag = kStopped;
-          if (w.n_tiles > 0) { mbar_wait_short<true>(q_full, 0, nullptr); mbar_wait_short<true>(&k_full[0], 0, nullptr); }
-        }
+        if (stopped) *abort_flag = kStopped;
         if (fail || stopped) break;
         // The next item is asked for now that this one's last loads are under way, and not earlier: the items that are left go to
         // the SMs that are free first.
@@ -563,6 +566,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           break;
         }
         fence_proxy_async_smem();                    // the answer has been read before the next one may overwrite it
+      }
+      // The last loads into each place have arrived, also those whose readers have given up (this lane alone starts phases of these barriers).
+      auto drain = [&](uint64_t* bar, uint32_t parity, int code) { if (!mbar_wait_short<true>(bar, parity, nullptr) && !fail) fail = code; };
+      if (q_used) drain(q_full, q_par, 301);
+      const uint32_t v_loads = use * KV_STAGES + st;
+#pragma unroll 1
+      for (uint32_t i = 0; i < KV_STAGES; ++i) {     // load n, counted from 0, is in stage n % KV_STAGES and phase n / KV_STAGES
+        if (k_loads > i) drain(&k_full[i], ((k_loads - 1 - i) / KV_STAGES) & 1, 302);
+        if (v_loads > i) drain(&v_full[i], ((v_loads - 1 - i) / KV_STAGES) & 1, 303);
       }
       if (fail) give_up(abort_flag, p.status, fail);
     }
@@ -585,6 +597,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       if (more < 0) { fail = kFailWork; break; }
       const int nt = warp_uniform(w.n_tiles);
       for (int j = 0; j < nt; ++j, ++t) {
+        if (stops<DUMP>(p, kPerturbQk256, j)) { fail = 302; break; }
         if (j == 0) {
           if (!__all_sync(0xffffffffu, mbar_wait_short(q_full, q_par, abort_flag))) { fail = 301; break; }
           q_par ^= 1;
@@ -640,6 +653,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const int nt = warp_uniform(w.n_tiles);
       for (int i = 0; i < nt; ++i, ++t) {
         const int pb = t & 1;
+        if (stops<DUMP>(p, kPerturbPv256, i)) { fail = 303; break; }
         if (!__all_sync(0xffffffffu, mbar_wait_short(&v_full[st], use_par, abort_flag))) { fail = 303; break; }
         if (!__all_sync(0xffffffffu, mbar_wait_short(&p_full[pb], (t >> 1) & 1, abort_flag))) { fail = 304; break; }      // (and O of the last item has been read)
         tc_fence_after();
@@ -806,7 +820,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
     if (rc != RK_OK) return rc;
     return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
   }
-  if (p.dbg)      // the stage dump lives in instantiations of its own: the kernels that ship carry none of its code
+  if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)
                : launch_cfg<2, 2, false, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st);
   return cap ? launch_cfg<2, 2, true, false>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)

@@ -38,7 +38,7 @@ struct PrefillParams {
   int q_tile_tx, kv_tile_tx;   // bytes one Q / K / V tile load adds to its mbarrier: 16384, 12288 for 6-bit, 8192 for 4-bit tensors
                                // (the transaction counts the packed source bytes, not the padded shared-memory image)
   int v_transposed;    // V tiles are [d][keys] (K-major B operand; 6-bit V) instead of [keys][d]
-  int perturb;         // test hook: warp role that sleeps a little at every key tile (0 = none)
+  int perturb;         // test hook: warp role that sleeps a little at every key tile, or kStopRole + one that gives up (0 = none)
   float scale_log2;    // softmax_scale * log2(e)
   float cap_log2;      // softcap * log2(e)
   float inv_cap_scale; // softmax_scale / softcap
@@ -49,6 +49,11 @@ constexpr int kStopped = 2;
 RK_DEVINL void give_up(volatile int* abort_flag, int* status, int code) {
   if (*abort_flag != kStopped) report_wait_failure(abort_flag, status, code);
 }
+
+// Test hook, in the instantiations for tests alone: the role acts as if its wait had run out, at its first key tile that is not an item's first.
+constexpr int kStopRole = 100;
+template <bool DUMP>
+RK_DEVINL bool stops(const PrefillParams& p, int role, int j) { return DUMP && p.perturb == kStopRole + role && j >= 1; }
 
 // 32 bytes of a row of O by one thread: a whole sector in one store where O is 32-byte aligned (rows are multiples of 64 bytes), which halves the
 // time of threads that have a row each (d = 256, 2 x 16/8 heads of 8192: 879 -> 866 us); O is guaranteed to be 16-byte aligned only.

@@ -178,6 +178,7 @@ __device__ __forceinline__ bool softmax_row_group(const PrefillParams& p, uint8_
     constexpr bool PLAIN = decltype(plain_tag)::value;
     const int t = t0 + j, pb = t & 1;                         // barriers, P buffers and rescale slots count on from item to item
     perturb<DUMP>(p, kPerturbSoftmaxA + (SPLIT ? half : grp), j);
+    if (stops<DUMP>(p, kPerturbSoftmaxA + (SPLIT ? half : grp), j)) { fail = 101; return false; }
     const bool stamp = (quad == 0 && lane == 0);
     if (stamp) RK_STAMP(grp, j, 0);
     if (__builtin_expect(!__all_sync(0xffffffffu, s_ready), 0)) {   // a test issued during the previous tile said "not yet"
@@ -507,6 +508,7 @@ __device__ __forceinline__ int correction_quadrant(const PrefillParams& p, const
   const int o_chunks = p.d / 32, n_all = max(nt0, nt1);
   for (int j = 0; j < n_all; ++j) {
     perturb<DUMP>(p, kPerturbCorr, j);
+    if (stops<DUMP>(p, kPerturbCorr, j)) return 401;
 #pragma unroll 1
     for (int g = 0; g < 2; ++g) {
       if (j >= (g == 0 ? nt0 : nt1)) continue;
@@ -672,12 +674,13 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (lane == 0) {
         prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
         int stopped = 0, st = 0, q_used = 0, q_par = 0;
-        uint32_t use = 0, block = blockIdx.x;
+        uint32_t use = 0, k_loads = 0, block = blockIdx.x;
         for (uint32_t k = 0;; ++k) {
           w = decode(block);
           const int n_all = max(w.nt0, w.nt1);
           for (int j = 0; j < n_all || j == 0; ++j) {
             perturb<DUMP>(p, kPerturbTma, j);
+            if (stops<DUMP>(p, kPerturbTma, j)) { fail = 201; break; }
             if (j == 0) {
               // everybody has read the last item: this one takes its place
               if (k > 0 && !mbar_wait_short<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
@@ -702,18 +705,14 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (n_all > 0) {
               if (use > 0 && !mbar_wait_short<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
               issue_kv(j, st);
+              ++k_loads;
               if (stopped) break;                    // O is written only where V has come
               if (use > 0 && !mbar_wait_short<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
               issue_v(j, st);
               if (++st == kStages) { st = 0; ++use; }
             }
           }
-          if (stopped) {
-            *abort_flag = kStopped;
-            if (w.nt0 > 0) drain(&bars[bQ], 0, 301);
-            if (w.nt1 > 0) drain(&bars[bQB], 0, 301);
-            if (n_all > 0) drain(&bars[bKF], 0, 302);
-          }
+          if (stopped) *abort_flag = kStopped;
           if (fail || stopped || SPLIT) break;
           // The next item is asked for now that this one's last loads are under way, three tiles before its end, and not earlier: the items
           // that are left go to the SMs that are free first.
@@ -729,6 +728,16 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             break;
           }
           fence_proxy_async_smem();                  // the answer has been read before the next one may overwrite it
+        }
+        // The last loads into each place have arrived, also those whose readers have given up (this lane alone starts phases of these barriers).
+#pragma unroll 1
+        for (int g = 0; g < 2; ++g)
+          if ((q_used >> g) & 1) drain(&bars[g == 0 ? bQ : bQB], (q_par >> g) & 1, 301);
+        const uint32_t v_loads = use * kStages + st;
+#pragma unroll 1
+        for (uint32_t i = 0; i < kStages; ++i) {     // load n, counted from 0, is in stage n % kStages and phase n / kStages
+          if (k_loads > i) drain(&bars[bKF + i], ((k_loads - 1 - i) / kStages) & 1, 302);
+          if (v_loads > i) drain(&bars[bVF + i], ((v_loads - 1 - i) / kStages) & 1, 303);
         }
       }
       __syncwarp();
@@ -752,6 +761,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int nt0 = warp_uniform(w.nt0), nt1 = warp_uniform(w.nt1), n_all = max(nt0, nt1);
         for (int j = 0; j < n_all && !fail; ++j) {
           perturb<DUMP>(p, kPerturbQk, j);
+          if (stops<DUMP>(p, kPerturbQk, j)) { fail = 302; break; }
           if (lane == 0) RK_STAMP(2, j, 0);
           if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfK + st * 4, dsfk + (uint32_t)(st * (kSfAtomBytes >> 4)));
@@ -808,6 +818,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int nt0 = warp_uniform(w.nt0), nt1 = warp_uniform(w.nt1), n_all = max(nt0, nt1);
         for (int i = 0; i < n_all && !fail; ++i) {
           perturb<DUMP>(p, kPerturbPv, i);
+          if (stops<DUMP>(p, kPerturbPv, i)) { fail = 303; break; }
           if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfV + st * 4, dsfv + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dvt = dv + (uint32_t)(st * (kTileBytes >> 4));

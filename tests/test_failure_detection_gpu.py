@@ -71,6 +71,30 @@ def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0):
     assert rk.last_device_status() == 0 and not (o == 7.0).all() and not (lse == 7.0).any()
 
 
+@pytest.mark.parametrize("H,S,d", [(2, 600, 128), (100, 600, 128), (200, 300, 64), (2, 600, 256), (100, 600, 256)])      # a CTA per query tile, and many items each
+def test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d):
+    """One warp role at a time (either softmax group, correction, TMA producer, Q K^T and P V issuer) acts after a key tile as if its
+    wait had run out: loads, MMAs and stores are under way, the other roles see the CTA's flag, the kernel ends, a code is reported and the next
+    call has every bit of the one before."""
+    L = rk.lib()
+    qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, S, S, d, seed=93))
+    want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
+    assert rk.last_device_status() == 0
+    for role in (1, 2, 3, 4, 5, 6):
+        if d == 256 and role == 3:
+            continue                                                    # no correction warps there
+        L.rk_debug_set_prefill_perturb(100 + role)
+        try:
+            rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
+            torch.cuda.synchronize()
+        finally:
+            L.rk_debug_set_prefill_perturb(0)
+            status = rk.last_device_status()
+        assert 100 < status < 600, (role, status)
+        assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False), want), role
+        assert rk.last_device_status() == 0
+
+
 def test_noalloc_decode_status_word_is_observable():
     L = rk.lib()
     g = torch.Generator(device="cuda").manual_seed(91)
