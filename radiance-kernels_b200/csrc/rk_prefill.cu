@@ -71,8 +71,10 @@ struct __align__(16) Item {
 };
 static_assert(sizeof(Item) == 32, "its place in shared memory");
 
-// test hook: roles
-constexpr int kPerturbGroup0 = 1 /* 2 = the other group */, kPerturbTma256 = 4, kPerturbQk256 = 5, kPerturbPv256 = 6;
+// test hook: which role sleeps a little at every key tile (schedule perturbation); kPerturbOut256: the upper part's warps while they write O out and
+// before they hand over their shares of the row sums
+constexpr int kPerturbGroup0 = 1 /* 2 = the other group */, kPerturbUpper256 = 3 /* keys 64-127 of a tile */, kPerturbTma256 = 4, kPerturbQk256 = 5,
+              kPerturbPv256 = 6, kPerturbOut256 = 7;
 
 constexpr int kNumSoftmaxWarps = 16;
 constexpr int kThreads256 = (kNumSoftmaxWarps + 4) * 32;
@@ -99,7 +101,9 @@ __device__ __forceinline__ bool write_out_rows(const PrefillParams& p, uint8_t* 
   using L = SmemLayout<DCH, KV_STAGES>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = (warp >> 2) & 1, row = quad * 32 + lane;
   const int item = st.items - 1;
+  if (part == 1) perturb<DUMP>(p, kPerturbOut256, quad);
   if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.end_bar[quad], item & 1, abort_flag))) return false;
+  if (part == 1) perturb<DUMP>(p, kPerturbOut256, quad);      // (its partner has read the shares and goes on)
   const float2* share = reinterpret_cast<const float2*>(smem + L::end_off) + (item & 1) * 4 * 128 + row;
   const float NEG_INF = __int_as_float(0xff800000);
   const float m = fmaxf(fmaxf(share[0].y, share[128].y), fmaxf(share[256].y, share[384].y));
@@ -174,6 +178,8 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
   auto tile = [&](const int j, auto plain_tag) -> bool {
     constexpr bool PLAIN = decltype(plain_tag)::value;
     const int t = state.t + j;                                // barriers and buffers count on from item to item; t & 1 == grp
+    perturb<DUMP>(p, kPerturbGroup0 + grp, j);
+    if (part == 1) perturb<DUMP>(p, kPerturbUpper256, j);
     if (stops<DUMP>(p, kPerturbGroup0 + grp, j)) { fail = 101; return false; }
     if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.s_full[grp], (t >> 1) & 1, abort_flag))) { fail = 101; return false; }
     tc_fence_after();
@@ -348,6 +354,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
   // The shares go over by threads that had a tile of the item, and by them alone: such a thread's last tile has waited for all that the shares' readers of
   // the item before did (a P V of this item needs their O written out), so neither the shares of two items nor two phases of a barrier
   // can meet.  One that had none, for an item of one key tile, would run ahead of its own partner; the group with the tile hands over empty shares for it.
+  if (part == 1) perturb<DUMP>(p, kPerturbOut256, quad);
   const int odd = grp ^ (state.t & 1);                         // this group had the item's tiles 0, 2, .. or 1, 3, ..
   if (odd < n_tiles) {
     float2* share = reinterpret_cast<float2*>(smem + L::end_off) + ((state.items & 1) * 4 + part) * 128 + row;
@@ -517,6 +524,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           stopped = *reinterpret_cast<volatile int*>(p.status);       // an earlier launch gave up on a wait
         }
         for (int j = 0; j < w.n_tiles; ++j) {
+          perturb<DUMP>(p, kPerturbTma256, j);
           if (stops<DUMP>(p, kPerturbTma256, j)) { fail = 201; break; }
           if (j == 0) {
             if (q_used) {                            // Q K^T of the last item has finished
@@ -597,6 +605,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       if (more < 0) { fail = kFailWork; break; }
       const int nt = warp_uniform(w.n_tiles);
       for (int j = 0; j < nt; ++j, ++t) {
+        perturb<DUMP>(p, kPerturbQk256, j);
         if (stops<DUMP>(p, kPerturbQk256, j)) { fail = 302; break; }
         if (j == 0) {
           if (!__all_sync(0xffffffffu, mbar_wait_short(q_full, q_par, abort_flag))) { fail = 301; break; }
@@ -653,6 +662,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const int nt = warp_uniform(w.n_tiles);
       for (int i = 0; i < nt; ++i, ++t) {
         const int pb = t & 1;
+        perturb<DUMP>(p, kPerturbPv256, i);
         if (stops<DUMP>(p, kPerturbPv256, i)) { fail = 303; break; }
         if (!__all_sync(0xffffffffu, mbar_wait_short(&v_full[st], use_par, abort_flag))) { fail = 303; break; }
         if (!__all_sync(0xffffffffu, mbar_wait_short(&p_full[pb], (t >> 1) & 1, abort_flag))) { fail = 304; break; }      // (and O of the last item has been read)

@@ -50,7 +50,12 @@ RK_DEVINL void give_up(volatile int* abort_flag, int* status, int code) {
   if (*abort_flag != kStopped) report_wait_failure(abort_flag, status, code);
 }
 
-// Test hook, in the instantiations for tests alone: the role acts as if its wait had run out, at its first key tile that is not an item's first.
+// Test hooks, in the instantiations for tests alone.  perturb: the role sleeps a little, longer or shorter from key tile to key tile.
+template <bool DUMP>
+RK_DEVINL void perturb(const PrefillParams& p, int role, int j) {
+  if (DUMP && __builtin_expect(p.perturb == role, 0)) __nanosleep(400 + 97 * (j & 7));
+}
+// stops: the role acts as if its wait had run out, at its first key tile that is not an item's first.
 constexpr int kStopRole = 100;
 template <bool DUMP>
 RK_DEVINL bool stops(const PrefillParams& p, int role, int j) { return DUMP && p.perturb == kStopRole + role && j >= 1; }

@@ -172,6 +172,35 @@ def test_schedule_perturbation_leaves_every_bit_of_o(shape):
     assert rk.last_device_status() == 0
 
 
+# heads, queries, d, cap, options; heads 0: as many as it takes to have at least three items per SM
+@pytest.mark.parametrize("shape", [(0, 100, 128, 0.0, {}), (0, 384, 64, 0.0, {}), (0, 200, 128, 30.0, dict(causal=False)), (0, 700, 128, 0.0, dict(window=150)),
+                                   (0, 390, 128, 0.0, dict(q_pos0=-130)),
+                                   (4, 600, 256, 0.0, {}), (0, 100, 256, 0.0, {}), (0, 128, 256, 50.0, dict(causal=False)), (0, 300, 256, 50.0, {}),
+                                   (0, 640, 256, 0.0, dict(causal=False)), (0, 390, 256, 0.0, dict(q_pos0=-130)), (0, 700, 256, 0.0, dict(window=150))])
+def test_schedule_perturbation_where_ctas_take_item_after_item(shape):
+    """The same where a CTA goes on to other items, with a seventh role, O's way out (in it the delays lie between chunks, and before what the softmax
+    warps leave behind of an item), and at d = 256: softmax group 0, group 1, the upper keys' warps of both, TMA producer, the issuers, O's way out.
+    Items of one key tile and of none, odd and even numbers of them; O and the log-sum-exps."""
+    H, S, d, cap, kw = shape
+    L = rk.lib()
+    if H == 0:
+        per_head = (S + 127) // 128 if d == 256 else (S + 255) // 256
+        H = -(-3 * torch.cuda.get_device_properties(0).multi_processor_count // per_head)
+    qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, S, S, d, seed=94))
+    kw = dict(dict(causal=True, softcap=cap), **kw)
+    lse0, lse = torch.empty(1, H, S, device="cuda"), torch.empty(1, H, S, device="cuda")
+    base = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse0, **kw)
+    try:
+        for role in (1, 2, 3, 4, 5, 6, 7):
+            L.rk_debug_set_prefill_perturb(role)
+            for _ in range(2):
+                assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw), base), role
+                assert torch.equal(lse, lse0), role
+    finally:
+        L.rk_debug_set_prefill_perturb(0)
+    assert rk.last_device_status() == 0
+
+
 def test_tensor_pipe_ceiling_loop_never_runs_into_its_waits():
     """The GEMM-only loop bench.py measures the tensor-pipe ceiling with paces itself through two alternating
     mbarriers (one barrier per batch in flight: a barrier that completes two phases before its waiter looks reads as
