@@ -575,7 +575,7 @@ RK_API int rk_debug_verify_encoder(int fmt, unsigned long long* mismatches, uint
   return launch_verify_encoder(fmt, mismatches, first_bad, (cudaStream_t)stream);
 }
 
-/* Test hook (not in the public header): stage dump of the first query tile / first key tile of
+/* Test hook (not in the public header): stage dump of the last query tile of the first head / first key tile of
  * the next prefill launches into `buf` (>= 32768 floats), or NULL to switch it off. */
 RK_API void rk_debug_set_prefill_dump(float* buf) { g_prefill_dbg = buf; }
 
@@ -601,8 +601,10 @@ RK_API int rk_debug_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile,
   return launch_mxfp8_mma_loop(a_tile, b_tile, iters, (cudaStream_t)stream);
 }
 
-/* Test hook (not in the public header): which warp role of the d <= 128 prefill kernel sleeps a little at every key
- * tile (0 = none; 1, 2 = softmax of query tile A, B; 3 = correction; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer). */
+/* Test hook (not in the public header): which warp role of the prefill kernels sleeps a little at every key tile (0 = none;
+ * 1, 2 = softmax of query tile A, B, of the lower and upper keys where a CTA has one query tile, at d = 256 of the two groups; 3 = correction, at
+ * d = 256 the upper keys' softmax warps; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer; 7 = O on its way out).
+ * 100 + role: the role acts after a key tile as if its wait had run out (not 103 at d = 256, nor 107). */
 RK_API void rk_debug_set_prefill_perturb(int role) { g_prefill_perturb = role; }
 
 }  // extern "C"

@@ -9,8 +9,8 @@
 // mapped onto Blackwell units:
 //   mxgemm_prefetch_tile / mxgemm_compute_tile (mesh)  -> TMA + tcgen05.mma
 //   fused_softmax_requant_tpr (one lane per row,
-//     flash_mx_impl.hpp:314-394)                       -> four threads per row, one 32-key block each in registers
-//   pack_scales_to_sfmem (flash_mx_impl.hpp:625-639)   -> one st.shared per row + tcgen05.cp
+//     flash_mx_impl.hpp:314-394)                       -> two threads per row, two 32-key blocks each in registers
+//   pack_scales_to_sfmem (flash_mx_impl.hpp:625-639)   -> one st.shared per thread + tcgen05.cp
 //   rescale_accumulate / finalize_O (:508-553)         -> O kept in TMEM, rescaled in place
 //
 // A CTA works on one 128-row query tile of one (batch, head) at a time.  640 threads:
@@ -23,7 +23,8 @@
 //   warp  19    fills the warpgroup (registers are moved between warpgroups with setmaxnreg)
 // The two groups are half a tile apart: while one forms exponentials (special-function unit) the other caps scores, takes maxima and
 // rescales O (FMA and integer pipes).  All sixteen warps in the same phase of the same tile took 3600 cycles a tile with the
-// cap and 2900 without; 2 x 16/8 heads of 8192: capped 974 -> 894 us, without the cap 796 -> 726, two heads of 300 keys 14.5 -> 11.9.
+// cap and 2900 without; 2 x 16/8 heads of 8192: capped 974 -> 894 us, without the cap 796 -> 726, two heads of 300 keys 14.5 -> 11.9 (full clock; with what
+// came after 865 capped, and 958 call after call under the power cap).
 // Keys are walked in tiles of 128 (the online-softmax step, "block_n").
 //
 // Roofline: tensor-core bound by FLOP count (4*S_q*S_kv*d per head, half of it
@@ -78,7 +79,8 @@ constexpr int kPerturbGroup0 = 1 /* 2 = the other group */, kPerturbUpper256 = 3
 
 constexpr int kNumSoftmaxWarps = 16;
 constexpr int kThreads256 = (kNumSoftmaxWarps + 4) * 32;
-// 512 * 104 + 128 * 64 = 640 * 96, the registers the block is launched with
+// 512 * 104 + 128 * 64 = 640 * 96, the registers the block is launched with.  ptxas allocates by the 96, and spills 28 bytes of a thread
+// (76 bytes of reloads in the code).
 constexpr uint32_t kRegSoftmax256 = 104, kRegIssue256 = 64;
 template <uint32_t N> RK_DEVINL void reg_inc256() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <uint32_t N> RK_DEVINL void reg_dec256() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }

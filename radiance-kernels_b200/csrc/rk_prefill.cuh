@@ -29,7 +29,7 @@ struct PrefillParams {
   __nv_bfloat16* o;
   float* lse;
   int* status;
-  float* dbg;          // optional stage dump of CTA (0,0,0), first key tile
+  float* dbg;          // optional stage dump (tests): last query tile of the first head, first key tile
   int B, H, H_kv, S_q, S_kv, d;
   int group;           // query heads per KV head
   int n_q_tiles, n_kv_tiles;
@@ -60,8 +60,9 @@ constexpr int kStopRole = 100;
 template <bool DUMP>
 RK_DEVINL bool stops(const PrefillParams& p, int role, int j) { return DUMP && p.perturb == kStopRole + role && j >= 1; }
 
-// 32 bytes of a row of O by one thread: a whole sector in one store where O is 32-byte aligned (rows are multiples of 64 bytes), which halves the
-// time of threads that have a row each (d = 256, 2 x 16/8 heads of 8192: 879 -> 866 us); O is guaranteed to be 16-byte aligned only.
+// 32 bytes of a row of O by one thread: a whole sector in one store where O is 32-byte aligned (rows are multiples of 64 bytes), where two stores of
+// a thread with a row of its own are half a sector each (d = 256, 2 x 16/8 heads of 8192, under the power cap: 969 -> 958 us); O is guaranteed to be
+// 16-byte aligned only.
 RK_DEVINL void store_row32(__nv_bfloat16* dst, const uint32_t (&w)[8], bool aligned32) {
   if (aligned32) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -168,13 +169,13 @@ RK_DEVINL uint32_t pack_u8x2(uint32_t hi, uint32_t lo, uint32_t c) {
 }
 
 #ifdef RK_X_STAMPS
-// Timeline stamps (measurement builds only): clock64 of chosen events of one CTA, written into the dump buffer.
-// The CTA is RK_X_STAMP_BLOCK, or the block index b when the perturbation hook is set to 1000 + b (+ 100000 * (s + 1)
-// to pick the s-th work item of a persistent CTA).
+// Timeline stamps (measurement builds of the d <= 128 kernel only): clock64 of chosen events of one CTA, written into the dump buffer, by role and key
+// tile of an item.  A CTA that takes several items leaves those of the last one that had the tile.
+// The CTA is RK_X_STAMP_BLOCK, or the block index b when the perturbation hook is set to 1000 + b.
 #ifndef RK_X_STAMP_BLOCK
 #define RK_X_STAMP_BLOCK 0
 #endif
-#define RK_STAMP_CTA ((int)blockIdx.x == (p.perturb % 100000 >= 1000 ? p.perturb % 100000 - 1000 : RK_X_STAMP_BLOCK))
+#define RK_STAMP_CTA ((int)blockIdx.x == (p.perturb >= 1000 ? p.perturb - 1000 : RK_X_STAMP_BLOCK))
 #define RK_STAMP(slot, j, k) do { if (p.dbg && RK_STAMP_CTA && (j) < 32) \
     reinterpret_cast<unsigned*>(p.dbg)[24576 + (slot) * 512 + (j) * 8 + (k)] = (unsigned)clock64(); } while (0)
 #define RK_STAMP_RAW(idx) do { if (p.dbg && RK_STAMP_CTA) \

@@ -26,12 +26,12 @@
 // on while group B, one tile longer under a causal mask, finishes, and the correction warps write an item's O out while the softmax
 // warps are in their next tile.  With a CTA per pair an item of 16 tiles cost 17 000 cycles on top of them (start 4400, first loads,
 // a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
-// 8192 2030 -> 1764 us.
+// 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.
 //
 // SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle (chunks of a prompt, short prompts).  A key tile's time is
 // then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
 // on the same tile, group A on keys 0-63 of each key tile and group B on keys 64-127, and exchange their row maxima through
-// shared memory.  32 heads x 509 queries behind 3581 keys: the call 76 us with tile pairs on 64 SMs, 43.5 us now.
+// shared memory.  32 heads x 509 queries behind 3581 keys: the call 76 us with tile pairs on 64 SMs, 42.6 us now.
 #include <type_traits>
 
 #include "rk_prefill.cuh"
@@ -43,7 +43,9 @@ constexpr int kStages = 3;
 constexpr int kThreads = 512;
 constexpr int kWarpCorr = 8, kWarpTma = 12, kWarpQk = 13, kWarpPv = 14;
 // Registers of a softmax, correction and issuer thread: 128 * (2 * softmax + correction + issuer) = 65536.  Measured (8 x 16 heads of
-// 4096): softmax 168 515 us, 176 518, 184 521, 192 523, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
+// 4096, full clock): softmax 168 515 us, 176 518, 184 521, 192 523, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
+// 176 and not 168 for the capped form, which is 1 % slower with 168 (8 x 16 heads of 4096 791 us and 784, 4 x 32 / 8 of 8192 2659 and 2629); without
+// the cap 168 is 0.5 % faster (555.1 and 558.1, 1885 and 1893 under the power cap).
 constexpr uint32_t kRegSoftmax = 176, kRegCorr = 88, kRegIssue = 72;
 constexpr uint32_t kRegSoftmaxSplit = 176, kRegCorrSplit = 80, kRegIssueSplit = 80;      // 509 queries behind 3581 keys: softmax 144 43.9 us, 160 44.4, 176 43.5, 192 43.6
 // TMEM columns
@@ -115,8 +117,8 @@ __device__ __forceinline__ void mask_scores(uint32_t s_addr, const PrefillParams
   tc_wait_st();
 }
 
-// The blocking form of the two waits a key tile starts with (its S, and the P buffer it will write): out of line, so
-// that the tile body carries only the test of two flags.  Returns 0, or the code of the wait that gave up.
+// The blocking form of the two waits a key tile starts with (its S, and the P buffer it will write), for tiles whose
+// early tests said "not yet".  Inline: as a function call it made the kernel 23 % slower.  Returns 0, or the code of the wait that gave up.
 __device__ __forceinline__ int wait_tile_inputs(uint64_t* s_full, uint32_t s_parity, uint64_t* pv_done, uint32_t pv_parity,
                                              int need_pv, volatile int* abort_flag) {
   if (!mbar_wait_short(s_full, s_parity, abort_flag)) return 101;
