@@ -82,8 +82,6 @@ constexpr int kThreads256 = (kNumSoftmaxWarps + 4) * 32;
 // 512 * 104 + 128 * 64 = 640 * 96, the registers the block is launched with.  ptxas allocates by the 96, and spills 28 bytes of a thread
 // (76 bytes of reloads in the code).
 constexpr uint32_t kRegSoftmax256 = 104, kRegIssue256 = 64;
-template <uint32_t N> RK_DEVINL void reg_inc256() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <uint32_t N> RK_DEVINL void reg_dec256() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // What a softmax thread keeps from item to item.
 struct SoftmaxState {
@@ -408,23 +406,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int fail = 0;                                      // which wait of an issuer gave up
-  // work order over the block indices: see PrefillParams::head_group (heaviest query tiles of a whole group of heads first)
   auto decode = [&](uint32_t block) -> Item {
     Item w;
-    const uint32_t n_bh = p.B * p.H, per_group = p.n_q_tiles * p.head_group;
-    const uint32_t grp_i = block / per_group, r = block - grp_i * per_group;
-    const uint32_t heads_here = min((uint32_t)p.head_group, n_bh - grp_i * p.head_group);
-    const uint32_t down = r / heads_here;
-    w.qt = p.n_q_tiles - 1 - (int)down;
-    w.bh = grp_i * p.head_group + (r - down * heads_here);
-    w.bhkv = (uint32_t)w.bh / (uint32_t)p.group;
-    // key tiles this query tile needs: causal tiles wholly above the diagonal are never touched
-    // (blocks_used, kernels/flash_attention_mx_gqa/flash_attention_model.py:182-186)
-    w.n_tiles = p.n_kv_tiles;
-    if (p.causal) {
-      const int max_qpos = p.q_pos0 + min(w.qt * kBlockM + kBlockM, p.S_q) - 1;
-      w.n_tiles = max_qpos < 0 ? 0 : min(w.n_tiles, max_qpos / kBlockN + 1);
-    }
+    const Place at = place_of_block(p, block, p.n_q_tiles);
+    w.qt = at.index; w.bh = at.bh; w.bhkv = at.bhkv;
+    w.n_tiles = key_tiles(p, w.qt);
     // sliding window: key tiles wholly below the window of the tile's first row are masked for every row of it
     w.j0 = 0;
     if (p.window > 0) {
@@ -480,7 +466,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   constexpr int kFailWork = 501;
 
   if (warp < kNumSoftmaxWarps) {
-    reg_inc256<kRegSoftmax256>();
+    reg_inc<kRegSoftmax256>();
     SoftmaxState state = {0, 0, 0, 0};
     const SoftmaxBars sb = {s_full, s_empty, p_full, pv_done, row_bar, end_bar};
     int more;
@@ -510,7 +496,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
   } else if (warp == kNumSoftmaxWarps) {
     // ================= TMA producer; hands out the items =================
-    reg_dec256<kRegIssue256>();
+    reg_dec<kRegIssue256>();
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
       int stopped = 0, st = 0, q_used = 0;
@@ -590,9 +576,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
     __syncwarp();
   } else if (warp == kNumSoftmaxWarps + 3) {
-    reg_dec256<kRegIssue256>();
+    reg_dec<kRegIssue256>();
   } else if (warp == kNumSoftmaxWarps + 1) {
-    reg_dec256<kRegIssue256>();
+    reg_dec<kRegIssue256>();
     // ================= issuer of S = Q K^T =================
     // The whole warp runs the loop and one elected lane issues: what an MMA takes (descriptors, addresses) then is in uniform registers.
     // Inside one lane's branch each operand was moved there for every MMA (d <= 128: 660 cycles to issue four).
@@ -646,7 +632,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     if (fail) give_up(abort_flag, p.status, fail);
     __syncwarp();
   } else {
-    reg_dec256<kRegIssue256>();
+    reg_dec<kRegIssue256>();
     // ================= issuer of O += P V =================
     const uint32_t tm = warp_uniform(tmem_base);
     const uint64_t dp = make_smem_desc(smem_u32(smem + L::p_off), 16, 1024, kLayoutSw128);

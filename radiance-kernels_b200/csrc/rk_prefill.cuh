@@ -50,6 +50,33 @@ RK_DEVINL void give_up(volatile int* abort_flag, int* status, int code) {
   if (*abort_flag != kStopped) report_wait_failure(abort_flag, status, code);
 }
 
+// Registers moved between warpgroups.
+template <uint32_t N> RK_DEVINL void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <uint32_t N> RK_DEVINL void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Work order over the block indices: (batch, head) pairs are taken in groups of p.head_group; inside a group the heaviest (latest) of the n places
+// of a head -- query tiles, or pairs of them -- come first for all its heads and the lightest last, so the grid ends on short items, while a
+// group's K/V still fits in L2.
+struct Place { int index, bh, bhkv; };      // place within the head, b * H + h, b * H_kv + h / group
+RK_DEVINL Place place_of_block(const PrefillParams& p, uint32_t block, int n) {
+  const uint32_t n_bh = p.B * p.H, per_group = n * p.head_group;
+  const uint32_t grp_i = block / per_group, r = block - grp_i * per_group;
+  const uint32_t heads_here = min((uint32_t)p.head_group, n_bh - grp_i * p.head_group);
+  const uint32_t down = r / heads_here;
+  Place w;
+  w.index = n - 1 - (int)down;
+  w.bh = grp_i * p.head_group + (r - down * heads_here);
+  w.bhkv = (uint32_t)w.bh / (uint32_t)p.group;
+  return w;
+}
+// Key tiles a query tile needs, from the first: causal tiles wholly above the diagonal are never touched (blocks_used,
+// kernels/flash_attention_mx_gqa/flash_attention_model.py:182-186).
+RK_DEVINL int key_tiles(const PrefillParams& p, int qt) {
+  if (!p.causal) return p.n_kv_tiles;
+  const int max_qpos = p.q_pos0 + min(qt * kBlockM + kBlockM, p.S_q) - 1;
+  return max_qpos < 0 ? 0 : min(p.n_kv_tiles, max_qpos / kBlockN + 1);
+}
+
 // Test hooks, in the instantiations for tests alone.  perturb: the role sleeps a little, longer or shorter from key tile to key tile.
 template <bool DUMP>
 RK_DEVINL void perturb(const PrefillParams& p, int role, int j) {

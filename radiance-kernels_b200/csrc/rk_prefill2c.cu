@@ -89,9 +89,6 @@ static_assert(sizeof(Work) == 32, "its place in shared memory");
 constexpr int kReaders = 8 + 4 + 2;      // warps that read an item: softmax, correction, Q K^T, P V
 }  // namespace c2
 
-template <uint32_t N> RK_DEVINL void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <uint32_t N> RK_DEVINL void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-
 // ---- softmax warps: thread = query row -----------------------------------------------------------------------
 // The loop over key tiles is what runs nearly all the time, and it is kept small: an SM's instruction cache holds 32 KB, a body is
 // 15 KB of straight-line code, and code that is not in the cache runs at a third of the speed.  So there is one body; the few
@@ -565,30 +562,15 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (threadIdx.x == 0) RK_STAMP(2, 0, 6);
   constexpr int kQt = SPLIT ? 1 : 2;                                  // query tiles per item
   const int n_pairs = (p.n_q_tiles + kQt - 1) / kQt;
-  // Work order over the block indices: (batch, head) pairs are taken in groups of p.head_group; inside a group the
-  // heaviest (latest) query-tile pairs of all its heads come first and the lightest last, so the grid ends on
-  // short items, while a group's K/V still fits in L2.
   auto decode = [&](uint32_t block) -> Work {
     Work w;
-    const uint32_t n_bh = p.B * p.H, per_group = n_pairs * p.head_group;
-    const uint32_t grp_i = block / per_group, r = block - grp_i * per_group;
-    const uint32_t heads_here = min((uint32_t)p.head_group, n_bh - grp_i * p.head_group);
-    const uint32_t down = r / heads_here;
-    w.qp = n_pairs - 1 - (int)down;
-    w.bh = grp_i * p.head_group + (r - down * heads_here);
-    w.bhkv = (uint32_t)w.bh / (uint32_t)p.group;
-    // key tiles each query tile needs (causal tiles wholly above the diagonal are never touched,
-    // kernels/flash_attention_mx_gqa/flash_attention_model.py:182-186); a tile past S_q needs none
-    int nt[2];
+    const Place at = place_of_block(p, block, n_pairs);
+    w.qp = at.index; w.bh = at.bh; w.bhkv = at.bhkv;
+    int nt[2];                                                        // a tile past S_q needs none
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
       const int qt = kQt * w.qp + g;
-      int n = (g < kQt && qt < p.n_q_tiles) ? p.n_kv_tiles : 0;
-      if (n > 0 && p.causal) {
-        const int max_qpos = p.q_pos0 + min(qt * kBlockM + kBlockM, p.S_q) - 1;
-        n = max_qpos < 0 ? 0 : min(n, max_qpos / kBlockN + 1);
-      }
-      nt[g] = n;
+      nt[g] = (g < kQt && qt < p.n_q_tiles) ? key_tiles(p, qt) : 0;
     }
     // sliding window: key tiles wholly below the window of the pair's first row are masked for every row of both tiles
     w.j0 = 0;
