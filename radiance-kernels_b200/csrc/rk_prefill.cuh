@@ -143,8 +143,8 @@ RK_DEVINL uint64_t mul2p(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2
 // softcap_pair, which is kept for the scores that are not small.  The decision is per warp and 64 keys of a key tile, whether a thread has
 // 64 scores of the tile or all 128: the two forms differ in a score's last bits, and a row comes out the same in every form of the kernels.
 // Both sets of a thread with 128 are decided by one reduction over the warp, and the series of both is one run of code, against two votes and a
-// branch for each: 8 x 16 heads of 4096 at d = 128, cap 50, 810 us and 786; decided for all 128 at once 792. (Logits of standard deviation 4, all
-// exponential: 1 242, 1 235 and 1 201.)
+// branch for each: 8 x 16 heads of 4096 at d = 128, cap 50, 810 us and 784; decided for all 128 at once 791. (Logits of standard deviation 4, all
+// exponential: 1 242, 1 247 and 1 206.)
 template <int N>
 RK_DEVINL void softcap_scores(float (&s)[N], float scale_log2, float cap_log2, float inv_cap_scale) {
   static_assert(N == 64 || N == 128, "one or two sets of 64 scores");
