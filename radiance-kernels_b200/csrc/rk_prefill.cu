@@ -765,6 +765,26 @@ static int launch_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 float* g_prefill_dbg = nullptr;   // set by rk_debug_set_prefill_dump (tests only)
 int g_prefill_perturb = 0;
 
+// d <= 128: one query tile per CTA at a time with the softmax groups on alternate key tiles (rk_prefill1.cu), or pairs of query tiles (rk_prefill2c.cu,
+// which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1700 cycles in the former and
+// half of 3450 in the latter, which loads K and V half as often and so loses less under the power cap: it has the large grids.  Measured (us, the pairs'
+// kernel and this one):
+//   no more query tiles than SMs: 8 / 32 heads of 512 11.1 10.5 / 13.9 13.4, 16 of 1024 18.5 17.2, 8 of 2048 27.7 24.3, 32 x 509 queries behind 3581 keys
+//     42.1 36.8.  Up to three key tiles the time is that of code run for the first time, of which the other form has less: 42 heads of 300 12.1 12.5, 128 of
+//     100 10.6 11.0.  With the cap 54.5 56.5 on the same chunk.
+//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  512 queries behind 4096 keys, 72 heads (288 tiles) 70.8 71.8,
+//     96 heads 126 100; without a mask 500 by 700 keys 40 heads 20.9 22.0; capped, 64 heads 90.7 102, 96 heads 160 143.
+//   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 40.6 24.9, 16 40.9 28.6, 23 42.3 37.8,
+//     27 43.3 43.0; 23 heads of 1024 25.9 18.1, 37 26.9 24.4, 47 27.4 27.9; 24 capped heads of 1024 31.8 22.3; 24 of 2048 with a window of 512 33.0 27.1.
+static bool alternate_key_tiles(const PrefillParams& p, bool cap) {
+  const int64_t sms = num_sms(), heads = (int64_t)p.B * p.H, tiles = p.n_q_tiles * heads, pairs = (p.n_q_tiles + 1) / 2 * heads;
+  const int item_tiles = p.window > 0 ? std::min(p.n_kv_tiles, (p.window + kBlockM - 2) / kBlockN + 2) : p.n_kv_tiles;     // at most
+  if (tiles <= sms) return item_tiles > 3 && !cap;
+  const bool level = p.window == 0 && (!p.causal || 2 * ((int64_t)p.q_pos0 + kBlockM) > p.S_kv);
+  if (level) return 10 * ((tiles + sms - 1) / sms) < 19 * ((pairs + sms - 1) / sms);
+  return 2 * tiles <= (item_tiles > 8 ? 6 : 5) * sms;
+}
+
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
@@ -816,7 +836,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
     CUtensorMap to;
     rc = make_tmap_o(&to, a.o, (int64_t)a.B * a.H, a.S_q, a.d);
     if (rc != RK_OK) return rc;
-    return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
+    return (alternate_key_tiles(p, cap) ? launch_prefill1 : launch_prefill2c)(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
   }
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)

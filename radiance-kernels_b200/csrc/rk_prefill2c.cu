@@ -28,10 +28,10 @@
 // a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
 // 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.
 //
-// SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle (chunks of a prompt, short prompts).  A key tile's time is
-// then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
+// SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle and whose items are too short for rk_prefill1.cu, or capped.  A key
+// tile's time is then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
 // on the same tile, group A on keys 0-63 of each key tile and group B on keys 64-127, and exchange their row maxima through
-// shared memory.  32 heads x 509 queries behind 3581 keys: the call 76 us with tile pairs on 64 SMs, 42.6 us now.
+// shared memory.
 #include <type_traits>
 
 #include "rk_prefill.cuh"
@@ -910,8 +910,7 @@ static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                      uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st) {
-  // One query tile per CTA while every tile can have an SM: above that, two tiles per CTA share K, V and the SM (256 tiles:
-  // 91 us in one wave of pairs against 110 in two of single tiles).
+  // One query tile per CTA while every tile can have an SM: above that, two tiles per CTA share K, V and the SM.
   const bool split = (int64_t)p.n_q_tiles * p.H * p.B <= num_sms();
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return split ? (softcap ? launch2c_cfg<true, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)

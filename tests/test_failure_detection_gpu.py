@@ -201,6 +201,20 @@ def test_schedule_perturbation_where_ctas_take_item_after_item(shape):
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("shape", [(118, 300, 128, 0.0, {}), (88, 390, 64, 0.0, dict(q_pos0=-130)), (58, 700, 128, 0.0, dict(window=150)), (80, 500, 128, 30.0, {}),
+                                   (420, 100, 64, 0.0, dict(causal=False)),           # one query tile at a time, key tiles in turn
+                                   (240, 500, 128, 0.0, {}), (300, 300, 64, 30.0, {})])        # pairs
+def test_schedule_perturbation_in_both_kernels_of_narrow_heads(shape):
+    """The delays of the test above where a CTA has some three query tiles one after the other, and where it has as many pairs of them."""
+    H, S, d, cap, kw = shape
+    test_schedule_perturbation_where_ctas_take_item_after_item((H, S, d, cap, kw))
+
+
+@pytest.mark.parametrize("H,S,d", [(2, 300, 128), (300, 512, 128), (250, 1024, 64)])      # 64 keys a group; pairs
+def test_a_role_that_gives_up_in_the_other_forms_for_narrow_heads(H, S, d):
+    test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d)
+
+
 def test_tensor_pipe_ceiling_loop_never_runs_into_its_waits():
     """The GEMM-only loop bench.py measures the tensor-pipe ceiling with paces itself through two alternating
     mbarriers (one barrier per batch in flight: a barrier that completes two phases before its waiter looks reads as

@@ -321,6 +321,19 @@ def test_grids_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, Sq, Skv, d, kw)
     _check(prefill_vs_oracle(B, H, Hkv, Sq, Skv, d, seed=61, **kw))
 
 
+@pytest.mark.parametrize("B,H,Hkv,Sq,Skv,d,kw", [
+    (1, 4, 2, 130, 513, 128, dict(causal=True, q_pos0=383)),      # one item per CTA, five key tiles, the last of one key
+    (2, 59, 59, 260, 260, 128, dict(causal=True)),                # three items of 1, 2, 3 key tiles per head, 354 in all: a CTA's items start on either group
+    (1, 350, 7, 40, 100, 64, dict(causal=False)),                 # items of one key tile one after the other
+    (1, 88, 8, 390, 390, 64, dict(causal=True, q_pos0=-130)),     # items without a key tile between others
+    (1, 58, 2, 700, 700, 128, dict(causal=True, window=150)),     # windows: masks at both ends of an item's key tiles
+    (1, 80, 8, 500, 500, 128, dict(causal=True, softcap=5.0)),    # the mask in registers
+    (1, 16, 4, 1100, 1100, 128, dict(causal=True))])
+def test_query_tiles_one_after_the_other_with_key_tiles_in_turn(B, H, Hkv, Sq, Skv, d, kw):
+    """Calls of few query tiles: a CTA has one at a time, its softmax groups take the key tiles in turn."""
+    _check(prefill_vs_oracle(B, H, Hkv, Sq, Skv, d, seed=63, **kw))
+
+
 @pytest.mark.parametrize("fmt", [rk.E4M3, rk.E5M2, rk.E2M3, rk.E3M2, rk.E2M1])
 @pytest.mark.parametrize("S,d", [(31, 64), (129, 64), (333, 128), (160, 256)])
 def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
