@@ -161,6 +161,10 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
   float m_run = NEG_INF;   // running maximum at this thread's last tile, log2 domain (score * log2 e)
   float l_run = 0.0f;      // this thread's share of the row sum, relative to it
   bool ok = true;
+  // A wait for something that is there takes some 300 cycles where the scheduler's other softmax warps have exponentials queued, and a tile had four of them
+  // in a row, so what it needs is asked for ahead, without blocking, and waited for only where the answer was no: 16 heads of 8192 379 -> 369 us, capped
+  // 443 -> 436.  (O in two halves of 128 columns, each rescaled under the P V of the other: 396 and 466; the issuer, alone on its warp, then sets the pace.)
+  bool s_ready = false;
   int fail = 0;            // which wait gave up
 
   // Tiles n_low .. n_high-1 need no mask for any row of this query tile: all 128 keys inside S_kv, the tile's last key not beyond the first
@@ -181,11 +185,19 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     perturb<DUMP>(p, kPerturbGroup0 + grp, j);
     if (part == 1) perturb<DUMP>(p, kPerturbUpper256, j);
     if (stops<DUMP>(p, kPerturbGroup0 + grp, j)) { fail = 101; return false; }
-    if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.s_full[grp], (t >> 1) & 1, abort_flag))) { fail = 101; return false; }
+    if (!__all_sync(0xffffffffu, s_ready) && !__all_sync(0xffffffffu, mbar_wait_short(&bars.s_full[grp], (t >> 1) & 1, abort_flag))) { fail = 101; return false; }
     tc_fence_after();
     float s[64];
     tmem_ld32(tmem_base + lane_addr + kColS + part * 64, reinterpret_cast<uint32_t*>(s));
     tmem_ld32(tmem_base + lane_addr + kColS + part * 64 + 32, reinterpret_cast<uint32_t*>(s) + 32);
+    // Asked for here and used further down: the maxima of the tile before (the other group has left them half a tile ago), and whether the P buffer is free.
+    bool last_max = true, p_free = true;
+    float m_last = NEG_INF;
+    if (j > 0) {
+      last_max = mbar_test_wait(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1);
+      m_last = fmaxf(ld_shared_f32(&xchg[((t - 1) & 3) * 256]), ld_shared_f32(&xchg[((t - 1) & 3) * 256 + 128]));
+    }
+    if (t >= 2) p_free = mbar_test_wait(&bars.pv_done[grp], ((t - 2) >> 1) & 1);
     tc_wait_ld();
     tc_fence_before();
     __syncwarp();
@@ -230,11 +242,11 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     xchg[((t & 3) * 2 + part) * 128] = tmax;
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars.row_bar[(t & 3) * 4 + quad]);
-    float m_prev = m_run;                                     // running maximum before this tile: the other group's last tile counts too
-    if (j > 0) {
+    if (!__all_sync(0xffffffffu, last_max)) {
       if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag))) { fail = 104; return false; }
-      m_prev = fmax3(m_prev, xchg[((t - 1) & 3) * 256], xchg[((t - 1) & 3) * 256 + 128]);
+      m_last = fmaxf(xchg[((t - 1) & 3) * 256], xchg[((t - 1) & 3) * 256 + 128]);
     }
+    const float m_prev = fmaxf(m_run, m_last);                // running maximum before this tile: the other group's last tile counts too
     if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.row_bar[(t & 3) * 4 + quad], (t >> 2) & 1, abort_flag))) { fail = 106; return false; }
     tmax = fmaxf(tmax, xchg[((t & 3) * 2 + (part ^ 1)) * 128]);
     const float m_new = fmaxf(m_prev, tmax);
@@ -246,7 +258,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     const float corr = (m_prev == NEG_INF) ? 1.0f : ex2_approx(m_prev - m_new);       // of O
     const float l_corr = (m_run == NEG_INF) ? 1.0f : ex2_approx(m_run - m_new);       // of this thread's share of the sum
     m_run = m_new;
-    if (t >= 2 && !__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp], ((t - 2) >> 1) & 1, abort_flag))) { fail = 107; return false; }   // P buffer free
+    if (!__all_sync(0xffffffffu, p_free) && !__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp], ((t - 2) >> 1) & 1, abort_flag))) { fail = 107; return false; }
 
     // ---- p = 2^(x - m), row sum from the unquantised p, requant per 32-key block ---------------------
     // y = p * 2^(7-sc) has exponent field E - se + 7 = the E4M3 exponent field and keeps the mantissa, so the truncated code is y's
@@ -254,6 +266,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     // is (a block whose maximum lies below 2^-120 needs no other path: its non-zero elements all lie within 2^6 of that maximum).
     uint8_t* p_tile = smem + L::p_off + grp * kTileBytes + row * 128;
     uint64_t lsA = 0ull, lsB = 0ull;
+    bool pv_there = false;
     uint32_t scale_pair = 0;
     uint64_t fmul2[2];
 #pragma unroll
@@ -296,6 +309,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
         if (g == 0) exp4(1, q * 4);
         w[q] = requant4(g, q * 4);
       }
+      if (g == 0) pv_there = t > 0 && mbar_test_wait(&bars.pv_done[grp ^ 1], ((t - 1) >> 1) & 1);
       const int c0 = (4 * part + 2 * g) ^ (row & 7), c1 = (4 * part + 2 * g + 1) ^ (row & 7);     // 128-byte swizzle
       *reinterpret_cast<uint4*>(p_tile + c0 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4*>(p_tile + c1 * 16) = make_uint4(w[4], w[5], w[6], w[7]);
@@ -321,7 +335,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
 
     // ---- rescale this thread's half of the row's O in TMEM once the other group's P V has landed ----------------------
     if (t > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp ^ 1], ((t - 1) >> 1) & 1, abort_flag))) { fail = 102; return false; }
+      if (!__all_sync(0xffffffffu, pv_there) && !__all_sync(0xffffffffu, mbar_wait_short(&bars.pv_done[grp ^ 1], ((t - 1) >> 1) & 1, abort_flag))) { fail = 102; return false; }
       tc_fence_after();
       if (j == 0) {                                           // O of the item before this one: its last P V ran under this tile's softmax
         if (!write_out_rows<DCH, KV_STAGES, DUMP>(p, smem, bars, tmem_base, abort_flag, state)) { fail = 105; return false; }
@@ -339,6 +353,7 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
         tc_wait_st();
       }
     }
+    s_ready = j + 2 < n_tiles && mbar_test_wait(&bars.s_full[grp], ((t + 2) >> 1) & 1);      // used at the top of the group's next tile
     fence_proxy_async_smem();   // make the st.shared P tile + scales visible to the tensor-core (async) proxy
     tc_fence_before();
     __syncwarp();

@@ -195,6 +195,8 @@ RK_DEVINL uint32_t pack_u8x2(uint32_t hi, uint32_t lo, uint32_t c) {
   uint32_t d; asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(c)); return d;
 }
 
+RK_DEVINL float ld_shared_f32(const float* p) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)) : "memory"); return v; }
+
 #ifdef RK_X_STAMPS
 // Timeline stamps (measurement builds of the d <= 128 kernel only): clock64 of chosen events of one CTA, written into the dump buffer, by role and key
 // tile of an item.  A CTA that takes several items leaves those of the last one that had the tile.

@@ -193,8 +193,6 @@ RK_DEVINL uint32_t exponentiate_and_requantize(float (&s)[128], const float (&bm
   return scale_word;
 }
 
-RK_DEVINL float ld_shared_f32(const float* p) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)) : "memory"); return v; }
-
 // The tiles of one item that fall to this group; t0: the CTA's key tiles of earlier items.
 template <bool SOFTCAP, bool DUMP>
 __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p, uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
