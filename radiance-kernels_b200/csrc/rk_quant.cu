@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(128) rope_quantize_rows_kernel(const float* __
 // bytes) gives eight lanes reading 16 bytes of their own rows eight different bank groups.  When the chains are done all
 // warps normalize and quantize; the input then comes from L2 (DRAM reads it once).  Over the whole kernel 53 % of the issue
 // slots and 22 % of DRAM's rate are used: the two phases of a CTA run one after the other, and neither fills the machine.
-// 8192 x 4096 bf16: 1362 us with one warp per 32 rows doing both passes from 4-byte shared-memory reads, now 38.5 us.
+// 8192 x 4096 bf16: 1362 us with one warp per 32 rows doing both passes from 4-byte shared-memory reads, 38.5 us this way, 33.4 by bulk copies (below).
 namespace rms {
 constexpr int kThreads = 256, kWarps = kThreads / 32, kHelpers = 4, kCtasPerSm = 4;
 constexpr int kChunk = 256, kPitch = kChunk * 4 + 16, kBufs = 2;        // elements per chunk, bytes of a row of squares
@@ -339,6 +339,82 @@ template <int ID> RK_DEVINL void named_sync(int which) {
 template <int ID> RK_DEVINL void named_arrive(int which) {
   if (which) asm volatile("bar.arrive %0, %1;" ::"n"(ID + 1), "n"((1 + rms::kHelpers) * 32) : "memory");
   else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"((1 + rms::kHelpers) * 32) : "memory");
+}
+
+// The second phase of the RMSNorm kernels: y = (x rms) gamma of the CTA's rows, quantized.  rms_smem: shared memory to put the scale bytes together in,
+// room bytes of it for every row.
+template <bool BF16IN, int PIECE>
+RK_DEVINL void load_pair(Raw8<BF16IN> (&r)[2], const uint8_t* src, bool a32) {
+  if (BF16IN && PIECE == 16 && a32) {
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(r[0].w[0]), "=r"(r[0].w[1]), "=r"(r[0].w[2]), "=r"(r[0].w[3]), "=r"(r[1].w[0]), "=r"(r[1].w[1]), "=r"(r[1].w[2]), "=r"(r[1].w[3]) : "l"(src));
+  } else { r[0] = load_raw8<BF16IN, PIECE>(src); r[1] = load_raw8<BF16IN, PIECE>(src + 8 * (BF16IN ? 2 : 4)); }
+}
+template <int FMT, bool BF16IN, bool UNIT, int PIECE, int kThreads>
+RK_DEVINL void rmsnorm_rows(const uint8_t* __restrict__ xr, int64_t row0, int n_rows, int K, const float* __restrict__ gamma, const float* rms_row,
+                            uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, uint8_t* rms_smem, int room) {
+  constexpr int kElem = BF16IN ? 2 : 4, kWarps = kThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row_bytes = (int64_t)K * kElem;
+  // ---- normalize and quantize: a warp keeps 512 columns (16 per lane, 2 lanes per block; gamma in registers) and walks
+  // the rows, the load of one more row in flight; with fewer column units than warps several warps share one ------------
+  // (Scale bytes meet in shared memory first: a byte store per 32 elements cost a fifth of this phase.)
+  const bool stage_scales = K / 32 <= room;                   // they fit where the squares were
+  const bool a32 = (reinterpret_cast<uintptr_t>(xr) & 31) == 0;
+  const int per_row = (K + 511) / 512, parts = max(1, kWarps / per_row);
+  const int part = warp / per_row;
+  auto quantize_rows = [&](auto cold_tag) -> bool {
+    constexpr bool COLD = decltype(cold_tag)::value;
+    bool finite = true;
+    if (part >= parts) return finite;
+    for (int u = warp - part * per_row; u < per_row; u += kWarps) {
+      const int col = u * 512 + lane * 16;
+      if (col >= K) continue;                                           // whole 2-lane groups: K % 32 == 0
+      const int64_t src_step = parts * row_bytes, dst_step = (int64_t)parts * K;
+      const int sc_step = parts * (K / 32);
+      const uint8_t* src = xr + part * row_bytes + (int64_t)col * kElem;
+      uint8_t* dst = codes + (row0 + part) * K + col;
+      uint8_t* sdst = (stage_scales ? rms_smem : scales + row0 * (K / 32)) + part * (K / 32) + col / 32;
+      float g[2][8];
+      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col)), g[0]);
+      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col + 8)), g[1]);
+            Raw8<BF16IN> raw[2];
+      if (part < n_rows) load_pair<BF16IN, PIECE>(raw, src, a32);
+      src += src_step;
+#pragma unroll 1
+      for (int r = part; r < n_rows; r += parts) {
+        const float rms = rms_row[r];
+        float v[2][8];
+        widen8<BF16IN>(raw[0], v[0]);
+        widen8<BF16IN>(raw[1], v[1]);
+        if (r + parts < n_rows) load_pair<BF16IN, PIECE>(raw, src, a32);
+        src += src_step;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[h][j] = __fmul_rn(__fmul_rn(v[h][j], rms), g[h][j]);
+        uint32_t scode;
+        uint2 w[2];
+        finite &= quantize_lanes<FMT, UNIT, 2, COLD>(v, lane, w, scode);
+        __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0].x, w[0].y, w[1].x, w[1].y));
+        if ((lane & 1) == 0) *sdst = (uint8_t)scode;
+        dst += dst_step;
+        sdst += sc_step;
+      }
+    }
+    return finite;
+  };
+  if (__syncthreads_or(!quantize_rows(std::false_type{}))) quantize_rows(std::true_type{});
+  if (stage_scales) {
+    __syncthreads();
+    const int n = n_rows * (K / 32);                                    // contiguous in memory, as the CTA's rows are
+    uint8_t* out = scales + row0 * (K / 32);
+    if ((reinterpret_cast<uintptr_t>(out) & 3) == 0 && (n & 3) == 0) {
+      for (int i = threadIdx.x; i < n / 4; i += kThreads) reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(rms_smem)[i];
+    } else {
+      for (int i = threadIdx.x; i < n; i += kThreads) out[i] = rms_smem[i];
+    }
+  }
 }
 
 // PIECE: bytes of one global load: 16, or 4 where x or gamma is not 16-byte aligned.
@@ -454,74 +530,106 @@ rmsnorm_quantize_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int 
   }
   __syncthreads();
 
-  // ---- normalize and quantize: a warp keeps 512 columns (16 per lane, 2 lanes per block; gamma in registers) and walks
-  // the rows, the loads of two more rows in flight; with fewer column units than warps several warps share one ------------
-  // (Scale bytes meet in shared memory first: a byte store per 32 elements cost a fifth of this phase.)
-  const bool stage_scales = K / 32 <= kBufs * kPitch;                   // they fit where the squares were
-  const int per_row = (K + 511) / 512, parts = max(1, kWarps / per_row);
-  const int part = warp / per_row;
-  auto quantize_rows = [&](auto cold_tag) -> bool {
-    constexpr bool COLD = decltype(cold_tag)::value;
-    bool finite = true;
-    if (part >= parts) return finite;
-    for (int u = warp - part * per_row; u < per_row; u += kWarps) {
-      const int col = u * 512 + lane * 16;
-      if (col >= K) continue;                                           // whole 2-lane groups: K % 32 == 0
-      const int64_t src_step = parts * row_bytes, dst_step = (int64_t)parts * K;
-      const int sc_step = parts * (K / 32);
-      const uint8_t* src = xr + part * row_bytes + (int64_t)col * kElem;
-      uint8_t* dst = codes + (row0 + part) * K + col;
-      uint8_t* sdst = (stage_scales ? rms_smem : scales + row0 * (K / 32)) + part * (K / 32) + col / 32;
-      float g[2][8];
-      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col)), g[0]);
-      widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col + 8)), g[1]);
-      constexpr int kAhead = COLD || !BF16IN ? 1 : 2;
-      Raw8<BF16IN> raw[kAhead][2];
-#pragma unroll
-      for (int a = 0; a < kAhead; ++a) {
-        if (part + a * parts < n_rows) { raw[a][0] = load_raw8<BF16IN, PIECE>(src); raw[a][1] = load_raw8<BF16IN, PIECE>(src + 8 * kElem); }
-        src += src_step;
-      }
+  rmsnorm_rows<FMT, BF16IN, UNIT, PIECE, kThreads>(xr, row0, n_rows, K, gamma, rms_row, codes, scales, rms_smem, kBufs * kPitch);
+}
+
+// The same for bf16 rows, which come by bulk copies, a warp's lanes each asking for one row's next 1024 bytes; the chain warp, up to 32 rows of it in lanes,
+// squares what it reads itself, and no other warp has anything to do with the rows until the chains are done.  A chain step takes 6 cycles (4.3 the addition
+// alone; squares and additions are in one instruction stream; fused multiply-adds, exact but for squares below 2^-133, 5.1), against 6.1 with one row and 10
+// with 8192 of them staged through other warps' registers and shared memory as squares, two barriers per 256 elements.
+// 8192 x 4096: 37.7 -> 33.4 us, about half of it the chains, half the quantization from L2 (67 MB in, 35 MB out).  The latter with one 32-byte load per
+// lane and row, one row ahead: two rows ahead 37.2, 16-byte loads two rows ahead 34.0.  Four CTAs of 256 threads 38.8, one of 1024 49.8.
+namespace rmb {
+constexpr int kThreads = 512, kCtasPerSm = 2, kMaxRows = 32, kStages = 3, kPieceBytes = 1024, kPitch = kPieceBytes + 16;      // pitch: eight lanes, eight bank groups
+}  // namespace rmb
+template <int FMT, bool UNIT>
+__global__ void __launch_bounds__(rmb::kThreads, rmb::kCtasPerSm)
+rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int rows_per_cta, const float* __restrict__ gamma,
+                             float eps, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status) {
+  using namespace rmb;
+  extern __shared__ __align__(16) uint8_t rmb_smem[];                   // [kStages][n_rows][kPitch]
+  __shared__ float rms_row[kMaxRows];
+  __shared__ uint64_t full[kStages], empty[kStages];
+  constexpr int kElem = 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kStages) { mbar_init(&full[threadIdx.x], 1); mbar_init(&empty[threadIdx.x], 1); }
+  fence_barrier_init();
+  __syncthreads();
+  grid_dependency_wait();
+  grid_dependents_launch();
+  const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
+  const int n_rows = (int)min((int64_t)rows_per_cta, rows - row0);
+  const int64_t row_bytes = (int64_t)K * kElem;
+  const uint8_t* xr = x + row0 * row_bytes;
+  const int n_pieces = (int)((row_bytes + kPieceBytes - 1) / kPieceBytes), stage_bytes = n_rows * kPitch;
+  // the chains of the CTAs of an SM on schedulers of their own: blocks go to the SMs in rounds of gridDim / kCtasPerSm
+  const int chain_warp = (int)(blockIdx.x / ((gridDim.x + kCtasPerSm - 1) / kCtasPerSm)) % kCtasPerSm;
+  bool ok = true;
+  auto wait = [&](uint64_t* bar, int use) -> bool {                     // bounded: about two seconds
 #pragma unroll 1
-      for (int r0 = part; r0 < n_rows; r0 += kAhead * parts) {
+    for (int it = 0; it < 1 << 20; ++it)
+      if (mbar_try_wait<2000>(bar, use & 1)) return true;
+    return false;
+  };
+  if (warp == chain_warp) {
+    float ss = 0.0f;
+    for (int c = 0; c < n_pieces && ok; ++c) {
+      const int st = c % kStages;
+      ok = __all_sync(0xffffffffu, wait(&full[st], c / kStages));
+      if (!ok) break;
+      if (lane < n_rows) {
+        const uint4* src = reinterpret_cast<const uint4*>(rmb_smem + st * stage_bytes + lane * kPitch);
+        const int n16 = (int)min((int64_t)kPieceBytes, row_bytes - (int64_t)c * kPieceBytes) / 16;      // a multiple of 4
+        constexpr int kSq = 16 / kElem;                                 // elements of 16 bytes
+        auto square = [&](const uint4& q, float (&d)[kSq]) {
+          const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int a = 0; a < kAhead; ++a) {
-          const int r = r0 + a * parts;
-          if (r < n_rows) {
-            const float rms = rms_row[r];
-            float v[2][8];
-            widen8<BF16IN>(raw[a][0], v[0]);
-            widen8<BF16IN>(raw[a][1], v[1]);
-            if (r + kAhead * parts < n_rows) { raw[a][0] = load_raw8<BF16IN, PIECE>(src); raw[a][1] = load_raw8<BF16IN, PIECE>(src + 8 * kElem); }
-            src += src_step;
+          for (int j = 0; j < 4; ++j) {
+            const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xFFFF0000u);
+            d[2 * j] = __fmul_rn(lo, lo);
+            d[2 * j + 1] = __fmul_rn(hi, hi);
+          }
+        };
+        auto chain = [&](const float (&d)[kSq]) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+          for (int j = 0; j < kSq; ++j) ss = __fadd_rn(ss, d[j]);
+        };
+        uint4 q[4];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) v[h][j] = __fmul_rn(__fmul_rn(v[h][j], rms), g[h][j]);
-            uint32_t scode;
-            uint2 w[2];
-            finite &= quantize_lanes<FMT, UNIT, 2, COLD>(v, lane, w, scode);
-            __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0].x, w[0].y, w[1].x, w[1].y));
-            if ((lane & 1) == 0) *sdst = (uint8_t)scode;
-            dst += dst_step;
-            sdst += sc_step;
+        for (int k = 0; k < 4; ++k) q[k] = src[k];
+        float sq[2][kSq];
+        square(q[0], sq[0]);
+#pragma unroll 1
+        for (int i = 0; i < n16; i += 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {                                 // squares a piece of 16 bytes ahead, loads four
+            if (i + k + 4 < n16) q[k] = src[i + k + 4];
+            square(q[(k + 1) & 3], sq[(k + 1) & 1]);
+            chain(sq[k & 1]);
           }
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
     }
-    return finite;
-  };
-  if (__syncthreads_or(!quantize_rows(std::false_type{}))) quantize_rows(std::true_type{});
-  if (stage_scales) {
-    __syncthreads();
-    const int n = n_rows * (K / 32);                                    // contiguous in memory, as the CTA's rows are
-    uint8_t* out = scales + row0 * (K / 32);
-    if ((reinterpret_cast<uintptr_t>(out) & 3) == 0 && (n & 3) == 0) {
-      for (int i = threadIdx.x; i < n / 4; i += kThreads) reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(rms_smem)[i];
-    } else {
-      for (int i = threadIdx.x; i < n; i += kThreads) out[i] = rms_smem[i];
+    if (lane < n_rows) rms_row[lane] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+  } else if (warp == kThreads / 32 - 1) {
+    for (int c = 0; c < n_pieces && ok; ++c) {
+      const int st = c % kStages;
+      if (c >= kStages) ok = __all_sync(0xffffffffu, wait(&empty[st], c / kStages - 1));
+      if (!ok) break;
+      const uint32_t bytes = (uint32_t)min((int64_t)kPieceBytes, row_bytes - (int64_t)c * kPieceBytes);
+      if (lane == 0) mbar_arrive_expect_tx(&full[st], bytes * n_rows);
+      __syncwarp();
+      if (lane < n_rows) bulk_load_1d(rmb_smem + st * stage_bytes + lane * kPitch, xr + lane * row_bytes + (int64_t)c * kPieceBytes, bytes, &full[st]);
     }
+    for (int c = max(0, n_pieces - kStages); c < n_pieces && !ok; ++c) wait(&full[c % kStages], c / kStages);      // what may be under way
   }
+  if (__syncthreads_or(!ok)) {
+    if (threadIdx.x == 0) atomicCAS(status, 0, 602);
+    return;
+  }
+  rmsnorm_rows<FMT, true, UNIT, 16, kThreads>(xr, row0, n_rows, K, gamma, rms_row, codes, scales, rmb_smem, kStages * kPitch);
 }
 
 // Append one token to a KV cache: row pos[b] of every (batch, KV head) of K and of V is quantized (blocks of 32
@@ -1246,6 +1354,29 @@ int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads
 int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const float* gamma, float eps, int fmt,
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   if (rows == 0 || K == 0) return RK_OK;
+  const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
+  // Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so: 4096 bf16 columns, 1 row 17.2 16.3, 600 rows 22.2 18.6,
+  // 8192 37.7 33.4; 12288 columns, 1500 rows 65.6 52.3; 2048 columns, 7 rows 9.9 9.8; 1024 columns, 64 rows 6.3 6.7, 9000 rows 13.5 12.1; 512 columns, 1000 rows 5.8
+  // 6.3), and not for fp32, whose 134 MB of 8192 x 4096 come from HBM twice either way (55.0 56.4; one row 17.4 20.3).
+  if (wide && bf16 && (K >= 2048 || (K >= 1024 && rows >= 4096))) {
+    int* status = device_status_word();
+    if (!status) return RK_ERR_NO_DEVICE;
+    const int64_t slots = (int64_t)num_sms() * rmb::kCtasPerSm, waves = (rows + slots * rmb::kMaxRows - 1) / (slots * rmb::kMaxRows);
+    const int per_cta = (int)((rows + slots * waves - 1) / (slots * waves));
+    const int64_t grid = (rows + per_cta - 1) / per_cta;
+    if (grid > 0x7FFFFFFF) return RK_ERR_BAD_SHAPE;
+    const int smem = rmb::kStages * per_cta * rmb::kPitch;
+#define RK_RN(UN) RK_DISPATCH_FMT(fmt, {                                                                                \
+    auto kern = rmsnorm_quantize_bulk_kernel<F, UN>;                                                                   \
+    if (smem > 48 * 1024) {                                                                                                \
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rmb::kStages * rmb::kMaxRows * rmb::kPitch); \
+      if (e != cudaSuccess) return (int)e;                                                                                 \
+    }                                                                                                                      \
+    return (int)launch_pdl(kern, dim3((unsigned)grid), dim3(rmb::kThreads), smem, st, reinterpret_cast<const uint8_t*>(x), rows, K, per_cta, gamma, eps, codes, scales, status); \
+  })
+    if (unit_scale) { RK_RN(true); } else { RK_RN(false); }
+#undef RK_RN
+  }
   // Rows per CTA: as few whole waves of resident CTAs as kMaxRows each allow, with the rows spread evenly over them (one
   // wave and 14 rows for 8192); one row per CTA below one CTA per slot, so that few rows still reach every SM.
   const int64_t slots = (int64_t)num_sms() * rms::kCtasPerSm;
@@ -1254,7 +1385,6 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
   const int64_t grid = (rows + per_cta - 1) / per_cta;
   if (grid > 0x7FFFFFFF) return RK_ERR_BAD_SHAPE;
   const int smem = rms::kBufs * per_cta * rms::kPitch;
-  const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
   const uint8_t* xb = reinterpret_cast<const uint8_t*>(x);
 #define RK_RN(BF, UN, PC) RK_DISPATCH_FMT(fmt, {                                                                            \
     auto kern = rmsnorm_quantize_kernel<F, BF, UN, PC>;                                                                    \

@@ -83,3 +83,30 @@ def test_row_groups_chunks_and_alignment(rows, K, bf16, shift, inf_gamma):
     c, s = rk.rmsnorm_mx_quantize(xt, torch.from_numpy(gamma).cuda(), 1e-5)
     assert np.array_equal(np_(s), want_s)
     assert np.array_equal(np_(c), want_c)
+
+
+@pytest.mark.parametrize("rows,K,fmt,unit", [(1, 2048, 0, False), (33, 2080, 0, False), (9473, 2048, 0, False), (4099, 1024, 0, True), (298, 4128, 3, False)])
+def test_bf16_rows_by_bulk_copy(rows, K, fmt, unit):
+    """One row and one wave of row groups and more, rows that end inside a piece of 1024 bytes, more pieces than the ring holds; rows of zeros, of values whose
+    squares are subnormal or overflow, and blocks with a NaN or an infinity."""
+    rng = np.random.default_rng(rows + K)
+    x = (rng.standard_normal((rows, K)) * np.exp2(rng.integers(-6, 7, (rows, 1)))).astype(np.float32)
+    if rows > 10:
+        x[3] = 0.0
+        x[5] *= 2.0 ** -70
+        x[7, ::3] *= 2.0 ** 62
+        x[9, K - 40] = np.inf
+        x[10, 17] = np.nan
+    gamma = (0.75 + 0.5 * rng.random(K)).astype(np.float32)
+    xt = torch.from_numpy(x).cuda().bfloat16()
+    want_c, want_s = _expect(np_(xt.float()), gamma, 1e-5, fmt, unit)
+    c, s = rk.rmsnorm_mx_quantize(xt, torch.from_numpy(gamma).cuda(), 1e-5, fmt=fmt, unit_scale=unit)
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+    assert np.array_equal(np_(s), want_s)
+    got_c = np_(c).copy()
+    if rows > 10:                                      # rows 9 and 10: inf x 0 and sums with a NaN; x86 and the GPU give such a NaN different signs, the codes keep them
+        sign = 0x80 if fmt == 0 else 0x20
+        got_c[9:11] &= ~np.uint8(sign)
+        want_c[9:11] &= ~np.uint8(sign)
+    assert np.array_equal(got_c, want_c)
