@@ -307,6 +307,102 @@ __global__ void __launch_bounds__(128) rope_quantize_rows_kernel(const float* __
   if (__syncthreads_or(!finite)) rope_rows<FMT, U, true>(x, rows, d, pos, seq_len, pos0, cos_h, sin_h, codes, scales);      // the same rows
 }
 
+// The same for large inputs with several rows per position: a CTA has a range of positions, kTileBytes of one head's rows, keeps what it needs of the caches in
+// registers and walks every gridDim.y-th head, the next one's rows on their way by a bulk copy.  HBM bound (134 MB in and 35 MB out, which stay in L2 here:
+// 21 us as the plain quantizer does it) once enough warps are there for a row's instructions: 33.5 M elements 30.7 us with two rows per thread in registers (117
+// of them, 16 warps per SM), 31.2 with the next two rows loaded ahead (96, 20 warps), 28.4 by bulk copies four deep (24 warps), 27.8 now (64 registers, 32
+// warps), 32.5 with 40 warps of 48 registers.
+namespace ropec {
+constexpr int kThreads = 128, kCtasPerSm = 8, kStages = 2, kTileBytes = kThreads * 64;      // a thread has 8 elements of either half of a row
+}  // namespace ropec
+struct RopeRing { uint8_t* data; uint64_t* full; uint32_t loads; };      // loads: so far
+template <int FMT, bool COLD>
+RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int seq_len, int pos0, const float* __restrict__ cos_h,
+                           const float* __restrict__ sin_h, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, RopeRing& ring, int* status) {
+  using namespace ropec;
+  const int half = d / 2, cpr = half / 8, lane = threadIdx.x & 31, groups = gridDim.y;
+  const int per_tile = kTileBytes / (d * 4), p0 = blockIdx.x * per_tile, n_rows = min(per_tile, seq_len - p0);
+  const int row = threadIdx.x / cpr, i0 = (threadIdx.x - row * cpr) * 8;
+  const bool live = row < n_rows;                             // (the four lanes of a block agree)
+  const uint32_t bytes = (uint32_t)n_rows * d * 4;
+  auto load = [&](int u, uint32_t n) {                        // rows of copy u, the n-th load
+    uint64_t* bar = &ring.full[n % kStages];
+    mbar_arrive_expect_tx(bar, bytes);
+    bulk_load_1d(ring.data + (n % kStages) * kTileBytes, x + ((int64_t)u * seq_len + p0) * d, bytes, bar);
+  };
+  auto wait = [&](uint32_t n) -> bool {                       // bounded: about two seconds
+#pragma unroll 1
+    for (int it = 0; it < 1 << 20; ++it)
+      if (mbar_try_wait<2000>(&ring.full[n % kStages], (n / kStages) & 1)) return true;
+    return false;
+  };
+  const int first = blockIdx.y, mine = (copies - first + groups - 1) / groups;
+  if (threadIdx.x == 0)
+    for (int k = 0; k < min(mine, kStages); ++k) load(first + k * groups, ring.loads + k);
+  float cs[8], sn[8];
+  if (live) {
+    const int64_t at = ((int64_t)pos0 + p0 + row) * half + i0;
+    const float4* cp = reinterpret_cast<const float4*>(cos_h + at);
+    const float4* sp = reinterpret_cast<const float4*>(sin_h + at);
+    const float4 c0 = __ldg(cp), c1 = __ldg(cp + 1), s0 = __ldg(sp), s1 = __ldg(sp + 1);
+    cs[0] = c0.x; cs[1] = c0.y; cs[2] = c0.z; cs[3] = c0.w; cs[4] = c1.x; cs[5] = c1.y; cs[6] = c1.z; cs[7] = c1.w;
+    sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+  }
+  bool finite = true;
+  for (int k = 0; k < mine; ++k) {
+    const uint32_t n = ring.loads + k;
+    const bool there = wait(n);
+    const float4* src = reinterpret_cast<const float4*>(ring.data + (n % kStages) * kTileBytes + (live ? row : 0) * d * 4 + i0 * 4);      // (a branch around the loads: 8.98 us instead of 8.3 for 8.4 M elements)
+    const float4 a0 = src[0], a1 = src[1], a2 = src[half / 4], a3 = src[half / 4 + 1];
+    if (__syncthreads_or(!there)) {                           // (and read by all: the place is free)
+      if (threadIdx.x == 0) {
+        atomicCAS(status, 0, 601);
+        for (int i = k + 1; i < min(mine, k + kStages); ++i) wait(ring.loads + i);      // what is under way
+      }
+      return true;
+    }
+    if (threadIdx.x == 0 && k + kStages < mine) load(first + (k + kStages) * groups, n + kStages);
+    if (live) {
+      const float lo[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const float hi[8] = {a2.x, a2.y, a2.z, a2.w, a3.x, a3.y, a3.z, a3.w};
+      float o0[1][8], o1[1][8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        o0[0][j] = __fsub_rn(__fmul_rn(lo[j], cs[j]), __fmul_rn(hi[j], sn[j]));
+        o1[0][j] = __fadd_rn(__fmul_rn(hi[j], cs[j]), __fmul_rn(lo[j], sn[j]));
+      }
+      uint2 w0[1], w1[1];
+      uint32_t sc0, sc1;
+      finite &= quantize_lanes<FMT, false, 1, COLD>(o0, lane, w0, sc0);
+      finite &= quantize_lanes<FMT, false, 1, COLD>(o1, lane, w1, sc1);
+      const int64_t r = (int64_t)(first + k * groups) * seq_len + p0 + row;
+      __stcs(reinterpret_cast<uint2*>(codes + r * d + i0), w0[0]);
+      __stcs(reinterpret_cast<uint2*>(codes + r * d + half + i0), w1[0]);
+      if ((lane & 3) == 0) {
+        scales[r * (d / 32) + i0 / 32] = (uint8_t)sc0;
+        scales[r * (d / 32) + (half + i0) / 32] = (uint8_t)sc1;
+      }
+    }
+  }
+  ring.loads += mine;
+  return finite;
+}
+template <int FMT>
+__global__ void __launch_bounds__(ropec::kThreads, ropec::kCtasPerSm)
+rope_quantize_copies_kernel(const float* __restrict__ x, int copies, int d, int seq_len, int pos0, const float* __restrict__ cos_h, const float* __restrict__ sin_h,
+                            uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status) {
+  __shared__ __align__(128) uint8_t rope_data[ropec::kStages * ropec::kTileBytes];
+  __shared__ uint64_t rope_full[ropec::kStages];
+  if (threadIdx.x < ropec::kStages) mbar_init(&rope_full[threadIdx.x], 1);
+  fence_barrier_init();
+  __syncthreads();
+  grid_dependency_wait();
+  grid_dependents_launch();
+  RopeRing ring = {rope_data, rope_full, 0};
+  const bool finite = rope_copies<FMT, false>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);
+  if (__syncthreads_or(!finite)) rope_copies<FMT, true>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);      // the same rows
+}
+
 // RMSNorm fused with the block quantizer: the prologue of the QKV projection (kernels/rmsnorm_qkv_fused), so that the
 // normalized activation never exists in HBM as fp32.  Bit-exact with the reference's fp32 path
 // (lib/golden/golden.py:203-216): the sum of squares runs in index order with every product and sum rounded on its
@@ -1425,6 +1521,18 @@ int launch_rope_quantize_rows(const float* x, int64_t rows, int d, const int32_t
                               const float* sin_h, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   const int64_t nchunks = rows * (d / 16);
   if (nchunks == 0) return RK_OK;
+  // By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (8 heads of 16384 at d = 256 28.2 29.2;
+  // chunks per SM, us, rows in registers and so: 2 768 7.2 7.6, 3 542 8.7 8.3,
+  // 5 191 12.1 11.1, 7 085 15.8 14.2, 14 170 30.7 27.8).
+  const int64_t copies = pos ? 0 : rows / seq_len;
+  const int per_tile = ropec::kTileBytes / (d * 4);
+  if (copies >= 16 && copies <= 65535 && rows % seq_len == 0 && per_tile > 0 && nchunks >= (int64_t)num_sms() * 3000 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    int* status = device_status_word();
+    if (!status) return RK_ERR_NO_DEVICE;
+    const int64_t ctas = (seq_len + per_tile - 1) / per_tile, slots = 2 * (int64_t)num_sms() * ropec::kCtasPerSm;
+    const dim3 grid((unsigned)ctas, (unsigned)std::min<int64_t>(std::max<int64_t>(1, slots / ctas), copies));
+    RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rope_quantize_copies_kernel<F>, grid, dim3(ropec::kThreads), 0, st, x, (int)copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, status));
+  }
   // two rows per thread where every position has at least two and halving the threads still leaves every SM full
   const bool two = !pos && rows % seq_len == 0 && rows / seq_len >= 2 && nchunks >= (int64_t)num_sms() * 4096;
   // one wave of the CTAs that fit an SM, so that all end together (52 us against 49 for the Q, K, V of 8192 tokens with four)

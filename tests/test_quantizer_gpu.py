@@ -327,3 +327,24 @@ def test_errors_and_types_of_the_re_blocking_entry_points():
     want, ws = rk.mx_rebase_v(codes, scales)
     got, gs = rk.mx_rebase_v(codes.view(torch.int8), scales)
     assert got.dtype == torch.int8 and torch.equal(got.view(torch.uint8), want) and torch.equal(gs, ws)
+
+
+@pytest.mark.parametrize("B,H,S,d,pos0,fmt", [(2, 8, 3500, 128, 0, rk.E4M3), (1, 17, 6700, 64, 77, rk.E4M3), (2, 9, 1601, 256, 3, rk.E3M2), (1, 19, 2000, 192, 0, rk.E2M1),
+                                              (300, 4, 47, 128, 5, rk.E4M3)])
+def test_rope_of_many_rows_per_position_equals_the_same_rows_a_few_at_a_time(B, H, S, d, pos0, fmt):
+    """Inputs of the size that goes through bulk copies, a range of positions per CTA: ranges that end inside a tile, tiles that are no whole number of rows, more and
+    fewer heads than CTAs per range, blocks with a NaN and an infinity.  Codes and scales equal those of one sequence and a few heads at a time, which are below it
+    and pinned to the reference by the test above."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    x = torch.randn(B, H, S, d, generator=g, device="cuda")
+    x[0, 1, 3, 5], x[0, 2, S - 1, d - 1] = float("nan"), float("inf")
+    assert x.numel() // 16 >= 3000 * torch.cuda.get_device_properties(0).multi_processor_count
+    ang = torch.arange(pos0 + S, device="cuda", dtype=torch.float64)[:, None] * 10000.0 ** (-torch.arange(0, d, 2, device="cuda", dtype=torch.float64) / d)[None]
+    cos, sin = ang.cos().float().contiguous(), ang.sin().float().contiguous()
+    c, s = rk.rope_mx_quantize(x, cos, sin, pos0=pos0, fmt=fmt)
+    assert rk.last_device_status() == 0
+    for b in range(0, B, 64):
+        for h in range(0, H, 2):
+            part = x[b:b + 64, h:h + 2].contiguous()
+            c1, s1 = rk.rope_mx_quantize(part, cos, sin, pos0=pos0, fmt=fmt)
+            assert torch.equal(c1, c[b:b + 64, h:h + 2]) and torch.equal(s1, s[b:b + 64, h:h + 2]), (b, h)
