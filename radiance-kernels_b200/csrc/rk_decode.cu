@@ -472,12 +472,11 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
     for (int s = 16; s > 0; s >>= 1) { total += __shfl_xor_sync(0xffffffffu, total, s); before += __shfl_xor_sync(0xffffffffu, before, s); }
     total *= p.H_kv;
     const int64_t first = (int64_t)before * p.H_kv + (int64_t)hkv * n_unit;
-    c0 = (int)(((first + 1) * main_grid - 1) / total);             // the CTA whose range holds a tile
-    n = (int)(((first + n_unit) * main_grid - 1) / total) - c0 + 1;
+    const int ranges = dtc_ranges(total, main_grid);               // none of them is empty
+    c0 = (int)(((first + 1) * ranges - 1) / total);                // the CTA whose range holds a tile
+    n = (int)(((first + n_unit) * ranges - 1) / total) - c0 + 1;
   }
   auto at = [&](int i) -> size_t { return p.nsplit > 0 ? (size_t)bh * p.nsplit + i : ((size_t)(c0 + i) * 2 + (i == 0 ? 1 : 0)) * p.grp + hg; };
-  // with fewer tiles than CTAs some ranges are empty and left nothing
-  auto none = [&](int i) { return p.nsplit == 0 && total < main_grid && dtc_first(total, c0 + i, main_grid) == dtc_first(total, c0 + i + 1, main_grid); };
   grid_dependency_wait();
   grid_dependents_launch();
   if (n == 1) return;
@@ -491,7 +490,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
       const int i = i0 + k * kCombineWarps;
       ml[k] = make_float2(NEG_INF, 0.0f);
       row[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (i < n && !none(i)) {
+      if (i < n) {
         ml[k] = __ldcg(reinterpret_cast<const float2*>(p.part_ml) + at(i));
         row[k] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at(i) * 128) + lane);
       }

@@ -418,3 +418,10 @@ def test_workspaces_sized_by_the_helpers(B, H, Hkv, L, num_splits, fmt):
     with pytest.raises(rk.RkError):
         rk.attn_decode(q, kc, vc, ks, vs, workspace=buf[:256], **kw)
     assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,L,lens", [(1, 8, 2, 20000, [90]), (1, 8, 2, 20000, [128 * 74]), (1, 8, 2, 20000, [128 * 74 + 1]), (3, 16, 2, 20000, [0, 700, 129]),
+                                            (1, 4, 1, 512, None), (1, 4, 4, 4864, None)])
+def test_fewer_key_tiles_than_ctas(B, H, Hkv, L, lens):
+    """As many ranges as there are key tiles, as many tiles as SMs (148) and two more; CTAs without a range beside them, with lengths and without."""
+    run(B, H, Hkv, L, lens=lens, seed=17 + B + L, want_lse=lens is None)
