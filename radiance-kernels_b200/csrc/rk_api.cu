@@ -602,8 +602,8 @@ RK_API int rk_debug_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile,
 }
 
 /* Test hook (not in the public header): which warp role of the prefill kernels sleeps a little at every key tile (0 = none;
- * 1, 2 = softmax of query tile A, B, of the lower and upper keys where a CTA has one query tile, at d = 256 of the two groups; 3 = correction, at
- * d = 256 the upper keys' softmax warps; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer; 7 = O on its way out).
+ * 1, 2 = softmax of query tile A, B, of the lower and upper keys where a CTA has one query tile, of the two groups where they take the key tiles
+ * in turn and at d = 256; 3 = correction, at d = 256 the upper keys' softmax warps; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer; 7 = O on its way out).
  * 100 + role: the role acts after a key tile as if its wait had run out (not 103 at d = 256, nor 107). */
 RK_API void rk_debug_set_prefill_perturb(int role) { g_prefill_perturb = role; }
 

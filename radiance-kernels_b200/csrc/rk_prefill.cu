@@ -782,22 +782,23 @@ int g_prefill_perturb = 0;
 
 // d <= 128: one query tile per CTA at a time with the softmax groups on alternate key tiles (rk_prefill1.cu), or pairs of query tiles (rk_prefill2c.cu,
 // which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1700 cycles in the former and
-// half of 3450 in the latter, which loads K and V half as often and so loses less under the power cap: it has the large grids.  Measured (us, the pairs'
+// half of 3400 in the latter, which loads K and V half as often and so loses less under the power cap: it has the large grids.  Measured (us, the pairs'
 // kernel and this one):
-//   no more query tiles than SMs: 8 / 32 heads of 512 11.1 10.5 / 13.9 13.4, 16 of 1024 18.5 17.2, 8 of 2048 27.7 24.3, 32 x 509 queries behind 3581 keys
-//     42.1 36.8.  Up to three key tiles the time is that of code run for the first time, of which the other form has less: 42 heads of 300 12.1 12.5, 128 of
-//     100 10.6 11.0.  With the cap 54.5 56.5 on the same chunk.
-//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  512 queries behind 4096 keys, 72 heads (288 tiles) 70.8 71.8,
-//     96 heads 126 100; without a mask 500 by 700 keys 40 heads 20.9 22.0; capped, 64 heads 90.7 102, 96 heads 160 143.
-//   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 40.6 24.9, 16 40.9 28.6, 23 42.3 37.8,
-//     27 43.3 43.0; 23 heads of 1024 25.9 18.1, 37 26.9 24.4, 47 27.4 27.9; 24 capped heads of 1024 31.8 22.3; 24 of 2048 with a window of 512 33.0 27.1.
+//   no more query tiles than SMs: 8 / 32 heads of 512 11.1 10.3 / 13.9 13.5, 16 of 1024 18.4 17.0, 8 of 2048 27.8 24.1, 32 x 509 queries behind 3581 keys
+//     42.1 35.6.  Up to three key tiles the time is that of code run for the first time, of which the other form has less: 42 heads of 300 12.1 12.4, 128 of
+//     100 10.7 10.9.  With the cap: 8 of 2048 34.9 33.9, but 42.5 57.1 (32 x 512 by 1536, d = 64) where the 64 keys of a half differ in tanh's form.
+//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  512 queries behind 4096 keys, 72 heads (288 tiles) 98.3 96.7,
+//     96 heads 166 137; 500 by 2000 keys without a mask, 64 heads 46.5 46.9; capped, 72 heads 135 146, 96 heads 229 206.
+//   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 40.2 24.3, 16 40.7 27.8, 23 41.5 36.4,
+//     27 42.4 41.0, 31 44.7 45.6; 23 heads of 1024 25.6 17.4, 37 26.5 22.6, 47 26.9 26.6, 56 29.2 30.1; 144 of 300 21.8 20.3; capped, with a cap of 50 and of
+//     30, 24 heads of 1024 32.5 22.0 and 69.2 38.2, 26 of 2048 65.1 56.0 and 162 134; 24 of 2048 with a window of 512 33.2 27.1.
 static bool alternate_key_tiles(const PrefillParams& p, bool cap) {
   const int64_t sms = num_sms(), heads = (int64_t)p.B * p.H, tiles = p.n_q_tiles * heads, pairs = (p.n_q_tiles + 1) / 2 * heads;
   const int item_tiles = p.window > 0 ? std::min(p.n_kv_tiles, (p.window + kBlockM - 2) / kBlockN + 2) : p.n_kv_tiles;     // at most
   if (tiles <= sms) return item_tiles > 3 && !cap;
   const bool level = p.window == 0 && (!p.causal || 2 * ((int64_t)p.q_pos0 + kBlockM) > p.S_kv);
   if (level) return 10 * ((tiles + sms - 1) / sms) < 19 * ((pairs + sms - 1) / sms);
-  return 2 * tiles <= (item_tiles > 8 ? 6 : 5) * sms;
+  return tiles <= 3 * sms;
 }
 
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,

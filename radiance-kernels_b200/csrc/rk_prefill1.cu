@@ -17,7 +17,7 @@
 // from cold instruction memory: 750 for the rescale, 250 and 300 to the issuer and back).  Without it the softmax groups would take 1 580, and alone on
 // the SM 1 320.  (The P V issued by a correction warp: 2 700, its other waits then lie in the chain.  The rescale in chunks of 64 columns: spills, 1 830.)
 // Both groups on every key tile, 64 keys each, with an exchange of row maxima (rk_prefill2c.cu, the form for one query tile per CTA): 2 250.
-// 32 heads x 509 queries behind 3581 keys 42.1 -> 36.8 us, 8 heads of 4096 70.2 -> 42.3 (pairs of query tiles), 16 of 2048 40.9 -> 28.6.
+// 32 heads x 509 queries behind 3581 keys 42.1 -> 35.6 us, 8 heads of 4096 69.5 -> 40.2 (pairs of query tiles), 16 of 2048 40.7 -> 27.8.
 //
 // As in rk_prefill2c.cu a CTA stays on its SM and takes one query tile after the other, and everything counts on from item to item.  An item costs about
 // 3 600 cycles on top of its tiles: the mask of the diagonal tile, and O's way out, for which the next item's first P V waits only until O is in registers.
@@ -238,13 +238,13 @@ __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p,
   }
 
   // the blocking forms; they return 0, or the code of the wait that gave up
-  auto wait_scores = [&](const int t) -> int { return __all_sync(0xffffffffu, mbar_wait_short(s_full, (t >> 1) & 1, abort_flag)) ? 0 : 101; };
+  auto wait_scores = [&](const int t) -> int { return __all_sync(0xffffffffu, mbar_wait_compact(s_full, (t >> 1) & 1, abort_flag)) ? 0 : 101; };
   auto wait_rest = [&](const int j) -> int {
     const int t = t0 + j;
     int code = 0;
-    if (t >= kPBufs && !mbar_wait_short(&bars[bPV + (t & 3)], ((t >> 2) - 1) & 1, abort_flag)) code = 102;
+    if (t >= kPBufs && !mbar_wait_compact(&bars[bPV + (t & 3)], ((t >> 2) - 1) & 1, abort_flag)) code = 102;
     else if (kMaxAhead && j > 0) {
-      if (!mbar_wait_short(&bars[bMX + ((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag)) code = 106;
+      if (!mbar_wait_compact(&bars[bMX + ((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag)) code = 106;
       m_run = ld_shared_f32(&row_max[((t - 1) & 3) * 128 + row]);
     }
     return __any_sync(0xffffffffu, code != 0) ? (code ? code : 102) : 0;
@@ -288,7 +288,7 @@ __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p,
     // Barrier and slot are those of t - 5 as well: that phase is over, since the P buffer of this tile was free only after the P V of tile t - 4, for which the
     // correction warps had waited for it.
     if (!kMaxAhead && j > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait_short(&bars[bMX + ((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag))) { fail = 106; return false; }
+      if (!__all_sync(0xffffffffu, mbar_wait_compact(&bars[bMX + ((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag))) { fail = 106; return false; }
       m_run = ld_shared_f32(&row_max[((t - 1) & 3) * 128 + row]);
     }
     const float m_new = fmaxf(m_run, mx * sc_mul);
@@ -489,10 +489,10 @@ __device__ __forceinline__ int correct_quadrant(const PrefillParams& p, const CU
   const float2* row_sum = reinterpret_cast<const float2*>(smem + sum_off);
   const float NEG_INF = __int_as_float(0xff800000);
   const int o_chunks = p.d / 32;
-  auto wait_max = [&]() { return __all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bMX + (st.t & 3) * 4 + quad], (st.t >> 2) & 1, abort_flag)); };
+  auto wait_max = [&]() { return __all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bMX + (st.t & 3) * 4 + quad], (st.t >> 2) & 1, abort_flag)); };
   // Always waited for, rescale or not: an arrival on the O-ready barrier then
   // implies that its previous phase has been consumed, which is what keeps the two-deep barrier from wrapping.
-  auto wait_pv = [&]() { return __all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPV + ((st.t - 1) & 3)], ((st.t - 1) >> 2) & 1, abort_flag)); };
+  auto wait_pv = [&]() { return __all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bPV + ((st.t - 1) & 3)], ((st.t - 1) >> 2) & 1, abort_flag)); };
   auto release = [&]() {                                       // the tile's P V may accumulate into O now
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars[bOR + (st.t & 1)]);
@@ -608,7 +608,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   // The next item, for every warp but the TMA producer's: 1 taken, 0 none left, -1 a wait gave up.
   uint32_t work_par = 0;
   auto next_work = [&]() -> int {
-    if (!__all_sync(0xffffffffu, mbar_wait_short(&bars[bWF], work_par, abort_flag))) return -1;
+    if (!__all_sync(0xffffffffu, mbar_wait_compact(&bars[bWF], work_par, abort_flag))) return -1;
     work_par ^= 1;
     w = *reinterpret_cast<const Work*>(smem + work_off);
     if (w.qt < 0) return 0;
@@ -633,7 +633,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         bool asked = false;                          // a request for the next item is on its way
         uint32_t kuse = 0, vuse = 0, qn = 0, block = blockIdx.x;     // rounds through the stages; items with key tiles
         auto load_k = [&](int j) -> bool {
-          if (kuse > 0 && !mbar_wait_short<true>(&bars[bKE + kst], (kuse - 1) & 1, abort_flag)) { fail = 201; return false; }
+          if (kuse > 0 && !mbar_wait_compact<true>(&bars[bKE + kst], (kuse - 1) & 1, abort_flag)) { fail = 201; return false; }
           mbar_arrive_expect_tx(&bars[bKF + kst], p.kv_tile_tx + kSfAtomBytes);
           tma_load_3d(smem + k_off + kst * kTileBytes, &tmap_k, &bars[bKF + kst], 0, (j + w.j0) * kBlockN, w.bhkv);
           bulk_load_1d(smem + sfk_off + kst * kSfAtomBytes, p.k_sf + ((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * kSfAtomBytes,
@@ -647,7 +647,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         uint32_t v_atom = 0;
         auto load_v = [&]() -> bool {
           if (v_key < 0) return true;
-          if (vuse > 0 && !mbar_wait_short<true>(&bars[bVE + vst], (vuse - 1) & 1, abort_flag)) { fail = 202; return false; }
+          if (vuse > 0 && !mbar_wait_compact<true>(&bars[bVE + vst], (vuse - 1) & 1, abort_flag)) { fail = 202; return false; }
           mbar_arrive_expect_tx(&bars[bVF + vst], p.kv_tile_tx + kSfAtomBytes);
           tma_load_3d(smem + v_off + vst * kTileBytes, &tmap_v, &bars[bVF + vst], p.v_transposed ? v_key : 0, p.v_transposed ? 0 : v_key, v_bhkv);   // transposed V: [d][keys]
           bulk_load_1d(smem + sfv_off + vst * kSfAtomBytes, p.v_sf + (size_t)v_atom * kSfAtomBytes, kSfAtomBytes, &bars[bVF + vst]);
@@ -658,7 +658,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (uint32_t k = 0;; ++k) {
           w = decode(block);
           // everybody has read the last item: this one takes its place
-          if (k > 0 && !mbar_wait_short<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
+          if (k > 0 && !mbar_wait_compact<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
           *reinterpret_cast<Work*>(smem + work_off) = w;
           mbar_arrive(&bars[bWF]);
           if (k == 0) {
@@ -667,7 +667,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           }
           if (w.n_tiles > 0) {
             const int qb = qn & 1;
-            if (qn >= 2 && !mbar_wait_short<true>(&bars[bQE + qb], ((qn >> 1) - 1) & 1, abort_flag)) { fail = 203; break; }
+            if (qn >= 2 && !mbar_wait_compact<true>(&bars[bQE + qb], ((qn >> 1) - 1) & 1, abort_flag)) { fail = 203; break; }
             ++qn;
             mbar_arrive_expect_tx(&bars[bQ + qb], p.q_tile_tx + kSfAtomBytes);
             tma_load_3d(smem + q_off + qb * kTileBytes, &tmap_q, &bars[bQ + qb], 0, w.qt * kBlockM, w.bh);
@@ -696,7 +696,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (fail || stopped) break;
           if (!clc_answer(smem + clc_off, block)) {
             if (!load_v()) break;
-            if (!mbar_wait_short<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
+            if (!mbar_wait_compact<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
             w.qt = -1;
             *reinterpret_cast<Work*>(smem + work_off) = w;
             mbar_arrive(&bars[bWF]);
@@ -743,7 +743,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const int nt = warp_uniform(w.n_tiles);
         const int qb = qn & 1;
         if (nt > 0) {
-          if (!__all_sync(0xffffffffu, mbar_wait_short(&bars[bQ + qb], (qn >> 1) & 1, abort_flag))) { fail = 301; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_compact(&bars[bQ + qb], (qn >> 1) & 1, abort_flag))) { fail = 301; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfQ + qb * 4, dsfq + (uint32_t)(qb * (kSfAtomBytes >> 4)));
           ++qn;
         }
@@ -753,8 +753,8 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           perturb<DUMP>(p, kPerturbQk, j);
           if (stops<DUMP>(p, kPerturbQk, j)) { fail = 302; break; }
           if (lane == 0) RK_STAMP(2, j, 0);
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
-          if (t >= 2 && !__all_sync(0xffffffffu, mbar_wait_short(&bars[bSE + (t & 1)], ((t >> 1) - 1) & 1, abort_flag))) { fail = 305; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
+          if (t >= 2 && !__all_sync(0xffffffffu, mbar_wait_compact(&bars[bSE + (t & 1)], ((t >> 1) - 1) & 1, abort_flag))) { fail = 305; break; }
           tc_fence_after();
           if (lane == 0) RK_STAMP(2, j, 1);
           if (elect_one()) {
@@ -797,15 +797,15 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           perturb<DUMP>(p, kPerturbPv, i);
           if (stops<DUMP>(p, kPerturbPv, i)) { fail = 303; break; }
           const int pb = t & 3;
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPF + pb], (t >> 2) & 1, abort_flag))) { fail = 304; break; }      // P written
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bPF + pb], (t >> 2) & 1, abort_flag))) { fail = 304; break; }      // P written
           tc_fence_after();
           if (elect_one()) {
             tc_cp_32x128b_warpx4(tm + cSfV + st * 4, dsfv + (uint32_t)(st * (kSfAtomBytes >> 4)));
             tc_cp_32x128b_warpx4(tm + cSfP + pb * 4, dsfp + (uint32_t)(pb * (kSfAtomBytes >> 4)));
           }
           const uint64_t dvt = dv + (uint32_t)(st * (kTileBytes >> 4)), dpt = dp + (uint32_t)(pb * (kTileBytes >> 4));
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bOR + (t & 1)], (t >> 1) & 1, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's read
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bOR + (t & 1)], (t >> 1) & 1, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's read
           tc_fence_after();
           if (elect_one()) {
 #pragma unroll
@@ -835,7 +835,7 @@ prefill1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (w.n_tiles > 0) { st.out_qt = w.qt; st.out_bh = w.bh; }
     }
     if (!fail && st.t > 0) {                         // O of the last item
-      if (__all_sync(0xffffffffu, mbar_wait_short(&bars[bPV + ((st.t - 1) & 3)], ((st.t - 1) >> 2) & 1, abort_flag)))
+      if (__all_sync(0xffffffffu, mbar_wait_compact(&bars[bPV + ((st.t - 1) & 3)], ((st.t - 1) >> 2) & 1, abort_flag)))
         last_out<DUMP>(p, smem, tmem_base, st);
       else fail = 403;
     }

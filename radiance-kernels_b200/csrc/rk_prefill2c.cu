@@ -513,13 +513,13 @@ __device__ __forceinline__ int correction_quadrant(const PrefillParams& p, const
       if (j >= (g == 0 ? nt0 : nt1)) continue;
       const int t = (g == 0 ? t0 : t1) + j;                   // this group's tile, counted over all items of the CTA
       if (quad == 0 && lane == 0) RK_STAMP(3, j, g * 4 + 0);
-      if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bCF + (g * 4 + (t & 3)) * 4 + quad], (t >> 2) & 1, abort_flag))) return 401;
+      if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bCF + (g * 4 + (t & 3)) * 4 + quad], (t >> 2) & 1, abort_flag))) return 401;
       const float corr = corr_sm[(g * 4 + (t & 3)) * 128 + row];
       if (quad == 0 && lane == 0) RK_STAMP(3, j, g * 4 + 1);
       if (t > 0) {
         // Always wait for the previous P.V of this tile, rescale or not: an arrival on the O-ready barrier then
         // implies that its previous phase has been consumed, which is what keeps the two-deep barrier from wrapping.
-        if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPV + g * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort_flag))) return 402;
+        if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bPV + g * 2 + ((t - 1) & 1)], ((t - 1) >> 1) & 1, abort_flag))) return 402;
       }
       if (j == 0) {
         if (!SPLIT && t > 0) write_out_quadrant<DUMP>(p, tmap_o, smem, tmem_base, g, t, g == 0 ? out0 : out1);   // the group's item before this one
@@ -636,7 +636,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint32_t work_par = 0;
   auto next_work = [&]() -> int {
     if (SPLIT && work_par) return 0;
-    if (!__all_sync(0xffffffffu, mbar_wait_short(&bars[bWF], work_par, abort_flag))) return -1;
+    if (!__all_sync(0xffffffffu, mbar_wait_compact(&bars[bWF], work_par, abort_flag))) return -1;
     work_par ^= 1;
     w = *reinterpret_cast<const Work*>(smem + work_off);
     if (w.qp < 0) return 0;
@@ -667,7 +667,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (stops<DUMP>(p, kPerturbTma, j)) { fail = 201; break; }
             if (j == 0) {
               // everybody has read the last item: this one takes its place
-              if (k > 0 && !mbar_wait_short<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
+              if (k > 0 && !mbar_wait_compact<true>(&bars[bWE], (k - 1) & 1, abort_flag)) { fail = 502; break; }
               *reinterpret_cast<Work*>(smem + work_off) = w;
               mbar_arrive(&bars[bWF]);
               if (k == 0) {
@@ -678,7 +678,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               for (int g = 0; g < 2; ++g) {
                 if ((g == 0 ? w.nt0 : w.nt1) == 0) continue;
                 if ((q_used >> g) & 1) {             // Q K^T of the last item that had a tile in this place has finished
-                  if (!mbar_wait_short<true>(&bars[bQE + g], (q_par >> g) & 1, abort_flag)) { fail = 203; break; }
+                  if (!mbar_wait_compact<true>(&bars[bQE + g], (q_par >> g) & 1, abort_flag)) { fail = 203; break; }
                   q_par ^= 1 << g;
                 }
                 q_used |= 1 << g;
@@ -687,10 +687,10 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               if (fail) break;
             }
             if (n_all > 0) {
-              if (use > 0 && !mbar_wait_short<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
+              if (use > 0 && !mbar_wait_compact<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
               issue_kv(j, st);
               if (stopped) break;                    // O is written only where V has come
-              if (use > 0 && !mbar_wait_short<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
+              if (use > 0 && !mbar_wait_compact<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
               issue_v(j, st);
               if (++st == kStages) { st = 0; ++use; }
             }
@@ -704,7 +704,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           drain(&bars[bClc], k & 1, 503);
           if (fail) break;
           if (!clc_answer(smem + clc_off, block)) {
-            if (!mbar_wait_short<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
+            if (!mbar_wait_compact<true>(&bars[bWE], k & 1, abort_flag)) { fail = 502; break; }
             w.qp = -1;
             *reinterpret_cast<Work*>(smem + work_off) = w;
             mbar_arrive(&bars[bWF]);
@@ -754,7 +754,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           perturb<DUMP>(p, kPerturbQk, j);
           if (stops<DUMP>(p, kPerturbQk, j)) { fail = 302; break; }
           if (lane == 0) RK_STAMP(2, j, 0);
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfK + st * 4, dsfk + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dkt = dk + (uint32_t)(st * (kTileBytes >> 4));
           if (lane == 0) RK_STAMP(2, j, 1);
@@ -765,11 +765,11 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             const int n_mine = g == 0 ? nt0 : nt1;
             if (j >= n_mine) continue;
             if (j == 0) {
-              if (!__all_sync(0xffffffffu, mbar_wait_short(&bars[g == 0 ? bQ : bQB], (q_par >> g) & 1, abort_flag))) { fail = 301; break; }
+              if (!__all_sync(0xffffffffu, mbar_wait_compact(&bars[g == 0 ? bQ : bQB], (q_par >> g) & 1, abort_flag))) { fail = 301; break; }
               q_par ^= 1u << g;
               if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfQ + g * 4, dsfq + (uint32_t)(g * (kSfAtomBytes >> 4)));
             }
-            if (last_g >= 0 && !__all_sync(0xffffffffu, mbar_wait_short(&bars[bSE + last_g], last_par, abort_flag))) { fail = 305; break; }
+            if (last_g >= 0 && !__all_sync(0xffffffffu, mbar_wait_compact(&bars[bSE + last_g], last_par, abort_flag))) { fail = 305; break; }
             tc_fence_after();
             const uint64_t dqt = dq + (uint32_t)(g * (kTileBytes >> 4));
             if (elect_one()) {
@@ -810,7 +810,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         for (int i = 0; i < n_all && !fail; ++i) {
           perturb<DUMP>(p, kPerturbPv, i);
           if (stops<DUMP>(p, kPerturbPv, i)) { fail = 303; break; }
-          if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bVF + st], use_par, abort_flag))) { fail = 303; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfV + st * 4, dsfv + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dvt = dv + (uint32_t)(st * (kTileBytes >> 4));
 #pragma unroll 1
@@ -818,8 +818,8 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             if (i >= (g == 0 ? nt0 : nt1)) continue;
             const int t = (g == 0 ? t0 : t1) + i, gb = g * 2 + (t & 1);
             const uint32_t par2 = (t >> 1) & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bPF + gb], par2, abort_flag))) { fail = 304; break; }      // P written
-            if (!__all_sync(0xffffffffu, mbar_wait_short<true>(&bars[bOR + gb], par2, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's written out
+            if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bPF + gb], par2, abort_flag))) { fail = 304; break; }      // P written
+            if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bOR + gb], par2, abort_flag))) { fail = 307; break; }      // O rescaled for this tile, or the last item's written out
             tc_fence_after();
             const uint64_t dpt = dp + (uint32_t)(gb * (kTileBytes >> 4));
             if (elect_one()) {
