@@ -781,7 +781,7 @@ float* g_prefill_dbg = nullptr;   // set by rk_debug_set_prefill_dump (tests onl
 int g_prefill_perturb = 0;
 
 // d <= 128: one query tile per CTA at a time with the softmax groups on alternate key tiles (rk_prefill1.cu), or pairs of query tiles (rk_prefill2c.cu,
-// which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1700 cycles in the former and
+// which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1650 cycles in the former and
 // half of 3400 in the latter, which loads K and V half as often and so loses less under the power cap: it has the large grids.  Measured (us, the pairs'
 // kernel and this one):
 //   no more query tiles than SMs: 8 / 32 heads of 512 11.1 10.3 / 13.9 13.5, 16 of 1024 18.4 17.0, 8 of 2048 27.8 24.1, 32 x 509 queries behind 3581 keys

@@ -26,7 +26,8 @@
 // on while group B, one tile longer under a causal mask, finishes, and the correction warps write an item's O out while the softmax
 // warps are in their next tile.  With a CTA per pair an item of 16 tiles cost 17 000 cycles on top of them (start 4400, first loads,
 // a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
-// 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.
+// 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.  Since the waits outside the softmax
+// warps are short in code (mbar_wait_compact), 512 and 1742; 538 and 1855.
 //
 // SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle and whose items are too short for rk_prefill1.cu, or capped.  A key
 // tile's time is then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
