@@ -27,7 +27,7 @@
 // warps are in their next tile.  With a CTA per pair an item of 16 tiles cost 17 000 cycles on top of them (start 4400, first loads,
 // a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
 // 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.  Since the waits outside the softmax
-// warps are short in code (mbar_wait_compact), 512 and 1742; 538 and 1855.
+// warps are short in code (mbar_wait_compact) and the registers split as below, 536 and 1851 under the cap.
 //
 // SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle and whose items are too short for rk_prefill1.cu, or capped.  A key
 // tile's time is then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
@@ -45,9 +45,12 @@ constexpr int kThreads = 512;
 constexpr int kWarpCorr = 8, kWarpTma = 12, kWarpQk = 13, kWarpPv = 14;
 // Registers of a softmax, correction and issuer thread: 128 * (2 * softmax + correction + issuer) = 65536.  Measured (8 x 16 heads of
 // 4096, full clock): softmax 168 515 us, 176 518, 184 521, 192 523, 200 550 (no spills up to 192; what changes is the order ptxas gives the tile body).
-// 176 and not 168 for the capped form, which is 1 % slower with 168 (8 x 16 heads of 4096 791 us and 784, 4 x 32 / 8 of 8192 2659 and 2629); without
-// the cap 168 is 0.5 % faster (555.1 and 558.1, 1885 and 1893 under the power cap).
-constexpr uint32_t kRegSoftmax = 176, kRegCorr = 88, kRegIssue = 72;
+// With the short waits, 4 x 32 / 8 of 8192 under the power cap: 168 / 104 / 72 1858 us, 168 / 96 / 80 1860, 168 / 88 / 88 1857, 176 / 88 / 72 1866, 176 / 80 / 80 1868;
+// 32 / 8 heads of 8192 445.1, 446.4, 445.2, 448.0, 448.2.  The capped form is 1 % slower with 168 (2 x 16 heads of 4096 213.6 and 216.0; 8 x 16 784 and 791).
+template <bool SOFTCAP> constexpr uint32_t kRegSoftmax = SOFTCAP ? 176 : 168;
+template <bool SOFTCAP> constexpr uint32_t kRegCorr = SOFTCAP ? 88 : 104;
+constexpr uint32_t kRegIssue = 72;
+static_assert(2 * kRegSoftmax<false> + kRegCorr<false> + kRegIssue == 512 && 2 * kRegSoftmax<true> + kRegCorr<true> + kRegIssue == 512);
 constexpr uint32_t kRegSoftmaxSplit = 176, kRegCorrSplit = 80, kRegIssueSplit = 80;      // 509 queries behind 3581 keys: softmax 144 43.9 us, 160 44.4, 176 43.5, 192 43.6
 // TMEM columns
 constexpr uint32_t cS = 0, cO = 128 /* + g*128 */, cSfQ = 384 /* + g*4 */, cSfK = 392 /* + st*4 */,
@@ -845,7 +848,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
     if (fail) give_up(abort_flag, p.status, fail);
   } else if (warp >= kWarpCorr) {
-    reg_dec<SPLIT ? kRegCorrSplit : kRegCorr>();
+    reg_dec<SPLIT ? kRegCorrSplit : kRegCorr<SOFTCAP>>();
     int t0 = 0, t1 = 0, fail = 0;                    // t0, t1: the groups' key tiles of earlier items
     Pending out0{0, 0}, out1{0, 0};
     for (;;) {
@@ -862,7 +865,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     if (!SPLIT && lane == 0) bulk_wait_all();
     if (fail) give_up(abort_flag, p.status, fail);
   } else {
-    reg_inc<SPLIT ? kRegSoftmaxSplit : kRegSoftmax>();
+    reg_inc<SPLIT ? kRegSoftmaxSplit : kRegSoftmax<SOFTCAP>>();
     if (threadIdx.x == 0) RK_STAMP_RAW(5);
     const int grp = warp >> 2;
     int t0 = 0;                                      // this group's key tiles of earlier items
