@@ -794,12 +794,16 @@ int g_prefill_perturb = 0;
 //     30, 24 heads of 1024 32.5 22.0 and 69.2 38.2, 26 of 2048 65.1 56.0 and 162 134; 24 of 2048 with a window of 512 33.2 27.1.
 static bool alternate_key_tiles(const PrefillParams& p, bool cap) {
   const int64_t sms = num_sms(), heads = (int64_t)p.B * p.H, tiles = p.n_q_tiles * heads, pairs = (p.n_q_tiles + 1) / 2 * heads;
-  const int item_tiles = p.window > 0 ? std::min(p.n_kv_tiles, (p.window + kBlockM - 2) / kBlockN + 2) : p.n_kv_tiles;     // at most
+  const int item_tiles = p.window > 0 ? (int)std::min<int64_t>(p.n_kv_tiles, ((int64_t)p.window + kBlockM - 2) / kBlockN + 2) : p.n_kv_tiles;     // at most
   if (tiles <= sms) return item_tiles > 3 && !cap;
   const bool level = p.window == 0 && (!p.causal || 2 * ((int64_t)p.q_pos0 + kBlockM) > p.S_kv);
   if (level) return 10 * ((tiles + sms - 1) / sms) < 19 * ((pairs + sms - 1) / sms);
   return tiles <= 3 * sms;
 }
+
+// A window that reaches beyond the first key for every row masks nothing.  Any other is at most the last row's position, so that the kernels' position - window
+// - key stays within 32 bits (a caller's "no limit", a window near 2^31, wrapped and masked keys that the row sees).
+static int effective_window(const rk_prefill_args& a) { return a.window > (int64_t)a.q_pos0 + a.S_q - 1 ? 0 : a.window; }
 
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st) {
@@ -834,7 +838,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
   }
   p.n_q_tiles = (a.S_q + kBlockM - 1) / kBlockM;
   p.n_kv_tiles = (a.S_kv + kBlockN - 1) / kBlockN;
-  p.q_pos0 = a.q_pos0; p.causal = a.causal; p.window = a.window;
+  p.q_pos0 = a.q_pos0; p.causal = a.causal; p.window = effective_window(a);
   p.v_transposed = kv6 ? 1 : 0;
   p.perturb = g_prefill_perturb;
   p.q_tile_tx = q6 ? kTileBytes * qbits / 8 : kTileBytes;

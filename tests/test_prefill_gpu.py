@@ -441,3 +441,19 @@ def test_o_at_a_16_byte_boundary(H, Sq, d):
     assert out.data_ptr() % 32 == 16
     rk.attn_prefill(q, k, v, qs, ks, vs, causal=True, out=out)
     assert torch.equal(out, want) and (flat[:8] == 7.0).all() and (flat[-8:] == 7.0).all()
+
+
+@pytest.mark.parametrize("H,Sq,Skv,d,causal,q_pos0", [(2, 300, 300, 128, False, 0), (160, 200, 333, 64, False, -130), (200, 520, 700, 128, False, -130),
+                                                     (2, 300, 300, 256, False, -130), (2, 300, 300, 128, True, 0)])
+@pytest.mark.parametrize("beyond", [True, False])
+def test_windows_that_mask_nothing_or_little(H, Sq, Skv, d, causal, q_pos0, beyond):
+    """A window near 2^31, a caller's "no limit", masks no key: the bits of a call without one.  The largest window that masks one, the first key for the last
+    row alone: the bits of that call in every other row."""
+    qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, Sq, Skv, d, seed=34))
+    kw = dict(causal=causal, q_pos0=q_pos0)
+    want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+    last = q_pos0 + Sq - 1
+    for window in ((2 ** 31 - 1, 2 ** 31 - 100, last + 1) if beyond else (last,)):
+        got = rk.attn_prefill(qc, kc, vc, qs, ks, vs, window=window, **kw)
+        assert torch.equal(got[:, :, :-1], want[:, :, :-1]) and torch.equal(got[:, :, -1], want[:, :, -1]) == beyond, window
+    assert rk.last_device_status() == 0
