@@ -1517,16 +1517,24 @@ int launch_quantize_keys(const float* x, int64_t batch, int64_t rows, int64_t co
   return RK_OK;
 }
 
+// By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (8 heads of 16384 at d = 256 28.2 29.2;
+// chunks per SM, us, rows in registers and so: 2 768 7.2 7.6, 3 542 8.7 8.3, 5 191 12.1 11.1, 7 085 15.8 14.2, 14 170 30.7 27.8: one call behind another on the
+// same buffers; with nothing of them in L2 22.5 22.5 and 36.9 36.8).  A CTA's tile is a range of positions of one sequence, and the threads of the rows that the
+// last one lacks are idle: it pays where the tiles are three quarters full (some 8 M elements at d = 128, 16 rows a tile; sequences of 1 7.2 41.7, 4 8.3 14.0,
+// 8 8.3 8.9, 17 15.6 18.3, 33 15.0 15.3, 24 11.3 11.0, 49 11.8 11.2, 15 13.9 11.5).
+bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms) {
+  const int64_t copies = rows / seq_len, per_tile = ropec::kTileBytes / (d * 4);
+  if (copies < 16 || copies > 65535 || rows % seq_len != 0 || per_tile == 0 || rows * (d / 16) < sms * 3000) return false;
+  return 4 * seq_len >= 3 * ((seq_len + per_tile - 1) / per_tile) * per_tile;
+}
+
 int launch_rope_quantize_rows(const float* x, int64_t rows, int d, const int32_t* pos, int seq_len, int pos0, const float* cos_h,
                               const float* sin_h, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   const int64_t nchunks = rows * (d / 16);
   if (nchunks == 0) return RK_OK;
-  // By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (8 heads of 16384 at d = 256 28.2 29.2;
-  // chunks per SM, us, rows in registers and so: 2 768 7.2 7.6, 3 542 8.7 8.3,
-  // 5 191 12.1 11.1, 7 085 15.8 14.2, 14 170 30.7 27.8).
-  const int64_t copies = pos ? 0 : rows / seq_len;
-  const int per_tile = ropec::kTileBytes / (d * 4);
-  if (copies >= 16 && copies <= 65535 && rows % seq_len == 0 && per_tile > 0 && nchunks >= (int64_t)num_sms() * 3000 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+  if (!pos && rope_by_copies(rows, d, seq_len, num_sms()) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    const int64_t copies = rows / seq_len;
+    const int per_tile = ropec::kTileBytes / (d * 4);
     int* status = device_status_word();
     if (!status) return RK_ERR_NO_DEVICE;
     const int64_t ctas = (seq_len + per_tile - 1) / per_tile, slots = 2 * (int64_t)num_sms() * ropec::kCtasPerSm;
