@@ -101,6 +101,8 @@ def lib():
         L.rk_debug_verify_encoder.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
         L.rk_debug_set_prefill_dump.restype = None
         L.rk_debug_set_prefill_dump.argtypes = [C.c_void_p]
+        L.rk_debug_set_ring_stop.restype = None
+        L.rk_debug_set_ring_stop.argtypes = [C.c_int]
         L.rk_debug_rope_by_copies.restype = C.c_int
         L.rk_debug_rope_by_copies.argtypes = [C.c_int64, C.c_int, C.c_int64, C.c_int]
         L.rk_debug_set_decode_path.restype = None

@@ -579,6 +579,10 @@ RK_API int rk_debug_verify_encoder(int fmt, unsigned long long* mismatches, uint
  * the next prefill launches into `buf` (>= 32768 floats), or NULL to switch it off. */
 RK_API void rk_debug_set_prefill_dump(float* buf) { g_prefill_dbg = buf; }
 
+/* Test hook (not in the public header): the kernels that read by a ring of bulk copies (RoPE, RMSNorm; E4M3) act in every CTA as if a wait had run out, with
+ * copies under way: 1 = the readers, 2 = the warp that asks for the copies (RMSNorm), 0 = off. */
+RK_API void rk_debug_set_ring_stop(int role) { g_ring_stop = role; }
+
 /* Test hook (not in the public header): 1 where RoPE + quantization of so many rows goes through bulk copies on a device of `sms` SMs. */
 RK_API int rk_debug_rope_by_copies(int64_t rows, int d, int64_t seq_len, int sms) { return rope_by_copies(rows, d, seq_len, sms) ? 1 : 0; }
 

@@ -28,6 +28,8 @@
 
 namespace rk {
 
+int g_ring_stop = 0;   // set by rk_debug_set_ring_stop (tests only)
+
 // four floats -> four packed element codes (byte k = code of v[k]); finite inputs only
 template <int FMT> RK_DEVINL uint32_t hw_encode4(float a, float b, float c, float d) {
   uint32_t r;
@@ -316,7 +318,7 @@ namespace ropec {
 constexpr int kThreads = 128, kCtasPerSm = 8, kStages = 2, kTileBytes = kThreads * 64;      // a thread has 8 elements of either half of a row
 }  // namespace ropec
 struct RopeRing { uint8_t* data; uint64_t* full; uint32_t loads; };      // loads: so far
-template <int FMT, bool COLD>
+template <int FMT, bool COLD, bool STOPS>
 RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int seq_len, int pos0, const float* __restrict__ cos_h,
                            const float* __restrict__ sin_h, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, RopeRing& ring, int* status) {
   using namespace ropec;
@@ -330,7 +332,7 @@ RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int s
     mbar_arrive_expect_tx(bar, bytes);
     bulk_load_1d(ring.data + (n % kStages) * kTileBytes, x + ((int64_t)u * seq_len + p0) * d, bytes, bar);
   };
-  auto wait = [&](uint32_t n) -> bool {                       // bounded: about two seconds
+  auto wait = [&](uint32_t n) -> bool {                       // at most 2^20 polls of up to 2 us
 #pragma unroll 1
     for (int it = 0; it < 1 << 20; ++it)
       if (mbar_try_wait<2000>(&ring.full[n % kStages], (n / kStages) & 1)) return true;
@@ -351,13 +353,13 @@ RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int s
   bool finite = true;
   for (int k = 0; k < mine; ++k) {
     const uint32_t n = ring.loads + k;
-    const bool there = wait(n);
+    const bool there = wait(n) && !(STOPS && k == 1);          // (test hook: as if the wait had run out)
     const float4* src = reinterpret_cast<const float4*>(ring.data + (n % kStages) * kTileBytes + (live ? row : 0) * d * 4 + i0 * 4);      // (a branch around the loads: 8.98 us instead of 8.3 for 8.4 M elements)
     const float4 a0 = src[0], a1 = src[1], a2 = src[half / 4], a3 = src[half / 4 + 1];
     if (__syncthreads_or(!there)) {                           // (and read by all: the place is free)
       if (threadIdx.x == 0) {
         atomicCAS(status, 0, 601);
-        for (int i = k + 1; i < min(mine, k + kStages); ++i) wait(ring.loads + i);      // what is under way
+        for (int i = k; i < min(mine, k + kStages); ++i) wait(ring.loads + i);      // what is under way
       }
       return true;
     }
@@ -387,7 +389,7 @@ RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int s
   ring.loads += mine;
   return finite;
 }
-template <int FMT>
+template <int FMT, bool STOPS>
 __global__ void __launch_bounds__(ropec::kThreads, ropec::kCtasPerSm)
 rope_quantize_copies_kernel(const float* __restrict__ x, int copies, int d, int seq_len, int pos0, const float* __restrict__ cos_h, const float* __restrict__ sin_h,
                             uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status) {
@@ -399,8 +401,8 @@ rope_quantize_copies_kernel(const float* __restrict__ x, int copies, int d, int 
   grid_dependency_wait();
   grid_dependents_launch();
   RopeRing ring = {rope_data, rope_full, 0};
-  const bool finite = rope_copies<FMT, false>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);
-  if (__syncthreads_or(!finite)) rope_copies<FMT, true>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);      // the same rows
+  const bool finite = rope_copies<FMT, false, STOPS>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);
+  if (__syncthreads_or(!finite)) rope_copies<FMT, true, STOPS>(x, copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, ring, status);      // the same rows
 }
 
 // RMSNorm fused with the block quantizer: the prologue of the QKV projection (kernels/rmsnorm_qkv_fused), so that the
@@ -437,8 +439,6 @@ template <int ID> RK_DEVINL void named_arrive(int which) {
   else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"((1 + rms::kHelpers) * 32) : "memory");
 }
 
-// The second phase of the RMSNorm kernels: y = (x rms) gamma of the CTA's rows, quantized.  rms_smem: shared memory to put the scale bytes together in,
-// room bytes of it for every row.
 template <bool BF16IN, int PIECE>
 RK_DEVINL void load_pair(Raw8<BF16IN> (&r)[2], const uint8_t* src, bool a32) {
   if (BF16IN && PIECE == 16 && a32) {
@@ -446,6 +446,8 @@ RK_DEVINL void load_pair(Raw8<BF16IN> (&r)[2], const uint8_t* src, bool a32) {
       : "=r"(r[0].w[0]), "=r"(r[0].w[1]), "=r"(r[0].w[2]), "=r"(r[0].w[3]), "=r"(r[1].w[0]), "=r"(r[1].w[1]), "=r"(r[1].w[2]), "=r"(r[1].w[3]) : "l"(src));
   } else { r[0] = load_raw8<BF16IN, PIECE>(src); r[1] = load_raw8<BF16IN, PIECE>(src + 8 * (BF16IN ? 2 : 4)); }
 }
+// The second phase of the RMSNorm kernels: y = (x rms) gamma of the CTA's rows, quantized.  rms_smem: shared memory to put the scale bytes together in,
+// room bytes of it for every row.
 template <int FMT, bool BF16IN, bool UNIT, int PIECE, int kThreads>
 RK_DEVINL void rmsnorm_rows(const uint8_t* __restrict__ xr, int64_t row0, int n_rows, int K, const float* __restrict__ gamma, const float* rms_row,
                             uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, uint8_t* rms_smem, int room) {
@@ -474,7 +476,7 @@ RK_DEVINL void rmsnorm_rows(const uint8_t* __restrict__ xr, int64_t row0, int n_
       float g[2][8];
       widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col)), g[0]);
       widen8<false>(load_raw8<false, PIECE>(reinterpret_cast<const uint8_t*>(gamma + col + 8)), g[1]);
-            Raw8<BF16IN> raw[2];
+      Raw8<BF16IN> raw[2];
       if (part < n_rows) load_pair<BF16IN, PIECE>(raw, src, a32);
       src += src_step;
 #pragma unroll 1
@@ -638,10 +640,10 @@ rmsnorm_quantize_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int 
 namespace rmb {
 constexpr int kThreads = 512, kCtasPerSm = 2, kMaxRows = 32, kStages = 3, kPieceBytes = 1024, kPitch = kPieceBytes + 16;      // pitch: eight lanes, eight bank groups
 }  // namespace rmb
-template <int FMT, bool UNIT>
+template <int FMT, bool UNIT, bool STOPS>
 __global__ void __launch_bounds__(rmb::kThreads, rmb::kCtasPerSm)
 rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int rows_per_cta, const float* __restrict__ gamma,
-                             float eps, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status) {
+                             float eps, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status, int stop) {
   using namespace rmb;
   extern __shared__ __align__(16) uint8_t rmb_smem[];                   // [kStages][n_rows][kPitch]
   __shared__ float rms_row[kMaxRows];
@@ -661,17 +663,19 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
   // the chains of the CTAs of an SM on schedulers of their own: blocks go to the SMs in rounds of gridDim / kCtasPerSm
   const int chain_warp = (int)(blockIdx.x / ((gridDim.x + kCtasPerSm - 1) / kCtasPerSm)) % kCtasPerSm;
   bool ok = true;
-  auto wait = [&](uint64_t* bar, int use) -> bool {                     // bounded: about two seconds
+  int issued = 0;                                                       // pieces the producer has asked for
+  auto wait = [&](uint64_t* bar, int use) -> bool {                     // at most 2^20 polls of up to 2 us (a look at a flag of the other role's: 1-2 % of a call)
 #pragma unroll 1
     for (int it = 0; it < 1 << 20; ++it)
       if (mbar_try_wait<2000>(bar, use & 1)) return true;
     return false;
   };
+  auto stops = [&](int role, int c) { return STOPS && stop == role && c == kStages + 1; };      // test hook: the role acts as if its wait had run out
   if (warp == chain_warp) {
     float ss = 0.0f;
     for (int c = 0; c < n_pieces && ok; ++c) {
       const int st = c % kStages;
-      ok = __all_sync(0xffffffffu, wait(&full[st], c / kStages));
+      ok = __all_sync(0xffffffffu, !stops(1, c) && wait(&full[st], c / kStages));
       if (!ok) break;
       if (lane < n_rows) {
         const uint4* src = reinterpret_cast<const uint4*>(rmb_smem + st * stage_bytes + lane * kPitch);
@@ -712,16 +716,18 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
   } else if (warp == kThreads / 32 - 1) {
     for (int c = 0; c < n_pieces && ok; ++c) {
       const int st = c % kStages;
-      if (c >= kStages) ok = __all_sync(0xffffffffu, wait(&empty[st], c / kStages - 1));
+      if (c >= kStages) ok = __all_sync(0xffffffffu, !stops(2, c) && wait(&empty[st], c / kStages - 1));
       if (!ok) break;
       const uint32_t bytes = (uint32_t)min((int64_t)kPieceBytes, row_bytes - (int64_t)c * kPieceBytes);
       if (lane == 0) mbar_arrive_expect_tx(&full[st], bytes * n_rows);
       __syncwarp();
       if (lane < n_rows) bulk_load_1d(rmb_smem + st * stage_bytes + lane * kPitch, xr + lane * row_bytes + (int64_t)c * kPieceBytes, bytes, &full[st]);
+      ++issued;
     }
-    for (int c = max(0, n_pieces - kStages); c < n_pieces && !ok; ++c) wait(&full[c % kStages], c / kStages);      // what may be under way
   }
   if (__syncthreads_or(!ok)) {
+    // the copies under way, whichever role gave up, before shared memory goes to another CTA
+    for (int c = max(0, issued - kStages); c < issued; ++c) wait(&full[c % kStages], c / kStages);
     if (threadIdx.x == 0) atomicCAS(status, 0, 602);
     return;
   }
@@ -1463,12 +1469,12 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
     if (grid > 0x7FFFFFFF) return RK_ERR_BAD_SHAPE;
     const int smem = rmb::kStages * per_cta * rmb::kPitch;
 #define RK_RN(UN) RK_DISPATCH_FMT(fmt, {                                                                                \
-    auto kern = rmsnorm_quantize_bulk_kernel<F, UN>;                                                                   \
+    auto kern = F == RK_FMT_E4M3 && !UN && g_ring_stop ? rmsnorm_quantize_bulk_kernel<RK_FMT_E4M3, false, true> : rmsnorm_quantize_bulk_kernel<F, UN, false>; \
     if (smem > 48 * 1024) {                                                                                                \
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rmb::kStages * rmb::kMaxRows * rmb::kPitch); \
       if (e != cudaSuccess) return (int)e;                                                                                 \
     }                                                                                                                      \
-    return (int)launch_pdl(kern, dim3((unsigned)grid), dim3(rmb::kThreads), smem, st, reinterpret_cast<const uint8_t*>(x), rows, K, per_cta, gamma, eps, codes, scales, status); \
+    return (int)launch_pdl(kern, dim3((unsigned)grid), dim3(rmb::kThreads), smem, st, reinterpret_cast<const uint8_t*>(x), rows, K, per_cta, gamma, eps, codes, scales, status, g_ring_stop); \
   })
     if (unit_scale) { RK_RN(true); } else { RK_RN(false); }
 #undef RK_RN
@@ -1539,7 +1545,7 @@ int launch_rope_quantize_rows(const float* x, int64_t rows, int d, const int32_t
     if (!status) return RK_ERR_NO_DEVICE;
     const int64_t ctas = (seq_len + per_tile - 1) / per_tile, slots = 2 * (int64_t)num_sms() * ropec::kCtasPerSm;
     const dim3 grid((unsigned)ctas, (unsigned)std::min<int64_t>(std::max<int64_t>(1, slots / ctas), copies));
-    RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rope_quantize_copies_kernel<F>, grid, dim3(ropec::kThreads), 0, st, x, (int)copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, status));
+    RK_DISPATCH_FMT(fmt, return (int)launch_pdl(F == RK_FMT_E4M3 && g_ring_stop ? rope_quantize_copies_kernel<RK_FMT_E4M3, true> : rope_quantize_copies_kernel<F, false>, grid, dim3(ropec::kThreads), 0, st, x, (int)copies, d, seq_len, pos0, cos_h, sin_h, codes, scales, status));
   }
   // two rows per thread where every position has at least two and halving the threads still leaves every SM full
   const bool two = !pos && rows % seq_len == 0 && rows / seq_len >= 2 && nchunks >= (int64_t)num_sms() * 4096;

@@ -95,6 +95,37 @@ def test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d):
         assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("kernel,role,code", [("rmsnorm", 1, 602), ("rmsnorm", 2, 602), ("rope", 1, 601)])
+def test_a_ring_of_copies_that_gives_up_ends_the_call_and_the_next_one_is_whole(kernel, role, code):
+    """The RoPE and RMSNorm kernels that read by bulk copies: the readers, or the warp that asks for the copies, act after a few of them as if their wait had
+    run out, with others under way.  The kernel waits for those, reports a code (RMSNorm: without a byte written), and the next calls have every bit."""
+    L = rk.lib()
+    g = torch.Generator(device="cuda").manual_seed(95)
+    if kernel == "rmsnorm":
+        x, gamma = torch.randn(1200, 4096, generator=g, device="cuda").bfloat16(), torch.rand(4096, generator=g, device="cuda") + 0.5
+        call = lambda: rk.rmsnorm_mx_quantize(x, gamma, 1e-5)
+    else:
+        S, d = 4096, 128
+        x = torch.randn(1, 32, S, d, generator=g, device="cuda")
+        ang = torch.rand(S, d // 2, generator=g, device="cuda")
+        cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+        assert L.rk_debug_rope_by_copies(32 * S, d, S, torch.cuda.get_device_properties(0).multi_processor_count)
+        call = lambda: rk.rope_mx_quantize(x, cos, sin)
+    want = call()
+    assert rk.last_device_status() == 0
+    L.rk_debug_set_ring_stop(role)
+    try:
+        call()
+        torch.cuda.synchronize()
+    finally:
+        L.rk_debug_set_ring_stop(0)
+        status = rk.last_device_status()
+    assert status == code
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(call(), want))
+    assert rk.last_device_status() == 0
+
+
 def test_noalloc_decode_status_word_is_observable():
     L = rk.lib()
     g = torch.Generator(device="cuda").manual_seed(91)
