@@ -10,7 +10,7 @@
 #include "rk_internal.h"
 
 namespace rk {
-extern int g_prefill_perturb;
+extern int g_prefill_perturb, g_prefill_form;
 
 // The status word kernels record a given-up wait in: part of the library image (zero at load) on every device,
 // so it can never fail to allocate; its device address is looked up once per device.
@@ -607,6 +607,11 @@ RK_API int rk_debug_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile,
   if (!aligned(a_tile, 16) || !aligned(b_tile, 16)) return RK_ERR_MISALIGNED;
   return launch_mxfp8_mma_loop(a_tile, b_tile, iters, (cudaStream_t)stream);
 }
+
+/* Test hooks (not in the public header): the form (PrefillForm: 1, 2 or 3) the next prefill launches at d <= 128 take, 0 = the one the rule chooses; and
+ * the rule's choice for a call on a device of `sms` SMs (0 = the current one). */
+RK_API void rk_debug_set_prefill_form(int form) { g_prefill_form = form; }
+RK_API int rk_debug_prefill_form(const rk_prefill_args* a, int sms) { return prefill_form(*a, sms > 0 ? sms : num_sms()); }
 
 /* Test hook (not in the public header): which warp role of the prefill kernels sleeps a little at every key tile (0 = none;
  * 1, 2 = softmax of query tile A, B, of the lower and upper keys where a CTA has one query tile, of the two groups where they take the key tiles

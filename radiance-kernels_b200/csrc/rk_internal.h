@@ -47,6 +47,11 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st);
 
 bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms);      // which RoPE kernel a call without positions of its own takes
+// Which kernel a prefill call takes on a device of `sms` SMs: d = 256, pairs of query tiles, one query tile at a time with the softmax groups on alternate
+// key tiles, one query tile per CTA with both groups on every key tile.
+enum PrefillForm { kFormWide = 0, kFormPairs = 1, kFormTurns = 2, kFormSplit = 3 };
+int prefill_form(const rk_prefill_args& a, int64_t sms);
+
 int launch_rope_quantize_rows(const float* x, int64_t rows, int d, const int32_t* pos, int seq_len, int pos0, const float* cos_h,
                               const float* sin_h, int fmt, uint8_t* codes, uint8_t* scales, cudaStream_t st);
 int launch_kv_append(const float* k_new, const float* v_new, int B, int H_kv, int L, int d, const int32_t* pos, int fmt,

@@ -778,32 +778,40 @@ static int launch_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 }
 
 float* g_prefill_dbg = nullptr;   // set by rk_debug_set_prefill_dump (tests only)
-int g_prefill_perturb = 0;
-
-// d <= 128: one query tile per CTA at a time with the softmax groups on alternate key tiles (rk_prefill1.cu), or pairs of query tiles (rk_prefill2c.cu,
-// which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1650 cycles in the former and
-// half of 3400 in the latter, which loads K and V half as often and so loses less under the power cap: it has the large grids.  Measured (us, the pairs'
-// kernel and this one):
-//   no more query tiles than SMs: 8 / 32 heads of 512 11.1 10.3 / 13.9 13.5, 16 of 1024 18.4 17.0, 8 of 2048 27.8 24.1, 32 x 509 queries behind 3581 keys
-//     42.1 35.6.  Up to three key tiles the time is that of code run for the first time, of which the other form has less: 42 heads of 300 12.1 12.4, 128 of
-//     100 10.7 10.9.  With the cap: 8 of 2048 34.9 33.9, but 42.5 57.1 (32 x 512 by 1536, d = 64) where the 64 keys of a half differ in tanh's form.
-//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  512 queries behind 4096 keys, 72 heads (288 tiles) 98.3 96.7,
-//     96 heads 166 137; 500 by 2000 keys without a mask, 64 heads 46.5 46.9; capped, 72 heads 135 146, 96 heads 229 206.
-//   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 40.2 24.3, 16 40.7 27.8, 23 41.5 36.4,
-//     27 42.4 41.0, 31 44.7 45.6; 23 heads of 1024 25.6 17.4, 37 26.5 22.6, 47 26.9 26.6, 56 29.2 30.1; 144 of 300 21.8 20.3; capped, with a cap of 50 and of
-//     30, 24 heads of 1024 32.5 22.0 and 69.2 38.2, 26 of 2048 65.1 56.0 and 162 134; 24 of 2048 with a window of 512 33.2 27.1.
-static bool alternate_key_tiles(const PrefillParams& p, bool cap) {
-  const int64_t sms = num_sms(), heads = (int64_t)p.B * p.H, tiles = p.n_q_tiles * heads, pairs = (p.n_q_tiles + 1) / 2 * heads;
-  const int item_tiles = p.window > 0 ? (int)std::min<int64_t>(p.n_kv_tiles, ((int64_t)p.window + kBlockM - 2) / kBlockN + 2) : p.n_kv_tiles;     // at most
-  if (tiles <= sms) return item_tiles > 3 && !cap;
-  const bool level = p.window == 0 && (!p.causal || 2 * ((int64_t)p.q_pos0 + kBlockM) > p.S_kv);
-  if (level) return 10 * ((tiles + sms - 1) / sms) < 19 * ((pairs + sms - 1) / sms);
-  return tiles <= 3 * sms;
-}
+int g_prefill_perturb = 0, g_prefill_form = 0;
 
 // A window that reaches beyond the first key for every row masks nothing.  Any other is at most the last row's position, so that the kernels' position - window
 // - key stays within 32 bits (a caller's "no limit", a window near 2^31, wrapped and masked keys that the row sees).
 static int effective_window(const rk_prefill_args& a) { return a.window > (int64_t)a.q_pos0 + a.S_q - 1 ? 0 : a.window; }
+
+// d <= 128: one query tile per CTA at a time with the softmax groups on alternate key tiles (rk_prefill1.cu), or pairs of query tiles (rk_prefill2c.cu,
+// which has a form of its own for one query tile per CTA, both groups on every key tile).  A key tile of one query tile takes 1650 cycles in the former and
+// half of 3400 in the latter, which loads K and V half as often and so loses less under the power cap.  Measured (us, one call behind another in a graph, the
+// attention kernel alone on prepared operands, as many KV heads as heads where no other number is given; the pairs' kernel and this one):
+//   no more query tiles than SMs (both groups on every key tile, and this one): 8 / 32 heads of 512 9.0 8.3 / 9.5 9.2, 16 of 1024 14.0 12.8, 8 of 2048 23.4
+//     19.9, 32 x 509 queries behind 3581 keys 37.7 32.1.  Up to three key tiles the time is that of code run for the first time, of which the other form has
+//     less: 42 heads of 300 7.7 8.1, 128 of 100 6.1 6.5.  With a cap of 50 1-5 % faster, but with one of 30, where the 64 keys of a half differ in tanh's form,
+//     8 of 2048 42.7 67.1, the chunk 72.0 129.
+//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  Without a mask, 8 KV heads of 2048 keys, by rounds of this
+//     kernel over rounds of pairs: 4 / 3 (192 heads of 384) 87.2 67.1, 3 / 2 (96 of 512) 65.8 51.0, 7 / 4 (192 of 640) 118.2 112.7, 2 (72 of 512) 36.2 35.5; call
+//     after call under the power cap 1.64 (8 x 64 of 640, 4096 keys) 609 604, 1.78 (4 x 64 of 1152, 4096 keys) 520 520, 1.82 (192 of 1920) 337 337, 1.875 (192
+//     of 1408) 246 250: up to 1.8.  Capped at 50, 4 / 3 123 109, 3 / 2 90.2 81.8, 5 / 3 (64 of 1408) 133.5 133.8, 7 / 4 169 184, 15 / 8 342 387, 2 49.1 55.9; at 30,
+//     3 / 2 215 203, 12 / 7 873 892, 15 / 8 1051 1088: up to 1.6.
+//   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 35.7 20.3, 16 36.1 22.9, 23 36.4 31.3,
+//     27 36.5 35.4; 24 heads of 1024 21.2 13.6, 37 21.5 16.9, 47 21.7 21.0; 144 of 300 16.3 14.9; 24 of 2048 with a window of 512 27.8 22.0; capped at 50 and at
+//     30, 24 heads of 1024 26.6 18.6 and 64.6 33.5, 27 of 2048 53.4 51.0 and 156 134.  (Above three tiles per SM, 31 of 2048 and 56 of 1024, 2-3 % slower.)
+int prefill_form(const rk_prefill_args& a, int64_t sms) {
+  if (a.d > 128) return kFormWide;
+  const int64_t heads = (int64_t)a.B * a.H, q_tiles = (a.S_q + kBlockM - 1) / kBlockM, tiles = q_tiles * heads, pairs = (q_tiles + 1) / 2 * heads;
+  const int64_t kv_tiles = (a.S_kv + kBlockN - 1) / kBlockN;
+  const int window = effective_window(a);
+  const int64_t item_tiles = window > 0 ? std::min(kv_tiles, ((int64_t)window + kBlockM - 2) / kBlockN + 2) : kv_tiles;     // at most
+  const bool cap = a.softcap > 0.0f;
+  if (tiles <= sms) return item_tiles > 3 && !cap ? kFormTurns : kFormSplit;
+  const bool level = window == 0 && (!a.causal || 2 * ((int64_t)a.q_pos0 + kBlockM) > a.S_kv);
+  if (level) return 10 * ((tiles + sms - 1) / sms) < (cap ? 16 : 18) * ((pairs + sms - 1) / sms) ? kFormTurns : kFormPairs;
+  return tiles <= 3 * sms ? kFormTurns : kFormPairs;
+}
 
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st) {
@@ -852,11 +860,13 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
   const uint32_t idesc_pv = make_idesc(RK_FMT_E4M3, a.kv_fmt, false, /*B MN-major*/ !kv6, 128, 128);
   dim3 grid(p.n_q_tiles * a.H * a.B, 1, 1);
   const bool cap = a.softcap > 0.0f;
-  if (a.d <= 128) {                                                                      // two query tiles per CTA
+  if (a.d <= 128) {
     CUtensorMap to;
     rc = make_tmap_o(&to, a.o, (int64_t)a.B * a.H, a.S_q, a.d);
     if (rc != RK_OK) return rc;
-    return (alternate_key_tiles(p, cap) ? launch_prefill1 : launch_prefill2c)(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
+    const int form = g_prefill_form ? g_prefill_form : prefill_form(a, num_sms());
+    if (form == kFormTurns) return launch_prefill1(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
+    return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, form == kFormSplit, st);
   }
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)

@@ -219,12 +219,13 @@ int make_tmap_u8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t S, int
 int make_tmap_sub8_3d(CUtensorMap* m, const void* base, int64_t BH, int64_t rows, int64_t cols_padded, int bits);
 extern float* g_prefill_dbg;
 
-// Two query tiles per CTA, one thread per row, correction warps (d <= 128); defined in rk_prefill2c.cu.
+// Two query tiles per CTA, one thread per row, correction warps (d <= 128), or with `split` one query tile; defined in rk_prefill2c.cu.
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
-                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st);
+                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, cudaStream_t st);
 // One query tile per CTA at a time, two softmax groups on alternate key tiles (d <= 128, few query tiles); defined in rk_prefill1.cu.
 int launch_prefill1(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st);
 extern int g_prefill_perturb;   // test hook: PrefillParams::perturb of the next launches
+extern int g_prefill_form;      // test hook: the form of the next launches at d <= 128, 0 = by prefill_form
 
 }  // namespace rk

@@ -913,9 +913,7 @@ static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 }
 
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
-                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st) {
-  // One query tile per CTA while every tile can have an SM: above that, two tiles per CTA share K, V and the SM.
-  const bool split = (int64_t)p.n_q_tiles * p.H * p.B <= num_sms();
+                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, cudaStream_t st) {
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return split ? (softcap ? launch2c_cfg<true, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
                             : launch2c_cfg<false, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st))

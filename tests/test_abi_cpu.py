@@ -228,3 +228,22 @@ def test_rope_goes_by_copies_where_its_tiles_are_full(copies, seq_len, d, want):
     """RoPE + quantization through bulk copies has a range of positions of one sequence per CTA: not for many short sequences, whose tiles would be mostly empty
     (2048 x 28 rows of one position took 41.7 us instead of 7.2)."""
     assert rk.lib().rk_debug_rope_by_copies(copies * seq_len, d, seq_len, 148) == want
+
+
+WIDE, PAIRS, TURNS, SPLIT = 0, 1, 2, 3
+
+
+@pytest.mark.parametrize("kw,want", [
+    (dict(H=192, S_q=384), TURNS), (dict(H=96, S_q=512), TURNS), (dict(H=192, S_q=640), TURNS), (dict(H=72, S_q=512), PAIRS), (dict(H=192, S_q=1408), PAIRS),
+    (dict(H=192, S_q=384, softcap=50.0), TURNS), (dict(H=96, S_q=512, softcap=50.0), TURNS), (dict(H=64, S_q=1408, softcap=30.0), PAIRS),
+    (dict(H=192, S_q=640, softcap=50.0), PAIRS), (dict(H=192, S_q=1408, softcap=50.0), PAIRS), (dict(H=192, S_q=1920, softcap=30.0), PAIRS),      # items of equal length
+    (dict(H=96, S_q=512, S_kv=4096, q_pos0=3584, causal=1, softcap=50.0), TURNS), (dict(H=192, S_q=640, S_kv=4096, q_pos0=3456, causal=1, softcap=50.0), PAIRS),
+    (dict(H=24, S_q=2048, causal=1), TURNS), (dict(H=28, S_q=2048, causal=1), PAIRS), (dict(H=24, S_q=2048, causal=1, softcap=30.0), TURNS),
+    (dict(H=16, S_q=1024, S_kv=1024, causal=1), TURNS), (dict(H=16, S_q=1024, S_kv=1024, causal=1, softcap=50.0), SPLIT), (dict(H=42, S_q=300, S_kv=300, causal=1), SPLIT),
+    (dict(H=16, S_q=1024, causal=1, window=2 ** 31 - 1), TURNS), (dict(H=16, S_q=1024, causal=1, window=64), SPLIT), (dict(H=96, S_q=512, window=2 ** 31 - 1), TURNS),
+    (dict(H=16, S_q=1024, d=256), WIDE)])
+def test_prefill_form_on_148_sms(kw, want):
+    """Which kernel a call takes: pairs of query tiles, one at a time with the softmax groups on alternate key tiles, or one per CTA with both on every key tile.
+    A capped call of equally long items keeps to pairs unless single tiles save a good part of the last round (192 heads of 1408 by 2048 342 us against 387)."""
+    a = _pargs(**dict(dict(S_kv=2048, H_kv=1), **kw))
+    assert rk.lib().rk_debug_prefill_form(C.byref(a), 148) == want
