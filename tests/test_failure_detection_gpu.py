@@ -10,7 +10,7 @@ import torch
 
 import radiance_kernels_b200 as rk
 from radiance_kernels_b200._lib import DecodeArgs
-from helpers import quantize_inputs, randn_qkv
+from helpers import PAIRS, SPLIT, TURNS, prefill_form, quantize_inputs, randn_qkv
 
 pytestmark = pytest.mark.gpu
 
@@ -49,8 +49,9 @@ def test_bounded_wait_runs_out_and_is_reported_and_clears():
     assert rk.last_device_status() == 0
 
 
-@pytest.mark.parametrize("H,S,d,q_pos0", [(2, 300, 256, 0), (160, 200, 256, -130), (160, 100, 128, 0), (160, 200, 64, -130)])
-def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0):
+@pytest.mark.parametrize("H,S,d,q_pos0,form", [(2, 300, 256, 0, 0), (160, 200, 256, -130, 0), (160, 100, 128, 0, TURNS), (160, 200, 64, -130, TURNS),
+                                               (300, 300, 128, 0, PAIRS), (300, 200, 64, -130, PAIRS), (2, 300, 128, 0, SPLIT), (60, 200, 64, -130, SPLIT)])
+def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0, form):
     """Every form of the prefill kernels, items of one key tile and query tiles without a visible key among them: neither O nor the
     log-sum-exps are touched."""
     L = rk.lib()
@@ -61,38 +62,42 @@ def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0):
     assert L.rk_debug_wait_runs_out(1000, 0, _stream()) == 0
     torch.cuda.synchronize()
     try:
-        rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
+        with prefill_form(form):
+            rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
         torch.cuda.synchronize()
     finally:
         status = rk.last_device_status()
     assert status == WAIT_GAVE_UP and (o == 7.0).all() and (lse == 7.0).all()
-    rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
+    with prefill_form(form):
+        rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_pos0=q_pos0, out=o, lse=lse)
     torch.cuda.synchronize()
     assert rk.last_device_status() == 0 and not (o == 7.0).all() and not (lse == 7.0).any()
 
 
-@pytest.mark.parametrize("H,S,d", [(2, 600, 128), (100, 600, 128), (200, 300, 64), (2, 600, 256), (100, 600, 256)])      # a CTA per query tile, and many items each
-def test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d):
+@pytest.mark.parametrize("H,S,d,form", [(2, 600, 128, TURNS), (100, 600, 128, TURNS), (200, 300, 64, TURNS), (2, 300, 128, SPLIT), (30, 600, 64, SPLIT),
+                                        (2, 600, 128, PAIRS), (300, 512, 128, PAIRS), (250, 1024, 64, PAIRS), (2, 600, 256, 0), (100, 600, 256, 0)])
+def test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d, form):
     """One warp role at a time (either softmax group, correction, TMA producer, Q K^T and P V issuer) acts after a key tile as if its
     wait had run out: loads, MMAs and stores are under way, the other roles see the CTA's flag, the kernel ends, a code is reported and the next
-    call has every bit of the one before."""
+    call has every bit of the one before.  At d <= 128 in every form, one item per CTA and many."""
     L = rk.lib()
     qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, S, S, d, seed=93))
-    want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
-    assert rk.last_device_status() == 0
-    for role in (1, 2, 3, 4, 5, 6):
-        if d == 256 and role == 3:
-            continue                                                    # no correction warps there
-        L.rk_debug_set_prefill_perturb(100 + role)
-        try:
-            rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
-            torch.cuda.synchronize()
-        finally:
-            L.rk_debug_set_prefill_perturb(0)
-            status = rk.last_device_status()
-        assert 100 < status < 600, (role, status)
-        assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False), want), role
+    with prefill_form(form):
+        want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
         assert rk.last_device_status() == 0
+        for role in (1, 2, 3, 4, 5, 6):
+            if d == 256 and role == 3:
+                continue                                                # no correction warps there
+            L.rk_debug_set_prefill_perturb(100 + role)
+            try:
+                rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False)
+                torch.cuda.synchronize()
+            finally:
+                L.rk_debug_set_prefill_perturb(0)
+                status = rk.last_device_status()
+            assert 100 < status < 600, (role, status)
+            assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False), want), role
+            assert rk.last_device_status() == 0
 
 
 @pytest.mark.parametrize("kernel,role,code", [("rmsnorm", 1, 602), ("rmsnorm", 2, 602), ("rope", 1, 601)])
@@ -181,12 +186,14 @@ def test_a_failed_launch_is_reported_once():
     assert rk.last_device_status() == 0
 
 
-@pytest.mark.parametrize("shape", [(2, 4, 2, 1024, 128, False), (1, 2, 1, 640, 64, False), (1, 4, 4, 512, 128, True),      # one query tile per CTA
-                                   (2, 16, 4, 900, 128, False), (1, 40, 8, 520, 64, False), (1, 52, 4, 384, 128, True)])  # two
-def test_schedule_perturbation_leaves_every_bit_of_o(shape):
+@pytest.mark.parametrize("form", [PAIRS, TURNS, SPLIT])
+@pytest.mark.parametrize("shape", [(2, 4, 2, 1024, 128, False), (1, 2, 1, 640, 64, False), (1, 4, 4, 512, 128, True),      # no more query tiles than SMs
+                                   (2, 16, 4, 900, 128, False), (1, 40, 8, 520, 64, False), (1, 52, 4, 384, 128, True)])  # more
+def test_schedule_perturbation_leaves_every_bit_of_o(shape, form):
     """A few hundred nanoseconds of sleep at every key tile in one warp role at a time (softmax of query tile A,
-    of tile B -- of the lower and of the upper keys where a CTA has one query tile --, correction, TMA producer, Q K^T issuer, P V issuer): if a hand-off between roles lacked a barrier the delayed
-    role would read or overwrite something too early and O would change."""
+    of tile B -- of the lower and of the upper keys, or of the even and the odd key tiles, where a CTA has one query tile --, correction, TMA producer,
+    Q K^T issuer, P V issuer): if a hand-off between roles lacked a barrier the delayed
+    role would read or overwrite something too early and O would change.  In every form, against the form the library chooses."""
     B, H, Hkv, S, d, cap = shape
     L = rk.lib()
     Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=92)
@@ -194,10 +201,11 @@ def test_schedule_perturbation_leaves_every_bit_of_o(shape):
     kw = dict(causal=True, softcap=30.0 if cap else 0.0)
     base = rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
     try:
-        for role in (1, 2, 3, 4, 5, 6):
-            L.rk_debug_set_prefill_perturb(role)
-            for _ in range(2):
-                assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw), base), role
+        with prefill_form(form):
+            for role in (1, 2, 3, 4, 5, 6):
+                L.rk_debug_set_prefill_perturb(role)
+                for _ in range(2):
+                    assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw), base), role
     finally:
         L.rk_debug_set_prefill_perturb(0)
     assert rk.last_device_status() == 0
@@ -239,11 +247,6 @@ def test_schedule_perturbation_in_both_kernels_of_narrow_heads(shape):
     """The delays of the test above where a CTA has some three query tiles one after the other, and where it has as many pairs of them."""
     H, S, d, cap, kw = shape
     test_schedule_perturbation_where_ctas_take_item_after_item((H, S, d, cap, kw))
-
-
-@pytest.mark.parametrize("H,S,d", [(2, 300, 128), (300, 512, 128), (250, 1024, 64)])      # 64 keys a group; pairs
-def test_a_role_that_gives_up_in_the_other_forms_for_narrow_heads(H, S, d):
-    test_a_role_that_gives_up_ends_the_call_and_the_next_one_is_whole(H, S, d)
 
 
 def test_tensor_pipe_ceiling_loop_never_runs_into_its_waits():

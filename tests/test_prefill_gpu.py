@@ -5,7 +5,7 @@ import torch
 
 import oracle
 import radiance_kernels_b200 as rk
-from helpers import MAX_ABS, REL_L2, errors, np_, prefill_vs_oracle, quantize_inputs, randn_qkv
+from helpers import MAX_ABS, PAIRS, REL_L2, SPLIT, TURNS, chosen_form, errors, np_, prefill_form, prefill_vs_oracle, quantize_inputs, randn_qkv
 
 pytestmark = pytest.mark.gpu
 
@@ -66,7 +66,7 @@ def test_sliding_window_d128():
                                                       (256, 1280, 200, 0, 50.0), (128, 900, 1, 0, 0.0)])
 def test_sliding_window_skips_key_tiles_below_the_window(d, S, window, q_pos0, softcap):
     """Long sequences with a short window: most key tiles lie wholly below the window and are never loaded; the
-    result must equal the oracle's, which masks them (d = 128 with one query tile per CTA and, at 20 heads, with two; d = 256)."""
+    result must equal the oracle's, which masks them (d = 128 in every form; d = 256)."""
     for H in (2, 20) if d == 128 else (2,):
         _check(prefill_vs_oracle(1, H, 1, S, S + q_pos0, d, causal=True, window=window, q_pos0=q_pos0, softcap=softcap,
                                  mul=0.5 if d == 256 else 1.0, seed=60 + window))
@@ -91,7 +91,7 @@ def test_v_scales_along_keys_reference_layout():
 
 
 def test_e5m2_operands():
-    for H in (2, 76):                                              # a CTA per query tile, and one for two of them
+    for H in (2, 76):                                              # one item per CTA, and more
         _check(prefill_vs_oracle(1, H, 1, 256, 256, 128, causal=True, fmt=rk.E5M2, seed=11))
 
 
@@ -99,7 +99,7 @@ def test_mxfp6_operands_e2m3_q_e3m2_kv():
     """MXFP6 variant: E2M3 queries, E3M2 keys and values (P stays E4M3), 6-bit codes packed for the tensor core."""
     import oracle
     for (B, H, Hkv, Sq, Skv, d, axis) in ((1, 2, 1, 256, 256, 128, rk.V_SCALES_ALONG_D), (1, 4, 2, 200, 333, 64, rk.V_SCALES_ALONG_KEYS),
-                                          (1, 76, 2, 256, 256, 128, rk.V_SCALES_ALONG_D), (2, 40, 2, 200, 333, 64, rk.V_SCALES_ALONG_KEYS),   # two query tiles per CTA
+                                          (1, 76, 2, 256, 256, 128, rk.V_SCALES_ALONG_D), (2, 40, 2, 200, 333, 64, rk.V_SCALES_ALONG_KEYS),   # more items than CTAs
                                           (1, 2, 1, 384, 384, 256, rk.V_SCALES_ALONG_D)):
         Q, K, V = randn_qkv(B, H, Hkv, Sq, Skv, d, seed=31, mul=0.5)
         qc, qs = rk.mx_quantize(Q, rk.E2M3)
@@ -113,6 +113,10 @@ def test_mxfp6_operands_e2m3_q_e3m2_kv():
                                   softcap=50.0 if d == 256 else 0.0, q_fmt=rk.E2M3, kv_fmt=rk.E3M2, v_scale_axis=axis, block_n=128)
         ma, rl = errors(np_(o.float()), ref["o_f32"])
         assert ma <= MAX_ABS and rl <= REL_L2, (d, ma, rl)
+        for form in (PAIRS, TURNS, SPLIT) if d <= 128 else ():
+            with prefill_form(form):
+                assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True, q_fmt=rk.E2M3, kv_fmt=rk.E3M2, v_scale_axis=axis), o), (H, form)
+    assert rk.last_device_status() == 0
 
 
 def test_mxfp4_operands_e2m1():
@@ -189,9 +193,11 @@ def test_a_key_tile_of_nan_scores_leaves_no_finite_row(H, d, tile, softcap):
     that is not positive gives), whichever thread or group of threads had the tile."""
     qc, qs, kc, ks, vc, vs = quantize_inputs(*randn_qkv(1, H, H, 256, 256, d, seed=64), fmt=rk.E5M2)
     kc[:, :, tile * 128:(tile + 1) * 128] = 0x7C
-    lse = torch.zeros(1, H, 256, device="cuda")
-    o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False, softcap=softcap, lse=lse, q_fmt=rk.E5M2, kv_fmt=rk.E5M2)
-    assert torch.isnan(o).all() and torch.isneginf(lse).all()
+    for form in (0, PAIRS, TURNS, SPLIT) if d <= 128 else (0,):
+        lse = torch.zeros(1, H, 256, device="cuda")
+        with prefill_form(form):
+            o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=False, softcap=softcap, lse=lse, q_fmt=rk.E5M2, kv_fmt=rk.E5M2)
+        assert torch.isnan(o).all() and torch.isneginf(lse).all(), form
     assert rk.last_device_status() == 0
 
 
@@ -201,19 +207,21 @@ def test_lse_output():
     assert np.abs(r["lse"] - r["ref"]["lse"]).max() < 1e-3
 
 
-@pytest.mark.parametrize("B,H,Hkv,S,d,causal", [
-    (2, 4, 2, 1024, 128, True),
-    (8, 64, 64, 200, 64, False), (8, 64, 64, 160, 128, False),      # the second query tile of every pair ends inside its TMEM lane quadrants
-    (2, 20, 10, 640, 256, False)])                                  # 200 query tiles of five key tiles
-def test_bit_identical_across_runs(B, H, Hkv, S, d, causal):
+@pytest.mark.parametrize("B,H,Hkv,S,d,causal,form", [
+    (2, 4, 2, 1024, 128, True, 0),
+    (8, 64, 64, 200, 64, False, PAIRS), (8, 64, 64, 160, 128, False, PAIRS),      # the second query tile of every pair ends inside its TMEM lane quadrants
+    (8, 64, 64, 200, 64, False, TURNS), (8, 64, 64, 160, 128, False, TURNS),
+    (2, 20, 10, 640, 256, False, 0)])                               # 200 query tiles of five key tiles
+def test_bit_identical_across_runs(B, H, Hkv, S, d, causal, form):
     """Race check borrowed from the reference ("bit-identical O across 13 runs",
     kernels/flash_attention_mx/kernel.cpp:158-160)."""
     Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=13)
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
-    first = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
-    for _ in range(5):
-        again = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
-        assert torch.equal(first, again)
+    with prefill_form(form):
+        first = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
+        for _ in range(5):
+            again = rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=causal)
+            assert torch.equal(first, again)
     assert rk.last_device_status() == 0
 
 
@@ -266,10 +274,11 @@ def test_full_size_head_slices_match_oracle():
         assert ma <= MAX_ABS and rl <= REL_L2, (sl, ma, rl)
 
 
+@pytest.mark.parametrize("form", [PAIRS, TURNS, SPLIT])
 @pytest.mark.parametrize("d,qmul,H", [(128, 1.0, 1), (128, 6.0, 1), (64, 1.0, 1), (128, 1.0, 75), (128, 6.0, 75), (64, 1.0, 75)])
-def test_stage_parity_s_and_requantized_p(d, qmul, H):
-    """Stage-level parity on the first key tile of the last query tile of head 0 (the kernels' debug dump; one query tile per CTA with
-    one head, two with 75): S = Q K^T within
+def test_stage_parity_s_and_requantized_p(d, qmul, H, form):
+    """Stage-level parity on the first key tile of the last query tile of head 0 (the kernels' debug dump), in every form, with one item per
+    CTA (one head) and more (75): S = Q K^T within
     fp32 reassociation error, and the requantized P -- E4M3 codes and E8M0 block scales -- equal to the oracle's.
     A code may differ by one step where the fp32 p sits on a truncation boundary; such elements are counted and
     must stay below 0.05 %."""
@@ -280,7 +289,8 @@ def test_stage_parity_s_and_requantized_p(d, qmul, H):
     dbg = torch.zeros(32768, dtype=torch.float32, device="cuda")
     rk.lib().rk_debug_set_prefill_dump(C.c_void_p(dbg.data_ptr()))
     try:
-        rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True)
+        with prefill_form(form):
+            rk.attn_prefill(qc, kc, vc, qs, ks, vs, causal=True)
         torch.cuda.synchronize()
     finally:
         rk.lib().rk_debug_set_prefill_dump(None)
@@ -316,8 +326,7 @@ def test_stage_parity_s_and_requantized_p(d, qmul, H):
     (1, 2, 1, 1, 129, 128, dict(causal=True, q_pos0=128)),        # one query, one key in the last key tile
     (1, 2, 2, 130, 65, 64, dict(causal=True))])                   # keys of one half of a key tile, and one of the other
 def test_grids_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, Sq, Skv, d, kw):
-    """Grids of at most one query tile per SM put both softmax groups on one tile (64 keys each of every key tile), larger
-    ones give a CTA two tiles; odd numbers of tiles, masks that cut a key tile in either half."""
+    """Grids of no more query tiles than SMs and of a few more; odd numbers of tiles, masks that cut a key tile in either half."""
     _check(prefill_vs_oracle(B, H, Hkv, Sq, Skv, d, seed=61, **kw))
 
 
@@ -356,10 +365,14 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
 
 
 @pytest.mark.parametrize("B,H,Hkv,S,d,kw", [
-    (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles, chunks of at most 128
-    (2, 12, 4, 1090, 64, dict(causal=True, window=300)),          # 216, odd numbers of tiles per head
-    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0)),       # 160
-    (2, 100, 50, 200, 64, dict(causal=False)),                    # lane quadrants of the second query tile that have no row, after ones of the first that have
+    (1, 16, 16, 2048, 128, dict(causal=True)),                    # 256 query tiles: one at a time, also in the pieces
+    (1, 32, 32, 2048, 128, dict(causal=True)),                    # 512: pairs, and the pieces one at a time
+    (2, 32, 16, 1090, 64, dict(causal=True, window=300)),         # 576, odd numbers of tiles per head: the same
+    (8, 18, 9, 512, 64, dict(causal=False)),                      # 576 of equal length: the same
+    (1, 40, 10, 500, 128, dict(causal=True, softcap=5.0)),        # 160: one at a time, the pieces with both groups on every key tile
+    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0)),       # pairs, the pieces with both groups on every key tile
+    (2, 12, 4, 1090, 64, dict(causal=True, window=300)),
+    (2, 100, 50, 200, 64, dict(causal=False)),                    # lane quadrants that have no row
     (2, 90, 90, 140, 128, dict(causal=False)),
     (1, 20, 10, 1200, 128, dict(causal=True)),
     (2, 20, 10, 640, 256, dict(causal=False)),                    # 200 of five key tiles: a CTA's second item starts on an odd one
@@ -368,12 +381,16 @@ def test_v_preparation_equals_the_oracle_re_blocking(S, d, fmt):
     (2, 100, 100, 128, 256, dict(causal=False, softcap=50.0))])
 def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm(B, H, Hkv, S, d, kw):
     """A call whose query tiles outnumber the SMs, against the same call cut by the host entry point and unit by unit, where each
-    piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in both forms, and at d = 256
-    whatever the CTA worked on before)."""
+    piece has a CTA per tile: O and the log-sum-exp are equal bit for bit (the row sum is taken in one order in every form, and at d = 256
+    whatever the CTA worked on before).  At d <= 128 the whole call in the other forms too."""
     Q, K, V = randn_qkv(B, H, Hkv, S, S, d, seed=62)
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
     lse = torch.empty(B, H, S, dtype=torch.float32, device="cuda")
     o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw)
+    for form in (PAIRS, TURNS, SPLIT) if d <= 128 else ():
+        with prefill_form(form):
+            l1 = torch.empty_like(lse)
+            assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=l1, **kw), o) and torch.equal(l1, lse), form
     sms, grp = torch.cuda.get_device_properties(0).multi_processor_count, H // Hkv
     assert B * H * ((S + 127) // 128) > sms >= grp * ((S + 127) // 128)
     for b in range(B):
@@ -387,16 +404,31 @@ def test_smaller_calls_give_the_same_bits_on_both_sides_of_one_query_tile_per_sm
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("B,H,Hkv,S,d,kw,whole,piece", [
+    (1, 32, 32, 2048, 128, dict(causal=True), PAIRS, TURNS), (2, 32, 16, 1090, 64, dict(causal=True, window=300), PAIRS, TURNS),
+    (8, 18, 9, 512, 64, dict(causal=False), PAIRS, TURNS), (1, 40, 10, 500, 128, dict(causal=True, softcap=5.0), TURNS, SPLIT),
+    (1, 40, 10, 500, 128, dict(causal=False, softcap=5.0), PAIRS, SPLIT), (2, 100, 50, 200, 64, dict(causal=False), TURNS, SPLIT)])
+def test_forms_of_a_call_and_of_its_pieces(B, H, Hkv, S, d, kw, whole, piece):
+    """The test above sees every pair of forms that a call and its pieces can have (148 SMs)."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shapes are chosen for 148 SMs")
+    assert chosen_form(B, H, S, S, d, **kw) == whole and chosen_form(1, H // Hkv, S, S, d, **kw) == piece
+
+
 @pytest.mark.parametrize("key,factor", [(5, 20.0), (5, 30.0), (70, 20.0), (70, 30.0)])
 def test_smaller_calls_give_the_same_bits_around_the_soft_caps_series_limit(key, factor):
     """One key of every key tile has logits on both sides of cap / 8, the others far below: the exponential form of the cap for that key's
-    half of the tile and the series for the other, in pairs of query tiles (160) and with a CTA per tile."""
+    half of the tile and the series for the other, in every form and with a CTA per tile."""
     Q, K, V = randn_qkv(1, 40, 10, 500, 500, 128, seed=63, mul=0.3)
     K[:, :, key::128] *= factor                                   # logits of standard deviation 1.8 and 2.7, 128 rows x 4 tiles of them a head
     qc, qs, kc, ks, vc, vs = quantize_inputs(Q, K, V)
     kw = dict(causal=False, softcap=50.0)
     lse = torch.empty(1, 40, 500, dtype=torch.float32, device="cuda")
     o = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw)
+    for form in (PAIRS, TURNS, SPLIT):
+        with prefill_form(form):
+            l1 = torch.empty_like(lse)
+            assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=l1, **kw), o) and torch.equal(l1, lse), form
     for h in range(10):
         part = [t[:, h * 4:(h + 1) * 4].contiguous() for t in (qc, qs)] + [t[:, h:h + 1].contiguous() for t in (kc, ks, vc, vs)]
         l1 = torch.empty(1, 4, 500, dtype=torch.float32, device="cuda")
@@ -431,15 +463,16 @@ def test_window_edges_against_tile_edges(d, window):
     _check(prefill_vs_oracle(2, 4, 2, 515, 600, d, causal=True, q_pos0=85, window=window, seed=32))
 
 
-@pytest.mark.parametrize("H,Sq,d", [(2, 150, 64), (2, 150, 128), (160, 150, 128), (2, 150, 256)])
-def test_o_at_a_16_byte_boundary(H, Sq, d):
+@pytest.mark.parametrize("H,Sq,d,form", [(2, 150, 64, SPLIT), (2, 150, 128, SPLIT), (160, 150, 128, PAIRS), (160, 150, 128, TURNS), (2, 150, 64, TURNS), (2, 150, 256, 0)])
+def test_o_at_a_16_byte_boundary(H, Sq, d, form):
     """O need not be 32-byte aligned: rows then leave in 16-byte stores.  The same bits, nothing beside them."""
     q, qs, k, ks, v, vs = quantize_inputs(*randn_qkv(1, H, H, Sq, Sq, d, 33))
     want = rk.attn_prefill(q, k, v, qs, ks, vs, causal=True)
     flat = torch.full((want.numel() + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
     out = flat[8:8 + want.numel()].view(want.shape)
     assert out.data_ptr() % 32 == 16
-    rk.attn_prefill(q, k, v, qs, ks, vs, causal=True, out=out)
+    with prefill_form(form):
+        rk.attn_prefill(q, k, v, qs, ks, vs, causal=True, out=out)
     assert torch.equal(out, want) and (flat[:8] == 7.0).all() and (flat[-8:] == 7.0).all()
 
 
