@@ -111,6 +111,8 @@ def lib():
         L.rk_debug_mxfp8_mma_loop.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]
         L.rk_debug_wait_runs_out.restype = C.c_int
         L.rk_debug_wait_runs_out.argtypes = [C.c_int, C.c_int, C.c_void_p]
+        L.rk_debug_compact_wait_runs_out.restype = C.c_int
+        L.rk_debug_compact_wait_runs_out.argtypes = [C.c_int, C.c_int, C.c_void_p]
         L.rk_debug_set_prefill_form.restype = None
         L.rk_debug_set_prefill_form.argtypes = [C.c_int]
         L.rk_debug_prefill_form.restype = C.c_int

@@ -597,6 +597,12 @@ RK_API int rk_debug_wait_runs_out(int limit_us, int noalloc, void* stream) {
   return launch_wait_runs_out(limit_us, noalloc != 0, (cudaStream_t)stream);
 }
 
+/* The same for the waits that are bounded by a number of polls, with 1/64 of it: code 902, or 903 for the longer polls (`longer`).  With `aborted` the CTA's
+ * abort flag is set and the wait ends at once. */
+RK_API int rk_debug_compact_wait_runs_out(int longer, int aborted, void* stream) {
+  return launch_compact_wait_runs_out(longer != 0, aborted != 0, (cudaStream_t)stream);
+}
+
 /* Measurement hook (not in the public header): on every SM, `iters` back-to-back 128 x 128 x 128 block-scaled
  * MXFP8 products (four tcgen05.mma kind::mxf8f6f4 M=128 N=128 K=32 each) on one resident A tile and one resident
  * B tile of 16 KiB each (device pointers, 16-byte aligned, any valid E4M3 codes): the tensor-pipe ceiling for the

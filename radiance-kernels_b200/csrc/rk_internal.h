@@ -61,6 +61,7 @@ int launch_decode_noalloc(const rk_decode_args& a, cudaStream_t st);
 int noalloc_status_read_clear();                            // status word of the no-allocation decode path: read, then clear
 int launch_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile, int iters, cudaStream_t st);   // tensor-pipe ceiling probe
 int launch_wait_runs_out(int limit_us, bool noalloc, cudaStream_t st);   // test hook: a bounded wait that must give up
+int launch_compact_wait_runs_out(bool longer, bool aborted, cudaStream_t st);      // test hook: the same for the waits bounded by a number of polls
 extern int g_ring_stop;                                     // test hook: a role of the RoPE and RMSNorm kernels' rings of copies acts as if its wait had run out
 extern int g_decode_path;                                   // test hook: 0 = by shape, 1 = mma.sync kernel only
 bool decode_uses_tc(const rk_decode_args& a);                // true when the tcgen05 decode kernel serves this call

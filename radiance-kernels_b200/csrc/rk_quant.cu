@@ -332,9 +332,9 @@ RK_DEVINL bool rope_copies(const float* __restrict__ x, int copies, int d, int s
     mbar_arrive_expect_tx(bar, bytes);
     bulk_load_1d(ring.data + (n % kStages) * kTileBytes, x + ((int64_t)u * seq_len + p0) * d, bytes, bar);
   };
-  auto wait = [&](uint32_t n) -> bool {                       // at most 2^20 polls of up to 2 us
+  auto wait = [&](uint32_t n) -> bool {                       // bounded by 2^19 polls
 #pragma unroll 1
-    for (int it = 0; it < 1 << 20; ++it)
+    for (int it = 0; it < 1 << 19; ++it)
       if (mbar_try_wait<2000>(&ring.full[n % kStages], (n / kStages) & 1)) return true;
     return false;
   };
@@ -664,9 +664,9 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
   const int chain_warp = (int)(blockIdx.x / ((gridDim.x + kCtasPerSm - 1) / kCtasPerSm)) % kCtasPerSm;
   bool ok = true;
   int issued = 0;                                                       // pieces the producer has asked for
-  auto wait = [&](uint64_t* bar, int use) -> bool {                     // at most 2^20 polls of up to 2 us (a look at a flag of the other role's: 1-2 % of a call)
+  auto wait = [&](uint64_t* bar, int use) -> bool {                     // bounded by 2^19 polls, about two seconds (a look at a flag of the other role's: 1-2 % of a call)
 #pragma unroll 1
-    for (int it = 0; it < 1 << 20; ++it)
+    for (int it = 0; it < 1 << 19; ++it)
       if (mbar_try_wait<2000>(bar, use & 1)) return true;
     return false;
   };

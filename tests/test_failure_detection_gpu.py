@@ -49,6 +49,23 @@ def test_bounded_wait_runs_out_and_is_reported_and_clears():
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("longer", [0, 1])
+def test_waits_bounded_by_polls_run_out_after_about_two_seconds(longer):
+    """The waits of the prefill kernels that count polls instead of time, with 1/64 of the polls: they run out, and 64 times that lies between half a second
+    and five.  The CTA's abort flag ends them at once."""
+    L = rk.lib()
+    assert rk.last_device_status() == 0
+    for aborted in (0, 1):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        assert L.rk_debug_compact_wait_runs_out(longer, aborted, _stream()) == 0
+        e1.record()
+        torch.cuda.synchronize()
+        assert rk.last_device_status() == 902 + longer
+        seconds = e0.elapsed_time(e1) * 64 / 1000
+        assert seconds < 0.02 if aborted else 0.5 < seconds < 5.0, (aborted, seconds)
+
+
 @pytest.mark.parametrize("H,S,d,q_pos0,form", [(2, 300, 256, 0, 0), (160, 200, 256, -130, 0), (160, 100, 128, 0, TURNS), (160, 200, 64, -130, TURNS),
                                                (300, 300, 128, 0, PAIRS), (300, 200, 64, -130, PAIRS), (2, 300, 128, 0, SPLIT), (60, 200, 64, -130, SPLIT)])
 def test_prefill_writes_nothing_while_the_status_word_is_set(H, S, d, q_pos0, form):
