@@ -162,8 +162,10 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
   float l_run = 0.0f;      // this thread's share of the row sum, relative to it
   bool ok = true;
   // A wait for something that is there takes some 300 cycles where the scheduler's other softmax warps have exponentials queued, and a tile had four of them
-  // in a row, so what it needs is asked for ahead, without blocking, and waited for only where the answer was no: 16 heads of 8192 379 -> 369 us, capped
-  // 443 -> 436.  (O in two halves of 128 columns, each rescaled under the P V of the other: 396 and 466; the issuer, alone on its warp, then sets the pace.)
+  // in a row, so what it needs is asked for ahead, without blocking, and waited for only where the answer was no: 16 heads of 4096 106.7 -> 105.2 us, of 8192
+  // 379 -> 369; capped, 16 of 4096 125.4 -> 123.4.  With the cap not the maxima of the tile before, which by then have been there for a while: with them
+  // 124.7, and short calls 1-3 % slower than without any look ahead (4 heads of 100 8.97 -> 9.25, 2 x 16 of 1024 31.0 -> 31.7; now 8.89, 31.1).  (O in two halves of 128 columns, each rescaled under the P V of the other: 396 and 466; the issuer, alone on its warp, then sets the pace.)
+  constexpr bool kMaxAhead = !SOFTCAP;
   bool s_ready = false;
   int fail = 0;            // which wait gave up
 
@@ -191,9 +193,9 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     tmem_ld32(tmem_base + lane_addr + kColS + part * 64, reinterpret_cast<uint32_t*>(s));
     tmem_ld32(tmem_base + lane_addr + kColS + part * 64 + 32, reinterpret_cast<uint32_t*>(s) + 32);
     // Asked for here and used further down: the maxima of the tile before (the other group has left them half a tile ago), and whether the P buffer is free.
-    bool last_max = true, p_free = true;
+    bool last_max = j == 0, p_free = true;
     float m_last = NEG_INF;
-    if (j > 0) {
+    if (kMaxAhead && j > 0) {
       last_max = mbar_test_wait(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1);
       m_last = fmaxf(ld_shared_f32(&xchg[((t - 1) & 3) * 256]), ld_shared_f32(&xchg[((t - 1) & 3) * 256 + 128]));
     }
