@@ -794,11 +794,12 @@ static int effective_window(const rk_prefill_args& a) { return a.window > (int64
 //     19.9, 32 x 509 queries behind 3581 keys 37.7 32.1.  Up to three key tiles the time is that of code run for the first time, of which the other form has
 //     less: 42 heads of 300 7.7 8.1, 128 of 100 6.1 6.5.  With a cap of 50 1-5 % faster, but with one of 30, where the 64 keys of a half differ in tanh's form,
 //     8 of 2048 42.7 67.1, the chunk 72.0 129.
-//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  Without a mask, 8 KV heads of 2048 keys, by rounds of this
-//     kernel over rounds of pairs: 4 / 3 (192 heads of 384) 87.2 67.1, 3 / 2 (96 of 512) 65.8 51.0, 7 / 4 (192 of 640) 118.2 112.7, 2 (72 of 512) 36.2 35.5; call
-//     after call under the power cap 1.64 (8 x 64 of 640, 4096 keys) 609 604, 1.78 (4 x 64 of 1152, 4096 keys) 520 520, 1.82 (192 of 1920) 337 337, 1.875 (192
-//     of 1408) 246 250: up to 1.8.  Capped at 50, 4 / 3 123 109, 3 / 2 90.2 81.8, 5 / 3 (64 of 1408) 133.5 133.8, 7 / 4 169 184, 15 / 8 342 387, 2 49.1 55.9; at 30,
-//     3 / 2 215 203, 12 / 7 873 892, 15 / 8 1051 1088: up to 1.6.
+//   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  Time of this kernel over the pairs' by rounds of the one over
+//     rounds of the other, 500 calls of up to 20 rounds and 300 to 6000 keys, d of 64 and 128: without a cap 4 / 3 0.77, 3 / 2 0.78-0.95; from nine key tiles on
+//     7 / 4 0.90-0.95, 11 / 6 0.95-0.99 (call after call under the power cap 0.94-1.02), 13 / 7 0.97-0.99 (1.01), 15 / 8 0.98 (1.015), 2 0.99-1.11; of six to
+//     eight 7 / 4 0.98, 16 / 9 1.04-1.05; of up to five 3 / 2 0.95, 8 / 5 1.02, 7 / 4 1.01-1.02, 2 1.02-1.15 (an item costs 3600 cycles on top of its tiles here).
+//     With a cap of 50 and of 30 a key tile of one query tile is 0.57-0.6 of one of a pair: 3 / 2 0.79-1.0 and 0.84-0.98 (of up to five key tiles to 1.02 and 1.17),
+//     8 / 5 0.92 and 0.90, 18 / 11 1.03 and 0.95, 5 / 3 0.95-1.05 and 0.98-1.13, 7 / 4 1.01-1.11 and 0.85-1.28, 15 / 8 1.13 and 1.04.
 //   others (causal, a window): short items fill the rounds up, and there are twice as many of them.  11 heads of 2048 35.7 20.3, 16 36.1 22.9, 23 36.4 31.3,
 //     27 36.5 35.4; 24 heads of 1024 21.2 13.6, 37 21.5 16.9, 47 21.7 21.0; 144 of 300 16.3 14.9; 24 of 2048 with a window of 512 27.8 22.0; capped at 50 and at
 //     30, 24 heads of 1024 26.6 18.6 and 64.6 33.5, 27 of 2048 53.4 51.0 and 156 134.  (Above three tiles per SM, 31 of 2048 and 56 of 1024, 2-3 % slower.)
@@ -811,7 +812,11 @@ int prefill_form(const rk_prefill_args& a, int64_t sms) {
   const bool cap = a.softcap > 0.0f;
   if (tiles <= sms) return item_tiles > 3 && !cap ? kFormTurns : kFormSplit;
   const bool level = window == 0 && (!a.causal || 2 * ((int64_t)a.q_pos0 + kBlockM) > a.S_kv);
-  if (level) return 10 * ((tiles + sms - 1) / sms) < (cap ? 16 : 18) * ((pairs + sms - 1) / sms) ? kFormTurns : kFormPairs;
+  if (level) {
+    const int64_t single_rounds = (tiles + sms - 1) / sms, pair_rounds = (pairs + sms - 1) / sms;
+    const int limit = cap ? (kv_tiles <= 5 ? 149 : 160) : kv_tiles <= 5 ? 159 : kv_tiles <= 8 ? 176 : 184;       // hundredths
+    return 100 * single_rounds <= limit * pair_rounds ? kFormTurns : kFormPairs;
+  }
   return tiles <= 3 * sms ? kFormTurns : kFormPairs;
 }
 

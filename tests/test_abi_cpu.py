@@ -237,6 +237,9 @@ WIDE, PAIRS, TURNS, SPLIT = 0, 1, 2, 3
     (dict(H=192, S_q=384), TURNS), (dict(H=96, S_q=512), TURNS), (dict(H=192, S_q=640), TURNS), (dict(H=72, S_q=512), PAIRS), (dict(H=192, S_q=1408), PAIRS),
     (dict(H=192, S_q=384, softcap=50.0), TURNS), (dict(H=96, S_q=512, softcap=50.0), TURNS), (dict(H=64, S_q=1408, softcap=30.0), PAIRS),
     (dict(H=192, S_q=640, softcap=50.0), PAIRS), (dict(H=192, S_q=1408, softcap=50.0), PAIRS), (dict(H=192, S_q=1920, softcap=30.0), PAIRS),      # items of equal length
+    (dict(H=128, S_q=1024, S_kv=2300), TURNS), (dict(H=96, S_q=2048), TURNS), (dict(H=128, S_q=1024, S_kv=1000), TURNS), (dict(H=256, S_q=1152, S_kv=1000), PAIRS),
+    (dict(H=128, S_q=1152, S_kv=640), PAIRS), (dict(H=96, S_q=512, S_kv=640), TURNS),                               # by key tiles
+    (dict(H=128, S_q=1152, S_kv=1100, softcap=50.0), TURNS), (dict(H=96, S_q=512, S_kv=640, softcap=30.0), PAIRS), (dict(H=96, S_q=512, S_kv=641, softcap=30.0), TURNS),
     (dict(H=96, S_q=512, S_kv=4096, q_pos0=3584, causal=1, softcap=50.0), TURNS), (dict(H=192, S_q=640, S_kv=4096, q_pos0=3456, causal=1, softcap=50.0), PAIRS),
     (dict(H=24, S_q=2048, causal=1), TURNS), (dict(H=28, S_q=2048, causal=1), PAIRS), (dict(H=24, S_q=2048, causal=1, softcap=30.0), TURNS),
     (dict(H=16, S_q=1024, S_kv=1024, causal=1), TURNS), (dict(H=16, S_q=1024, S_kv=1024, causal=1, softcap=50.0), SPLIT), (dict(H=42, S_q=300, S_kv=300, causal=1), SPLIT),
