@@ -1526,12 +1526,12 @@ int launch_quantize_keys(const float* x, int64_t batch, int64_t rows, int64_t co
 // By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (8 heads of 16384 at d = 256 28.2 29.2;
 // chunks per SM, us, rows in registers and so: 2 768 7.2 7.6, 3 542 8.7 8.3, 5 191 12.1 11.1, 7 085 15.8 14.2, 14 170 30.7 27.8: one call behind another on the
 // same buffers; with nothing of them in L2 22.5 22.5 and 36.9 36.8).  A CTA's tile is a range of positions of one sequence, and the threads of the rows that the
-// last one lacks are idle: it pays where the tiles are three quarters full (some 8 M elements at d = 128, 16 rows a tile; sequences of 1 7.2 41.7, 4 8.3 14.0,
-// 8 8.3 8.9, 17 15.6 18.3, 33 15.0 15.3, 24 11.3 11.0, 49 11.8 11.2, 15 13.9 11.5).
+// last one lacks are idle, which shows least where HBM sets the pace.  130 shapes, this kernel's time over the other's by how full the tiles are: from 7 000 chunks
+// per SM on 0.72-1.0 0.74-0.98, 0.62-0.71 0.91-1.07, 0.53-0.56 1.03-1.17; below that 0.9-1.0 0.82-0.97, 0.75-0.9 0.95-1.11, sequences of 8, 4 and 1 rows in tiles of 16 1.08, 1.7 and 5.8.
 bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms) {
-  const int64_t copies = rows / seq_len, per_tile = ropec::kTileBytes / (d * 4);
-  if (copies < 16 || copies > 65535 || rows % seq_len != 0 || per_tile == 0 || rows * (d / 16) < sms * 3000) return false;
-  return 4 * seq_len >= 3 * ((seq_len + per_tile - 1) / per_tile) * per_tile;
+  const int64_t copies = rows / seq_len, per_tile = ropec::kTileBytes / (d * 4), chunks = rows * (d / 16);
+  if (copies < 16 || copies > 65535 || rows % seq_len != 0 || per_tile == 0 || chunks < sms * 3000) return false;
+  return 100 * seq_len >= (chunks < sms * 7000 ? 90 : 72) * ((seq_len + per_tile - 1) / per_tile * per_tile);
 }
 
 int launch_rope_quantize_rows(const float* x, int64_t rows, int d, const int32_t* pos, int seq_len, int pos0, const float* cos_h,

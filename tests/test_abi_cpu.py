@@ -221,7 +221,8 @@ def test_front_end_rejects_wrong_dtypes_and_shapes():
 
 
 @pytest.mark.parametrize("copies,seq_len,d,want", [(57344, 1, 128, 0), (30720, 2, 128, 0), (16384, 4, 128, 0), (8192, 8, 128, 0), (8192, 17, 128, 0), (4096, 33, 64, 0),
-                                                  (4096, 9, 256, 0), (8192, 5, 192, 0),                # tiles that would be a sixteenth to 0.69 full
+                                                  (4096, 9, 256, 0), (8192, 5, 192, 0), (5000, 33, 128, 0), (3840, 17, 256, 0),                # tiles that would be a sixteenth to 0.71 full
+                                                  (1968, 49, 128, 0), (1420, 28, 256, 0), (7200, 35, 128, 1), (4196, 76, 64, 1),      # 0.77 and 0.88 full in short calls, 0.73 and 0.79 in long ones
                                                   (8192, 15, 128, 1), (4096, 31, 128, 1), (2048, 47, 128, 1), (1024, 129, 128, 1), (64, 4096, 128, 1), (16, 4096, 128, 1),
                                                   (15, 8192, 128, 0), (16, 2000, 128, 0), (65536, 16, 128, 0)])
 def test_rope_goes_by_copies_where_its_tiles_are_full(copies, seq_len, d, want):
