@@ -200,7 +200,7 @@ constexpr uint32_t kPollsLong = 1u << 20, kPollsShort = 1u << 22;
 // The same in nine instructions, without a clock: bounded by the number of polls, which the hardware may hold for 2 us (LONG) and 0.5 us each, and does: with an
 // idle SM either form runs out after 2.15 s.  (A poll may come back sooner; the limit is then shorter, 2^20 or 2^22 polls of some 40 cycles at least.)  A kernel whose warps are in different
 // code all the time lives by the size of that code (an SM's instruction cache holds 32 KB): one query tile per CTA, d <= 128, 166 K instruction requests to the
-// next cache level in 38.9 us, 61 % of what it can serve.  With these waits there 73.3 -> 66.8 KB of code and 36.8 -> 35.9 us, 8 heads of 4096 42.0 -> 39.2.  In
+// next cache level in 38.9 us, 61 % of what it can serve.  With these waits there 73.3 -> 66.8 KB of code and 36.8 -> 35.6 us, 8 heads of 4096 42.3 -> 40.2.  In
 // all warps but the softmax's of pairs of query tiles, 2 x 16 heads of 4096 137.7 -> 134.1 us, 32 / 8 of 8192 455 -> 448 (in the softmax warps as well: 467).
 // Not at d = 256, whose long sequences lose: 16 / 8 heads of 8192 with a cap 957 -> 966, whichever of its warps wait so.
 template <bool LONG = false, uint32_t POLLS = LONG ? kPollsLong : kPollsShort>

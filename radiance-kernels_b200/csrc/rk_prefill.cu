@@ -792,7 +792,8 @@ static int effective_window(const rk_prefill_args& a) { return a.window > (int64
 // attention kernel alone on prepared operands, as many KV heads as heads where no other number is given; the pairs' kernel and this one):
 //   no more query tiles than SMs (both groups on every key tile, and this one): 8 / 32 heads of 512 9.0 8.3 / 9.5 9.2, 16 of 1024 14.0 12.8, 8 of 2048 23.4
 //     19.9, 32 x 509 queries behind 3581 keys 37.7 32.1.  Up to three key tiles the time is that of code run for the first time, of which the other form has
-//     less: 42 heads of 300 7.7 8.1, 128 of 100 6.1 6.5.  With a cap of 50 1-5 % faster, but with one of 30, where the 64 keys of a half differ in tanh's form,
+//     less: 42 heads of 300 7.7 8.1, 128 of 100 6.1 6.5; over 250 calls 1.00-1.12 of its time with one key tile, 0.88-1.05 with two and three, 0.79-0.96 with more.
+//     With a cap of 50 1-5 % faster, but with one of 30, where the 64 keys of a half differ in tanh's form,
 //     8 of 2048 42.7 67.1, the chunk 72.0 129.
 //   items of about the same length (no mask, or a long prefix): whole rounds of the SMs count.  Time of this kernel over the pairs' by rounds of the one over
 //     rounds of the other, 500 calls of up to 20 rounds and 300 to 6000 keys, d of 64 and 128: without a cap 4 / 3 0.77, 3 / 2 0.78-0.95; from nine key tiles on

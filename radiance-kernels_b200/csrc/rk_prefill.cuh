@@ -1,4 +1,4 @@
-// Definitions shared by the two prefill kernels (one 128-row query tile per CTA / two of them).
+// Definitions shared by the prefill kernels (d = 256; d <= 128: pairs of query tiles, and one at a time).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -13,8 +13,8 @@
 // What bounds a key tile of one query tile is the softmax of one thread's row, so two groups take key tiles in turn, half a tile apart: one forms
 // exponentials (special-function unit) while the other copies S and takes maxima.  All that goes from tile to tile is the running maximum, which a group
 // publishes as soon as it knows it.  S has a TMEM buffer per group, so that Q K^T is a tile ahead; O has one, and its chain from tile to tile -- P V,
-// rescale, P V -- is what sets the pace now: 1 650 cycles a key tile (450 the four MMAs, the rest a few hundred instructions of warps that run alone and
-// from cold instruction memory: 750 for the rescale, 250 and 300 to the issuer and back).  Without it the softmax groups would take 1 580, and alone on
+// rescale, P V -- is what sets the pace now: 1 650 cycles a key tile (450 the four MMAs, 750 the rescale, the other 450 the way to the issuer and back: a few
+// hundred instructions of warps that run alone and from cold instruction memory).  Without the rescale the softmax groups would take 1 580, and alone on
 // the SM 1 320.  (The P V issued by a correction warp: 2 700, its other waits then lie in the chain.  The rescale in chunks of 64 columns: spills, 1 830.)
 // Both groups on every key tile, 64 keys each, with an exchange of row maxima (rk_prefill2c.cu, the form for one query tile per CTA): 2 250.
 // 32 heads x 509 queries behind 3581 keys 42.1 -> 35.6 us, 8 heads of 4096 69.5 -> 40.2 (pairs of query tiles), 16 of 2048 40.7 -> 27.8.

@@ -27,7 +27,7 @@
 // warps are in their next tile.  With a CTA per pair an item of 16 tiles cost 17 000 cycles on top of them (start 4400, first loads,
 // a masked tile in cold code, the last tile of B alone, epilogue 3700): 8 x 16 heads of 4096 620 -> 518 us, 4 x 32 / 8 heads of
 // 8192 2030 -> 1764 us at full clock; call after call under the power cap 619 -> 555 and 2036 -> 1890.  Since the waits outside the softmax
-// warps are short in code (mbar_wait_compact) and the registers split as below, 536 and 1851 under the cap.
+// warps are short in code (mbar_wait_compact) and the registers split as below, 534 and 1838 under the cap (544 and 1857 before them on the same machine).
 //
 // SPLIT: one query tile per CTA and no second item, for grids that leave SMs idle and whose items are too short for rk_prefill1.cu, or capped.  A key
 // tile's time is then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work

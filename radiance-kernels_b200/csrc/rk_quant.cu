@@ -420,9 +420,9 @@ rope_quantize_copies_kernel(const float* __restrict__ x, int copies, int d, int 
 // bytes) gives eight lanes reading 16 bytes of their own rows eight different bank groups.  When the chains are done all
 // warps normalize and quantize; the input then comes from L2 (DRAM reads it once).  Over the whole kernel 53 % of the issue
 // slots and 22 % of DRAM's rate are used: the two phases of a CTA run one after the other, and neither fills the machine.
-// 8192 x 4096 bf16: 1362 us with one warp per 32 rows doing both passes from 4-byte shared-memory reads, 38.5 us this way, 33.4 by bulk copies (below).
+// 8192 x 4096 bf16: 1362 us with one warp per 32 rows doing both passes from 4-byte shared-memory reads, 36.5 us this way, 31.8 by bulk copies (below).
 namespace rms {
-constexpr int kThreads = 256, kWarps = kThreads / 32, kHelpers = 4, kCtasPerSm = 4;
+constexpr int kThreads = 256, kHelpers = 4, kCtasPerSm = 4;
 constexpr int kChunk = 256, kPitch = kChunk * 4 + 16, kBufs = 2;        // elements per chunk, bytes of a row of squares
 constexpr int kHalf = kChunk / 8;                                       // float4s of a row: first halves of the lanes' eight, then second
 constexpr int kMaxRows = 16;
@@ -635,7 +635,7 @@ rmsnorm_quantize_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int 
 // squares what it reads itself, and no other warp has anything to do with the rows until the chains are done.  A chain step takes 6 cycles (4.3 the addition
 // alone; squares and additions are in one instruction stream; fused multiply-adds, exact but for squares below 2^-133, 5.1), against 6.1 with one row and 10
 // with 8192 of them staged through other warps' registers and shared memory as squares, two barriers per 256 elements.
-// 8192 x 4096: 37.7 -> 33.4 us, about half of it the chains, half the quantization from L2 (67 MB in, 35 MB out).  The latter with one 32-byte load per
+// 8192 x 4096: 36.5 -> 31.8 us, about half of it the chains, half the quantization from L2 (67 MB in, 35 MB out).  The latter with one 32-byte load per
 // lane and row, one row ahead: two rows ahead 37.2, 16-byte loads two rows ahead 34.0.  Four CTAs of 256 threads 38.8, one of 1024 49.8.
 namespace rmb {
 constexpr int kThreads = 512, kCtasPerSm = 2, kMaxRows = 32, kStages = 3, kPieceBytes = 1024, kPitch = kPieceBytes + 16;      // pitch: eight lanes, eight bank groups
@@ -1457,9 +1457,10 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   if (rows == 0 || K == 0) return RK_OK;
   const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
-  // Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so: 4096 bf16 columns, 1 row 17.2 16.3, 600 rows 22.2 18.6,
-  // 8192 37.7 33.4; 12288 columns, 1500 rows 65.6 52.3; 2048 columns, 7 rows 9.9 9.8; 1024 columns, 64 rows 6.3 6.7, 9000 rows 13.5 12.1; 512 columns, 1000 rows 5.8
-  // 6.3), and not for fp32, whose 134 MB of 8192 x 4096 come from HBM twice either way (55.0 56.4; one row 17.4 20.3).
+  // Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so, one call behind another on the same buffers: 4096 bf16
+  // columns, 8192 rows 36.5 31.8, one 17.1 15.5; 12288 columns, 1500 rows 64.7 51.7; 2048 columns, 1 and 64 rows 9.0 9.2, 300 10.9 10.2, 4096 15.5 14.1, 16384 37.4
+  // 34.2; 1536 columns, 64 7.4 7.6, 300 8.7 8.3, 4096 12.3 11.6; 1024 columns, 64 5.8 6.0, 300 6.6 6.5, 4096 9.3 9.2, 9000 12.3 11.5; 512 columns 2-9 % slower
+  // throughout), and not for fp32, whose 134 MB of 8192 x 4096 come from HBM twice either way (55.0 56.4; one row 17.4 20.3).
   if (wide && bf16 && (K >= 2048 || (K >= 1024 && rows >= 4096))) {
     int* status = device_status_word();
     if (!status) return RK_ERR_NO_DEVICE;
@@ -1523,11 +1524,12 @@ int launch_quantize_keys(const float* x, int64_t batch, int64_t rows, int64_t co
   return RK_OK;
 }
 
-// By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (8 heads of 16384 at d = 256 28.2 29.2;
-// chunks per SM, us, rows in registers and so: 2 768 7.2 7.6, 3 542 8.7 8.3, 5 191 12.1 11.1, 7 085 15.8 14.2, 14 170 30.7 27.8: one call behind another on the
-// same buffers; with nothing of them in L2 22.5 22.5 and 36.9 36.8).  A CTA's tile is a range of positions of one sequence, and the threads of the rows that the
-// last one lacks are idle, which shows least where HBM sets the pace.  130 shapes, this kernel's time over the other's by how full the tiles are: from 7 000 chunks
-// per SM on 0.72-1.0 0.74-0.98, 0.62-0.71 0.91-1.07, 0.53-0.56 1.03-1.17; below that 0.9-1.0 0.82-0.97, 0.75-0.9 0.95-1.11, sequences of 8, 4 and 1 rows in tiles of 16 1.08, 1.7 and 5.8.
+// By bulk copies from where there are several tiles for each of two rounds of CTAs, and rows enough to share the caches (by chunks per SM, us, rows in
+// registers and so: 1 771 4.8 5.2, 3 542 8.3 7.2, 7 085 14.5 11.8, 14 170 28.9 27.8, 28 340 57.2 52.3, one call behind another on the same buffers; with nothing
+// of them in L2 the two are equal, 22.5 us and 36.9 at 7 085 and 14 170.  Eight copies: 3 542 8.3 7.4, 7 085 15.1 12.2, 14 170 28.1 29.4).
+// A CTA's tile is a range of positions of one sequence, and the threads of the rows that the last one lacks are idle, which shows least where HBM sets the
+// pace.  130 shapes, this kernel's time over the other's by how full the tiles are: from 7 000 chunks per SM on 0.72-1.0 0.74-0.98, 0.62-0.71 0.91-1.07, 0.53-0.56
+// 1.03-1.17; below that 0.9-1.0 0.82-0.97, 0.75-0.9 0.95-1.11, sequences of 8, 4 and 1 rows in tiles of 16 1.08, 1.7 and 5.8.
 bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms) {
   const int64_t copies = rows / seq_len, per_tile = ropec::kTileBytes / (d * 4), chunks = rows * (d / 16);
   if (copies < 16 || copies > 65535 || rows % seq_len != 0 || per_tile == 0 || chunks < sms * 3000) return false;
