@@ -97,4 +97,24 @@ int launch_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile, int iter
   return (int)cudaGetLastError();
 }
 
+// Test hook, beside no kernel that ships: one CTA waits on an mbarrier nobody arrives at, by the waits that count polls, with 1 / 64 of the polls; codes 902 and
+// 903.  aborted: the CTA's flag is set, and ends the wait at once.
+template <bool LONG>
+__global__ void compact_wait_runs_out_kernel(int* status, int aborted) {
+  __shared__ uint64_t bar;
+  __shared__ int abort_flag;
+  if (threadIdx.x == 0) { mbar_init(&bar, 1); abort_flag = aborted; fence_barrier_init(); }
+  __syncthreads();
+  if (threadIdx.x == 0 && !mbar_wait_compact<LONG, (LONG ? kPollsLong : kPollsShort) / 64>(&bar, 0, &abort_flag)) atomicCAS(status, 0, LONG ? 903 : 902);
+  __syncthreads();
+}
+
+int launch_compact_wait_runs_out(bool longer, bool aborted, cudaStream_t st) {
+  int* status = device_status_word();
+  if (!status) return RK_ERR_NO_DEVICE;
+  if (longer) compact_wait_runs_out_kernel<true><<<1, 32, 0, st>>>(status, aborted);
+  else compact_wait_runs_out_kernel<false><<<1, 32, 0, st>>>(status, aborted);
+  return (int)cudaGetLastError();
+}
+
 }  // namespace rk
