@@ -185,6 +185,15 @@ template <bool BF16IN> RK_DEVINL void widen8(const Raw8<BF16IN>& r, float (&v)[8
   }
 }
 
+// Pairs of fp32 in one 64-bit register.  (A product and a sum of pairs are contracted to one rounding, .rn or not: where both roundings count the products are scalar.)
+RK_DEVINL uint64_t pair_u32(uint32_t a, uint32_t b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
+RK_DEVINL uint64_t pair_f32(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+RK_DEVINL void unpair_u32(uint64_t p, uint32_t& a, uint32_t& b) { asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(p)); }
+RK_DEVINL void unpair_f32(uint64_t p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+RK_DEVINL uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+RK_DEVINL uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+RK_DEVINL uint64_t fma_sq_f32x2(uint64_t v, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(v), "l"(c)); return d; }
+
 // (Scalar products on purpose: mul.f32x2 takes two cycles of the heavy FMA pipe, and packing its operands adds moves.)
 // max(|a|, |b|, |c|), NaN if any of them is
 RK_DEVINL float max3_abs_nan(float a, float b, float c) { float d; asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
@@ -195,8 +204,8 @@ RK_DEVINL float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2
 // comparison tells): its codes are then those of the COLD form, which takes the maximum without the NaNs, as the
 // reference's compare loop does, and the integer encoder.  A caller runs the hot form over all it has and the cold one
 // again only if some block asked for it, so that the hot loop carries no code that never runs.
-// UNIT: no block scale (codes under 2^0, scale code 127).
-template <int FMT, bool UNIT, int N, bool COLD> RK_DEVINL bool quantize_lanes(const float (&v)[N][8], int lane, uint2 (&w)[N], uint32_t& scode) {
+// UNIT: no block scale (codes under 2^0, scale code 127).  PACKED: products two at a time, where issue slots are short (RMSNorm's segments kernel).
+template <int FMT, bool UNIT, int N, bool COLD, bool PACKED = false> RK_DEVINL bool quantize_lanes(const float (&v)[N][8], int lane, uint2 (&w)[N], uint32_t& scode) {
   constexpr int kLanes = 4 / N;
   const uint32_t mask = (0xFu >> (4 - kLanes)) << (lane & (32 - kLanes));
   float m = 0.0f;
@@ -216,7 +225,10 @@ template <int FMT, bool UNIT, int N, bool COLD> RK_DEVINL bool quantize_lanes(co
   for (int h = 0; h < N; ++h) {
     float s[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s[j] = __fmul_rn(v[h][j], p2);
+    for (int j = 0; j < 8; j += 2) {
+      if (PACKED) unpair_f32(mul_f32x2(pair_f32(v[h][j], v[h][j + 1]), pair_f32(p2, p2)), s[j], s[j + 1]);
+      else { s[j] = __fmul_rn(v[h][j], p2); s[j + 1] = __fmul_rn(v[h][j + 1], p2); }
+    }
     w[h] = COLD ? make_uint2(ref_encode4<FMT>(s[0], s[1], s[2], s[3]), ref_encode4<FMT>(s[4], s[5], s[6], s[7]))
                 : make_uint2(hw_encode4<FMT>(s[0], s[1], s[2], s[3]), hw_encode4<FMT>(s[4], s[5], s[6], s[7]));
   }
@@ -439,9 +451,18 @@ template <int ID> RK_DEVINL void named_arrive(int which) {
   else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"((1 + rms::kHelpers) * 32) : "memory");
 }
 
+constexpr int kPieceShared = 0;                                         // PIECE of rows that lie in shared memory
 template <bool BF16IN, int PIECE>
 RK_DEVINL void load_pair(Raw8<BF16IN> (&r)[2], const uint8_t* src, bool a32) {
-  if (BF16IN && PIECE == 16 && a32) {
+  if (PIECE == kPieceShared) {
+    constexpr int kQuads = BF16IN ? 1 : 2;
+#pragma unroll
+    for (int i = 0; i < 2 * kQuads; ++i) {
+      const uint4 q = reinterpret_cast<const uint4*>(src)[i];
+      uint32_t* w = r[i / kQuads].w + 4 * (i % kQuads);
+      w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+    }
+  } else if (BF16IN && PIECE == 16 && a32) {
     asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=r"(r[0].w[0]), "=r"(r[0].w[1]), "=r"(r[0].w[2]), "=r"(r[0].w[3]), "=r"(r[1].w[0]), "=r"(r[1].w[1]), "=r"(r[1].w[2]), "=r"(r[1].w[3]) : "l"(src));
   } else { r[0] = load_raw8<BF16IN, PIECE>(src); r[1] = load_raw8<BF16IN, PIECE>(src + 8 * (BF16IN ? 2 : 4)); }
@@ -732,6 +753,294 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
     return;
   }
   rmsnorm_rows<FMT, true, UNIT, 16, kThreads>(xr, row0, n_rows, K, gamma, rms_row, codes, scales, rmb_smem, kStages * kPitch);
+}
+
+// The same where every row is on the chip at once and few of them share an SM: the chain of a row is cut into segments that lanes walk side by side.
+// As long as an index-order sum stays in one binade [2^e, 2^(e+1)) with steps of u between its fp32 values, adding x >= 0 with round to nearest even
+// commutes with a shift of the sum by a multiple of 2u: what a segment adds depends only on whether the sum before it is an even or an odd multiple of u.
+// So each segment is added up twice, from 2^e and from 2^e + u, two segments of a lane side by side, and its result is the pair of gains in steps of u; runs
+// of segments of one binade compose to such a pair.  e comes from sums in another order, which are off by little: a segment whose guess may be wrong, or in
+// which the binade ends, is marked, as are those below 2^-87 (for bf16 the chains are fused multiply-adds: a square is exact in fp32, or below 2^-133 and
+// then no part of a sum of 2^-87 and more).  In the end one lane per row goes over the runs with the sum itself, asks of each run that the sum starts and ends in the
+// binade the gain was taken in -- sums only grow, so it has then been there all along -- and adds what is marked, or fails the question, in order as it lies.
+// Any input gives the bits of the index-order sum; a wrong guess costs time.  (N(0,1): a segment per doubling of the sum, 7 or 8 of the 103 of 4096 columns.)
+//
+// One row of 4096 bf16: 15.5 -> 7.3 us, 12288 columns 42.0 -> 9.8; 300 rows of 4096 17.4 -> 9.1, 1500 rows 20.1 -> 15.0.  With more rows on an SM than its shared memory holds the
+// rounds of CTAs follow one another with little overlap, and the ring above, whose chains all run at once, is faster (4500 rows 25.3, so 33.8).
+// The quantization reads the rows where they are; products two at a time (88 instead of 112 instructions per 16 elements and lane).
+namespace rms_seg {
+constexpr int kThreads = 256, kWarps = kThreads / 32, kCtasPerSm = 3, kMaxRows = 8;
+constexpr int kSmem = 227 * 1024, kStatic = 1024, kReserved = 1024;     // of an SM; of a CTA beside its dynamic part, ours and the system's
+constexpr uint32_t kMarked = 0x3FF;                                     // in the place of an exponent
+constexpr int kLongest = 72;                                            // elements of a segment
+
+// How a call is laid out: rows per CTA, warps that share a row's segments, segment in elements, bytes from row to row in shared memory.
+struct Shape { int rows, warps, seg, pitch; int64_t smem, grid; };
+// Segments are an odd number of 16-byte pieces, so that eight lanes reading 16 bytes of their own find eight bank groups.
+static Shape shape(int64_t n, int K, bool bf16, int rows) {
+  const int elem = bf16 ? 2 : 4, piece = 16 / elem, least = rows == 1 && !bf16 ? 24 : 40;      // shorter segments do not pay: more of them to go over in the end
+  Shape f;
+  f.rows = rows;
+  f.warps = 1;
+  while (f.warps * 2 * rows <= kWarps && (int64_t)f.warps * 64 * least < K) f.warps *= 2;
+  const int64_t lanes = (int64_t)64 * f.warps * ((K + (int64_t)64 * f.warps * kLongest - 1) / ((int64_t)64 * f.warps * kLongest));      // segments there is room for
+  f.seg = ((int)(((K + lanes - 1) / lanes + piece - 1) / piece) | 1) * piece;
+  const int n_seg = (K + f.seg - 1) / f.seg;
+  f.pitch = n_seg * f.seg * elem;
+  f.pitch += (f.pitch & 16) ? 0 : 16;
+  f.smem = (int64_t)rows * (f.pitch + (n_seg | 1) * 16 + (n_seg + 31) / 32 * 4) + f.seg * elem;
+  f.grid = (n + rows - 1) / rows;
+  return f;
+}
+// Where this kernel is the faster one (times per call, us, staged or by the ring and so): from more than 1024 columns on (512 3.9 4.8, 1024 5.5 5.2 to 9.0 9.8, 1536 7.2 5.5) as long
+// as all CTAs are on the SMs in one round, and in more rounds the longer the chain is that the others have to wait for (6144 columns 1500 rows 27.8 19.8, in two rounds 2200 rows
+// 29.4 32.2; 8192 columns in two rounds 1500 rows 35.6 23.7, in three 2200 37.6 37.4; 12288 columns 1500 rows 52.3 37.3).  fp32 from 1777 rows on, eight of them to a CTA, is
+// level (2048 columns, 2200 rows 16.4 16.7; 3000 17.8 17.7).
+static bool pays(int64_t n, int K, bool bf16, int64_t sms, Shape& f) {
+  if (K <= 1024 || K > (1 << 17)) return false;
+  f = shape(n, K, bf16, 1);
+  while (f.grid > sms * kCtasPerSm && f.rows < (bf16 ? kMaxRows : kMaxRows / 2)) {
+    const Shape two = shape(n, K, bf16, 2 * f.rows);
+    if (two.smem + kStatic / 2 + kReserved > kSmem / kCtasPerSm) break;
+    f = two;
+  }
+  const int64_t per_sm = std::min<int64_t>(kCtasPerSm, kSmem / (f.smem + kStatic / 2 + kReserved));
+  return per_sm > 0 && f.grid <= per_sm * sms * std::max(1, K / 4096);
+}
+}  // namespace rms_seg
+template <int FMT, bool BF16IN, bool UNIT, bool STOPS>
+__global__ void __launch_bounds__(rms_seg::kThreads, rms_seg::kCtasPerSm)
+rmsnorm_quantize_segments_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int rows_per_cta, int seg, int warps_per_row, int row_pitch,
+                                 const float* __restrict__ gamma, float eps, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int* status, int stop) {
+  using namespace rms_seg;
+  extern __shared__ __align__(16) uint8_t seg_smem[];                   // rows | a segment of zeros | segments' gains | ends of runs
+  __shared__ float rms_row[kMaxRows], warp_total[kWarps];
+  __shared__ uint64_t full[kMaxRows];
+  constexpr int kElem = BF16IN ? 2 : 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_seg = (K + seg - 1) / seg, seg_bytes = seg * kElem, gain_pitch = (n_seg | 1) * 16, masks = (n_seg + 31) / 32;
+  const int row_bytes = K * kElem;
+  uint8_t* const zeros = seg_smem + rows_per_cta * row_pitch;
+  uint8_t* const gains = zeros + seg_bytes;
+  uint32_t* const ends = reinterpret_cast<uint32_t*>(gains + rows_per_cta * gain_pitch);
+  const int64_t row0 = (int64_t)blockIdx.x * rows_per_cta;
+  const int n_rows = (int)min((int64_t)rows_per_cta, rows - row0);
+  if (threadIdx.x < n_rows) mbar_init(&full[threadIdx.x], 1);
+  fence_barrier_init();
+  for (int r = warp; r < n_rows; r += kWarps)                           // zeros from the end of a row to the end of its last segment
+    for (int i = row_bytes + lane * 16; i < n_seg * seg_bytes; i += 512) *reinterpret_cast<uint4*>(seg_smem + r * row_pitch + i) = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x * 16; i < seg_bytes; i += kThreads * 16) *reinterpret_cast<uint4*>(zeros + i) = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  grid_dependency_wait();
+  grid_dependents_launch();
+  const int asked = STOPS && stop == 2 ? n_rows / 2 : n_rows;           // test hook: the warp that asks for the rows stops half way
+  if (warp == 0 && lane < asked) {
+    mbar_arrive_expect_tx(&full[lane], (uint32_t)row_bytes);
+    bulk_load_1d(seg_smem + lane * row_pitch, x + (row0 + lane) * row_bytes, (uint32_t)row_bytes, &full[lane]);
+  }
+  auto wait = [&](uint64_t* bar) -> bool {                              // bounded by 2^19 polls, about two seconds
+#pragma unroll 1
+    for (int it = 0; it < 1 << 19; ++it)
+      if (mbar_try_wait<2000>(bar, 0)) return true;
+    return false;
+  };
+  // step(v, i) for the elements (bf16) or squares (fp32) of two segments, in order
+  auto walk = [&](const uint8_t* pa, const uint8_t* pb, auto&& step) {
+#pragma unroll 1
+    for (int j = 0; j < seg_bytes; j += 16) {
+      const uint4 qa = *reinterpret_cast<const uint4*>(pa + j), qb = *reinterpret_cast<const uint4*>(pb + j);
+      const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (BF16IN) {
+          step(pair_u32(wa[i] << 16, wb[i] << 16), 0);
+          step(pair_u32(wa[i] & 0xFFFF0000u, wb[i] & 0xFFFF0000u), 1);
+        } else {
+          const float fa = __uint_as_float(wa[i]), fb = __uint_as_float(wb[i]);
+          step(pair_f32(__fmul_rn(fa, fa), __fmul_rn(fb, fb)), i & 1);
+        }
+      }
+    }
+  };
+  auto add_square = [](uint64_t v, uint64_t c) { return BF16IN ? fma_sq_f32x2(v, c) : add_f32x2(c, v); };
+  const int part = warp % warps_per_row, n_groups = kWarps / warps_per_row;
+  const int per_part = ((n_seg + warps_per_row - 1) / warps_per_row + 63) / 64 * 64;   // segments of a warp, in groups of 64
+  bool ok = true;
+  for (int r0 = 0; r0 < n_rows; r0 += n_groups) {                       // (one pass where several warps share a row)
+    const int r = r0 + warp / warps_per_row;
+    const bool mine = r < n_rows;
+    const uint8_t* row = seg_smem + r * row_pitch;
+    if (mine && ok) ok = __all_sync(0xffffffffu, !(STOPS && stop == 1 && r >= n_rows / 2) && wait(&full[r]));
+    const bool go = mine && ok;
+    const int s_begin = part * per_part, s_end = min(n_seg, s_begin + per_part);
+    auto segment = [&](int s) -> const uint8_t* { return s < s_end ? row + s * seg_bytes : zeros; };
+    auto add_up = [&](int s0, float& sa, float& sb) {                   // about the sums of segments s0 + lane and s0 + 32 + lane
+      uint64_t s[2] = {0, 0};
+      walk(segment(s0 + lane), segment(s0 + 32 + lane), [&](uint64_t v, int which) { s[which] = add_square(v, s[which]); });
+      unpair_f32(add_f32x2(s[0], s[1]), sa, sb);
+    };
+    float carry = 0.0f;                                                 // about the sum of what lies before
+    if (warps_per_row > 1) {
+      float total = 0.0f;
+      if (go)
+        for (int s0 = s_begin; s0 < s_end; s0 += 64) { float sa, sb; add_up(s0, sa, sb); total += sa + sb; }
+#pragma unroll
+      for (int o = 16; o > 0; o /= 2) total += __shfl_xor_sync(0xffffffffu, total, o);
+      if (lane == 0) warp_total[warp] = total;
+      __syncthreads();
+      for (int w = warp - part; w < warp; ++w) carry += warp_total[w];
+    }
+    if (!go) continue;
+    for (int s0 = s_begin; s0 < s_end; s0 += 64) {
+      float sum[2], upto[2];
+      add_up(s0, sum[0], sum[1]);
+      upto[0] = sum[0];
+      upto[1] = sum[1];
+#pragma unroll
+      for (int o = 1; o < 32; o *= 2) {
+        const float ua = __shfl_up_sync(0xffffffffu, upto[0], o), ub = __shfl_up_sync(0xffffffffu, upto[1], o);
+        if (lane >= o) { upto[0] += ua; upto[1] += ub; }
+      }
+      const float all_a = __shfl_sync(0xffffffffu, upto[0], 31), all_b = __shfl_sync(0xffffffffu, upto[1], 31);
+      uint32_t e[2], even[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float end = (h ? carry + all_a : carry) + upto[h], begin = end - sum[h];
+        constexpr float kMargin = 1.0f / 8192;                          // more than the sums in two orders differ by
+        const uint32_t lo = __float_as_uint(begin * (1.0f - kMargin)) >> 23, hi = __float_as_uint(end * (1.0f + kMargin)) >> 23;
+        e[h] = sum[h] == 0.0f && begin == 0.0f ? 0u : lo == hi && lo >= 40 && lo < 255 ? lo : kMarked;
+        even[h] = (lo & 0xFFu) << 23;
+      }
+      carry += all_a + all_b;
+      uint64_t ce = pair_u32(even[0], even[1]), co = pair_u32(even[0] | 1u, even[1] | 1u);
+      walk(segment(s0 + lane), segment(s0 + 32 + lane), [&](uint64_t v, int) { ce = add_square(v, ce); co = add_square(v, co); });
+      uint32_t end_even[2], end_odd[2];
+      unpair_u32(ce, end_even[0], end_even[1]);
+      unpair_u32(co, end_odd[0], end_odd[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // A gain that leaves the binade does so from any start; kept small, the gains of 32 segments fit.
+        constexpr uint32_t kLeaves = 1u << 24;
+        uint32_t d0 = min(end_even[h] - even[h], kLeaves), d1 = min(end_odd[h] - (even[h] | 1u), kLeaves);
+        const uint32_t before = __shfl_up_sync(0xffffffffu, e[h], 1);
+        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || before != e[h] || e[h] == kMarked);
+        const int head = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {                               // gains from the head of the run to this segment
+          const uint32_t f0 = __shfl_up_sync(0xffffffffu, d0, o), f1 = __shfl_up_sync(0xffffffffu, d1, o);
+          if (lane - o >= head) {
+            const uint32_t g0 = d0, g1 = d1;
+            d0 = f0 + ((f0 & 1u) ? g1 : g0);
+            d1 = f1 + ((f1 & 1u) ? g0 : g1);
+          }
+        }
+        const int s = s0 + 32 * h + lane, n_here = min(32, s_end - s0 - 32 * h);
+        if (s < s_end) *reinterpret_cast<uint4*>(gains + r * gain_pitch + s * 16) = make_uint4(e[h], d0, d1, 0u);
+        if (lane == 0 && n_here > 0) ends[r * masks + (s >> 5)] = (heads >> 1) | (1u << (n_here - 1));
+      }
+    }
+  }
+  if (__syncthreads_or(!ok)) {
+    // the copies under way before shared memory goes to another CTA
+    for (int r = 0; r < asked; ++r) wait(&full[r]);
+    if (threadIdx.x == 0) atomicCAS(status, 0, 602);
+    return;
+  }
+  if (warp == 0) {
+    const int r = min(lane, n_rows - 1);
+    const uint8_t* row = seg_smem + r * row_pitch;
+    const uint4* gain = reinterpret_cast<const uint4*>(gains + r * gain_pitch);
+    float ss = 0.0f;
+    int i = 0, last = -1;                                               // segments that are in the sum; last segment of the next run
+    uint32_t left = ends[r * masks];
+    while (true) {
+      bool stuck = false;
+#pragma unroll 1
+      while (i < n_seg && !stuck) {
+        if (left == 0) left = ends[r * masks + (i >> 5)];
+        last = (i & ~31) + __ffs(left) - 1;
+        left &= left - 1;
+        const uint4 q = gain[last];
+        const uint32_t bits = __float_as_uint(ss), next = bits + ((bits & 1u) ? q.z : q.y);
+        stuck = (bits >> 23) != q.x || (next >> 23) != q.x;
+        if (!stuck) { ss = __uint_as_float(next); i = last + 1; }
+      }
+      if (__all_sync(0xffffffffu, i >= n_seg)) break;
+      if (stuck) {                                                      // segments i to last as they lie
+        const uint8_t* p = row + i * seg_bytes;
+        const int n = (last + 1 - i) * seg_bytes;
+        uint4 ahead = *reinterpret_cast<const uint4*>(p);
+#pragma unroll 1
+        for (int j = 16; j <= n; j += 16) {
+          const uint32_t w[4] = {ahead.x, ahead.y, ahead.z, ahead.w};
+          if (j < n) ahead = *reinterpret_cast<const uint4*>(p + j);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (BF16IN) {
+              const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
+              ss = __fadd_rn(ss, __fmul_rn(lo, lo));
+              ss = __fadd_rn(ss, __fmul_rn(hi, hi));
+            } else {
+              ss = __fadd_rn(ss, __fmul_rn(__uint_as_float(w[k]), __uint_as_float(w[k])));
+            }
+          }
+        }
+        i = last + 1;
+      }
+      __syncwarp();
+    }
+    if (lane < n_rows) rms_row[lane] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+  }
+  __syncthreads();
+  // y = (x rms) gamma, quantized: a warp keeps 512 columns (16 per lane, 2 lanes per block) and walks the rows; with fewer column units than warps several share one
+  const int units = (K + 511) / 512, parts = max(1, kWarps / units), first = warp / units;
+  uint8_t* const scale_bytes = gains;                                   // n_rows K / 32 bytes, less than the gains took
+  auto quantize_rows = [&](auto cold_tag) -> bool {
+    constexpr bool COLD = decltype(cold_tag)::value;
+    bool finite = true;
+    if (first >= parts) return finite;
+    for (int u = warp - first * units; u < units; u += kWarps) {
+      const int col = u * 512 + lane * 16;
+      if (col >= K) continue;                                           // whole 2-lane groups: K % 32 == 0
+      float g[2][8];
+      widen8<false>(load_raw8<false, 16>(reinterpret_cast<const uint8_t*>(gamma + col)), g[0]);
+      widen8<false>(load_raw8<false, 16>(reinterpret_cast<const uint8_t*>(gamma + col + 8)), g[1]);
+      const uint8_t* src = seg_smem + first * row_pitch + col * kElem;
+      uint8_t* dst = codes + (row0 + first) * K + col;
+      uint8_t* sdst = scale_bytes + first * (K / 32) + col / 32;
+#pragma unroll 1
+      for (int r = first; r < n_rows; r += parts) {
+        Raw8<BF16IN> raw[2];
+        load_pair<BF16IN, kPieceShared>(raw, src, false);
+        const float rms = rms_row[r];
+        float v[2][8];
+        widen8<BF16IN>(raw[0], v[0]);
+        widen8<BF16IN>(raw[1], v[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 8; j += 2)
+            unpair_f32(mul_f32x2(mul_f32x2(pair_f32(v[h][j], v[h][j + 1]), pair_f32(rms, rms)), pair_f32(g[h][j], g[h][j + 1])), v[h][j], v[h][j + 1]);
+        uint32_t scode;
+        uint2 w[2];
+        finite &= quantize_lanes<FMT, UNIT, 2, COLD, true>(v, lane, w, scode);
+        __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0].x, w[0].y, w[1].x, w[1].y));
+        if ((lane & 1) == 0) *sdst = (uint8_t)scode;
+        src += parts * row_pitch;
+        dst += (int64_t)parts * K;
+        sdst += parts * (K / 32);
+      }
+    }
+    return finite;
+  };
+  if (__syncthreads_or(!quantize_rows(std::false_type{}))) { quantize_rows(std::true_type{}); __syncthreads(); }
+  const int n = n_rows * (K / 32);                                      // contiguous in memory, as the CTA's rows are
+  uint8_t* out = scales + row0 * (K / 32);
+  if ((reinterpret_cast<uintptr_t>(out) & 3) == 0 && (n & 3) == 0) {
+    for (int i = threadIdx.x; i < n / 4; i += kThreads) reinterpret_cast<uint32_t*>(out)[i] = reinterpret_cast<const uint32_t*>(scale_bytes)[i];
+  } else {
+    for (int i = threadIdx.x; i < n; i += kThreads) out[i] = scale_bytes[i];
+  }
 }
 
 // Append one token to a KV cache: row pos[b] of every (batch, KV head) of K and of V is quantized (blocks of 32
@@ -1457,6 +1766,22 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   if (rows == 0 || K == 0) return RK_OK;
   const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
+  rms_seg::Shape f;
+  if (wide && rms_seg::pays(rows, K, bf16, num_sms(), f)) {
+    int* status = device_status_word();
+    if (!status) return RK_ERR_NO_DEVICE;
+#define RK_RN(BF, UN) RK_DISPATCH_FMT(fmt, {                                                                                \
+    auto kern = F == RK_FMT_E4M3 && BF && !UN && g_ring_stop ? rmsnorm_quantize_segments_kernel<RK_FMT_E4M3, true, false, true> : rmsnorm_quantize_segments_kernel<F, BF, UN, false>; \
+    if (f.smem + rms_seg::kStatic > 48 * 1024) {                                                                           \
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, rms_seg::kSmem - rms_seg::kStatic); \
+      if (e != cudaSuccess) return (int)e;                                                                                 \
+    }                                                                                                                      \
+    return (int)launch_pdl(kern, dim3((unsigned)f.grid), dim3(rms_seg::kThreads), (size_t)f.smem, st, reinterpret_cast<const uint8_t*>(x), rows, K, f.rows, f.seg, f.warps, f.pitch, gamma, eps, codes, scales, status, g_ring_stop); \
+  })
+    if (bf16) { if (unit_scale) { RK_RN(true, true); } else { RK_RN(true, false); } }
+    else      { if (unit_scale) { RK_RN(false, true); } else { RK_RN(false, false); } }
+#undef RK_RN
+  }
   // Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so, one call behind another on the same buffers: 4096 bf16
   // columns, 8192 rows 36.5 31.8, one 17.1 15.5; 12288 columns, 1500 rows 64.7 51.7; 2048 columns, 1 and 64 rows 9.0 9.2, 300 10.9 10.2, 4096 15.5 14.1, 16384 37.4
   // 34.2; 1536 columns, 64 7.4 7.6, 300 8.7 8.3, 4096 12.3 11.6; 1024 columns, 64 5.8 6.0, 300 6.6 6.5, 4096 9.3 9.2, 9000 12.3 11.5; 512 columns 2-9 % slower

@@ -148,6 +148,26 @@ def test_a_ring_of_copies_that_gives_up_ends_the_call_and_the_next_one_is_whole(
     assert rk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("role", [1, 2])
+def test_the_ring_of_a_large_rmsnorm_call_that_gives_up(role):
+    """The same for RMSNorm calls of more rows than lie on the chip at once (the test above has fewer, which come in one copy each)."""
+    L = rk.lib()
+    g = torch.Generator(device="cuda").manual_seed(96)
+    x, gamma = torch.randn(4500, 4096, generator=g, device="cuda").bfloat16(), torch.rand(4096, generator=g, device="cuda") + 0.5
+    want = rk.rmsnorm_mx_quantize(x, gamma, 1e-5)
+    L.rk_debug_set_ring_stop(role)
+    try:
+        rk.rmsnorm_mx_quantize(x, gamma, 1e-5)
+        torch.cuda.synchronize()
+    finally:
+        L.rk_debug_set_ring_stop(0)
+        status = rk.last_device_status()
+    assert status == 602
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(rk.rmsnorm_mx_quantize(x, gamma, 1e-5), want))
+    assert rk.last_device_status() == 0
+
+
 def test_noalloc_decode_status_word_is_observable():
     L = rk.lib()
     g = torch.Generator(device="cuda").manual_seed(91)

@@ -110,3 +110,37 @@ def test_bf16_rows_by_bulk_copy(rows, K, fmt, unit):
         got_c[9:11] &= ~np.uint8(sign)
         want_c[9:11] &= ~np.uint8(sign)
     assert np.array_equal(got_c, want_c)
+
+
+@pytest.mark.parametrize("rows,K,bf16,fmt,unit", [(1, 1056, True, 0, False), (1, 4096, False, 0, True), (37, 4128, True, 0, False), (445, 2080, False, 1, False), (889, 1536, True, 0, False),
+                                                  (1777, 1792, True, 2, False), (3552, 1056, True, 0, False), (900, 8224, True, 4, False), (30, 12288, False, 3, False),
+                                                  (12, 50016, True, 0, False), (12, 50016, False, 0, False)])
+def test_chains_cut_into_segments(rows, K, bf16, fmt, unit):
+    """Rows whose index-order sums are taken by segments: one to eight of them to a CTA, segments of a warp and of several, ragged last segments.  Sums that
+    stay in a binade for long, cross several in one segment, start late, tie at nearly every addition, cannot be guessed (the share of one value), overflow or hold a NaN."""
+    rng = np.random.default_rng(rows + K)
+    x = (rng.standard_normal((rows, K)) * np.exp2(rng.integers(-6, 7, (rows, 1)))).astype(np.float32)
+    ramp = np.exp2(np.linspace(-40, 40, K)).astype(np.float32)
+    forms = [lambda v: 0 * v, lambda v: v * 2.0 ** -70, lambda v: v * 2.0 ** -45, lambda v: v * ramp, lambda v: v * ramp[::-1], lambda v: np.sign(v), lambda v: np.sign(v) * 1.5,
+             lambda v: np.where(np.arange(K) < K // 2, 0, v), lambda v: np.where(np.arange(K) % 97, v * 2.0 ** -30, v), lambda v: np.where(np.arange(K) == K // 3, 3.0e4, v),
+             lambda v: np.where(np.arange(K) % 3, v, v * 2.0 ** 62), lambda v: np.round(v * 4) / 4]
+    for i, f in enumerate(forms):
+        if i < rows:
+            x[i * (rows // min(rows, len(forms)))] = f(x[i * (rows // min(rows, len(forms)))])
+    if rows > 30:
+        x[rows - 2, K - 40] = np.inf
+        x[rows - 1, 17] = np.nan
+    gamma = (0.75 + 0.5 * rng.random(K)).astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    xt = xt.bfloat16() if bf16 else xt
+    want_c, want_s = _expect(np_(xt.float()), gamma, 1e-5, fmt, unit)
+    c, s = rk.rmsnorm_mx_quantize(xt, torch.from_numpy(gamma).cuda(), 1e-5, fmt=fmt, unit_scale=unit)
+    torch.cuda.synchronize()
+    assert rk.last_device_status() == 0
+    got_c = np_(c).copy()
+    if rows > 30:                                      # signs of NaN: as in the test above
+        sign = (0x80, 0x80, 0x20, 0x20, 0x08)[fmt]
+        got_c[-2:] &= ~np.uint8(sign)
+        want_c[-2:] &= ~np.uint8(sign)
+    assert np.array_equal(np_(s), want_s)
+    assert np.array_equal(got_c, want_c)
