@@ -204,7 +204,8 @@ RK_DEVINL float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2
 // comparison tells): its codes are then those of the COLD form, which takes the maximum without the NaNs, as the
 // reference's compare loop does, and the integer encoder.  A caller runs the hot form over all it has and the cold one
 // again only if some block asked for it, so that the hot loop carries no code that never runs.
-// UNIT: no block scale (codes under 2^0, scale code 127).  PACKED: products two at a time, where issue slots are short (RMSNorm's segments kernel).
+// UNIT: no block scale (codes under 2^0, scale code 127).  PACKED: products two at a time, where issue slots are short (RMSNorm: 16384 x 4064 bf16
+// 68.6 -> 67.2 us, 8192 x 4096 fp32 50.4 -> 49.6).
 template <int FMT, bool UNIT, int N, bool COLD, bool PACKED = false> RK_DEVINL bool quantize_lanes(const float (&v)[N][8], int lane, uint2 (&w)[N], uint32_t& scode) {
   constexpr int kLanes = 4 / N;
   const uint32_t mask = (0xFu >> (4 - kLanes)) << (lane & (32 - kLanes));
@@ -511,10 +512,11 @@ RK_DEVINL void rmsnorm_rows(const uint8_t* __restrict__ xr, int64_t row0, int n_
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[h][j] = __fmul_rn(__fmul_rn(v[h][j], rms), g[h][j]);
+          for (int j = 0; j < 8; j += 2)
+            unpair_f32(mul_f32x2(mul_f32x2(pair_f32(v[h][j], v[h][j + 1]), pair_f32(rms, rms)), pair_f32(g[h][j], g[h][j + 1])), v[h][j], v[h][j + 1]);
         uint32_t scode;
         uint2 w[2];
-        finite &= quantize_lanes<FMT, UNIT, 2, COLD>(v, lane, w, scode);
+        finite &= quantize_lanes<FMT, UNIT, 2, COLD, true>(v, lane, w, scode);
         __stcs(reinterpret_cast<uint4*>(dst), make_uint4(w[0].x, w[0].y, w[1].x, w[1].y));
         if ((lane & 1) == 0) *sdst = (uint8_t)scode;
         dst += dst_step;
@@ -653,10 +655,13 @@ rmsnorm_quantize_kernel(const uint8_t* __restrict__ x, int64_t rows, int K, int 
 }
 
 // The same for bf16 rows, which come by bulk copies, a warp's lanes each asking for one row's next 1024 bytes; the chain warp, up to 32 rows of it in lanes,
-// squares what it reads itself, and no other warp has anything to do with the rows until the chains are done.  A chain step takes 6 cycles (4.3 the addition
-// alone; squares and additions are in one instruction stream; fused multiply-adds, exact but for squares below 2^-133, 5.1), against 6.1 with one row and 10
-// with 8192 of them staged through other warps' registers and shared memory as squares, two barriers per 256 elements.
-// 8192 x 4096: 36.5 -> 31.8 us, about half of it the chains, half the quantization from L2 (67 MB in, 35 MB out).  The latter with one 32-byte load per
+// squares what it reads itself, and no other warp has anything to do with the rows until the chains are done.  A chain step takes 5.1 cycles as a fused
+// multiply-add (4.3 the addition alone), 6 as a product and a sum in one instruction stream, against 6.1 with one row and 10 with 8192 of them staged through
+// other warps' registers and shared memory as squares, two barriers per 256 elements.  The square of a bf16 is exact in fp32, so fusing changes nothing, unless
+// it is below 2^-133; where the first element of every row is 2^-50 or more, such a square is less than half a step of any sum and adds nothing
+// either way.  Other rows (that begin with a zero, say) keep products and sums.  16384 x 4064: 67.2 -> 66.1 us, 16384 x 2048 36.5 -> 35.8.
+// 8192 x 4096: 36.5 -> 31.8 us (inputs that change from call to call 34.5, fused 33.7), about half of it the chains, half the quantization from L2 (67 MB in, 35 MB out). The
+// pieces that are still in shared memory read from there: no change.  The quantization with one 32-byte load per
 // lane and row, one row ahead: two rows ahead 37.2, 16-byte loads two rows ahead 34.0.  Four CTAs of 256 threads 38.8, one of 1024 49.8.
 namespace rmb {
 constexpr int kThreads = 512, kCtasPerSm = 2, kMaxRows = 32, kStages = 3, kPieceBytes = 1024, kPitch = kPieceBytes + 16;      // pitch: eight lanes, eight bank groups
@@ -694,41 +699,48 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
   auto stops = [&](int role, int c) { return STOPS && stop == role && c == kStages + 1; };      // test hook: the role acts as if its wait had run out
   if (warp == chain_warp) {
     float ss = 0.0f;
+    // elements 8 i to 8 (i + n16) of a piece, as products and sums or as fused multiply-adds
+    auto add_piece = [&](const uint4* src, int n16, auto fused_tag) {
+      constexpr bool kFused = decltype(fused_tag)::value;
+      constexpr int kSq = 16 / kElem;                                   // elements of 16 bytes
+      auto widen = [&](const uint4& q, float (&d)[kSq]) {
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xFFFF0000u);
+          d[2 * j] = kFused ? lo : __fmul_rn(lo, lo);
+          d[2 * j + 1] = kFused ? hi : __fmul_rn(hi, hi);
+        }
+      };
+      auto chain = [&](const float (&d)[kSq]) {
+#pragma unroll
+        for (int j = 0; j < kSq; ++j) ss = kFused ? __fmaf_rn(d[j], d[j], ss) : __fadd_rn(ss, d[j]);
+      };
+      uint4 q[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = src[k];
+      float d[2][kSq];
+      widen(q[0], d[0]);
+#pragma unroll 1
+      for (int i = 0; i < n16; i += 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {                                   // elements a piece of 16 bytes ahead, loads four
+          if (i + k + 4 < n16) q[k] = src[i + k + 4];
+          widen(q[(k + 1) & 3], d[(k + 1) & 1]);
+          chain(d[k & 1]);
+        }
+      }
+    };
+    bool fused = false;
     for (int c = 0; c < n_pieces && ok; ++c) {
       const int st = c % kStages;
       ok = __all_sync(0xffffffffu, !stops(1, c) && wait(&full[st], c / kStages));
       if (!ok) break;
+      const uint4* src = reinterpret_cast<const uint4*>(rmb_smem + st * stage_bytes + lane * kPitch);
+      if (c == 0) fused = __all_sync(0xffffffffu, lane >= n_rows || (src[0].x & 0x7FFFu) >= (127u - 50u) << 7);
       if (lane < n_rows) {
-        const uint4* src = reinterpret_cast<const uint4*>(rmb_smem + st * stage_bytes + lane * kPitch);
         const int n16 = (int)min((int64_t)kPieceBytes, row_bytes - (int64_t)c * kPieceBytes) / 16;      // a multiple of 4
-        constexpr int kSq = 16 / kElem;                                 // elements of 16 bytes
-        auto square = [&](const uint4& q, float (&d)[kSq]) {
-          const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xFFFF0000u);
-            d[2 * j] = __fmul_rn(lo, lo);
-            d[2 * j + 1] = __fmul_rn(hi, hi);
-          }
-        };
-        auto chain = [&](const float (&d)[kSq]) {
-#pragma unroll
-          for (int j = 0; j < kSq; ++j) ss = __fadd_rn(ss, d[j]);
-        };
-        uint4 q[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = src[k];
-        float sq[2][kSq];
-        square(q[0], sq[0]);
-#pragma unroll 1
-        for (int i = 0; i < n16; i += 4) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {                                 // squares a piece of 16 bytes ahead, loads four
-            if (i + k + 4 < n16) q[k] = src[i + k + 4];
-            square(q[(k + 1) & 3], sq[(k + 1) & 1]);
-            chain(sq[k & 1]);
-          }
-        }
+        if (fused) add_piece(src, n16, std::true_type{}); else add_piece(src, n16, std::false_type{});
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[st]);

@@ -144,3 +144,20 @@ def test_chains_cut_into_segments(rows, K, bf16, fmt, unit):
         want_c[-2:] &= ~np.uint8(sign)
     assert np.array_equal(np_(s), want_s)
     assert np.array_equal(got_c, want_c)
+
+
+@pytest.mark.parametrize("rows,K,first", [(4500, 2048, 1.0), (4500, 2048, 0.0), (4500, 4096, 2.0 ** -50), (4500, 2080, 2.0 ** -51)])
+def test_fused_chains_of_large_calls(rows, K, first):
+    """Rows that begin with an element from which on a fused multiply-add gives the bits of a product and a sum, and rows that do not: beside elements whose
+    squares round to subnormal numbers, and sums that stay small."""
+    rng = np.random.default_rng(rows + K)
+    x = rng.standard_normal((rows, K)).astype(np.float32)
+    x[::3] *= np.exp2(rng.integers(-75, -45, (rows, K)))[::3]
+    x[:, 0] = first
+    gamma = (0.75 + 0.5 * rng.random(K)).astype(np.float32)
+    xt = torch.from_numpy(x).cuda().bfloat16()
+    want_c, want_s = _expect(np_(xt.float()), gamma, 1e-30, 0, False)
+    c, s = rk.rmsnorm_mx_quantize(xt, torch.from_numpy(gamma).cuda(), 1e-30)
+    torch.cuda.synchronize()
+    assert np.array_equal(np_(s), want_s)
+    assert np.array_equal(np_(c), want_c)
