@@ -447,7 +447,8 @@ namespace rk {
 // The kernel is a chain of memory latencies on top of the main kernel's end (7.4 us of a 23 us step when it read the status,
 // the length, the unit's first tile, the maxima and the rows one after the other, 40 us for 148 partials).  Which partials it
 // needs depends on kv_len alone, which nothing still running writes (the main kernel lets this one start only after its own
-// wait), so that is worked out before the wait; after it the maxima and the rows of a warp's first partials load together.
+// wait), so that is worked out before the wait, the rows' places included; after it the status, the maxima and the rows of a warp's first partials load together
+// (the status after them, as it was, and 64-bit places in the loop: one sequence of 6000 keys 0.3 us more, 8 of 4096 keys with 64 heads 0.4).
 constexpr int kCombineWarps = 8;
 __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(const DecodeTcParams p, int main_grid) {
   constexpr int kBatch = 4;                                        // partials of a warp in flight
@@ -476,10 +477,16 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
     c0 = (int)(((first + 1) * ranges - 1) / total);                // the CTA whose range holds a tile
     n = (int)(((first + n_unit) * ranges - 1) / total) - c0 + 1;
   }
-  auto at = [&](int i) -> size_t { return p.nsplit > 0 ? (size_t)bh * p.nsplit + i : ((size_t)(c0 + i) * 2 + (i == 0 ? 1 : 0)) * p.grp + hg; };
+  // Partial i is row first_row + skip + i step of part_ml and part_o (i = 0 without the skip: a unit's first CTA leaves it in its slot 1, the others in slot 0).
+  // (fewer than 2^31: 130 floats each)
+  const uint32_t first_row = p.nsplit > 0 ? (uint32_t)bh * p.nsplit : ((uint32_t)c0 * 2 + 1) * p.grp + hg;
+  const int step = p.nsplit > 0 ? 1 : 2 * p.grp, skip = p.nsplit > 0 ? 0 : -p.grp;
+  const float2* const part_ml = reinterpret_cast<const float2*>(p.part_ml);
+  const float4* const part_o = reinterpret_cast<const float4*>(p.part_o) + lane;
   grid_dependency_wait();
   grid_dependents_launch();
   if (n == 1) return;
+  const int stopped = tid == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0;     // the partials are not all there (asked for with them: one latency, not two)
   float m = NEG_INF, l = 0.0f;                                     // of this warp's partials
   float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   for (int i0 = warp; i0 < n; i0 += kBatch * kCombineWarps) {
@@ -491,8 +498,9 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
       ml[k] = make_float2(NEG_INF, 0.0f);
       row[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (i < n) {
-        ml[k] = __ldcg(reinterpret_cast<const float2*>(p.part_ml) + at(i));
-        row[k] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at(i) * 128) + lane);
+        const uint32_t w = first_row + (uint32_t)(i == 0 ? 0 : skip + i * step);
+        ml[k] = __ldcg(part_ml + w);
+        row[k] = __ldcg(part_o + (size_t)w * 32);
       }
     }
     float top = m;
@@ -511,7 +519,6 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_tc_combine_kernel(c
   }
   acc_sm[warp][lane] = acc;
   if (lane == 0) ml_sm[warp] = make_float2(m, l);
-  const int stopped = tid == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0;     // the partials are not all there
   if (__syncthreads_or(stopped) || warp != 0) return;
   float top = NEG_INF;
 #pragma unroll
