@@ -186,10 +186,16 @@ struct DtcSegments {
       return;
     }
     const int len0 = lane < p.B ? dtc_len(p, lane) : 0;           // the first 32 lengths are read once (a load is 0.4 us here)
-    total = dtc_tiles(len0);
-    for (int i = lane + 32; i < p.B; i += 32) total += dtc_tiles(dtc_len(p, i));
+    const int tiles0 = dtc_tiles(len0);
+    int incl0 = tiles0;                                            // of those, up to and with this lane's; their total comes with it (a reduction of its own: 0.15 us a call)
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
+    for (int s = 1; s < 32; s <<= 1) { const int o = __shfl_up_sync(0xffffffffu, incl0, s); if (lane >= s) incl0 += o; }
+    if (p.B > 32) {
+      for (int i = lane + 32; i < p.B; i += 32) total += dtc_tiles(dtc_len(p, i));
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
+    }
+    total += __shfl_sync(0xffffffffu, incl0, 31);
     total *= p.H_kv;
     const int g = dtc_ranges(total, gridDim.x), c = min((int)blockIdx.x, g);
     first = dtc_first(total, c, g);
@@ -199,10 +205,13 @@ struct DtcSegments {
     int base = 0;                                              // tiles of the sequences before this block of 32
     for (int i0 = 0;; i0 += 32) {
       const int my_len = i0 == 0 ? len0 : i0 + lane < p.B ? dtc_len(p, i0 + lane) : 0;
-      const int mine = dtc_tiles(my_len) * p.H_kv;
-      int incl = mine;
+      const int mine = (i0 == 0 ? tiles0 : dtc_tiles(my_len)) * p.H_kv;
+      int incl = incl0 * p.H_kv;
+      if (i0 > 0) {
+        incl = mine;
 #pragma unroll
-      for (int s = 1; s < 32; s <<= 1) { const int o = __shfl_up_sync(0xffffffffu, incl, s); if (lane >= s) incl += o; }
+        for (int s = 1; s < 32; s <<= 1) { const int o = __shfl_up_sync(0xffffffffu, incl, s); if (lane >= s) incl += o; }
+      }
       const uint32_t past = __ballot_sync(0xffffffffu, base + incl > first);
       if (past) {
         const int w = __ffs(past) - 1;
