@@ -195,15 +195,14 @@ __device__ __forceinline__ bool softmax_rows(const PrefillParams& p, uint8_t* sm
     // Asked for here and used further down: the maxima of the tile before (the other group has left them half a tile ago), and whether the P buffer is free.
     bool last_max = j == 0, p_free = true;
     float m_last = NEG_INF;
-    if (kMaxAhead && j > 0) {
-      last_max = mbar_test_wait(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1);
-      m_last = fmaxf(ld_shared_f32(&xchg[((t - 1) & 3) * 256]), ld_shared_f32(&xchg[((t - 1) & 3) * 256 + 128]));
-    }
+    if (kMaxAhead && j > 0) last_max = mbar_test_wait(&bars.row_bar[((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1);
     if (t >= 2) p_free = mbar_test_wait(&bars.pv_done[grp], ((t - 2) >> 1) & 1);
     tc_wait_ld();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bars.s_empty);                 // one arrival per warp: the next Q K^T may have S once all 8 have read
+    if (kMaxAhead && j > 0)
+      m_last = fmaxf(ld_shared_f32_if(last_max, &xchg[((t - 1) & 3) * 256], NEG_INF), ld_shared_f32_if(last_max, &xchg[((t - 1) & 3) * 256 + 128], NEG_INF));
     if (DUMP && p.dbg && qt == p.n_q_tiles - 1 && bh == 0 && j == 0) {
 #pragma unroll
       for (int c = 0; c < 64; ++c) p.dbg[row * 128 + part * 64 + c] = s[c];

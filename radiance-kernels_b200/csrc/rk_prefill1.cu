@@ -245,7 +245,6 @@ __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p,
     if (t >= kPBufs && !mbar_wait_compact(&bars[bPV + (t & 3)], ((t >> 2) - 1) & 1, abort_flag)) code = 102;
     else if (kMaxAhead && j > 0) {
       if (!mbar_wait_compact(&bars[bMX + ((t - 1) & 3) * 4 + quad], ((t - 1) >> 2) & 1, abort_flag)) code = 106;
-      m_run = ld_shared_f32(&row_max[((t - 1) & 3) * 128 + row]);
     }
     return __any_sync(0xffffffffu, code != 0) ? (code ? code : 102) : 0;
   };
@@ -260,6 +259,9 @@ __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p,
       if (!fail) fail = wait_rest(j);
       if (fail) return false;
     }
+    // Here, behind the vote on the answers, and not beside the test at the end of the tile before: a load that does not depend on the answer can be served before the test is, and
+    // bring the maximum of four tiles ago beside a yes.
+    if (kMaxAhead && j > 0) m_run = ld_shared_f32(&row_max[((t - 1) & 3) * 128 + row]);
     tc_fence_after();
     if (stamp) RK_STAMP(grp, j, 1);
 
@@ -324,7 +326,6 @@ __device__ __forceinline__ bool softmax_every_other_tile(const PrefillParams& p,
     if (ready) {
       const bool r0 = mbar_test_wait(s_full, ((t + 2) >> 1) & 1), r1 = t + 2 < kPBufs || mbar_test_wait(&bars[bPV + ((t + 2) & 3)], (((t + 2) >> 2) - 1) & 1),
                  r2 = !kMaxAhead || mbar_test_wait(&bars[bMX + ((t + 1) & 3) * 4 + quad], ((t + 1) >> 2) & 1);
-      if (kMaxAhead) m_run = ld_shared_f32(&row_max[((t + 1) & 3) * 128 + row]);
       ready = r0 && r1 && r2;
     }
     if (stamp) RK_STAMP(grp, j, 4);
