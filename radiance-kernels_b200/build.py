@@ -16,7 +16,7 @@ import sysconfig
 HERE = pathlib.Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 SOURCES = ["rk_api.cu", "rk_quant.cu", "rk_prefill.cu", "rk_prefill1.cu", "rk_prefill2c.cu", "rk_peak.cu", "rk_mxgemm.cu", "rk_decode.cu"]
-HEADERS = ["rk_common.cuh", "rk_internal.h", "rk_prefill.cuh", "rk_decode_tc.cuh"]
+HEADERS = ["rk_common.cuh", "rk_internal.h", "rk_rebase.cuh", "rk_prefill.cuh", "rk_decode_tc.cuh"]
 LIB = HERE / "librk_mx_attn.so"
 FRONT_SRC = CSRC / "rk_front.cpp"
 FRONT = HERE / "_rk_front.so"

@@ -96,6 +96,12 @@ template <int FMT> RK_DEVINL float decode_elem(uint32_t code) {
 // E8M0 -> fp32 (code 0 = 2^-127 is an fp32 denormal; 0xFF must not be passed).
 RK_DEVINL float e8m0_to_f32(uint32_t c) { return __uint_as_float(c == 0 ? 0x00400000u : (c << 23)); }
 
+// Offset of (row r of a 128-row tile, 32-element block kb of a 128-element
+// chunk) inside a 512-byte scale-factor atom: 32 rows x 16 bytes, row r%32,
+// byte (r/32)*4 + kb.  One tcgen05.cp 32x128b.warpx4 moves an atom to 4 TMEM
+// columns (lane = r%32, column = r/32, byte = kb).
+__host__ __device__ inline int sf_atom_offset(int r, int kb) { return (r & 31) * 16 + (r >> 5) * 4 + kb; }
+
 // ----------------------------------------------------------------------------
 // PTX wrappers
 // ----------------------------------------------------------------------------

@@ -25,34 +25,12 @@
 
 #include "rk_common.cuh"
 #include "rk_internal.h"
+#include "rk_rebase.cuh"
 
 namespace rk {
 
 int g_ring_stop = 0;   // set by rk_debug_set_ring_stop (tests only)
 
-// four floats -> four packed element codes (byte k = code of v[k]); finite inputs only
-template <int FMT> RK_DEVINL uint32_t hw_encode4(float a, float b, float c, float d) {
-  uint32_t r;
-  if (FMT == 0)
-    asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-  else if (FMT == 1)
-    asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e5m2x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e5m2x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-  else if (FMT == 4) {    // two codes per byte, which cross the interfaces one per byte (67 M codes through the integer encoder: 187 us, now 60)
-    asm("{\n\t.reg .b8 l, h;\n\tcvt.rn.satfinite.e2m1x2.f32 l, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 h, %4, %3;\n\tmov.b32 %0, {l, h, l, h};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-    r = __byte_perm(r, 0u, 0x4140);
-    r = (r | (r << 4)) & 0x0F0F0F0Fu;
-  }
-  else if (FMT == 2)
-    asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e2m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e2m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-  else
-    asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e3m2x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e3m2x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
-  return r;
-}
 template <int FMT> RK_DEVINL uint32_t ref_encode4(float a, float b, float c, float d) {
   return encode_rne<FMT>(a) | (encode_rne<FMT>(b) << 8) | (encode_rne<FMT>(c) << 16) | (encode_rne<FMT>(d) << 24);
 }
@@ -74,12 +52,6 @@ __global__ void verify_encoder_kernel(uint64_t first, uint64_t count, unsigned l
 }
 
 // BF16IN: the input is bf16 (one 16-byte load per chunk, widened exactly to fp32) instead of fp32.
-// Offset of (row r of a 128-row tile, 32-element block kb of a 128-element
-// chunk) inside a 512-byte scale-factor atom: 32 rows x 16 bytes, row r%32,
-// byte (r/32)*4 + kb.  One tcgen05.cp 32x128b.warpx4 moves an atom to 4 TMEM
-// columns (lane = r%32, column = r/32, byte = kb).
-__host__ __device__ inline int sf_atom_offset(int r, int kb) { return (r & 31) * 16 + (r >> 5) * 4 + kb; }
-
 // LAYOUT: where a block's scale byte goes -- 0 row-major [rows][d/32]; 1 group-major [batch][d/32][S]; 2 the
 // 512-byte scale-factor atoms [batch][ceil(S/128)][ceil(d/128)][512] the attention kernel copies into TMEM
 // (S = rows per matrix of the batch, nbd = d/32; both unused for layout 0).
@@ -1171,48 +1143,23 @@ __global__ void __launch_bounds__(128) quantize_keys_kernel(const float* __restr
 // Exact value of element code `c` times 2^(s-127) as an fp32.  Normal codes under ordinary scales are
 // placed by integer arithmetic (E4M3: bits = (mag + 8 s - 56) << 20); everything else (subnormal codes,
 // scale codes near the ends of the range, the other formats) takes the generic multiply.
-template <int FMT> RK_DEVINL float decode_scaled(uint32_t c, uint32_t s) {
-  if (FMT == 0) {
-    const uint32_t mag = c & 0x7Fu;
-    if (mag >= 8u && s >= 16u && s <= 240u) return __uint_as_float(((c & 0x80u) << 24) | ((mag + 8u * s - 56u) << 20));
-  }
-  return decode_elem<FMT>(c) * e8m0_to_f32(s);
-}
-
-// The slow form: a thread's NC columns of a block, element by element through fp32; keys k0 .. k0 + 7 are written, and the
-// scale codes of NC / 4 columns from c0 on are returned.
-template <int FMT, int NC>
-__device__ __noinline__ void rebase_slow(const uint8_t* cb, const uint8_t* sb, int n, int k0, int64_t d, int64_t nbd, uint8_t* ob, int c0, uint32_t (&sc)[NC / 4]) {
-#pragma unroll 1
-  for (int c = 0; c < NC; ++c) {
-    float amax = 0.0f, p2 = 1.0f;
-    uint32_t code = 0;
-    for (int j = 0; j < n; ++j) amax = fmaxf(amax, fabsf(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd])));
-    if (amax > 0.0f) block_scale<FMT>(amax, code, p2);
-#pragma unroll
-    for (int h = 0; h < NC / 4; ++h)
-      if (c == c0 + h) sc[h] = code;
-    for (int j = k0; j < min(n, k0 + 8); ++j) ob[j * d + c] = (uint8_t)encode_rne<FMT>(decode_scaled<FMT>(cb[j * d + c], sb[j * nbd]) * p2);
-  }
-}
-
-// Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one thread per (atom, row or column)
-// writes 4 bytes; rows, columns and blocks past the edge get code 0x7F = 2^0.
+// Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one warp per atom, a lane writes the 16 bytes of rows or columns lane,
+// lane + 32, + 64 and + 96; rows, columns and blocks past the edge get code 0x7F = 2^0.  (A thread per row or column, with the divisions that find its place, was a fifth
+// of the time of the re-blocking kernel beside which the scales of Q and K are re-tiled: 8 x 16 heads of 4096, d = 128, 33.8 -> 31.6 us, 4 x 32 / 8 of 8192 22.2 -> 18.8, 2 x 16 / 8 of 8192, d = 256, 20.2 -> 18.5.)
 //   kRows   along d, row-major [batch][S][d/32]
 //   kGroups along d, group-major [batch][d/32][S] (the reference's QK_A_scales_row[FA_GK][FA_SQ] per head,
 //           kernels/flash_attention_mx/gen_data.py:82-83)
 //   kKeys   along keys, row-major [batch][ceil(S/32)][d]
 enum RetileKind { kRows = 0, kGroups = 1, kKeys = 2 };
-RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t tid, int64_t nthreads) {
+RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t warp, int64_t warps) {
   const int64_t S = job.S, d = job.d;
-  const int64_t nbd = d / 32, nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
-  const int64_t total = job.batch * ntile * dch * 128;
-  for (int64_t t = tid; t < total; t += nthreads) {
-    const int r = (int)(t % 128);
-    const int64_t atom = t / 128;
+  const int64_t nbd = d / 32, nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128, total = job.batch * ntile * dch;
+  const int lane = threadIdx.x & 31;
+  const bool words = job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;
+  for (int64_t atom = warp; atom < total; atom += warps) {
     int64_t ch, tile, bt;
     if (total < (int64_t)1 << 31) {           // 32-bit divisions whenever the index fits
-      const uint32_t a32 = (uint32_t)atom, q = a32 / (uint32_t)dch;
+      const uint32_t a32 = (uint32_t)atom, q = dch == 1 ? a32 : a32 / (uint32_t)dch;
       ch = a32 - q * (uint32_t)dch;
       const uint32_t b32 = q / (uint32_t)ntile;
       tile = q - b32 * (uint32_t)ntile;
@@ -1220,30 +1167,35 @@ RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t tid, int64_t nth
     } else {
       ch = atom % dch; tile = (atom / dch) % ntile; bt = atom / (dch * ntile);
     }
-    uint32_t w = 0x7F7F7F7Fu;
-    if (job.kind == kKeys) {
-      const int64_t col = ch * 128 + r;
-      if (col < d) {
-        w = 0;
+    uint32_t w[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) w |= (tile * 4 + k < nkb ? (uint32_t)job.in[(bt * nkb + tile * 4 + k) * d + col] : 0x7Fu) << (8 * k);
-      }
-    } else {
-      const int64_t row = tile * 128 + r;
-      if (row < S) {
-        if (job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0) {
-          w = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
-        } else {
-          w = 0;
+    for (int i = 0; i < 4; ++i) {
+      const int r = i * 32 + lane;
+      w[i] = 0x7F7F7F7Fu;
+      if (job.kind == kKeys) {
+        const int64_t col = ch * 128 + r;
+        if (col < d) {
+          w[i] = 0;
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const int64_t blk = ch * 4 + k;
-            w |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
+          for (int k = 0; k < 4; k++) w[i] |= (tile * 4 + k < nkb ? (uint32_t)job.in[(bt * nkb + tile * 4 + k) * d + col] : 0x7Fu) << (8 * k);
+        }
+      } else {
+        const int64_t row = tile * 128 + r;
+        if (row < S) {
+          if (words) {
+            w[i] = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
+          } else {
+            w[i] = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const int64_t blk = ch * 4 + k;
+              w[i] |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
+            }
           }
         }
       }
     }
-    *reinterpret_cast<uint32_t*>(job.out + atom * 512 + sf_atom_offset(r, 0)) = w;
+    *reinterpret_cast<uint4*>(job.out + atom * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 // The jobs of a prefill call ride along with whichever preparation kernel it needs anyway (a launch costs more than they do):
@@ -1252,7 +1204,7 @@ RK_DEVINL bool retile_jobs(const RetileJobs& jobs) {
   if ((int)blockIdx.x >= jobs.ctas) return false;
 #pragma unroll 1
   for (int i = 0; i < jobs.n; ++i)
-    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)jobs.ctas * blockDim.x);
+    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), (int64_t)jobs.ctas * (blockDim.x / 32));
   return true;
 }
 __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs jobs) {
@@ -1261,56 +1213,24 @@ __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs job
   retile_jobs(jobs);
 }
 
-// ---- V re-blocking: scales along d -> MX blocks along the keys --------------------------------------------------------
-// Decode exactly, then the block rule down each column: the same as decoding to fp32 and quantizing again.  The hot form does
-// it in f16: a pair of codes goes through the hardware converter, times the row's scale relative to the block's largest, the
-// column maxima are packed maxima, the column's factor (a power of two, at least 1) is one more packed product, and the
-// pair goes back through the converter.  All of it is exact: values of a format are multiples of 2^-9 (E4M3), 2^-16 (E5M2) or
-// 2^-4 (the others) and f16 reaches down to 2^-24, so it holds while the block's scales span no more than kSpan and a column's
-// factor stays an f16; other blocks and columns take the slow form through fp32, element by element.
-template <int FMT> struct RebaseT { static constexpr int kSpan = FMT == 1 ? 8 : 14; };
-// two codes in the low bytes -> packed f16 (exact); an E2M1 code, shifted, is the E2M3 code of its value
-template <int FMT> RK_DEVINL uint32_t decode_f16x2(uint32_t codes) {
-  uint32_t r;
-  if (FMT == 0) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  else if (FMT == 1) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e5m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  else if (FMT == 3) asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e3m2x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  else asm("{\n\t.reg .b16 c, z;\n\tmov.b32 {c, z}, %1;\n\tcvt.rn.f16x2.e2m3x2 %0, c;\n\t}" : "=r"(r) : "r"(codes));
-  return r;
-}
-// a word of four codes as the converter takes them
-template <int FMT> RK_DEVINL uint32_t clean_codes(uint32_t w) {
-  return FMT == 4 ? (w & 0x0F0F0F0Fu) << 2 : FMT >= 2 ? w & 0x3F3F3F3Fu : w;
-}
-RK_DEVINL uint32_t max_u16x2(uint32_t a, uint32_t b) { uint32_t r; asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-RK_DEVINL uint32_t hmul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
-RK_DEVINL float f16_lo(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, l;\n\t}" : "=f"(r) : "r"(v)); return r; }
-RK_DEVINL float f16_hi(uint32_t v) { float r; asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "r"(v)); return r; }
-// packed f16 pairs -> four codes (finite, exact values: as encode_rne)
-template <int FMT> RK_DEVINL uint32_t encode_f16x4(uint32_t lo, uint32_t hi) {
-  uint32_t r;
-  if (FMT == 0) asm("{\n\t.reg .b16 a, b;\n\tcvt.rn.satfinite.e4m3x2.f16x2 a, %1;\n\tcvt.rn.satfinite.e4m3x2.f16x2 b, %2;\n\tmov.b32 %0, {a, b};\n\t}" : "=r"(r) : "r"(lo), "r"(hi));
-  else if (FMT == 1) asm("{\n\t.reg .b16 a, b;\n\tcvt.rn.satfinite.e5m2x2.f16x2 a, %1;\n\tcvt.rn.satfinite.e5m2x2.f16x2 b, %2;\n\tmov.b32 %0, {a, b};\n\t}" : "=r"(r) : "r"(lo), "r"(hi));
-  else r = hw_encode4<FMT>(f16_lo(lo), f16_hi(lo), f16_lo(hi), f16_hi(hi));
-  return r;
-}
-
+// ---- V re-blocking: scales along d -> MX blocks along the keys (rk_rebase.cuh) ---------------------------------------
 // A CTA = 128 keys x 8 NC columns at a time, a warp = 32 of the keys, a lane = 8 of them x NC adjacent columns, all its loads
 // in flight; the column maxima meet by the shuffles of a reduce-scatter.  NC = 8, or 4 where the codes are not 8-byte aligned.
 // 67 M codes E4M3: 53 us in integer arithmetic on the codes (12 instructions per code, 16 warps per SM, rows with a zero or
-// subnormal code on a path of their own), 30 us here (33 beside the scales' re-tiling).
+// subnormal code on a path of their own), 31.6 us here beside the scales' re-tiling.  (All columns of 128 keys by one CTA: 30.4, but 33.5 M codes 18.8 -> 19.8 and calls of few
+// keys 0.2 us more.  On the codes as bytes, where a power of two is a step of 8: 35 us, and 55 with the words done again in which a code is or becomes subnormal.)
 constexpr int kRebaseThreads = 128;
 template <int FMT, bool TILED, int NC>
 __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
                                                                  int64_t batch, int64_t S, int64_t d, uint8_t* __restrict__ out_codes,
                                                                  uint8_t* __restrict__ out_scales, const RetileJobs jobs) {
-  constexpr int NW = NC / 4, NB = NC / 4;                          // words per key of a thread; 32-column blocks of a warp
+  constexpr int NW = NC / 4, NB = NC / 4, CP = NC / 4;             // words per key of a thread; 32-column blocks of a warp; columns whose scales a thread works out
   __shared__ __align__(4) uint8_t sc_sm[8 * NC * 4];
   __shared__ __align__(16) uint32_t fac_sm[kRebaseThreads / 32][NB][32];
   grid_dependency_wait();
   grid_dependents_launch();
   if (retile_jobs(jobs)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k0 = (lane >> 3) * 8, b = (lane & 7) * NC / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t nkb = (S + 31) / 32, nbd = d / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
   const int64_t cun = TILED ? dch * (16 / NC) : (d + 8 * NC - 1) / (8 * NC), units = batch * ntile * cun, stride = gridDim.x - jobs.ctas;
   for (int64_t u = (int64_t)blockIdx.x - jobs.ctas; u < units; u += stride) {
@@ -1328,100 +1248,15 @@ __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8
     const int64_t row0 = bt * S + kb * 32, col = cu * 8 * NC + (lane & 7) * NC;
     const int n = (int)max((int64_t)0, min((int64_t)32, S - kb * 32));   // keys of this block that exist
     const bool in = col < d && n > 0;
-    const uint8_t* src = codes + row0 * d + col;
-    uint32_t w[8][NW];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const bool live = in && k0 + i < n;
-      const uint8_t* q = src + (k0 + i) * d;
-      if (NC == 8) {
-        const uint2 v = live ? __ldg(reinterpret_cast<const uint2*>(q)) : make_uint2(0u, 0u);
-        w[i][0] = v.x; w[i][NW - 1] = v.y;
-      } else {
-        w[i][0] = live ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
-      }
-    }
-    // the rows' scales relative to the block's largest, as packed f16; lane = key
-    int smax = 0;
-    bool hot = true;
-    const uint8_t* sk = scales + (row0 + lane) * nbd + cu * NB;
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      const bool live = lane < n && cu * NB + c < nbd;
-      const int s = live ? (int)__ldg(sk + c) : -1;
-      const int top = __reduce_max_sync(0xffffffffu, s), low = __reduce_min_sync(0xffffffffu, live ? s : 255);
-      fac_sm[warp][c][lane] = live ? (uint32_t)max(15 + s - top, 1) * 0x04000400u : 0u;
-      if (c == b) { smax = max(top, 0); hot = low >= 20 && top <= 235 && top - low <= RebaseT<FMT>::kSpan; }
-    }
-    __syncwarp();
-    uint32_t m[2 * NW];                                            // maxima of column pairs
-#pragma unroll
-    for (int i = 0; i < 2 * NW; ++i) m[i] = 0u;
-    uint32_t x[8][2 * NW];
-#pragma unroll
-    for (int i = 0; i < 8; i += 4) {
-      const uint4 f4 = *reinterpret_cast<const uint4*>(&fac_sm[warp][b][k0 + i]);
-      const uint32_t f[4] = {f4.x, f4.y, f4.z, f4.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          const uint32_t c = clean_codes<FMT>(w[i + e][q]);
-          x[i + e][2 * q] = hmul2(decode_f16x2<FMT>(c), f[e]);
-          x[i + e][2 * q + 1] = hmul2(decode_f16x2<FMT>(c >> 16), f[e]);
-          m[2 * q] = max_u16x2(m[2 * q], x[i + e][2 * q] & 0x7FFF7FFFu);
-          m[2 * q + 1] = max_u16x2(m[2 * q + 1], x[i + e][2 * q + 1] & 0x7FFF7FFFu);
-        }
-    }
-    __syncwarp();                                                  // fac_sm has been read
-    // The four lanes of a column group end up with the maxima of a quarter of its columns each, work out those scales and
-    // hand the factors back.
-    constexpr int CP = NC / 4;                                     // columns of a lane's quarter
-    const bool h16 = lane & 16, h8 = lane & 8;
-    uint32_t mine;
-    if (NC == 8) {
-      const uint32_t a = max_u16x2(h16 ? m[NW] : m[0], __shfl_xor_sync(0xffffffffu, h16 ? m[0] : m[NW], 16));
-      const uint32_t c = max_u16x2(h16 ? m[2 * NW - 1] : m[1], __shfl_xor_sync(0xffffffffu, h16 ? m[1] : m[2 * NW - 1], 16));
-      mine = max_u16x2(h8 ? c : a, __shfl_xor_sync(0xffffffffu, h8 ? a : c, 8));
-    } else {
-      mine = max_u16x2(h16 ? m[1] : m[0], __shfl_xor_sync(0xffffffffu, h16 ? m[0] : m[1], 16));
-      mine = max_u16x2(mine, __shfl_xor_sync(0xffffffffu, mine, 8));
-      if (h8) mine >>= 16;
-    }
-    const float unit = __uint_as_float((uint32_t)smax << 23);      // 2^(smax - 127)
-    uint32_t sc[CP], fac = 0u, f[2 * NW];
-#pragma unroll
-    for (int h = 0; h < CP; ++h) {
-      const float am = (h ? f16_hi(mine) : f16_lo(mine)) * unit;
-      uint32_t code = 0; float p2;
-      int up = 0;                                                  // log2 of the column's factor
-      if (am > 0.0f) { block_scale<FMT>(am, code, p2); up = (int)(__float_as_uint(p2) >> 23) - 254 + smax; }
-      hot = hot && up <= 15 && (FMT > 1 || am < __int_as_float(0x7f800000));        // (NaN and infinity encodings are numbers here)
-      sc[h] = in ? code : 0x7Fu;                                   // of columns and key blocks that do not exist: 2^0
-      fac |= (uint32_t)((15 + up) & 31) << (10 + 16 * h);
-    }
-    hot = (__ballot_sync(0xffffffffu, !hot) & (0x01010101u << (lane & 7))) == 0u;
-#pragma unroll
-    for (int i = 0; i < 2 * NW; ++i) {
-      f[i] = __shfl_sync(0xffffffffu, fac, (lane & 7) + (NC == 8 ? 8 * i : 16 * i));
-      if (NC == 4) f[i] |= __shfl_sync(0xffffffffu, fac, (lane & 7) + 16 * i + 8) << 16;
-    }
-    if (in) {
-      uint8_t* dst = out_codes + row0 * d + col;
-      if (hot) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if (k0 + i >= n) break;
-          uint32_t o[NW];
-#pragma unroll
-          for (int q = 0; q < NW; ++q) o[q] = encode_f16x4<FMT>(hmul2(x[i][2 * q], f[2 * q]), hmul2(x[i][2 * q + 1], f[2 * q + 1]));
-          if (NC == 8) *reinterpret_cast<uint2*>(dst + (k0 + i) * d) = make_uint2(o[0], o[NW - 1]);
-          else *reinterpret_cast<uint32_t*>(dst + (k0 + i) * d) = o[0];
-        }
-      } else {
-        rebase_slow<FMT, NC>(src, scales + row0 * nbd + col / 32, n, k0, d, nbd, dst, (lane >> 3) * CP, sc);
-      }
-    }
+    uint32_t sc[CP];
+    uint8_t* const dst = out_codes + row0 * d + col;
+    const int di = (int)d;
+    rebase_block<FMT, NC, false>(codes + row0 * d, scales + row0 * nbd, (int)d, (int)cu, n, fac_sm[warp], lane,
+                                 [=](int k, const uint32_t (&o)[NW]) {
+                                   if (NC == 8) *reinterpret_cast<uint2*>(dst + k * di) = make_uint2(o[0], o[NW - 1]);
+                                   else *reinterpret_cast<uint32_t*>(dst + k * di) = o[0];
+                                 },
+                                 [=](int k, int c, uint8_t code) { dst[k * di + c] = code; }, sc);
     if (TILED) {
       // the four warps' scale bytes of a column are one word of its atom
 #pragma unroll
@@ -1760,7 +1595,7 @@ int launch_quantize_keys_atoms(const float* x, int64_t batch, int64_t rows, int6
 // CTAs of `threads` threads for the re-tiling jobs beside other work
 static int retile_ctas(const RetileJobs& jobs, int threads) {
   int64_t most = 0;
-  for (int i = 0; i < jobs.n; ++i) most = std::max(most, jobs.job[i].batch * ((jobs.job[i].S + 127) / 128) * ((jobs.job[i].d + 127) / 128) * 128);
+  for (int i = 0; i < jobs.n; ++i) most = std::max(most, jobs.job[i].batch * ((jobs.job[i].S + 127) / 128) * ((jobs.job[i].d + 127) / 128) * 32);      // a warp each
   return most == 0 ? 0 : grid_for(most, threads, 4);
 }
 
