@@ -1151,60 +1151,75 @@ __global__ void __launch_bounds__(128) quantize_keys_kernel(const float* __restr
 //           kernels/flash_attention_mx/gen_data.py:82-83)
 //   kKeys   along keys, row-major [batch][ceil(S/32)][d]
 enum RetileKind { kRows = 0, kGroups = 1, kKeys = 2 };
-RK_DEVINL void retile_scales_body(const RetileJob& job, int64_t warp, int64_t warps) {
+RK_DEVINL void retile_atom(const RetileJob& job, int64_t atom, int64_t total) {
   const int64_t S = job.S, d = job.d;
-  const int64_t nbd = d / 32, nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128, total = job.batch * ntile * dch;
+  const int64_t nbd = d / 32, nkb = (S + 31) / 32, ntile = (S + 127) / 128, dch = (d + 127) / 128;
   const int lane = threadIdx.x & 31;
-  const bool words = job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;
-  for (int64_t atom = warp; atom < total; atom += warps) {
-    int64_t ch, tile, bt;
-    if (total < (int64_t)1 << 31) {           // 32-bit divisions whenever the index fits
-      const uint32_t a32 = (uint32_t)atom, q = dch == 1 ? a32 : a32 / (uint32_t)dch;
-      ch = a32 - q * (uint32_t)dch;
-      const uint32_t b32 = q / (uint32_t)ntile;
-      tile = q - b32 * (uint32_t)ntile;
-      bt = b32;
-    } else {
-      ch = atom % dch; tile = (atom / dch) % ntile; bt = atom / (dch * ntile);
+  uint8_t* const out = job.out + atom * 512;
+  int64_t ch, tile, bt;
+  if (total < (int64_t)1 << 31) {           // 32-bit divisions whenever the index fits
+    const uint32_t a32 = (uint32_t)atom, q = dch == 1 ? a32 : a32 / (uint32_t)dch;
+    ch = a32 - q * (uint32_t)dch;
+    const uint32_t b32 = q / (uint32_t)ntile;
+    tile = q - b32 * (uint32_t)ntile;
+    bt = b32;
+  } else {
+    ch = atom % dch; tile = (atom / dch) % ntile; bt = atom / (dch * ntile);
+  }
+  uint32_t w[4];
+  if (job.kind == kKeys) {                  // four adjacent columns of the four key blocks, turned
+    const int64_t col = ch * 128 + lane * 4;
+    const uint8_t* const in = job.in + (bt * nkb + tile * 4) * d + col;
+    const bool words = (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;      // (d is a multiple of 32)
+    uint32_t r[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      r[k] = 0x7F7F7F7Fu;
+      if (col < d && tile * 4 + k < nkb) {
+        if (words) r[k] = *reinterpret_cast<const uint32_t*>(in + k * d);
+        else r[k] = in[k * d] | ((uint32_t)in[k * d + 1] << 8) | ((uint32_t)in[k * d + 2] << 16) | ((uint32_t)in[k * d + 3] << 24);
+      }
     }
-    uint32_t w[4];
+    const uint32_t a = __byte_perm(r[0], r[1], 0x5140), b = __byte_perm(r[2], r[3], 0x5140), c = __byte_perm(r[0], r[1], 0x7362), e = __byte_perm(r[2], r[3], 0x7362);
+    w[0] = __byte_perm(a, b, 0x5410); w[1] = __byte_perm(a, b, 0x7632); w[2] = __byte_perm(c, e, 0x5410); w[3] = __byte_perm(c, e, 0x7632);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = i * 32 + lane;
-      w[i] = 0x7F7F7F7Fu;
-      if (job.kind == kKeys) {
-        const int64_t col = ch * 128 + r;
-        if (col < d) {
-          w[i] = 0;
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(out + sf_atom_offset(lane * 4 + i, 0)) = w[i];
+    return;
+  }
+  const bool words = job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;
 #pragma unroll
-          for (int k = 0; k < 4; k++) w[i] |= (tile * 4 + k < nkb ? (uint32_t)job.in[(bt * nkb + tile * 4 + k) * d + col] : 0x7Fu) << (8 * k);
-        }
+  for (int i = 0; i < 4; ++i) {
+    const int64_t row = tile * 128 + i * 32 + lane;
+    w[i] = 0x7F7F7F7Fu;
+    if (row < S) {
+      if (words) {
+        w[i] = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
       } else {
-        const int64_t row = tile * 128 + r;
-        if (row < S) {
-          if (words) {
-            w[i] = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
-          } else {
-            w[i] = 0;
+        w[i] = 0;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-              const int64_t blk = ch * 4 + k;
-              w[i] |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
-            }
-          }
+        for (int k = 0; k < 4; k++) {
+          const int64_t blk = ch * 4 + k;
+          w[i] |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
         }
       }
     }
-    *reinterpret_cast<uint4*>(job.out + atom * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
+  *reinterpret_cast<uint4*>(out + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
 }
+__host__ __device__ inline int64_t retile_atoms(const RetileJob& job) { return job.batch * ((job.S + 127) / 128) * ((job.d + 127) / 128); }
 // The jobs of a prefill call ride along with whichever preparation kernel it needs anyway (a launch costs more than they do):
-// its first jobs.ctas CTAs do them, true for those.
+// its first jobs.ctas CTAs do them, true for those.  The atoms of all jobs in a row, so that a small call has one for each warp at most.
 RK_DEVINL bool retile_jobs(const RetileJobs& jobs) {
   if ((int)blockIdx.x >= jobs.ctas) return false;
+  const int64_t warps = (int64_t)jobs.ctas * (blockDim.x / 32);
+  int64_t at = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
 #pragma unroll 1
-  for (int i = 0; i < jobs.n; ++i)
-    retile_scales_body(jobs.job[i], (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), (int64_t)jobs.ctas * (blockDim.x / 32));
+  for (int i = 0; i < jobs.n; ++i) {
+    const int64_t n = retile_atoms(jobs.job[i]);
+#pragma unroll 1
+    for (; at < n; at += warps) retile_atom(jobs.job[i], at, n);
+    at -= n;
+  }
   return true;
 }
 __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs jobs) {
@@ -1594,9 +1609,9 @@ int launch_quantize_keys_atoms(const float* x, int64_t batch, int64_t rows, int6
 
 // CTAs of `threads` threads for the re-tiling jobs beside other work
 static int retile_ctas(const RetileJobs& jobs, int threads) {
-  int64_t most = 0;
-  for (int i = 0; i < jobs.n; ++i) most = std::max(most, jobs.job[i].batch * ((jobs.job[i].S + 127) / 128) * ((jobs.job[i].d + 127) / 128) * 32);      // a warp each
-  return most == 0 ? 0 : grid_for(most, threads, 4);
+  int64_t atoms = 0;
+  for (int i = 0; i < jobs.n; ++i) atoms += retile_atoms(jobs.job[i]);
+  return atoms == 0 ? 0 : grid_for(atoms * 32, threads, 4);      // a warp each
 }
 
 int launch_retile_scales(RetileJobs jobs, cudaStream_t st) {
