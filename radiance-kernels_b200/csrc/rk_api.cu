@@ -241,6 +241,7 @@ int rk_attn_prefill(const rk_prefill_args* a, void* stream) {
   const PrefillWs w = prefill_ws(*a);
   if (!a->workspace || a->workspace_bytes < w.total || !aligned(a->workspace, 256)) return RK_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
+  if (prefill_prepares(*a)) return launch_prefill(*a, a->q, a->k, a->v, a->q_scale, a->k_scale, a->v_scale, true, st);
   uint8_t* ws = reinterpret_cast<uint8_t*>(a->workspace);
   const int64_t bhq = (int64_t)a->B * a->H, bhkv = (int64_t)a->B * a->H_kv;
 
@@ -284,7 +285,7 @@ int rk_attn_prefill(const rk_prefill_args* a, void* stream) {
     v_codes = ws + w.v_codes;
   }
   if (jobs.n > 0 && (rc = launch_retile_scales(jobs, st)) != RK_OK) return rc;
-  return launch_prefill(*a, q_codes, k_codes, v_codes, q_sf, k_sf, v_sf, st);
+  return launch_prefill(*a, q_codes, k_codes, v_codes, q_sf, k_sf, v_sf, false, st);
 }
 
 size_t rk_attn_prefill_host_arena_bytes(const rk_prefill_args* a) {

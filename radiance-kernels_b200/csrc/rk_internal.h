@@ -43,8 +43,10 @@ int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads
 
 // q/k/v_codes: byte codes as the caller gave them, or -- for 6- and 4-bit formats -- the packed copies made by
 // launch_pack_rows (Q, K) and launch_pack_v (V, stored [d][keys]).
+// prepares: the attention kernel puts the scales into atoms and re-blocks V itself (prefill_prepares); codes and scales are then the caller's.
 int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* v_codes,
-                   const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, cudaStream_t st);
+                   const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, bool prepares, cudaStream_t st);
+bool prefill_prepares(const rk_prefill_args& a);
 
 bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms);      // which RoPE kernel a call without positions of its own takes
 // Which kernel a prefill call takes on a device of `sms` SMs: d = 256, pairs of query tiles, one query tile at a time with the softmax groups on alternate

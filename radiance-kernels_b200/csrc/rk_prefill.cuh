@@ -26,6 +26,7 @@ struct PrefillParams {
   const uint8_t* q_sf;
   const uint8_t* k_sf;
   const uint8_t* v_sf;
+  const uint8_t* v;    // a call whose attention kernel does the preparation: V's codes, and q_sf, k_sf, v_sf as the caller gave them
   __nv_bfloat16* o;
   float* lse;
   int* status;
@@ -228,7 +229,7 @@ extern float* g_prefill_dbg;
 
 // Two query tiles per CTA, one thread per row, correction warps (d <= 128), or with `split` one query tile; defined in rk_prefill2c.cu.
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
-                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, cudaStream_t st);
+                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, int prep, cudaStream_t st);
 // One query tile per CTA at a time, two softmax groups on alternate key tiles (d <= 128, few query tiles); defined in rk_prefill1.cu.
 int launch_prefill1(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, cudaStream_t st);

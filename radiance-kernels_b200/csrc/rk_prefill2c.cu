@@ -33,9 +33,17 @@
 // tile's time is then the softmax of one thread's row (about 3200 cycles for 128 scores, the tensor core waits), so both softmax groups work
 // on the same tile, group A on keys 0-63 of each key tile and group B on keys 64-127, and exchange their row maxima through
 // shared memory.
+//
+// SPLIT with PREP = the format of K and V (E4M3, E5M2): the preparation of a small call, which is otherwise a launch of its own.  The issuers and the warp that fills the warpgroup put the
+// row-major scales of Q and K into atoms, softmax and correction warps re-block V, scaled along d, into the stages V is read from, in the time Q and K take to arrive and the
+// first scores to be formed: there is a stage for every key tile.  A query tile of every head re-blocks V for itself, so this is for items of at most three key tiles and grids
+// of one round of the SMs.  (A launch whose results the next one waits for costs 1.2 us,
+// its own chain of latencies 2 to 4.)  Without a mask, us a call: one head of 256 keys, d = 64, 9.2 -> 6.3; 32 / 8 heads of 128 keys, d = 128, 7.1 -> 5.8; 8 x 18 heads of 128 10.6 -> 6.9; 40
+// heads of 384, d = 128, 12.6 -> 10.5, d = 64, 12.0 -> 8.7.
 #include <type_traits>
 
 #include "rk_prefill.cuh"
+#include "rk_rebase.cuh"
 
 namespace rk {
 
@@ -91,6 +99,7 @@ struct __align__(16) Work {
 };
 static_assert(sizeof(Work) == 32, "its place in shared memory");
 constexpr int kReaders = 8 + 4 + 2;      // warps that read an item: softmax, correction, Q K^T, P V
+constexpr int bPrep = bClc;              // PREP: the scale atoms of Q and K are there (no second item is asked for)
 }  // namespace c2
 
 // ---- softmax warps: thread = query row -----------------------------------------------------------------------
@@ -550,7 +559,54 @@ __device__ __forceinline__ int correction_quadrant(const PrefillParams& p, const
   return 0;
 }
 
-template <bool SOFTCAP, bool DUMP, bool SPLIT>
+// PREP: 64 columns (unit cu) of key tile `tile` of V, re-blocked along the keys by four warps (32 keys each), as TMA would have left them in their stage: rows of 128 bytes,
+// 128-byte swizzle, zeros for keys that do not exist, and their part of the scale atom.  (Columns past d are left as they are: they meet columns of O that nobody reads.)
+template <int FMT>
+__device__ __forceinline__ void rebase_v_unit(const PrefillParams& p, uint8_t* smem, int warp, int lane, int st, int tile, int cu, int bhkv) {
+  using namespace c2;
+  const int quad = warp & 3, key0 = tile * kBlockN + quad * 32, n = max(0, min(32, p.S_kv - key0)), col = cu * 64 + (lane & 7) * 8;
+  const int64_t row0 = (int64_t)bhkv * p.S_kv + (n > 0 ? key0 : 0);
+  uint8_t* const dst = smem + v_off + st * kTileBytes + quad * 32 * 128;
+  uint8_t* const atom = smem + sfv_off + st * kSfAtomBytes;
+  uint32_t sc[2];
+  auto at = [=](int k, int c) { return dst + k * 128 + (((c >> 4) ^ (k & 7)) << 4) + (c & 15); };
+  rebase_block<FMT, 8, true>(p.v + row0 * p.d, p.v_sf + row0 * (p.d / 32), p.d, cu, n, reinterpret_cast<uint32_t (*)[32]>(smem + stage_off + warp * 256), lane,
+                             [=](int k, const uint32_t (&o)[2]) { *reinterpret_cast<uint2*>(at(k, col)) = make_uint2(o[0], o[1]); },
+                             [=](int k, int c, uint8_t code) { *at(k, col + c) = code; }, sc);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = col + (lane >> 3) * 2 + h;
+    atom[sf_atom_offset(c, quad)] = (uint8_t)sc[h];
+    if (p.d <= 64) atom[sf_atom_offset(c + 64, quad)] = 0x7F;
+  }
+}
+
+// PREP: the scale atom of 128 rows from row0 of a matrix of S rows, by one warp, four rows a lane.
+RK_DEVINL void scale_atom(const uint8_t* scales, int64_t bh, int S, int row0, int nbd, uint8_t* atom, int lane) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(scales);
+  const uint8_t* src = scales + (bh * S + row0 + lane) * nbd;
+  const int n = S - row0 - lane;                              // row i * 32 exists if it is below
+  uint32_t w[4];
+  if (nbd == 4 && (at & 3) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = i * 32 < n ? __ldg(reinterpret_cast<const uint32_t*>(src + i * 128)) : 0x7F7F7F7Fu;
+  } else if (nbd == 2 && (at & 1) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = i * 32 < n ? 0x7F7F0000u | __ldg(reinterpret_cast<const uint16_t*>(src + i * 64)) : 0x7F7F7F7Fu;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t c[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[k] = k < nbd && i * 32 < n ? (uint32_t)__ldg(src + i * 32 * nbd + k) : 0x7Fu;
+      w[i] = c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(atom + sf_atom_offset(i * 32 + lane, 0)) = w[i];
+}
+
+template <bool SOFTCAP, bool DUMP, bool SPLIT, int PREP>
 __global__ void __launch_bounds__(c2::kThreads, 1)
 prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const PrefillParams p, const uint32_t idesc_qk,
@@ -565,6 +621,8 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) RK_STAMP(2, 0, 6);
   constexpr int kQt = SPLIT ? 1 : 2;                                  // query tiles per item
+  constexpr bool kPrep = PREP >= 0;
+  constexpr int kAtomTx = kPrep ? 0 : kSfAtomBytes;                   // of Q and K, by copy
   const int n_pairs = (p.n_q_tiles + kQt - 1) / kQt;
   auto decode = [&](uint32_t block) -> Work {
     Work w;
@@ -592,14 +650,14 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   auto issue_q = [&](int g) {
     uint64_t* bar = &bars[g == 0 ? bQ : bQB];
-    mbar_arrive_expect_tx(bar, p.q_tile_tx + kSfAtomBytes);
+    mbar_arrive_expect_tx(bar, p.q_tile_tx + kAtomTx);
     tma_load_3d(smem + q_off + g * kTileBytes, &tmap_q, bar, 0, (kQt * w.qp + g) * kBlockM, w.bh);
-    bulk_load_1d(smem + sfq_off + g * kSfAtomBytes, p.q_sf + ((size_t)w.bh * p.n_q_tiles + kQt * w.qp + g) * kSfAtomBytes, kSfAtomBytes, bar);
+    if (!kPrep) bulk_load_1d(smem + sfq_off + g * kSfAtomBytes, p.q_sf + ((size_t)w.bh * p.n_q_tiles + kQt * w.qp + g) * kSfAtomBytes, kSfAtomBytes, bar);
   };
   auto issue_kv = [&](int j, int st) {
-    mbar_arrive_expect_tx(&bars[bKF + st], p.kv_tile_tx + kSfAtomBytes);
+    mbar_arrive_expect_tx(&bars[bKF + st], p.kv_tile_tx + kAtomTx);
     tma_load_3d(smem + k_off + st * kTileBytes, &tmap_k, &bars[bKF + st], 0, (j + w.j0) * kBlockN, w.bhkv);
-    bulk_load_1d(smem + sfk_off + st * kSfAtomBytes, p.k_sf + ((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * kSfAtomBytes,
+    if (!kPrep) bulk_load_1d(smem + sfk_off + st * kSfAtomBytes, p.k_sf + ((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * kSfAtomBytes,
                  kSfAtomBytes, &bars[bKF + st]);
   };
   auto issue_v = [&](int j, int st) {
@@ -616,7 +674,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const bool per_warp = (i >= bSE && i < bSE + 2) || (i >= bPF && i < bPF + 4) || (i >= bOR && i < bOR + 4);
       // SPLIT: both groups hand back S and write P, and the exchange takes a warp of each
       const bool both = SPLIT && (i < bPV || i >= bCF + 16) && i < bOR;
-      mbar_init(&bars[i], per_warp ? (both ? 8 : 4) : both && i >= bCF + 16 ? 2 : i == bWE ? kReaders : 1);
+      mbar_init(&bars[i], per_warp ? (both ? 8 : 4) : both && i >= bCF + 16 ? 2 : i == bWE ? kReaders : kPrep && i >= bVF && i < bVF + kStages ? (p.d > 64 ? 8 : 4) : kPrep && i == bPrep ? 3 : 1);
     }
     if (lane == 0) *abort_flag = 0;
     fence_barrier_init();
@@ -650,6 +708,34 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   };
   constexpr int kFailWork = 501;
 
+  if constexpr (kPrep) {
+    w = decode(blockIdx.x);
+    if (warp > kWarpTma) {
+      // Atoms of Q and of the key tiles by the three warps that have nothing to do before these are there.  (By one of them, atom after atom or all loads at once: one head of 256
+      // keys 2 us more.)
+#pragma unroll 1
+      for (int a = warp - kWarpTma - 1; a <= w.nt0 && w.nt0 > 0; a += 3)
+        scale_atom(a == 0 ? p.q_sf : p.k_sf, a == 0 ? w.bh : w.bhkv, a == 0 ? p.S_q : p.S_kv, a == 0 ? w.qp * kBlockM : (a - 1 + w.j0) * kBlockN, p.d / 32,
+                   smem + (a == 0 ? sfq_off : sfk_off + (a - 1) * kSfAtomBytes), lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[bPrep]);
+    } else if (warp < kWarpTma) {
+      // V, by the twelve warps that have nothing to do before the first scores are there: units of 64 columns, in the order of the tiles; the correction warps, which are needed last, take
+      // the fourth as well.  Where an earlier launch gave up V does not come, and O is not written.
+      const int units = p.d > 64 ? 2 : 1, n = w.nt0 * units, grp = warp >> 2;
+      if (__shfl_sync(0xffffffffu, lane == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0, 0) == 0) {
+#pragma unroll 1
+        for (int i = grp; i < n; i += grp == 2 ? (i == 2 ? 1 : n) : 4) {
+          const int st = units == 2 ? i >> 1 : i;
+          rebase_v_unit<PREP>(p, smem, warp, lane, st, st + w.j0, units == 2 ? i & 1 : 0, w.bhkv);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[bVF + st]);
+        }
+      }
+    }
+  }
   // (The softmax branch comes last in the code: measured 1-1.5 % faster than first.)
   if (warp >= kWarpTma) {
     reg_dec<SPLIT ? kRegIssueSplit : kRegIssue>();
@@ -694,6 +780,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               if (use > 0 && !mbar_wait_compact<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
               issue_kv(j, st);
               if (stopped) break;                    // O is written only where V has come
+              if (kPrep) { ++st; continue; }         // (a stage for every tile)
               if (use > 0 && !mbar_wait_compact<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
               issue_v(j, st);
               if (++st == kStages) { st = 0; ++use; }
@@ -726,7 +813,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < kStages; ++i) {
           const uint32_t nv = use + (i < st), nk = nv + (i == st && k_ahead);      // loads into this stage
-          want |= (uint32_t)(nk > 0) << (bKF + i) | (uint32_t)(nv > 0) << (bVF + i);
+          want |= (uint32_t)(nk > 0) << (bKF + i) | (uint32_t)(nv > 0 && !kPrep) << (bVF + i);
           par |= ((nk - 1) & 1) << (bKF + i) | ((nv - 1) & 1) << (bVF + i);
         }
 #pragma unroll 1
@@ -758,6 +845,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           perturb<DUMP>(p, kPerturbQk, j);
           if (stops<DUMP>(p, kPerturbQk, j)) { fail = 302; break; }
           if (lane == 0) RK_STAMP(2, j, 0);
+          if (kPrep && j == 0 && !__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bPrep], 0, abort_flag))) { fail = 309; break; }
           if (!__all_sync(0xffffffffu, mbar_wait_compact<true>(&bars[bKF + st], use_par, abort_flag))) { fail = 302; break; }
           if (elect_one()) tc_cp_32x128b_warpx4(tm + cSfK + st * 4, dsfk + (uint32_t)(st * (kSfAtomBytes >> 4)));
           const uint64_t dkt = dk + (uint32_t)(st * (kTileBytes >> 4));
@@ -898,12 +986,12 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (warp == kWarpQk) { tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols); }
 }
 
-template <bool SOFTCAP, bool DUMP, bool SPLIT>
+template <bool SOFTCAP, bool DUMP, bool SPLIT, int PREP = -1>
 static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                         uint32_t idesc_qk, uint32_t idesc_pv, cudaStream_t st) {
   const int smem_bytes = c2::total + 1024;
   const dim3 grid((SPLIT ? p.n_q_tiles : (p.n_q_tiles + 1) / 2) * p.H * p.B);
-  auto kern = prefill2c_kernel<SOFTCAP, DUMP, SPLIT>;
+  auto kern = prefill2c_kernel<SOFTCAP, DUMP, SPLIT, PREP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return (int)e;
   if (g_ev_before && g_ev_after) cudaEventRecord(g_ev_before, st);
@@ -913,7 +1001,13 @@ static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 }
 
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
-                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, cudaStream_t st) {
+                     uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, int prep, cudaStream_t st) {
+  if (prep >= 0) {
+    if (p.dbg || p.perturb) return prep == RK_FMT_E4M3 ? launch2c_cfg<false, true, true, RK_FMT_E4M3>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
+                                                       : launch2c_cfg<false, true, true, RK_FMT_E5M2>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st);
+    return prep == RK_FMT_E4M3 ? launch2c_cfg<false, false, true, RK_FMT_E4M3>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
+                               : launch2c_cfg<false, false, true, RK_FMT_E5M2>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st);
+  }
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return split ? (softcap ? launch2c_cfg<true, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
                             : launch2c_cfg<false, true, true>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st))

@@ -490,3 +490,38 @@ def test_windows_that_mask_nothing_or_little(H, Sq, Skv, d, causal, q_pos0, beyo
         got = rk.attn_prefill(qc, kc, vc, qs, ks, vs, window=window, **kw)
         assert torch.equal(got[:, :, :-1], want[:, :, :-1]) and torch.equal(got[:, :, -1], want[:, :, -1]) == beyond, window
     assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("S_q,S_kv,d,fmt,kw", [(1, 1, 128, 0, {}), (17, 31, 64, 0, {}), (128, 128, 128, 0, {}), (129, 129, 64, 1, {}), (40, 33, 128, 0, dict(causal=False)), (200, 256, 128, 1, dict(q_pos0=56)),
+                                               (256, 256, 64, 0, dict(causal=False)), (7, 257, 64, 0, dict(q_pos0=250)), (300, 383, 128, 0, dict(q_pos0=83, window=100)), (130, 384, 64, 1, dict(causal=False)),
+                                               (384, 384, 128, 0, {}), (64, 128, 128, 0, dict(q_pos0=-70))])
+@pytest.mark.parametrize("hard", [False, True])
+def test_calls_that_prepare_their_operands_themselves(S_q, S_kv, d, fmt, kw, hard):
+    """Calls of up to three key tiles re-block V and order the scales inside the attention kernel: the same bits as with V re-blocked beforehand, which has the preparation launch. Edges of key
+    blocks and tiles, scales at odd addresses; hard: V of any code, zeros and subnormals, under scales that are close, far apart or extreme."""
+    B, H, H_kv = 2, 16, 8
+    g = torch.Generator(device="cuda").manual_seed(S_q + S_kv + d)
+    def odd(t):
+        flat = torch.empty(t.numel() + 1, dtype=torch.uint8, device="cuda")
+        flat[1:] = t.flatten()
+        return flat[1:].view(t.shape)
+    q, qs = rk.mx_quantize(torch.randn(B, H, S_q, d, generator=g, device="cuda"), fmt)
+    k, ks = rk.mx_quantize(torch.randn(B, H_kv, S_kv, d, generator=g, device="cuda"), fmt)
+    v, vs = rk.mx_quantize(torch.randn(B, H_kv, S_kv, d, generator=g, device="cuda"), fmt)
+    if hard:
+        v = torch.randint(0, 256, v.shape, generator=g, device="cuda", dtype=torch.uint8)
+        v[(v & 0x7F) >= (0x7F if fmt == 0 else 0x7C)] = 0x38
+        v[0, 0, :, :4] = 0
+        v[0, 1] &= 0x87 if fmt == 0 else 0x83
+        vs = torch.randint(118, 130, vs.shape, generator=g, device="cuda", dtype=torch.uint8)
+        vs[1, 0] = torch.randint(90, 140, vs[1, 0].shape, generator=g, device="cuda", dtype=torch.uint8)
+        vs[1, 1] = torch.randint(1, 30, vs[1, 1].shape, generator=g, device="cuda", dtype=torch.uint8)
+    kw = dict(dict(causal=True), **kw)
+    vr, vrs = rk.mx_rebase_v(v, vs, fmt)
+    lse = [torch.full((B, H, S_q), 7.0, device="cuda") for _ in range(3)]
+    want = rk.attn_prefill(q, k, vr, qs, ks, vrs, q_fmt=fmt, kv_fmt=fmt, v_scale_axis=rk.V_SCALES_ALONG_KEYS, lse=lse[0], **kw)
+    for i, shift in ((1, lambda t: t), (2, odd)):
+        got = rk.attn_prefill(q, k, v, shift(qs), shift(ks), shift(vs), q_fmt=fmt, kv_fmt=fmt, lse=lse[i], **kw)
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+        assert torch.equal(lse[i], lse[0])
+    assert rk.last_device_status() == 0
