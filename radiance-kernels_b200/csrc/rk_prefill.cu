@@ -820,13 +820,14 @@ int prefill_form(const rk_prefill_args& a, int64_t sms) {
   return tiles <= 3 * sms ? kFormTurns : kFormPairs;
 }
 
-// Calls whose attention kernel prepares its operands itself (rk_prefill2c.cu, PREP): 8-bit operands with row-major scales, V scaled along d, one query tile per CTA with both
+// Calls whose attention kernel prepares its operands itself (rk_prefill2c.cu, PREP): 8-bit operands with row-major scales, one query tile per CTA with both
 // softmax groups on every key tile, and of those at most as many as there are stages.  Time over that of the same call with the preparation launch, 180 calls of 1 to 144 heads: one key
 // tile 0.59-0.84, two 0.67-0.72 (d = 64) and 0.89-0.99 (d = 128), three 0.70-0.80 and, with six units of V for three groups of warps, 0.82-1.04: from 16 KV heads on 0.82-0.96, below 0.98-1.04.
 bool prefill_prepares(const rk_prefill_args& a) {
   const int kv_tiles = (a.S_kv + kBlockN - 1) / kBlockN;
-  return a.d <= 128 && a.q_fmt <= RK_FMT_E5M2 && a.kv_fmt <= RK_FMT_E5M2 && a.v_scale_axis == RK_V_SCALES_ALONG_D && a.q_scale_layout == RK_SCALES_ROWMAJOR &&
-         a.k_scale_layout == RK_SCALES_ROWMAJOR && a.softcap <= 0.0f && (kv_tiles < 3 || (kv_tiles == 3 && (a.d <= 64 || (int64_t)a.B * a.H_kv >= 16))) &&
+  const bool rebase = a.v_scale_axis == RK_V_SCALES_ALONG_D;
+  return a.d <= 128 && a.q_fmt <= RK_FMT_E5M2 && a.kv_fmt <= RK_FMT_E5M2 && a.v_scale_layout == RK_SCALES_ROWMAJOR && a.q_scale_layout == RK_SCALES_ROWMAJOR &&
+         a.k_scale_layout == RK_SCALES_ROWMAJOR && a.softcap <= 0.0f && (kv_tiles < 3 || (kv_tiles == 3 && (!rebase || a.d <= 64 || (int64_t)a.B * a.H_kv >= 16))) &&
          (g_prefill_form ? g_prefill_form : prefill_form(a, num_sms())) == kFormSplit;
 }
 
@@ -883,7 +884,7 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
     if (rc != RK_OK) return rc;
     const int form = g_prefill_form ? g_prefill_form : prefill_form(a, num_sms());
     if (form == kFormTurns) return launch_prefill1(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, st);
-    return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, form == kFormSplit, prepares ? a.kv_fmt : -1, st);
+    return launch_prefill2c(tq, tk, tv, to, p, idesc_qk, idesc_pv, cap, form == kFormSplit, !prepares ? -1 : a.v_scale_axis == RK_V_SCALES_ALONG_D ? a.kv_fmt : 2 /* its scales alone */, st);
   }
   if (p.dbg || p.perturb)      // the tests' stage dump and delays live in instantiations of their own: the kernels that ship carry none of their code
     return cap ? launch_cfg<2, 2, true, true>(tq, tk, tv, p, idesc_qk, idesc_pv, grid, st)

@@ -100,6 +100,7 @@ struct __align__(16) Work {
 static_assert(sizeof(Work) == 32, "its place in shared memory");
 constexpr int kReaders = 8 + 4 + 2;      // warps that read an item: softmax, correction, Q K^T, P V
 constexpr int bPrep = bClc;              // PREP: the scale atoms of Q and K are there (no second item is asked for)
+constexpr int kPrepScales = 2;           // PREP beside the formats: V is scaled along the keys and comes as it lies, only its scales have to be put into atoms
 }  // namespace c2
 
 // ---- softmax warps: thread = query row -----------------------------------------------------------------------
@@ -621,7 +622,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) RK_STAMP(2, 0, 6);
   constexpr int kQt = SPLIT ? 1 : 2;                                  // query tiles per item
-  constexpr bool kPrep = PREP >= 0;
+  constexpr bool kPrep = PREP >= 0, kPrepV = kPrep && PREP < kPrepScales;
   constexpr int kAtomTx = kPrep ? 0 : kSfAtomBytes;                   // of Q and K, by copy
   const int n_pairs = (p.n_q_tiles + kQt - 1) / kQt;
   auto decode = [&](uint32_t block) -> Work {
@@ -661,10 +662,10 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                  kSfAtomBytes, &bars[bKF + st]);
   };
   auto issue_v = [&](int j, int st) {
-    mbar_arrive_expect_tx(&bars[bVF + st], p.kv_tile_tx + kSfAtomBytes);
+    mbar_arrive_expect_tx(&bars[bVF + st], p.kv_tile_tx + kAtomTx);
     const int key = (j + w.j0) * kBlockN;            // transposed V: [d][keys]
     tma_load_3d(smem + v_off + st * kTileBytes, &tmap_v, &bars[bVF + st], p.v_transposed ? key : 0, p.v_transposed ? 0 : key, w.bhkv);
-    bulk_load_1d(smem + sfv_off + st * kSfAtomBytes, p.v_sf + ((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * kSfAtomBytes,
+    if (!kPrep) bulk_load_1d(smem + sfv_off + st * kSfAtomBytes, p.v_sf + ((size_t)w.bhkv * p.n_kv_tiles + j + w.j0) * kSfAtomBytes,
                  kSfAtomBytes, &bars[bVF + st]);
   };
   // The TMA warp sets up the barriers and goes on to its loads without waiting for the others, so that their latency runs under the
@@ -674,7 +675,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       const bool per_warp = (i >= bSE && i < bSE + 2) || (i >= bPF && i < bPF + 4) || (i >= bOR && i < bOR + 4);
       // SPLIT: both groups hand back S and write P, and the exchange takes a warp of each
       const bool both = SPLIT && (i < bPV || i >= bCF + 16) && i < bOR;
-      mbar_init(&bars[i], per_warp ? (both ? 8 : 4) : both && i >= bCF + 16 ? 2 : i == bWE ? kReaders : kPrep && i >= bVF && i < bVF + kStages ? (p.d > 64 ? 8 : 4) : kPrep && i == bPrep ? 3 : 1);
+      mbar_init(&bars[i], per_warp ? (both ? 8 : 4) : both && i >= bCF + 16 ? 2 : i == bWE ? kReaders : kPrep && i >= bVF && i < bVF + kStages ? (!kPrepV ? 2 : p.d > 64 ? 8 : 4) : kPrep && i == bPrep ? 3 : 1);
     }
     if (lane == 0) *abort_flag = 0;
     fence_barrier_init();
@@ -720,6 +721,17 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[bPrep]);
+    } else if (!kPrepV) {
+      if (warp < w.nt0 && __shfl_sync(0xffffffffu, lane == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0, 0) == 0) {      // V's scales: a warp per key tile
+        const int nkb = (p.S_kv + 31) / 32, block = (warp + w.j0) * 4;
+        uint32_t words[4];
+        key_scale_words(p.v_sf + ((int64_t)w.bhkv * nkb + block) * p.d + lane * 4, p.d, nkb - block, lane * 4 < p.d, (reinterpret_cast<uintptr_t>(p.v_sf) & 3) == 0, words);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(smem + sfv_off + warp * kSfAtomBytes + sf_atom_offset(lane * 4 + i, 0)) = words[i];
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[bVF + warp]);
+      }
     } else if (warp < kWarpTma) {
       // V, by the twelve warps that have nothing to do before the first scores are there: units of 64 columns, in the order of the tiles; the correction warps, which are needed last, take
       // the fourth as well.  Where an earlier launch gave up V does not come, and O is not written.
@@ -728,7 +740,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll 1
         for (int i = grp; i < n; i += grp == 2 ? (i == 2 ? 1 : n) : 4) {
           const int st = units == 2 ? i >> 1 : i;
-          rebase_v_unit<PREP>(p, smem, warp, lane, st, st + w.j0, units == 2 ? i & 1 : 0, w.bhkv);
+          rebase_v_unit<kPrepV ? PREP : 0>(p, smem, warp, lane, st, st + w.j0, units == 2 ? i & 1 : 0, w.bhkv);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[bVF + st]);
@@ -780,7 +792,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               if (use > 0 && !mbar_wait_compact<true>(&bars[bKE + st], (use - 1) & 1, abort_flag)) { fail = 201; break; }
               issue_kv(j, st);
               if (stopped) break;                    // O is written only where V has come
-              if (kPrep) { ++st; continue; }         // (a stage for every tile)
+              if (kPrepV) { ++st; continue; }        // (a stage for every tile)
               if (use > 0 && !mbar_wait_compact<true>(&bars[bVE + st], (use - 1) & 1, abort_flag)) { fail = 202; break; }
               issue_v(j, st);
               if (++st == kStages) { st = 0; ++use; }
@@ -813,7 +825,7 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < kStages; ++i) {
           const uint32_t nv = use + (i < st), nk = nv + (i == st && k_ahead);      // loads into this stage
-          want |= (uint32_t)(nk > 0) << (bKF + i) | (uint32_t)(nv > 0 && !kPrep) << (bVF + i);
+          want |= (uint32_t)(nk > 0) << (bKF + i) | (uint32_t)(nv > 0 && !kPrepV) << (bVF + i);
           par |= ((nk - 1) & 1) << (bKF + i) | ((nv - 1) & 1) << (bVF + i);
         }
 #pragma unroll 1
@@ -1002,6 +1014,9 @@ static int launch2c_cfg(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 
 int launch_prefill2c(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                      uint32_t idesc_qk, uint32_t idesc_pv, bool softcap, bool split, int prep, cudaStream_t st) {
+  if (prep == c2::kPrepScales)
+    return p.dbg || p.perturb ? launch2c_cfg<false, true, true, c2::kPrepScales>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
+                              : launch2c_cfg<false, false, true, c2::kPrepScales>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st);
   if (prep >= 0) {
     if (p.dbg || p.perturb) return prep == RK_FMT_E4M3 ? launch2c_cfg<false, true, true, RK_FMT_E4M3>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st)
                                                        : launch2c_cfg<false, true, true, RK_FMT_E5M2>(tq, tk, tv, to, p, idesc_qk, idesc_pv, st);

@@ -1169,19 +1169,7 @@ RK_DEVINL void retile_atom(const RetileJob& job, int64_t atom, int64_t total) {
   uint32_t w[4];
   if (job.kind == kKeys) {                  // four adjacent columns of the four key blocks, turned
     const int64_t col = ch * 128 + lane * 4;
-    const uint8_t* const in = job.in + (bt * nkb + tile * 4) * d + col;
-    const bool words = (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;      // (d is a multiple of 32)
-    uint32_t r[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      r[k] = 0x7F7F7F7Fu;
-      if (col < d && tile * 4 + k < nkb) {
-        if (words) r[k] = *reinterpret_cast<const uint32_t*>(in + k * d);
-        else r[k] = in[k * d] | ((uint32_t)in[k * d + 1] << 8) | ((uint32_t)in[k * d + 2] << 16) | ((uint32_t)in[k * d + 3] << 24);
-      }
-    }
-    const uint32_t a = __byte_perm(r[0], r[1], 0x5140), b = __byte_perm(r[2], r[3], 0x5140), c = __byte_perm(r[0], r[1], 0x7362), e = __byte_perm(r[2], r[3], 0x7362);
-    w[0] = __byte_perm(a, b, 0x5410); w[1] = __byte_perm(a, b, 0x7632); w[2] = __byte_perm(c, e, 0x5410); w[3] = __byte_perm(c, e, 0x7632);
+    key_scale_words(job.in + (bt * nkb + tile * 4) * d + col, d, (int)min((int64_t)4, nkb - tile * 4), col < d, (reinterpret_cast<uintptr_t>(job.in) & 3) == 0, w);      // (d is a multiple of 32)
 #pragma unroll
     for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(out + sf_atom_offset(lane * 4 + i, 0)) = w[i];
     return;

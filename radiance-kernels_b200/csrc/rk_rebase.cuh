@@ -55,6 +55,22 @@ __device__ __noinline__ void rebase_slow(const uint8_t* cb, const uint8_t* sb, i
   }
 }
 
+// Scales along the keys, row-major [key blocks][d]: four adjacent columns of a tile's four key blocks (n_blocks of them exist; in: its first, at the first of the columns) as words of
+// a scale atom, a word per column.
+RK_DEVINL void key_scale_words(const uint8_t* in, int64_t d, int n_blocks, bool exist, bool aligned, uint32_t (&w)[4]) {
+  uint32_t r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    r[k] = 0x7F7F7F7Fu;
+    if (exist && k < n_blocks) {
+      if (aligned) r[k] = *reinterpret_cast<const uint32_t*>(in + k * d);
+      else r[k] = in[k * d] | ((uint32_t)in[k * d + 1] << 8) | ((uint32_t)in[k * d + 2] << 16) | ((uint32_t)in[k * d + 3] << 24);
+    }
+  }
+  const uint32_t a = __byte_perm(r[0], r[1], 0x5140), b = __byte_perm(r[2], r[3], 0x5140), c = __byte_perm(r[0], r[1], 0x7362), e = __byte_perm(r[2], r[3], 0x7362);
+  w[0] = __byte_perm(a, b, 0x5410); w[1] = __byte_perm(a, b, 0x7632); w[2] = __byte_perm(c, e, 0x5410); w[3] = __byte_perm(c, e, 0x7632);
+}
+
 // ---- V re-blocking: scales along d -> MX blocks along the keys --------------------------------------------------------
 // Decode exactly, then the block rule down each column: the same as decoding to fp32 and quantizing again.  The hot form does
 // it in f16: a pair of codes goes through the hardware converter, times the row's scale relative to the block's largest, the

@@ -497,7 +497,7 @@ def test_windows_that_mask_nothing_or_little(H, Sq, Skv, d, causal, q_pos0, beyo
                                                (384, 384, 128, 0, {}), (64, 128, 128, 0, dict(q_pos0=-70))])
 @pytest.mark.parametrize("hard", [False, True])
 def test_calls_that_prepare_their_operands_themselves(S_q, S_kv, d, fmt, kw, hard):
-    """Calls of up to three key tiles re-block V and order the scales inside the attention kernel: the same bits as with V re-blocked beforehand, which has the preparation launch. Edges of key
+    """Calls of up to three key tiles re-block V and order the scales inside the attention kernel: the same bits as by pairs of query tiles, which have the preparation launch, V scaled along d or along the keys. Edges of key
     blocks and tiles, scales at odd addresses; hard: V of any code, zeros and subnormals, under scales that are close, far apart or extreme."""
     B, H, H_kv = 2, 16, 8
     g = torch.Generator(device="cuda").manual_seed(S_q + S_kv + d)
@@ -518,10 +518,14 @@ def test_calls_that_prepare_their_operands_themselves(S_q, S_kv, d, fmt, kw, har
         vs[1, 1] = torch.randint(1, 30, vs[1, 1].shape, generator=g, device="cuda", dtype=torch.uint8)
     kw = dict(dict(causal=True), **kw)
     vr, vrs = rk.mx_rebase_v(v, vs, fmt)
-    lse = [torch.full((B, H, S_q), 7.0, device="cuda") for _ in range(3)]
-    want = rk.attn_prefill(q, k, vr, qs, ks, vrs, q_fmt=fmt, kv_fmt=fmt, v_scale_axis=rk.V_SCALES_ALONG_KEYS, lse=lse[0], **kw)
-    for i, shift in ((1, lambda t: t), (2, odd)):
-        got = rk.attn_prefill(q, k, v, shift(qs), shift(ks), shift(vs), q_fmt=fmt, kv_fmt=fmt, lse=lse[i], **kw)
-        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
-        assert torch.equal(lse[i], lse[0])
+    lse = [torch.full((B, H, S_q), 7.0, device="cuda") for _ in range(2)]
+    along_keys = dict(v_scale_axis=rk.V_SCALES_ALONG_KEYS)
+    with prefill_form(PAIRS):
+        want = rk.attn_prefill(q, k, vr, qs, ks, vrs, q_fmt=fmt, kv_fmt=fmt, lse=lse[0], **along_keys, **kw)
+    for shift in (lambda t: t, odd):
+        for axis, codes, scales in (({}, v, vs), (along_keys, vr, vrs)):
+            lse[1].fill_(7.0)
+            got = rk.attn_prefill(q, k, codes, shift(qs), shift(ks), shift(scales), q_fmt=fmt, kv_fmt=fmt, lse=lse[1], **axis, **kw)
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+            assert torch.equal(lse[1], lse[0])
     assert rk.last_device_status() == 0
