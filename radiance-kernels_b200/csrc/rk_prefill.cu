@@ -822,7 +822,7 @@ int prefill_form(const rk_prefill_args& a, int64_t sms) {
 
 // Calls whose attention kernel prepares its operands itself (rk_prefill2c.cu, PREP): 8-bit operands with row-major scales, one query tile per CTA with both
 // softmax groups on every key tile, and of those at most as many as there are stages.  Time over that of the same call with the preparation launch, 180 calls of 1 to 144 heads: one key
-// tile 0.59-0.84, two 0.67-0.72 (d = 64) and 0.89-0.99 (d = 128), three 0.70-0.80 and, with six units of V for three groups of warps, 0.82-1.04: from 16 KV heads on 0.82-0.96, below 0.98-1.04.
+// tile 0.59-0.84, two 0.67-0.72 (d = 64) and 0.89-0.99 (d = 128), three 0.70-0.80 and, with six units of V for three groups of warps, 0.82-1.04: from 16 KV heads on 0.82-0.96, below 0.98-1.04.  V scaled along the keys: 0.62-0.90.
 bool prefill_prepares(const rk_prefill_args& a) {
   const int kv_tiles = (a.S_kv + kBlockN - 1) / kBlockN;
   const bool rebase = a.v_scale_axis == RK_V_SCALES_ALONG_D;

@@ -34,7 +34,7 @@
 // on the same tile, group A on keys 0-63 of each key tile and group B on keys 64-127, and exchange their row maxima through
 // shared memory.
 //
-// SPLIT with PREP = the format of K and V (E4M3, E5M2): the preparation of a small call, which is otherwise a launch of its own.  The issuers and the warp that fills the warpgroup put the
+// SPLIT with PREP = the format of K and V (E4M3, E5M2; kPrepScales where V is scaled along the keys): the preparation of a small call, which is otherwise a launch of its own.  The issuers and the warp that fills the warpgroup put the
 // row-major scales of Q and K into atoms, softmax and correction warps re-block V, scaled along d, into the stages V is read from, in the time Q and K take to arrive and the
 // first scores to be formed: there is a stage for every key tile.  A query tile of every head re-blocks V for itself, so this is for items of at most three key tiles and grids
 // of one round of the SMs.  (A launch whose results the next one waits for costs 1.2 us,
