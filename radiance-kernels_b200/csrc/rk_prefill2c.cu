@@ -571,7 +571,7 @@ __device__ __forceinline__ void rebase_v_unit(const PrefillParams& p, uint8_t* s
   uint8_t* const atom = smem + sfv_off + st * kSfAtomBytes;
   uint32_t sc[2];
   auto at = [=](int k, int c) { return dst + k * 128 + (((c >> 4) ^ (k & 7)) << 4) + (c & 15); };
-  rebase_block<FMT, 8, true>(p.v + row0 * p.d, p.v_sf + row0 * (p.d / 32), p.d, cu, n, reinterpret_cast<uint32_t (*)[32]>(smem + stage_off + warp * 256), lane,
+  rebase_block<FMT, 8, true, int>(p.v + row0 * p.d, p.v_sf + row0 * (p.d / 32), p.d, cu, n, reinterpret_cast<uint32_t (*)[32]>(smem + stage_off + warp * 256), lane,
                              [=](int k, const uint32_t (&o)[2]) { *reinterpret_cast<uint2*>(at(k, col)) = make_uint2(o[0], o[1]); },
                              [=](int k, int c, uint8_t code) { *at(k, col + c) = code; }, sc);
 #pragma unroll

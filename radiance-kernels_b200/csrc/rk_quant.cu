@@ -21,6 +21,7 @@
 // to it on every finite fp32 input (all 2^32 bit patterns are swept in the GPU
 // tests); blocks that hold a NaN or an infinity take the integer encoder.
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "rk_common.cuh"
@@ -1222,8 +1223,9 @@ __global__ void __launch_bounds__(128) retile_scales_kernel(const RetileJobs job
 // 67 M codes E4M3: 53 us in integer arithmetic on the codes (12 instructions per code, 16 warps per SM, rows with a zero or
 // subnormal code on a path of their own), 31.6 us here beside the scales' re-tiling.  (All columns of 128 keys by one CTA: 30.4, but 33.5 M codes 18.8 -> 19.8 and calls of few
 // keys 0.2 us more.  On the codes as bytes, where a power of two is a step of 8: 35 us, and 55 with the words done again in which a code is or becomes subnormal.)
+// Idx: of an element within 32 rows; int64_t where these are longer than 2^31 bytes (for all calls: 33.5 M codes 13.6 -> 13.9 us).
 constexpr int kRebaseThreads = 128;
-template <int FMT, bool TILED, int NC>
+template <int FMT, bool TILED, int NC, class Idx = int>
 __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
                                                                  int64_t batch, int64_t S, int64_t d, uint8_t* __restrict__ out_codes,
                                                                  uint8_t* __restrict__ out_scales, const RetileJobs jobs) {
@@ -1253,13 +1255,13 @@ __global__ void __launch_bounds__(kRebaseThreads, 7) rebase_v_kernel(const uint8
     const bool in = col < d && n > 0;
     uint32_t sc[CP];
     uint8_t* const dst = out_codes + row0 * d + col;
-    const int di = (int)d;
-    rebase_block<FMT, NC, false>(codes + row0 * d, scales + row0 * nbd, (int)d, (int)cu, n, fac_sm[warp], lane,
-                                 [=](int k, const uint32_t (&o)[NW]) {
-                                   if (NC == 8) *reinterpret_cast<uint2*>(dst + k * di) = make_uint2(o[0], o[NW - 1]);
-                                   else *reinterpret_cast<uint32_t*>(dst + k * di) = o[0];
-                                 },
-                                 [=](int k, int c, uint8_t code) { dst[k * di + c] = code; }, sc);
+    const Idx di = (Idx)d;
+    rebase_block<FMT, NC, false, Idx>(codes + row0 * d, scales + row0 * nbd, di, (Idx)cu, n, fac_sm[warp], lane,
+                                      [=](int k, const uint32_t (&o)[NW]) {
+                                        if (NC == 8) *reinterpret_cast<uint2*>(dst + k * di) = make_uint2(o[0], o[NW - 1]);
+                                        else *reinterpret_cast<uint32_t*>(dst + k * di) = o[0];
+                                      },
+                                      [=](int k, int c, uint8_t code) { dst[k * di + c] = code; }, sc);
     if (TILED) {
       // the four warps' scale bytes of a column are one word of its atom
 #pragma unroll
@@ -1746,15 +1748,17 @@ int launch_kv_append(const float* k_new, const float* v_new, int B, int H_kv, in
 
 int launch_rebase_v(const uint8_t* codes, const uint8_t* scales, int64_t batch, int64_t S, int64_t d, int fmt,
                     uint8_t* out_codes, uint8_t* out_scales, bool tiled, cudaStream_t st, RetileJobs jobs) {
-  const bool wide = ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out_codes)) & 7) == 0;
+  const bool small = d <= INT_MAX / 32;                  // 32 rows can be indexed by an int
+  const bool wide = small && ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out_codes)) & 7) == 0;
   const int64_t units = batch * ((S + 127) / 128) * (wide ? (d + 63) / 64 : d / 32);
   if (units == 0) return RK_OK;
   jobs.ctas = retile_ctas(jobs, kRebaseThreads);
   const dim3 grid(jobs.ctas + grid_for(units * kRebaseThreads, kRebaseThreads, 28)), block(kRebaseThreads);      // four waves of the resident CTAs
-#define RK_RB(TI, N) RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, TI, N>, grid, block, 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs))
-  if (wide) { if (tiled) { RK_RB(true, 8); } else { RK_RB(false, 8); } }
+#define RK_RB(TI, N, IDX) RK_DISPATCH_FMT(fmt, return (int)launch_pdl(rebase_v_kernel<F, TI, N, IDX>, grid, block, 0, st, codes, scales, batch, S, d, out_codes, out_scales, jobs))
+  if (wide) { if (tiled) { RK_RB(true, 8, int); } else { RK_RB(false, 8, int); } }
   else if (tiled) return RK_ERR_MISALIGNED;              // (prefill's codes and workspace lie on 16-byte boundaries)
-  else { RK_RB(false, 4); }
+  else if (small) { RK_RB(false, 4, int); }
+  else { RK_RB(false, 4, int64_t); }
 #undef RK_RB
   return RK_OK;
 }

@@ -114,12 +114,13 @@ template <int FMT> RK_DEVINL uint32_t encode_f16x4(uint32_t lo, uint32_t hi) {
 // One warp's 32 keys x 8 NC columns (unit cu of them): codes and scales are those of the block's first key, n keys exist.  A lane has keys k0 = 8 (lane / 8) to k0 + 7 and NC
 // adjacent columns; put(key, words) takes its codes of a key, put_byte(key, column of its NC, code) one of them in the slow form.  ALL: put is called for keys that do
 // not exist as well, with zeros.  sc: the new scale codes of columns NC (lane % 8) + (NC / 4) (lane / 8) + 0 .. of the unit.  fac_sm: scratch of this warp.
-template <int FMT, int NC, bool ALL, class Put, class PutByte>
-RK_DEVINL void rebase_block(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, int d, int cu, int n, uint32_t (*fac_sm)[32], int lane, Put put,
+// Idx: of an element within the 32 rows of d columns; int where d <= INT_MAX / 32, as in the attention calls.
+template <int FMT, int NC, bool ALL, class Idx, class Put, class PutByte>
+RK_DEVINL void rebase_block(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, Idx d, Idx cu, int n, uint32_t (*fac_sm)[32], int lane, Put put,
                             PutByte put_byte, uint32_t (&sc)[NC / 4]) {
   constexpr int NW = NC / 4, NB = NC / 4, CP = NC / 4;             // words per key of a thread; 32-column blocks of a warp; columns of a lane's quarter
   const int k0 = (lane >> 3) * 8, b = (lane & 7) * NC / 32;
-  const int nbd = d >> 5, col = cu * 8 * NC + (lane & 7) * NC;
+  const Idx nbd = d >> 5, col = cu * 8 * NC + (lane & 7) * NC;
   const bool in = col < d && n > 0;
   const uint8_t* src = codes + col;
   const uint8_t* const src0 = src + k0 * d;

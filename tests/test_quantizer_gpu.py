@@ -242,6 +242,30 @@ def test_rebase_of_codes_on_a_four_byte_boundary(S, d, fmt):
         assert np.array_equal(np_(rc[b]), oc) and np.array_equal(np_(rs[b]), os_)
 
 
+@pytest.mark.parametrize("shift", [0, 4])
+def test_rebase_of_rows_whose_block_is_longer_than_two_gigabytes(shift):
+    """Rows of so many columns that the last of a block's 32 keys lies 2^31 bytes behind the first, and one key more: columns repeat every 2048, so the result of
+    2048 of them says what all are.  Half the blocks of a row take the form through fp32 (scales that span more than 2^14)."""
+    S, period = 33, 2048
+    copies = -(-2 ** 31 // (31 * period)) + 1
+    d = copies * period
+    assert 31 * (d - period) >= 2 ** 31
+    rng = np.random.default_rng(82)
+    codes = rng.integers(0, 256, size=(S, period), dtype=np.uint8)
+    codes[(codes & 0x7F) == 0x7F] = 0x7E
+    scales = rng.integers(120, 130, size=(S, period // 32), dtype=np.uint8)
+    scales[:, ::2] = rng.integers(100, 140, size=(S, period // 64), dtype=np.uint8)
+    c = torch.empty(S * d + shift, dtype=torch.uint8, device="cuda")[shift:].view(S, copies, period)
+    c.copy_(torch.from_numpy(codes).cuda()[:, None])
+    s = torch.from_numpy(scales).cuda()[:, None].expand(S, copies, period // 32).contiguous()
+    rc, rs = rk.mx_rebase_v(c.view(S, d), s.view(S, d // 32))
+    oc, os_ = oracle.rebase_v(codes, scales)
+    for got, want in ((rs.view(2, copies, period), os_), (rc.view(S, copies, period), oc)):
+        want = torch.from_numpy(np.ascontiguousarray(want)).cuda()
+        for i in range(got.shape[0]):
+            assert (got[i] == want[i]).all(), i
+
+
 @pytest.mark.parametrize("copies,S,d", [(37, 2051, 128), (2, 18945, 256)])
 def test_rope_quantize_two_rows_of_a_position_per_thread(copies, S, d):
     """Large inputs: two rows of one position share a thread's reads of the caches (an odd number of rows leaves one alone);
