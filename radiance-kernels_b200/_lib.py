@@ -105,6 +105,10 @@ def lib():
         L.rk_debug_set_ring_stop.argtypes = [C.c_int]
         L.rk_debug_rope_by_copies.restype = C.c_int
         L.rk_debug_rope_by_copies.argtypes = [C.c_int64, C.c_int, C.c_int64, C.c_int]
+        L.rk_debug_set_rmsnorm_form.restype = None
+        L.rk_debug_set_rmsnorm_form.argtypes = [C.c_int]
+        L.rk_debug_rmsnorm_form.restype = C.c_int
+        L.rk_debug_rmsnorm_form.argtypes = [C.c_int64, C.c_int, C.c_int, C.c_int]
         L.rk_debug_set_decode_path.restype = None
         L.rk_debug_set_decode_path.argtypes = [C.c_int]
         L.rk_debug_mxfp8_mma_loop.restype = C.c_int

@@ -587,6 +587,11 @@ RK_API void rk_debug_set_ring_stop(int role) { g_ring_stop = role; }
 /* Test hook (not in the public header): 1 where RoPE + quantization of so many rows goes through bulk copies on a device of `sms` SMs. */
 RK_API int rk_debug_rope_by_copies(int64_t rows, int d, int64_t seq_len, int sms) { return rope_by_copies(rows, d, seq_len, sms) ? 1 : 0; }
 
+/* Test hooks (not in the public header): the form (RmsnormForm: 1 staged, 2 ring) the next RMSNorm calls take that can, 0 = the one the rule chooses; and
+ * the form that a call with x and gamma on 16-byte boundaries takes on a device of `sms` SMs (0 = the current one). */
+RK_API void rk_debug_set_rmsnorm_form(int form) { g_rmsnorm_form = form; }
+RK_API int rk_debug_rmsnorm_form(int64_t rows, int K, int bf16, int sms) { return rmsnorm_form(rows, K, bf16 != 0, sms > 0 ? sms : num_sms()); }
+
 /* Test hook (not in the public header): 0 = choose the decode kernel by shape, 1 = always the mma.sync kernel. */
 RK_API void rk_debug_set_decode_path(int path) { g_decode_path = path; }
 

@@ -48,6 +48,9 @@ int launch_prefill(const rk_prefill_args& a, const uint8_t* q_codes, const uint8
                    const uint8_t* q_sf, const uint8_t* k_sf, const uint8_t* v_sf, bool prepares, cudaStream_t st);
 bool prefill_prepares(const rk_prefill_args& a);
 
+// RMSNorm: rows staged through registers, by bulk copies in a ring with a chain per lane, or whole on the chip with their chains cut into segments.
+enum RmsnormForm { kRmsnormStaged = 1, kRmsnormRing = 2, kRmsnormSegments = 3 };
+int rmsnorm_form(int64_t rows, int K, bool bf16, int64_t sms);               // which of them a call with x and gamma on 16-byte boundaries takes
 bool rope_by_copies(int64_t rows, int d, int64_t seq_len, int64_t sms);      // which RoPE kernel a call without positions of its own takes
 // Which kernel a prefill call takes on a device of `sms` SMs: d = 256, pairs of query tiles, one query tile at a time with the softmax groups on alternate
 // key tiles, one query tile per CTA with both groups on every key tile.
@@ -65,6 +68,7 @@ int launch_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile, int iter
 int launch_wait_runs_out(int limit_us, bool noalloc, cudaStream_t st);   // test hook: a bounded wait that must give up
 int launch_compact_wait_runs_out(bool longer, bool aborted, cudaStream_t st);      // test hook: the same for the waits bounded by a number of polls
 extern int g_ring_stop;                                     // test hook: a role of the RoPE and RMSNorm kernels' rings of copies acts as if its wait had run out
+extern int g_rmsnorm_form;                                  // test hook: RmsnormForm of the next calls that can take it (staged; ring), 0 = by the rule
 extern int g_decode_path;                                   // test hook: 0 = by shape, 1 = mma.sync kernel only
 bool decode_uses_tc(const rk_decode_args& a);                // true when the tcgen05 decode kernel serves this call
 size_t decode_workspace_bytes(const rk_decode_args& a, int num_splits);   // of the kernel that serves the call, at its full grid

@@ -31,6 +31,7 @@
 namespace rk {
 
 int g_ring_stop = 0;   // set by rk_debug_set_ring_stop (tests only)
+int g_rmsnorm_form = 0;   // set by rk_debug_set_rmsnorm_form (tests only)
 
 template <int FMT> RK_DEVINL uint32_t ref_encode4(float a, float b, float c, float d) {
   return encode_rne<FMT>(a) | (encode_rne<FMT>(b) << 8) | (encode_rne<FMT>(c) << 16) | (encode_rne<FMT>(d) << 24);
@@ -1617,12 +1618,25 @@ int launch_import_kt_blocks(const uint8_t* kt, const uint8_t* kts, int64_t heads
   return (int)cudaGetLastError();
 }
 
+// Which kernel a call takes; `wide`: x and gamma lie on 16-byte boundaries.
+// Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so, one call behind another on the same buffers: 4096 bf16
+// columns, 8192 rows 36.5 31.8, one 17.1 15.5; 12288 columns, 1500 rows 64.7 51.7; 2048 columns, 1 and 64 rows 9.0 9.2, 300 10.9 10.2, 4096 15.5 14.1, 16384 37.4
+// 34.2; 1536 columns, 64 7.4 7.6, 300 8.7 8.3, 4096 12.3 11.6; 1024 columns, 64 5.8 6.0, 300 6.6 6.5, 4096 9.3 9.2, 9000 12.3 11.5; 512 columns 2-9 % slower
+// throughout), and not for fp32, whose 134 MB of 8192 x 4096 come from HBM twice either way (55.0 56.4; one row 17.4 20.3).
+static int rmsnorm_form(int64_t rows, int K, bool bf16, bool wide, int64_t sms, rms_seg::Shape& f) {
+  if (g_rmsnorm_form == kRmsnormStaged || (g_rmsnorm_form == kRmsnormRing && wide && bf16)) return g_rmsnorm_form;
+  if (wide && rms_seg::pays(rows, K, bf16, sms, f)) return kRmsnormSegments;
+  return wide && bf16 && (K >= 2048 || (K >= 1024 && rows >= 4096)) ? kRmsnormRing : kRmsnormStaged;
+}
+int rmsnorm_form(int64_t rows, int K, bool bf16, int64_t sms) { rms_seg::Shape f; return rmsnorm_form(rows, K, bf16, true, sms, f); }
+
 int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const float* gamma, float eps, int fmt,
                             bool unit_scale, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
   if (rows == 0 || K == 0) return RK_OK;
   const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma)) & 15) == 0;
   rms_seg::Shape f;
-  if (wide && rms_seg::pays(rows, K, bf16, num_sms(), f)) {
+  const int form = rmsnorm_form(rows, K, bf16, wide, num_sms(), f);
+  if (form == kRmsnormSegments) {
     int* status = device_status_word();
     if (!status) return RK_ERR_NO_DEVICE;
 #define RK_RN(BF, UN) RK_DISPATCH_FMT(fmt, {                                                                                \
@@ -1637,11 +1651,7 @@ int launch_rmsnorm_quantize(const void* x, bool bf16, int64_t rows, int K, const
     else      { if (unit_scale) { RK_RN(false, true); } else { RK_RN(false, false); } }
 #undef RK_RN
   }
-  // Rows by bulk copy: from a chain long enough to pay for the ring (us, staged through registers and so, one call behind another on the same buffers: 4096 bf16
-  // columns, 8192 rows 36.5 31.8, one 17.1 15.5; 12288 columns, 1500 rows 64.7 51.7; 2048 columns, 1 and 64 rows 9.0 9.2, 300 10.9 10.2, 4096 15.5 14.1, 16384 37.4
-  // 34.2; 1536 columns, 64 7.4 7.6, 300 8.7 8.3, 4096 12.3 11.6; 1024 columns, 64 5.8 6.0, 300 6.6 6.5, 4096 9.3 9.2, 9000 12.3 11.5; 512 columns 2-9 % slower
-  // throughout), and not for fp32, whose 134 MB of 8192 x 4096 come from HBM twice either way (55.0 56.4; one row 17.4 20.3).
-  if (wide && bf16 && (K >= 2048 || (K >= 1024 && rows >= 4096))) {
+  if (form == kRmsnormRing) {
     int* status = device_status_word();
     if (!status) return RK_ERR_NO_DEVICE;
     const int64_t slots = (int64_t)num_sms() * rmb::kCtasPerSm, waves = (rows + slots * rmb::kMaxRows - 1) / (slots * rmb::kMaxRows);

@@ -1,5 +1,6 @@
 """RMSNorm fused with the MX quantizer (the QKV-projection prologue of kernels/rmsnorm_qkv_fused) on the GPU: codes and
 scales bit-exact with the reference's rmsnorm golden followed by the block quantizer."""
+import contextlib
 import os
 
 import numpy as np
@@ -161,3 +162,39 @@ def test_fused_chains_of_large_calls(rows, K, first):
     torch.cuda.synchronize()
     assert np.array_equal(np_(s), want_s)
     assert np.array_equal(np_(c), want_c)
+
+
+STAGED, RING, SEGMENTS = 1, 2, 3
+
+
+@contextlib.contextmanager
+def rmsnorm_form(form):
+    """RMSNorm calls take this form (rows staged through registers; by bulk copies in a ring, bf16 alone)."""
+    rk.lib().rk_debug_set_rmsnorm_form(form)
+    try:
+        yield
+    finally:
+        rk.lib().rk_debug_set_rmsnorm_form(0)
+
+
+@pytest.mark.parametrize("form,rows,K,bf16,fmt,unit", [
+    (RING, 1, 2048, True, 0, False), (RING, 33, 2080, True, 0, False), (RING, 300, 1056, True, 1, False), (RING, 37, 4128, True, 2, True), (RING, 298, 4128, True, 3, False),
+    (RING, 64, 12288, True, 4, False), (RING, 597, 2048, True, 0, True),
+    (STAGED, 100, 4096, False, 0, False), (STAGED, 445, 2080, False, 1, True), (STAGED, 70, 2048, False, 2, False), (STAGED, 37, 4128, False, 3, False),
+    (STAGED, 300, 1056, False, 4, False), (STAGED, 593, 1536, False, 0, True),
+    (STAGED, 3, 66592, True, 0, False), (STAGED, 297, 1536, True, 1, False), (STAGED, 64, 2048, True, 4, True)])
+def test_the_forms_of_large_calls_on_rows_that_segments_take(form, rows, K, bf16, fmt, unit):
+    """The kernels that calls of more rows take, in every format, on the rows of the test of the segments: such calls are too large to check in number.  Ragged row groups and pieces, more
+    pieces than the ring holds, scale rows too long to meet in shared memory."""
+    assert rk.lib().rk_debug_rmsnorm_form(rows, K, bf16, 0) == SEGMENTS
+    with rmsnorm_form(form):
+        assert rk.lib().rk_debug_rmsnorm_form(rows, K, bf16, 0) == form
+        test_chains_cut_into_segments(rows, K, bf16, fmt, unit)
+
+
+@pytest.mark.parametrize("form,rows,K,bf16,fmt,unit", [(STAGED, 3600, 1056, False, 0, False), (RING, 9473, 2048, True, 1, False), (STAGED, 300, 1024, False, 2, False)])
+def test_the_forms_that_calls_take_by_themselves(form, rows, K, bf16, fmt, unit):
+    """fp32 rows of more than 1024 columns, more of them than lie on the chip at once; bf16 rows of a whole wave; short rows."""
+    if torch.cuda.get_device_properties(0).multi_processor_count <= 160:
+        assert rk.lib().rk_debug_rmsnorm_form(rows, K, bf16, 0) == form
+    test_chains_cut_into_segments(rows, K, bf16, fmt, unit)
