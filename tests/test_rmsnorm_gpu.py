@@ -198,3 +198,42 @@ def test_the_forms_that_calls_take_by_themselves(form, rows, K, bf16, fmt, unit)
     if torch.cuda.get_device_properties(0).multi_processor_count <= 160:
         assert rk.lib().rk_debug_rmsnorm_form(rows, K, bf16, 0) == form
     test_chains_cut_into_segments(rows, K, bf16, fmt, unit)
+
+
+def _us_per_call(call, calls=20):
+    """Median of replays of a graph of calls: neither the host nor a neighbour on the machine counts."""
+    call()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(calls):
+            call()
+    times = []
+    for _ in range(15):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        graph.replay()
+        start.record()
+        graph.replay()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(end) * 1000 / calls)
+    return sorted(times)[len(times) // 2]
+
+
+@pytest.mark.parametrize("rows,K,bf16", [(1, 4096, True), (300, 12288, True), (1, 4096, False), (300, 4096, False)])
+@pytest.mark.parametrize("kind", ["tiny", "nan", "inf"])
+def test_rows_that_are_added_as_they_lie_cost_a_chain(rows, K, bf16, kind):
+    """Rows whose sums stay below 2^-87 or hold a NaN or an infinity have no binade to take segments in, and one lane adds them up in the end: at the pace of the kernel that walks
+    every chain as it lies, plus the two passes over the segments (1.0-1.2 of its time; 2-4 where a segment at a time was looked up and added)."""
+    g = torch.Generator(device="cuda").manual_seed(97)
+    x = torch.randn(rows, K, generator=g, device="cuda")
+    if kind == "tiny":
+        x *= 2.0 ** -52
+    else:
+        x[:, 17] = float(kind)
+    x = x.bfloat16() if bf16 else x
+    gamma = torch.rand(K, generator=g, device="cuda") + 0.5
+    assert rk.lib().rk_debug_rmsnorm_form(rows, K, bf16, 0) == SEGMENTS
+    segments = _us_per_call(lambda: rk.rmsnorm_mx_quantize(x, gamma, 1e-5))
+    with rmsnorm_form(RING if bf16 else STAGED):
+        chain = _us_per_call(lambda: rk.rmsnorm_mx_quantize(x, gamma, 1e-5))
+    assert segments < 1.7 * chain, (segments, chain)
