@@ -121,6 +121,8 @@ def lib():
         L.rk_debug_set_prefill_form.argtypes = [C.c_int]
         L.rk_debug_prefill_form.restype = C.c_int
         L.rk_debug_prefill_form.argtypes = [C.POINTER(PrefillArgs), C.c_int]
+        L.rk_debug_prefill_prepares.restype = C.c_int
+        L.rk_debug_prefill_prepares.argtypes = [C.POINTER(PrefillArgs)]
         L.rk_debug_set_prefill_perturb.restype = None
         L.rk_debug_set_prefill_perturb.argtypes = [C.c_int]
         _LIB = L

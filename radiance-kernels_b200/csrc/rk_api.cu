@@ -624,11 +624,15 @@ RK_API int rk_debug_mxfp8_mma_loop(const uint8_t* a_tile, const uint8_t* b_tile,
  * the rule's choice for a call on a device of `sms` SMs (0 = the current one). */
 RK_API void rk_debug_set_prefill_form(int form) { g_prefill_form = form; }
 RK_API int rk_debug_prefill_form(const rk_prefill_args* a, int sms) { return prefill_form(*a, sms > 0 ? sms : num_sms()); }
+/* Test hook (not in the public header): 1 where the attention kernel of a call prepares its operands itself. */
+RK_API int rk_debug_prefill_prepares(const rk_prefill_args* a) { return prefill_prepares(*a) ? 1 : 0; }
 
 /* Test hook (not in the public header): which warp role of the prefill kernels sleeps a little at every key tile (0 = none;
  * 1, 2 = softmax of query tile A, B, of the lower and upper keys where a CTA has one query tile, of the two groups where they take the key tiles
- * in turn and at d = 256; 3 = correction, at d = 256 the upper keys' softmax warps; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer; 7 = O on its way out).
- * 100 + role: the role acts after a key tile as if its wait had run out (not 103 at d = 256, nor 107). */
+ * in turn and at d = 256; 3 = correction, at d = 256 the upper keys' softmax warps; 4 = TMA producer; 5 = Q K^T issuer; 6 = P V issuer; 7 = O on its way out;
+ * where the kernel prepares its operands itself, 8 = scale atoms of Q and K, 9 = V).
+ * 100 + role: the role acts after a key tile as if its wait had run out (not 103 at d = 256, nor 107); 108, 109: some of its warps do not hand over, and the waits for
+ * them run out. */
 RK_API void rk_debug_set_prefill_perturb(int role) { g_prefill_perturb = role; }
 
 }  // extern "C"

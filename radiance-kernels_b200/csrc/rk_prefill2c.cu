@@ -87,8 +87,10 @@ constexpr int lse_off = corr_off + 2 * 4 * 128 * 4;        // the same places: l
 constexpr int total = lse_off + 2 * 4 * 128 * 4;
 // test hook: which role sleeps a little at every key tile (schedule perturbation); kPerturbOut: at every chunk of O on its way out, and between the
 // softmax warps' last tile of an item and what they leave for it
+// PREP: kPerturbAtoms before the scale atoms of Q and of each key tile, kPerturbV before each unit of V; where these stop, some warps do not hand over (all but Q's;
+// the upper three quarters of V's keys, or its last tile's scales) and the waits for them run out.
 constexpr int kPerturbSoftmaxA = 1 /* 2 = softmax of tile B (SPLIT: of keys 64-127) */, kPerturbCorr = 3, kPerturbTma = 4, kPerturbQk = 5, kPerturbPv = 6,
-              kPerturbOut = 7;
+              kPerturbOut = 7, kPerturbAtoms = 8, kPerturbV = 9;
 // One work item: a pair of query tiles (SPLIT: one) of a (batch, head).
 struct __align__(16) Work {
   int qp;                  // pair index; -1: no item is left
@@ -715,22 +717,25 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       // Atoms of Q and of the key tiles by the three warps that have nothing to do before these are there.  (By one of them, atom after atom or all loads at once: one head of 256
       // keys 2 us more.)
 #pragma unroll 1
-      for (int a = warp - kWarpTma - 1; a <= w.nt0 && w.nt0 > 0; a += 3)
+      for (int a = warp - kWarpTma - 1; a <= w.nt0 && w.nt0 > 0; a += 3) {
+        perturb<DUMP>(p, kPerturbAtoms, a);
         scale_atom(a == 0 ? p.q_sf : p.k_sf, a == 0 ? w.bh : w.bhkv, a == 0 ? p.S_q : p.S_kv, a == 0 ? w.qp * kBlockM : (a - 1 + w.j0) * kBlockN, p.d / 32,
                    smem + (a == 0 ? sfq_off : sfk_off + (a - 1) * kSfAtomBytes), lane);
+      }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[bPrep]);
+      if (lane == 0 && !stops<DUMP>(p, kPerturbAtoms, warp - kWarpTma - 1)) mbar_arrive(&bars[bPrep]);
     } else if (!kPrepV) {
       if (warp < w.nt0 && __shfl_sync(0xffffffffu, lane == 0 ? *reinterpret_cast<volatile int*>(p.status) : 0, 0) == 0) {      // V's scales: a warp per key tile
         const int nkb = (p.S_kv + 31) / 32, block = (warp + w.j0) * 4;
         uint32_t words[4];
+        perturb<DUMP>(p, kPerturbV, warp);
         key_scale_words(p.v_sf + ((int64_t)w.bhkv * nkb + block) * p.d + lane * 4, p.d, nkb - block, lane * 4 < p.d, (reinterpret_cast<uintptr_t>(p.v_sf) & 3) == 0, words);
 #pragma unroll
         for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(smem + sfv_off + warp * kSfAtomBytes + sf_atom_offset(lane * 4 + i, 0)) = words[i];
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[bVF + warp]);
+        if (lane == 0 && !stops<DUMP>(p, kPerturbV, warp + 2 - w.nt0)) mbar_arrive(&bars[bVF + warp]);
       }
     } else if (warp < kWarpTma) {
       // V, by the twelve warps that have nothing to do before the first scores are there: units of 64 columns, in the order of the tiles; the correction warps, which are needed last, take
@@ -740,10 +745,11 @@ prefill2c_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll 1
         for (int i = grp; i < n; i += grp == 2 ? (i == 2 ? 1 : n) : 4) {
           const int st = units == 2 ? i >> 1 : i;
+          perturb<DUMP>(p, kPerturbV, i);
           rebase_v_unit<kPrepV ? PREP : 0>(p, smem, warp, lane, st, st + w.j0, units == 2 ? i & 1 : 0, w.bhkv);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[bVF + st]);
+          if (lane == 0 && !stops<DUMP>(p, kPerturbV, warp & 3)) mbar_arrive(&bars[bVF + st]);
         }
       }
     }

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import radiance_kernels_b200 as rk
-from radiance_kernels_b200._lib import DecodeArgs
+from radiance_kernels_b200._lib import DecodeArgs, PrefillArgs
 from helpers import PAIRS, SPLIT, TURNS, prefill_form, quantize_inputs, randn_qkv
 
 pytestmark = pytest.mark.gpu
@@ -284,6 +284,84 @@ def test_schedule_perturbation_in_both_kernels_of_narrow_heads(shape):
     """The delays of the test above where a CTA has some three query tiles one after the other, and where it has as many pairs of them."""
     H, S, d, cap, kw = shape
     test_schedule_perturbation_where_ctas_take_item_after_item((H, S, d, cap, kw))
+
+
+# heads, KV heads, queries, keys, d, V scaled along the keys, options
+PREPARED = [(2, 2, 100, 128, 64, False, {}), (8, 2, 130, 100, 128, False, dict(causal=False)), (3, 3, 128, 128, 128, True, {}), (2, 1, 70, 90, 64, True, dict(causal=False)),
+            (2, 2, 256, 256, 64, False, dict(causal=False)), (6, 2, 200, 250, 128, False, dict(q_pos0=50)), (4, 2, 256, 256, 128, True, {}), (2, 2, 129, 200, 64, True, dict(q_pos0=71)),
+            (16, 16, 300, 384, 128, False, dict(causal=False)), (16, 16, 384, 300, 128, False, dict(window=150)), (4, 2, 300, 300, 64, False, dict(q_pos0=-130)),
+            (6, 3, 384, 384, 64, False, {}), (4, 2, 260, 380, 128, True, dict(causal=False)), (4, 4, 300, 384, 64, True, dict(window=100, q_pos0=84))]
+
+
+def _prepared(H, Hkv, Sq, Skv, d, along_keys, kw, fmt=rk.E4M3):
+    """Operands, options and, asked of the library, that the attention kernel of this call prepares its operands itself."""
+    axis = rk.V_SCALES_ALONG_KEYS if along_keys else rk.V_SCALES_ALONG_D
+    kw = dict(dict(causal=True), **kw, v_scale_axis=axis, q_fmt=fmt, kv_fmt=fmt)
+    a = PrefillArgs()
+    a.B, a.H, a.H_kv, a.S_q, a.S_kv, a.d, a.v_scale_axis, a.q_fmt, a.kv_fmt = 1, H, Hkv, Sq, Skv, d, axis, fmt, fmt
+    a.causal, a.q_pos0, a.window = int(kw["causal"]), kw.get("q_pos0", 0), kw.get("window", 0)
+    assert rk.lib().rk_debug_prefill_prepares(C.byref(a))
+    return quantize_inputs(*randn_qkv(1, H, Hkv, Sq, Skv, d, seed=98), axis, fmt), kw
+
+
+@pytest.mark.parametrize("fmt", [rk.E4M3, rk.E5M2])
+@pytest.mark.parametrize("shape", PREPARED)
+def test_schedule_perturbation_where_the_kernel_prepares_its_operands(shape, fmt):
+    """The same in calls of one to three key tiles, with two roles more: the warps that put the scales of Q and K into atoms and those that re-block V, or put its scales into atoms."""
+    (qc, qs, kc, ks, vc, vs), kw = _prepared(*shape, fmt=fmt)
+    H, S = shape[0], shape[2]
+    lse0, lse = torch.empty(1, H, S, device="cuda"), torch.empty(1, H, S, device="cuda")
+    base = rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse0, **kw)
+    try:
+        for role in (1, 2, 3, 4, 5, 6, 7, 8, 9):
+            rk.lib().rk_debug_set_prefill_perturb(role)
+            for _ in range(2):
+                assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, lse=lse, **kw), base), role
+                assert torch.equal(lse, lse0), role
+    finally:
+        rk.lib().rk_debug_set_prefill_perturb(0)
+    assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [PREPARED[0], PREPARED[3], PREPARED[5], PREPARED[6], PREPARED[8], PREPARED[12]])
+def test_a_preparation_that_is_not_handed_over_ends_the_call_and_the_next_one_is_whole(shape):
+    """Some of the warps that prepare the operands do not hand over (scale atoms of K; keys of V's tiles, the scales of its last tile): the waits for them run out, with the
+    other roles' behind them, the call ends and the next one has every bit."""
+    (qc, qs, kc, ks, vc, vs), kw = _prepared(*shape)
+    L = rk.lib()
+    want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+    assert rk.last_device_status() == 0
+    for role in (8, 9):
+        L.rk_debug_set_prefill_perturb(100 + role)
+        try:
+            rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+            torch.cuda.synchronize()
+        finally:
+            L.rk_debug_set_prefill_perturb(0)
+            status = rk.last_device_status()
+        assert 100 < status < 600, (role, status)
+        assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw), want), role
+        assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [PREPARED[4], PREPARED[6], PREPARED[8], PREPARED[12]])
+def test_a_role_that_gives_up_where_the_kernel_prepares_its_operands(shape):
+    """The roles of the other tests, in calls of two and three key tiles of this kind: without a mask, so that all have a second tile."""
+    (qc, qs, kc, ks, vc, vs), kw = _prepared(*shape[:-1], dict(causal=False))
+    L = rk.lib()
+    want = rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+    assert rk.last_device_status() == 0
+    for role in (1, 2, 3, 4, 5, 6):
+        L.rk_debug_set_prefill_perturb(100 + role)
+        try:
+            rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw)
+            torch.cuda.synchronize()
+        finally:
+            L.rk_debug_set_prefill_perturb(0)
+            status = rk.last_device_status()
+        assert 100 < status < 600, (role, status)
+        assert torch.equal(rk.attn_prefill(qc, kc, vc, qs, ks, vs, **kw), want), role
+        assert rk.last_device_status() == 0
 
 
 def test_tensor_pipe_ceiling_loop_never_runs_into_its_waits():
