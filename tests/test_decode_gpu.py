@@ -256,6 +256,33 @@ def test_kv_cache_append_then_decode_in_a_loop(fmt):
     assert np.array_equal(np_(vc[0, 0, :T]), oc) and np.array_equal(np_(vs[0, 0, :T]), os_)
 
 
+# 0 sequences: as many as it takes for a second pass of the append kernel's grid (four CTAs of 128 threads per SM for K and as many for V, 8 elements a thread)
+@pytest.mark.parametrize("B,Hkv,L,d,fmt", [(1, 1, 1, 32, rk.E4M3), (3, 5, 2, 96, rk.E5M2), (7, 3, 4, 64, rk.E2M1), (33, 1, 3, 160, rk.E2M3), (5, 2, 300, 256, rk.E3M2),
+                                           (0, 2, 3, 128, rk.E4M3), (0, 3, 2, 96, rk.E3M2), (0, 1, 2, 32, rk.E4M3)])
+def test_kv_cache_append_writes_the_rows_it_is_given_and_no_other(B, Hkv, L, d, fmt):
+    """Row widths that are no power of two, numbers of chunks that do not fill a warp, one thread's second row; positions outside the cache are skipped; rows of
+    zeros and blocks with a NaN or an infinity among the new ones."""
+    if B == 0:
+        B = -(-(torch.cuda.get_device_properties(0).multi_processor_count * 4 * 128 + 77) * 8 // (Hkv * d))
+    rng = np.random.default_rng(B + d)
+    new = [(rng.standard_normal((B, Hkv, d)) * np.exp2(rng.integers(-8, 9, (B, Hkv, 1)))).astype(np.float32) for _ in range(2)]
+    new[0][B // 2, 0] = 0.0
+    if B > 2:
+        new[0][B - 1, Hkv - 1, d - 1] = np.inf
+        new[1][0, 0, 3] = np.nan
+    pos = rng.integers(0, L, B).astype(np.int32)
+    pos[1::7], pos[2::7], pos[4::7] = -1, L, 2 ** 31 - 1
+    cache = [torch.full((B, Hkv, L, n), 0xA5, dtype=torch.uint8, device="cuda") for n in (d, d // 32) * 2]
+    rk.kv_cache_append(*(torch.from_numpy(x).cuda() for x in new), torch.from_numpy(pos).cuda(), *cache, fmt=fmt)
+    torch.cuda.synchronize()
+    inside = np.flatnonzero((pos >= 0) & (pos < L))
+    for x, got in zip(new, (cache[:2], cache[2:])):
+        for part, rows in zip(got, oracle.quantize(x.reshape(B * Hkv, d), fmt)):
+            want = np.full(part.shape, 0xA5, np.uint8)
+            want[inside, :, pos[inside]] = rows.reshape(B, Hkv, -1)[inside]
+            assert np.array_equal(np_(part), want)
+
+
 @pytest.mark.parametrize("grp,case", [(4, "short"), (8, "short"), (4, "many"), (8, "many"), (4, "rising"), (8, "rising"), (4, "v jump"), (8, "v jump"), (1, "few tiles")])
 def test_ranges_and_references(grp, case):
     """The tcgen05 kernel's equal ranges of tiles and its running references: a few and many short sequences per CTA (empty ones,
