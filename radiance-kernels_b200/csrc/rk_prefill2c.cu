@@ -586,25 +586,8 @@ __device__ __forceinline__ void rebase_v_unit(const PrefillParams& p, uint8_t* s
 
 // PREP: the scale atom of 128 rows from row0 of a matrix of S rows, by one warp, four rows a lane.
 RK_DEVINL void scale_atom(const uint8_t* scales, int64_t bh, int S, int row0, int nbd, uint8_t* atom, int lane) {
-  const uintptr_t at = reinterpret_cast<uintptr_t>(scales);
-  const uint8_t* src = scales + (bh * S + row0 + lane) * nbd;
-  const int n = S - row0 - lane;                              // row i * 32 exists if it is below
   uint32_t w[4];
-  if (nbd == 4 && (at & 3) == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = i * 32 < n ? __ldg(reinterpret_cast<const uint32_t*>(src + i * 128)) : 0x7F7F7F7Fu;
-  } else if (nbd == 2 && (at & 1) == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = i * 32 < n ? 0x7F7F0000u | __ldg(reinterpret_cast<const uint16_t*>(src + i * 64)) : 0x7F7F7F7Fu;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t c[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) c[k] = k < nbd && i * 32 < n ? (uint32_t)__ldg(src + i * 32 * nbd + k) : 0x7Fu;
-      w[i] = c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24);
-    }
-  }
+  row_scale_words(scales + (bh * S + row0 + lane) * nbd, scales, nbd, S - row0 - lane, nbd, w);
 #pragma unroll
   for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(atom + sf_atom_offset(i * 32 + lane, 0)) = w[i];
 }

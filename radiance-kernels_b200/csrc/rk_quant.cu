@@ -1193,20 +1193,19 @@ RK_DEVINL void retile_atom(const RetileJob& job, int64_t atom, int64_t total) {
     for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(out + sf_atom_offset(lane * 4 + i, 0)) = w[i];
     return;
   }
-  const bool words = job.kind == kRows && nbd % 4 == 0 && (reinterpret_cast<uintptr_t>(job.in) & 3) == 0;
+  const int64_t row = tile * 128 + lane;
+  if (job.kind == kRows) {
+    row_scale_words(job.in + (bt * S + row) * nbd + ch * 4, job.in, nbd, (int)min((int64_t)128, S - row), (int)min((int64_t)4, nbd - ch * 4), w);
+  } else {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t row = tile * 128 + i * 32 + lane;
-    w[i] = 0x7F7F7F7Fu;
-    if (row < S) {
-      if (words) {
-        w[i] = *reinterpret_cast<const uint32_t*>(job.in + (bt * S + row) * nbd + ch * 4);
-      } else {
+    for (int i = 0; i < 4; ++i) {
+      w[i] = 0x7F7F7F7Fu;
+      if (row + i * 32 < S) {
         w[i] = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           const int64_t blk = ch * 4 + k;
-          w[i] |= (blk < nbd ? (uint32_t)job.in[job.kind == kRows ? (bt * S + row) * nbd + blk : (bt * nbd + blk) * S + row] : 0x7Fu) << (8 * k);
+          w[i] |= (blk < nbd ? (uint32_t)job.in[(bt * nbd + blk) * S + row + i * 32] : 0x7Fu) << (8 * k);
         }
       }
     }

@@ -529,3 +529,22 @@ def test_calls_that_prepare_their_operands_themselves(S_q, S_kv, d, fmt, kw, har
             assert torch.equal(got.view(torch.int16), want.view(torch.int16))
             assert torch.equal(lse[1], lse[0])
     assert rk.last_device_status() == 0
+
+
+@pytest.mark.parametrize("S_q,S_kv,d,fmt", [(130, 700, 64, rk.E4M3), (257, 513, 64, rk.E2M3), (33, 640, 128, rk.E4M3), (300, 600, 256, rk.E4M3), (140, 200, 256, rk.E2M1)])
+def test_scales_at_any_address(S_q, S_kv, d, fmt):
+    """Row-major scales of calls with a preparation launch, read as words, halves or bytes: the same bits from every address, ragged tiles among them."""
+    g = torch.Generator(device="cuda").manual_seed(S_q + d)
+    q, qs = rk.mx_quantize(torch.randn(2, 4, S_q, d, generator=g, device="cuda"), fmt)
+    k, ks = rk.mx_quantize(torch.randn(2, 2, S_kv, d, generator=g, device="cuda"), fmt)
+    v, vs = rk.mx_quantize(torch.randn(2, 2, S_kv, d, generator=g, device="cuda"), fmt)
+    def moved(t, n):
+        flat = torch.full((t.numel() + n + 256,), 0xFE, dtype=torch.uint8, device="cuda")
+        flat[n:n + t.numel()] = t.flatten()
+        return flat[n:n + t.numel()].view(t.shape)
+    kw = dict(causal=True, q_pos0=S_kv - S_q, q_fmt=fmt, kv_fmt=fmt)
+    with prefill_form(PAIRS):
+        want = rk.attn_prefill(q, k, v, qs, ks, vs, **kw)
+        for n in (1, 2, 3):
+            assert torch.equal(rk.attn_prefill(q, k, v, moved(qs, n), moved(ks, n), moved(vs, n), **kw), want), n
+    assert rk.last_device_status() == 0
