@@ -168,7 +168,6 @@ RK_DEVINL uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f
 RK_DEVINL uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 RK_DEVINL uint64_t fma_sq_f32x2(uint64_t v, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(v), "l"(c)); return d; }
 
-// (Scalar products on purpose: mul.f32x2 takes two cycles of the heavy FMA pipe, and packing its operands adds moves.)
 // max(|a|, |b|, |c|), NaN if any of them is
 RK_DEVINL float max3_abs_nan(float a, float b, float c) { float d; asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 RK_DEVINL float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
@@ -179,7 +178,8 @@ RK_DEVINL float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2
 // reference's compare loop does, and the integer encoder.  A caller runs the hot form over all it has and the cold one
 // again only if some block asked for it, so that the hot loop carries no code that never runs.
 // UNIT: no block scale (codes under 2^0, scale code 127).  PACKED: products two at a time, where issue slots are short (RMSNorm: 16384 x 4064 bf16
-// 68.6 -> 67.2 us, 8192 x 4096 fp32 50.4 -> 49.6).
+// 68.6 -> 67.2 us, 8192 x 4096 fp32 50.4 -> 49.6); scalar in the quantizer and RoPE, which HBM bounds: mul.f32x2 takes two cycles of the heavy FMA pipe, and packing its operands
+// adds moves.
 template <int FMT, bool UNIT, int N, bool COLD, bool PACKED = false> RK_DEVINL bool quantize_lanes(const float (&v)[N][8], int lane, uint2 (&w)[N], uint32_t& scode) {
   constexpr int kLanes = 4 / N;
   const uint32_t mask = (0xFu >> (4 - kLanes)) << (lane & (32 - kLanes));
@@ -735,7 +735,7 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
   if (__syncthreads_or(!ok)) {
     // the copies under way, whichever role gave up, before shared memory goes to another CTA
     for (int c = max(0, issued - kStages); c < issued; ++c) wait(&full[c % kStages], c / kStages);
-    if (threadIdx.x == 0) atomicCAS(status, 0, 602);
+    if (threadIdx.x == 0) atomicCAS(status, 0, 602);                   // an RMSNorm call's copies, in this kernel and the one below
     return;
   }
   rmsnorm_rows<FMT, true, UNIT, 16, kThreads>(xr, row0, n_rows, K, gamma, rms_row, codes, scales, rmb_smem, kStages * kPitch);
@@ -761,13 +761,13 @@ namespace rms_seg {
 constexpr int kThreads = 256, kWarps = kThreads / 32, kCtasPerSm = 3, kMaxRows = 8;
 constexpr int kSmem = 227 * 1024, kStatic = 1024, kReserved = 1024;     // of an SM; of a CTA beside its dynamic part, ours and the system's
 constexpr uint32_t kMarked = 0x3FF;                                     // in the place of an exponent
-constexpr int kLongest = 72;                                            // elements of a segment
+constexpr int kLongest = 72;                                            // elements of a segment, before they are rounded up to whole pieces (24 to 72 bf16, 20 to 76 fp32 then)
 
 // How a call is laid out: rows per CTA, warps that share a row's segments, segment in elements, bytes from row to row in shared memory.
 struct Shape { int rows, warps, seg, pitch; int64_t smem, grid; };
 // Segments are an odd number of 16-byte pieces, so that eight lanes reading 16 bytes of their own find eight bank groups.
 static Shape shape(int64_t n, int K, bool bf16, int rows) {
-  const int elem = bf16 ? 2 : 4, piece = 16 / elem, least = rows == 1 && !bf16 ? 24 : 40;      // shorter segments do not pay: more of them to go over in the end
+  const int elem = bf16 ? 2 : 4, piece = 16 / elem, least = rows == 1 && !bf16 ? 24 : 40;      // elements: a row goes to more warps while their segments are longer than these
   Shape f;
   f.rows = rows;
   f.warps = 1;
@@ -1159,9 +1159,6 @@ __global__ void __launch_bounds__(128) quantize_keys_kernel(const float* __restr
   }
 }
 
-// Exact value of element code `c` times 2^(s-127) as an fp32.  Normal codes under ordinary scales are
-// placed by integer arithmetic (E4M3: bits = (mag + 8 s - 56) << 20); everything else (subnormal codes,
-// scale codes near the ends of the range, the other formats) takes the generic multiply.
 // Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one warp per atom, a lane writes the 16 bytes of rows or columns lane,
 // lane + 32, + 64 and + 96; rows, columns and blocks past the edge get code 0x7F = 2^0.  (A thread per row or column, with the divisions that find its place, was a fifth
 // of the time of the re-blocking kernel beside which the scales of Q and K are re-tiled: 8 x 16 heads of 4096, d = 128, 33.8 -> 31.6 us, 4 x 32 / 8 of 8192 22.2 -> 18.8, 2 x 16 / 8 of 8192, d = 256, 20.2 -> 18.5.)

@@ -28,6 +28,9 @@ template <int FMT> RK_DEVINL uint32_t hw_encode4(float a, float b, float c, floa
         : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
   return r;
 }
+// Exact value of element code `c` times 2^(s-127) as an fp32.  Normal codes under ordinary scales are
+// placed by integer arithmetic (E4M3: bits = (mag + 8 s - 56) << 20); everything else (subnormal codes,
+// scale codes near the ends of the range, the other formats) takes the generic multiply.
 template <int FMT> RK_DEVINL float decode_scaled(uint32_t c, uint32_t s) {
   if (FMT == 0) {
     const uint32_t mag = c & 0x7Fu;
