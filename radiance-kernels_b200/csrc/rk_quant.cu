@@ -754,8 +754,8 @@ rmsnorm_quantize_bulk_kernel(const uint8_t* __restrict__ x, int64_t rows, int K,
 // pieces of 16 bytes at a time, so that the addition's latency is what counts.  One row of 4096 bf16 of 2^-52 N(0,1) 17.6 us (the chain as it lies in the ring 15.6, a run per segment
 // 40.7), fp32 19.7 (17.2, 76.3), 300 rows of 12288 bf16 49.6 (45.7, 155.6), 1200 of 4096 24.0 (19.5, 47.6); N(0,1) gains by it too (300 rows of 4096 fp32 11.0 -> 9.8, one 9.0 -> 7.7).
 //
-// One row of 4096 bf16: 15.5 -> 7.3 us, 12288 columns 42.0 -> 9.8; 300 rows of 4096 17.4 -> 9.1, 1500 rows 20.1 -> 15.0.  With more rows on an SM than its shared memory holds the
-// rounds of CTAs follow one another with little overlap, and the ring above, whose chains all run at once, is faster (4500 rows 25.3, so 33.8).
+// One row of 4096 bf16: 15.7 -> 7.2 us, 12288 columns 42.1 -> 10.0; 300 rows of 4096 17.5 -> 8.9, 1500 rows 19.8 -> 13.9; fp32, one row of 4096 17.3 -> 7.4.  With more rows on an SM than its shared
+// memory holds the rounds of CTAs follow one another with little overlap, and the ring above, whose chains all run at once, is faster (4500 rows 25.3, so 33.8).
 // The quantization reads the rows where they are; products two at a time (88 instead of 112 instructions per 16 elements and lane).
 namespace rms_seg {
 constexpr int kThreads = 256, kWarps = kThreads / 32, kCtasPerSm = 3, kMaxRows = 8;
@@ -781,10 +781,11 @@ static Shape shape(int64_t n, int K, bool bf16, int rows) {
   f.grid = (n + rows - 1) / rows;
   return f;
 }
-// Where this kernel is the faster one (times per call, us, staged or by the ring and so): from more than 1024 columns on (512 3.9 4.8, 1024 5.5 5.2 to 9.0 9.8, 1536 7.2 5.5) as long
-// as all CTAs are on the SMs in one round, and in more rounds the longer the chain is that the others have to wait for (6144 columns 1500 rows 27.8 19.8, in two rounds 2200 rows
-// 29.4 32.2; 8192 columns in two rounds 1500 rows 35.6 23.7, in three 2200 37.6 37.4; 12288 columns 1500 rows 52.3 37.3).  fp32 from 1777 rows on, eight of them to a CTA, is
-// level (2048 columns, 2200 rows 16.4 16.7; 3000 17.8 17.7).
+// Where this kernel is the faster one: from more than 1024 columns on (512 3.9 4.8, 1024 5.5 5.2 to 9.0 9.8: us, staged or by the ring and so) as long as all CTAs are on the SMs in one
+// round, and in more rounds the longer the chain is that the others have to wait for.  Its time over theirs, 1 / 300 / 888 / 1776 / 2400 / 3552 rows of bf16: 1056 columns 0.90 0.88 0.91 0.95
+// 1.08 1.05, 1152 0.87 0.89 0.88 0.94 1.04 1.03, 1280 0.84 0.83 0.84 0.89 1.01 0.97, 1536 0.76 0.75 0.76 0.80 0.91 0.89, 2048 0.65 0.74 0.80 0.84 0.97 0.96, 4096 0.48 0.54 0.62 0.75 0.85 0.81;
+// 8192 (two and three rounds) 0.33 0.38 0.48 0.61 0.92 0.97, 12288 0.25 0.31 0.40 0.69 0.87, 16384 0.21 0.28 0.37 0.64 0.85 1.00.  So eight rows to a CTA, above 1776 of them, from more than 1280 columns on.
+// fp32, four rows to a CTA at most: 1056 columns 0.92 0.87 0.89 0.90, 4096 0.43 0.44 0.50 0.63, 16384 0.19 0.24 0.43 0.77; eight are level (2048 columns, 2200 rows 16.4 16.7; 3000 17.8 17.7).
 static bool pays(int64_t n, int K, bool bf16, int64_t sms, Shape& f) {
   if (K <= 1024 || K > (1 << 17)) return false;
   f = shape(n, K, bf16, 1);
@@ -793,6 +794,7 @@ static bool pays(int64_t n, int K, bool bf16, int64_t sms, Shape& f) {
     if (two.smem + kStatic / 2 + kReserved > kSmem / kCtasPerSm) break;
     f = two;
   }
+  if (f.rows == kMaxRows && K <= 1280) return false;
   const int64_t per_sm = std::min<int64_t>(kCtasPerSm, kSmem / (f.smem + kStatic / 2 + kReserved));
   return per_sm > 0 && f.grid <= per_sm * sms * std::max(1, K / 4096);
 }
