@@ -1163,7 +1163,8 @@ __global__ void __launch_bounds__(128) quantize_keys_kernel(const float* __restr
 
 // Scale-factor atoms [batch][ntile][dch][512] from the other layouts of block scales: one warp per atom, a lane writes the 16 bytes of rows or columns lane,
 // lane + 32, + 64 and + 96; rows, columns and blocks past the edge get code 0x7F = 2^0.  (A thread per row or column, with the divisions that find its place, was a fifth
-// of the time of the re-blocking kernel beside which the scales of Q and K are re-tiled: 8 x 16 heads of 4096, d = 128, 33.8 -> 31.6 us, 4 x 32 / 8 of 8192 22.2 -> 18.8, 2 x 16 / 8 of 8192, d = 256, 20.2 -> 18.5.)
+// of the time of the re-blocking kernel beside which the scales of Q and K are re-tiled: 8 x 16 heads of 4096, d = 128, 33.8 -> 31.6 us, 4 x 32 / 8 of 8192 22.2 -> 18.8, 2 x 16 / 8 of 8192, d = 256, 20.2 -> 18.5.
+// Row-major and group-major scales in one loop, a row after the other: 8 / 2 heads of 640 keys, d = 128, group-major 12.6 -> 13.9 us a call, apart 11.9; 2 x 16 / 8 of 700, d = 256, 20.4, 21.2, 20.4.)
 //   kRows   along d, row-major [batch][S][d/32]
 //   kGroups along d, group-major [batch][d/32][S] (the reference's QK_A_scales_row[FA_GK][FA_SQ] per head,
 //           kernels/flash_attention_mx/gen_data.py:82-83)
